@@ -491,6 +491,19 @@ def test_linear_simt(K, M, N, K_, adt, wdt):
     assert torch.allclose(got.cpu().double(), x.double() + want + b.double(), atol=1e-4, rtol=1e-5)
 
 
+@pytest.mark.parametrize("M", [1, 4, 5, 16, 17, 64, 65])
+@pytest.mark.parametrize("N,K_", [(96, 352), (33, 300), (2056, 132), (130, 1217), (12300, 48)])
+def test_linear_simt_ranges_of_k(K, M, N, K_):
+    """Both kernels (up to 16 rows, more), every number of ranges, rows and columns beside the tiles: against float64, and a row's sums
+    are bit for bit the same whatever kernel it runs in."""
+    a, w = rnd(70, K_, seed=1), rnd(N, K_, seed=2)
+    want = a[:M].double() @ w.double().T
+    got = K.linear_simt(dev(a[:M].contiguous()), dev(w), out_dtype=torch.float32)
+    # K products and sums of about unit size in float32: an error of about sqrt(K) * 2^-24 * sqrt(K) at most a few times over
+    assert float((got.cpu().double() - want).abs().max()) <= 8 * K_ * 2.0 ** -24
+    assert torch.equal(got, K.linear_simt(dev(a), dev(w), out_dtype=torch.float32)[:M])
+
+
 def test_linear_simt_rows_do_not_depend_on_their_neighbours(K):
     a, w = rnd(70, 352, seed=1), rnd(96, 352, seed=2)
     whole = K.linear_simt(dev(a), dev(w), out_dtype=torch.float32)
