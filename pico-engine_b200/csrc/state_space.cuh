@@ -1,0 +1,24 @@
+// What the recurrence of the state-space mixer (state_space.cu) and its form as products of tiles (state_space_tiles.cu) share.
+#pragma once
+#include "common.cuh"
+
+#define SS_CHUNK 64          // tokens of a chunk of a prompt
+
+struct ScanArgs {
+    const float* xbc; int xbc_ld;             // [T, inner + 2 G N] float32: x | B | C after the convolution
+    const void* proj; int proj_ld, dt_off;    // dt_raw at columns dt_off .. dt_off + H - 1 of proj (the step's dtype)
+    const void* dt_bias; int dtb_dtype; const void* a_log; int al_dtype; const void* d_skip; int d_dtype;   // [H] each
+    float* state; long long state_stride;     // row slots[b] holds the sequence's state
+    const int* row_first; const int* row_lens; const int* slots;
+    float* y;                                 // [T, H * P]
+    int B, H, P, N, G, NS, NR, NRP, PT;
+    float* chunk_state;                       // [chunks][H][N][P]: a chunk's own contribution, then its incoming state
+    float* chunk_decay;                       // [chunks][H]: the product of a chunk's decays
+    float* chunk_scores;                      // [chunks][G][64 s][64 t]: C_t . B_s
+    int max_chunks;
+};
+
+__device__ __forceinline__ float ss_silu(float v) { return v / (1.0f + expf(-v)); }
+__device__ __forceinline__ float ss_softplus(float v) { return fmaxf(v, 0.f) + log1pf(expf(-fabsf(v))); }
+
+int ss_tiles(const ScanArgs& a, int dtype, cudaStream_t s);     // prompts: contributions, carry, outputs

@@ -1259,9 +1259,9 @@ def state_space_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_offset: int, dt_b
                      n_heads: int, head_dim: int, n_state: int, n_groups: int, chunked: bool = False) -> torch.Tensor:
     """y float32 [T, H * P] of S_t = exp(-exp(A_log) dt) S_(t-1) + dt B_t x_t^T, y_t = S_t^T C_t + D x_t with dt = softplus(raw + bias):
     x | B | C are the columns of ``xbc`` float32 [T, H*P + 2 G N], the raw step sizes columns ``dt_offset`` .. of proj.  The states
-    come from and return to the sequences' float32 state at ``state_offset``.  ``chunked``: prompts, three launches over chunks of 64
-    tokens (every chunk from zero, a carry pass, every chunk from its incoming state) instead of one walk a sequence; both give the
-    same numbers up to float32 rounding."""
+    come from and return to the sequences' float32 state at ``state_offset``.  ``chunked``: prompts, as products of tiles over chunks of 64
+    tokens (three launches: every chunk's contribution to the state, a carry pass, the outputs) instead of one walk a sequence; both give
+    the same numbers up to float32 rounding."""
     from .library import state_space
     T = xbc.shape[0]
     H, P, N, G = n_heads, head_dim, n_state, n_groups
@@ -1273,7 +1273,7 @@ def state_space_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_offset: int, dt_b
     ws = 0
     if chunked:
         from .workspace import scratch
-        ws = scratch("state_space_scan", 4 * state_space().pe_state_space_scratch_floats(T, slots.shape[0], H, P, N), xbc.device).data_ptr()
+        ws = scratch("state_space_scan", 4 * state_space().pe_state_space_scratch_floats(T, slots.shape[0], H, P, N, G), xbc.device).data_ptr()
     check(state_space().pe_state_space_scan(xbc.data_ptr(), xbc.shape[1], proj.data_ptr(), _code(proj, "proj"), proj.shape[1], dt_offset,
                                             dt_bias.data_ptr(), _code(dt_bias, "dt_bias"), a_log.data_ptr(), _code(a_log, "a_log"),
                                             d_skip.data_ptr(), _code(d_skip, "d_skip"), sp, stride, row_first.data_ptr(),

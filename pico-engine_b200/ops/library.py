@@ -27,7 +27,7 @@ MIXER_SOURCES = ("layernorm_conv.cu", "attention_headmix.cu", "attention_headmix
 GATED_SOURCES = ("linear_attention.cu", "linear_attention_tiles.cu", "gated_ops.cu", "branch_ops.cu")
 # The kernels of the state-space mixer (short convolution with silu, the recurrence with a scalar decay, gate then norm) and of
 # attention over one low-rank row per position.
-STATE_SOURCES = ("state_space.cu", "latent_ops.cu")
+STATE_SOURCES = ("state_space.cu", "state_space_tiles.cu", "latent_ops.cu")
 # The kernels of sublayers that read the same rows and share their first and last product, of heads with several maps, and of routers
 # that read normed rows.
 JOINED_SOURCES = ("joined_ops.cu", "attention_diff.cu", "attention_diff_tcgen05.cu")
@@ -223,7 +223,7 @@ def state_space() -> ctypes.CDLL:
         lib.pe_state_space_split.restype = c_int
         lib.pe_state_space_elems.argtypes = [I, I, I]
         lib.pe_state_space_elems.restype = c_longlong
-        lib.pe_state_space_scratch_floats.argtypes = [I, I, I, I, I]
+        lib.pe_state_space_scratch_floats.argtypes = [I, I, I, I, I, I]
         lib.pe_state_space_scratch_floats.restype = c_longlong
         _state = lib
     return _state

@@ -73,20 +73,10 @@ class StateSpace(Mixer):
         return CacheNeeds(kv=None, state_elems=self.matrix_state_elems() + (s.taps - 1) * self._sizes()[2])
 
     def chunks_pay(self, lens) -> bool:
-        """Whether a step with these numbers of tokens a row runs its recurrence in chunks.  One walk a sequence takes as long as
-        the longest row, however empty that leaves the GPU; in chunks of 64 every token is walked twice, but all chunks run side
-        by side.  Both are counted in token times a wave of blocks (about two blocks of 256 threads an SM on 148 SMs), the
-        carry pass as one chunk more.  Either way gives the same numbers up to float32 rounding."""
-        longest = max(lens, default=0)
-        if longest <= 64:
-            return False
-        s = self.spec
-        split = kernels.state_space_split(s.state)
-        per = s.n_heads * -(-s.head_dim // min(s.head_dim, 256 // split))     # blocks a sequence or chunk
-        wave = 296
-        walk = longest * -(-sum(1 for n in lens if n > 0) * per // wave)
-        chunks = sum(-(-n // 64) for n in lens)
-        return 64 * (2 * -(-chunks * per // wave) + 1) < walk
+        """Whether a step with these numbers of tokens a row runs its recurrence as products of tiles over chunks of 64 tokens.  One walk
+        a sequence takes as long as the longest row (0.7 us a token on a B200, where a chunk of 64 takes 20 us at least
+        whatever it holds), so it is left to rows that bring a few tokens.  Either way gives the same numbers up to float32 rounding."""
+        return max(lens, default=0) > 16
 
     def normed_output(self, h, ctx, cache_entry):
         s = self.spec

@@ -376,6 +376,14 @@ def test_state_space_kernels(dtype, H, P, N, G, taps, groups):
             assert (got.double() - want).abs().max() < tol, (cuts, chunked)
 
 
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("H,P,N,G,taps,groups", [(2, 72, 130, 1, 4, 1), (4, 64, 128, 2, 3, 2), (1, 68, 33, 1, 2, 1), (20, 64, 20, 1, 4, 1), (36, 64, 4, 2, 4, 1)])
+def test_state_space_kernels_at_the_edges_of_their_tiles(dtype, H, P, N, G, taps, groups):
+    """More state rows than 128 and columns than 64, sizes that fill a tile, sizes whose rows are no whole vectors, norms over runs of
+    more than 1,024 and 2,048 channels."""
+    test_state_space_kernels(dtype, H, P, N, G, taps, groups)
+
+
 @pytest.mark.parametrize("far", [0, 1, 7, 8, 9, 63, 64, 65, 447, 511, 512])
 def test_state_keeps_an_input_from_far_back(far):
     """With a decay of nearly 1 an input whose B matches the last token's C must come through from any distance: the first
