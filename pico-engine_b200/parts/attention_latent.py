@@ -113,9 +113,16 @@ class LatentAttention(Mixer):
         kernels.latent_prepare(proj, H, D, R, rank, q_w, self.dkv_norm, s.norm_eps, self.freq, s.position.dims, None,
                                ctx.tok_pos, ctx.tok_row, kv.k if owns_cache else None, kv.table if owns_cache else None, kv.stride,
                                halves=isinstance(s.position, RotaryHalvesSpec), q_rows=q_rows, q_out=q)
-        a = kernels.attention_headmix(q, q.shape[1], H, 1, rank + R, rank, kv.k, None, kv.table, kv.stride, ctx.tok_pos, ctx.tok_row,
-                                      s.window, s.scale, None, None, ctx, values_in_keys=True)
-        if s.gate is None:                                 # no gate: the batched product writes token-major rows itself
+        # prompts: the gate, a number a head and token, is applied to the heads' rows before the batched product (it commutes with it)
+        gated = s.gate is None
+        a = kernels.attention_latent_prompt(q, q.shape[1], H, rank + R, rank, kv.k, kv.table, kv.stride, s.window, s.scale, ctx,
+                                            None if gated else proj, q_w + dkv_w)
+        if a is not None:
+            gated = True
+        else:
+            a = kernels.attention_headmix(q, q.shape[1], H, 1, rank + R, rank, kv.k, None, kv.table, kv.stride, ctx.tok_pos, ctx.tok_row,
+                                          s.window, s.scale, None, None, ctx, values_in_keys=True)
+        if gated:                                          # nothing follows the batched product: it writes token-major rows itself
             out = torch.empty(T, H * s.v_head_dim, dtype=a.dtype, device=a.device)
             torch.bmm(a.view(T, H, rank).transpose(0, 1), self.w_uv, out=out.view(T, H, s.v_head_dim).transpose(0, 1))
             return out

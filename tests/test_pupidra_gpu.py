@@ -297,6 +297,51 @@ def test_a_key_from_far_back(dtype, far):
             assert (got[-1] - 8.0).abs().max() < 0.1, (far, in_keys, got[-1])
 
 
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("H,width,rank,window", [(1, 64, 64, None), (3, 96, 64, 70), (14, 160, 128, None), (5, 192, 128, 128), (2, 256, 192, None),
+                                                 (16, 256, 192, 200), (2, 208, 192, 1)])
+def test_prompts_over_low_rank_rows(H, width, rank, window, gated):
+    """The tcgen05 kernel at every number of panels: whole prompts and portions that begin and end off the borders of pages and of runs
+    of 128 tokens, several sequences in a step, pages that the window has left given back, a gate a head."""
+    from pico_engine.ops import kernels
+    g = torch.Generator().manual_seed(H * 1000 + width)
+    lens, dt = [1, 63, 129, 470], torch.bfloat16
+    scale = 1.5 * width ** -0.5
+    q, k = (torch.randn(sum(lens), h, width, generator=g).to(dt).float() for h in (H, 1))
+    logits = (2 * torch.randn(sum(lens), H + 3, generator=g)).to(dt)
+    pages = sum((n + 63) // 64 for n in lens)
+    pool = torch.full((pages + 1, 1, 64, width), 3.0, dtype=dt)          # what no sequence has written is not seen
+    table = torch.full((len(lens), 9), -1, dtype=torch.int32)
+    want, at, page = [], 0, 1
+    for b, n in enumerate(lens):
+        for j in range((n + 63) // 64):
+            m = min(64, n - 64 * j)
+            pool[page, 0, :m], table[b, j], page = k[at + 64 * j: at + 64 * j + m, 0].to(dt), page, page + 1
+        i, j = torch.arange(n)[:, None], torch.arange(n)[None]
+        seen = (j <= i) if window is None else (j <= i) & (i - j < window)
+        s = torch.einsum("ihd,jd->hij", q[at: at + n].double(), k[at: at + n, 0].double()) * scale
+        w = torch.softmax(s.masked_fill(~seen, float("-inf")), -1)
+        want.append(torch.einsum("hij,jd->ihd", w, k[at: at + n, 0, :rank].double()))
+        at += n
+    want = torch.cat(want)
+    if gated:
+        want = want * torch.sigmoid(logits[:, 2: 2 + H].double())[..., None]
+    want = want.reshape(-1, H * rank)
+    first = np.concatenate([[0], np.cumsum(lens)])
+    for cuts in ([(0, n) for n in lens], [(n // 3, n) for n in lens], [(n - min(n, 2), n) for n in lens]):
+        idx = torch.cat([torch.arange(first[b] + lo, first[b] + hi) for b, (lo, hi) in enumerate(cuts)])
+        tab = table.clone()
+        if window is not None:
+            for b, (lo, _) in enumerate(cuts):
+                tab[b, : max(0, lo - window + 1) // 64] = -1
+        ctx = SimpleNamespace(one_token_each=False, scratch={}, lens=[hi - lo for lo, hi in cuts], starts=[lo for lo, _ in cuts], dtype=dt)
+        got = kernels.attention_latent_prompt(q[idx].reshape(len(idx), -1).to(dt).cuda(), H * width, H, width, rank, pool.cuda(), tab.cuda(), tab.shape[1],
+                                              window, scale, ctx, logits[idx].cuda() if gated else None, 2)
+        kernels.check_status(torch.device("cuda", torch.cuda.current_device()))
+        # weights and results are rounded to bfloat16 (2^-9 each), values reach four: 2e-2 as for the other bfloat16 attention kernels
+        assert (got.double().cpu() - want[idx]).abs().max() < 2e-2 * max(1.0, float(want.abs().max())), cuts
+
+
 # ------------------------------------------------------------------ the state-space mixer's kernels, alone
 
 def run_state_space(proj, m, conv_w, conv_b, dt_bias, a_log, d_skip, norm_w, eps, dt, lens, cuts, chunked=False):
