@@ -1,11 +1,11 @@
 // Softmax attention of any number of tokens over the paged key/value cache, for every head
 // size up to 256 and either dtype: the attention of the true 32-bit path, and the one that
-// takes the shapes the tensor-core kernels refuse.  One block per (token, query head).
+// takes the shapes the tensor-core kernels refuse.
 //
 // A query at position p of its sequence sees the keys lo..p of that sequence, lo = 0 or
-// p - window + 1.  Keys are visited in increasing position in chunks of the block size that
-// start at lo, so the arithmetic of one (sequence, position, head) is the same whether the
-// token came in a long prompt, alone, or beside other sequences.
+// p - window + 1.  Keys are visited in increasing position, page by page (the kernel of one block a
+// (token, head): in chunks that start at lo), so the arithmetic of one (sequence, position, head) is the
+// same whether the token came in a long prompt, alone, or beside other sequences.
 //
 // Scores, softmax and the weighted sum are float32 (pico-engine: src/pico_engine/kernels.py:
 // 108-125; its result is stored through float16 at kernels.py:126, which is not done here).
@@ -78,13 +78,260 @@ __global__ void __launch_bounds__(AG_THREADS) attention_generic_kernel(
     if (tid + AG_THREADS < hd) op[tid + AG_THREADS] = from_f<T>(acc1 * inv);
 }
 
+// ---------------------------------------------------------------------------- tiles of rows
+// A block: R rows, each a (token, query head); the rows of neighbouring tokens and of the heads that share a key/value head, so that a
+// page is read once for all of them.  A step is a page: thread (ty, tx) of 16 x 16 has the scores of R / 16 rows and four keys, then
+// R / 16 rows and hd / 16 columns of the outputs.  Tokens of several sequences in a block are served one sequence after the other.
+// Whatever R is, a row's scores are sums over the entries in order, its weights are added in the same tree, its outputs in the order of
+// the keys: R = 16 (single tokens) and R = 64 (prompts) give the same bits.  A key that a row does not see adds nothing to it, not even
+// a value that is no number.  Bound by float32 multiply-adds and the reads from shared memory that feed them.  Two layers' attention of
+// 14 heads of 64, prompts of 301 and 207 tokens, on a B200: 645 us by the kernel above (a block a token and head, which read every key
+// and value once a head), 75 us here; single tokens at 1,500 keys: 1,180 us a layer before, 89 us here.
+#define AT_THREADS 256
+
+struct AttentionTileArgs {
+    const void* q; int q_stride; void* out; const void* k_pool; const void* v_pool;
+    const int* table; int table_stride; const int* tok_pos; const int* tok_row;
+    int T, nh, nkv, hd, window; float scale;
+    int heads, slices, tokens;                     // query heads and tokens of a block's rows; blocks that share a key/value head's heads
+};
+
+__device__ __forceinline__ float4 ag_load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 ag_load4(const bf16* p) {
+    const uint2 r = *reinterpret_cast<const uint2*>(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ void ag_store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void ag_store4(bf16* p, float4 v) {
+    __nv_bfloat162 h[2] = {__floats2bfloat162_rn(v.x, v.y), __floats2bfloat162_rn(v.z, v.w)};
+    *reinterpret_cast<uint2*>(p) = *reinterpret_cast<const uint2*>(h);
+}
+// acc += a * b on four entries, two multiply-adds an instruction (each half rounds as a plain one does)
+__device__ __forceinline__ void ag_fma4(float4& acc, float a, const float4& b) {
+    asm("{\n\t.reg .b64 pa, b0, b1, c0, c1;\n\t"
+        "mov.b64 pa, {%4, %4};\n\tmov.b64 b0, {%5, %6};\n\tmov.b64 b1, {%7, %8};\n\tmov.b64 c0, {%0, %1};\n\tmov.b64 c1, {%2, %3};\n\t"
+        "fma.rn.f32x2 c0, pa, b0, c0;\n\tfma.rn.f32x2 c1, pa, b1, c1;\n\t"
+        "mov.b64 {%0, %1}, c0;\n\tmov.b64 {%2, %3}, c1;\n\t}"
+        : "+f"(acc.x), "+f"(acc.y), "+f"(acc.z), "+f"(acc.w) : "f"(a), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w));
+}
+// entry d of key (or row) j in a turned tile [hd][64]: neither a thread's four stores nor the reads of four neighbours meet in a bank
+__device__ __forceinline__ int ag_turned(int d, int j) { return d * 64 + (j ^ (((d >> 2) & 7) << 2)); }
+struct ag_yes { static constexpr bool value = true; };
+struct ag_no { static constexpr bool value = false; };
+
+template <typename T, int R, int NJ>
+__global__ void __launch_bounds__(AT_THREADS) attention_tile_kernel(AttentionTileArgs a) {
+    pdl_launch_dependents();
+    pdl_wait();
+    constexpr int RT = R / 16;                             // rows a thread
+    extern __shared__ __align__(16) float ag_smem[];
+    __shared__ int pos_s[R], seq_s[R];
+    const int hd = a.hd, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, per4 = hd / 4;
+    float* qt = ag_smem;                                   // [hd][64]: the rows' queries, turned (R of 64 places used)
+    float* kt = qt + hd * 64;                              // [hd][64]: a page's keys, turned
+    float* vs = kt + hd * 64;                              // [64][hd]
+    float* ps = vs + hd * 64;                              // [64 keys][R]: weights, rows in groups of four exchanged by the key
+    const int per = a.nh / a.nkv, kvh = blockIdx.y / a.slices, h0 = kvh * per + blockIdx.y % a.slices * a.heads;
+    const int n_heads = min(a.heads, kvh * per + per - h0), t0 = blockIdx.x * a.tokens, n_tok = min(a.tokens, a.T - t0);
+    const int rows = n_heads * n_tok;                      // row r: token t0 + r / n_heads, head h0 + r % n_heads
+    if (tid < R) {
+        const int t = t0 + min(tid, rows - 1) / n_heads;
+        pos_s[tid] = a.tok_pos[t];
+        seq_s[tid] = tid < rows ? a.tok_row[t] : -1;
+    }
+    for (int i = tid; i < R * per4; i += AT_THREADS) {
+        const int r = i / per4, c = i % per4 * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < rows) v = ag_load4((const T*)a.q + (size_t)(t0 + r / n_heads) * a.q_stride + (size_t)(h0 + r % n_heads) * hd + c);
+        qt[ag_turned(c, r)] = v.x; qt[ag_turned(c + 1, r)] = v.y; qt[ag_turned(c + 2, r)] = v.z; qt[ag_turned(c + 3, r)] = v.w;
+    }
+    __syncthreads();
+    float m[RT], l[RT];
+    float4 acc[RT][NJ];
+    int my_pos[RT], my_seq[RT];
+#pragma unroll
+    for (int i = 0; i < RT; ++i) {
+        m[i] = -INFINITY; l[i] = 0.f;
+        my_pos[i] = pos_s[ty * RT + i]; my_seq[i] = seq_s[ty * RT + i];
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) acc[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    // Where a page's rows are few enough registers (PRE: a thread's share of up to PU vectors of keys and of values), the next page
+    // travels while this one is used.  A thread's vectors are AT_THREADS apart: their (key, entry) advance by fixed steps.
+    constexpr int PU = 4 * NJ;
+    constexpr bool PRE = NJ == 1 || (NJ == 2 && RT == 1);
+    float4 pk[PRE ? PU : 1], pv[PRE ? PU : 1];
+    const int j_first = tid / per4, c_first = tid % per4 * 4, j_step = AT_THREADS / per4, c_step = AT_THREADS % per4 * 4;
+    auto fetch = [&](size_t base) {
+#pragma unroll
+        for (int u = 0; u < PU; ++u) {
+            const int i = tid + u * AT_THREADS;
+            if (i < PE_PAGE * per4) {
+                pk[PRE ? u : 0] = ag_load4((const T*)a.k_pool + base + (size_t)i * 4);
+                pv[PRE ? u : 0] = ag_load4((const T*)a.v_pool + base + (size_t)i * 4);
+            }
+        }
+    };
+    auto turn = [&](int j, int c, const float4& k) { kt[ag_turned(c, j)] = k.x; kt[ag_turned(c + 1, j)] = k.y; kt[ag_turned(c + 2, j)] = k.z; kt[ag_turned(c + 3, j)] = k.w; };
+    for (int from = 0; from < rows;) {                     // the rows of one sequence after the other
+        const int seq = seq_s[from];
+        int to = from + n_heads, lowest = pos_s[from], highest = lowest;
+        while (to < rows && seq_s[to] == seq) { lowest = min(lowest, pos_s[to]); highest = max(highest, pos_s[to]); to += n_heads; }
+        const int* table = a.table + (size_t)seq * a.table_stride;
+        const int page_lo = a.window > 0 && lowest - a.window + 1 > 0 ? (lowest - a.window + 1) / PE_PAGE : 0;
+        const int page_hi = highest / PE_PAGE;
+        int page = table[page_lo];
+        const auto base_of = [&](int pg) { return ((size_t)pg * a.nkv + kvh) * PE_PAGE * hd; };
+        if (PRE && page >= 0) fetch(base_of(page));
+        for (int pg = page_lo; pg <= page_hi; ++pg) {
+            const int here = page;
+            page = pg < page_hi ? table[pg + 1] : -1;
+            if (here < 0) {
+                if (PRE && page >= 0) fetch(base_of(page));
+                continue;
+            }
+            __syncthreads();                               // the page before has been used
+            int j = j_first, c = c_first;
+            if constexpr (PRE) {
+#pragma unroll
+                for (int u = 0; u < PU; ++u) {
+                    if (j < PE_PAGE) {
+                        turn(j, c, pk[u]);
+                        *reinterpret_cast<float4*>(vs + j * hd + c) = pv[u];
+                    }
+                    j += j_step; c += c_step;
+                    if (c >= hd) { c -= hd; ++j; }
+                }
+                if (page >= 0) fetch(base_of(page));
+            } else {
+                const size_t base = base_of(here);
+#pragma unroll 4
+                while (j < PE_PAGE) {
+                    turn(j, c, ag_load4((const T*)a.k_pool + base + (size_t)j * hd + c));
+                    *reinterpret_cast<float4*>(vs + j * hd + c) = ag_load4((const T*)a.v_pool + base + (size_t)j * hd + c);
+                    j += j_step; c += c_step;
+                    if (c >= hd) { c -= hd; ++j; }
+                }
+            }
+            __syncthreads();
+            float4 s[RT];
+#pragma unroll
+            for (int i = 0; i < RT; ++i) s[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+            for (int d = 0; d < hd; ++d) {
+                const float4 k = *reinterpret_cast<const float4*>(kt + ag_turned(d, tx * 4));
+                if constexpr (RT == 4) {
+                    const float4 q = *reinterpret_cast<const float4*>(qt + ag_turned(d, ty * 4));
+                    ag_fma4(s[0], q.x, k); ag_fma4(s[1], q.y, k); ag_fma4(s[2], q.z, k); ag_fma4(s[3], q.w, k);
+                } else ag_fma4(s[0], qt[ag_turned(d, ty)], k);
+            }
+            // which of the four keys a row sees; the rows' new maxima and weights
+            const int key0 = pg * PE_PAGE + tx * 4;
+            bool whole = true;                             // this thread's rows see the whole page
+#pragma unroll
+            for (int i = 0; i < RT; ++i) {
+                const int hi = my_seq[i] == seq ? my_pos[i] - key0 : -1, lo = a.window > 0 ? hi - a.window + 1 : 0;      // keys lo .. hi of the four
+                s[i].x = hi >= 0 && lo <= 0 ? s[i].x * a.scale : -INFINITY;
+                s[i].y = hi >= 1 && lo <= 1 ? s[i].y * a.scale : -INFINITY;
+                s[i].z = hi >= 2 && lo <= 2 ? s[i].z * a.scale : -INFINITY;
+                s[i].w = hi >= 3 && lo <= 3 ? s[i].w * a.scale : -INFINITY;
+                float mx = fmaxf(fmaxf(s[i].x, s[i].y), fmaxf(s[i].z, s[i].w));
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+                const float m_new = fmaxf(m[i], mx), alpha = m[i] == -INFINITY ? 0.f : expf(m[i] - m_new);
+                s[i].x = s[i].x == -INFINITY ? 0.f : expf(s[i].x - m_new); s[i].y = s[i].y == -INFINITY ? 0.f : expf(s[i].y - m_new);
+                s[i].z = s[i].z == -INFINITY ? 0.f : expf(s[i].z - m_new); s[i].w = s[i].w == -INFINITY ? 0.f : expf(s[i].w - m_new);
+                float sum = (s[i].x + s[i].y) + (s[i].z + s[i].w);
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                if (my_seq[i] == seq) {
+                    l[i] = l[i] * alpha + sum;
+                    m[i] = m_new;
+#pragma unroll
+                    for (int j = 0; j < NJ; ++j) { acc[i][j].x *= alpha; acc[i][j].y *= alpha; acc[i][j].z *= alpha; acc[i][j].w *= alpha; }
+                }
+                const int first_key = pg * PE_PAGE;
+                whole = whole && my_seq[i] == seq && my_pos[i] >= first_key + PE_PAGE - 1 && (a.window <= 0 || my_pos[i] - first_key < a.window);
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const auto at = [e](const float4& v) { return e == 0 ? v.x : e == 1 ? v.y : e == 2 ? v.z : v.w; };
+                float* p = ps + (tx * 4 + e) * R;
+                if constexpr (RT == 4) *reinterpret_cast<float4*>(p + ((ty * 4) ^ ((tx & 7) << 2))) = make_float4(at(s[0]), at(s[1]), at(s[2]), at(s[3]));
+                else p[ty] = at(s[0]);
+            }
+            __syncthreads();
+            // guarded: a row adds nothing of a key whose weight is zero (a weight that is no number joins)
+            const auto add_values = [&](int keys, auto guarded) {
+#pragma unroll 8
+                for (int k = 0; k < keys; ++k) {
+                    float p[RT];
+                    if constexpr (RT == 4) *reinterpret_cast<float4*>(p) = *reinterpret_cast<const float4*>(ps + k * R + ((ty * 4) ^ (((k >> 2) & 7) << 2)));
+                    else p[0] = ps[k * R + ty];
+#pragma unroll
+                    for (int j = 0; j < NJ; ++j) {
+                        const int c = tx * 4 + 64 * j;
+                        const float4 v = *reinterpret_cast<const float4*>(vs + k * hd + (c < hd ? c : 0));      // (columns that are none are not stored)
+#pragma unroll
+                        for (int i = 0; i < RT; ++i)
+                            if (!decltype(guarded)::value || p[i] != 0.f) ag_fma4(acc[i][j], p[i], v);
+                    }
+                }
+            };
+            if (__all_sync(0xffffffffu, whole)) add_values(PE_PAGE, ag_no());
+            else add_values(min(PE_PAGE, highest - pg * PE_PAGE + 1), ag_yes());
+        }
+        from = to;
+    }
+#pragma unroll
+    for (int i = 0; i < RT; ++i) {
+        const int r = ty * RT + i;
+        if (r >= rows) continue;
+        const float inv = l[i] > 0.f ? 1.0f / l[i] : 0.f;
+        T* o = (T*)a.out + ((size_t)(t0 + r / n_heads) * a.nh + h0 + r % n_heads) * hd;
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+            const int c = tx * 4 + 64 * j;
+            if (c < hd) ag_store4(o + c, make_float4(acc[i][j].x * inv, acc[i][j].y * inv, acc[i][j].z * inv, acc[i][j].w * inv));
+        }
+    }
+}
+
+template <typename T, int R, int NJ>
+static int attention_tile_as(AttentionTileArgs a, cudaStream_t s) {
+    const int per = a.nh / a.nkv;
+    a.heads = per < R ? per : R;
+    a.slices = (per + a.heads - 1) / a.heads;
+    a.tokens = R == 16 ? 1 : R / a.heads;                  // single tokens are of different sequences: a block each
+    const size_t smem = sizeof(float) * ((size_t)3 * a.hd * 64 + 64 * R);
+    auto kernel = attention_tile_kernel<T, R, NJ>;
+    PE_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PE_TRY(pe_launch(kernel, dim3((a.T + a.tokens - 1) / a.tokens, a.nkv * a.slices), AT_THREADS, smem, s, a));
+    PE_LAUNCH_CHECK();
+    return 0;
+}
+template <typename T>
+static int attention_tile(const AttentionTileArgs& a, bool runs, cudaStream_t s) {
+    if (a.hd <= 64) return runs ? attention_tile_as<T, 64, 1>(a, s) : attention_tile_as<T, 16, 1>(a, s);
+    if (a.hd <= 128) return runs ? attention_tile_as<T, 64, 2>(a, s) : attention_tile_as<T, 16, 2>(a, s);
+    return runs ? attention_tile_as<T, 64, 4>(a, s) : attention_tile_as<T, 16, 4>(a, s);
+}
+
 extern "C" int pe_attention_generic(const void* q, int q_stride, void* out, const void* k_pool, const void* v_pool,
                                     int dtype, const int* block_table, int table_stride, const int* tok_pos,
-                                    const int* tok_row, int T, int nh, int nkv, int hd, int window, float scale,
+                                    const int* tok_row, int T, int nh, int nkv, int hd, int window, float scale, int sequences,
                                     void* stream) {
     if (T <= 0) return 0;
     if (hd <= 0 || hd > AG_MAX_HD || nkv <= 0 || nh % nkv || nh > 65535) return PE_ERR_UNSUPPORTED;
     cudaStream_t s = (cudaStream_t)stream;
+    const size_t size = dtype == PE_F32 ? 4 : 2;
+    if ((dtype == PE_F32 || dtype == PE_BF16) && hd % 4 == 0 && q_stride % 4 == 0 && !(((uintptr_t)q | (uintptr_t)out | (uintptr_t)k_pool | (uintptr_t)v_pool) % (4 * size))) {
+        // rows of four entries that can be read at once: tiles of rows; 64 of them where a sequence brings several tokens
+        const AttentionTileArgs a = {q, q_stride, out, k_pool, v_pool, block_table, table_stride, tok_pos, tok_row, T, nh, nkv, hd, window, scale, 0, 0, 0};
+        const bool runs = sequences > 0 && T >= 2 * sequences;
+        return dtype == PE_F32 ? attention_tile<float>(a, runs, s) : attention_tile<bf16>(a, runs, s);
+    }
     dim3 grid(T, nh);
     if (dtype == PE_F32)
         PE_TRY(pe_launch(attention_generic_kernel<float>, grid, AG_THREADS, 0, s, (const float*)q, q_stride, (float*)out,

@@ -190,7 +190,7 @@ def attention_generic(q: torch.Tensor, q_stride: int, n_heads: int, n_kv_heads: 
     check(core().pe_attention_generic(q.data_ptr(), q_stride, out.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(),
                                       _code(q, "q"), block_table.data_ptr(), table_stride, tok_pos.data_ptr(),
                                       tok_row.data_ptr(), T, n_heads, n_kv_heads, head_dim, window or 0, float(scale),
-                                      stream_ptr()), "attention_generic")
+                                      block_table.shape[0] if block_table.dim() == 2 else 0, stream_ptr()), "attention_generic")
     return out
 
 

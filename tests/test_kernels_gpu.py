@@ -215,6 +215,25 @@ def test_attention_generic(K, nh, nkv, hd, lens, window, dtype):
         assert err < ATTENTION_BOUND, err
 
 
+@pytest.mark.parametrize("nh,nkv,hd,lens,window", CASES + [(2, 2, 256, [70, 3], None), (70, 1, 16, [66, 9], 20)])
+def test_attention_generic_alone_and_among_others(K, nh, nkv, hd, lens, window):
+    """Whole prompts of several sequences in one step (64 rows a block) against the plain attention, and every token alone (16 rows a
+    block, one sequence) gives the same bits."""
+    paged = Paged(lens, nkv, hd, torch.float32, seed=hd)
+    tok_row = [b for b, n in enumerate(lens) for _ in range(n)]
+    tok_pos = [p for n in lens for p in range(n)]
+    q = rnd(len(tok_row), nh, hd, seed=nh)
+    kp, vp, table = paged.cuda()
+    run = lambda i: K.attention_generic(dev(q[i].reshape(len(i), -1).contiguous()), nh * hd, nh, nkv, hd, kp, vp, table, table.shape[1],
+                                        dev(torch.tensor([tok_pos[j] for j in i], dtype=torch.int32)),
+                                        dev(torch.tensor([tok_row[j] for j in i], dtype=torch.int32)), window, hd ** -0.5)
+    whole = run(list(range(len(tok_row))))
+    want = reference_attention(q, paged, tok_row, tok_pos, nh, window)
+    assert torch.allclose(whole.cpu(), want.reshape(len(tok_row), -1), atol=2e-5, rtol=2e-5)
+    for j in {0, 1, lens[0] // 2, lens[0] - 1, len(tok_row) - lens[-1], len(tok_row) - 1}:
+        assert torch.equal(run([j])[0], whole[j]), j
+
+
 @pytest.mark.parametrize("nh,nkv,hd,lens,window", CASES)
 @pytest.mark.parametrize("max_context", [None, 4096])
 def test_attention_decode(K, nh, nkv, hd, lens, window, max_context):
