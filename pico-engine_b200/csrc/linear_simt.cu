@@ -12,8 +12,9 @@
 
 // How many ranges K is cut into.  A product with few columns has few tiles (896 columns and 508 rows: 56 of 64 x 128 for
 // 148 SMs), a wide one fills the GPU without; a range of less than 64 entries would cost more in its sum than it saves.
+#define LS_MOST_RANGES 8
 static int ls_ranges(int N, int K) {
-    int s = N <= 2048 ? 4 : N <= 12288 ? 2 : 1;
+    int s = N <= 2048 ? (K >= 2048 ? 8 : 4) : N <= 12288 ? 2 : 1;
     while (s > 1 && K / s < 64) s /= 2;
     return s;
 }
@@ -27,6 +28,18 @@ __device__ __forceinline__ float ls_peer_value(const float* mine, int rank) {   
     float v;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(at), "r"(rank));
     asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(peer) : "memory");
+    return v;
+}
+
+// the ranges' sums of one place, added in their order (all of them asked for before any is used)
+__device__ __forceinline__ float ls_sum(const float* mine, int ranges) {
+    float part[LS_MOST_RANGES];
+#pragma unroll
+    for (int c = 0; c < LS_MOST_RANGES; ++c) part[c] = c < ranges ? ls_peer_value(mine, c) : 0.f;
+    float v = part[0] + part[1];
+#pragma unroll
+    for (int c = 2; c < LS_MOST_RANGES; c += 2)
+        if (c < ranges) v = (v + part[c]) + part[c + 1];
     return v;
 }
 
@@ -52,61 +65,63 @@ __device__ __forceinline__ float4 ls_load4(const T* p, int left, bool vec) {    
 }
 
 // ---------------------------------------------------------------------------- many rows
-// A CTA of 128 threads: a tile of 64 rows and 128 columns over one range of K; a thread 8 x 8 of it, as multiply-adds in pairs
-// (fma.rn.f32x2: each half rounds as a plain one does).  Bound by the multiply-adds: a thread reads 16 entries from shared memory
-// for 64 of them, a warp's reads of either operand are one broadcast wavefront, and the next 16 entries of K are on their way in
-// registers meanwhile.  The ranges of a tile are a cluster; its CTAs add up a slice of the tile each from the others' shared memory.
-// Two layers of the Qwen2.5-0.5B widths at 508 rows on a B200: 3.47 ms before (tiles of 64 x 64, 4 x 4 a thread, nothing in flight), 1.53 ms.
+// A CTA of 128 threads: a tile of 64 rows and BN columns over one range of K; a thread 8 x 8 (BN = 128) or 8 x 4 (64) of it, as
+// multiply-adds in pairs (fma.rn.f32x2: each half rounds as a plain one does).  Bound by the multiply-adds: a thread reads 16 entries from shared memory
+// for 64 of them, a warp's reads of either operand are one broadcast wavefront, and the next 16 (BN = 64: 32) entries of K are on their
+// way in registers meanwhile.  The ranges of a tile are a cluster; its CTAs add up a slice of the tile each from the others' shared memory.
+// The products of two layers of the Qwen2.5-0.5B widths at 508 rows on a B200: about 2.9 ms as tiles of 64 x 64 with 4 x 4 a thread and
+// nothing in flight, 0.79 ms here (38 TFLOP/s).
 #define LS_BM 64
-#define LS_BN 128
-#define LS_BK 16
-#define LS_SA (LS_BM + 4)
-#define LS_SW (LS_BN + 4)
 #define LS_THREADS 128
 
-template <typename TA, typename TW>
-__global__ void __launch_bounds__(LS_THREADS, 3) linear_simt_kernel(const TA* A, const TW* W, const void* bias, int bias_dtype,
+template <typename TA, typename TW, int LS_BN>
+__global__ void __launch_bounds__(LS_THREADS, LS_BN == 128 ? 3 : 4) linear_simt_kernel(const TA* A, const TW* W, const void* bias, int bias_dtype,
                                                                     void* out, int epilogue, int M, int N, int K, int ranges, int vec_a, int vec_w) {
     pdl_launch_dependents();
     pdl_wait();
-    __shared__ __align__(16) float smem[LS_BM * LS_SW > 2 * LS_BK * (LS_SA + LS_SW) ? LS_BM * LS_SW : 2 * LS_BK * (LS_SA + LS_SW)];
+    constexpr int LS_SW = LS_BN + 4, NP = LS_BN / 32;      // NP: pairs of columns a thread
+    constexpr int LS_BK = LS_BN == 64 ? 32 : 16, STAGE = LS_BK * (LS_BM + LS_BN);      // entries of K on their way while as many are used
+    constexpr int KQ = LS_BK / 4, LR = LS_THREADS / KQ;    // threads that share a row's entries; rows brought at a time
+    __shared__ __align__(16) float smem[LS_BM * LS_SW > 2 * STAGE ? LS_BM * LS_SW : 2 * STAGE];
+    // row r at entry k: groups of four rows exchanged by k, so that neither a thread's four stores nor four neighbours' reads meet in a bank
+    const auto place = [](int k, int r, int width) { return k * width + (r ^ (((k >> 2) & 7) << 2)); };
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int ty = (warp >> 1) * 4 + (lane >> 3), tx = (warp & 1) * 8 + (lane & 7);     // rows ty * 4 + 32 i, columns tx * 4 + 64 j
     const int rank = blockIdx.x % ranges, n0 = blockIdx.x / ranges * LS_BN, m0 = blockIdx.y * LS_BM;
     const int len = ls_range_len(K, ranges), k_begin = rank * len, k_end = min(K, k_begin + len);
 
-    unsigned long long acc[8][4];                          // row i, column pairs
+    unsigned long long acc[8][NP];                         // row i, column pairs
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+        for (int j = 0; j < NP; ++j) acc[i][j] = 0ull;
 
-    const int lr = tid >> 2, lk = (tid & 3) * 4;           // a thread brings four entries of K of rows lr + 32 e
-    float4 ra[LS_BM / 32], rw[LS_BN / 32];
+    const int lr = tid / KQ, lk = tid % KQ * 4;            // a thread brings four entries of K of rows lr + LR e
+    float4 ra[LS_BM / LR], rw[LS_BN / LR];
     auto fetch = [&](int k0) {
         const int left = k_end - k0 - lk;
 #pragma unroll
-        for (int e = 0; e < LS_BM / 32; ++e) {
-            const int m = m0 + lr + 32 * e;
+        for (int e = 0; e < LS_BM / LR; ++e) {
+            const int m = m0 + lr + LR * e;
             ra[e] = ls_load4(A + (size_t)min(m, M - 1) * K + k0 + lk, m < M ? left : 0, vec_a);
         }
 #pragma unroll
-        for (int e = 0; e < LS_BN / 32; ++e) {
-            const int n = n0 + lr + 32 * e;
+        for (int e = 0; e < LS_BN / LR; ++e) {
+            const int n = n0 + lr + LR * e;
             rw[e] = ls_load4(W + (size_t)min(n, N - 1) * K + k0 + lk, n < N ? left : 0, vec_w);
         }
     };
     auto put = [&](float* as) {
-        float* ws = as + LS_BK * LS_SA;
+        float* ws = as + LS_BK * LS_BM;
 #pragma unroll
-        for (int e = 0; e < LS_BM / 32; ++e) {
-            float* p = as + lk * LS_SA + lr + 32 * e;
-            p[0] = ra[e].x; p[LS_SA] = ra[e].y; p[2 * LS_SA] = ra[e].z; p[3 * LS_SA] = ra[e].w;
+        for (int e = 0; e < LS_BM / LR; ++e) {
+            float* p = as + place(lk, lr + LR * e, LS_BM);
+            p[0] = ra[e].x; p[LS_BM] = ra[e].y; p[2 * LS_BM] = ra[e].z; p[3 * LS_BM] = ra[e].w;
         }
 #pragma unroll
-        for (int e = 0; e < LS_BN / 32; ++e) {
-            float* p = ws + lk * LS_SW + lr + 32 * e;
-            p[0] = rw[e].x; p[LS_SW] = rw[e].y; p[2 * LS_SW] = rw[e].z; p[3 * LS_SW] = rw[e].w;
+        for (int e = 0; e < LS_BN / LR; ++e) {
+            float* p = ws + place(lk, lr + LR * e, LS_BN);
+            p[0] = rw[e].x; p[LS_BN] = rw[e].y; p[2 * LS_BN] = rw[e].z; p[3 * LS_BN] = rw[e].w;
         }
     };
     if (k_begin < k_end) {
@@ -117,49 +132,41 @@ __global__ void __launch_bounds__(LS_THREADS, 3) linear_simt_kernel(const TA* A,
     for (int k0 = k_begin, b = 0; k0 < k_end; k0 += LS_BK, b ^= 1) {
         const bool more = k0 + LS_BK < k_end;
         if (more) fetch(k0 + LS_BK);
-        const float* as = smem + b * LS_BK * (LS_SA + LS_SW) + ty * 4;
-        const float* ws = smem + b * LS_BK * (LS_SA + LS_SW) + LS_BK * LS_SA + tx * 4;
+        const float* as = smem + b * STAGE;
+        const float* ws = as + LS_BK * LS_BM;
 #pragma unroll
         for (int k = 0; k < LS_BK; ++k) {                  // (entries behind the range are zeros: they add nothing)
             float a[8];
-            unsigned long long w[4];
-            *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(as + k * LS_SA);
-            *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(as + k * LS_SA + 32);
-            *reinterpret_cast<ulonglong2*>(w) = *reinterpret_cast<const ulonglong2*>(ws + k * LS_SW);
-            *reinterpret_cast<ulonglong2*>(w + 2) = *reinterpret_cast<const ulonglong2*>(ws + k * LS_SW + 64);
+            unsigned long long w[NP];
+            *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(as + place(k, ty * 4, LS_BM));
+            *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(as + place(k, ty * 4, LS_BM) + 32);
+#pragma unroll
+            for (int j = 0; j < NP; j += 2) *reinterpret_cast<ulonglong2*>(w + j) = *reinterpret_cast<const ulonglong2*>(ws + place(k, tx * 4, LS_BN) + 32 * j);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 unsigned long long aa;
                 asm("mov.b64 %0, {%1, %1};" : "=l"(aa) : "f"(a[i]));
 #pragma unroll
-                for (int j = 0; j < 4; ++j) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][j]) : "l"(aa), "l"(w[j]));
+                for (int j = 0; j < NP; ++j) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][j]) : "l"(aa), "l"(w[j]));
             }
         }
-        if (more) put(smem + (b ^ 1) * LS_BK * (LS_SA + LS_SW));
+        if (more) put(smem + (b ^ 1) * STAGE);
         __syncthreads();
     }
     // the tile through shared memory: rows of neighbouring columns go out together, and the other ranges' CTAs can read it
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         float* row = smem + (ty * 4 + 32 * (i / 4) + i % 4) * LS_SW + tx * 4;
-        *reinterpret_cast<ulonglong2*>(row) = make_ulonglong2(acc[i][0], acc[i][1]);
-        *reinterpret_cast<ulonglong2*>(row + 64) = make_ulonglong2(acc[i][2], acc[i][3]);
+#pragma unroll
+        for (int j = 0; j < NP; j += 2) *reinterpret_cast<ulonglong2*>(row + 32 * j) = make_ulonglong2(acc[i][j], acc[i][j + 1]);
     }
     if (ranges > 1) ls_cluster_sync(); else __syncthreads();
-    const int n = n0 + tid, rows = LS_BM / ranges;
+    const int col = tid % LS_BN, n = n0 + col, rows = LS_BM / ranges;
 #pragma unroll 4
-    for (int i = 0; i < rows; ++i) {
+    for (int i = tid / LS_BN; i < rows; i += LS_THREADS / LS_BN) {
         const int r = rank * rows + i, m = m0 + r;
         if (m >= M || n >= N) break;
-        float v = 0.f;
-        if (ranges == 1) v = smem[r * LS_SW + tid];
-        else {
-            float part[4];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) part[c] = c < ranges ? ls_peer_value(smem + r * LS_SW + tid, c) : 0.f;
-            v = part[0] + part[1];
-            if (ranges > 2) v = (v + part[2]) + part[3];
-        }
+        const float v = ranges == 1 ? smem[r * LS_SW + col] : ls_sum(smem + r * LS_SW + col, ranges);
         ls_finish(v, out, (size_t)m * N + n, bias, bias_dtype, n, epilogue);
     }
     if (ranges > 1) ls_cluster_sync();                     // nobody leaves while its tile is being read
@@ -247,12 +254,7 @@ __global__ void __launch_bounds__(LR_THREADS) linear_simt_rows_kernel(const TA* 
     ls_cluster_sync();
     for (int m = warp * ranges + rank; m < MT; m += 4 * ranges) {      // the rows dealt out to the cluster's warps
         if (m >= M || n >= N) break;
-        float part[4];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) part[c] = c < ranges ? ls_peer_value(sums + m * LR_BN + lane, c) : 0.f;
-        float v = part[0] + part[1];
-        if (ranges > 2) v = (v + part[2]) + part[3];
-        ls_finish(v, out, (size_t)m * N + n, bias, bias_dtype, n, epilogue);
+        ls_finish(ls_sum(sums + m * LR_BN + lane, ranges), out, (size_t)m * N + n, bias, bias_dtype, n, epilogue);
     }
     ls_cluster_sync();
 }
@@ -281,10 +283,16 @@ static int ls_go(const void* A, const void* W, const void* bias, int bias_dtype,
                                               : ls_rows<TA, TW, 4, true>(A, W, bias, bias_dtype, out, epilogue, M, N, K, ranges, s);
         return ls_rows<TA, TW, 4, false>(A, W, bias, bias_dtype, out, epilogue, M, N, K, ranges, s);
     }
-    dim3 grid((N + LS_BN - 1) / LS_BN * ranges, (M + LS_BM - 1) / LS_BM);
-    if (grid.y > 65535) return PE_ERR_UNSUPPORTED;
-    PE_TRY(pe_launch_cluster(linear_simt_kernel<TA, TW>, grid, LS_THREADS, 0, s, ranges, (const TA*)A, (const TW*)W, bias, bias_dtype, out, epilogue,
-                             M, N, K, ranges, vec_a, vec_w));
+    const int mt = (M + LS_BM - 1) / LS_BM;
+    if (mt > 65535) return PE_ERR_UNSUPPORTED;
+#define LS_TILES(BN) PE_TRY(pe_launch_cluster(linear_simt_kernel<TA, TW, BN>, dim3((N + BN - 1) / BN * ranges, mt), LS_THREADS, 0, s, ranges, (const TA*)A, \
+                                              (const TW*)W, bias, bias_dtype, out, epilogue, M, N, K, ranges, vec_a, vec_w))
+    // Tiles of 64 columns where those of 128 would leave an SM with fewer than four CTAs: with so few, one more or less is what a product
+    // waits for.  Measured on a B200, columns x K, 64 wide / 128 wide: 60 rows 1152 x 896 13 / 20 us, 896 x 4864 30 / 42 us; 508 rows
+    // 1152 x 896 35 / 40, 896 x 896 30 / 39, 896 x 4864 113 / 127 (all below the line); 9728 x 896 215 / 205 (above it).
+    if ((long long)((N + 127) / 128) * ranges * mt < 4 * 148) LS_TILES(64);
+    else LS_TILES(128);
+#undef LS_TILES
     PE_LAUNCH_CHECK();
     return 0;
 }
