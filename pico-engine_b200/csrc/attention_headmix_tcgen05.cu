@@ -1,0 +1,382 @@
+// Attention with mixed heads for prompts on the 5th-generation tensor cores.
+//
+// The mixing is linear, so it can follow the product with the values:
+//     o_h(i) = sum_j (sum_g mix[h, g] p_g(i, j)) v_c(h)(j) = sum_g mix[h, g] O_g,c(h)(i),    O_g,c(i) = sum_j p_g(i, j) v_c(j).
+// The first kernel is flash attention whose every head g keeps an output for every key/value head c of a group, both products as
+// tcgen05.mma with their accumulators in tensor memory; it divides by the softmax denominator (with exp(sink_g) in it) and leaves O_g,c
+// in float32.  The second kernel mixes: a thread has a value column of a key/value head and the heads that read it.
+//
+//   one CTA   = a run of up to 128 consecutive tokens of one sequence x one query head x a group of value heads
+//   a step    = two pages of the cache (128 keys)
+//   warp 0      loader: TMA tiled loads (128-byte swizzle) of the run's queries and of the pages' keys and the group's values into a ring
+//               of stages; it alone reads the page table and tells the others through flags which pages are there
+//   warp 1      allocates tensor memory; one lane issues S = Q K^T (128 x 128) into one of two buffers and O_c += P V_c for the group's
+//               heads: S of the next step before P V of this one
+//   warps 2-9   softmax, two threads a query row, one for each page of the step; P goes as bfloat16 back into the S buffer's own columns,
+//               from where it is the A operand of P V.  O is rescaled only when a row's reference point has moved by more than 2^8.
+//
+// Tensor memory has 256 columns for S and 256 for O: two value heads of 128 or four of 64 a CTA; more are further CTAs, which make S again.
+// Bound by a step's chain (scores, maximum, exponentials, P) rather than by the tensor cores.
+// Measured on a B200, 1,024 tokens, 16 heads of 128 on four key/value heads: 40 + 15 us, where the mma.sync kernel and its merge
+// (attention_headmix_flash.cu) take 198 + 83.
+// Head sizes: D a multiple of 16, Dv of 16.  Every mbarrier wait is bounded by the clock; a wait that runs out sets *status to 5, the
+// roles leave their loops, tensor memory is freed and the CTA returns (status 6: shared memory did not start on a 1024-byte boundary).
+#include "tcgen05_attention.cuh"
+
+#define HT_QTILE 128
+#define HT_KTILE PE_PAGE
+#define HT_MAX_STAGES 4
+#define HT_THREADS 320                             // loader, MMA issuer, and two softmax warps for each 32 rows
+#define HT_PANEL (2 * HT_KTILE * 128)              // 128 rows of 64 columns: one swizzled panel, of the queries or of a step's keys or values
+#define HT_BAR_WORDS (13 + 2 * HT_MAX_STAGES)
+#define HT_TMEM_COLS 512                           // S (then P) at columns 0 and 128, O of the group's heads from column 256
+#define HT_O_COL 256
+#define HT_LAZY 8.0f
+#define HT_SMALL_BYTES (8 * HT_BAR_WORDS + 8 * HT_MAX_STAGES + 2 * 2 * HT_QTILE * 4)
+#define HT_SMEM_LIMIT 232448
+
+struct HeadmixArgs {
+    float* o; const int* block_table; int table_stride; const int4* tiles;      // o [tokens][H][G][Dv]
+    int H, G, D, Dv, cg, window; float scale_log2e;
+    const float* sink;                             // [H] or null
+    int qp, vp, stages;                            // 64-column panels of a query (and key) row and of a value row; stages of the ring
+    int pool_rows;                                 // rows of the pools seen as matrices [rows][D] and [rows][Dv]
+};
+
+// A from tensor memory (a column holds two neighbouring entries of a row), B from shared memory
+__device__ __forceinline__ void ht_mma_ts(unsigned tmem_d, unsigned tmem_a, unsigned long long b, unsigned idesc, unsigned accumulate) {
+    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+                 " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n}"
+                 ::"r"(tmem_d), "r"(tmem_a), "l"(b), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+}
+
+// tiles[i] = (batch row, first packed token, number of tokens (<= 128), position of the first token)
+__global__ void __launch_bounds__(HT_THREADS, 1) attention_headmix_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q,
+                                                                                  const __grid_constant__ CUtensorMap map_k,
+                                                                                  const __grid_constant__ CUtensorMap map_v,
+                                                                                  const HeadmixArgs p, int* status) {
+    extern __shared__ __align__(1024) unsigned char ht_mem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned stage_bytes = (unsigned)(p.qp + p.cg * p.vp) * HT_PANEL;
+    const unsigned q_s = at_smem(ht_mem), kv_s = q_s + p.qp * HT_PANEL;
+    unsigned long long* bars = reinterpret_cast<unsigned long long*>(ht_mem + (size_t)p.qp * HT_PANEL + (size_t)p.stages * stage_bytes);
+    unsigned long long &q_full = bars[0];
+    unsigned long long *p_full = bars + 2, *pv_done = bars + 4, *s_full = bars + 6, *kv_full = bars + 8, *kv_empty = bars + 8 + HT_MAX_STAGES;
+    unsigned long long* pair_bar = bars + 8 + 2 * HT_MAX_STAGES;   // one for the two softmax warps of each 32 rows
+    unsigned& tmem_base_s = *reinterpret_cast<unsigned*>(bars + 12 + 2 * HT_MAX_STAGES);
+    volatile unsigned* stage_flags = reinterpret_cast<volatile unsigned*>(bars + HT_BAR_WORDS);   // bit g: page g of the stage exists
+    float* exchange = reinterpret_cast<float*>(bars + HT_BAR_WORDS + HT_MAX_STAGES);    // [meeting parity][half][row]: what the halves of a row tell each other
+    if (q_s & 1023u) {                                              // every thread alike: nothing is allocated yet
+        if (threadIdx.x == 0) atomicExch(status, 6);
+        return;
+    }
+    if (threadIdx.x == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(at_smem(&q_full)) : "memory");
+        for (int q = 0; q < 4; ++q) asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;" ::"r"(at_smem(&pair_bar[q])) : "memory");
+        for (int s = 0; s < HT_MAX_STAGES; ++s) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(at_smem(&kv_full[s])) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(at_smem(&kv_empty[s])) : "memory");
+        }
+        for (int b = 0; b < 2; ++b) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(at_smem(&s_full[b])) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 8;" ::"r"(at_smem(&p_full[b])) : "memory");      // the eight softmax warps
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(at_smem(&pv_done[b])) : "memory");
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(at_smem(&tmem_base_s)), "r"((unsigned)HT_TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const unsigned tmem = tmem_base_s;
+    // only now may the next kernel of the stream be scheduled: it could take tensor memory that a CTA of this grid still waits for
+    pdl_launch_dependents();
+    pdl_wait();
+
+    const int4 info = p.tiles[blockIdx.y];                          // heads vary fastest: the runs that see the most keys start first
+    const int brow = info.x, tok0 = info.y, n = info.z, pos0 = info.w;
+    const int groups = p.G / p.cg, h = blockIdx.x / groups, c_lo = blockIdx.x % groups * p.cg, kvh = h / (p.H / p.G);
+    const int first_key = (p.window > 0 && pos0 - p.window + 1 > 0) ? pos0 - p.window + 1 : 0;
+    const int page_lo = first_key / HT_KTILE, page_hi = (pos0 + n - 1) / HT_KTILE;
+    const int n_pages = page_hi - page_lo + 1, n_steps = (n_pages + 1) / 2;
+
+    if (warp == 0) {
+        if (lane == 0) {                                            // ---------------- loader
+            const int* table = p.block_table + (size_t)brow * p.table_stride;
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(at_smem(&q_full)), "r"((unsigned)(p.qp * HT_PANEL)) : "memory");
+            for (int c = 0; c < p.qp; ++c) at_tma_2d(q_s + c * HT_PANEL, &map_q, h * p.D + 64 * c, tok0, at_smem(&q_full));
+            int page[2] = {table[page_lo], 1 < n_pages ? table[page_lo + 1] : -1};
+            int s = 0;
+            unsigned round = 0;                                     // how often the ring has been filled
+            for (int it = 0; it < n_steps; ++it) {
+                int next[2] = {-1, -1};                             // the step after this one: its entries travel during the wait
+                if (2 * it + 2 < n_pages) next[0] = table[page_lo + 2 * it + 2];
+                if (2 * it + 3 < n_pages) next[1] = table[page_lo + 2 * it + 3];
+                if (round > 0 && !at_wait(at_smem(&kv_empty[s]), (round - 1) & 1u)) { atomicExch(status, 5); break; }
+                const unsigned bar = at_smem(&kv_full[s]), k_dst = kv_s + s * stage_bytes, v_dst = k_dst + p.qp * HT_PANEL;
+                stage_flags[s] = (page[0] >= 0 ? 1u : 0u) | (page[1] >= 0 ? 2u : 0u);
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(stage_bytes) : "memory");
+                for (int g = 0; g < 2; ++g) {
+                    // a page that is not there is read from beyond the pool's end, which gives zeros: its scores are masked and its
+                    // values add nothing; so are a row's entries behind its size (the queries hold the next head's there)
+                    const unsigned at = g * (HT_KTILE * 128);
+                    for (int c = 0; c < p.qp; ++c)
+                        at_tma_2d(k_dst + c * HT_PANEL + at, &map_k, 64 * c, page[g] >= 0 ? (page[g] * p.G + kvh) * HT_KTILE : p.pool_rows, bar);
+                    for (int v = 0; v < p.cg; ++v)
+                        for (int c = 0; c < p.vp; ++c)
+                            at_tma_2d(v_dst + (v * p.vp + c) * HT_PANEL + at, &map_v, 64 * c,
+                                      page[g] >= 0 ? (page[g] * p.G + c_lo + v) * HT_KTILE : p.pool_rows, bar);
+                }
+                page[0] = next[0]; page[1] = next[1];
+                if (++s == p.stages) { s = 0; ++round; }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {                                            // ---------------- MMA issuer
+            // instruction descriptors: float32 accumulator, bfloat16 operands, M = 128; S: A and B K-major, N = 128 keys;
+            // O: A from tensor memory, B MN-major (bit 16), N = Dv
+            const unsigned idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)((2 * HT_KTILE) >> 3) << 17) | ((unsigned)(HT_QTILE >> 4) << 24);
+            const unsigned idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((unsigned)(p.Dv >> 3) << 17) | ((unsigned)(HT_QTILE >> 4) << 24);
+            const unsigned long long dq = at_desc(q_s, 0, 1024), dk = at_desc(kv_s, 0, 1024), dv = at_desc(kv_s + p.qp * HT_PANEL, HT_PANEL, 1024);
+            const int k_steps = p.D / 16;
+            bool ok = at_wait(at_smem(&q_full), 0u);
+            int s_next = 0, s_here = 0;                             // the stages of the S issued next and of the P V issued next
+            unsigned s_round = 0;
+            auto issue_s = [&](int it) -> bool {                    // S of step `it` into buffer it & 1, when P V has read the P that lay there
+                const int b = it & 1;
+                if (it >= 2 && !at_wait(at_smem(&pv_done[b]), (unsigned)((it >> 1) - 1) & 1u)) return false;
+                if (!at_wait(at_smem(&kv_full[s_next]), s_round & 1u)) return false;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const unsigned long long dks = dk + (unsigned long long)(s_next * (stage_bytes >> 4));
+                for (int kk = 0; kk < k_steps; ++kk) {              // 16 columns = 32 bytes inside the swizzle atom; 64 columns = one panel
+                    const unsigned off = ((kk / 4) * HT_PANEL + (kk % 4) * 32) >> 4;
+                    at_mma(tmem + b * (2 * HT_KTILE), dq + off, dks + off, idesc_s, kk > 0 ? 1u : 0u);
+                }
+                at_commit(at_smem(&s_full[b]));
+                if (++s_next == p.stages) { s_next = 0; ++s_round; }
+                return true;
+            };
+            if (ok) ok = issue_s(0);
+            for (int it = 0; it < n_steps && ok; ++it) {
+                if (it + 1 < n_steps && !issue_s(it + 1)) { ok = false; break; }
+                const int b = it & 1;
+                if (!at_wait(at_smem(&p_full[b]), (unsigned)(it >> 1) & 1u)) { ok = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (int v = 0; v < p.cg; ++v) {
+                    const unsigned long long dvs = dv + (unsigned long long)(s_here * (stage_bytes >> 4) + v * p.vp * (HT_PANEL >> 4));
+#pragma unroll
+                    for (int kk = 0; kk < 2 * HT_KTILE / 16; ++kk)  // 16 keys: 8 columns further in P, 16 rows further in the panels
+                        ht_mma_ts(tmem + HT_O_COL + v * p.Dv, tmem + b * (2 * HT_KTILE) + kk * 8, dvs + ((kk * 16 * 128) >> 4), idesc_o, (it > 0 || kk > 0) ? 1u : 0u);
+                }
+                at_commit(at_smem(&kv_empty[s_here]));              // the stage's keys and values have been read
+                at_commit(at_smem(&pv_done[b]));                    // and O holds this step's share
+                if (++s_here == p.stages) s_here = 0;
+            }
+            if (!ok) atomicExch(status, 5);
+        }
+    } else {                                                        // ---------------- softmax, warps 2..9
+        // Two threads a query row: thread (row, g) has the scores of the step's page g (64 keys) and half of the row of O.  The two tell
+        // each other their maxima, and at the end their sums, through shared memory.
+        const int quarter = warp & 3;                               // the 32 lanes of tensor memory this warp may touch
+        const int g = (warp - 2) >> 2;
+        const int r = quarter * 32 + lane, p_r = pos0 + r;          // this thread's query row
+        const unsigned lane_addr = tmem + ((unsigned)(quarter * 32) << 16);
+        const int half = p.cg * p.Dv / 2;
+        const unsigned o_addr = lane_addr + HT_O_COL + g * half;
+        const unsigned pair = at_smem(&pair_bar[quarter]);
+        float m_run = -INFINITY, l_run = 0.f;
+        bool ok = true;
+        int it = 0, met = 0, st = 0;                                // met: how often the row's two threads have met; st: the step's stage
+        unsigned st_round = 0;
+        auto swap = [&](float mine, float& theirs) -> bool {        // tell the other half `mine`, learn what it tells
+            float* slot = exchange + (met & 1) * (2 * HT_QTILE);
+            slot[g * HT_QTILE + r] = mine;
+            __syncwarp();
+            if (lane == 0) at_arrive(pair);
+            if (!at_wait_warp(pair, (unsigned)met & 1u)) return false;
+            theirs = slot[(g ^ 1) * HT_QTILE + r];
+            ++met;
+            return true;
+        };
+        for (; it < n_steps; ++it) {
+            const int b = it & 1;
+            if (!at_wait_warp(at_smem(&s_full[b]), (unsigned)(it >> 1) & 1u)) { ok = false; break; }
+            // (S of the step exists, so its rows have landed; the flags were written before they were asked for)
+            if (!at_wait_warp(at_smem(&kv_full[st]), st_round & 1u)) { ok = false; break; }
+            const bool there = (stage_flags[st] >> g) & 1u;
+            if (++st == p.stages) { st = 0; ++st_round; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int key0 = (page_lo + 2 * it + g) * HT_KTILE;
+            unsigned raw[HT_KTILE];
+            at_ld32_start(lane_addr + b * (2 * HT_KTILE) + g * HT_KTILE, raw);
+            at_ld32_start(lane_addr + b * (2 * HT_KTILE) + g * HT_KTILE + 32, raw + 32);
+            at_ld_wait();
+            at_pin32(raw); at_pin32(raw + 32);
+            // the row sees the keys up to its own position and inside its window
+            float s[HT_KTILE];
+#pragma unroll
+            for (int c = 0; c < HT_KTILE; ++c) s[c] = __uint_as_float(raw[c]);
+            if (!(there && key0 + HT_KTILE - 1 <= p_r && (p.window <= 0 || key0 > p_r - p.window))) {
+#pragma unroll
+                for (int c = 0; c < HT_KTILE; ++c) {
+                    const int key = key0 + c;
+                    if (!there || key > p_r || (p.window > 0 && key <= p_r - p.window)) s[c] = -INFINITY;
+                }
+            }
+            float mx[4] = {s[0], s[1], s[2], s[3]};                 // four chains: a warp has little else to hide their latency
+#pragma unroll
+            for (int c = 4; c < HT_KTILE; ++c) mx[c & 3] = fmaxf(mx[c & 3], s[c]);
+            const float m_mine = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+            float m_theirs;
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            if (!swap(m_mine, m_theirs)) { ok = false; break; }     // (after this the other half has read its scores too: their columns take P)
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            // The reference point of the exponentials follows the row's maximum only when that has grown by more than HT_LAZY (in powers
+            // of two).  Both threads of a row compute the same from the same numbers.
+            const float m_tile = fmaxf(m_mine, m_theirs) * p.scale_log2e;
+            const float m_new = (m_run != -INFINITY && m_tile <= m_run + HT_LAZY) ? m_run : fmaxf(m_run, m_tile);
+            const float m_use = m_new == -INFINITY ? 0.f : m_new;
+            const float alpha = m_run == -INFINITY ? 1.0f : at_exp2(m_run - m_use);
+            m_run = m_new;
+            float sum[4] = {0.f, 0.f, 0.f, 0.f};
+            float packed[HT_KTILE / 2];
+#pragma unroll
+            for (int c = 0; c < HT_KTILE; c += 2) {
+                const float e0 = at_exp2(fmaf(s[c], p.scale_log2e, -m_use)), e1 = at_exp2(fmaf(s[c + 1], p.scale_log2e, -m_use));
+                sum[c & 3] += e0; sum[(c + 1) & 3] += e1;
+                packed[c >> 1] = __uint_as_float(at_pack(e0, e1));
+            }
+            l_run = l_run * alpha + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
+            at_st32(lane_addr + b * (2 * HT_KTILE) + g * (HT_KTILE / 2), packed);
+            if (it > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) { // a row's reference point moved: rescale this half of the warp's rows of O
+                if (!at_wait_warp(at_smem(&pv_done[b ^ 1]), (unsigned)((it - 1) >> 1) & 1u)) { ok = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+                for (int c = 0; c < half; c += 32) {
+                    float o[32];
+                    at_ld32(o_addr + c, o);
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) o[i] *= alpha;
+                    at_st32(o_addr + c, o);
+                }
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) at_arrive(at_smem(&p_full[b]));
+        }
+        // the row's sum, and the last P V (products complete in the order they were issued)
+        float l_theirs = 0.f;
+        if (ok && !swap(l_run, l_theirs)) ok = false;
+        if (ok && it > 0 && !at_wait_warp(at_smem(&pv_done[(it - 1) & 1]), (unsigned)((it - 1) >> 1) & 1u)) ok = false;
+        if (ok && it > 0) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            float l = g == 0 ? l_run + l_theirs : l_theirs + l_run;         // the same sum in both threads
+            if (p.sink) l += at_exp2(fmaf(p.sink[h], 1.4426950408889634f, -m_run));       // (a row that saw no key: 2^inf, and 1 / l = 0)
+            const float inv = l > 0.f ? 1.0f / l : 0.f;
+            float* o_row = p.o + (((size_t)(tok0 + r) * p.H + h) * p.G + c_lo) * p.Dv + g * half;      // the group's heads lie side by side
+#pragma unroll 1
+            for (int c = 0; c < half; c += 32) {
+                float o[32];
+                at_ld32(o_addr + c, o);
+                if (r < n) {
+#pragma unroll
+                    for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(o_row + c + i) = make_float4(o[i] * inv, o[i + 1] * inv, o[i + 2] * inv, o[i + 3] * inv);
+                }
+            }
+        }
+        if (!ok) atomicExch(status, 5);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((unsigned)HT_TMEM_COLS) : "memory");
+    }
+}
+
+// out[t][h][d] = sum_g mix[h, g] o[t][g][c(h)][d].  A thread has column d of key/value head c and up to eight of the heads that read it
+// (blockIdx.y: which eight): a head's outputs are read once for all of them, neighbouring threads side by side, and no read waits for
+// another.  Bound by reading o.
+#define HT_MIX_HEADS 8
+__global__ void __launch_bounds__(256) headmix_mix_kernel(const float* o, const float* mix, bf16* out, int T, int H, int G, int Dv) {
+    pdl_launch_dependents();
+    pdl_wait();
+    extern __shared__ float ht_mix[];                               // [H][H]
+    const int per = H / G, cols = G * Dv;
+    for (int i = threadIdx.x; i < H * H; i += blockDim.x) ht_mix[i] = mix[i];
+    __syncthreads();
+    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= (long long)T * cols) return;
+    const int t = (int)(e / cols), col = (int)(e % cols), c = col / Dv, d = col % Dv;
+    const int h0 = c * per + blockIdx.y * HT_MIX_HEADS, n_h = min(HT_MIX_HEADS, c * per + per - h0);
+    const float* src = o + (size_t)t * H * cols + col;
+    float acc[HT_MIX_HEADS];
+#pragma unroll
+    for (int i = 0; i < HT_MIX_HEADS; ++i) acc[i] = 0.f;
+#pragma unroll 8
+    for (int g = 0; g < H; ++g) {
+        const float v = src[(size_t)g * cols];
+#pragma unroll
+        for (int i = 0; i < HT_MIX_HEADS; ++i) acc[i] = fmaf(ht_mix[min(h0 + i, H - 1) * H + g], v, acc[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < HT_MIX_HEADS; ++i)
+        if (i < n_h) out[((size_t)t * H + h0 + i) * Dv + d] = __float2bfloat16_rn(acc[i]);
+}
+
+// How the sizes are laid out: value heads a CTA and stages of the ring; false: not taken.
+static bool ht_plan(int H, int G, int D, int Dv, HeadmixArgs& a) {
+    if (H < 1 || G < 1 || H % G || H > 128 || D < 16 || D % 16 || D > 256 || Dv < 16 || Dv % 16 || Dv > 256) return false;
+    a.qp = (D + 63) / 64;
+    a.vp = (Dv + 63) / 64;
+    for (int cg = G; cg >= 1; --cg) {
+        if (G % cg || cg * Dv > 256 || cg * Dv % 64) continue;
+        const int stage = (a.qp + cg * a.vp) * HT_PANEL;
+        int stages = (HT_SMEM_LIMIT - HT_SMALL_BYTES - a.qp * HT_PANEL) / stage;
+        if (stages > HT_MAX_STAGES) stages = HT_MAX_STAGES;
+        if (stages < 2) continue;                                   // S of a step is made before P V of the step before: two stages at least
+        a.cg = cg;
+        a.stages = stages;
+        return true;
+    }
+    return false;
+}
+extern "C" int pe_attention_headmix_tcgen05_takes(int H, int G, int D, int Dv) {
+    HeadmixArgs a;
+    return ht_plan(H, G, D, Dv, a) ? 1 : 0;
+}
+
+// q: [T][q_stride] with head h at columns h * D; pools: [pool_pages][G][64][D] and [..][Dv]; scratch: float32 [T][H][G][Dv]; out [T][H * Dv]
+extern "C" int pe_attention_headmix_tcgen05(const void* q, int q_stride, void* out, const void* k_pool, const void* v_pool, long long pool_pages,
+                                            const int* block_table, int table_stride, const void* tiles, int n_tiles, int T, int H, int G, int D,
+                                            int Dv, int window, float scale, const float* sink, const float* mix, float* scratch, int* status, void* stream) {
+    if (n_tiles <= 0) return 0;
+    HeadmixArgs a = {scratch, block_table, table_stride, (const int4*)tiles, H, G, D, Dv, 0, window, scale * 1.4426950408889634f, sink, 0, 0, 0,
+                     (int)(pool_pages * G * HT_KTILE)};
+    if (!ht_plan(H, G, D, Dv, a) || n_tiles > 65535 || q_stride % 8 || !(scale > 0.f) || !status || !mix) return PE_ERR_UNSUPPORTED;
+    if (((uintptr_t)q | (uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)tiles | (uintptr_t)scratch) & 15) return PE_ERR_UNSUPPORTED;
+    if (pool_pages * G * HT_KTILE > 0x7fffff00ll) return PE_ERR_UNSUPPORTED;         // TMA coordinates are 32-bit
+    CUtensorMap mq, mk, mv;
+    int rc = at_make_map(&mq, q, T, (long long)H * D, q_stride, HT_QTILE);
+    if (rc) return rc;
+    rc = at_make_map(&mk, k_pool, pool_pages * G * HT_KTILE, D, D, HT_KTILE);
+    if (rc) return rc;
+    rc = at_make_map(&mv, v_pool, pool_pages * G * HT_KTILE, Dv, Dv, HT_KTILE);
+    if (rc) return rc;
+    cudaStream_t s = (cudaStream_t)stream;
+    size_t smem = (size_t)a.qp * HT_PANEL + (size_t)a.stages * (a.qp + a.cg * a.vp) * HT_PANEL + HT_SMALL_BYTES;
+    if (smem < 120 * 1024) smem = 120 * 1024;                       // one CTA an SM: it takes all of tensor memory
+    PE_TRY(cudaFuncSetAttribute(attention_headmix_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, HT_SMEM_LIMIT));
+    PE_TRY(pe_launch(attention_headmix_tcgen05_kernel, dim3(H * (G / a.cg), n_tiles), HT_THREADS, smem, s, mq, mk, mv, a, status));
+    PE_LAUNCH_CHECK();
+    const size_t mix_smem = sizeof(float) * H * H;
+    if (mix_smem > 48 * 1024) PE_TRY(cudaFuncSetAttribute(headmix_mix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mix_smem));
+    const dim3 grid((unsigned)(((long long)T * G * Dv + 255) / 256), (H / G + HT_MIX_HEADS - 1) / HT_MIX_HEADS);
+    PE_TRY(pe_launch(headmix_mix_kernel, grid, 256, mix_smem, s, (const float*)scratch, mix, (bf16*)out, T, H, G, Dv));
+    PE_LAUNCH_CHECK();
+    return 0;
+}

@@ -858,7 +858,8 @@ def qknorm_store(qkv: torch.Tensor, n_heads: int, n_kv: int, head_dim: int, v_he
                                    1 if store else 0, stream_ptr()), "qknorm_store")
 
 
-# Which kernel runs head-mixing attention in bfloat16: "1" the one-pass tensor-core kernel (attention_headmix_flash.cu) where
+# Which kernel runs head-mixing attention in bfloat16: "1" the tcgen05 kernel for prompts (attention_headmix_tcgen05.cu) and the one-pass
+# mma.sync kernel (attention_headmix_flash.cu) for single tokens and where
 # it takes the sizes, else the two-pass one (attention_headmix_mma.cu), else float32 FMAs; "two-pass" and "0" skip the first
 # or both (the tests run all three).
 HEADMIX_TENSOR_CORES = os.environ.get("PICO_ENGINE_HEADMIX_MMA", "1")
@@ -968,6 +969,18 @@ def attention_headmix(q: torch.Tensor, q_stride: int, n_heads: int, n_kv: int, h
     from .workspace import scratch
     out = torch.empty(T, n_heads * v_head_dim, dtype=out_dtype or q.dtype, device=q.device)
     floats = all(t is None or t.dtype == torch.float32 for t in (sink, mix))
+    if (plain_out and q.dtype == torch.bfloat16 and tiles is not None and HEADMIX_TENSOR_CORES == "1" and floats and plain_mask and mix is not None
+            and scale > 0 and q_stride % 8 == 0 and (q.data_ptr() | k_pool.data_ptr() | v_pool.data_ptr()) % 16 == 0
+            and lib.pe_attention_headmix_tcgen05_takes(n_heads, n_kv, head_dim, v_head_dim)):
+        # prompts whose weights are mixed: both products on tcgen05, the mixing behind them (1,024 tokens, 16
+        # heads of 128 on four key/value heads on a B200: 55 us against 281 us of the mma.sync kernel and its merge)
+        runs = _step_tiles(ctx, PREFILL_TILE_TCGEN05, q.device)
+        ws = scratch("attention_headmix", 4 * T * n_heads * n_kv * v_head_dim, q.device)
+        check(lib.pe_attention_headmix_tcgen05(q.data_ptr(), q_stride, out.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), k_pool.shape[0],
+                                               block_table.data_ptr(), table_stride, runs.data_ptr(), runs.shape[0], T, n_heads, n_kv, head_dim,
+                                               v_head_dim, window or 0, float(scale), _ptr(sink), _ptr(mix), ws.data_ptr(),
+                                               status_ptr(q.device), stream_ptr()), "attention_headmix_tcgen05", 2)
+        return out
     if plain_out and q.dtype == torch.bfloat16 and HEADMIX_TENSOR_CORES == "1" and floats:
         cg = lib.pe_attention_flashmix_group(n_heads, n_kv, head_dim, v_head_dim)
         if cg and q_stride % 2 == 0 and v_ld % 8 == 0:

@@ -20,7 +20,7 @@ EXTRA_SOURCES = ("linear_mma.cu", "linear_batch.cu", "gemm_splitk.cu")
 # The kernels of parts that only some designs have (layer norm with the short convolution on a sublayer's input, attention
 # whose weights are mixed across heads, the gated recurrence): compiled when a model with such a part is built.
 MIXER_SOURCES = ("layernorm_conv.cu", "attention_headmix.cu", "attention_headmix_mma.cu", "attention_headmix_flash.cu",
-                 "gated_recurrence.cu")
+                 "attention_headmix_tcgen05.cu", "gated_recurrence.cu")
 # The kernels of gated mixers and routed feed-forwards (the linear-attention recurrence, rotation of pairs with unit norm and
 # cache write, norms over groups of channels with a gate, sums of normed branches, gated activations, the choice of experts;
 # branches that share their first and last product, and residuals of several streams).
@@ -69,6 +69,8 @@ _MIXER_SIGNATURES = {
     "pe_mingru": [P, I, P, LL, P, P, P, P, P, I, I, I, I, P, P],
     "pe_attention_headmix": [P, I, P, P, P, I, P, I, P, P, P, I, I, I, I, I, I, I, I, F, P, I, P, I, I, I, P, P, I, I, I, I, I, P],
     "pe_qknorm_store": [P, I, I, I, I, I, I, P, I, P, I, F, P, P, P, P, P, I, I, P],
+    "pe_attention_headmix_tcgen05_takes": [I, I, I, I],
+    "pe_attention_headmix_tcgen05": [P, I, P, P, P, LL, P, I, P, I, I, I, I, I, I, I, F, P, P, P, P, P],
     "pe_attention_flashmix": [P, I, P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, F, P, P, I, P, P, I, I, P],
     "pe_attention_headmix_mma": [P, I, P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, F, P, P, I, P, P],
 }

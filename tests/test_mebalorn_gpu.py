@@ -243,6 +243,51 @@ def test_headmix_kernel_sink_alone_scales_the_output():
         assert abs(float(got[0, 0, 0]) - 1 / (1 + math.exp(sink - 1.6))) < 1e-6 and abs(float(got[0, 1, 0]) - 0.5) < 1e-6
 
 
+@pytest.mark.parametrize("H,G,D,Dv,window", [(2, 1, 16, 64, None), (6, 2, 48, 96, 100), (3, 3, 64, 64, None), (16, 4, 128, 128, None),
+                                             (20, 2, 64, 64, 1), (4, 4, 128, 128, 300), (5, 1, 64, 256, None), (7, 7, 32, 64, 64)])
+def test_headmix_prompts_in_tensor_memory(H, G, D, Dv, window):
+    """The tcgen05 kernel at every grouping of value heads: several sequences in a step, whole and in portions off the borders of pages and
+    of runs of 128 tokens, against the same in float64; the sizes are ones that it takes."""
+    from pico_engine.ops import kernels
+    from pico_engine.ops.library import mixers
+    assert mixers().pe_attention_headmix_tcgen05_takes(H, G, D, Dv)
+    g = torch.Generator().manual_seed(H * 100 + D)
+    lens, dt, scale = [1, 65, 400], torch.bfloat16, 1.5 * D ** -0.5
+    T = sum(lens)
+    q, k, v = (rounded(torch.randn(T, h, d, generator=g), dt) for h, d in ((H, D), (G, D), (G, Dv)))
+    sink, talk = torch.randn(H, generator=g), (torch.eye(H) + 0.4 * torch.randn(H, H, generator=g))
+    want, pools, table, at, pages = [], [], torch.full((len(lens), 7), -1, dtype=torch.int32), 0, 0
+    for b, n in enumerate(lens):
+        kp, vp, tab = paged(k[at: at + n], v[at: at + n], dt)
+        pools.append((kp, vp))
+        table[b, : tab.shape[1]] = tab[0].cpu() + pages
+        pages += kp.shape[0]
+        i, j = torch.arange(n)[:, None], torch.arange(n)[None]
+        seen = (j <= i) if window is None else (j <= i) & (i - j < window)
+        kk, vv = (t[at: at + n].repeat_interleave(H // G, 1) for t in (k, v))
+        s = (torch.einsum("ihd,jhd->hij", q[at: at + n], kk) * scale).masked_fill(~seen, float("-inf"))
+        w = torch.softmax(torch.cat([s, sink.double().view(H, 1, 1).expand(H, n, 1)], -1), -1)[..., :n]
+        want.append(torch.einsum("hij,jhd->ihd", torch.einsum("hg,gij->hij", talk.double(), w), vv))
+        at += n
+    want = torch.cat(want).reshape(T, H * Dv)
+    kp, vp = (torch.cat([p[x] for p in pools]).contiguous() for x in (0, 1))
+    first = np.concatenate([[0], np.cumsum(lens)])
+    for cuts in ([(0, n) for n in lens], [(n // 3, n) for n in lens], [(n - min(n, 2), n) for n in lens]):
+        idx = torch.cat([torch.arange(first[b] + lo, first[b] + hi) for b, (lo, hi) in enumerate(cuts)])
+        tab = table.clone()
+        if window is not None:
+            for b, (lo, _) in enumerate(cuts):
+                tab[b, : max(0, lo - window + 1) // 64] = -1
+        ctx = SimpleNamespace(one_token_each=False, scratch={}, lens=[hi - lo for lo, hi in cuts], starts=[lo for lo, _ in cuts], max_context=max(lens))
+        pos = torch.cat([torch.arange(lo, hi, dtype=torch.int32) for lo, hi in cuts]).cuda()
+        row = torch.cat([torch.full((hi - lo,), b, dtype=torch.int32) for b, (lo, hi) in enumerate(cuts)]).cuda()
+        got = kernels.attention_headmix(q[idx].reshape(len(idx), -1).to(dt).cuda(), H * D, H, G, D, Dv, kp, vp, tab.cuda(), tab.shape[1], pos, row,
+                                        window, scale, sink.cuda(), talk.cuda().contiguous(), ctx)
+        kernels.check_status(torch.device("cuda", torch.cuda.current_device()))
+        # as the other bfloat16 kernels of this attention: weights and results rounded to 2^-9, mixed with weights of up to two
+        assert (got.double().cpu() - want[idx]).abs().max() < 1.5e-2 * max(1.0, float(want.abs().max())), cuts
+
+
 # ------------------------------------------------------------------ the recurrence, alone
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
