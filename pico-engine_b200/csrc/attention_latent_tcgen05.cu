@@ -40,13 +40,6 @@ struct LatentArgs {
     const bf16* gate; int gate_ld;                 // null, or: head h of token t leaves times sigmoid(gate[t * gate_ld + h])
 };
 
-// A from tensor memory (a column holds two neighbouring entries of a row), B from shared memory
-__device__ __forceinline__ void lt_mma_ts(unsigned tmem_d, unsigned tmem_a, unsigned long long b, unsigned idesc, unsigned accumulate) {
-    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                 " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n}"
-                 ::"r"(tmem_d), "r"(tmem_a), "l"(b), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
-}
-
 // tiles[i] = (batch row, first packed token, number of tokens (<= 128), position of the first token); KP: 64-column panels of a row
 template <int KP>
 __global__ void __launch_bounds__(LT_THREADS, 1) attention_latent_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q,
@@ -157,7 +150,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) attention_latent_tcgen05_kernel
                 const unsigned long long dvs = dv + (unsigned long long)(s * (STAGE >> 4));
 #pragma unroll
                 for (int kk = 0; kk < 2 * LT_KTILE / 16; ++kk)      // 16 keys: 8 columns further in P, 16 rows further in the panels
-                    lt_mma_ts(tmem + LT_O_COL, tmem + b * (2 * LT_KTILE) + kk * 8, dvs + ((kk * 16 * 128) >> 4), idesc_o, (it > 0 || kk > 0) ? 1u : 0u);
+                    at_mma_ts(tmem + LT_O_COL, tmem + b * (2 * LT_KTILE) + kk * 8, dvs + ((kk * 16 * 128) >> 4), idesc_o, (it > 0 || kk > 0) ? 1u : 0u);
                 at_commit(at_smem(&kv_empty[s]));                   // the stage's rows have been read
                 at_commit(at_smem(&pv_done[b]));                    // and O holds this step's share
             }

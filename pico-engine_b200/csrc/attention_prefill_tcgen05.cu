@@ -6,19 +6,24 @@
 //   a step    = two pages of the cache (128 keys): products this small cost the tensor core more in
 //               fixed latency than in work, so fewer and larger ones are issued
 //   warp 0      loader: TMA tiled loads (cp.async.bulk.tensor.2d, 128-byte swizzle) of the run's
-//               queries and, step after step, of the pages' keys and values into a ring; it alone
-//               reads the page table and tells the others through flags which pages are there
+//               queries and, step after step, of the pages' keys and values into a ring
 //   warp 1      allocates tensor memory; one lane issues S = Q.K^T (128 x 128, K = head size) into
-//               one of two S buffers and O += P.V (128 x head size, K = 128 keys): S of the next
-//               step is issued before P.V of this one, so the softmax never waits for the product
-//   warps 2-9   softmax, two threads a query row, one for each page of the step: tcgen05.ld of its
-//               64 scores, mask, maximum (the two tell each other theirs through shared memory),
-//               P = 2^(s - max) rounded to bfloat16 into one of two swizzled shared-memory tiles,
-//               the A operand of P.V, and the row sum in float32; when a row's reference point
-//               moves, the row of O in tensor memory is rescaled (tcgen05.ld / tcgen05.st), each
-//               thread its half, before P.V runs.  Two warps on each of the SM's four schedulers
-//               hide each other's latencies; the exponentials (one special-function unit a
-//               scheduler) and the tensor core's time for the two products then bound a step.
+//               one of three S buffers and O += P.V (128 x head size, K = 128 keys); S runs three
+//               steps ahead of P.V.  A stage's keys are free for the next ones when S has read them,
+//               its values when P.V has
+//   warps 2-9   softmax, two warpgroups that take the steps in turn, a thread a query row: tcgen05.ld
+//               of its 128 scores, mask, maximum, P = 2^(s - reference) rounded to bfloat16 back into
+//               the S buffer's own columns (tcgen05.st), where it is the A operand of P.V, and a row sum
+//               in float32 a warpgroup.  From step to step only a row's reference point goes from one
+//               warpgroup to the other (through shared memory, before the exponentials), so that one
+//               group's waits, loads and maxima lie under the other's exponentials.  When a reference
+//               point moves, the row of O in tensor memory is rescaled (tcgen05.ld / tcgen05.st) before P.V.
+//
+// What bounds a step: its 16,384 exponentials take 1,024 cycles of the special-function units.  With all
+// eight warps on one step (two threads a row that told each other their maxima) a step was a chain of
+// 2,480 cycles (clock stamps: waits 370, maxima 430, exponentials 1,100, P through shared memory 350);
+// with the warpgroups in turn it is 1,500 (head size 64) and about 1,700 (128).  2,048 tokens, 14 heads of 64, on a B200: 30 us before,
+// 26 us here; 28 heads of 128, prompts of 5,001 / 1,807 / 700 / 33 tokens: 341 us before, 278 us here.
 //
 // Values lie in the cache as [key][head size], which is the MN-major form of the B operand of
 // P.V: its shared-memory descriptor steps 8 keys by 1024 bytes and 64 columns by one panel.
@@ -38,16 +43,17 @@
 #define AT_QTILE 128
 #define AT_KTILE PE_PAGE
 #define AT_PANELS (AT_HD / 64)                     // 64-column panels of a row: one 128-byte swizzle atom each
-#define AT_STAGES (AT_HD == 64 ? 3 : 2)            // steps in flight or in use; a step is two pages (128 keys)
-#define AT_THREADS 320                             // loader, MMA issuer, and two softmax warps for each 32 rows
+#define AT_STAGES (AT_HD == 64 ? 5 : 3)            // steps in flight or in use; a step is two pages (128 keys)
+#define AT_AHEAD 3                                 // steps that S is issued ahead of P.V (no more than stages or S buffers)
+#define AT_THREADS 320                             // loader, MMA issuer, and two softmax warpgroups
 #define AT_Q_BYTES (AT_QTILE * AT_HD * 2)
 #define AT_STAGE_BYTES (2 * 2 * AT_KTILE * AT_HD * 2)   // keys, then values, of two pages and one head
-#define AT_P_BYTES (AT_QTILE * 2 * AT_KTILE * 2)   // P of one step: the A operand of P.V, two panels of 64 keys
-#define AT_TILE_BYTES (AT_Q_BYTES + AT_STAGES * AT_STAGE_BYTES + 2 * AT_P_BYTES)
-#define AT_BAR_WORDS (13 + 2 * AT_STAGES)
-#define AT_SMEM_BYTES (AT_TILE_BYTES + 8 * AT_BAR_WORDS + 8 * AT_STAGES + 2 * 2 * AT_QTILE * 4)
-#define AT_TMEM_COLS 512                           // S buffers at columns 0 and 128, O from column 256
-#define AT_O_COL 256
+#define AT_TILE_BYTES (AT_Q_BYTES + AT_STAGES * AT_STAGE_BYTES)
+#define AT_BUFFERS 3                               // S buffers
+#define AT_BAR_WORDS (2 + 3 * AT_BUFFERS + 4 * AT_STAGES + 12)
+#define AT_SMEM_BYTES (AT_TILE_BYTES + 8 * AT_BAR_WORDS + 2 * 2 * AT_QTILE * 4)
+#define AT_TMEM_COLS 512                           // S buffers (then P) at columns 0, 128 and 256, O from column 384
+#define AT_O_COL (AT_BUFFERS * 2 * AT_KTILE)
 #define AT_LAZY 8.0f
 
 struct AtArgs {
@@ -64,36 +70,32 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_prefill_tcgen05_kerne
                                                                                   const __grid_constant__ CUtensorMap map_k,
                                                                                   const __grid_constant__ CUtensorMap map_v,
                                                                                   const AtArgs p, int* status) {
-    // Q | stages of (K, V of two pages) | two P tiles | barriers and the stages' flags.  The tiles need 1024-byte
+    // Q | stages of (K, V of two pages) | barriers | what the warpgroups tell each other.  The tiles need 1024-byte
     // alignment for the swizzle, which the declaration asks for and the kernel checks.
     extern __shared__ __align__(1024) unsigned char at_mem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const unsigned q_s = at_smem(at_mem), kv_s = q_s + AT_Q_BYTES, p_s = kv_s + AT_STAGES * AT_STAGE_BYTES;
+    const unsigned q_s = at_smem(at_mem), kv_s = q_s + AT_Q_BYTES;
     unsigned long long* bars = reinterpret_cast<unsigned long long*>(at_mem + AT_TILE_BYTES);
-    unsigned long long &q_full = bars[0], &p_full = bars[1];
-    unsigned long long *pv_done = bars + 2, *s_full = bars + 4, *s_free = bars + 6, *kv_full = bars + 8, *kv_empty = bars + 8 + AT_STAGES;
-    unsigned long long* pair_bar = bars + 8 + 2 * AT_STAGES;       // one for the two softmax warps of each 32 rows
-    unsigned& tmem_base_s = *reinterpret_cast<unsigned*>(bars + 12 + 2 * AT_STAGES);
-    volatile unsigned* stage_flags = reinterpret_cast<volatile unsigned*>(bars + AT_BAR_WORDS);   // bit g: page g of the stage exists
-    float* exchange = reinterpret_cast<float*>(bars + AT_BAR_WORDS + AT_STAGES);    // [step parity][half][row]: what the halves of a row tell each other
+    unsigned long long& q_full = bars[0];
+    unsigned& tmem_base_s = *reinterpret_cast<unsigned*>(bars + 1);
+    unsigned long long *s_full = bars + 2, *p_full = s_full + AT_BUFFERS, *pv_done = p_full + AT_BUFFERS;
+    unsigned long long *k_full = pv_done + AT_BUFFERS, *v_full = k_full + AT_STAGES, *k_empty = v_full + AT_STAGES, *v_empty = k_empty + AT_STAGES;
+    unsigned long long* told = v_empty + AT_STAGES;                 // [warpgroup][32 rows]: a step's reference points are there
+    unsigned long long* met = told + 8;                             // [32 rows]: both warpgroups have come to the end
+    float* refs = reinterpret_cast<float*>(bars + AT_BAR_WORDS);    // [warpgroup][row]: reference point of the group's last step
+    float* sums = refs + 2 * AT_QTILE;                              // [warpgroup][row]: at the end, the group's share of the row's sum
     if (q_s & 1023u) {                                              // every thread alike: nothing is allocated yet
         if (threadIdx.x == 0) atomicExch(status, 6);
         return;
     }
 
     if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(at_smem(&q_full)) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 8;" ::"r"(at_smem(&p_full)) : "memory");          // the eight softmax warps
-        for (int q = 0; q < 4; ++q) asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;" ::"r"(at_smem(&pair_bar[q])) : "memory");
-        for (int s = 0; s < AT_STAGES; ++s) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(at_smem(&kv_full[s])) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(at_smem(&kv_empty[s])) : "memory");
-        }
-        for (int b = 0; b < 2; ++b) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(at_smem(&s_full[b])) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 8;" ::"r"(at_smem(&s_free[b])) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(at_smem(&pv_done[b])) : "memory");
-        }
+        auto init = [](unsigned long long* bar, unsigned count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(at_smem(bar)), "r"(count) : "memory"); };
+        init(&q_full, 1);
+        for (int s = 0; s < AT_STAGES; ++s) { init(&k_full[s], 1); init(&v_full[s], 1); init(&k_empty[s], 1); init(&v_empty[s], 1); }
+        for (int b = 0; b < AT_BUFFERS; ++b) { init(&s_full[b], 1); init(&p_full[b], 4); init(&pv_done[b], 1); }     // p_full: a warpgroup's four warps
+        for (int w = 0; w < 8; ++w) init(&told[w], 1);
+        for (int q = 0; q < 4; ++q) init(&met[q], 2);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -136,21 +138,23 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_prefill_tcgen05_kerne
                 int next[2] = {-1, -1};                             // the step after this one: its entries travel during the wait
                 if (2 * it + 2 < n_pages) next[0] = table[page_at(2 * it + 2)];
                 if (2 * it + 3 < n_pages) next[1] = table[page_at(2 * it + 3)];
-                if (it >= AT_STAGES && !at_wait(at_smem(&kv_empty[s]), (unsigned)((it / AT_STAGES) - 1) & 1u)) { atomicExch(status, 5); break; }
-                const unsigned bar = at_smem(&kv_full[s]), k_dst = kv_s + s * AT_STAGE_BYTES, v_dst = k_dst + AT_STAGE_BYTES / 2;
-                stage_flags[s] = (page[0] >= 0 ? 1u : 0u) | (page[1] >= 0 ? 2u : 0u);
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((unsigned)AT_STAGE_BYTES) : "memory");
+                const unsigned k_dst = kv_s + s * AT_STAGE_BYTES, v_dst = k_dst + AT_STAGE_BYTES / 2, round = (unsigned)((it / AT_STAGES) - 1) & 1u;
+                // a page that is not there (beyond the run's last page, or left behind by the window) is read from
+                // beyond the pool's end, which gives zeros: its scores are masked and its values add nothing
+                int y[2];
 #pragma unroll
-                for (int g = 0; g < 2; ++g) {
-                    // a page that is not there (beyond the run's last page, or left behind by the window) is read from
-                    // beyond the pool's end, which gives zeros: its scores are masked and its values add nothing
-                    const int y = page[g] >= 0 ? (page[g] * p.nkv + kvh) * AT_KTILE : p.pool_rows;
+                for (int g = 0; g < 2; ++g) y[g] = page[g] >= 0 ? (page[g] * p.nkv + kvh) * AT_KTILE : p.pool_rows;
+                auto bring = [&](const CUtensorMap* map, unsigned dst, unsigned bar) {
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((unsigned)AT_STAGE_BYTES / 2) : "memory");
 #pragma unroll
-                    for (int c = 0; c < AT_PANELS; ++c) {
-                        at_tma_2d(k_dst + c * (2 * AT_KTILE * 128) + g * (AT_KTILE * 128), &map_k, 64 * c, y, bar);
-                        at_tma_2d(v_dst + c * (2 * AT_KTILE * 128) + g * (AT_KTILE * 128), &map_v, 64 * c, y, bar);
-                    }
-                }
+                    for (int g = 0; g < 2; ++g)
+#pragma unroll
+                        for (int c = 0; c < AT_PANELS; ++c) at_tma_2d(dst + c * (2 * AT_KTILE * 128) + g * (AT_KTILE * 128), map, 64 * c, y[g], bar);
+                };
+                if (it >= AT_STAGES && !at_wait(at_smem(&k_empty[s]), round)) { atomicExch(status, 5); break; }
+                bring(&map_k, k_dst, at_smem(&k_full[s]));
+                if (it >= AT_STAGES && !at_wait(at_smem(&v_empty[s]), round)) { atomicExch(status, 5); break; }
+                bring(&map_v, v_dst, at_smem(&v_full[s]));
                 page[0] = next[0]; page[1] = next[1];
             }
         }
@@ -160,14 +164,14 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_prefill_tcgen05_kerne
             // S: A and B K-major, N = 128 keys;  O: B MN-major (bit 16), N = head size
             const unsigned idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)((2 * AT_KTILE) >> 3) << 17) | ((unsigned)(AT_QTILE >> 4) << 24);
             const unsigned idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((unsigned)(AT_HD >> 3) << 17) | ((unsigned)(AT_QTILE >> 4) << 24);
-            // operand descriptors of stage 0 and P tile 0; a stage or tile further on adds its offset in 16-byte units
-            const unsigned long long dq = at_desc(q_s, 0, 1024), dk = at_desc(kv_s, 0, 1024), dp = at_desc(p_s, 0, 1024);
+            // operand descriptors of stage 0; a stage further on adds its offset in 16-byte units
+            const unsigned long long dq = at_desc(q_s, 0, 1024), dk = at_desc(kv_s, 0, 1024);
             const unsigned long long dv = at_desc(kv_s + AT_STAGE_BYTES / 2, 2 * AT_KTILE * 128, 1024);
             bool ok = at_wait(at_smem(&q_full), 0u);
-            auto issue_s = [&](int it) -> bool {                    // S = Q . K^T of step `it` into S buffer it & 1
-                const int s = it % AT_STAGES, b = it & 1;
-                if (!at_wait(at_smem(&kv_full[s]), (unsigned)(it / AT_STAGES) & 1u)) return false;
-                if (it >= 2 && !at_wait(at_smem(&s_free[b]), (unsigned)((it >> 1) - 1) & 1u)) return false;
+            auto issue_s = [&](int it) -> bool {                    // S = Q . K^T of step `it`, when P.V has read the P that lay in its buffer
+                const int s = it % AT_STAGES, b = it % AT_BUFFERS;
+                if (it >= AT_BUFFERS && !at_wait(at_smem(&pv_done[b]), (unsigned)(it / AT_BUFFERS - 1) & 1u)) return false;
+                if (!at_wait(at_smem(&k_full[s]), (unsigned)(it / AT_STAGES) & 1u)) return false;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const unsigned long long dks = dk + (unsigned long long)(s * (AT_STAGE_BYTES >> 4));
 #pragma unroll
@@ -175,146 +179,156 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_prefill_tcgen05_kerne
                     const unsigned off_q = ((kk / 4) * (AT_QTILE * 128) + (kk % 4) * 32) >> 4, off_k = ((kk / 4) * (2 * AT_KTILE * 128) + (kk % 4) * 32) >> 4;
                     at_mma(tmem + b * (2 * AT_KTILE), dq + off_q, dks + off_k, idesc_s, kk > 0 ? 1u : 0u);
                 }
+                at_commit(at_smem(&k_empty[s]));                    // the stage's keys have been read
                 at_commit(at_smem(&s_full[b]));
                 return true;
             };
-            if (ok) ok = issue_s(0);
+            for (int it = 0; it < min(AT_AHEAD, n_steps) && ok; ++it) ok = issue_s(it);
             for (int it = 0; it < n_steps && ok; ++it) {
-                if (it + 1 < n_steps && !issue_s(it + 1)) { ok = false; break; }
-                const int s = it % AT_STAGES, b = it & 1;
-                if (!at_wait(at_smem(&p_full), (unsigned)it & 1u)) { ok = false; break; }
+                const int s = it % AT_STAGES, b = it % AT_BUFFERS;
+                if (!at_wait(at_smem(&v_full[s]), (unsigned)(it / AT_STAGES) & 1u)) { ok = false; break; }
+                if (!at_wait(at_smem(&p_full[b]), (unsigned)(it / AT_BUFFERS) & 1u)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const unsigned long long dps = dp + (unsigned long long)(b * (AT_P_BYTES >> 4)), dvs = dv + (unsigned long long)(s * (AT_STAGE_BYTES >> 4));
+                const unsigned long long dvs = dv + (unsigned long long)(s * (AT_STAGE_BYTES >> 4));
 #pragma unroll
-                for (int kk = 0; kk < 2 * AT_KTILE / 16; ++kk) {    // 16 keys: 32 bytes further in P's rows (64 keys a panel), 16 rows further in V
-                    const unsigned off_p = ((kk / 4) * (AT_QTILE * 128) + (kk % 4) * 32) >> 4, off_v = (kk * 16 * 128) >> 4;
-                    at_mma(tmem + AT_O_COL, dps + off_p, dvs + off_v, idesc_o, (it > 0 || kk > 0) ? 1u : 0u);
-                }
-                at_commit(at_smem(&kv_empty[s]));                   // the stage's keys and values have been read
+                for (int kk = 0; kk < 2 * AT_KTILE / 16; ++kk)      // 16 keys: 8 columns further in P, 16 rows further in V
+                    at_mma_ts(tmem + AT_O_COL, tmem + b * (2 * AT_KTILE) + kk * 8, dvs + ((kk * 16 * 128) >> 4), idesc_o, (it > 0 || kk > 0) ? 1u : 0u);
+                at_commit(at_smem(&v_empty[s]));                    // the stage's values have been read
                 at_commit(at_smem(&pv_done[b]));                    // and O holds this step's share
+                if (it + AT_AHEAD < n_steps && !issue_s(it + AT_AHEAD)) ok = false;
             }
             if (!ok) atomicExch(status, 5);
         }
     } else {                                                        // ---------------- softmax, warps 2..9
-        // Two threads a query row: thread (row, g) has the scores of the step's page g (64 keys) and half of the
-        // row of O.  The two tell each other their maxima, and at the end their sums, through shared memory.
         const int quarter = warp & 3;                               // the 32 lanes of tensor memory this warp may touch
-        const int g = (warp - 2) >> 2;
+        const int g = (warp - 2) >> 2;                              // the warpgroup: steps g, g + 2, ..
         const int r = quarter * 32 + lane;                          // this thread's query row
         const int p_r = pos0 + r;
         const unsigned lane_addr = tmem + ((unsigned)(quarter * 32) << 16);
-        const unsigned o_addr = lane_addr + AT_O_COL + g * (AT_HD / 2);
-        const unsigned pair = at_smem(&pair_bar[quarter]);
-        float m_run = -INFINITY, l_run = 0.f;
+        const int* table = p.block_table + (size_t)brow * p.table_stride;
         const float slope = p.slopes ? p.slopes[h] * p.inv_scale : 0.f;     // in units of the unscaled score
+        float m_mine = -INFINITY, l_mine = 0.f;                     // the reference point of this group's last step; its share of the row's sum
         bool ok = true;
-        int it = 0, met = 0;                                        // met: how often the row's two threads have met
-        // tell the other half `mine`, learn what it tells
-        auto swap = [&](float mine, float& theirs) -> bool {
-            float* slot = exchange + (met & 1) * (2 * AT_QTILE);
-            slot[g * AT_QTILE + r] = mine;
-            __syncwarp();
-            if (lane == 0) at_arrive(pair);
-            if (!at_wait_warp(pair, (unsigned)met & 1u)) return false;
-            theirs = slot[(g ^ 1) * AT_QTILE + r];
-            ++met;
-            return true;
-        };
-        for (; it < n_steps; ++it) {
-            const int b = it & 1, st = it % AT_STAGES;
-            if (!at_wait_warp(at_smem(&kv_full[st]), (unsigned)(it / AT_STAGES) & 1u)) { ok = false; break; }   // the loader's flags
-            const bool there = (stage_flags[st] >> g) & 1u;
-            if (!at_wait_warp(at_smem(&s_full[b]), (unsigned)(it >> 1) & 1u)) { ok = false; break; }
+        int entry[2];                                               // the page table's entries of the next step of this group
+#pragma unroll
+        for (int x = 0; x < 2; ++x) entry[x] = 2 * g + x < n_pages ? table[page_at(2 * g + x)] : -1;
+        for (int it = g; it < n_steps; it += 2) {
+            const int b = it % AT_BUFFERS;
+            const unsigned s_addr = lane_addr + b * (2 * AT_KTILE);
+            const bool there[2] = {entry[0] >= 0, entry[1] >= 0};   // (a page that is not there was read as zeros and is masked)
+#pragma unroll
+            for (int x = 0; x < 2; ++x) entry[x] = 2 * it + 4 + x < n_pages ? table[page_at(2 * it + 4 + x)] : -1;
+            if (!at_wait_warp(at_smem(&s_full[b]), (unsigned)(it / AT_BUFFERS) & 1u)) { ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int key0 = page_at(2 * it + g) * AT_KTILE;
-            unsigned raw[AT_KTILE];
-            at_ld32_start(lane_addr + b * (2 * AT_KTILE) + g * AT_KTILE, raw);
-            at_ld32_start(lane_addr + b * (2 * AT_KTILE) + g * AT_KTILE + 32, raw + 32);
+            unsigned raw[2 * AT_KTILE];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) at_ld32_start(s_addr + 32 * c, raw + 32 * c);
             at_ld_wait();
-            at_pin32(raw); at_pin32(raw + 32);
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) at_arrive(at_smem(&s_free[b]));          // the buffer may take S of the step after next
+#pragma unroll
+            for (int c = 0; c < 4; ++c) at_pin32(raw + 32 * c);
             // the row sees the keys up to its own position and inside its window
-            float s[AT_KTILE];
+            float s[2 * AT_KTILE], base[2] = {0.f, 0.f}, mx[8];
 #pragma unroll
-            for (int c = 0; c < AT_KTILE; ++c) s[c] = __uint_as_float(raw[c]);
-            const bool whole = there && key0 + AT_KTILE - 1 <= p_r &&
-                               (p.window <= 0 || key0 > p_r - p.window || key0 + AT_KTILE - 1 < p.keep_first);
-            if (!whole) {
+            for (int c = 0; c < 2 * AT_KTILE; ++c) s[c] = __uint_as_float(raw[c]);
 #pragma unroll
-                for (int c = 0; c < AT_KTILE; ++c) {
-                    const int key = key0 + c;
-                    if (!there || key > p_r || (p.window > 0 && key <= p_r - p.window && key >= p.keep_first)) s[c] = -INFINITY;
+            for (int x = 0; x < 2; ++x) {
+                const int key0 = page_at(2 * it + x) * AT_KTILE;
+                float* sx = s + x * AT_KTILE;
+                if (!(there[x] && key0 + AT_KTILE - 1 <= p_r && (p.window <= 0 || key0 > p_r - p.window || key0 + AT_KTILE - 1 < p.keep_first))) {
+#pragma unroll
+                    for (int c = 0; c < AT_KTILE; ++c) {
+                        const int key = key0 + c;
+                        if (!there[x] || key > p_r || (p.window > 0 && key <= p_r - p.window && key >= p.keep_first)) sx[c] = -INFINITY;
+                    }
                 }
-            }
-            // the distance's share of the score, slope * (key - row): the part that grows along the page is added here, the
-            // page's own part (`base`, one number a thread) joins the maximum and the exponent's offset
-            float base = 0.f;
-            if (p.slopes) {
-                base = slope * (float)(key0 - p_r);
+                // the distance's share of the score, slope * (key - row): the part that grows along the page is added here, the
+                // page's own part (`base`, one number a page) joins the maximum and the exponent's offset
+                if (p.slopes) {
+                    base[x] = slope * (float)(key0 - p_r);
 #pragma unroll
-                for (int c = 0; c < AT_KTILE; ++c) s[c] = fmaf(slope, (float)c, s[c]);
-            }
-            float mx[4] = {s[0], s[1], s[2], s[3]};                 // four chains: a warp has little else to hide their latency
+                    for (int c = 0; c < AT_KTILE; ++c) sx[c] = fmaf(slope, (float)c, sx[c]);
+                }
+                // four chains a page: a warp has little else to hide their latency
 #pragma unroll
-            for (int c = 4; c < AT_KTILE; ++c) mx[c & 3] = fmaxf(mx[c & 3], s[c]);
-            const float m_mine = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) + base;
-            float m_theirs;
-            if (!swap(m_mine, m_theirs)) { ok = false; break; }
+                for (int c = 0; c < 4; ++c) mx[4 * x + c] = fmaxf(fmaxf(sx[c], sx[c + 4]), sx[c + 8]);
+#pragma unroll
+                for (int c = 12; c < AT_KTILE - 4; c += 8) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) mx[4 * x + i] = fmaxf(fmaxf(mx[4 * x + i], sx[c + i]), sx[c + 4 + i]);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) mx[4 * x + i] = fmaxf(mx[4 * x + i], sx[AT_KTILE - 4 + i]);
+            }
+            const float m_step = fmaxf(fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) + base[0], fmaxf(fmaxf(mx[4], mx[5]), fmaxf(mx[6], mx[7])) + base[1]);
+            // the row's reference point up to the step before, from the other warpgroup
+            float m_run = -INFINITY;
+            if (it > 0) {
+                if (!at_wait_warp(at_smem(&told[4 * (g ^ 1) + quarter]), (unsigned)((it - 1) >> 1) & 1u)) { ok = false; break; }
+                m_run = refs[(g ^ 1) * AT_QTILE + r];
+            }
             // The reference point of the exponentials follows the row's maximum only when that has grown by more than
             // AT_LAZY (in powers of two): P then holds values up to 2^AT_LAZY, which bfloat16 and the float32 sums take
-            // as well as values up to 1, and O is rescaled on few steps instead of on nearly all.  Both threads of a
-            // row compute the same from the same numbers.
-            const float m_tile = fmaxf(m_mine, m_theirs) * p.scale_log2e;
+            // as well as values up to 1, and O is rescaled on few steps instead of on nearly all.
+            const float m_tile = m_step * p.scale_log2e;
             const float m_new = (m_run != -INFINITY && m_tile <= m_run + AT_LAZY) ? m_run : fmaxf(m_run, m_tile);
+            refs[g * AT_QTILE + r] = m_new;
+            __syncwarp();
+            if (lane == 0) at_arrive(at_smem(&told[4 * g + quarter]));
             const float m_use = m_new == -INFINITY ? 0.f : m_new;
-            const float alpha = m_run == -INFINITY ? 1.0f : at_exp2(m_run - m_use);
-            m_run = m_new;
+            const float alpha = m_run == -INFINITY ? 1.0f : at_exp2(m_run - m_use);          // for O
+            l_mine *= m_mine == -INFINITY ? 1.0f : at_exp2(m_mine - m_use);                  // (no sum yet: it is zero)
+            m_mine = m_new;
             float sum[4] = {0.f, 0.f, 0.f, 0.f};
-            unsigned packed[AT_KTILE / 2];
-            const float off = fmaf(base, p.scale_log2e, -m_use);
 #pragma unroll
-            for (int c = 0; c < AT_KTILE; c += 2) {
-                const float e0 = at_exp2(fmaf(s[c], p.scale_log2e, off)), e1 = at_exp2(fmaf(s[c + 1], p.scale_log2e, off));
-                sum[c & 3] += e0; sum[(c + 1) & 3] += e1;
-                packed[c >> 1] = at_pack(e0, e1);
+            for (int x = 0; x < 2; ++x) {
+                float packed[AT_KTILE / 2];
+                const float off = fmaf(base[x], p.scale_log2e, -m_use);
+#pragma unroll
+                for (int c = 0; c < AT_KTILE; c += 2) {
+                    const float e0 = at_exp2(fmaf(s[x * AT_KTILE + c], p.scale_log2e, off)), e1 = at_exp2(fmaf(s[x * AT_KTILE + c + 1], p.scale_log2e, off));
+                    sum[c & 3] += e0; sum[(c + 1) & 3] += e1;
+                    packed[c >> 1] = __uint_as_float(at_pack(e0, e1));
+                }
+                at_st32(s_addr + x * (AT_KTILE / 2), packed);       // P over the scores, two keys a column
             }
-            l_run = l_run * alpha + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
-            // this P tile is free once P.V of the step before last is done
-            if (it >= 2 && !at_wait_warp(at_smem(&pv_done[b]), (unsigned)((it >> 1) - 1) & 1u)) { ok = false; break; }
-            if (it > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) { // a row's reference point moved: rescale this half of the warp's rows of O
-                if (!at_wait_warp(at_smem(&pv_done[b ^ 1]), (unsigned)((it - 1) >> 1) & 1u)) { ok = false; break; }
+            l_mine += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+            if (it > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) { // a row's reference point moved: rescale the warp's rows of O
+                if (!at_wait_warp(at_smem(&pv_done[(it - 1) % AT_BUFFERS]), (unsigned)((it - 1) / AT_BUFFERS) & 1u)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
-                for (int c = 0; c < AT_HD / 2; c += 32) {
+                for (int c = 0; c < AT_HD; c += 32) {
                     float o[32];
-                    at_ld32(o_addr + c, o);
+                    at_ld32(lane_addr + AT_O_COL + c, o);
 #pragma unroll
                     for (int i = 0; i < 32; ++i) o[i] *= alpha;
-                    at_st32(o_addr + c, o);
+                    at_st32(lane_addr + AT_O_COL + c, o);
                 }
-                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             }
-            // P as bfloat16 for P.V: panel g of the tile (64 keys = 128 bytes a row)
-            unsigned char* p_row = at_mem + (p_s - q_s) + b * AT_P_BYTES + g * (AT_QTILE * 128) + r * 128;
-#pragma unroll
-            for (int c = 0; c < AT_KTILE / 8; ++c)
-                *reinterpret_cast<uint4*>(p_row + ((c ^ (r & 7)) << 4)) = make_uint4(packed[4 * c], packed[4 * c + 1], packed[4 * c + 2], packed[4 * c + 3]);
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // P is read by the tensor core's proxy
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) at_arrive(at_smem(&p_full));
+            if (lane == 0) at_arrive(at_smem(&p_full[b]));
         }
-        // the row's sum, and the last P.V (products complete in the order they were issued)
-        float l_theirs = 0.f;
-        if (ok && !swap(l_run, l_theirs)) ok = false;
-        if (ok && it > 0 && !at_wait_warp(at_smem(&pv_done[(it - 1) & 1]), (unsigned)((it - 1) >> 1) & 1u)) ok = false;
-        if (ok && it > 0) {
+        // the row's sum, in powers of two of the last step's reference point, and the last P.V (products complete in the order they were issued)
+        refs[g * AT_QTILE + r] = m_mine;                            // (what stands there already, or, for a group without a step, nothing)
+        sums[g * AT_QTILE + r] = l_mine;
+        __syncwarp();
+        if (lane == 0) at_arrive(at_smem(&met[quarter]));
+        const int last = n_steps - 1;
+        if (ok && !at_wait_warp(at_smem(&met[quarter]), 0u)) ok = false;
+        if (ok && !at_wait_warp(at_smem(&pv_done[last % AT_BUFFERS]), (unsigned)(last / AT_BUFFERS) & 1u)) ok = false;
+        if (ok) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            float l = g == 0 ? l_run + l_theirs : l_theirs + l_run;         // the same sum in both threads
+            const float m_run = refs[(last & 1) * AT_QTILE + r];
+            float l = 0.f;                                          // the same sum in both threads
+#pragma unroll
+            for (int w = 0; w < 2; ++w) {
+                const float m = refs[w * AT_QTILE + r];
+                if (m != -INFINITY) l = fmaf(sums[w * AT_QTILE + r], at_exp2(m - m_run), l);
+            }
             if (p.sinks) l += at_exp2(fmaf(p.sinks[h], 1.4426950408889634f, -m_run));   // (a row that saw no key: 2^inf, and 1 / l = 0)
             const float inv = l > 0.f ? 1.0f / l : 0.f;
+            const unsigned o_addr = lane_addr + AT_O_COL + g * (AT_HD / 2);
             bf16* o_row = p.out + ((size_t)(tok0 + r) * p.nh + h) * AT_HD + g * (AT_HD / 2);
 #pragma unroll 1
             for (int c = 0; c < AT_HD / 2; c += 32) {
