@@ -1,0 +1,61 @@
+// Pieces of float32 products over chunks of 64 tokens (state_space_tiles.cu, linear_attention_channels.cu): vector reads with a ragged end,
+// multiply-adds in pairs, slices of a chunk's rows turned in shared memory, and where a thread's results lie.
+#pragma once
+#include "common.cuh"
+
+#define ST_CHUNK 64                                       // tokens of a chunk
+#define ST_THREADS 128
+#define ST_SLICE 32                                       // state rows of C and S in shared memory at a time
+
+__device__ __forceinline__ float4 st_load4(const float* p, int left, bool vec) {          // up to four entries, zeros behind `left`
+    if (vec && left >= 4) return *reinterpret_cast<const float4*>(p);
+    return make_float4(left > 0 ? p[0] : 0.f, left > 1 ? p[1] : 0.f, left > 2 ? p[2] : 0.f, left > 3 ? p[3] : 0.f);
+}
+__device__ __forceinline__ void st_store4(float* p, int left, bool vec, float4 v) {
+    if (vec && left >= 4) { *reinterpret_cast<float4*>(p) = v; return; }
+    if (left > 0) p[0] = v.x;
+    if (left > 1) p[1] = v.y;
+    if (left > 2) p[2] = v.z;
+    if (left > 3) p[3] = v.w;
+}
+typedef unsigned long long st_pair;                        // two float32 numbers
+__device__ __forceinline__ void st_fma(st_pair& acc, float a, st_pair b) {
+    asm("{\n\t.reg .b64 aa;\n\tmov.b64 aa, {%1, %1};\n\tfma.rn.f32x2 %0, aa, %2, %0;\n\t}" : "+l"(acc) : "f"(a), "l"(b));
+}
+__device__ __forceinline__ float2 st_two(st_pair v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ float4 st_four(st_pair a, st_pair b) {
+    const float2 x = st_two(a), y = st_two(b);
+    return make_float4(x.x, x.y, y.x, y.y);
+}
+
+// Columns c0 .. c0 + 31 of 64 rows (tokens) into dst[column][token]; entry (column k, token t) lies at k * 64 + (t ^ 4 ((k / 4) % 8)), so
+// that neither the four stores of a thread nor the reads of four neighbouring tokens meet in a bank.
+__device__ __forceinline__ int st_turned(int k, int t) { return k * ST_CHUNK + (t ^ (((k >> 2) & 7) << 2)); }
+struct STSlice {
+    float4 v[ST_CHUNK * ST_SLICE / 4 / ST_THREADS];
+    __device__ __forceinline__ void load(const float* src, int ld, int n, int left, bool vec) {
+#pragma unroll
+        for (int e = 0; e < ST_CHUNK * ST_SLICE / 4 / ST_THREADS; ++e) {
+            const int i = threadIdx.x + e * ST_THREADS, t = i >> 3, c = (i & 7) * 4;
+            v[e] = t < n ? st_load4(src + (size_t)t * ld + c, left - c, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+    __device__ __forceinline__ void store_turned(float* dst) const {
+#pragma unroll
+        for (int e = 0; e < ST_CHUNK * ST_SLICE / 4 / ST_THREADS; ++e) {
+            const int i = threadIdx.x + e * ST_THREADS, t = i >> 3, c = (i & 7) * 4;
+            dst[st_turned(c, t)] = v[e].x; dst[st_turned(c + 1, t)] = v[e].y;
+            dst[st_turned(c + 2, t)] = v[e].z; dst[st_turned(c + 3, t)] = v[e].w;
+        }
+    }
+};
+// 8 x 16 threads over 64 x 64 results: a thread the rows ty * 4 + 32 i + 0..3 and columns tx * 4 + 0..3; a warp is four by eight threads.
+__device__ __forceinline__ void st_place(int& ty, int& tx) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    ty = (warp >> 1) * 4 + (lane >> 3);
+    tx = (warp & 1) * 8 + (lane & 7);
+}

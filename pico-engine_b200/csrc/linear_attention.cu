@@ -23,8 +23,8 @@
 //    S_end = diag(A) S_in + L with A the product of the chunk's decays and L the chunk's own contribution, so
 //    pass 1 computes (A, L) of every chunk from S_in = 0, pass 2 walks a sequence's chunks in order (an element
 //    a thread), leaves each chunk's S_in where its L was and stores the sequence's new state, and pass 3 runs
-//    every chunk again from its S_in and writes the outputs.  With a decay per head passes 1 and 3 are products of tiles
-//    (linear_attention_tiles.cu); with one per channel they walk a chunk's tokens.  Chunks never cross sequences: chunk c of the step
+//    every chunk again from its S_in and writes the outputs.  Passes 1 and 3 are products of tiles (a decay per head:
+//    linear_attention_tiles.cu, per channel: linear_attention_channels.cu).  Chunks never cross sequences: chunk c of the step
 //    is found from the rows' lengths on the device, so the grid depends on (T, B) only.
 #include "linear_attention.cuh"
 
@@ -40,10 +40,10 @@ __device__ __forceinline__ float la_channel_decay(float z, float inv_tau) {
     return expf(-sp * inv_tau);
 }
 
-// MODE 0: a sequence's tokens from its stored state; 1: a chunk from zero, leaving (A, L); 2: a chunk from its S_in.
+// A sequence's tokens one after the other, from its stored state.
 // NC: columns of the state a thread keeps (j and j + 32): with two, a block owns 64 columns, and every q, k and decay entry read
 // from shared memory meets two columns' multiply-adds.
-template <typename T, typename TQ, typename TZ, int R, int NC, bool PER_CHANNEL, int MODE>
+template <typename T, typename TQ, typename TZ, int R, int NC, bool PER_CHANNEL>
 __global__ void __launch_bounds__(LA_THREADS) la_walk_kernel(LAArgs a) {
     pdl_launch_dependents();
     pdl_wait();
@@ -55,34 +55,23 @@ __global__ void __launch_bounds__(LA_THREADS) la_walk_kernel(LAArgs a) {
     __shared__ __align__(16) float sa[PER_CHANNEL ? LA_GROUP : 1][PER_CHANNEL ? DP : 4];
     __shared__ float sv[LA_GROUP][COLS];
     __shared__ float part[LA_GROUP][LA_DS][COLS];
-    __shared__ int where[3];
 
     const int tid = threadIdx.x, jl = tid & (LA_COLS - 1), ds = tid / LA_COLS;
     const int h = blockIdx.y, j0 = blockIdx.z * COLS + jl;
     const int D = a.D, Dv = a.Dv, H = a.H;
-    int row, first, count;
-    if (MODE == 0) {
-        row = blockIdx.x; first = a.row_first[row]; count = a.row_lens[row];
-    } else {
-        if (tid == 0) { la_find_chunk(a.row_first, a.row_lens, a.B, blockIdx.x, row, first, count); where[0] = row; where[1] = first; where[2] = count; }
-        __syncthreads();
-        row = where[0]; first = where[1]; count = where[2];
-    }
+    const int row = blockIdx.x, first = a.row_first[row], count = a.row_lens[row];
     if (count <= 0) return;
     const int d0 = ds * R;
 
     float S[NC][R];
-    float* sp = nullptr;
-    if (MODE == 0) sp = a.state + (size_t)a.slots[row] * a.state_stride + (size_t)h * D * Dv;
-    if (MODE == 2) sp = a.chunk_state + ((size_t)blockIdx.x * H + h) * D * Dv;
+    float* sp = a.state + (size_t)a.slots[row] * a.state_stride + (size_t)h * D * Dv;
 #pragma unroll
     for (int c = 0; c < NC; ++c)
 #pragma unroll
         for (int r = 0; r < R; ++r)
-            S[c][r] = (MODE != 1 && j0 + c * LA_COLS < Dv && d0 + r < D) ? sp[(size_t)(d0 + r) * Dv + j0 + c * LA_COLS] : 0.f;
+            S[c][r] = (j0 + c * LA_COLS < Dv && d0 + r < D) ? sp[(size_t)(d0 + r) * Dv + j0 + c * LA_COLS] : 0.f;
 
     const float hd = PER_CHANNEL ? 0.f : a.head_decay[h];
-    float A = 1.f;                                       // MODE 1: the product of this chunk's decays on channel tid
     const T* proj = (const T*)a.proj;
     const TQ* qk = (const TQ*)a.qk;
     const TZ* zp = (const TZ*)a.z;
@@ -127,9 +116,6 @@ __global__ void __launch_bounds__(LA_THREADS) la_walk_kernel(LAArgs a) {
         }
         __syncthreads();
         if (g0 + LA_GROUP < count) fetch(g0 + LA_GROUP);
-        if (MODE == 1 && tid < D) {
-            for (int tb = 0; tb < ng; ++tb) { if constexpr (PER_CHANNEL) A *= sa[tb][tid]; else A *= hd; }
-        }
         auto token = [&](const int tb) {
             float v[NC], acc[NC][2];
 #pragma unroll
@@ -146,16 +132,13 @@ __global__ void __launch_bounds__(LA_THREADS) la_walk_kernel(LAArgs a) {
                     S[c][r + 1] = fmaf(a4.y, S[c][r + 1], k4.y * v[c]);
                     S[c][r + 2] = fmaf(a4.z, S[c][r + 2], k4.z * v[c]);
                     S[c][r + 3] = fmaf(a4.w, S[c][r + 3], k4.w * v[c]);
-                    if (MODE != 1) {                     // two chains a column, so that no sum waits long for the one before it
-                        acc[c][0] = fmaf(S[c][r + 0], q4.x, acc[c][0]); acc[c][1] = fmaf(S[c][r + 1], q4.y, acc[c][1]);
-                        acc[c][0] = fmaf(S[c][r + 2], q4.z, acc[c][0]); acc[c][1] = fmaf(S[c][r + 3], q4.w, acc[c][1]);
-                    }
+                    // two chains a column, so that no sum waits long for the one before it
+                    acc[c][0] = fmaf(S[c][r + 0], q4.x, acc[c][0]); acc[c][1] = fmaf(S[c][r + 1], q4.y, acc[c][1]);
+                    acc[c][0] = fmaf(S[c][r + 2], q4.z, acc[c][0]); acc[c][1] = fmaf(S[c][r + 3], q4.w, acc[c][1]);
                 }
             }
-            if (MODE != 1) {
 #pragma unroll
-                for (int c = 0; c < NC; ++c) part[tb][ds][c * LA_COLS + jl] = acc[c][0] + acc[c][1];
-            }
+            for (int c = 0; c < NC; ++c) part[tb][ds][c * LA_COLS + jl] = acc[c][0] + acc[c][1];
         };
         if (ng == LA_GROUP) {                            // a full group: constant addresses, no loop
 #pragma unroll
@@ -163,29 +146,23 @@ __global__ void __launch_bounds__(LA_THREADS) la_walk_kernel(LAArgs a) {
         } else {
             for (int tb = 0; tb < ng; ++tb) token(tb);
         }
-        if (MODE != 1) {
-            __syncthreads();
+        __syncthreads();
 #pragma unroll
-            for (int c = 0; c < NC; ++c) {               // LA_GROUP * COLS outputs a group, LA_THREADS a turn
-                const int i = tid + c * LA_THREADS, tb = i / COLS, col = blockIdx.z * COLS + i % COLS;
-                if (tb < ng && col < Dv) {
-                    float o = 0.f;
+        for (int c = 0; c < NC; ++c) {                   // LA_GROUP * COLS outputs a group, LA_THREADS a turn
+            const int i = tid + c * LA_THREADS, tb = i / COLS, col = blockIdx.z * COLS + i % COLS;
+            if (tb < ng && col < Dv) {
+                float o = 0.f;
 #pragma unroll
-                    for (int s = 0; s < LA_DS; ++s) o += part[tb][s][i % COLS];
-                    a.out[(size_t)(first + g0 + tb) * ((size_t)H * Dv) + (size_t)h * Dv + col] = o;
-                }
+                for (int s = 0; s < LA_DS; ++s) o += part[tb][s][i % COLS];
+                a.out[(size_t)(first + g0 + tb) * ((size_t)H * Dv) + (size_t)h * Dv + col] = o;
             }
         }
     }
-    if (MODE == 0 || MODE == 1) {
-        float* dst = MODE == 0 ? sp : a.chunk_state + ((size_t)blockIdx.x * H + h) * D * Dv;
 #pragma unroll
-        for (int c = 0; c < NC; ++c)
+    for (int c = 0; c < NC; ++c)
 #pragma unroll
-            for (int r = 0; r < R; ++r)
-                if (j0 + c * LA_COLS < Dv && d0 + r < D) dst[(size_t)(d0 + r) * Dv + j0 + c * LA_COLS] = S[c][r];
-        if (MODE == 1 && blockIdx.z == 0 && tid < D) a.chunk_decay[((size_t)blockIdx.x * H + h) * D + tid] = A;
-    }
+        for (int r = 0; r < R; ++r)
+            if (j0 + c * LA_COLS < Dv && d0 + r < D) sp[(size_t)(d0 + r) * Dv + j0 + c * LA_COLS] = S[c][r];
 }
 
 // Pass 2: an element of a sequence's state a thread; the sequence's chunks in order.
@@ -228,7 +205,7 @@ template <typename T, typename TQ, typename TZ, int R, int NC, bool PC>
 static int la_run(const LAArgs& a, int chunked, cudaStream_t s) {
     const int tiles = (a.Dv + LA_COLS * NC - 1) / (LA_COLS * NC);
     if (!chunked) {
-        PE_TRY(pe_launch(la_walk_kernel<T, TQ, TZ, R, NC, PC, 0>, dim3(a.B, a.H, tiles), LA_THREADS, 0, s, a));
+        PE_TRY(pe_launch(la_walk_kernel<T, TQ, TZ, R, NC, PC>, dim3(a.B, a.H, tiles), LA_THREADS, 0, s, a));
         PE_LAUNCH_CHECK();
         return 0;
     }
@@ -241,13 +218,10 @@ static int la_run(const LAArgs& a, int chunked, cudaStream_t s) {
         PE_LAUNCH_CHECK();
         return la_tiles_outputs(a, types, s);
     } else {
-        PE_TRY(pe_launch(la_walk_kernel<T, TQ, TZ, R, NC, PC, 1>, dim3(a.max_chunks, a.H, tiles), LA_THREADS, 0, s, a));
-        PE_LAUNCH_CHECK();
+        if (const int e = la_channels_contributions(a, sizeof(T) == 4, a.channel_scratch, s)) return e;
         PE_TRY(pe_launch(la_carry_kernel, carry, 256, 0, s, a));
         PE_LAUNCH_CHECK();
-        PE_TRY(pe_launch(la_walk_kernel<T, TQ, TZ, R, NC, PC, 2>, dim3(a.max_chunks, a.H, tiles), LA_THREADS, 0, s, a));
-        PE_LAUNCH_CHECK();
-        return 0;
+        return la_channels_outputs(a, sizeof(T) == 4, a.channel_scratch, s);
     }
 }
 
@@ -265,8 +239,8 @@ static int la_by_rows(const LAArgs& a, int chunked, cudaStream_t s) {
 extern "C" int pe_linear_attention_chunks(int T, int B) { return (T + LA_CHUNK - 1) / LA_CHUNK + B; }
 
 // Floats of scratch the chunked way needs.
-extern "C" long long pe_linear_attention_scratch_floats(int T, int B, int H, int D, int Dv) {
-    return (long long)pe_linear_attention_chunks(T, B) * H * D * ((long long)Dv + 1);
+extern "C" long long pe_linear_attention_scratch_floats(int T, int B, int H, int D, int Dv, int per_channel) {
+    return (long long)pe_linear_attention_chunks(T, B) * H * D * ((long long)Dv + 1) + (per_channel ? 3 + la_channels_scratch_floats(pe_linear_attention_chunks(T, B), H, D) : 0);
 }
 
 extern "C" int pe_linear_attention(const void* proj, int dtype, int ld, int q_off, int k_off, int v_off, const void* z, int z_dtype,
@@ -287,6 +261,7 @@ extern "C" int pe_linear_attention(const void* proj, int dtype, int ld, int q_of
     a.max_chunks = pe_linear_attention_chunks(T, B);
     a.chunk_state = scratch;
     a.chunk_decay = scratch ? scratch + (size_t)a.max_chunks * H * D * Dv : nullptr;
+    a.channel_scratch = scratch ? scratch + ((size_t)a.max_chunks * H * D * ((size_t)Dv + 1) + 3) / 4 * 4 : nullptr;      // (read in vectors)
     cudaStream_t s = (cudaStream_t)stream;
     const bool pc = z != nullptr;
     if (dtype == PE_F32) {

@@ -19,6 +19,7 @@ struct LAArgs {
     float* chunk_state;      // [chunks, H, D, Dv]
     float* chunk_decay;      // [chunks, H, D]
     int max_chunks;
+    float* channel_scratch;  // with a decay per channel: weights, decayed queries and keys of every chunk
 };
 
 // silu of a projection.  FAST (the bfloat16 engine, whose projections carry 8 bits): 2^x and the reciprocal from the
@@ -57,3 +58,7 @@ __device__ __forceinline__ void la_find_chunk(const int* row_first, const int* r
 // 2 bfloat16 rows with float32 queries and keys of their own.
 int la_tiles_contributions(const LAArgs& a, int types, cudaStream_t s);
 int la_tiles_outputs(const LAArgs& a, int types, cudaStream_t s);
+// The same with a decay per channel (linear_attention_channels.cu).
+long long la_channels_scratch_floats(int chunks, int H, int D);
+int la_channels_contributions(const LAArgs& a, bool f32, float* scratch, cudaStream_t s);
+int la_channels_outputs(const LAArgs& a, bool f32, float* scratch, cudaStream_t s);

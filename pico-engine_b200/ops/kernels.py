@@ -1083,13 +1083,13 @@ def linear_attention(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, n_h
     ws = None
     if chunked:
         from .workspace import scratch
-        ws = scratch("linear_attention", 4 * lib.pe_linear_attention_scratch_floats(T, B, H, D, Dv), proj.device).data_ptr()
+        ws = scratch("linear_attention", 4 * lib.pe_linear_attention_scratch_floats(T, B, H, D, Dv, 0 if decay_logits is None else 1), proj.device).data_ptr()
     check(lib.pe_linear_attention(proj.data_ptr(), _code(proj, "proj"), ld, q_off, k_off, v_off, _ptr(decay_logits),
                                   0 if decay_logits is None else _code(decay_logits, "decay_logits"), H * D, _ptr(head_decay),
                                   float(inv_tau), float(q_scale), LA_ACTIVATIONS[qk_activation], LA_ACTIVATIONS[v_activation],
                                   sp, stride, row_first.data_ptr(), row_lens.data_ptr(), slots.data_ptr(), out.data_ptr(),
                                   T, B, H, D, Dv, 1 if chunked else 0, ws, _ptr(qk), qk_ld, stream_ptr()),
-          "linear_attention", 3 if chunked else 1)
+          "linear_attention", (3 if decay_logits is None else 4) if chunked else 1)
     return out
 
 

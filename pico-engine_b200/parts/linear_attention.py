@@ -111,15 +111,11 @@ class LinearAttention(Mixer, SharedProducts):
     def mixed_rows(self, proj, col, turned, ctx, cache_entry, owns_cache, logits=None):
         s = self.spec
         qk, vo = self._sizes()
-        # With a decay per head, prompts run as products of tiles over chunks of 64 tokens; rows that bring a few tokens walk them.
-        # With a decay per channel a chunk is walked twice, which pays only where the walk would leave the GPU empty: token after token
-        # is a block a (sequence, head, 32 columns of the state).  Measured on a B200 (16 heads of 128 x 128): one prompt of 2,048
-        # tokens 319 us in chunks against 709 us, four such prompts 1,985 us against 1,062 us.  (Every way gives the same numbers up to
-        # float32 rounding; rows that bring a few tokens, such as the idle rows of a padded step, do not count.)
-        if self.head_decay is not None:
-            chunked = any(n > 16 for n in ctx.lens)
-        else:
-            chunked = 0 < sum(1 for n in ctx.lens if n > 64) * s.n_heads * ((s.v_head_dim + 31) // 32) < 192
+        # Prompts run as products of tiles over chunks of 64 tokens; rows that bring a few tokens walk them.  (Either way gives the same
+        # numbers up to float32 rounding.)  A walk takes as long as the longest row
+        # whatever it leaves idle (2,048 tokens of 16 heads of 128 x 128 on a B200: 709 us against 180 us, four such prompts 1,062 us against
+        # 650); a chunk costs its tiles even where it holds a few tokens.
+        chunked = any(n > 16 for n in ctx.lens)
         # (keys that are scaled but not turned: the scale moves to the queries, the output being linear in either)
         q_scale = s.q_scale if turned is not None else s.q_scale * s.k_scale
         first = 0 if turned is not None else col

@@ -247,6 +247,28 @@ def test_recurrence_kernel_decay_per_channel(H, D, Dv, tau):
         assert (s.double() - want_s).abs().max() < 2e-4 * max(1.0, float(want_s.abs().max()))
 
 
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("H,D,Dv,tau", [(2, 10, 6, 1.0), (1, 37, 70, 16.0), (2, 128, 128, 16.0), (1, 256, 66, 4.0), (3, 64, 64, 0.5)])
+def test_tiles_with_a_decay_per_channel(dtype, H, D, Dv, tau):
+    """Chunks and runs of 16 tokens that end on, before and behind their borders, channels that fill no vector and more than one tile,
+    and decays from nothing to one: the products of decays are formed forwards and lose no digits."""
+    dt = DTYPES[dtype]
+    g = torch.Generator().manual_seed(D)
+    lens = [1, 15, 16, 17, 64, 65, 130]
+    T = sum(lens)
+    q, k, v = ((torch.randn(T, H, d, generator=g)).to(dt).float() for d in (D, D, Dv))
+    z = 6.0 * torch.randn(T, H, D, generator=g) + 2.0
+    z[::7] = -60.0
+    z[3::11] = 60.0
+    alpha = plain.sigmoid(z.double()) ** (1.0 / tau)
+    want_o, want_s = plain_recurrence(q.double() * 0.25, k.double(), v.double(), lens, alpha)
+    for cuts in ((1.0,), (0.5, 1.0)):
+        o, s = run_recurrence(q, k, v, dt, lens, logits=z, tau=tau, q_scale=0.25, act="none", cuts=cuts, chunked=True)
+        # float32 sums of at most 130 + 256 products whose inputs are exact in either dtype, decays good to a few 2^-24
+        assert (o.double() - want_o).abs().max() < 2e-5 * max(1.0, float(want_o.abs().max())), cuts
+        assert (s.double() - want_s).abs().max() < 2e-5 * max(1.0, float(want_s.abs().max())), cuts
+
+
 @pytest.mark.parametrize("far", [0, 1, 63, 64, 65, 447])
 def test_recurrence_keeps_a_key_from_far_back(far):
     """With decay 1 one key that matches the last query and carries a value nobody else has must come through whole
