@@ -75,9 +75,11 @@ __device__ __forceinline__ bool ad_bar_wait(unsigned bar, unsigned parity) {
     if (ad_bar_test(bar, parity)) return true;               // the usual case costs one test
     const long long deadline = clock64() + AD_WAIT_CYCLES;
     for (;;) {
-        if (ad_bar_test(bar, parity)) return true;
+        unsigned done;
+        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                     : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+        if (done) return true;
         if (clock64() > deadline) return false;
-        __nanosleep(32);
     }
 }
 __device__ __forceinline__ void ad_cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }

@@ -80,14 +80,16 @@ __device__ __forceinline__ void lf_bulk_copy(unsigned dst, const void* src, unsi
 }
 // true when the phase with this parity has completed; false when the wait ran out
 __device__ __forceinline__ bool lf_bar_wait(unsigned bar, unsigned parity) {
+    unsigned done;
+    asm volatile("{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    if (done) return true;                                   // the usual case costs neither a clock read nor a suspended wait
     const long long deadline = clock64() + LF_WAIT_CYCLES;
     for (;;) {
-        unsigned done;
-        asm volatile("{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
                      : "=r"(done) : "r"(bar), "r"(parity) : "memory");
         if (done) return true;
         if (clock64() > deadline) return false;
-        __nanosleep(40);
     }
 }
 __device__ __forceinline__ void lf_cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
@@ -231,6 +233,14 @@ __global__ void __launch_bounds__(32 * LF_WARPS, LF_MIN_CTAS(NT, RT, EPI)) linea
 
     pdl_launch_dependents();
     for (int c = 0; c < n_chunks && c < stages; ++c) issue(c);      // W first: no kernel writes it, so it need not wait
+    // The norm's weights too, into L1: a step streams more weights than L2 holds, so that they come from DRAM, and behind the wait
+    // they would be as long on their way as everything else the kernel does there (clock stamps: 1.9 us from the wait to the first product;
+    // with this and waits that are not slept over, a step of 24 layers of the Qwen2.5-0.5B widths 724 -> 706 us at 8 rows).
+    if (PRO == LF_RMSNORM) {
+        const unsigned bytes = (unsigned)p.K * (p.norm_w_dtype == PE_BF16 ? 2u : 4u);
+        for (unsigned o = threadIdx.x * 128u; o < bytes; o += 32u * LF_WARPS * 128u)
+            asm volatile("prefetch.global.L1 [%0];" ::"l"((const char*)p.norm_w + o) : "memory");
+    }
     // ROPE: what the epilogue needs of the step's description (positions, pages) and of the rotation tables is
     // asked for now: none of it is written by a kernel of the step, and the epilogue then waits for no load.
     int ep_pos = 0, ep_page = -1;
