@@ -3,7 +3,7 @@
 //   per head:   S_t = diag(a_t) S_(t-1) + k_t v_t^T        o_t = S_t^T q_t        S [D, Dv], float32
 //
 // a_t is either one constant per head (`head_decay` [H]) or one number per key channel and token,
-// a = sigmoid(z)^(inv_tau) = exp(-softplus(-z) * inv_tau) from float32 logits `z` [T, H*D].  q, k and v are columns of
+// a = sigmoid(z)^(inv_tau) = exp(-softplus(-z) * inv_tau), worked out in float32, from logits `z` [T, H*D] of either dtype.  q, k and v are columns of
 // `proj` [T, ld] (heads side by side, q_off / k_off / v_off the first column of each), or, where q and k were worked on in
 // between and are float32 (`qk` [T, qk_ld]), q and k of those rows; an activation (0: none,
 // 1: silu) is applied to q and k and to v while they are loaded, and q is multiplied by `q_scale`.  Everything
@@ -218,7 +218,7 @@ static int la_run(const LAArgs& a, int chunked, cudaStream_t s) {
         PE_LAUNCH_CHECK();
         return la_tiles_outputs(a, types, s);
     } else {
-        if (const int e = la_channels_contributions(a, sizeof(T) == 4, a.channel_scratch, s)) return e;
+        if (const int e = la_channels_contributions(a, sizeof(T) == 4, sizeof(TZ) == 4, a.channel_scratch, s)) return e;
         PE_TRY(pe_launch(la_carry_kernel, carry, 256, 0, s, a));
         PE_LAUNCH_CHECK();
         return la_channels_outputs(a, sizeof(T) == 4, a.channel_scratch, s);
@@ -272,6 +272,7 @@ extern "C" int pe_linear_attention(const void* proj, int dtype, int ld, int q_of
     if (dtype == PE_BF16) {
         if (!pc) return qk ? la_by_rows<bf16, float, float, false>(a, chunked, s) : la_by_rows<bf16, bf16, bf16, false>(a, chunked, s);
         if (z_dtype == PE_F32 && !qk) return la_by_rows<bf16, bf16, float, true>(a, chunked, s);
+        if (z_dtype == PE_BF16 && !qk) return la_by_rows<bf16, bf16, bf16, true>(a, chunked, s);
     }
     return PE_ERR_UNSUPPORTED;
 }

@@ -60,5 +60,5 @@ int la_tiles_contributions(const LAArgs& a, int types, cudaStream_t s);
 int la_tiles_outputs(const LAArgs& a, int types, cudaStream_t s);
 // The same with a decay per channel (linear_attention_channels.cu).
 long long la_channels_scratch_floats(int chunks, int H, int D);
-int la_channels_contributions(const LAArgs& a, bool f32, float* scratch, cudaStream_t s);
+int la_channels_contributions(const LAArgs& a, bool f32, bool z_f32, float* scratch, cudaStream_t s);
 int la_channels_outputs(const LAArgs& a, bool f32, float* scratch, cudaStream_t s);

@@ -36,8 +36,17 @@ __device__ __forceinline__ float4 lc_load4(const T* p, int left, bool vec) {    
     }
 }
 
+__device__ __forceinline__ void lc_read16(float (&v)[LC_RUN], const float* p) {
+#pragma unroll
+    for (int t = 0; t < LC_RUN; t += 4) *reinterpret_cast<float4*>(v + t) = *reinterpret_cast<const float4*>(p + t);
+}
+__device__ __forceinline__ void lc_write16(float* p, const float (&v)[LC_RUN]) {
+#pragma unroll
+    for (int t = 0; t < LC_RUN; t += 4) *reinterpret_cast<float4*>(p + t) = *reinterpret_cast<const float4*>(v + t);
+}
+
 // A chunk and head: weights [64 s][64 t], decayed queries and keys [64][D], and the product of the chunk's decays.
-template <typename T>
+template <typename T, typename TZ>
 __global__ void __launch_bounds__(LC_THREADS) lc_prepare_kernel(LAArgs a, float* weights, float* queries, float* keys, int vec_q, int vec_z) {
     pdl_launch_dependents();
     pdl_wait();
@@ -60,7 +69,7 @@ __global__ void __launch_bounds__(LC_THREADS) lc_prepare_kernel(LAArgs a, float*
             const T* p = (const T*)a.qk + (size_t)(first + t) * a.qk_ld + h * D + d;
             q = lc_load4(p + a.q_off, D - d, vec_q);
             k = lc_load4(p + a.k_off, D - d, vec_q);
-            z = st_load4((const float*)a.z + (size_t)(first + t) * a.z_ld + h * D + d, D - d, vec_z);
+            z = lc_load4((const TZ*)a.z + (size_t)(first + t) * a.z_ld + h * D + d, D - d, vec_z);
             q = make_float4(la_act<FAST>(q.x, a.act_qk) * a.q_scale, la_act<FAST>(q.y, a.act_qk) * a.q_scale, la_act<FAST>(q.z, a.act_qk) * a.q_scale, la_act<FAST>(q.w, a.act_qk) * a.q_scale);
             k = make_float4(la_act<FAST>(k.x, a.act_qk), la_act<FAST>(k.y, a.act_qk), la_act<FAST>(k.z, a.act_qk), la_act<FAST>(k.w, a.act_qk));
             z = make_float4(lc_decay(z.x, a.inv_tau), lc_decay(z.y, a.inv_tau), lc_decay(z.z, a.inv_tau), lc_decay(z.w, a.inv_tau));
@@ -113,9 +122,9 @@ __global__ void __launch_bounds__(LC_THREADS) lc_prepare_kernel(LAArgs a, float*
     // queries times what leads to them in their run, keys times what follows them there; thread (channel, run)
     for (int i = tid; i < 4 * DP; i += LC_THREADS) {
         const int d = i % DP, run = i / DP;
-        float* q = qt + d * LC_LD + run * LC_RUN;
-        float* k = kt + d * LC_LD + run * LC_RUN;
-        const float* c = at + d * LC_LD + run * LC_RUN;
+        const int at_run = d * LC_LD + run * LC_RUN;
+        float q[LC_RUN], k[LC_RUN], c[LC_RUN];
+        lc_read16(q, qt + at_run); lc_read16(k, kt + at_run); lc_read16(c, at + at_run);
         float x = 1.f;
 #pragma unroll
         for (int t = 0; t < LC_RUN; ++t) { x *= c[t]; q[t] *= x; }
@@ -123,6 +132,7 @@ __global__ void __launch_bounds__(LC_THREADS) lc_prepare_kernel(LAArgs a, float*
         x = 1.f;
 #pragma unroll
         for (int t = LC_RUN - 1; t >= 0; --t) { k[t] *= x; x *= c[t]; }
+        lc_write16(qt + at_run, q); lc_write16(kt + at_run, k);
     }
     __syncthreads();
     // between runs j < i: 16 threads of 4 x 4 weights for each of the six pairs, two of them sharing the channels
@@ -156,23 +166,19 @@ __global__ void __launch_bounds__(LC_THREADS) lc_prepare_kernel(LAArgs a, float*
     // queries times all decays from the chunk's start, keys times all to its end, channels side by side
     float* q_out = queries + ((size_t)blockIdx.x * a.H + h) * ST_CHUNK * D;
     float* k_out = keys + ((size_t)blockIdx.x * a.H + h) * ST_CHUNK * D;
+    const int r = tid / 64;                               // four groups of threads, a run each
     for (int d = tid % 64; d < D; d += 64) {
-        float lead[4], follow[4];
-        lead[0] = 1.f; follow[3] = 1.f;
+        float lead = 1.f, follow = 1.f;
+        for (int x = 0; x < r; ++x) lead *= whole[x * DP + d];
+        for (int x = 3; x > r; --x) follow *= whole[x * DP + d];
+        float q[LC_RUN], k[LC_RUN];
+        lc_read16(q, qt + d * LC_LD + r * LC_RUN); lc_read16(k, kt + d * LC_LD + r * LC_RUN);
 #pragma unroll
-        for (int r = 1; r < 4; ++r) { lead[r] = lead[r - 1] * whole[(r - 1) * DP + d]; }
-#pragma unroll
-        for (int r = 2; r >= 0; --r) follow[r] = follow[r + 1] * whole[(r + 1) * DP + d];
-        const int r = tid / 64;                           // four groups of threads, a run each
-#pragma unroll 4
-        for (int t = r * LC_RUN; t < (r + 1) * LC_RUN; ++t) {
-            float l = lead[0], f = follow[0];
-#pragma unroll
-            for (int x = 1; x < 4; ++x) if (r == x) { l = lead[x]; f = follow[x]; }
-            q_out[(size_t)t * D + d] = qt[d * LC_LD + t] * l;
-            k_out[(size_t)t * D + d] = kt[d * LC_LD + t] * f;
+        for (int t = 0; t < LC_RUN; ++t) {
+            q_out[(size_t)(r * LC_RUN + t) * D + d] = q[t] * lead;
+            k_out[(size_t)(r * LC_RUN + t) * D + d] = k[t] * follow;
         }
-        if (r == 0) a.chunk_decay[((size_t)blockIdx.x * a.H + h) * D + d] = follow[0] * whole[d];
+        if (r == 0) a.chunk_decay[((size_t)blockIdx.x * a.H + h) * D + d] = follow * whole[d];
     }
 }
 
@@ -328,18 +334,18 @@ __global__ void __launch_bounds__(ST_THREADS) lc_output_kernel(LAArgs a, const f
 
 long long la_channels_scratch_floats(int chunks, int H, int D) { return (long long)chunks * H * (ST_CHUNK * ST_CHUNK + 2ll * ST_CHUNK * D); }
 
-template <typename T>
+template <typename T, typename TZ>
 static int lc_prepare_and_contribute(const LAArgs& a, float* scratch, cudaStream_t s) {
     float* weights = scratch;
     float* queries = weights + (size_t)a.max_chunks * a.H * ST_CHUNK * ST_CHUNK;
     float* keys = queries + (size_t)a.max_chunks * a.H * ST_CHUNK * a.D;
     const int DP = (a.D + 3) / 4 * 4, size = sizeof(T);
     const int vec_q = (uintptr_t)a.qk % (4 * size) == 0 && a.qk_ld % 4 == 0 && a.q_off % 4 == 0 && a.k_off % 4 == 0 && a.D % 4 == 0;
-    const int vec_z = (uintptr_t)a.z % 16 == 0 && a.z_ld % 4 == 0 && a.D % 4 == 0;
+    const int vec_z = (uintptr_t)a.z % (4 * sizeof(TZ)) == 0 && a.z_ld % 4 == 0 && a.D % 4 == 0;
     const int vec_v = (uintptr_t)a.proj % (4 * size) == 0 && a.ld % 4 == 0 && a.v_off % 4 == 0 && a.Dv % 4 == 0;
     const size_t smem = sizeof(float) * ((size_t)3 * DP * LC_LD + 4 * DP);
-    PE_TRY(cudaFuncSetAttribute(lc_prepare_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    PE_TRY(pe_launch(lc_prepare_kernel<T>, dim3(a.max_chunks, a.H), LC_THREADS, smem, s, a, weights, queries, keys, vec_q, vec_z));
+    PE_TRY(cudaFuncSetAttribute(lc_prepare_kernel<T, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PE_TRY(pe_launch(lc_prepare_kernel<T, TZ>, dim3(a.max_chunks, a.H), LC_THREADS, smem, s, a, weights, queries, keys, vec_q, vec_z));
     PE_LAUNCH_CHECK();
     const int td = (a.D + 127) / 128, tv = (a.Dv + 63) / 64;
     PE_TRY(pe_launch(lc_contribution_kernel<T>, dim3(a.max_chunks, a.H, td * tv), ST_THREADS, 0, s, a, (const float*)keys, vec_v, td));
@@ -355,8 +361,9 @@ static int lc_outputs(const LAArgs& a, float* scratch, cudaStream_t s) {
     return 0;
 }
 
-int la_channels_contributions(const LAArgs& a, bool f32, float* scratch, cudaStream_t s) {
+int la_channels_contributions(const LAArgs& a, bool f32, bool z_f32, float* scratch, cudaStream_t s) {
     if (a.D > 256 || a.H > 65535) return PE_ERR_UNSUPPORTED;
-    return f32 ? lc_prepare_and_contribute<float>(a, scratch, s) : lc_prepare_and_contribute<bf16>(a, scratch, s);
+    if (f32) return lc_prepare_and_contribute<float, float>(a, scratch, s);
+    return z_f32 ? lc_prepare_and_contribute<bf16, float>(a, scratch, s) : lc_prepare_and_contribute<bf16, bf16>(a, scratch, s);
 }
 int la_channels_outputs(const LAArgs& a, bool f32, float* scratch, cudaStream_t s) { return f32 ? lc_outputs<float>(a, scratch, s) : lc_outputs<bf16>(a, scratch, s); }

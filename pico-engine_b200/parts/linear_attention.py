@@ -100,7 +100,11 @@ class LinearAttention(Mixer, SharedProducts):
         if self.w_a1 is not None:
             if rows[0] is None and not kernels.fused_takes(proj.shape[0], self.w_a1, rows[1]):
                 rows = (x_norm[1].forward(x_norm[0], ctx.dtype), None, None, 0.0)
-            logits = linear(first_product(*rows, self.w_a1, ctx), self.w_a2, self.b_a2, out_dtype=torch.float32)
+            # The decode product and the library's product without a bias give their float32 sums; the library's with a bias comes rounded
+            # to the rows' dtype, and is read as it is.
+            a1 = first_product(*rows, self.w_a1, ctx)
+            rounded = self.b_a2 is not None and not kernels.fused_takes(a1.shape[0], self.w_a2, a1)
+            logits = linear(a1, self.w_a2, self.b_a2, out_dtype=None if rounded else torch.float32)
         turned = None
         if s.position is not None:
             turned = kernels.heads_prepare(proj, ctx.tok_pos, ctx.tok_row, turned=self.prepare_jobs(proj, 0, ctx, cache_entry, False)[1])

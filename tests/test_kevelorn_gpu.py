@@ -269,6 +269,26 @@ def test_tiles_with_a_decay_per_channel(dtype, H, D, Dv, tau):
         assert (s.double() - want_s).abs().max() < 2e-5 * max(1.0, float(want_s.abs().max())), cuts
 
 
+@pytest.mark.parametrize("chunked", [False, True])
+@pytest.mark.parametrize("D,pad", [(128, 0), (20, 2), (7, 0)])              # rows that do and do not allow vector reads
+def test_decay_logits_of_the_rows_dtype(chunked, D, pad):
+    """Logits in bfloat16 are the same numbers as those logits in float32, bit for bit, in the walk and in the tiles."""
+    from pico_engine.ops import kernels
+    H, Dv, lens = 3, 24, [1, 65, 17]
+    T = sum(lens)
+    g = torch.Generator().manual_seed(D)
+    proj = torch.randn(T, 2 * H * D + H * Dv, generator=g).bfloat16().cuda()
+    z = torch.empty(T * H * D + pad, dtype=torch.bfloat16, device="cuda")[pad:].view(T, H * D).copy_(4 * torch.randn(T, H * D, generator=g))
+    first = torch.tensor([0, 1, 66, 83], dtype=torch.int32, device="cuda")
+    rows, slots = torch.tensor(lens, dtype=torch.int32, device="cuda"), torch.arange(3, dtype=torch.int32, device="cuda")
+    got = []
+    for logits in (z, z.float()):
+        state = torch.ones(3, H * D * Dv, device="cuda")
+        got.append((kernels.linear_attention(proj, 0, H * D, 2 * H * D, H, D, Dv, state, 0, first, rows, slots, chunked,
+                                             decay_logits=logits, inv_tau=0.5), state))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
 @pytest.mark.parametrize("far", [0, 1, 63, 64, 65, 447])
 def test_recurrence_keeps_a_key_from_far_back(far):
     """With decay 1 one key that matches the last query and carries a value nobody else has must come through whole
