@@ -10,7 +10,7 @@
 // bytes in flight do not depend on registers or on how many warps are resident.  The copies
 // start before this kernel waits for the one before it: that kernel can have written only the
 // newest token's key and value, and the warp that meets this row fetches it again after the
-// wait.  The consumer warps (8 or 16, see below) take 16 keys of a page each:
+// wait.  The consumer warps (4, 8 or 16, see below) take 16 keys of a page each:
 // scores S = Q.K^T with mma.sync m16n8k16 (16-byte loads from shared memory straight into B
 // fragments, the head dimension permuted identically in Q), online softmax in float32 on the
 // accumulator registers, then O += P.V where V fragments are transposed in registers with
@@ -36,11 +36,12 @@
 
 #define AD_HD PE_HEAD_DIM
 #define AD_NCHUNK ((AD_HD + 31) / 32)
-// The kernel is compiled for 8 and for 16 consumer warps (one more warp is the producer).  Four warps share a
-// page, so 2 or 4 pages are under way at once.  16 warps (one CTA an SM) are quicker where few sequences
-// have long contexts; 8 warps (two CTAs an SM for head sizes up to 64) everywhere else.
-#define AD_CTAS(WARPS) (((WARPS) == 16 || AD_HD > 64) ? 1 : 2)
+// The kernel is compiled for 8 consumer warps (one more warp is the producer), for 16 (head sizes up to 64) and for 4 (up to 128); see
+// ad_choose.  Four warps share a page, so 1, 2 or 4 pages are under way at once.  A CTA of 16 warps has an SM for itself, and so has one
+// of 8 warps with larger heads; else an SM holds two.
+#define AD_CTAS(WARPS) ((WARPS) == 16 || ((WARPS) == 8 && AD_HD > 64) ? 1 : 2)
 #define AD_MAX_STAGES 12                             // pages in flight per CTA
+#define AD_RANKED 256                                // most tokens of a launch whose CTAs are ordered by length
 #define AD_MAX_SPLITS 16                             // page ranges of a sequence = CTAs of a cluster (8 is the portable limit)
 #define AD_KV_BYTES (PE_PAGE * AD_HD * 2)            // the keys (or the values) of one page and kv head
 #define AD_STAGE_BYTES (2 * AD_KV_BYTES)
@@ -226,16 +227,30 @@ __global__ void __launch_bounds__(32 * (AD_WARPS + 1), AD_CTAS(AD_WARPS)) attent
     const bf16* q, int q_stride, const bf16* k_pool, const bf16* v_pool,
     const int* block_table, int table_stride, const int* tok_pos,
     const int* tok_row, int nh, int nkv, int window, float scale_log2e, int n_splits, int stages,
-    int* status, bf16* out, int keep_first, const float* slopes, const float* sinks) {
+    int* status, bf16* out, int keep_first, const float* slopes, const float* sinks, int ranked) {
     constexpr int AD_GROUPS = AD_WARPS / 4, AD_THREADS = 32 * (AD_WARPS + 1);
     extern __shared__ __align__(128) unsigned char ad_smem[];   // result rows, then the ring (later: the warps' partial results)
     __shared__ __align__(8) unsigned long long bars[2 * AD_MAX_STAGES + 1];
     __shared__ int page_ok[AD_MAX_STAGES];                      // whether the stage holds a page (written by the producer)
     __shared__ float row_max[16];                               // the CTA's max of every row
     __shared__ int page_list[32];                               // the producer's next entries of the page table
+    __shared__ int lengths[AD_RANKED + 1];                      // positions of the launch's tokens; then the token this CTA takes
     pdl_launch_dependents();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-    const int tok = blockIdx.z;
+    int tok = blockIdx.z;
+    if (ranked) {                                               // the longest sequences first: CTA z takes the z-th longest
+        const int T = gridDim.z;
+        for (int i = threadIdx.x; i < T; i += AD_THREADS) lengths[i] = tok_pos[i];
+        __syncthreads();
+        for (int i = threadIdx.x; i < T; i += AD_THREADS) {
+            const int mine = lengths[i];
+            int before = 0;
+            for (int j = 0; j < T; ++j) before += lengths[j] > mine || (lengths[j] == mine && j < i);
+            if (before == (int)blockIdx.z) lengths[AD_RANKED] = i;
+        }
+        __syncthreads();
+        tok = lengths[AD_RANKED];
+    }
     const int split = n_splits > 1 ? (int)ad_cluster_rank() : 0;
     const int G = nh / nkv, head_tiles = (G + 15) / 16;
     const int kvh = blockIdx.y / head_tiles, ht = blockIdx.y % head_tiles;
@@ -555,7 +570,7 @@ struct AdVariant {
     static int launch(dim3 grid, int n_splits, int stages, cudaStream_t stream, const bf16* q, int q_stride, const bf16* k_pool,
                       const bf16* v_pool, const int* block_table, int table_stride, const int* tok_pos, const int* tok_row,
                       int nh, int nkv, int window, float scale_log2e, int* status, bf16* out, bool early, int keep_first,
-                      const float* slopes, const float* sinks) {
+                      const float* slopes, const float* sinks, int ranked) {
         const size_t smem = smem_bytes(stages);
         { const int e = allow_smem(smem); if (e) return e; }
         cudaLaunchConfig_t cfg = {};
@@ -578,7 +593,7 @@ struct AdVariant {
         cfg.attrs = attr;
         cfg.numAttrs = n_attr;
         PE_TRY(cudaLaunchKernelEx(&cfg, attention_decode_kernel<WARPS>, q, q_stride, k_pool, v_pool, block_table, table_stride,
-                                  tok_pos, tok_row, nh, nkv, window, scale_log2e, n_splits, stages, status, out, keep_first, slopes, sinks));
+                                  tok_pos, tok_row, nh, nkv, window, scale_log2e, n_splits, stages, status, out, keep_first, slopes, sinks, ranked));
         PE_LAUNCH_CHECK();
         return 0;
     }
@@ -590,28 +605,47 @@ static int& ad_split_limit() { static int limit = AD_MAX_SPLITS; return limit; }
 extern "C" void pe_attention_decode_set_max_splits(int n) { ad_split_limit() = n < 1 ? 1 : (n > AD_MAX_SPLITS ? AD_MAX_SPLITS : n); }
 
 // Which variant and shape a launch takes: a function of the launch's sizes (and of the GPU) only, never of
-// the sequences' lengths: the same launch is replayed as sequences grow.  Measured at head size 64: 16 warps
-// win where at most 32 CTA-triples have 8 or more pages each (8 sequences of 4,096 tokens: 8.1 us against
-// 8.3 us), 8 warps elsewhere (1 sequence: 4.9 us against 5.3 us; 64 sequences: 24 us against 27 us).
-static bool ad_choose(int T, int nh, int nkv, int max_context, int* splits_out, int* stages_out) {
-    const int G = nh / nkv, ctas = T * nkv * ((G + 15) / 16);
+// the sequences' lengths: the same launch is replayed as sequences grow.  Measured on a B200, sequences of a third of the
+// longest up to the longest, times of 8 warps against those of the variant taken:
+//   head size 64   16 warps where at most 32 CTA-triples have 8 or more pages each (8 sequences of 4,096 tokens: 8.3 against
+//                  8.1 us; 1 sequence: 4.9 against 5.3, 64 sequences 24 against 27 where the rule does not hold)
+//                  4 warps where a range is 1 or 2 pages long, the merge of fewer warps being most of what is left (1 sequence of
+//                  600 tokens 4.1 against 3.8 us, 8 of 2,000 7.2 against 6.5; with 3 pages a range they lose: 12 of 2,000 6.9, 7.2)
+//   head size 128  4 warps, two CTAs an SM, where one CTA an SM leaves the triples whole but two allow three ranges (19
+//                  sequences of 4,000 tokens and 4 kv heads 37.5 against 26.6 us, of 1,000 12.3 against 11.3; of 640 equal), and
+//                  where all triples of short sequences then run in one turn instead of two (64 sequences of 500 tokens 15.4
+//                  against 12.3 us, 48 of 800 17.9 against 16.9, 40 of 500 12.0 against 11.6; 40 of 800 would take 15.2 against 16.4)
+//                  8 warps with the longest sequences first where the triples take several turns (64 sequences of 300 to 4,000
+//                  tokens 62.3 in their own order, 47.5; 48 of 2,000 33.9 and 29.4; finding the order costs 1 us: 12 pages or less do not pay)
+struct AdShape { int warps, splits, stages; bool ranked; };
+static AdShape ad_choose(int T, int nh, int nkv, int max_context) {
+    const int G = nh / nkv, ctas = T * nkv * ((G + 15) / 16), limit = ad_split_limit();
     const int pages = (max_context + PE_PAGE - 1) / PE_PAGE;
-    if constexpr (AD_HD <= 64) {                             // larger heads need the registers: 8 warps only
+    const auto range = [&](int splits) { return (pages + splits - 1) / splits; };
+    AdShape c = {8, 1, 1, false};
+    c.splits = AdVariant<8>::shape(ctas, pages, limit, &c.stages);
+    if constexpr (AD_HD <= 64) {                             // larger heads need the registers
         if (ctas <= 32) {
-            int stages = 0;
-            const int splits = AdVariant<16>::shape(ctas, pages, ad_split_limit(), &stages);
-            if ((pages + splits - 1) / splits >= 8) { *splits_out = splits; *stages_out = stages; return true; }
+            AdShape w = {16, 1, 1, false};
+            w.splits = AdVariant<16>::shape(ctas, pages, limit, &w.stages);
+            if (range(w.splits) >= 8) return w;
         }
     }
-    *splits_out = AdVariant<8>::shape(ctas, pages, ad_split_limit(), stages_out);
-    return false;
+    if constexpr (AD_HD <= 128) {                            // larger heads leave room for one page only
+        AdShape n = {4, 1, 1, false};
+        n.splits = AdVariant<4>::shape(ctas, pages, limit, &n.stages);
+        if (AD_HD <= 64 ? range(n.splits) <= 2
+                        : (c.splits == 1 && n.splits >= 3 && pages >= 16) || (ctas > 148 && ctas <= 2 * 148 && pages <= (ctas < 192 ? 8 : 12)))
+            return n;
+    }
+    c.ranked = ctas > 148 * AdVariant<8>::ctas_per_sm && T > 1 && T <= AD_RANKED && pages > 12;
+    return c;
 }
 
 extern "C" int pe_attention_decode_splits(int T, int nh, int nkv, int max_context, int* stages_out) {
-    int splits = 1, stages = 1;
-    ad_choose(T, nh, nkv, max_context, &splits, &stages);
-    if (stages_out) *stages_out = stages;
-    return splits;
+    const AdShape c = ad_choose(T, nh, nkv, max_context);
+    if (stages_out) *stages_out = c.stages;
+    return c.splits;
 }
 
 extern "C" int pe_attention_decode(const void* q, int q_stride, void* out, const void* k_pool, const void* v_pool,
@@ -630,18 +664,16 @@ extern "C" int pe_attention_decode(const void* q, int q_stride, void* out, const
     if (((uintptr_t)q | (uintptr_t)k_pool | (uintptr_t)v_pool) & 15) return PE_ERR_UNSUPPORTED;
     const int G = nh / nkv;
     if ((long long)nkv * ((G + 15) / 16) > 65535) return PE_ERR_UNSUPPORTED;
-    int n_splits = 1, stages = 0;
-    const bool wide = ad_choose(T, nh, nkv, max_context, &n_splits, &stages);
-    if (stages < 1) return PE_ERR_UNSUPPORTED;
-    const dim3 grid(n_splits, nkv * ((G + 15) / 16), T);
+    const AdShape c = ad_choose(T, nh, nkv, max_context);
+    if (c.stages < 1) return PE_ERR_UNSUPPORTED;
+    const dim3 grid(c.splits, nkv * ((G + 15) / 16), T);
     const float scale_log2e = scale * 1.4426950408889634f;
-    if constexpr (AD_HD <= 64) {
-        if (wide)
-            return AdVariant<16>::launch(grid, n_splits, stages, (cudaStream_t)stream, (const bf16*)q, q_stride, (const bf16*)k_pool,
-                                         (const bf16*)v_pool, block_table, table_stride, tok_pos, tok_row, nh, nkv, window,
-                                         scale_log2e, status, (bf16*)out, early_pages != 0, keep_first, slopes, sinks);
-    }
-    return AdVariant<8>::launch(grid, n_splits, stages, (cudaStream_t)stream, (const bf16*)q, q_stride, (const bf16*)k_pool,
-                                (const bf16*)v_pool, block_table, table_stride, tok_pos, tok_row, nh, nkv, window, scale_log2e,
-                                status, (bf16*)out, early_pages != 0, keep_first, slopes, sinks);
+    const auto go = [&](auto variant) {
+        return decltype(variant)::launch(grid, c.splits, c.stages, (cudaStream_t)stream, (const bf16*)q, q_stride, (const bf16*)k_pool,
+                                         (const bf16*)v_pool, block_table, table_stride, tok_pos, tok_row, nh, nkv, window, scale_log2e,
+                                         status, (bf16*)out, early_pages != 0, keep_first, slopes, sinks, c.ranked ? 1 : 0);
+    };
+    if constexpr (AD_HD <= 64) { if (c.warps == 16) return go(AdVariant<16>()); }
+    if constexpr (AD_HD <= 128) { if (c.warps == 4) return go(AdVariant<4>()); }
+    return go(AdVariant<8>());
 }

@@ -258,6 +258,31 @@ def test_attention_decode(K, nh, nkv, hd, lens, window, max_context):
     assert torch.equal(late, got)
 
 
+SHAPE_CASES = [                       # (nh, nkv, hd, sequences, longest, bound on the context): the lines between launch shapes
+    (14, 2, 64, 1, 700, 2048), (14, 2, 64, 1, 700, 2112),             # 4 warps up to two pages a range, 8 behind
+    (14, 2, 64, 24, 128, 128), (2, 1, 16, 8, 300, 300),
+    (16, 4, 128, 19, 1024, 1024), (16, 4, 128, 19, 960, 960),         # three ranges instead of none, from 16 pages on
+    (16, 4, 128, 40, 500, 512), (16, 4, 128, 37, 500, 513),           # more triples than SMs: 4 warps up to 8 pages, then 8
+    (8, 2, 80, 74, 400, 512), (8, 2, 80, 75, 800, 833),               # as many as SMs, then the longest first
+    (4, 4, 128, 40, 833, 833), (1, 1, 128, 256, 900, 900), (1, 1, 128, 257, 900, 900),
+]
+
+
+@pytest.mark.parametrize("nh,nkv,hd,B,longest,bound", SHAPE_CASES)
+def test_attention_decode_launch_shapes(K, nh, nkv, hd, B, longest, bound):
+    """One token a sequence, sequences of one page up to the longest, several of the same length."""
+    lens = [longest] + [1 + (i * 37) % longest if i % 3 else longest // 2 for i in range(1, B)]
+    paged = Paged(lens, nkv, hd, torch.bfloat16, seed=hd)
+    rows, pos = list(range(B)), [n - 1 for n in lens]
+    q = rnd(B, nh, hd, seed=B).to(torch.bfloat16).float()
+    kp, vp, table = paged.cuda()
+    got = K.attention_decode(dev(q.reshape(B, -1).to(torch.bfloat16)), nh * hd, nh, nkv, hd, kp, vp, table, table.shape[1],
+                             dev(torch.tensor(pos, dtype=torch.int32)), dev(torch.tensor(rows, dtype=torch.int32)), None, hd ** -0.5, bound)
+    K.check_status("cuda")
+    err = attention_error(got, one_query_attention(q, paged, rows, pos, nh, None), "decode shapes")
+    assert err < ATTENTION_BOUND, err
+
+
 def one_query_attention(q_rows, paged, tok_row, tok_pos, nh, window):
     """The rows of ``reference_attention`` computed one query at a time (long sequences)."""
     out = []
