@@ -291,34 +291,58 @@ __global__ void __launch_bounds__(HT_THREADS, 1) attention_headmix_tcgen05_kerne
     }
 }
 
-// out[t][h][d] = sum_g mix[h, g] o[t][g][c(h)][d].  A thread has column d of key/value head c and up to eight of the heads that read it
-// (blockIdx.y: which eight): a head's outputs are read once for all of them, neighbouring threads side by side, and no read waits for
-// another.  Bound by reading o.
-#define HT_MIX_HEADS 8
+// out[t][h][d] = sum_g mix[h, g] o[t][g][c(h)][d].  A thread has four columns of key/value head c and HEADS of the heads that read it
+// (blockIdx.y: which): a head's outputs are read once for all of them, neighbouring threads side by side, and no read waits for another.
+// The weights of one g lie side by side in shared memory, so that one read serves them all.  Bound by reading o: 7.2 us at
+// 1,024 tokens of 16 heads over 4 x 128 columns (34 MB), against 15.1 with a column and eight heads a thread.
+#define HT_MIX_HEADS 8                                              // at most
+template <int HEADS>
 __global__ void __launch_bounds__(256) headmix_mix_kernel(const float* o, const float* mix, bf16* out, int T, int H, int G, int Dv) {
     pdl_launch_dependents();
+    extern __shared__ __align__(16) float ht_mix[];                 // [G][H][HEADS]: the weights of this block's heads of every c
     pdl_wait();
-    extern __shared__ float ht_mix[];                               // [H][H]
     const int per = H / G, cols = G * Dv;
-    for (int i = threadIdx.x; i < H * H; i += blockDim.x) ht_mix[i] = mix[i];
+    for (int i = threadIdx.x; i < G * H * HEADS; i += blockDim.x) {
+        const int h = blockIdx.y * HEADS + i % HEADS, g = i / HEADS % H, c = i / HEADS / H;
+        ht_mix[i] = h < per ? mix[(c * per + h) * H + g] : 0.f;
+    }
     __syncthreads();
-    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long e = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (e >= (long long)T * cols) return;
     const int t = (int)(e / cols), col = (int)(e % cols), c = col / Dv, d = col % Dv;
-    const int h0 = c * per + blockIdx.y * HT_MIX_HEADS, n_h = min(HT_MIX_HEADS, c * per + per - h0);
     const float* src = o + (size_t)t * H * cols + col;
-    float acc[HT_MIX_HEADS];
+    const float* w = ht_mix + c * H * HEADS;
+    float4 acc[HEADS];
 #pragma unroll
-    for (int i = 0; i < HT_MIX_HEADS; ++i) acc[i] = 0.f;
+    for (int i = 0; i < HEADS; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 8
     for (int g = 0; g < H; ++g) {
-        const float v = src[(size_t)g * cols];
+        const float4 v = *reinterpret_cast<const float4*>(src + (size_t)g * cols);
 #pragma unroll
-        for (int i = 0; i < HT_MIX_HEADS; ++i) acc[i] = fmaf(ht_mix[min(h0 + i, H - 1) * H + g], v, acc[i]);
+        for (int i = 0; i < HEADS; ++i) {
+            const float x = w[g * HEADS + i];
+            acc[i].x = fmaf(x, v.x, acc[i].x); acc[i].y = fmaf(x, v.y, acc[i].y); acc[i].z = fmaf(x, v.z, acc[i].z); acc[i].w = fmaf(x, v.w, acc[i].w);
+        }
     }
+    const int h0 = c * per + blockIdx.y * HEADS, n_h = min(HEADS, per - (int)blockIdx.y * HEADS);
 #pragma unroll
-    for (int i = 0; i < HT_MIX_HEADS; ++i)
-        if (i < n_h) out[((size_t)t * H + h0 + i) * Dv + d] = __float2bfloat16_rn(acc[i]);
+    for (int i = 0; i < HEADS; ++i) {
+        if (i >= n_h) break;
+        uint2 r;
+        *reinterpret_cast<__nv_bfloat162*>(&r.x) = __floats2bfloat162_rn(acc[i].x, acc[i].y);
+        *reinterpret_cast<__nv_bfloat162*>(&r.y) = __floats2bfloat162_rn(acc[i].z, acc[i].w);
+        *reinterpret_cast<uint2*>(out + ((size_t)t * H + h0 + i) * Dv + d) = r;
+    }
+}
+
+template <int HEADS>
+static int ht_mix_launch(const float* o, const float* mix, bf16* out, int T, int H, int G, int Dv, cudaStream_t s) {
+    const size_t smem = sizeof(float) * G * H * HEADS;              // HEADS < 2 H / G: less than 128 KB
+    if (smem > 48 * 1024) PE_TRY(cudaFuncSetAttribute(headmix_mix_kernel<HEADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const dim3 grid((unsigned)(((long long)T * G * Dv / 4 + 255) / 256), (H / G + HEADS - 1) / HEADS);
+    PE_TRY(pe_launch(headmix_mix_kernel<HEADS>, grid, 256, smem, s, o, mix, out, T, H, G, Dv));
+    PE_LAUNCH_CHECK();
+    return 0;
 }
 
 // How the sizes are laid out: value heads a CTA and stages of the ring; false: not taken.
@@ -366,10 +390,7 @@ extern "C" int pe_attention_headmix_tcgen05(const void* q, int q_stride, void* o
     PE_TRY(cudaFuncSetAttribute(attention_headmix_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, HT_SMEM_LIMIT));
     PE_TRY(pe_launch(attention_headmix_tcgen05_kernel, dim3(H * (G / a.cg), n_tiles), HT_THREADS, smem, s, mq, mk, mv, a, status));
     PE_LAUNCH_CHECK();
-    const size_t mix_smem = sizeof(float) * H * H;
-    if (mix_smem > 48 * 1024) PE_TRY(cudaFuncSetAttribute(headmix_mix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mix_smem));
-    const dim3 grid((unsigned)(((long long)T * G * Dv + 255) / 256), (H / G + HT_MIX_HEADS - 1) / HT_MIX_HEADS);
-    PE_TRY(pe_launch(headmix_mix_kernel, grid, 256, mix_smem, s, (const float*)scratch, mix, (bf16*)out, T, H, G, Dv));
-    PE_LAUNCH_CHECK();
-    return 0;
+    const int per = H / G;
+    const auto launch = per == 1 ? ht_mix_launch<1> : per == 2 ? ht_mix_launch<2> : per <= 4 ? ht_mix_launch<4> : ht_mix_launch<HT_MIX_HEADS>;
+    return launch((const float*)scratch, mix, (bf16*)out, T, H, G, Dv, s);
 }

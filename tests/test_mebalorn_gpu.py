@@ -243,6 +243,31 @@ def test_headmix_kernel_sink_alone_scales_the_output():
         assert abs(float(got[0, 0, 0]) - 1 / (1 + math.exp(sink - 1.6))) < 1e-6 and abs(float(got[0, 1, 0]) - 0.5) < 1e-6
 
 
+@pytest.mark.parametrize("H,G,D,Dv", [(1, 1, 8, 8), (5, 2, 48, 16), (30, 5, 64, 64), (16, 4, 128, 128), (3, 3, 72, 40), (9, 1, 256, 264), (4, 2, 20, 24), (2, 1, 264, 8)])
+@pytest.mark.parametrize("normed", ["both", "queries", "stored only"])
+def test_norm_of_queries_and_keys_and_the_store(H, G, D, Dv, normed):
+    """Heads that fill 8, 16 and 32 lanes, whole and in part, one and several turns of a block, and sizes of the general kernel."""
+    from pico_engine.ops import kernels
+    g = torch.Generator().manual_seed(D)
+    n = 70
+    rows = torch.randn(n, (H + G) * D + G * Dv, generator=g).bfloat16()
+    qw, kw = (1 + 0.2 * torch.randn(D, generator=g) for _ in range(2))
+    qw, kw = (qw.bfloat16() if normed != "stored only" else None), (kw if normed == "both" else None)
+    kp, vp, tab = paged(torch.zeros(n, G, D), torch.zeros(n, G, Dv), torch.bfloat16)
+    dev = rows.cuda()
+    kernels.qknorm_store(dev, H, G, D, Dv, None if qw is None else qw.cuda(), None if kw is None else kw.cuda(), 1e-5,
+                         torch.arange(n, dtype=torch.int32).cuda(), torch.zeros(n, dtype=torch.int32).cuda(), kp, vp, tab, tab.shape[1])
+    want = rows.double()
+    heads = want[:, :(H + G) * D].view(n, H + G, D)
+    for w, part in ((qw, slice(0, H)), (kw, slice(H, H + G))):
+        if w is not None:
+            heads[:, part] *= w.double() / (heads[:, part] ** 2).mean(-1, keepdim=True).add(1e-5).sqrt()
+    got = dev.cpu().double()
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all()       # half a step of bfloat16 and float32 arithmetic
+    k, v = (torch.cat([pool[page] for page in tab[0].tolist()], 1).transpose(0, 1)[:n].reshape(n, -1).cpu().double() for pool in (kp, vp))
+    assert torch.equal(k, got[:, H * D:(H + G) * D]) and torch.equal(v, rows[:, (H + G) * D:].double())
+
+
 @pytest.mark.parametrize("H,G,D,Dv,window", [(2, 1, 16, 64, None), (6, 2, 48, 96, 100), (3, 3, 64, 64, None), (16, 4, 128, 128, None),
                                              (20, 2, 64, 64, 1), (4, 4, 128, 128, 300), (5, 1, 64, 256, None), (7, 7, 32, 64, 64)])
 def test_headmix_prompts_in_tensor_memory(H, G, D, Dv, window):
