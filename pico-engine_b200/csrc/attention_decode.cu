@@ -222,23 +222,23 @@ __device__ __forceinline__ void ad_consume(float (&acc)[AD_NCHUNK][4][4], float 
     }
 }
 
-template <int AD_WARPS>
+template <int AD_WARPS, bool RANKED>
 __global__ void __launch_bounds__(32 * (AD_WARPS + 1), AD_CTAS(AD_WARPS)) attention_decode_kernel(
     const bf16* q, int q_stride, const bf16* k_pool, const bf16* v_pool,
     const int* block_table, int table_stride, const int* tok_pos,
     const int* tok_row, int nh, int nkv, int window, float scale_log2e, int n_splits, int stages,
-    int* status, bf16* out, int keep_first, const float* slopes, const float* sinks, int ranked) {
+    int* status, bf16* out, int keep_first, const float* slopes, const float* sinks) {
     constexpr int AD_GROUPS = AD_WARPS / 4, AD_THREADS = 32 * (AD_WARPS + 1);
     extern __shared__ __align__(128) unsigned char ad_smem[];   // result rows, then the ring (later: the warps' partial results)
     __shared__ __align__(8) unsigned long long bars[2 * AD_MAX_STAGES + 1];
     __shared__ int page_ok[AD_MAX_STAGES];                      // whether the stage holds a page (written by the producer)
     __shared__ float row_max[16];                               // the CTA's max of every row
     __shared__ int page_list[32];                               // the producer's next entries of the page table
-    __shared__ int lengths[AD_RANKED + 1];                      // positions of the launch's tokens; then the token this CTA takes
     pdl_launch_dependents();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     int tok = blockIdx.z;
-    if (ranked) {                                               // the longest sequences first: CTA z takes the z-th longest
+    if constexpr (RANKED) {                                     // the longest sequences first: CTA z takes the z-th longest
+        __shared__ int lengths[AD_RANKED + 1];                  // positions of the launch's tokens; then the token this CTA takes
         const int T = gridDim.z;
         for (int i = threadIdx.x; i < T; i += AD_THREADS) lengths[i] = tok_pos[i];
         __syncthreads();
@@ -493,7 +493,7 @@ extern "C" void pe_set_pdl(int on) { pe_pdl_enabled() = on ? 1 : 0; }
 // live in one process, and the function-local statics of a template with external linkage would be one
 // object for all of them (the dynamic linker makes such symbols unique across libraries).
 namespace {
-template <int WARPS>
+template <int WARPS, bool RANKED = false>
 struct AdVariant {
     static constexpr int threads = 32 * (WARPS + 1), groups = WARPS / 4, ctas_per_sm = AD_CTAS(WARPS);
 
@@ -507,12 +507,12 @@ struct AdVariant {
         static size_t allowed = 48 * 1024 - 512;
         static bool wide = false;
         if (!wide) {                                         // clusters of more than 8 CTAs are an opt-in; if it is refused,
-            cudaFuncSetAttribute(attention_decode_kernel<WARPS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);   // the
+            cudaFuncSetAttribute(attention_decode_kernel<WARPS, RANKED>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);   // the
             cudaGetLastError();                              // occupancy query below answers 0 for them and fewer ranges are used
             wide = true;
         }
         if (smem > allowed) {
-            PE_TRY(cudaFuncSetAttribute(attention_decode_kernel<WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            PE_TRY(cudaFuncSetAttribute(attention_decode_kernel<WARPS, RANKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             allowed = smem;
         }
         return 0;
@@ -537,7 +537,7 @@ struct AdVariant {
             attr[0].val.clusterDim.x = splits; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
             cfg.attrs = attr;
             cfg.numAttrs = 1;
-            if (cudaOccupancyMaxActiveClusters(&n, attention_decode_kernel<WARPS>, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+            if (cudaOccupancyMaxActiveClusters(&n, attention_decode_kernel<WARPS, RANKED>, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
         }
         known[{splits, smem}] = n;
         return n;
@@ -570,7 +570,7 @@ struct AdVariant {
     static int launch(dim3 grid, int n_splits, int stages, cudaStream_t stream, const bf16* q, int q_stride, const bf16* k_pool,
                       const bf16* v_pool, const int* block_table, int table_stride, const int* tok_pos, const int* tok_row,
                       int nh, int nkv, int window, float scale_log2e, int* status, bf16* out, bool early, int keep_first,
-                      const float* slopes, const float* sinks, int ranked) {
+                      const float* slopes, const float* sinks) {
         const size_t smem = smem_bytes(stages);
         { const int e = allow_smem(smem); if (e) return e; }
         cudaLaunchConfig_t cfg = {};
@@ -592,8 +592,8 @@ struct AdVariant {
         }
         cfg.attrs = attr;
         cfg.numAttrs = n_attr;
-        PE_TRY(cudaLaunchKernelEx(&cfg, attention_decode_kernel<WARPS>, q, q_stride, k_pool, v_pool, block_table, table_stride,
-                                  tok_pos, tok_row, nh, nkv, window, scale_log2e, n_splits, stages, status, out, keep_first, slopes, sinks, ranked));
+        PE_TRY(cudaLaunchKernelEx(&cfg, attention_decode_kernel<WARPS, RANKED>, q, q_stride, k_pool, v_pool, block_table, table_stride,
+                                  tok_pos, tok_row, nh, nkv, window, scale_log2e, n_splits, stages, status, out, keep_first, slopes, sinks));
         PE_LAUNCH_CHECK();
         return 0;
     }
@@ -671,9 +671,9 @@ extern "C" int pe_attention_decode(const void* q, int q_stride, void* out, const
     const auto go = [&](auto variant) {
         return decltype(variant)::launch(grid, c.splits, c.stages, (cudaStream_t)stream, (const bf16*)q, q_stride, (const bf16*)k_pool,
                                          (const bf16*)v_pool, block_table, table_stride, tok_pos, tok_row, nh, nkv, window, scale_log2e,
-                                         status, (bf16*)out, early_pages != 0, keep_first, slopes, sinks, c.ranked ? 1 : 0);
+                                         status, (bf16*)out, early_pages != 0, keep_first, slopes, sinks);
     };
     if constexpr (AD_HD <= 64) { if (c.warps == 16) return go(AdVariant<16>()); }
     if constexpr (AD_HD <= 128) { if (c.warps == 4) return go(AdVariant<4>()); }
-    return go(AdVariant<8>());
+    return c.ranked ? go(AdVariant<8, true>()) : go(AdVariant<8>());
 }
