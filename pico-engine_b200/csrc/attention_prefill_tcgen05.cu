@@ -22,7 +22,7 @@
 // What bounds a step: its 16,384 exponentials take 1,024 cycles of the special-function units.  With all
 // eight warps on one step (two threads a row that told each other their maxima) a step was a chain of
 // 2,480 cycles (clock stamps: waits 370, maxima 430, exponentials 1,100, P through shared memory 350);
-// with the warpgroups in turn it is 1,500 (head size 64) and about 1,700 (128).  2,048 tokens, 14 heads of 64, on a B200: 30 us before,
+// with the warpgroups in turn it is 1,500 (head size 64).  2,048 tokens, 14 heads of 64, on a B200: 30 us before,
 // 26 us here; 28 heads of 128, prompts of 5,001 / 1,807 / 700 / 33 tokens: 341 us before, 278 us here.
 //
 // Values lie in the cache as [key][head size], which is the MN-major form of the B operand of

@@ -10,7 +10,8 @@
 // decays, and what remains are plain products.
 //
 // Bound by float32 multiply-adds (fma.rn.f32x2) and, in the first kernel, by the decays' exponentials and logarithms.  2,048 tokens, 16
-// heads of 128 x 128, on a B200: 258 us as two walks of every chunk, 163 us here (weights 74, contributions 40, outputs 49).
+// heads of 128 x 128, on a B200: 258 us as two walks of every chunk, 160 us here (weights 71, contributions 39, outputs 50); the
+// logits come as the product before wrote them (as float32 they were converted first, 10.5 us).
 #include "linear_attention.cuh"
 #include "chunk_tiles.cuh"
 

@@ -117,8 +117,7 @@ class LinearAttention(Mixer, SharedProducts):
         qk, vo = self._sizes()
         # Prompts run as products of tiles over chunks of 64 tokens; rows that bring a few tokens walk them.  (Either way gives the same
         # numbers up to float32 rounding.)  A walk takes as long as the longest row
-        # whatever it leaves idle (2,048 tokens of 16 heads of 128 x 128 on a B200: 709 us against 180 us, four such prompts 1,062 us against
-        # 650); a chunk costs its tiles even where it holds a few tokens.
+        # whatever it leaves idle; a chunk costs its tiles even where it holds a few tokens.
         chunked = any(n > 16 for n in ctx.lens)
         # (keys that are scaled but not turned: the scale moves to the queries, the output being linear in either)
         q_scale = s.q_scale if turned is not None else s.q_scale * s.k_scale
