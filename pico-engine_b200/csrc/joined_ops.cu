@@ -79,6 +79,18 @@ __global__ void __launch_bounds__(HN_THREADS) heads_norm_store_kernel(HeadsNormA
             }
         }
         __syncthreads();
+        // Where half a rotation is whole lanes, entry e turns with entry e of the lane `turn` further on (or back), by angles that the lane
+        // keeps: no exchange through shared memory, whose reads eight entries apart met on four banks.  2,000 tokens of 32 + 8 heads of 64 that turn
+        // 48 entries: 17.8 to 16.3 us.
+        const int turn = half % 8 == 0 ? half / 8 : 0;
+        const bool front = l < turn, turns = turn && l < 2 * turn;
+        const int partner = front ? lane + turn : lane - turn;
+        float cs[8], sn[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const int d = front ? l * 8 + e : l * 8 + e - half;
+            cs[e] = turns ? s_cos[d] : 1.f; sn[e] = turns ? s_sin[d] : 0.f;
+        }
         for (int h_first = h - sub; h_first < n_heads; h_first += step, h += step) {      // (the whole warp together)
             const bool live = on && h < n_heads;
             uint4 next = make_uint4(0u, 0u, 0u, 0u);
@@ -99,7 +111,13 @@ __global__ void __launch_bounds__(HN_THREADS) heads_norm_store_kernel(HeadsNormA
 #pragma unroll
                 for (int e = 0; e < 8; ++e) f[e] *= rstd * (query ? qw[e] : kw[e]);
             }
-            if (half) {
+            if (turn) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const float other = __shfl_sync(0xffffffffu, f[e], turns ? partner : lane);
+                    if (turns) f[e] = front ? f[e] * cs[e] - other * sn[e] : f[e] * cs[e] + other * sn[e];
+                }
+            } else if (half) {
                 __syncwarp();
                 if (live) {
                     *reinterpret_cast<float4*>(buf + l * 8) = make_float4(f[0], f[1], f[2], f[3]);
