@@ -45,7 +45,7 @@ __device__ __forceinline__ void hn_weights8(const void* w, int dtype, int at, fl
 // rotation.  A block a token (VEC: or gridDim.y blocks, each with its share of the heads, where the tokens are few); a pass's entries are
 // asked for before the pass in front of it, and the first one's before the angles, are worked out.
 template <typename T, bool VEC>
-__global__ void __launch_bounds__(HN_THREADS) heads_norm_store_kernel(HeadsNormArgs a) {
+__global__ void __launch_bounds__(HN_THREADS, 4) heads_norm_store_kernel(HeadsNormArgs a) {
     pdl_launch_dependents();
     __shared__ float s_cos[HN_MAX_D / 2], s_sin[HN_MAX_D / 2];
     __shared__ __align__(16) float s_row[HN_THREADS / 32][8 * 32];
@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(HN_THREADS) heads_norm_store_kernel(HeadsNormA
         __syncthreads();
         // Where half a rotation is whole lanes, entry e turns with entry e of the lane `turn` further on (or back), by angles that the lane
         // keeps: no exchange through shared memory, whose reads eight entries apart met on four banks.  2,000 tokens of 32 + 8 heads of 64 that turn
-        // 48 entries: 17.8 to 16.3 us.
+        // 48 entries: 17.8 to 16.3 us, and 13.6 with eight blocks of 128 threads an SM instead of six (64 registers a thread).
         const int turn = half % 8 == 0 ? half / 8 : 0;
         const bool front = l < turn, turns = turn && l < 2 * turn;
         const int partner = front ? lane + turn : lane - turn;
