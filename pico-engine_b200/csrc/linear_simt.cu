@@ -20,8 +20,9 @@ static int ls_ranges(int N, int K) {
 }
 __host__ __device__ __forceinline__ int ls_range_len(int K, int ranges) { return ((K + ranges - 1) / ranges + 15) / 16 * 16; }
 
+// (not .aligned: the lanes of a warp come here from loops that they leave apart)
 __device__ __forceinline__ void ls_cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 __device__ __forceinline__ float ls_peer_value(const float* mine, int rank) {          // the same place in the shared memory of CTA `rank`
     unsigned at = (unsigned)__cvta_generic_to_shared(mine), peer;
