@@ -200,6 +200,8 @@ __global__ void __launch_bounds__(HT_THREADS, 1) attention_headmix_tcgen05_kerne
             // (S of the step exists, so its rows have landed; the flags were written before they were asked for)
             if (!at_wait_warp(at_smem(&kv_full[st]), st_round & 1u)) { ok = false; break; }
             const bool there = (stage_flags[st] >> g) & 1u;
+            if (it + 1 == n_steps)
+                at_clear_rows(kv_s + st * stage_bytes + p.qp * HT_PANEL, p.cg * p.vp, HT_PANEL, pos0 + n - (page_lo + 2 * it) * HT_KTILE, threadIdx.x - 64, HT_THREADS - 64);
             if (++st == p.stages) { st = 0; ++st_round; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int key0 = (page_lo + 2 * it + g) * HT_KTILE;

@@ -185,6 +185,8 @@ __global__ void __launch_bounds__(LT_THREADS, 1) attention_latent_tcgen05_kernel
             // (S of the step exists, so its rows have landed; the flags were written before they were asked for)
             if (!at_wait_warp(at_smem(&kv_full[st]), (unsigned)(it / LT_STAGES) & 1u)) { ok = false; break; }
             const bool there = (stage_flags[st] >> g) & 1u;
+            // (S of the last step exists: its rows are read as values only from here on)
+            if (it + 1 == n_steps) at_clear_rows(kv_s + st * STAGE, p.rank / 64, LT_PANEL, pos0 + n - (page_lo + 2 * it) * LT_KTILE, threadIdx.x - 64, LT_THREADS - 64);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int key0 = (page_lo + 2 * it + g) * LT_KTILE;
             unsigned raw[LT_KTILE];

@@ -50,6 +50,18 @@ __device__ __forceinline__ void at_mma_ts(unsigned tmem_d, unsigned tmem_a, unsi
 __device__ __forceinline__ void at_commit(unsigned bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
+// The value rows of a step (128 rows of 128 bytes in each of `panels` panels) from `used` on to the end of their page become zero.  They
+// lie behind the run's last token, and a page is taken as its last owner left it: a weight of zero would not keep a value that is no
+// number out of the outputs.  `threads` threads call it when the copies have landed and nothing but P V still reads the rows; each of
+// them arrives (behind a __syncwarp of its warp) at the barrier that P V waits for.
+__device__ __forceinline__ void at_clear_rows(unsigned values, int panels, int panel_bytes, int used, int thread, int threads) {
+    const int bytes = (-used & (PE_PAGE - 1)) * 128;
+    if (bytes == 0) return;
+    for (int c = 0; c < panels; ++c)
+        for (int i = thread * 16; i < bytes; i += threads * 16)
+            asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(values + c * panel_bytes + used * 128 + i), "r"(0u) : "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // P V reads them through the tensor core's proxy
+}
 // 32 columns of this thread's lane.  at_ld32_start only issues the load: the values are there after at_ld_wait, and
 // at_pin32 after that keeps the compiler from using the registers any earlier.
 __device__ __forceinline__ void at_ld32_start(unsigned taddr, unsigned* r) {

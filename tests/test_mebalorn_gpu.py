@@ -402,3 +402,30 @@ def test_pointwise_kernels():
         want = torch.stack([1 + plain.sinusoid(1, width, torch.float64, first=int(p))[0] for p in pos.cpu()])
         assert (kernels.add_sinusoid(x, pos, freq.float().cuda()).cpu() - want).abs().max() < 5e-3      # the angle is a float32 product
         assert (x[:3].cpu() - want[:3]).abs().max() < 1e-5
+
+
+@pytest.mark.parametrize("rubbish", [float("nan"), float("inf")])
+@pytest.mark.parametrize("H,G,D,Dv", [(2, 1, 16, 64), (6, 2, 48, 96), (16, 4, 128, 128), (5, 1, 64, 256)])
+def test_headmix_prompts_do_not_see_what_an_earlier_owner_left_in_a_page(H, G, D, Dv, rubbish):
+    """Cache rows that no live sequence has written may hold anything: with numbers that are none in all of them, prompts that end on,
+    before and behind the borders of pages and of runs give the same bits as with zeros."""
+    from pico_engine.ops import kernels
+    from pico_engine.ops.library import mixers
+    assert mixers().pe_attention_headmix_tcgen05_takes(H, G, D, Dv)
+    g = torch.Generator().manual_seed(H)
+    sink, talk = torch.randn(H, generator=g).cuda(), (torch.eye(H) + 0.4 * torch.randn(H, H, generator=g)).cuda()
+    for n, start in ((1, 0), (37, 0), (64, 0), (127, 0), (129, 0), (300, 0), (700, 650)):
+        k, v = torch.randn(n, G, D, generator=g), torch.randn(n, G, Dv, generator=g)
+        q = torch.randn(n - start, H * D, generator=g).bfloat16().cuda()
+        got = []
+        for fill in (0.0, rubbish):
+            kp, vp, table = paged(k, v, torch.bfloat16)
+            for pool, page in ((kp, int(table[0, -1])), (vp, int(table[0, -1]))):
+                if n % 64:
+                    pool[page, :, n % 64:] = fill
+                pool[[i for i in range(pool.shape[0]) if i not in table[0].tolist()]] = fill
+            ctx = SimpleNamespace(one_token_each=False, scratch={}, lens=[n - start], starts=[start], max_context=n)
+            pos, row = torch.arange(start, n, dtype=torch.int32).cuda(), torch.zeros(n - start, dtype=torch.int32).cuda()
+            got.append(kernels.attention_headmix(q, H * D, H, G, D, Dv, kp, vp, table, table.shape[1], pos, row, None, D ** -0.5, sink, talk, ctx))
+        kernels.check_status(torch.device("cuda", torch.cuda.current_device()))
+        assert torch.equal(*got), (n, start)

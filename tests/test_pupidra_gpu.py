@@ -524,3 +524,24 @@ def test_pairs_of_tokens_in_the_embedding(dtype):
             assert (a.double() - b).abs().max() < 1e-6
         assert int(state[0, 0]) == 77 and int(state[4, 0]) == 77
         assert state[1:4, 0].tolist() == [s[-1] for s in seqs]
+
+
+@pytest.mark.parametrize("rubbish", [float("nan"), float("inf")])
+@pytest.mark.parametrize("H,width,rank", [(3, 96, 64), (2, 192, 128), (16, 256, 192)])
+def test_prompts_over_low_rank_rows_do_not_see_what_an_earlier_owner_left_in_a_page(H, width, rank, rubbish):
+    """Cache rows that no live sequence has written may hold anything: with numbers that are none in all of them, prompts that end on,
+    before and behind the borders of pages and of runs give the same bits as with zeros."""
+    from pico_engine.ops import kernels
+    g = torch.Generator().manual_seed(width)
+    for n, start in ((1, 0), (37, 0), (64, 0), (127, 0), (129, 0), (300, 0), (700, 650)):
+        k, q = torch.randn(n, 1, width, generator=g), torch.randn(n - start, H * width, generator=g).bfloat16().cuda()
+        got = []
+        for fill in (0.0, rubbish):
+            pool, table = paged(k, torch.bfloat16)
+            pool[0] = fill
+            if n % 64:
+                pool[-1, :, n % 64:] = fill
+            ctx = SimpleNamespace(one_token_each=False, scratch={}, lens=[n - start], starts=[start], dtype=torch.bfloat16)
+            got.append(kernels.attention_latent_prompt(q, H * width, H, width, rank, pool, table, table.shape[1], None, width ** -0.5, ctx))
+        kernels.check_status(torch.device("cuda", torch.cuda.current_device()))
+        assert torch.equal(*got), (n, start)
