@@ -32,6 +32,11 @@ __device__ __forceinline__ float4 st_four(st_pair a, st_pair b) {
     return make_float4(x.x, x.y, y.x, y.y);
 }
 
+// Whether one of four numbers is an infinity or no number.  In a product of weights and a chunk's values a token's weight for the tokens in
+// front of it is zero, which keeps it out of their sums only while its values are finite: chunks where they are not take the products
+// token by token as far as they reach.
+__device__ __forceinline__ bool st_odd(const float4& v) { return !(fabsf(v.x) < INFINITY && fabsf(v.y) < INFINITY && fabsf(v.z) < INFINITY && fabsf(v.w) < INFINITY); }
+
 // Columns c0 .. c0 + 31 of 64 rows (tokens) into dst[column][token]; entry (column k, token t) lies at k * 64 + (t ^ 4 ((k / 4) % 8)), so
 // that neither the four stores of a thread nor the reads of four neighbouring tokens meet in a bank.
 __device__ __forceinline__ int st_turned(int k, int t) { return k * ST_CHUNK + (t ^ (((k >> 2) & 7) << 2)); }
@@ -58,4 +63,26 @@ __device__ __forceinline__ void st_place(int& ty, int& tx) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     ty = (warp >> 1) * 4 + (lane >> 3);
     tx = (warp & 1) * 8 + (lane & 7);
+}
+// acc += weights x values over a chunk's first `last` tokens: weights [64 s][64 t], values [64 s][64 columns].  guarded: some value is no
+// finite number, and a token joins the sums of none in front of it.
+__device__ __forceinline__ void st_weighted(st_pair (&acc)[8][2], const float* weights, const float* values, int last, int ty, int tx, bool guarded) {
+#pragma unroll 4
+    for (int s = 0; s < (guarded ? 0 : last); ++s) {
+        float w[8];
+        *reinterpret_cast<float4*>(w) = *reinterpret_cast<const float4*>(weights + s * ST_CHUNK + ty * 4);
+        *reinterpret_cast<float4*>(w + 4) = *reinterpret_cast<const float4*>(weights + s * ST_CHUNK + ty * 4 + 32);
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(values + s * 64 + tx * 4);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) { st_fma(acc[i][0], w[i], v.x); st_fma(acc[i][1], w[i], v.y); }
+    }
+#pragma unroll 1
+    for (int s = 0; s < (guarded ? last : 0); ++s) {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(values + s * 64 + tx * 4);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int t = ty * 4 + 32 * (i / 4) + i % 4;
+            if (s <= t) { st_fma(acc[i][0], weights[s * ST_CHUNK + t], v.x); st_fma(acc[i][1], weights[s * ST_CHUNK + t], v.y); }
+        }
+    }
 }

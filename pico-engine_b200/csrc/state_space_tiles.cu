@@ -255,6 +255,7 @@ __global__ void __launch_bounds__(ST_THREADS) st_output_kernel(ScanArgs a, int v
     float* xs = smem + SS_CHUNK * SS_CHUNK;                // [64 s][64 p]
     const float* scores = a.chunk_scores + ((size_t)blockIdx.x * a.G + g) * SS_CHUNK * SS_CHUNK;
     const float* x_src = a.xbc + (size_t)first * a.xbc_ld + h * P + p0;
+    bool odd = false;
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
         const int i = tid + e * ST_THREADS, s = i >> 4, t = (i & 15) * 4;
@@ -267,6 +268,7 @@ __global__ void __launch_bounds__(ST_THREADS) st_output_kernel(ScanArgs a, int v
         w.z = s <= t + 2 ? w.z * (d * expf((float)(las[t + 2] - ls))) : 0.f;
         w.w = s <= t + 3 ? w.w * (d * expf((float)(las[t + 3] - ls))) : 0.f;
         *reinterpret_cast<float4*>(pt + 4 * i) = w;
+        odd = odd || st_odd(x);
         *reinterpret_cast<float4*>(xs + 4 * i) = x;
     }
 #pragma unroll
@@ -276,17 +278,9 @@ __global__ void __launch_bounds__(ST_THREADS) st_output_kernel(ScanArgs a, int v
         asm("mov.b64 %0, {%1, %2};" : "=l"(acc[i][0]) : "f"(u.x * d), "f"(u.y * d));
         asm("mov.b64 %0, {%1, %2};" : "=l"(acc[i][1]) : "f"(v.x * d), "f"(v.y * d));
     }
-    __syncthreads();
+    const bool guarded = __syncthreads_or(odd);
     const int last = min(n, 32 + 16 * (tid >> 6) + 16);    // a warp's tokens reach this far: later ones have no weight
-#pragma unroll 4
-    for (int s = 0; s < last; ++s) {
-        float w[8];
-        *reinterpret_cast<float4*>(w) = *reinterpret_cast<const float4*>(pt + s * SS_CHUNK + ty * 4);
-        *reinterpret_cast<float4*>(w + 4) = *reinterpret_cast<const float4*>(pt + s * SS_CHUNK + ty * 4 + 32);
-        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(xs + s * 64 + tx * 4);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) { st_fma(acc[i][0], w[i], x.x); st_fma(acc[i][1], w[i], x.y); }
-    }
+    st_weighted(acc, pt, xs, last, ty, tx, guarded);
     const float Dh = load_as_f(a.d_skip, a.d_dtype, h);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {

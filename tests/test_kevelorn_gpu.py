@@ -524,3 +524,24 @@ def test_routing_of_a_model_picks_what_the_plain_router_picks(models):
     got = part.apply(h.cuda(), ctx).cpu()
     want = plain.mixture(h.double(), {n: t.double() for n, t in w.items()}, "l0.mlp.", cfg["layers"][0]["mlp"])
     assert (got - want).abs().max() < 2e-5 * max(1.0, float(want.abs().max()))
+
+
+@pytest.mark.parametrize("odd", [float("nan"), float("inf")])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("which", ["q", "k", "v", "z"])
+def test_a_token_that_is_no_number_does_not_reach_back(which, dtype, odd):
+    """Chunks against the walk: what comes before the token is bit for bit what it is without it, and what comes behind is lost in the
+    same places."""
+    dt, H, D, Dv, lens = DTYPES[dtype], 2, 24, 70, [130, 40]
+    g = torch.Generator().manual_seed(5)
+    T = sum(lens)
+    ins = {n: torch.randn(T, H, d, generator=g).to(dt).float() for n, d in (("q", D), ("k", D), ("v", Dv))}
+    ins["z"] = torch.randn(T, H, D, generator=g) + 2
+    run = lambda t, chunked: run_recurrence(t["q"], t["k"], t["v"], dt, lens, logits=t["z"], tau=16.0, chunked=chunked)
+    clean = run(ins, True)[0]
+    for at in (5, 63, 100):
+        bad = dict(ins, **{which: ins[which].clone()})
+        bad[which][at, 0, ::3] = -odd if which == "z" else odd
+        (o, s), (o_walk, s_walk) = run(bad, True), run(bad, False)
+        assert torch.equal(o[:at], clean[:at]) and torch.equal(o[lens[0]:], clean[lens[0]:]), at
+        assert torch.equal(o.isfinite(), o_walk.isfinite()) and torch.equal(s.isfinite(), s_walk.isfinite()), at

@@ -545,3 +545,31 @@ def test_prompts_over_low_rank_rows_do_not_see_what_an_earlier_owner_left_in_a_p
             got.append(kernels.attention_latent_prompt(q, H * width, H, width, rank, pool, table, table.shape[1], None, width ** -0.5, ctx))
         kernels.check_status(torch.device("cuda", torch.cuda.current_device()))
         assert torch.equal(*got), (n, start)
+
+
+@pytest.mark.parametrize("odd", [float("nan"), float("inf")])
+@pytest.mark.parametrize("which", ["x", "B", "C"])
+def test_a_token_that_is_no_number_does_not_reach_back(which, odd):
+    """The state-space recurrence in chunks against the walk: what comes before the token is bit for bit what it is without it, and what
+    comes behind is lost in the same places."""
+    from pico_engine.ops import kernels
+    H, P, N, G, lens = 2, 68, 32, 1, [130, 40]                                        # (no padding rows, whose zeros the walk multiplies too)
+    g = torch.Generator().manual_seed(6)
+    T, inner = sum(lens), H * P
+    xbc, dt_raw = torch.randn(T, inner + 2 * G * N, generator=g), torch.randn(T, H, generator=g)
+    first, rows, slots = (torch.tensor(v, dtype=torch.int32).cuda() for v in ([0, lens[0], T], lens, [0, 1]))
+
+    def run(rows_in, chunked):
+        state = torch.zeros(2, kernels.state_space_elems(H, P, N)).cuda()
+        y = kernels.state_space_scan(rows_in.cuda(), dt_raw.cuda(), 0, torch.zeros(H).cuda(), torch.full((H,), -3.0).cuda(), torch.ones(H).cuda(),
+                                     state, 0, first, rows, slots, H, P, N, G, chunked=chunked)
+        return y.cpu(), state.cpu()
+
+    clean = run(xbc, True)[0]
+    column = {"x": 3, "B": inner + 1, "C": inner + G * N + 1}[which]
+    for at in (5, 63, 100):
+        bad = xbc.clone()
+        bad[at, column] = odd
+        (y, s), (y_walk, s_walk) = run(bad, True), run(bad, False)
+        assert torch.equal(y[:at], clean[:at]) and torch.equal(y[lens[0]:], clean[lens[0]:]), at
+        assert torch.equal(y.isfinite(), y_walk.isfinite()) and torch.equal(s.isfinite(), s_walk.isfinite()), at
