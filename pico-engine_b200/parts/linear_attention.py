@@ -100,10 +100,11 @@ class LinearAttention(Mixer, SharedProducts):
         if self.w_a1 is not None:
             if rows[0] is None and not kernels.fused_takes(proj.shape[0], self.w_a1, rows[1]):
                 rows = (x_norm[1].forward(x_norm[0], ctx.dtype), None, None, 0.0)
-            # The decode product and the library's product without a bias give their float32 sums; the library's with a bias comes rounded
-            # to the rows' dtype, and is read as it is.
+            # Products give their float32 sums; only the library's with a bias (bfloat16 rows and weights that the decode product does not
+            # take) comes rounded to bfloat16, and is read as it is.
             a1 = first_product(*rows, self.w_a1, ctx)
-            rounded = self.b_a2 is not None and not kernels.fused_takes(a1.shape[0], self.w_a2, a1)
+            rounded = (self.b_a2 is not None and a1.dtype == self.w_a2.dtype == torch.bfloat16
+                       and not kernels.fused_takes(a1.shape[0], self.w_a2, a1))
             logits = linear(a1, self.w_a2, self.b_a2, out_dtype=None if rounded else torch.float32)
         turned = None
         if s.position is not None:

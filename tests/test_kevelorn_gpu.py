@@ -545,3 +545,34 @@ def test_a_token_that_is_no_number_does_not_reach_back(which, dtype, odd):
         (o, s), (o_walk, s_walk) = run(bad, True), run(bad, False)
         assert torch.equal(o[:at], clean[:at]) and torch.equal(o[lens[0]:], clean[lens[0]:]), at
         assert torch.equal(o.isfinite(), o_walk.isfinite()) and torch.equal(s.isfinite(), s_walk.isfinite()), at
+
+
+def test_decay_logits_keep_their_digits_where_a_weight_is_stored_in_32_bits(tmp_path, monkeypatch):
+    """The bfloat16 engine keeps such a weight as it is and multiplies in float32: the logits reach the recurrence as the product's float32
+    sums, in prompts and in single tokens, and are the product of the rows they were made of."""
+    from pico_engine.engine.engine import Engine
+    from pico_engine.ops import kernels
+    from pico_engine.parts import linear_attention as part
+    cfg = CONFIGS["K1"]
+    weights = make_weights(cfg, 40, RANKS["K1"])
+    names = [n for n in weights if n.endswith(".a2")]
+    for n in names:
+        weights[n] = weights[n] + 2.0 ** -12 * torch.randn(weights[n].shape, generator=torch.Generator().manual_seed(1))
+    eng = Engine(write_model(tmp_path / "m", cfg, weights, float32_names=names), dtype="bfloat16")
+    products, logits = [], []
+    linear, attend = part.linear, kernels.linear_attention
+    def spy_linear(a, w, bias=None, **kw):                                             # noqa: E306
+        if w.dtype == torch.float32:
+            products.append(a.double() @ w.double().T + bias.double())
+        return linear(a, w, bias, **kw)
+    def spy_attend(*a, decay_logits=None, **kw):                                       # noqa: E306
+        if decay_logits is not None:
+            logits.append(decay_logits)
+        return attend(*a, decay_logits=decay_logits, **kw)
+    monkeypatch.setattr(part, "linear", spy_linear)
+    monkeypatch.setattr(kernels, "linear_attention", spy_attend)
+    replay.run_in_process(eng, replay.tail(requests_for(cfg, [70], 1), 3))
+    assert len(products) == len(logits) == 4 * 3                                       # four steps, a layer that runs three times in each
+    for got, want in zip(logits, products):
+        # float32 sums of a rank's few products
+        assert got.dtype == torch.float32 and float((got.double() - want).abs().max()) < 1e-5 * max(1.0, float(want.abs().max()))
