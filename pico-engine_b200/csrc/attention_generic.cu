@@ -81,7 +81,8 @@ __global__ void __launch_bounds__(AG_THREADS) attention_generic_kernel(
 // ---------------------------------------------------------------------------- tiles of rows
 // A block: R rows, each a (token, query head); the rows of neighbouring tokens and of the heads that share a key/value head, so that a
 // page is read once for all of them.  A step is a page: thread (ty, tx) of 16 x 16 has the scores of R / 16 rows and four keys, then
-// R / 16 rows and hd / 16 columns of the outputs.  Tokens of several sequences in a block are served one sequence after the other.
+// R / 16 rows and hd / 16 columns of the outputs.  Tokens of several sequences in a block are served one after the other, each run of
+// neighbouring tokens of one sequence by itself (tokens of two sequences may come in any order).
 // Whatever R is, a row's scores are sums over the entries in order, its weights are added in the same tree, its outputs in the order of
 // the keys: R = 16 (single tokens) and R = 64 (prompts) give the same bits.  A key that a row does not see adds nothing to it, not even
 // a value that is no number.  Bound by float32 multiply-adds and the reads from shared memory that feed them.  Two layers' attention of
@@ -149,11 +150,11 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tile_kernel(AttentionTil
     __syncthreads();
     float m[RT], l[RT];
     float4 acc[RT][NJ];
-    int my_pos[RT], my_seq[RT];
+    int my_pos[RT];
 #pragma unroll
     for (int i = 0; i < RT; ++i) {
         m[i] = -INFINITY; l[i] = 0.f;
-        my_pos[i] = pos_s[ty * RT + i]; my_seq[i] = seq_s[ty * RT + i];
+        my_pos[i] = pos_s[ty * RT + i];
 #pragma unroll
         for (int j = 0; j < NJ; ++j) acc[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
@@ -174,7 +175,7 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tile_kernel(AttentionTil
         }
     };
     auto turn = [&](int j, int c, const float4& k) { kt[ag_turned(c, j)] = k.x; kt[ag_turned(c + 1, j)] = k.y; kt[ag_turned(c + 2, j)] = k.z; kt[ag_turned(c + 3, j)] = k.w; };
-    for (int from = 0; from < rows;) {                     // the rows of one sequence after the other
+    for (int from = 0; from < rows;) {                     // the rows of one sequence that stand together, after them the next ones
         const int seq = seq_s[from];
         int to = from + n_heads, lowest = pos_s[from], highest = lowest;
         while (to < rows && seq_s[to] == seq) { lowest = min(lowest, pos_s[to]); highest = max(highest, pos_s[to]); to += n_heads; }
@@ -231,7 +232,8 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tile_kernel(AttentionTil
             bool whole = true;                             // this thread's rows see the whole page
 #pragma unroll
             for (int i = 0; i < RT; ++i) {
-                const int hi = my_seq[i] == seq ? my_pos[i] - key0 : -1, lo = a.window > 0 ? hi - a.window + 1 : 0;      // keys lo .. hi of the four
+                const bool mine = ty * RT + i >= from && ty * RT + i < to;
+                const int hi = mine ? my_pos[i] - key0 : -1, lo = a.window > 0 ? hi - a.window + 1 : 0;      // keys lo .. hi of the four
                 s[i].x = hi >= 0 && lo <= 0 ? s[i].x * a.scale : -INFINITY;
                 s[i].y = hi >= 1 && lo <= 1 ? s[i].y * a.scale : -INFINITY;
                 s[i].z = hi >= 2 && lo <= 2 ? s[i].z * a.scale : -INFINITY;
@@ -245,14 +247,14 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tile_kernel(AttentionTil
                 float sum = (s[i].x + s[i].y) + (s[i].z + s[i].w);
 #pragma unroll
                 for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-                if (my_seq[i] == seq) {
+                if (mine) {
                     l[i] = l[i] * alpha + sum;
                     m[i] = m_new;
 #pragma unroll
                     for (int j = 0; j < NJ; ++j) { acc[i][j].x *= alpha; acc[i][j].y *= alpha; acc[i][j].z *= alpha; acc[i][j].w *= alpha; }
                 }
                 const int first_key = pg * PE_PAGE;
-                whole = whole && my_seq[i] == seq && my_pos[i] >= first_key + PE_PAGE - 1 && (a.window <= 0 || my_pos[i] - first_key < a.window);
+                whole = whole && mine && my_pos[i] >= first_key + PE_PAGE - 1 && (a.window <= 0 || my_pos[i] - first_key < a.window);
             }
 #pragma unroll
             for (int e = 0; e < 4; ++e) {

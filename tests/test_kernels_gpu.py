@@ -258,6 +258,26 @@ def test_attention_decode(K, nh, nkv, hd, lens, window, max_context):
     assert torch.equal(late, got)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nh,nkv,hd,window", [(14, 2, 64, None), (3, 3, 40, 70), (4, 1, 256, None)])
+def test_attention_generic_takes_tokens_in_any_order(K, nh, nkv, hd, window, dtype):
+    """Two sequences' tokens in turn, in runs of unequal length and backwards: the same bits as one sequence after the other."""
+    lens = [150, 90]
+    paged = Paged(lens, nkv, hd, dtype, seed=hd)
+    kp, vp, table = paged.cuda()
+    tokens = [(b, p) for b, n in enumerate(lens) for p in range(n)]
+    q = rnd(len(tokens), nh * hd, seed=nh).to(dtype)
+    i32 = lambda v: dev(torch.tensor(v, dtype=torch.int32))                          # noqa: E731
+    run = lambda order: K.attention_generic(dev(q[order].contiguous()), nh * hd, nh, nkv, hd, kp, vp, table, table.shape[1], i32([tokens[j][1] for j in order]),
+                                            i32([tokens[j][0] for j in order]), window, hd ** -0.5)
+    n = len(tokens)
+    want = run(list(range(n)))
+    in_turn = sorted(range(n), key=lambda j: (tokens[j][1], tokens[j][0]))
+    runs = sorted(range(n), key=lambda j: (tokens[j][1] // (3 + 4 * tokens[j][0]), tokens[j][0]))
+    for order in (in_turn, runs, list(range(n))[::-1]):
+        assert torch.equal(run(order), want[order])
+
+
 SHAPE_CASES = [                       # (nh, nkv, hd, sequences, longest, bound on the context): the lines between launch shapes
     (14, 2, 64, 1, 700, 2048), (14, 2, 64, 1, 700, 2112),             # 4 warps up to two pages a range, 8 behind
     (14, 2, 64, 24, 128, 128), (2, 1, 16, 8, 300, 300),
