@@ -175,24 +175,25 @@ __global__ void __launch_bounds__(256) la_carry_kernel(LAArgs a) {
     if (e >= per) return;
     int base = 0;
     for (int i = 0; i < b; ++i) base += (a.row_lens[i] + LA_CHUNK - 1) / LA_CHUNK;
-    const int nc = (a.row_lens[b] + LA_CHUNK - 1) / LA_CHUNK;
-    if (nc == 0) return;
+    // the sequence's chunks of this slab, by their places in it
+    const int begin = max(base - a.first_chunk, 0), end = min(base + (a.row_lens[b] + LA_CHUNK - 1) / LA_CHUNK - a.first_chunk, a.slab);
+    if (begin >= end) return;
     const size_t hd = e / a.Dv;                                              // (head, channel)
     float* sp = a.state + (size_t)a.slots[b] * a.state_stride + e;
     float carry = *sp;
     // Eight chunks' contributions and decays are read at once (they do not depend on the carry): one read in flight a thread
     // would leave the memory system idle, a chunk's data being a megabyte away from the next one's.
-    for (int c0 = base; c0 < base + nc; c0 += 8) {
+    for (int c0 = begin; c0 < end; c0 += 8) {
         float own[8], dec[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-            const bool on = c0 + u < base + nc;
+            const bool on = c0 + u < end;
             own[u] = on ? a.chunk_state[(size_t)(c0 + u) * per + e] : 0.f;
             dec[u] = on ? a.chunk_decay[(size_t)(c0 + u) * a.H * a.D + hd] : 0.f;
         }
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-            if (c0 + u < base + nc) {
+            if (c0 + u < end) {
                 a.chunk_state[(size_t)(c0 + u) * per + e] = carry;
                 carry = fmaf(dec[u], carry, own[u]);
             }
@@ -202,7 +203,7 @@ __global__ void __launch_bounds__(256) la_carry_kernel(LAArgs a) {
 }
 
 template <typename T, typename TQ, typename TZ, int R, int NC, bool PC>
-static int la_run(const LAArgs& a, int chunked, cudaStream_t s) {
+static int la_run(LAArgs a, int chunked, cudaStream_t s) {
     const int tiles = (a.Dv + LA_COLS * NC - 1) / (LA_COLS * NC);
     if (!chunked) {
         PE_TRY(pe_launch(la_walk_kernel<T, TQ, TZ, R, NC, PC>, dim3(a.B, a.H, tiles), LA_THREADS, 0, s, a));
@@ -211,18 +212,16 @@ static int la_run(const LAArgs& a, int chunked, cudaStream_t s) {
     }
     const size_t per = (size_t)a.H * a.D * a.Dv;
     const dim3 carry((unsigned)((per + 255) / 256), a.B);
-    if constexpr (!PC) {
-        const int types = sizeof(T) == 4 ? 0 : sizeof(TQ) == 2 ? 1 : 2;
-        if (const int e = la_tiles_contributions(a, types, s)) return e;
+    constexpr int types = sizeof(T) == 4 ? 0 : sizeof(TQ) == 2 ? 1 : 2;
+    for (; a.first_chunk < a.chunks; a.first_chunk += a.slab) {      // (the carry between two slabs lies in the sequences' states)
+        if constexpr (PC) { if (const int e = la_channels_contributions(a, sizeof(T) == 4, sizeof(TZ) == 4, a.channel_scratch, s)) return e; }
+        else if (const int e = la_tiles_contributions(a, types, s)) return e;
         PE_TRY(pe_launch(la_carry_kernel, carry, 256, 0, s, a));
         PE_LAUNCH_CHECK();
-        return la_tiles_outputs(a, types, s);
-    } else {
-        if (const int e = la_channels_contributions(a, sizeof(T) == 4, sizeof(TZ) == 4, a.channel_scratch, s)) return e;
-        PE_TRY(pe_launch(la_carry_kernel, carry, 256, 0, s, a));
-        PE_LAUNCH_CHECK();
-        return la_channels_outputs(a, sizeof(T) == 4, a.channel_scratch, s);
+        if constexpr (PC) { if (const int e = la_channels_outputs(a, sizeof(T) == 4, a.channel_scratch, s)) return e; }
+        else if (const int e = la_tiles_outputs(a, types, s)) return e;
     }
+    return 0;
 }
 
 // Two columns a thread where the state is at least 64 columns wide and a thread's rows leave the registers for it.
@@ -238,9 +237,23 @@ static int la_by_rows(const LAArgs& a, int chunked, cudaStream_t s) {
 // Chunks a step of T tokens in B sequences can have at most.
 extern "C" int pe_linear_attention_chunks(int T, int B) { return (T + LA_CHUNK - 1) / LA_CHUNK + B; }
 
+// Chunks that are worked on at a time: as many as LA_SCRATCH_FLOATS of scratch hold (one at least), in slabs of equal size.  A slab of the
+// sizes that fill it keeps the GPU full (16 heads of 128 x 128 with a decay per channel: 109 chunks, 1,744 blocks a launch), and batches of
+// prompts need no more scratch than it.
+#define LA_SCRATCH_FLOATS (64ll << 20)
+static int la_slab(int chunks, int H, int D, int Dv, int per_channel) {
+    const long long floats = (long long)H * D * ((long long)Dv + 1) + (per_channel ? la_channels_scratch_floats(1, H, D) : 0);
+    const long long most = floats >= LA_SCRATCH_FLOATS ? 1 : LA_SCRATCH_FLOATS / floats, slabs = (chunks + most - 1) / most;
+    return (int)((chunks + slabs - 1) / slabs);
+}
+extern "C" int pe_linear_attention_slabs(int T, int B, int H, int D, int Dv, int per_channel) {
+    const int chunks = pe_linear_attention_chunks(T, B), slab = la_slab(chunks, H, D, Dv, per_channel);
+    return (chunks + slab - 1) / slab;
+}
 // Floats of scratch the chunked way needs.
 extern "C" long long pe_linear_attention_scratch_floats(int T, int B, int H, int D, int Dv, int per_channel) {
-    return (long long)pe_linear_attention_chunks(T, B) * H * D * ((long long)Dv + 1) + (per_channel ? 3 + la_channels_scratch_floats(pe_linear_attention_chunks(T, B), H, D) : 0);
+    const int slab = la_slab(pe_linear_attention_chunks(T, B), H, D, Dv, per_channel);
+    return (long long)slab * H * D * ((long long)Dv + 1) + (per_channel ? 3 + la_channels_scratch_floats(slab, H, D) : 0);
 }
 
 extern "C" int pe_linear_attention(const void* proj, int dtype, int ld, int q_off, int k_off, int v_off, const void* z, int z_dtype,
@@ -258,12 +271,14 @@ extern "C" int pe_linear_attention(const void* proj, int dtype, int ld, int q_of
     a.act_qk = act_qk; a.act_v = act_v; a.state = state; a.state_stride = state_stride;
     a.row_first = row_first; a.row_lens = row_lens; a.slots = slots; a.out = out;
     a.B = B; a.H = H; a.D = D; a.Dv = Dv;
-    a.max_chunks = pe_linear_attention_chunks(T, B);
-    a.chunk_state = scratch;
-    a.chunk_decay = scratch ? scratch + (size_t)a.max_chunks * H * D * Dv : nullptr;
-    a.channel_scratch = scratch ? scratch + ((size_t)a.max_chunks * H * D * ((size_t)Dv + 1) + 3) / 4 * 4 : nullptr;      // (read in vectors)
-    cudaStream_t s = (cudaStream_t)stream;
     const bool pc = z != nullptr;
+    a.chunks = pe_linear_attention_chunks(T, B);
+    a.first_chunk = 0;
+    a.slab = la_slab(a.chunks, H, D, Dv, pc);
+    a.chunk_state = scratch;
+    a.chunk_decay = scratch ? scratch + (size_t)a.slab * H * D * Dv : nullptr;
+    a.channel_scratch = scratch ? scratch + ((size_t)a.slab * H * D * ((size_t)Dv + 1) + 3) / 4 * 4 : nullptr;      // (read in vectors)
+    cudaStream_t s = (cudaStream_t)stream;
     if (dtype == PE_F32) {
         if (!pc) return la_by_rows<float, float, float, false>(a, chunked, s);
         if (z_dtype == PE_F32) return la_by_rows<float, float, float, true>(a, chunked, s);

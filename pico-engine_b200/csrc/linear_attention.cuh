@@ -18,7 +18,8 @@ struct LAArgs {
     int B, H, D, Dv;
     float* chunk_state;      // [chunks, H, D, Dv]
     float* chunk_decay;      // [chunks, H, D]
-    int max_chunks;
+    int chunks;              // of the step, at most
+    int first_chunk, slab;   // those that this launch takes: from first_chunk on, `slab` of them at most
     float* channel_scratch;  // with a decay per channel: weights, decayed queries and keys of every chunk
 };
 

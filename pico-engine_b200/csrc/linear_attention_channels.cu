@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(LC_THREADS) lc_prepare_kernel(LAArgs a, float*
     float* at = kt + DP * LC_LD;                          // decays; one behind the chunk's tokens
     float* whole = at + DP * LC_LD;                       // [4][DP]: the product of each run's decays
     int row, first, n;
-    la_find_chunk(a.row_first, a.row_lens, a.B, blockIdx.x, row, first, n);
+    la_find_chunk(a.row_first, a.row_lens, a.B, a.first_chunk + blockIdx.x, row, first, n);
     if (n <= 0) return;
     // a lane a token: four channels are read as a run and stored to four rows, neighbouring lanes side by side
 #pragma unroll 2
@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(ST_THREADS) lc_contribution_kernel(LAArgs a, c
     __shared__ __align__(16) float ks[32 * 128], vs[32 * 64];
     const int tid = threadIdx.x, h = blockIdx.y, D = a.D, Dv = a.Dv, d0 = blockIdx.z % tiles_d * 128, c0 = blockIdx.z / tiles_d * 64;
     int row, first, n;
-    la_find_chunk(a.row_first, a.row_lens, a.B, blockIdx.x, row, first, n);
+    la_find_chunk(a.row_first, a.row_lens, a.B, a.first_chunk + blockIdx.x, row, first, n);
     if (n <= 0) return;
     const float* k_src = keys + ((size_t)blockIdx.x * a.H + h) * ST_CHUNK * D + d0;
     const T* v_src = (const T*)a.proj + (size_t)first * a.ld + a.v_off + h * Dv + c0;
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(ST_THREADS) lc_output_kernel(LAArgs a, const f
     __shared__ __align__(16) float smem[2 * ST_CHUNK * ST_CHUNK];       // two buffers of a slice of the queries and of S; then weights and values
     const int tid = threadIdx.x, h = blockIdx.y, D = a.D, Dv = a.Dv, c0 = blockIdx.z * 64;
     int row, first, n;
-    la_find_chunk(a.row_first, a.row_lens, a.B, blockIdx.x, row, first, n);
+    la_find_chunk(a.row_first, a.row_lens, a.B, a.first_chunk + blockIdx.x, row, first, n);
     if (n <= 0) return;
     int ty, tx;
     st_place(ty, tx);
@@ -333,26 +333,26 @@ long long la_channels_scratch_floats(int chunks, int H, int D) { return (long lo
 template <typename T, typename TZ>
 static int lc_prepare_and_contribute(const LAArgs& a, float* scratch, cudaStream_t s) {
     float* weights = scratch;
-    float* queries = weights + (size_t)a.max_chunks * a.H * ST_CHUNK * ST_CHUNK;
-    float* keys = queries + (size_t)a.max_chunks * a.H * ST_CHUNK * a.D;
+    float* queries = weights + (size_t)a.slab * a.H * ST_CHUNK * ST_CHUNK;
+    float* keys = queries + (size_t)a.slab * a.H * ST_CHUNK * a.D;
     const int DP = (a.D + 3) / 4 * 4, size = sizeof(T);
     const int vec_q = (uintptr_t)a.qk % (4 * size) == 0 && a.qk_ld % 4 == 0 && a.q_off % 4 == 0 && a.k_off % 4 == 0 && a.D % 4 == 0;
     const int vec_z = (uintptr_t)a.z % (4 * sizeof(TZ)) == 0 && a.z_ld % 4 == 0 && a.D % 4 == 0;
     const int vec_v = (uintptr_t)a.proj % (4 * size) == 0 && a.ld % 4 == 0 && a.v_off % 4 == 0 && a.Dv % 4 == 0;
     const size_t smem = sizeof(float) * ((size_t)3 * DP * LC_LD + 4 * DP);
     PE_TRY(cudaFuncSetAttribute(lc_prepare_kernel<T, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    PE_TRY(pe_launch(lc_prepare_kernel<T, TZ>, dim3(a.max_chunks, a.H), LC_THREADS, smem, s, a, weights, queries, keys, vec_q, vec_z));
+    PE_TRY(pe_launch(lc_prepare_kernel<T, TZ>, dim3(a.slab, a.H), LC_THREADS, smem, s, a, weights, queries, keys, vec_q, vec_z));
     PE_LAUNCH_CHECK();
     const int td = (a.D + 127) / 128, tv = (a.Dv + 63) / 64;
-    PE_TRY(pe_launch(lc_contribution_kernel<T>, dim3(a.max_chunks, a.H, td * tv), ST_THREADS, 0, s, a, (const float*)keys, vec_v, td));
+    PE_TRY(pe_launch(lc_contribution_kernel<T>, dim3(a.slab, a.H, td * tv), ST_THREADS, 0, s, a, (const float*)keys, vec_v, td));
     PE_LAUNCH_CHECK();
     return 0;
 }
 template <typename T>
 static int lc_outputs(const LAArgs& a, float* scratch, cudaStream_t s) {
     const int vec_v = (uintptr_t)a.proj % (4 * sizeof(T)) == 0 && a.ld % 4 == 0 && a.v_off % 4 == 0 && a.Dv % 4 == 0;
-    PE_TRY(pe_launch(lc_output_kernel<T>, dim3(a.max_chunks, a.H, (a.Dv + 63) / 64), ST_THREADS, 0, s, a, (const float*)scratch,
-                     (const float*)(scratch + (size_t)a.max_chunks * a.H * ST_CHUNK * ST_CHUNK), vec_v));
+    PE_TRY(pe_launch(lc_output_kernel<T>, dim3(a.slab, a.H, (a.Dv + 63) / 64), ST_THREADS, 0, s, a, (const float*)scratch,
+                     (const float*)(scratch + (size_t)a.slab * a.H * ST_CHUNK * ST_CHUNK), vec_v));
     PE_LAUNCH_CHECK();
     return 0;
 }

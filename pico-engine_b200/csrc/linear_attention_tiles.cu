@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(LT_THREADS) lt_contribution_kernel(LAArgs a, i
     int ty, tx, row, first, n;
     lt_place(ty, tx);
     const int d0 = (blockIdx.z % tiles_d) * TD, c0 = (blockIdx.z / tiles_d) * TV;
-    la_find_chunk(a.row_first, a.row_lens, a.B, blockIdx.x, row, first, n);
+    la_find_chunk(a.row_first, a.row_lens, a.B, a.first_chunk + blockIdx.x, row, first, n);
     if (n <= 0) return;
     LTRows<TQ, TD> k_rows;
     LTRows<T, TV> v_rows;
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(LT_THREADS, 2) lt_output_kernel(LAArgs a, int 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h = blockIdx.y, c0 = blockIdx.z * TV;
     int ty, tx, row, first, n;
     lt_place(ty, tx);
-    la_find_chunk(a.row_first, a.row_lens, a.B, blockIdx.x, row, first, n);
+    la_find_chunk(a.row_first, a.row_lens, a.B, a.first_chunk + blockIdx.x, row, first, n);
     if (n <= 0) return;
     LTRows<T, TV> v_rows;
     v_rows.load((const T*)a.proj + (size_t)first * a.ld + a.v_off + h * a.Dv + c0, a.ld, n, a.Dv - c0, vec_v);
@@ -279,7 +279,7 @@ static int lt_contributions(const LAArgs& a, cudaStream_t s) {
     const size_t smem = (size_t)LA_CHUNK * 16 * (RD + RV) * 4;
     auto kernel = lt_contribution_kernel<T, TQ, RD, RV>;
     PE_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    PE_TRY(pe_launch(kernel, dim3(a.max_chunks, a.H, td * tv), LT_THREADS, smem, s, a, td, lt_vec(a.qk, sizeof(TQ), a.qk_ld, a.q_off, a.k_off, a.D),
+    PE_TRY(pe_launch(kernel, dim3(a.slab, a.H, td * tv), LT_THREADS, smem, s, a, td, lt_vec(a.qk, sizeof(TQ), a.qk_ld, a.q_off, a.k_off, a.D),
                      lt_vec(a.proj, sizeof(T), a.ld, a.v_off, 0, a.Dv)));
     PE_LAUNCH_CHECK();
     return 0;
@@ -292,7 +292,7 @@ static int lt_outputs(const LAArgs& a, cudaStream_t s) {
     const size_t smem = ((size_t)DP * LA_CHUNK + LA_CHUNK * LA_CHUNK + LA_CHUNK * 16 * RV + (keys > rows ? keys : rows)) * 4;
     auto kernel = lt_output_kernel<T, TQ, RV>;
     PE_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    PE_TRY(pe_launch(kernel, dim3(a.max_chunks, a.H, tv), LT_THREADS, smem, s, a, DP, lt_vec(a.qk, sizeof(TQ), a.qk_ld, a.q_off, a.k_off, a.D),
+    PE_TRY(pe_launch(kernel, dim3(a.slab, a.H, tv), LT_THREADS, smem, s, a, DP, lt_vec(a.qk, sizeof(TQ), a.qk_ld, a.q_off, a.k_off, a.D),
                      lt_vec(a.proj, sizeof(T), a.ld, a.v_off, 0, a.Dv)));
     PE_LAUNCH_CHECK();
     return 0;

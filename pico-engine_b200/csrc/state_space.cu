@@ -170,10 +170,23 @@ extern "C" long long pe_state_space_elems(int H, int P, int N) {
     const int ns = pe_state_space_split(N);
     return (long long)H * ((N + ns - 1) / ns) * ns * P;
 }
-// Chunks a step of T tokens in B sequences can have at most, and the floats of scratch that the tiles need.
+// Chunks a step of T tokens in B sequences can have at most; those that are worked on at a time, as many as SS_SCRATCH_FLOATS of scratch
+// hold (one at least), in slabs of equal size; and the floats of scratch that a slab needs.  A slab of the sizes that fill it keeps the GPU
+// full (64 heads of 64 columns, 128 state rows: 125 chunks, 8,000 blocks a launch), and batches of prompts need no more scratch than it.
+#define SS_SCRATCH_FLOATS (64ll << 20)
 extern "C" int pe_state_space_chunks(int T, int B) { return (T + SS_CHUNK - 1) / SS_CHUNK + B; }
+static long long ss_chunk_floats(int H, int P, int N, int G) { return (long long)G * SS_CHUNK * SS_CHUNK + (long long)H * P * N + H; }
+static int ss_slab(int chunks, int H, int P, int N, int G) {
+    const long long floats = ss_chunk_floats(H, P, N, G), most = floats >= SS_SCRATCH_FLOATS ? 1 : SS_SCRATCH_FLOATS / floats;
+    const long long slabs = (chunks + most - 1) / most;
+    return (int)((chunks + slabs - 1) / slabs);
+}
+extern "C" int pe_state_space_slabs(int T, int B, int H, int P, int N, int G) {
+    const int chunks = pe_state_space_chunks(T, B), slab = ss_slab(chunks, H, P, N, G);
+    return (chunks + slab - 1) / slab;
+}
 extern "C" long long pe_state_space_scratch_floats(int T, int B, int H, int P, int N, int G) {
-    return (long long)pe_state_space_chunks(T, B) * ((long long)G * SS_CHUNK * SS_CHUNK + (long long)H * P * N + H);
+    return ss_slab(pe_state_space_chunks(T, B), H, P, N, G) * ss_chunk_floats(H, P, N, G);
 }
 
 // A sequence's tokens one after the other, from its stored state.
@@ -268,13 +281,14 @@ extern "C" int pe_state_space_scan(const float* xbc, int xbc_ld, const void* pro
     if (PT > P) PT = P;
     int threads = ((PT * NS + 31) / 32) * 32;
     ScanArgs a = {xbc, xbc_ld, proj, proj_ld, dt_off, dt_bias, dtb_dtype, a_log, al_dtype, d_skip, d_dtype, state, state_stride,
-                  row_first, row_lens, slots, y, B, H, P, N, G, NS, NR, NRP, PT, nullptr, nullptr, nullptr, 0};
+                  row_first, row_lens, slots, y, B, H, P, N, G, NS, NR, NRP, PT, nullptr, nullptr, nullptr, 0, 0, 0};
     if (dtype != PE_F32 && dtype != PE_BF16) return PE_ERR_UNSUPPORTED;
     if (chunked) {
-        a.max_chunks = pe_state_space_chunks(T, B);
+        a.chunks = pe_state_space_chunks(T, B);
+        a.slab = ss_slab(a.chunks, H, P, N, G);
         a.chunk_scores = scratch;
-        a.chunk_state = scratch + (size_t)a.max_chunks * G * SS_CHUNK * SS_CHUNK;
-        a.chunk_decay = a.chunk_state + (size_t)a.max_chunks * H * P * N;
+        a.chunk_state = scratch + (size_t)a.slab * G * SS_CHUNK * SS_CHUNK;
+        a.chunk_decay = a.chunk_state + (size_t)a.slab * H * P * N;
         return ss_tiles(a, dtype, (cudaStream_t)stream);
     }
     const size_t smem = sizeof(float) * ((size_t)SS_TOKENS * (2 * NS * NRP + PT) + 2 * SS_TOKENS);

@@ -15,7 +15,8 @@ struct ScanArgs {
     float* chunk_state;                       // [chunks][H][N][P]: a chunk's own contribution, then its incoming state
     float* chunk_decay;                       // [chunks][H]: the product of a chunk's decays
     float* chunk_scores;                      // [chunks][G][64 s][64 t]: C_t . B_s
-    int max_chunks;
+    int chunks;                               // of the step, at most
+    int first_chunk, slab;                    // those that a launch takes: from first_chunk on, `slab` of them at most
 };
 
 __device__ __forceinline__ float ss_silu(float v) { return v / (1.0f + expf(-v)); }

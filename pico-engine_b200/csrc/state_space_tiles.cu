@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(ST_THREADS) st_contribution_kernel(ScanArgs a,
     __shared__ double las[SS_CHUNK], half;
     const int tid = threadIdx.x, H = a.H, N = a.N, P = a.P, inner = H * P;
     int first, n;
-    st_find_chunk(a, blockIdx.x, first, n);
+    st_find_chunk(a, a.first_chunk + blockIdx.x, first, n);
     if (n <= 0) return;
     if ((int)blockIdx.y >= H) {
         if (blockIdx.z) return;
@@ -171,22 +171,23 @@ __global__ void __launch_bounds__(256) st_carry_kernel(ScanArgs a) {
     if (e >= per) return;
     int base = 0;
     for (int i = 0; i < b; ++i) base += (a.row_lens[i] + SS_CHUNK - 1) / SS_CHUNK;
-    const int nc = (a.row_lens[b] + SS_CHUNK - 1) / SS_CHUNK;
-    if (nc == 0) return;
+    // the sequence's chunks of this slab, by their places in it
+    const int begin = max(base - a.first_chunk, 0), end = min(base + (a.row_lens[b] + SS_CHUNK - 1) / SS_CHUNK - a.first_chunk, a.slab);
+    if (begin >= end) return;
     const int h = (int)(e / per_head), r = (int)(e % per_head) / a.P, p = (int)(e % per_head) % a.P;
     float* sp = a.state + (size_t)a.slots[b] * a.state_stride + (((size_t)h * a.NR + r % a.NR) * a.P + p) * a.NS + r / a.NR;
     float carry = *sp;
-    for (int c0 = base; c0 < base + nc; c0 += 8) {           // eight chunks' numbers in flight: they do not depend on the carry
+    for (int c0 = begin; c0 < end; c0 += 8) {           // eight chunks' numbers in flight: they do not depend on the carry
         float own[8], dec[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-            const bool there = c0 + u < base + nc;
+            const bool there = c0 + u < end;
             own[u] = there ? a.chunk_state[(size_t)(c0 + u) * per + e] : 0.f;
             dec[u] = there ? a.chunk_decay[(size_t)(c0 + u) * a.H + h] : 0.f;
         }
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-            if (c0 + u < base + nc) {
+            if (c0 + u < end) {
                 a.chunk_state[(size_t)(c0 + u) * per + e] = carry;
                 carry = fmaf(dec[u], carry, own[u]);
             }
@@ -205,7 +206,7 @@ __global__ void __launch_bounds__(ST_THREADS) st_output_kernel(ScanArgs a, int v
     __shared__ double las[SS_CHUNK], half;
     const int tid = threadIdx.x, H = a.H, N = a.N, P = a.P, inner = H * P, h = blockIdx.y, g = h / (H / a.G), p0 = blockIdx.z * 64;
     int first, n;
-    st_find_chunk(a, blockIdx.x, first, n);
+    st_find_chunk(a, a.first_chunk + blockIdx.x, first, n);
     if (n <= 0) return;
     int ty, tx;
     st_place(ty, tx);
@@ -293,16 +294,18 @@ __global__ void __launch_bounds__(ST_THREADS) st_output_kernel(ScanArgs a, int v
 }
 
 template <typename T>
-static int st_run(const ScanArgs& a, cudaStream_t s) {
+static int st_run(ScanArgs a, cudaStream_t s) {
     const bool rows = a.xbc_ld % 4 == 0 && (uintptr_t)a.xbc % 16 == 0;
     const int vec_x = rows && a.P % 4 == 0, vec_bc = rows && (a.H * a.P) % 4 == 0 && a.N % 4 == 0;
     const int tn = (a.N + 127) / 128, tp = (a.P + 63) / 64;
-    PE_TRY(pe_launch(st_contribution_kernel<T>, dim3(a.max_chunks, a.H + a.G, tn * tp), ST_THREADS, 0, s, a, vec_bc, vec_x, tn));
-    PE_LAUNCH_CHECK();
-    PE_TRY(pe_launch(st_carry_kernel, dim3((unsigned)(((size_t)a.H * a.N * a.P + 255) / 256), a.B), 256, 0, s, a));
-    PE_LAUNCH_CHECK();
-    PE_TRY(pe_launch(st_output_kernel<T>, dim3(a.max_chunks, a.H, tp), ST_THREADS, 0, s, a, vec_bc, vec_x));
-    PE_LAUNCH_CHECK();
+    for (; a.first_chunk < a.chunks; a.first_chunk += a.slab) {      // (the carry between two slabs lies in the sequences' states)
+        PE_TRY(pe_launch(st_contribution_kernel<T>, dim3(a.slab, a.H + a.G, tn * tp), ST_THREADS, 0, s, a, vec_bc, vec_x, tn));
+        PE_LAUNCH_CHECK();
+        PE_TRY(pe_launch(st_carry_kernel, dim3((unsigned)(((size_t)a.H * a.N * a.P + 255) / 256), a.B), 256, 0, s, a));
+        PE_LAUNCH_CHECK();
+        PE_TRY(pe_launch(st_output_kernel<T>, dim3(a.slab, a.H, tp), ST_THREADS, 0, s, a, vec_bc, vec_x));
+        PE_LAUNCH_CHECK();
+    }
     return 0;
 }
 

@@ -1054,8 +1054,8 @@ def linear_attention(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, n_h
     """o [T, H * Dv] float32 of S_t = diag(a_t) S_(t-1) + k_t v_t^T, o_t = S_t^T q_t per head, for q, k, v at columns
     ``q_off``, ``k_off``, ``v_off`` of proj [T, ld] (packed sequences).  The decay is ``head_decay`` [H] float32 (one constant
     a head) or sigmoid(``decay_logits`` [T, H * D], float32 or of proj's dtype)^``inv_tau`` (a number per key channel and token).  S [H, D, Dv] comes from
-    and returns to the sequences' float32 state at ``state_offset``.  ``chunked``: prompts, three launches over chunks of
-    the sequences; else token after token in one launch.  ``qk`` (float32 [T, ld2], with a decay per head): q and k are the columns
+    and returns to the sequences' float32 state at ``state_offset``.  ``chunked``: prompts, in slabs of chunks of the sequences, three
+    launches a slab (four with a decay per channel); else token after token in one launch.  ``qk`` (float32 [T, ld2], with a decay per head): q and k are the columns
     ``q_off`` and ``k_off`` of these rows instead (rotated ones, that are not rounded on their way into the recurrence)."""
     T, ld = proj.shape
     H, D, Dv = n_heads, head_dim, v_head_dim
@@ -1085,13 +1085,15 @@ def linear_attention(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, n_h
     ws = None
     if chunked:
         from .workspace import scratch
-        ws = scratch("linear_attention", 4 * lib.pe_linear_attention_scratch_floats(T, B, H, D, Dv, 0 if decay_logits is None else 1), proj.device).data_ptr()
+        sizes = (T, B, H, D, Dv, 0 if decay_logits is None else 1)
+        slabs = lib.pe_linear_attention_slabs(*sizes)
+        ws = scratch("linear_attention", 4 * lib.pe_linear_attention_scratch_floats(*sizes), proj.device).data_ptr()
     check(lib.pe_linear_attention(proj.data_ptr(), _code(proj, "proj"), ld, q_off, k_off, v_off, _ptr(decay_logits),
                                   0 if decay_logits is None else _code(decay_logits, "decay_logits"), H * D, _ptr(head_decay),
                                   float(inv_tau), float(q_scale), LA_ACTIVATIONS[qk_activation], LA_ACTIVATIONS[v_activation],
                                   sp, stride, row_first.data_ptr(), row_lens.data_ptr(), slots.data_ptr(), out.data_ptr(),
                                   T, B, H, D, Dv, 1 if chunked else 0, ws, _ptr(qk), qk_ld, stream_ptr()),
-          "linear_attention", (3 if decay_logits is None else 4) if chunked else 1)
+          "linear_attention", (3 if decay_logits is None else 4) * slabs if chunked else 1)
     return out
 
 
@@ -1309,7 +1311,7 @@ def state_space_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_offset: int, dt_b
     """y float32 [T, H * P] of S_t = exp(-exp(A_log) dt) S_(t-1) + dt B_t x_t^T, y_t = S_t^T C_t + D x_t with dt = softplus(raw + bias):
     x | B | C are the columns of ``xbc`` float32 [T, H*P + 2 G N], the raw step sizes columns ``dt_offset`` .. of proj.  The states
     come from and return to the sequences' float32 state at ``state_offset``.  ``chunked``: prompts, as products of tiles over chunks of 64
-    tokens (three launches: every chunk's contribution to the state, a carry pass, the outputs) instead of one walk a sequence; both give
+    tokens (in slabs of chunks, three launches each: every chunk's contribution to the state, a carry pass, the outputs) instead of one walk a sequence; both give
     the same numbers up to float32 rounding."""
     from .library import state_space
     T = xbc.shape[0]
@@ -1322,12 +1324,14 @@ def state_space_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_offset: int, dt_b
     ws = 0
     if chunked:
         from .workspace import scratch
-        ws = scratch("state_space_scan", 4 * state_space().pe_state_space_scratch_floats(T, slots.shape[0], H, P, N, G), xbc.device).data_ptr()
+        sizes = (T, slots.shape[0], H, P, N, G)
+        slabs = state_space().pe_state_space_slabs(*sizes)
+        ws = scratch("state_space_scan", 4 * state_space().pe_state_space_scratch_floats(*sizes), xbc.device).data_ptr()
     check(state_space().pe_state_space_scan(xbc.data_ptr(), xbc.shape[1], proj.data_ptr(), _code(proj, "proj"), proj.shape[1], dt_offset,
                                             dt_bias.data_ptr(), _code(dt_bias, "dt_bias"), a_log.data_ptr(), _code(a_log, "a_log"),
                                             d_skip.data_ptr(), _code(d_skip, "d_skip"), sp, stride, row_first.data_ptr(),
                                             row_lens.data_ptr(), slots.data_ptr(), y.data_ptr(), T, slots.shape[0], H, P, N, G,
-                                            1 if chunked else 0, ws, stream_ptr()), "state_space_scan", 3 if chunked else 1)
+                                            1 if chunked else 0, ws, stream_ptr()), "state_space_scan", 3 * slabs if chunked else 1)
     return y
 
 

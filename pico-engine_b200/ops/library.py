@@ -207,6 +207,8 @@ def gated() -> ctypes.CDLL:
         lib = build.load("gated", GATED_SOURCES)
         declare(lib, _GATED_SIGNATURES)
         lib.pe_set_pdl(0 if os.environ.get("PICO_ENGINE_PDL", "1") == "0" else 1)
+        lib.pe_linear_attention_slabs.argtypes = [I, I, I, I, I, I]
+        lib.pe_linear_attention_slabs.restype = c_int
         lib.pe_linear_attention_scratch_floats.argtypes = [I, I, I, I, I, I]
         lib.pe_linear_attention_scratch_floats.restype = c_longlong
         _gated = lib
@@ -227,6 +229,8 @@ def state_space() -> ctypes.CDLL:
         lib.pe_state_space_split.restype = c_int
         lib.pe_state_space_elems.argtypes = [I, I, I]
         lib.pe_state_space_elems.restype = c_longlong
+        lib.pe_state_space_slabs.argtypes = [I, I, I, I, I, I]
+        lib.pe_state_space_slabs.restype = c_int
         lib.pe_state_space_scratch_floats.argtypes = [I, I, I, I, I, I]
         lib.pe_state_space_scratch_floats.restype = c_longlong
         _state = lib

@@ -134,3 +134,15 @@ def test_layer_runs():
     assert plain.layer_runs({"layers": [0] * 4, "loop": {"start": 1, "stop": 3, "times": 2}}) == \
         [(0, None), (1, 0), (2, None), (1, 1), (2, None), (3, None)]
     assert plain.layer_runs({"layers": [0] * 2}) == [(0, None), (1, None)]
+
+
+@pytest.mark.parametrize("per_channel", [0, 1])
+def test_scratch_of_a_batch_of_prompts_is_bounded(per_channel):
+    """A recurrence in chunks takes a batch's chunks in slabs: 64 prompts of 2,048 tokens need no more scratch than a few prompts do."""
+    from pico_engine.ops.library import gated, state_space
+    for H, D in ((16, 128), (32, 128), (14, 64), (3, 250)):
+        one, many = (gated().pe_linear_attention_scratch_floats(2048 * n, n, H, D, D, per_channel) for n in (1, 64))
+        assert 0 < 4 * one <= 256 << 20 and 4 * many <= 256 << 20
+        assert gated().pe_linear_attention_slabs(2048, 1, H, D, D, per_channel) == 1 < gated().pe_linear_attention_slabs(2048 * 64, 64, H, D, D, per_channel)
+    assert 4 * state_space().pe_state_space_scratch_floats(2048 * 64, 64, 64, 64, 128, 2) <= 256 << 20
+    assert state_space().pe_state_space_slabs(2048, 1, 64, 64, 128, 2) == 1

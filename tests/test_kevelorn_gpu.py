@@ -576,3 +576,25 @@ def test_decay_logits_keep_their_digits_where_a_weight_is_stored_in_32_bits(tmp_
     for got, want in zip(logits, products):
         # float32 sums of a rank's few products
         assert got.dtype == torch.float32 and float((got.double() - want).abs().max()) < 1e-5 * max(1.0, float(want.abs().max()))
+
+
+@pytest.mark.parametrize("per_channel", [False, True])
+def test_chunks_in_slabs(per_channel):
+    """More chunks than the scratch holds at once, sequences that end on, before and behind the borders of slabs: chunks against the walk."""
+    from pico_engine.ops import kernels
+    from pico_engine.ops.library import gated
+    H, D, lens = 32, 128, [3000, 64, 1, 65, 4999]
+    T, B = sum(lens), len(lens)
+    assert gated().pe_linear_attention_slabs(T, B, H, D, D, int(per_channel)) > 1
+    g = torch.Generator("cuda").manual_seed(1)
+    proj = torch.randn(T, 3 * H * D, generator=g, device="cuda").bfloat16()
+    decay = {"decay_logits": 2 + torch.randn(T, H * D, generator=g, device="cuda")} if per_channel else {"head_decay": torch.linspace(0.5, 0.999, H, device="cuda")}
+    first, rows, slots = (torch.tensor(v, dtype=torch.int32).cuda() for v in (np.concatenate([[0], np.cumsum(lens)]), lens, range(B)))
+    got = []
+    for chunked in (False, True):
+        state = torch.ones(B, H * D * D, device="cuda")
+        got.append((kernels.linear_attention(proj, 0, H * D, 2 * H * D, H, D, D, state, 0, first, rows, slots, chunked, inv_tau=1 / 16, q_scale=D ** -0.5,
+                                             **decay), state))
+    for walk, chunks in zip(*got):
+        # float32 sums of the same products in another order (the bound of the tests above)
+        assert (walk - chunks).abs().max() < 2e-5 * max(1.0, float(walk.abs().max()))

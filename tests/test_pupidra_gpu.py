@@ -573,3 +573,23 @@ def test_a_token_that_is_no_number_does_not_reach_back(which, odd):
         (y, s), (y_walk, s_walk) = run(bad, True), run(bad, False)
         assert torch.equal(y[:at], clean[:at]) and torch.equal(y[lens[0]:], clean[lens[0]:]), at
         assert torch.equal(y.isfinite(), y_walk.isfinite()) and torch.equal(s.isfinite(), s_walk.isfinite()), at
+
+
+def test_state_space_chunks_in_slabs():
+    """More chunks than the scratch holds at once, sequences that end on, before and behind the borders of slabs: chunks against the walk."""
+    from pico_engine.ops import kernels
+    from pico_engine.ops.library import state_space
+    H, P, N, G, lens = 64, 64, 128, 2, [3000, 64, 1, 65, 4999]
+    T, B = sum(lens), len(lens)
+    assert state_space().pe_state_space_slabs(T, B, H, P, N, G) > 1
+    g = torch.Generator("cuda").manual_seed(2)
+    xbc, dt_raw = torch.randn(T, H * P + 2 * G * N, generator=g, device="cuda"), torch.randn(T, H, generator=g, device="cuda")
+    first, rows, slots = (torch.tensor(v, dtype=torch.int32).cuda() for v in (np.concatenate([[0], np.cumsum(lens)]), lens, range(B)))
+    got = []
+    for chunked in (False, True):
+        state = torch.ones(B, kernels.state_space_elems(H, P, N), device="cuda")
+        got.append((kernels.state_space_scan(xbc, dt_raw, 0, torch.full((H,), -3.0).cuda(), torch.linspace(-1, 1, H).cuda(), torch.ones(H).cuda(), state, 0,
+                                             first, rows, slots, H, P, N, G, chunked=chunked), state))
+    for walk, chunks in zip(*got):
+        # float32 sums of the same products in another order (the bound of the tests above)
+        assert (walk - chunks).abs().max() < 3e-5 * max(1.0, float(walk.abs().max()))
