@@ -504,8 +504,13 @@ struct AdVariant {
     }
 
     static int allow_smem(size_t smem) {
-        static size_t allowed = 48 * 1024 - 512;
+        static size_t allowed = 0;                           // 48 KB of an SM need no opt-in, the kernel's own variables among them
         static bool wide = false;
+        if (!allowed) {
+            cudaFuncAttributes own;
+            PE_TRY(cudaFuncGetAttributes(&own, attention_decode_kernel<WARPS, RANKED>));
+            allowed = 48 * 1024 - own.sharedSizeBytes;
+        }
         if (!wide) {                                         // clusters of more than 8 CTAs are an opt-in; if it is refused,
             cudaFuncSetAttribute(attention_decode_kernel<WARPS, RANKED>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);   // the
             cudaGetLastError();                              // occupancy query below answers 0 for them and fewer ranges are used
