@@ -380,6 +380,10 @@ __global__ void __launch_bounds__(32 * (AD_WARPS + 1), AD_CTAS(AD_WARPS)) attent
                         asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(kt + at), "r"(kr.x), "r"(kr.y), "r"(kr.z), "r"(kr.w) : "memory");
                         asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(vt + at), "r"(vr.x), "r"(vr.y), "r"(vr.z), "r"(vr.w) : "memory");
                     }
+                    // values behind it become zero: a page is taken as its last owner left it, and a weight of zero would not keep a value
+                    // that is no number out of the sums
+                    for (unsigned o = (unsigned)((pos - key0 + 1) * AD_HD * 2 + lane * 16); o < 16 * AD_HD * 2; o += 512)
+                        asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(vt + o), "r"(0u) : "memory");
                     __syncwarp();
                 }
                 ad_consume(acc, m_run, l_run, qf, kt, vt, key0, lo, pos, scale_log2e, g, t, keep_first, biased, bias);

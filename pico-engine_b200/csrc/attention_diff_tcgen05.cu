@@ -187,6 +187,8 @@ __global__ void __launch_bounds__(DT_THREADS, 1) attention_diff_tcgen05_kernel(c
             const int b = it & 1, st = it >> 1, s_at = st % DT_STAGES;
             if (!at_wait_warp(at_smem(&kv_full[s_at]), (unsigned)(st / DT_STAGES) & 1u)) { ok = false; break; }   // the loader's flags
             const bool there = (stage_flags[s_at] >> g) & 1u;
+            if (it + 2 == n_its)                                    // the first map's turn at the last step: P V of neither has read its values
+                at_clear_rows(kv_s + s_at * DT_STAGE_BYTES(VP) + 2 * DT_PANEL, VP, DT_PANEL, pos0 + n - (page_lo + 2 * st) * DT_KTILE, threadIdx.x - 64, DT_THREADS - 64);
             if (!at_wait_warp(at_smem(&s_full[b]), (unsigned)(it >> 1) & 1u)) { ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int key0 = (page_lo + 2 * st + g) * DT_KTILE;

@@ -38,8 +38,8 @@ __device__ __forceinline__ unsigned ap_smem(const void* p) { return (unsigned)__
 __device__ __forceinline__ unsigned ap_offset(int row, int chunk) {   // byte offset of a 16-byte chunk in a tile
     return (unsigned)(row * AP_HD * 2 + ((AP_SWIZZLE ? (chunk ^ (row & 7)) : chunk) << 4));
 }
-__device__ __forceinline__ void ap_cp16(unsigned dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+__device__ __forceinline__ void ap_cp16(unsigned dst, const void* src, int bytes = 16) {      // `bytes` 0 writes zeros
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void ap_ldmatrix(unsigned (&r)[4], unsigned addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -102,7 +102,8 @@ __global__ void __launch_bounds__(32 * AP_WARPS, AP_HD <= 64 ? 2 : 1) attention_
                 const int row = idx / AP_CHUNKS, chunk = idx % AP_CHUNKS;
                 const unsigned off = (AP_SPLIT * stage + h2) * tile_bytes + ap_offset(row, chunk);
                 ap_cp16(k_s + off, k_pool + base + (size_t)row * AP_HD + chunk * 8);
-                ap_cp16(v_s + off, v_pool + base + (size_t)row * AP_HD + chunk * 8);
+                // (values behind the run's last token are none of its sequence's: whatever they are, they stay out)
+                ap_cp16(v_s + off, v_pool + base + (size_t)row * AP_HD + chunk * 8, pi * AP_KTILE + row < pos0 + n ? 16 : 0);
             }
         }
         return there;

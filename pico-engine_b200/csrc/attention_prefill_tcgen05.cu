@@ -219,6 +219,11 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_prefill_tcgen05_kerne
 #pragma unroll
             for (int x = 0; x < 2; ++x) entry[x] = 2 * it + 4 + x < n_pages ? table[page_at(2 * it + 4 + x)] : -1;
             if (!at_wait_warp(at_smem(&s_full[b]), (unsigned)(it / AT_BUFFERS) & 1u)) { ok = false; break; }
+            if (it + 1 == n_steps && (pos0 + n) % AT_KTILE) {       // values behind the run's last token, in the second or the first of the step's pages
+                if (!at_wait_warp(at_smem(&v_full[it % AT_STAGES]), (unsigned)(it / AT_STAGES) & 1u)) { ok = false; break; }
+                at_clear_rows(kv_s + it % AT_STAGES * AT_STAGE_BYTES + AT_STAGE_BYTES / 2, AT_PANELS, 2 * AT_KTILE * 128,
+                              (n_pages - 1 - 2 * it) * AT_KTILE + (pos0 + n) % AT_KTILE, (threadIdx.x - 64) & 127, 128);
+            }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             unsigned raw[2 * AT_KTILE];
 #pragma unroll

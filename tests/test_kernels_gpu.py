@@ -278,6 +278,39 @@ def test_attention_generic_takes_tokens_in_any_order(K, nh, nkv, hd, window, dty
         assert torch.equal(run(order), want[order])
 
 
+@pytest.mark.parametrize("rubbish", [float("nan"), float("inf")])
+@pytest.mark.parametrize("nh,nkv,hd,window,keep", [(14, 2, 64, None, 0), (4, 1, 128, None, 0), (2, 2, 64, 100, 70), (6, 2, 48, None, 0), (4, 2, 16, 90, 0), (32, 1, 32, None, 0)])
+def test_attention_does_not_see_what_an_earlier_owner_left_in_a_page(K, nh, nkv, hd, window, keep, rubbish):
+    """Cache rows that no live sequence has written may hold anything: with numbers that are none in all of them, prompts and single tokens
+    that end on, before and behind the borders of pages, of runs and of tiles of keys give the same bits as with zeros."""
+    lens = [1, 15, 16, 64, 65, 127, 128, 300, 1000]
+    paged = Paged(lens, nkv, hd, torch.bfloat16, seed=hd)
+    q = dev(rnd(sum(lens), nh * hd, seed=nh).to(torch.bfloat16))
+    alone = torch.tensor([sum(lens[:b + 1]) - 1 for b in range(len(lens))])
+    got = []
+    for fill in (0.0, rubbish):
+        paged.k_pool.fill_(fill); paged.v_pool.fill_(fill)
+        paged.write()
+        kp, vp, table = paged.cuda()
+        outs = [K.attention_decode(q[alone.cuda()].contiguous(), nh * hd, nh, nkv, hd, kp, vp, table, table.shape[1],
+                                   dev(torch.tensor([n - 1 for n in lens], dtype=torch.int32)), dev(torch.arange(len(lens), dtype=torch.int32)),
+                                   window, hd ** -0.5, max(lens), keep_first=keep)]
+        for start in ([0] * len(lens), [n // 2 for n in lens]):
+            rows = torch.cat([torch.arange(sum(lens[:b]) + a, sum(lens[:b + 1])) for b, a in enumerate(start)])
+            new = [n - a for n, a in zip(lens, start)]
+            part = q[rows.cuda()].contiguous()
+            if not keep:
+                outs.append(K.attention_prefill(part, nh * hd, nh, nkv, hd, kp, vp, table, table.shape[1], K.prefill_tiles(new, start, "cuda"),
+                                                len(rows), window, hd ** -0.5))
+            if K.attention_prefill_tcgen05_takes(hd, hd ** -0.5):
+                outs.append(K.attention_prefill_tcgen05(part, nh * hd, nh, nkv, hd, kp, vp, table, table.shape[1],
+                                                        K.prefill_tiles(new, start, "cuda", K.PREFILL_TILE_TCGEN05), len(rows), window, hd ** -0.5, keep_first=keep))
+        got.append(outs)
+    K.check_status("cuda")
+    for i, (clean, other) in enumerate(zip(*got)):
+        assert torch.equal(clean, other), i
+
+
 SHAPE_CASES = [                       # (nh, nkv, hd, sequences, longest, bound on the context): the lines between launch shapes
     (14, 2, 64, 1, 700, 2048), (14, 2, 64, 1, 700, 2112),             # 4 warps up to two pages a range, 8 behind
     (14, 2, 64, 24, 128, 128), (2, 1, 16, 8, 300, 300),

@@ -217,7 +217,7 @@ def test_identity_experts_gates_and_lambdas_count(models, tmp_path):
 
 # ------------------------------------------------------------------ differential attention alone
 
-def run_maps(q, k, v, dt, spans, window, scale, lam, diff, eps, side_col=0, pad_cols=0, first_page=1):
+def run_maps(q, k, v, dt, spans, window, scale, lam, diff, eps, side_col=0, pad_cols=0, first_page=1, unwritten=0.0):
     """``kernels.attention_maps`` for the query positions of ``spans`` (each a step of one sequence); q [n, H, 2, D], k [n, G, 2, D], v [n, G, Dv].
     Returns (heads [n, H, Dv], the columns beside them)."""
     from pico_engine.ops import kernels
@@ -225,8 +225,8 @@ def run_maps(q, k, v, dt, spans, window, scale, lam, diff, eps, side_col=0, pad_
     G, Dv = k.shape[1], v.shape[2]
     per = H // G
     pages = (n + 63) // 64
-    kp = torch.zeros(pages + first_page, 2 * G, 64, D, dtype=dt)
-    vp = torch.zeros(pages + first_page, G, 64, Dv, dtype=dt)
+    kp = torch.full((pages + first_page, 2 * G, 64, D), unwritten, dtype=dt)
+    vp = torch.full((pages + first_page, G, 64, Dv), unwritten, dtype=dt)
     for p in range(n):
         kp[first_page + p // 64, :, p % 64] = k[p].reshape(2 * G, D).to(dt)
         vp[first_page + p // 64, :, p % 64] = v[p].to(dt)
@@ -478,3 +478,16 @@ def test_activation_into_the_side_rows(dtype, T, E, F, S, gated):
             f = torch.zeros(T).double() if grp == 0 else f * weights[:, grp].double()
         assert (out[:, out_col + c].double() - f).abs().max() < (1e-5 if dtype == "float32" else 2e-2) * max(1.0, float(f.abs().max())), c
     assert torch.equal(out[:, :out_col], torch.full((T, out_col), 7.0)) and torch.equal(out[:, out_col + I:], torch.full_like(out[:, out_col + I:], 7.0))
+
+
+@pytest.mark.parametrize("rubbish", [float("nan"), float("inf")])
+@pytest.mark.parametrize("H,G,D,Dv,window", [(4, 2, 64, 128, None), (3, 1, 64, 64, 70), (17, 1, 80, 136, 64)])
+def test_differential_attention_does_not_see_what_an_earlier_owner_left_in_a_page(H, G, D, Dv, window, rubbish):
+    """Cache rows that no live sequence has written may hold anything: with numbers that are none in all of them, prompts and single tokens
+    that end on, before and behind the borders of pages and of runs give the same bits as with zeros."""
+    g = torch.Generator().manual_seed(H)
+    for n in (1, 37, 64, 127, 129, 300):
+        q, k, v = torch.randn(n, H, 2, D, generator=g), torch.randn(n, G, 2, D, generator=g), torch.randn(n, G, Dv, generator=g)
+        for spans in ([(0, n)], [(0, n // 2), (n // 2, n)] if n > 1 else [], [(n - 1, n)]):
+            clean, other = (run_maps(q, k, v, torch.bfloat16, spans, window, D ** -0.5, 0.4, 0.3, 1e-5, unwritten=fill)[0] for fill in (0.0, rubbish))
+            assert torch.equal(clean, other), (n, spans)
