@@ -429,3 +429,49 @@ def test_headmix_prompts_do_not_see_what_an_earlier_owner_left_in_a_page(H, G, D
             got.append(kernels.attention_headmix(q, H * D, H, G, D, Dv, kp, vp, table, table.shape[1], pos, row, None, D ** -0.5, sink, talk, ctx))
         kernels.check_status(torch.device("cuda", torch.cuda.current_device()))
         assert torch.equal(*got), (n, start)
+
+
+def rising(n, H, G, D, g):
+    """Queries and keys whose scores (scale 1) rise by 12 from one 128 keys to the next, beside noise: the largest of a row moves on in
+    every step of the keys, by more than the reference point of its exponentials stands still for."""
+    q, k = 0.1 * torch.randn(n, H, D, generator=g), 0.1 * torch.randn(n, G, D, generator=g)
+    q[:, :, 5] = 2.0
+    k[:, :, 5] = 6.0 * torch.arange(n)[:, None] / 128
+    return q, k
+
+
+@pytest.mark.parametrize("H,G,D,Dv", [(4, 2, 64, 64), (16, 4, 128, 128), (20, 2, 64, 64)])
+def test_headmix_prompts_of_many_steps(H, G, D, Dv):
+    """1,100 tokens, more steps of 128 keys than the ring has stages, at sizes that the tcgen05 kernel takes: one key that the last queries
+    match, wherever it lies (the first positions, the borders of pages and of steps, late ones), and scores that rise from step to step,
+    so that the outputs are rescaled every time."""
+    from pico_engine.ops.library import mixers
+    assert mixers().pe_attention_headmix_tcgen05_takes(H, G, D, Dv)
+    n, dt = 1100, torch.bfloat16
+    g = torch.Generator().manual_seed(H)
+    talk = torch.eye(H).roll(1, 0).double()
+    sink = torch.full((H,), -2.0).double()
+    v0 = torch.randn(n, G, Dv, generator=g)
+
+    def attend(q, k, v, window=None):
+        i, j = torch.arange(n)[:, None], torch.arange(n)[None]
+        seen = (j <= i) if window is None else (j <= i) & (i - j < window)
+        kk, vv = (t.repeat_interleave(H // G, 1) for t in (k, v))
+        s = torch.einsum("ihd,jhd->hij", q, kk).masked_fill(~seen, float("-inf"))
+        w = torch.softmax(torch.cat([s, sink.view(H, 1, 1).expand(H, n, 1)], -1), -1)[..., :n]
+        return torch.einsum("hij,jhd->ihd", torch.einsum("hg,gij->hij", talk, w), vv)
+
+    for far in (0, 63, 64, 127, 128, 511, 512, 767, 1000):
+        q, k, v = 0.1 * torch.randn(n, H, D, generator=g), 0.1 * torch.randn(n, G, D, generator=g), v0.clone()
+        mark = torch.zeros(D); mark[3] = 6.0
+        k[far], q[-5:], v[far] = mark, mark, 50.0
+        q, k, v = rounded(q, dt), rounded(k, dt), rounded(v, dt)
+        want = attend(q, k, v)
+        assert float(want[-1].min()) > 49
+        # (the bound of the tests above: a value of 50 rounded to bfloat16)
+        assert (run_headmix(q, k, v, 1.0, sink, talk, None, dt) - want).abs().max() < 0.3, far
+    q, k = rising(n, H, G, D, g)
+    q, k, v = rounded(q, dt), rounded(k, dt), rounded(v0, dt)
+    for window in (None, 200):
+        want = attend(q, k, v, window)
+        assert (run_headmix(q, k, v, 1.0, sink, talk, window, dt) - want).abs().max() < 1.5e-2 * max(1.0, float(want.abs().max())), window

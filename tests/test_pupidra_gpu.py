@@ -593,3 +593,39 @@ def test_state_space_chunks_in_slabs():
     for walk, chunks in zip(*got):
         # float32 sums of the same products in another order (the bound of the tests above)
         assert (walk - chunks).abs().max() < 3e-5 * max(1.0, float(walk.abs().max()))
+
+
+@pytest.mark.parametrize("H,width,rank", [(3, 256, 192), (2, 96, 64)])
+def test_prompts_of_many_steps_over_low_rank_rows(H, width, rank):
+    """1,100 tokens, several rounds of the tcgen05 kernel's ring: one key that the last queries match, wherever it lies (the first
+    positions, the borders of pages and of steps of 128 keys, late ones), and scores that rise from step to step, so that the outputs are
+    rescaled every time."""
+    from pico_engine.ops.library import state_space
+    assert state_space().pe_attention_latent_tcgen05_takes(width, rank)
+    n, dt = 1100, torch.bfloat16
+    g = torch.Generator().manual_seed(H)
+
+    def check(q, k, window):
+        i, j = torch.arange(n)[:, None], torch.arange(n)[None]
+        seen = (j <= i) if window is None else (j <= i) & (i - j < window)
+        w = torch.softmax(torch.einsum("ihd,jd->hij", q.double(), k[:, 0].double()).masked_fill(~seen, float("-inf")), -1)
+        want = torch.einsum("hij,jd->ihd", w, k[:, 0, :rank].double())
+        kp, table = paged(k, dt)
+        got = run_attention(q, kp, None, table, dt, [(0, n)], window, 0, 1.0, None, rank, True)
+        # weights and results are rounded to bfloat16, as in the tests above
+        assert (got.double() - want).abs().max() < 2e-2 * max(1.0, float(want.abs().max()))
+        return want
+
+    noise = lambda *s: (0.02 * torch.randn(*s, generator=g)).to(dt).float()               # noqa: E731
+    for far in (0, 63, 64, 127, 128, 511, 512, 767, 1000):
+        q, k = noise(n, H, width), torch.randn(n, 1, width, generator=g).to(dt).float()
+        k[:, :, rank:] = 0
+        q[-5:] = 0
+        q[-5:, :, -1] = k[far, :, -1] = 6.0
+        k[far, :, :rank] = 8.0
+        assert float(check(q, k, None)[-1].min()) > 7.9, far
+    q, k = noise(n, H, width), torch.randn(n, 1, width, generator=g).to(dt).float()
+    q[:, :, -1] = 2.0
+    k[:, 0, -1] = (6.0 * torch.arange(n) / 128).to(dt).float()                             # 12 more with every 128 keys
+    for window in (None, 200):
+        check(q, k, window)
