@@ -113,19 +113,41 @@ class LinearAttention(Mixer, SharedProducts):
         return kernels.gated_norm(o, vo if s.norm_over == "heads" else s.v_head_dim, self.norm, s.norm_eps, proj, 2 * qk + vo,
                                   s.gate_activation, ctx.dtype)
 
+    def chunks_pay(self, lens) -> bool:
+        """Whether a step with these numbers of tokens a row runs its recurrence as products of tiles over chunks of 64 tokens, or walks it
+        token after token; either way gives the same numbers up to float32 rounding.
+
+        A walk is a block a row, head and 64 (or 32) columns: it takes as long as the longest row, and as all rows' tokens take where there
+        are more blocks than run side by side.  Tiles cost four launches, every chunk its products whatever it holds, and every row the pass that
+        carries its state.  The numbers (for microseconds on a B200) are fitted so that the two cross where they were measured to, for 1 to 64 rows of 8
+        to 2,048 tokens: with a decay per channel, 16 heads of 128 x 128, walk / tiles: 1 x 17 tokens 10 / 51 us, 1 x 128 53 / 61, 1 x 256
+        103 / 69, 1 x 2,048 841 / 182; 4 x 128 70 / 88, 4 x 256 137 / 103; 64 x 17 102 / 600, 64 x 256 1,250 / 1,684, 63 single tokens beside
+        2,048 1,259 / 722.  With a decay per head: 1 x 128 39 / 52, 1 x 256 74 / 53; 64 x 17 77 / 499, 63 x 1 and 2,048 906 / 591."""
+        longest = max(lens, default=0)
+        if longest <= 16:                                                     # (the walk wherever it was measured)
+            return False
+        tokens, rows, chunks = sum(lens), sum(n > 0 for n in lens), sum((n + 63) // 64 for n in lens)
+        s = self.spec
+        H, D, Dv = s.n_heads, s.head_dim, s.v_head_dim
+        held = 8 if D <= 64 else 16 if D <= 128 else 32                       # state rows a thread of the walk keeps
+        blocks = H * -(-Dv // (64 if Dv >= 64 and D <= 128 else 32))
+        if self.head_decay is None:
+            walk = 2.6 + (0.042 + 0.031 * held) * max(longest, 0.53 * tokens * blocks / 148)
+            tiles = 24.6 + 0.277 * D + H * (chunks * (0.044 + 1.0e-5 * D * Dv) + rows * 1.84e-5 * D * Dv)
+        else:
+            walk = 2.4 + (0.060 + 0.0215 * held) * max(longest, 0.455 * tokens * blocks / 148)
+            tiles = 19.0 + 0.26 * D + H * (chunks * 8.6e-6 * D * Dv + rows * 1.3e-5 * D * Dv)
+        return tiles < walk
+
     def mixed_rows(self, proj, col, turned, ctx, cache_entry, owns_cache, logits=None):
         s = self.spec
         qk, vo = self._sizes()
-        # Prompts run as products of tiles over chunks of 64 tokens; rows that bring a few tokens walk them.  (Either way gives the same
-        # numbers up to float32 rounding.)  A walk takes as long as the longest row
-        # whatever it leaves idle; a chunk costs its tiles even where it holds a few tokens.
-        chunked = any(n > 16 for n in ctx.lens)
         # (keys that are scaled but not turned: the scale moves to the queries, the output being linear in either)
         q_scale = s.q_scale if turned is not None else s.q_scale * s.k_scale
         first = 0 if turned is not None else col
         return kernels.linear_attention(proj, first, first + qk, col + 2 * qk, s.n_heads, s.head_dim, s.v_head_dim, ctx.state(cache_entry),
                                         self.state_offset, ctx.row_first, ctx.row_lens, ctx.slots,
-                                        chunked=chunked,
+                                        chunked=self.chunks_pay(ctx.lens),
                                         head_decay=self.head_decay, decay_logits=logits, inv_tau=1.0 / s.decay_tau,
                                         q_scale=q_scale, qk_activation=s.qk_activation, v_activation=s.v_activation, qk=turned)
 

@@ -73,10 +73,22 @@ class StateSpace(Mixer):
         return CacheNeeds(kv=None, state_elems=self.matrix_state_elems() + (s.taps - 1) * self._sizes()[2])
 
     def chunks_pay(self, lens) -> bool:
-        """Whether a step with these numbers of tokens a row runs its recurrence as products of tiles over chunks of 64 tokens.  One walk
-        a sequence takes as long as the longest row, a chunk its tiles whatever it holds, so the walk is left to rows that bring a few tokens
-        (rows of 1,400 and 647 tokens, the whole mixer on a B200: 1,220 us with walks of the chunks, 307 us with tiles).  Either way gives the same numbers up to float32 rounding."""
-        return max(lens, default=0) > 16
+        """Whether a step with these numbers of tokens a row runs its recurrence as products of tiles over chunks of 64 tokens, or walks it
+        token after token; either way gives the same numbers up to float32 rounding.
+
+        A walk takes as long as the longest row, and as all rows' tokens take where there are more blocks (a row, head and as many columns as
+        256 threads hold) than run side by side; tiles cost three launches, every chunk its products whatever it holds, and every row the
+        pass that carries its state.  The numbers (for microseconds on a B200) are fitted to both for 1 to 64 rows of 8 to 2,048 tokens.  64
+        heads of 64 columns, 128 state rows, walk / tiles: 1 x 17 tokens 17 / 36 us, 1 x 64 53 / 43, 1 x 2,048 1,583 / 179; 8 x 32 86 / 97,
+        8 x 48 127 / 103; 64 x 17 356 / 873, 64 x 64 1,174 / 1,024; 63 single tokens beside 200 261 / 840, beside 2,048 2,036 / 982."""
+        longest = max(lens, default=0)
+        if longest <= 16:                                                     # (the walk wherever it was measured)
+            return False
+        s = self.spec
+        blocks = s.n_heads * -(-s.head_dim // min(s.head_dim, 256 // kernels.state_space_split(s.state)))
+        walk = 0.85 * max(longest, 0.49 * sum(lens) * blocks / 148)
+        tiles = 23.0 + s.n_heads * (0.047 * sum((n + 63) // 64 for n in lens) + 1.76e-5 * s.state * s.head_dim * sum(n > 0 for n in lens))
+        return tiles < walk
 
     def normed_output(self, h, ctx, cache_entry):
         s = self.spec

@@ -4,6 +4,7 @@ from __future__ import annotations
 
 import copy
 import math
+from types import SimpleNamespace
 
 import pytest
 import torch
@@ -146,3 +147,34 @@ def test_scratch_of_a_batch_of_prompts_is_bounded(per_channel):
         assert gated().pe_linear_attention_slabs(2048, 1, H, D, D, per_channel) == 1 < gated().pe_linear_attention_slabs(2048 * 64, 64, H, D, D, per_channel)
     assert 4 * state_space().pe_state_space_scratch_floats(2048 * 64, 64, 64, 64, 128, 2) <= 256 << 20
     assert state_space().pe_state_space_slabs(2048, 1, 64, 64, 128, 2) == 1
+
+
+ONES = [1] * 63
+
+
+@pytest.mark.parametrize("per_channel,heads,dim,walks,chunks", [
+    (True, 16, 128, [[17], [64], [96], [10, 64, 54], [17] * 64, [64] * 64, [128] * 16, [200] + ONES], [[256], [512], [2048], [512] * 4, [2048] + ONES]),
+    (True, 14, 64, [[17], [64], [17] * 64, [128] * 64, [200] + ONES], [[256], [2048], [512] * 4, [2048] + ONES]),
+    (False, 16, 128, [[17], [64], [17] * 64, [64] * 64, [200] + ONES], [[256], [512], [2048], [512] * 4, [2048] + ONES]),
+    (False, 14, 64, [[17], [64], [17] * 64, [128] * 64, [200] + ONES], [[256], [2048], [512] * 4, [2048] + ONES])])
+def test_linear_attention_takes_the_way_that_was_measured_shorter(per_channel, heads, dim, walks, chunks):
+    """Steps whose two ways differed by a fifth and more on a B200 (tokens a row): from one row to 64, short and long, equal and not."""
+    from pico_engine.parts.linear_attention import LinearAttention
+    part = SimpleNamespace(spec=SimpleNamespace(n_heads=heads, head_dim=dim, v_head_dim=dim), head_decay=None if per_channel else object())
+    for way, steps in ((False, walks + [[1], [16], [1] * 64]), (True, chunks)):
+        for lens in steps:
+            assert LinearAttention.chunks_pay(part, lens) == way, lens
+
+
+@pytest.mark.parametrize("heads,state,walks,chunks", [
+    (64, 128, [[17], [24], [17] * 8, [24] * 64, [200] + ONES], [[96], [2048], [64] * 8, [128] * 64, [2048] + ONES]),
+    (28, 128, [[17], [24], [17] * 8, [24] * 64, [200] + ONES], [[64], [2048], [64] * 8, [128] * 64, [2048] + ONES]),
+    (16, 64, [[17], [17] * 16, [24] * 64], [[64], [2048], [96] * 8, [256] * 64, [2048] + ONES])])
+def test_state_space_takes_the_way_that_was_measured_shorter(heads, state, walks, chunks):
+    """The same for the state-space recurrence, 64 columns a head."""
+    from pico_engine.parts.state_space import StateSpace
+    part = SimpleNamespace(spec=SimpleNamespace(n_heads=heads, head_dim=64, state=state))
+    for way, steps in ((False, walks + [[1], [16], [1] * 64]), (True, chunks)):
+        for lens in steps:
+            assert StateSpace.chunks_pay(part, lens) == way, lens
+
