@@ -78,16 +78,19 @@ class StateSpace(Mixer):
 
         A walk takes as long as the longest row, and as all rows' tokens take where there are more blocks (a row, head and as many columns as
         256 threads hold) than run side by side; tiles cost three launches, every chunk its products whatever it holds, and every row the
-        pass that carries its state.  The numbers (for microseconds on a B200) are fitted to both for 1 to 64 rows of 8 to 2,048 tokens.  64
+        pass that carries its state.  The numbers (for microseconds on a B200) are fitted to 339 steps of 1 to 64 rows of 8 to 2,048 tokens, 16
+        to 256 state rows and 8 to 112 heads; the worst choice among them costs a third more than the better way.  64
         heads of 64 columns, 128 state rows, walk / tiles: 1 x 17 tokens 17 / 36 us, 1 x 64 53 / 43, 1 x 2,048 1,583 / 179; 8 x 32 86 / 97,
         8 x 48 127 / 103; 64 x 17 356 / 873, 64 x 64 1,174 / 1,024; 63 single tokens beside 200 261 / 840, beside 2,048 2,036 / 982."""
         longest = max(lens, default=0)
         if longest <= 16:                                                     # (the walk wherever it was measured)
             return False
         s = self.spec
-        blocks = s.n_heads * -(-s.head_dim // min(s.head_dim, 256 // kernels.state_space_split(s.state)))
-        walk = 0.85 * max(longest, 0.49 * sum(lens) * blocks / 148)
-        tiles = 23.0 + s.n_heads * (0.047 * sum((n + 63) // 64 for n in lens) + 1.76e-5 * s.state * s.head_dim * sum(n > 0 for n in lens))
+        split = kernels.state_space_split(s.state)
+        columns = min(s.head_dim, 256 // split)                               # of a block of the walk
+        warps = s.n_heads * -(-s.head_dim // columns) * columns * split / 32  # of a row
+        walk = 0.82 * max(longest, 0.54 * sum(lens) * warps / (8 * 148))
+        tiles = 22.0 + s.n_heads * (0.07 * sum((n + 63) // 64 for n in lens) + 1.62e-5 * s.state * s.head_dim * sum(n > 0 for n in lens))
         return tiles < walk
 
     def normed_output(self, h, ctx, cache_entry):
