@@ -41,7 +41,6 @@
 // of 8 warps with larger heads; else an SM holds two.
 #define AD_CTAS(WARPS) ((WARPS) == 16 || ((WARPS) == 8 && AD_HD > 64) ? 1 : 2)
 #define AD_MAX_STAGES 12                             // pages in flight per CTA
-#define AD_RANKED 256                                // most tokens of a launch whose CTAs are ordered by length
 #define AD_MAX_SPLITS 16                             // page ranges of a sequence = CTAs of a cluster (8 is the portable limit)
 #define AD_KV_BYTES (PE_PAGE * AD_HD * 2)            // the keys (or the values) of one page and kv head
 #define AD_STAGE_BYTES (2 * AD_KV_BYTES)
@@ -222,7 +221,7 @@ __device__ __forceinline__ void ad_consume(float (&acc)[AD_NCHUNK][4][4], float 
     }
 }
 
-template <int AD_WARPS, bool RANKED>
+template <int AD_WARPS>
 __global__ void __launch_bounds__(32 * (AD_WARPS + 1), AD_CTAS(AD_WARPS)) attention_decode_kernel(
     const bf16* q, int q_stride, const bf16* k_pool, const bf16* v_pool,
     const int* block_table, int table_stride, const int* tok_pos,
@@ -236,21 +235,7 @@ __global__ void __launch_bounds__(32 * (AD_WARPS + 1), AD_CTAS(AD_WARPS)) attent
     __shared__ int page_list[32];                               // the producer's next entries of the page table
     pdl_launch_dependents();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-    int tok = blockIdx.z;
-    if constexpr (RANKED) {                                     // the longest sequences first: CTA z takes the z-th longest
-        __shared__ int lengths[AD_RANKED + 1];                  // positions of the launch's tokens; then the token this CTA takes
-        const int T = gridDim.z;
-        for (int i = threadIdx.x; i < T; i += AD_THREADS) lengths[i] = tok_pos[i];
-        __syncthreads();
-        for (int i = threadIdx.x; i < T; i += AD_THREADS) {
-            const int mine = lengths[i];
-            int before = 0;
-            for (int j = 0; j < T; ++j) before += lengths[j] > mine || (lengths[j] == mine && j < i);
-            if (before == (int)blockIdx.z) lengths[AD_RANKED] = i;
-        }
-        __syncthreads();
-        tok = lengths[AD_RANKED];
-    }
+    const int tok = blockIdx.z;
     const int split = n_splits > 1 ? (int)ad_cluster_rank() : 0;
     const int G = nh / nkv, head_tiles = (G + 15) / 16;
     const int kvh = blockIdx.y / head_tiles, ht = blockIdx.y % head_tiles;
@@ -497,7 +482,7 @@ extern "C" void pe_set_pdl(int on) { pe_pdl_enabled() = on ? 1 : 0; }
 // live in one process, and the function-local statics of a template with external linkage would be one
 // object for all of them (the dynamic linker makes such symbols unique across libraries).
 namespace {
-template <int WARPS, bool RANKED = false>
+template <int WARPS>
 struct AdVariant {
     static constexpr int threads = 32 * (WARPS + 1), groups = WARPS / 4, ctas_per_sm = AD_CTAS(WARPS);
 
@@ -512,16 +497,16 @@ struct AdVariant {
         static bool wide = false;
         if (!allowed) {
             cudaFuncAttributes own;
-            PE_TRY(cudaFuncGetAttributes(&own, attention_decode_kernel<WARPS, RANKED>));
+            PE_TRY(cudaFuncGetAttributes(&own, attention_decode_kernel<WARPS>));
             allowed = 48 * 1024 - own.sharedSizeBytes;
         }
         if (!wide) {                                         // clusters of more than 8 CTAs are an opt-in; if it is refused,
-            cudaFuncSetAttribute(attention_decode_kernel<WARPS, RANKED>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);   // the
+            cudaFuncSetAttribute(attention_decode_kernel<WARPS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);   // the
             cudaGetLastError();                              // occupancy query below answers 0 for them and fewer ranges are used
             wide = true;
         }
         if (smem > allowed) {
-            PE_TRY(cudaFuncSetAttribute(attention_decode_kernel<WARPS, RANKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            PE_TRY(cudaFuncSetAttribute(attention_decode_kernel<WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             allowed = smem;
         }
         return 0;
@@ -546,7 +531,7 @@ struct AdVariant {
             attr[0].val.clusterDim.x = splits; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
             cfg.attrs = attr;
             cfg.numAttrs = 1;
-            if (cudaOccupancyMaxActiveClusters(&n, attention_decode_kernel<WARPS, RANKED>, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+            if (cudaOccupancyMaxActiveClusters(&n, attention_decode_kernel<WARPS>, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
         }
         known[{splits, smem}] = n;
         return n;
@@ -601,7 +586,7 @@ struct AdVariant {
         }
         cfg.attrs = attr;
         cfg.numAttrs = n_attr;
-        PE_TRY(cudaLaunchKernelEx(&cfg, attention_decode_kernel<WARPS, RANKED>, q, q_stride, k_pool, v_pool, block_table, table_stride,
+        PE_TRY(cudaLaunchKernelEx(&cfg, attention_decode_kernel<WARPS>, q, q_stride, k_pool, v_pool, block_table, table_stride,
                                   tok_pos, tok_row, nh, nkv, window, scale_log2e, n_splits, stages, status, out, keep_first, slopes, sinks));
         PE_LAUNCH_CHECK();
         return 0;
@@ -624,30 +609,27 @@ extern "C" void pe_attention_decode_set_max_splits(int n) { ad_split_limit() = n
 //                  sequences of 4,000 tokens and 4 kv heads 37.5 against 26.6 us, of 1,000 12.3 against 11.3; of 640 equal), and
 //                  where all triples of short sequences then run in one turn instead of two (64 sequences of 500 tokens 15.4
 //                  against 12.3 us, 48 of 800 17.9 against 16.9, 40 of 500 12.0 against 11.6; 40 of 800 would take 15.2 against 16.4)
-//                  8 warps with the longest sequences first where the triples take several turns (64 sequences of 300 to 4,000
-//                  tokens 62.3 in their own order, 47.5; 48 of 2,000 33.9 and 29.4; finding the order costs 1 us: 12 pages or less do not pay)
-struct AdShape { int warps, splits, stages; bool ranked; };
+struct AdShape { int warps, splits, stages; };
 static AdShape ad_choose(int T, int nh, int nkv, int max_context) {
     const int G = nh / nkv, ctas = T * nkv * ((G + 15) / 16), limit = ad_split_limit();
     const int pages = (max_context + PE_PAGE - 1) / PE_PAGE;
     const auto range = [&](int splits) { return (pages + splits - 1) / splits; };
-    AdShape c = {8, 1, 1, false};
+    AdShape c = {8, 1, 1};
     c.splits = AdVariant<8>::shape(ctas, pages, limit, &c.stages);
     if constexpr (AD_HD <= 64) {                             // larger heads need the registers
         if (ctas <= 32) {
-            AdShape w = {16, 1, 1, false};
+            AdShape w = {16, 1, 1};
             w.splits = AdVariant<16>::shape(ctas, pages, limit, &w.stages);
             if (range(w.splits) >= 8) return w;
         }
     }
     if constexpr (AD_HD <= 128) {                            // larger heads leave room for one page only
-        AdShape n = {4, 1, 1, false};
+        AdShape n = {4, 1, 1};
         n.splits = AdVariant<4>::shape(ctas, pages, limit, &n.stages);
         if (AD_HD <= 64 ? range(n.splits) <= 2
                         : (c.splits == 1 && n.splits >= 3 && pages >= 16) || (ctas > 148 && ctas <= 2 * 148 && pages <= (ctas < 192 ? 8 : 12)))
             return n;
     }
-    c.ranked = ctas > 148 * AdVariant<8>::ctas_per_sm && T > 1 && T <= AD_RANKED && pages > 12;
     return c;
 }
 
@@ -684,5 +666,5 @@ extern "C" int pe_attention_decode(const void* q, int q_stride, void* out, const
     };
     if constexpr (AD_HD <= 64) { if (c.warps == 16) return go(AdVariant<16>()); }
     if constexpr (AD_HD <= 128) { if (c.warps == 4) return go(AdVariant<4>()); }
-    return c.ranked ? go(AdVariant<8, true>()) : go(AdVariant<8>());
+    return go(AdVariant<8>());
 }
