@@ -141,9 +141,12 @@ extern "C" int pe_conv_silu(const void* proj, int dtype, int ld, int c_off, int 
     if (dtype != PE_F32 && dtype != PE_BF16) return PE_ERR_UNSUPPORTED;
     const size_t total = (size_t)T * C, size = dtype == PE_F32 ? 4 : 2;
     const unsigned blocks = (unsigned)((total + 255) / 256);
-    // runs of four channels where they can be read and written at once (grid.y holds up to 65,535 runs of tokens)
+    // Runs of four channels where they can be read and written at once (grid.y holds up to 65,535 runs of tokens) and where there are enough
+    // of them: a thread's eight tokens wait for one another's rows, which the kernel above takes side by side.  Measured on a B200, above /
+    // runs: 1 row of 17 tokens x 4,608 channels 4.3 / 6.7 us, of 100 7.0 / 6.8, of 128 7.9 / 6.8, of 400 17.4 / 8.1; 8 x 1 4.4 / 10.0, 64 x 1
+    // 6.8 / 12.5, 64 x 2 9.1 / 10.5, 64 x 4 13.4 / 9.6; 128 x 1 of 10,000 19.4 / 17.3.
     const bool vec = taps >= 2 && taps <= 4 && C % 4 == 0 && c_off % 4 == 0 && ld % 4 == 0 && (uintptr_t)proj % (4 * size) == 0 &&
-                     (uintptr_t)out % 16 == 0 && (T + CONV_TOKENS - 1) / CONV_TOKENS <= 65535;
+                     (uintptr_t)out % 16 == 0 && (T + CONV_TOKENS - 1) / CONV_TOKENS <= 65535 && total >= (T >= 8 * B ? 500000u : 1000000u);
     if (vec) {
         const int rc = dtype == PE_F32 ? conv_silu_vec((const float*)proj, ld, c_off, C, taps, w, w_dtype, bias, b_dtype, state, state_stride, tok_row, row_first, slots, out, T, s)
                                        : conv_silu_vec((const bf16*)proj, ld, c_off, C, taps, w, w_dtype, bias, b_dtype, state, state_stride, tok_row, row_first, slots, out, T, s);

@@ -629,3 +629,29 @@ def test_prompts_of_many_steps_over_low_rank_rows(H, width, rank):
     k[:, 0, -1] = (6.0 * torch.arange(n) / 128).to(dt).float()                             # 12 more with every 128 keys
     for window in (None, 200):
         check(q, k, window)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("taps,C,lens", [(4, 4608, [1, 2, 3, 127]), (2, 2048, [8, 9, 300]), (3, 4612, [5] * 44), (4, 5000, [1] * 70 + [2] * 69), (4, 1024, [1, 2, 127])])
+def test_convolution_in_runs_of_channels(dtype, taps, C, lens):
+    """Steps large enough for the kernel of four channels and eight tokens a thread (the last is not): rows that begin and end inside a thread's tokens, rows
+    shorter than the taps, in two steps whose second reads what the first left."""
+    from pico_engine.ops import kernels
+    dt, B, T = DTYPES[dtype], len(lens), sum(lens)
+    g = torch.Generator().manual_seed(C)
+    w, bias = (0.5 * torch.randn(C, taps, generator=g)).to(dt), torch.randn(C, generator=g).to(dt)
+    first, rows = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int32).cuda(), torch.tensor(lens, dtype=torch.int32).cuda()
+    tok_row = torch.tensor([b for b, n in enumerate(lens) for _ in range(n)], dtype=torch.int32).cuda()
+    slots = torch.arange(B, dtype=torch.int32).flip(0).contiguous().cuda()
+    state = torch.zeros(B, (taps - 1) * C).cuda()
+    past = [torch.zeros(taps - 1, C, dtype=torch.float64) for _ in lens]
+    for step in range(2):
+        proj = torch.randn(T, C + 8, generator=g).to(dt)
+        got = kernels.conv_silu(proj.cuda(), 4, C, w.cuda(), bias.cuda(), state, 0, tok_row, first, rows, slots).cpu().double()
+        at = 0
+        for b, n in enumerate(lens):
+            u = torch.cat([past[b], proj[at: at + n, 4: 4 + C].double()])
+            want = torch.nn.functional.silu(bias.double() + sum(w[:, j].double() * u[j: j + n] for j in range(taps)))
+            # a sum of at most four products in float32, then silu
+            assert (got[at: at + n] - want).abs().max() < 1e-5, (step, b)
+            past[b], at = u[-(taps - 1):], at + n
