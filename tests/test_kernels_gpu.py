@@ -1037,3 +1037,20 @@ def test_product_choice_is_made_once_and_both_ways_agree(K):
     err, at = rel_err(first.float(), other.float())
     assert err < 1.2e-2, (err, at)
     assert torch.equal(L.gate_up_swiglu(A, W), first)
+
+
+@pytest.mark.parametrize("ta,tw", [(torch.float32, torch.float32), (torch.bfloat16, torch.float32), (torch.float32, torch.bfloat16)])
+@pytest.mark.parametrize("N,K_", [(33, 1), (130, 16), (64, 17), (200, 32), (96, 33)])
+def test_linear_simt_with_a_short_k(K, N, K_, ta, tw):
+    """Products on both sides of the line to the kernel for a short K, rows and columns beside its tiles, with a bias and into a float32
+    stream: against float64, and a row's sums are the same alone and among others."""
+    a, w, bias = rnd(70, K_, seed=1).to(ta), rnd(N, K_, seed=2).to(tw), rnd(N, seed=3)
+    for M in (1, 16, 17, 64, 65, 70):
+        want = a[:M].double() @ w.double().T
+        got = K.linear_simt(dev(a[:M].contiguous()), dev(w), dev(bias), out_dtype=torch.float32)
+        # K products and sums of about unit size in float32
+        assert float((got.cpu().double() - want - bias.double()).abs().max()) <= 8 * (K_ + 1) * 2.0 ** -24
+        x = dev(torch.ones(M, N))
+        K.linear_simt(dev(a[:M].contiguous()), dev(w), accumulate_into=x)
+        assert float((x.cpu().double() - want - 1).abs().max()) <= 8 * (K_ + 1) * 2.0 ** -24
+        assert torch.equal(got, K.linear_simt(dev(a), dev(w), dev(bias), out_dtype=torch.float32)[:M])
