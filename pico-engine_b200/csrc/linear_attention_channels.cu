@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(ST_THREADS) lc_output_kernel(LAArgs a, const f
         *reinterpret_cast<float4*>(pt + 4 * i) = *reinterpret_cast<const float4*>(w_src + 4 * i);
         const float4 v = s < n ? lc_load4(v_src + (size_t)s * a.ld + c, Dv - c0 - c, vec_v) : make_float4(0.f, 0.f, 0.f, 0.f);
         const float4 u = make_float4(la_act<FAST>(v.x, a.act_v), la_act<FAST>(v.y, a.act_v), la_act<FAST>(v.z, a.act_v), la_act<FAST>(v.w, a.act_v));
-        odd = odd || st_odd(u);
+        odd |= st_odd(u);
         *reinterpret_cast<float4*>(vs + 4 * i) = u;
     }
     const bool guarded = __syncthreads_or(odd);

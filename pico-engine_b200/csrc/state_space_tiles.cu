@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(ST_THREADS) st_output_kernel(ScanArgs a, int v
         w.z = s <= t + 2 ? w.z * (d * expf((float)(las[t + 2] - ls))) : 0.f;
         w.w = s <= t + 3 ? w.w * (d * expf((float)(las[t + 3] - ls))) : 0.f;
         *reinterpret_cast<float4*>(pt + 4 * i) = w;
-        odd = odd || st_odd(x);
+        odd |= st_odd(x);
         *reinterpret_cast<float4*>(xs + 4 * i) = x;
     }
 #pragma unroll
