@@ -89,12 +89,14 @@ __global__ void __launch_bounds__(AG_THREADS) attention_generic_kernel(
 // 14 heads of 64, prompts of 301 and 207 tokens, on a B200: 645 us by the kernel above (a block a token and head, which read every key
 // and value once a head), 75 us here.
 #define AT_THREADS 256
+#define AG_RUN 64                                         // tokens of a run at most
 
 struct AttentionTileArgs {
     const void* q; int q_stride; void* out; const void* k_pool; const void* v_pool;
     const int* table; int table_stride; const int* tok_pos; const int* tok_row;
     int T, nh, nkv, hd, window; float scale;
     int heads, slices, tokens;                     // query heads and tokens of a block's rows; blocks that share a key/value head's heads
+    const int4* runs; int parts;                   // null: blocks of neighbouring packed tokens; else runs (row, first packed token, tokens, ..), `parts` blocks each
 };
 
 __device__ __forceinline__ float4 ag_load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
@@ -134,7 +136,14 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tile_kernel(AttentionTil
     float* vs = kt + hd * 64;                              // [64][hd]
     float* ps = vs + hd * 64;                              // [64 keys][R]: weights, rows in groups of four exchanged by the key
     const int per = a.nh / a.nkv, kvh = blockIdx.y / a.slices, h0 = kvh * per + blockIdx.y % a.slices * a.heads;
-    const int n_heads = min(a.heads, kvh * per + per - h0), t0 = blockIdx.x * a.tokens, n_tok = min(a.tokens, a.T - t0);
+    int t0 = blockIdx.x * a.tokens, left = a.T - t0;
+    if (a.runs) {
+        const int4 run = a.runs[blockIdx.x / a.parts];
+        const int behind = blockIdx.x % a.parts * a.tokens;
+        t0 = run.y + behind; left = run.z - behind;
+        if (left <= 0) return;
+    }
+    const int n_heads = min(a.heads, kvh * per + per - h0), n_tok = min(a.tokens, left);
     const int rows = n_heads * n_tok;                      // row r: token t0 + r / n_heads, head h0 + r % n_heads
     if (tid < R) {
         const int t = t0 + min(tid, rows - 1) / n_heads;
@@ -301,38 +310,50 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tile_kernel(AttentionTil
 }
 
 template <typename T, int R, int NJ>
-static int attention_tile_as(AttentionTileArgs a, cudaStream_t s) {
+static int attention_tile_as(AttentionTileArgs a, int n_runs, int most, cudaStream_t s) {
     const int per = a.nh / a.nkv;
     a.heads = per < R ? per : R;
     a.slices = (per + a.heads - 1) / a.heads;
-    a.tokens = R == 16 ? 1 : R / a.heads;                  // single tokens are of different sequences: a block each
+    a.tokens = R / a.heads < most ? R / a.heads : most;
+    a.parts = (AG_RUN + a.tokens - 1) / a.tokens;
+    if (a.runs) a.tokens = (AG_RUN + a.parts - 1) / a.parts;          // a whole run in equal parts
+    const int blocks = a.runs ? n_runs * a.parts : (a.T + a.tokens - 1) / a.tokens;
     const size_t smem = sizeof(float) * ((size_t)3 * a.hd * 64 + 64 * R);
     auto kernel = attention_tile_kernel<T, R, NJ>;
     PE_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    PE_TRY(pe_launch(kernel, dim3((a.T + a.tokens - 1) / a.tokens, a.nkv * a.slices), AT_THREADS, smem, s, a));
+    PE_TRY(pe_launch(kernel, dim3(blocks, a.nkv * a.slices), AT_THREADS, smem, s, a));
     PE_LAUNCH_CHECK();
     return 0;
 }
 template <typename T>
-static int attention_tile(const AttentionTileArgs& a, bool runs, cudaStream_t s) {
-    if (a.hd <= 64) return runs ? attention_tile_as<T, 64, 1>(a, s) : attention_tile_as<T, 16, 1>(a, s);
-    if (a.hd <= 128) return runs ? attention_tile_as<T, 64, 2>(a, s) : attention_tile_as<T, 16, 2>(a, s);
-    return runs ? attention_tile_as<T, 64, 4>(a, s) : attention_tile_as<T, 16, 4>(a, s);
+static int attention_tile(const AttentionTileArgs& a, int n_runs, int sequences, cudaStream_t s) {
+    const int per = a.nh / a.nkv, few = per < 16 ? 16 / per : 1;      // tokens of a block of 16 rows
+    // Which blocks: 16 rows while all those run at once, else 64.  Where no runs are known a block may get tokens of several sequences, which
+    // it serves one after the other: no more of them than an eighth of what a sequence brings on average, and so single ones where they bring few.
+    // One prompt of 40 tokens beside 30 single tokens at 600, float32, on a B200, a block a token and head / 64 rows of neighbouring tokens
+    // / runs: 14 heads of 64 on 2 255 / 506 / 69 us, 4 of 256 on one 275 / 3,801 / 138.
+    const int most = a.runs ? AG_RUN : sequences > 0 && a.T / sequences >= 16 ? a.T / sequences / 8 : 1;
+    const int blocks16 = (a.T + min(few, most) - 1) / min(few, most);
+    const bool wide = (long long)most * per > 16 && (long long)blocks16 * a.nkv * ((per + 15) / 16) > 148;
+    if (a.hd <= 64) return wide ? attention_tile_as<T, 64, 1>(a, n_runs, most, s) : attention_tile_as<T, 16, 1>(a, n_runs, most, s);
+    if (a.hd <= 128) return wide ? attention_tile_as<T, 64, 2>(a, n_runs, most, s) : attention_tile_as<T, 16, 2>(a, n_runs, most, s);
+    return wide ? attention_tile_as<T, 64, 4>(a, n_runs, most, s) : attention_tile_as<T, 16, 4>(a, n_runs, most, s);
 }
 
+// runs: null, or [n_runs] of (batch row, first packed token, number of tokens (<= 64), ..): the step's tokens, each in one of them
 extern "C" int pe_attention_generic(const void* q, int q_stride, void* out, const void* k_pool, const void* v_pool,
                                     int dtype, const int* block_table, int table_stride, const int* tok_pos,
                                     const int* tok_row, int T, int nh, int nkv, int hd, int window, float scale, int sequences,
-                                    void* stream) {
+                                    const void* runs, int n_runs, void* stream) {
     if (T <= 0) return 0;
     if (hd <= 0 || hd > AG_MAX_HD || nkv <= 0 || nh % nkv || nh > 65535) return PE_ERR_UNSUPPORTED;
     cudaStream_t s = (cudaStream_t)stream;
     const size_t size = dtype == PE_F32 ? 4 : 2;
     if ((dtype == PE_F32 || dtype == PE_BF16) && hd % 4 == 0 && q_stride % 4 == 0 && !(((uintptr_t)q | (uintptr_t)out | (uintptr_t)k_pool | (uintptr_t)v_pool) % (4 * size))) {
-        // rows of four entries that can be read at once: tiles of rows; 64 of them where a sequence brings several tokens
-        const AttentionTileArgs a = {q, q_stride, out, k_pool, v_pool, block_table, table_stride, tok_pos, tok_row, T, nh, nkv, hd, window, scale, 0, 0, 0};
-        const bool runs = sequences > 0 && T >= 2 * sequences;
-        return dtype == PE_F32 ? attention_tile<float>(a, runs, s) : attention_tile<bf16>(a, runs, s);
+        // rows of four entries that can be read at once: tiles of rows
+        const AttentionTileArgs a = {q, q_stride, out, k_pool, v_pool, block_table, table_stride, tok_pos, tok_row, T, nh, nkv, hd, window, scale, 0, 0, 0,
+                                     (const int4*)runs, 0};
+        return dtype == PE_F32 ? attention_tile<float>(a, n_runs, sequences, s) : attention_tile<bf16>(a, n_runs, sequences, s);
     }
     dim3 grid(T, nh);
     if (dtype == PE_F32)

@@ -175,9 +175,10 @@ def linear_simt(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] =
 def attention_generic(q: torch.Tensor, q_stride: int, n_heads: int, n_kv_heads: int, head_dim: int,
                       k_pool: torch.Tensor, v_pool: torch.Tensor, block_table: torch.Tensor, table_stride: int,
                       tok_pos: torch.Tensor, tok_row: torch.Tensor, window: Optional[int], scale: float,
-                      out: Optional[torch.Tensor] = None) -> torch.Tensor:
+                      out: Optional[torch.Tensor] = None, runs: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Attention of T tokens over the cache.  ``q`` holds the query heads of token t at
-    ``t * q_stride + h * head_dim``; the result is [T, n_heads * head_dim] in q's dtype."""
+    ``t * q_stride + h * head_dim``; the result is [T, n_heads * head_dim] in q's dtype.  ``runs``: the tokens as runs of at most 64 of
+    one sequence (``prefill_tiles``), for steps that bring prompts; the result does not depend on it."""
     T = tok_pos.shape[0]
     _need(q, "q"); _need(k_pool, "k_pool", q.dtype); _need(v_pool, "v_pool", q.dtype, k_pool.shape)
     if tuple(k_pool.shape[1:]) != (n_kv_heads, PAGE, head_dim):
@@ -187,10 +188,15 @@ def attention_generic(q: torch.Tensor, q_stride: int, n_heads: int, n_kv_heads: 
     if out is None:
         out = torch.empty(T, n_heads * head_dim, dtype=q.dtype, device=q.device)
     _need(out, "out", q.dtype, (T, n_heads * head_dim))
+    if runs is not None:
+        _need(runs, "runs", torch.int32)
+        if runs.dim() != 2 or runs.shape[1] != 4 or runs.data_ptr() % 16:
+            raise KernelError("runs must be rows of (batch row, first token, tokens, first position)")
     check(core().pe_attention_generic(q.data_ptr(), q_stride, out.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(),
                                       _code(q, "q"), block_table.data_ptr(), table_stride, tok_pos.data_ptr(),
                                       tok_row.data_ptr(), T, n_heads, n_kv_heads, head_dim, window or 0, float(scale),
-                                      block_table.shape[0] if block_table.dim() == 2 else 0, stream_ptr()), "attention_generic")
+                                      block_table.shape[0] if block_table.dim() == 2 else 0, _ptr(runs), 0 if runs is None else runs.shape[0],
+                                      stream_ptr()), "attention_generic")
     return out
 
 
@@ -412,8 +418,11 @@ def attention(q: torch.Tensor, q_stride: int, n_heads: int, n_kv_heads: int, hea
         run = attention_prefill_tcgen05 if tcgen05 else attention_prefill
         return run(q, q_stride, n_heads, n_kv_heads, head_dim, k_pool, v_pool, block_table, table_stride, tiles,
                    tok_pos.shape[0], window, scale)
+    # (where every row is a prompt, blocks of neighbouring tokens cross from one to the next so seldom that the runs' last, partly filled
+    # blocks cost more: prompts of 301 and 207 tokens, two layers of 14 heads of 64, 897 us without and 909 with)
+    runs = None if all(n == 0 or n >= PREFILL_TILE for n in ctx.lens) or ctx.one_token_each else _step_tiles(ctx, PREFILL_TILE, q.device)
     return attention_generic(q, q_stride, n_heads, n_kv_heads, head_dim, k_pool, v_pool, block_table, table_stride,
-                             tok_pos, tok_row, window, scale)
+                             tok_pos, tok_row, window, scale, runs=runs)
 
 
 # ---------------------------------------------------------------------------- fused decode products (bfloat16, up to 16 rows)

@@ -44,7 +44,7 @@ _SIGNATURES = {
     "pe_bias_add": [P, I, P, I, I, I, P],
     "pe_rope_store": [P, I, I, I, I, I, P, P, P, P, P, P, P, I, I, P],
     "pe_linear_simt": [P, I, P, I, P, I, P, I, I, I, I, P],
-    "pe_attention_generic": [P, I, P, P, P, I, P, I, P, P, I, I, I, I, I, F, I, P],
+    "pe_attention_generic": [P, I, P, P, P, I, P, I, P, P, I, I, I, I, I, F, I, P, I, P],
     "pe_argmax": [P, P, I, I, P, P],
     "pe_sample": [P, P, I, I, F, I, F, ULL, P, P, P, P, P],
     "pe_gemm_tcgen05": [P, P, P, I, P, I, I, I, I, I, P, P],
