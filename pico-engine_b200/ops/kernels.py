@@ -886,6 +886,50 @@ def headmix_mma_key_block(n_heads: int, n_kv: int, head_dim: int, v_head_dim: in
     return _headmix_plans[key]
 
 
+def flashmix_ranges(blocks: int, max_context: int, window: Optional[int], keep_first: int = 0) -> int:
+    """Ranges of keys that attention_headmix_flash.cu cuts a step of ``blocks`` blocks into."""
+    # Few blocks (single tokens with long contexts): the keys are cut into ranges until about one and a half blocks
+    # an SM run.  Measured on a B200 (8 tokens at 2,048 keys): 14 heads of 64 on 2 key/value heads 65 / 47 / 29 / 32 /
+    # 51 us at 2 / 4 / 8 / 16 / 32 ranges, 16 heads of 128 on 4 key/value heads 82 / 55 / 70 / 97 / 202 us: more ranges
+    # mean more partial outputs to write and merge.  A prompt has blocks enough and is not cut (2,048 tokens: 183 us
+    # uncut, 209 us in two ranges).
+    # (a window leaves a token the pages of its last `window` keys and of the kept first ones: no more ranges than those)
+    span = max_context if not window else min(max_context, window + PAGE - 1 + (keep_first + PAGE - 1) // PAGE * PAGE)
+    return max(1, min((224 + blocks - 1) // blocks, (span + 63) // 64, 64))
+
+
+def flashmix_prompts_pay(ctx, n_heads: int, n_kv: int, head_dim: int, v_head_dim: int, window: Optional[int], values_in_keys: bool = False) -> bool:
+    """Whether a step that brings prompts is left to attention_headmix_flash.cu although a tcgen05 kernel takes its sizes: that kernel visits a
+    run's pages one after the other, this one cuts them into ranges where there are few blocks, which pays for a few tokens over a long
+    context.  Both are estimated in microseconds on a B200: a range's pages and the merge of the partial results here, all pages there.
+    The numbers are fitted to 626 measured steps (2 to 256 tokens behind 0 to 16,384, 4 to 32 heads, each kind of tile): at their choice no step
+    is more than 6 % over the shorter way above 25 us.  17 tokens behind 4,096, ranges / whole: 14 heads of 64 on 2 key/value
+    heads with mixing 35 / 51 us, 16 of 128 on 4 89 / 86; rows of 128 + 32 28 / 55, of 192 + 64 86 / 63; behind 16,384 76 / 166, 272 / 313,
+    62 / 203 and 255 / 232."""
+    longest = max(a + n for a, n in zip(ctx.starts, ctx.lens))
+    tokens, runs = sum(ctx.lens), sum((n + PREFILL_TILE - 1) // PREFILL_TILE for n in ctx.lens)
+    group = max(1, min(n_kv, 256 // v_head_dim))                              # value heads a block of this kernel
+    ranges = flashmix_ranges(runs * n_heads * -(-n_kv // group), longest, window)
+    if ranges < 3:
+        return False
+    pages = (min(longest, window + PREFILL_TILE + PAGE) if window else longest) // PAGE + 1
+    wide = group * v_head_dim > 128
+    if wide:
+        a_page = 3.6 if head_dim <= 64 else 6.7 if head_dim <= 128 else 12.7
+    else:
+        a_page = 2.8 if head_dim <= 64 else 5.5 if head_dim <= 128 else 3.0
+    merged = 1e-6 * tokens * ranges * n_heads * n_kv * v_head_dim * (6.0 if values_in_keys or wide else 14.0)
+    here = (16.0 if wide else 11.0) + a_page * -(-pages // ranges) + merged
+    panels = -(-head_dim // 64)                                               # of 64 columns: what a page costs there
+    if values_in_keys:
+        there = 4.5 + pages * (0.43 + 0.113 * panels)
+    else:
+        fits = [c for c in range(1, n_kv + 1) if n_kv % c == 0 and c * v_head_dim <= 256 and c * v_head_dim % 64 == 0]
+        heads = max(fits, default=1)
+        there = 10.5 + pages * (0.28 if heads >= 4 else 0.2) * (panels + heads * -(-v_head_dim // 64))
+    return here < there
+
+
 def attention_latent_prompt(q: torch.Tensor, q_stride: int, n_heads: int, width: int, rank: int, pool: torch.Tensor, block_table: torch.Tensor,
                             table_stride: int, window: Optional[int], scale: float, ctx, gate: Optional[torch.Tensor] = None,
                             gate_offset: int = 0) -> Optional[torch.Tensor]:
@@ -957,7 +1001,8 @@ def attention_headmix(q: torch.Tensor, q_stride: int, n_heads: int, n_kv: int, h
             tiles = ctx.scratch["prefill_tiles_128"] = prefill_tiles(ctx.lens, ctx.starts, q.device, PREFILL_TILE_TCGEN05)
         return attention_prefill_tcgen05(q, q_stride, n_heads, n_kv, head_dim, k_pool, v_pool, block_table, table_stride, tiles, T,
                                          window, scale, keep_first=keep_first, slopes=slopes, sinks=sink)
-    if plain_out and values_in_keys and n_kv == 1 and sink is None and mix is None and slopes is None and not keep_first:
+    if (plain_out and values_in_keys and n_kv == 1 and sink is None and mix is None and slopes is None and not keep_first
+            and not ctx.one_token_each and q.dtype == torch.bfloat16 and not flashmix_prompts_pay(ctx, n_heads, 1, head_dim, v_head_dim, window, True)):
         out = attention_latent_prompt(q, q_stride, n_heads, head_dim, v_head_dim, k_pool, block_table, table_stride, window, scale, ctx)
         if out is not None:
             return out
@@ -980,7 +1025,8 @@ def attention_headmix(q: torch.Tensor, q_stride: int, n_heads: int, n_kv: int, h
     floats = all(t is None or t.dtype == torch.float32 for t in (sink, mix))
     if (plain_out and q.dtype == torch.bfloat16 and tiles is not None and HEADMIX_TENSOR_CORES == "1" and floats and plain_mask and mix is not None
             and scale > 0 and q_stride % 8 == 0 and (q.data_ptr() | k_pool.data_ptr() | v_pool.data_ptr()) % 16 == 0
-            and lib.pe_attention_headmix_tcgen05_takes(n_heads, n_kv, head_dim, v_head_dim)):
+            and lib.pe_attention_headmix_tcgen05_takes(n_heads, n_kv, head_dim, v_head_dim)
+            and not flashmix_prompts_pay(ctx, n_heads, n_kv, head_dim, v_head_dim, window)):
         # prompts whose weights are mixed: both products on tcgen05, the mixing behind them (1,024 tokens, 16
         # heads of 128 on four key/value heads on a B200: 55 us against 281 us of the mma.sync kernel and its merge)
         runs = _step_tiles(ctx, PREFILL_TILE_TCGEN05, q.device)
@@ -995,14 +1041,7 @@ def attention_headmix(q: torch.Tensor, q_stride: int, n_heads: int, n_kv: int, h
         if cg and q_stride % 2 == 0 and v_ld % 8 == 0:
             # one pass over the keys with an output for every (head, value head), then merge + sink + mixing
             blocks = (n_runs * n_heads if tiles is not None else T * n_kv) * ((n_kv + cg - 1) // cg)
-            # Few blocks (single tokens with long contexts): the keys are cut into ranges until about one and a half blocks
-            # an SM run.  Measured on a B200 (8 tokens at 2,048 keys): 14 heads of 64 on 2 key/value heads 65 / 47 / 29 / 32 /
-            # 51 us at 2 / 4 / 8 / 16 / 32 ranges, 16 heads of 128 on 4 key/value heads 82 / 55 / 70 / 97 / 202 us: more ranges
-            # mean more partial outputs to write and merge.  A prompt has blocks enough and is not cut (2,048 tokens: 183 us
-            # uncut, 209 us in two ranges).
-            # (a window leaves a token the pages of its last `window` keys and of the kept first ones: no more ranges than those)
-            span = ctx.max_context if not window else min(ctx.max_context, window + PAGE - 1 + (keep_first + PAGE - 1) // PAGE * PAGE)
-            splits = max(1, min((224 + blocks - 1) // blocks, (span + 63) // 64, 64))
+            splits = flashmix_ranges(blocks, ctx.max_context, window, keep_first)
             ws = scratch("attention_headmix", 4 * lib.pe_attention_flashmix_scratch_floats(T, splits, n_heads, n_kv, v_head_dim, 1 if tiles is None else 0), q.device)
             check(lib.pe_attention_flashmix(q.data_ptr(), q_stride, out.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(),
                                             block_table.data_ptr(), table_stride, tok_pos.data_ptr(), tok_row.data_ptr(), _ptr(tiles),

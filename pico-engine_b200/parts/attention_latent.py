@@ -115,8 +115,10 @@ class LatentAttention(Mixer):
                                halves=isinstance(s.position, RotaryHalvesSpec), q_rows=q_rows, q_out=q)
         # prompts: the gate, a number a head and token, is applied to the heads' rows before the batched product (it commutes with it)
         gated = s.gate is None
-        a = kernels.attention_latent_prompt(q, q.shape[1], H, rank + R, rank, kv.k, kv.table, kv.stride, s.window, s.scale, ctx,
-                                            None if gated else proj, q_w + dkv_w)
+        a = None
+        if not ctx.one_token_each and q.dtype == torch.bfloat16 and not kernels.flashmix_prompts_pay(ctx, H, 1, rank + R, rank, s.window, True):
+            a = kernels.attention_latent_prompt(q, q.shape[1], H, rank + R, rank, kv.k, kv.table, kv.stride, s.window, s.scale, ctx,
+                                                None if gated else proj, q_w + dkv_w)
         if a is not None:
             gated = True
         else:

@@ -316,7 +316,7 @@ SHAPE_CASES = [                       # (nh, nkv, hd, sequences, longest, bound 
     (14, 2, 64, 24, 128, 128), (2, 1, 16, 8, 300, 300),
     (16, 4, 128, 19, 1024, 1024), (16, 4, 128, 19, 960, 960),         # three ranges instead of none, from 16 pages on
     (16, 4, 128, 40, 500, 512), (16, 4, 128, 37, 500, 513),           # more triples than SMs: 4 warps up to 8 pages, then 8
-    (8, 2, 80, 74, 400, 512), (8, 2, 80, 75, 800, 833),               # as many as SMs, then more
+    (8, 2, 80, 74, 400, 512), (8, 2, 80, 75, 800, 833),               # as many as SMs, then the longest first
     (4, 4, 128, 40, 833, 833), (1, 1, 128, 256, 900, 900), (1, 1, 128, 257, 900, 900),
 ]
 
@@ -1039,23 +1039,6 @@ def test_product_choice_is_made_once_and_both_ways_agree(K):
     assert torch.equal(L.gate_up_swiglu(A, W), first)
 
 
-@pytest.mark.parametrize("ta,tw", [(torch.float32, torch.float32), (torch.bfloat16, torch.float32), (torch.float32, torch.bfloat16)])
-@pytest.mark.parametrize("N,K_", [(33, 1), (130, 16), (64, 17), (200, 32), (96, 33)])
-def test_linear_simt_with_a_short_k(K, N, K_, ta, tw):
-    """Products on both sides of the line to the kernel for a short K, rows and columns beside its tiles, with a bias and into a float32
-    stream: against float64, and a row's sums are the same alone and among others."""
-    a, w, bias = rnd(70, K_, seed=1).to(ta), rnd(N, K_, seed=2).to(tw), rnd(N, seed=3)
-    for M in (1, 16, 17, 64, 65, 70):
-        want = a[:M].double() @ w.double().T
-        got = K.linear_simt(dev(a[:M].contiguous()), dev(w), dev(bias), out_dtype=torch.float32)
-        # K products and sums of about unit size in float32
-        assert float((got.cpu().double() - want - bias.double()).abs().max()) <= 8 * (K_ + 1) * 2.0 ** -24
-        x = dev(torch.ones(M, N))
-        K.linear_simt(dev(a[:M].contiguous()), dev(w), accumulate_into=x)
-        assert float((x.cpu().double() - want - 1).abs().max()) <= 8 * (K_ + 1) * 2.0 ** -24
-        assert torch.equal(got, K.linear_simt(dev(a), dev(w), dev(bias), out_dtype=torch.float32)[:M])
-
-
 @pytest.mark.parametrize("nh,nkv,hd,window", [(14, 2, 64, None), (3, 3, 40, 70), (20, 1, 16, None), (4, 1, 256, None)])
 @pytest.mark.parametrize("new,before", [([40] + [1] * 9, [0] + [200] * 9), ([5], [130]), ([200, 1, 129, 64], [0, 300, 7, 64])])
 def test_attention_generic_in_runs_of_one_sequence(K, nh, nkv, hd, window, new, before):
@@ -1073,3 +1056,21 @@ def test_attention_generic_in_runs_of_one_sequence(K, nh, nkv, hd, window, new, 
     for j in sorted({0, len(row) - 1, len(row) // 2, new[0] - 1, new[0] % len(row)}):
         assert torch.equal(run([j], None)[0], whole[j]), j
     assert torch.equal(run(list(range(len(row))), None), whole)
+
+
+@pytest.mark.parametrize("ta,tw", [(torch.float32, torch.float32), (torch.bfloat16, torch.float32), (torch.float32, torch.bfloat16)])
+@pytest.mark.parametrize("N,K_", [(33, 1), (130, 16), (64, 17), (200, 32), (96, 33)])
+def test_linear_simt_with_a_short_k(K, N, K_, ta, tw):
+    """Products on both sides of the line to the kernel for a short K, rows and columns beside its tiles, with a bias and into a float32
+    stream: against float64, and a row's sums are the same alone and among others."""
+    a, w, bias = rnd(70, K_, seed=1).to(ta), rnd(N, K_, seed=2).to(tw), rnd(N, seed=3)
+    for M in (1, 16, 17, 64, 65, 70):
+        want = a[:M].double() @ w.double().T
+        got = K.linear_simt(dev(a[:M].contiguous()), dev(w), dev(bias), out_dtype=torch.float32)
+        # K products and sums of about unit size in float32
+        assert float((got.cpu().double() - want - bias.double()).abs().max()) <= 8 * (K_ + 1) * 2.0 ** -24
+        x = dev(torch.ones(M, N))
+        K.linear_simt(dev(a[:M].contiguous()), dev(w), accumulate_into=x)
+        assert float((x.cpu().double() - want - 1).abs().max()) <= 8 * (K_ + 1) * 2.0 ** -24
+        assert torch.equal(got, K.linear_simt(dev(a), dev(w), dev(bias), out_dtype=torch.float32)[:M])
+

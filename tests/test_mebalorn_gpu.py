@@ -270,12 +270,13 @@ def test_norm_of_queries_and_keys_and_the_store(H, G, D, Dv, normed):
 
 @pytest.mark.parametrize("H,G,D,Dv,window", [(2, 1, 16, 64, None), (6, 2, 48, 96, 100), (3, 3, 64, 64, None), (16, 4, 128, 128, None),
                                              (20, 2, 64, 64, 1), (4, 4, 128, 128, 300), (5, 1, 64, 256, None), (7, 7, 32, 64, 64)])
-def test_headmix_prompts_in_tensor_memory(H, G, D, Dv, window):
+def test_headmix_prompts_in_tensor_memory(monkeypatch, H, G, D, Dv, window):
     """The tcgen05 kernel at every grouping of value heads: several sequences in a step, whole and in portions off the borders of pages and
     of runs of 128 tokens, against the same in float64; the sizes are ones that it takes."""
     from pico_engine.ops import kernels
     from pico_engine.ops.library import mixers
     assert mixers().pe_attention_headmix_tcgen05_takes(H, G, D, Dv)
+    monkeypatch.setattr(kernels, "flashmix_prompts_pay", lambda *a: False)
     g = torch.Generator().manual_seed(H * 100 + D)
     lens, dt, scale = [1, 65, 400], torch.bfloat16, 1.5 * D ** -0.5
     T = sum(lens)
@@ -406,12 +407,13 @@ def test_pointwise_kernels():
 
 @pytest.mark.parametrize("rubbish", [float("nan"), float("inf")])
 @pytest.mark.parametrize("H,G,D,Dv", [(2, 1, 16, 64), (6, 2, 48, 96), (16, 4, 128, 128), (5, 1, 64, 256)])
-def test_headmix_prompts_do_not_see_what_an_earlier_owner_left_in_a_page(H, G, D, Dv, rubbish):
+def test_headmix_prompts_do_not_see_what_an_earlier_owner_left_in_a_page(monkeypatch, H, G, D, Dv, rubbish):
     """Cache rows that no live sequence has written may hold anything: with numbers that are none in all of them, prompts that end on,
     before and behind the borders of pages and of runs give the same bits as with zeros."""
     from pico_engine.ops import kernels
     from pico_engine.ops.library import mixers
     assert mixers().pe_attention_headmix_tcgen05_takes(H, G, D, Dv)
+    monkeypatch.setattr(kernels, "flashmix_prompts_pay", lambda *a: False)
     g = torch.Generator().manual_seed(H)
     sink, talk = torch.randn(H, generator=g).cuda(), (torch.eye(H) + 0.4 * torch.randn(H, H, generator=g)).cuda()
     for n, start in ((1, 0), (37, 0), (64, 0), (127, 0), (129, 0), (300, 0), (700, 650)):
@@ -441,12 +443,14 @@ def rising(n, H, G, D, g):
 
 
 @pytest.mark.parametrize("H,G,D,Dv", [(4, 2, 64, 64), (16, 4, 128, 128), (20, 2, 64, 64)])
-def test_headmix_prompts_of_many_steps(H, G, D, Dv):
+def test_headmix_prompts_of_many_steps(monkeypatch, H, G, D, Dv):
     """1,100 tokens, more steps of 128 keys than the ring has stages, at sizes that the tcgen05 kernel takes: one key that the last queries
     match, wherever it lies (the first positions, the borders of pages and of steps, late ones), and scores that rise from step to step,
     so that the outputs are rescaled every time."""
+    from pico_engine.ops import kernels
     from pico_engine.ops.library import mixers
     assert mixers().pe_attention_headmix_tcgen05_takes(H, G, D, Dv)
+    monkeypatch.setattr(kernels, "flashmix_prompts_pay", lambda *a: False)
     n, dt = 1100, torch.bfloat16
     g = torch.Generator().manual_seed(H)
     talk = torch.eye(H).roll(1, 0).double()

@@ -147,3 +147,25 @@ def test_plain_prefix_does_not_depend_on_what_follows():
     with torch.no_grad():
         a, b = plain.logits(toks, cfg, w), plain.logits(toks[:47], cfg, w)
     assert torch.allclose(a[:47], b, atol=1e-10)
+
+
+@pytest.mark.parametrize("sizes,in_ranges,whole", [
+    ((14, 2, 64, 64, False), [(17, 4096), (64, 16384)], [(64, 1000), (256, 4096), (1024, 0)]),        # heads, key/value heads, sizes, values in the rows
+    ((16, 4, 128, 128, False), [(2, 16384), (17, 16384)], [(64, 4096), (128, 16384), (17, 0)]),
+    ((8, 8, 64, 64, False), [(2, 1000), (64, 2000), (256, 16384)], [(128, 500), (256, 1000)]),
+    ((16, 1, 160, 128, True), [(2, 2000), (64, 4096), (128, 16384)], [(64, 500), (128, 1000), (2048, 0)]),
+    ((16, 1, 256, 192, True), [], [(2, 1000), (17, 4096), (64, 4096), (2048, 0)]),
+    ((4, 1, 256, 192, True), [(2, 16384), (64, 16384)], [(2, 1000), (64, 1000)])])
+def test_prompts_take_the_attention_that_was_measured_shorter(sizes, in_ranges, whole):
+    """Portions of a few tokens over a long context, whose keys can be cut into ranges, and what is shorter in one go: (tokens, cached
+    tokens) at which the two ways differed by a twentieth and more on a B200."""
+    from types import SimpleNamespace
+    from pico_engine.ops import kernels
+    H, G, D, Dv, in_keys = sizes
+    for way, steps in ((True, in_ranges), (False, whole)):
+        for new, before in steps:
+            ctx = SimpleNamespace(lens=[new], starts=[before])
+            assert kernels.flashmix_prompts_pay(ctx, H, G, D, Dv, None, in_keys) == way, (new, before)
+    ctx = SimpleNamespace(lens=[17], starts=[16384])                          # a window leaves few pages of a long context
+    assert not kernels.flashmix_prompts_pay(ctx, H, G, D, Dv, 100, in_keys)
+
