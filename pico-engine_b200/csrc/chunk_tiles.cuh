@@ -32,10 +32,11 @@ __device__ __forceinline__ float4 st_four(st_pair a, st_pair b) {
     return make_float4(x.x, x.y, y.x, y.y);
 }
 
-// Whether one of four numbers is an infinity or no number.  In a product of weights and a chunk's values a token's weight for the tokens in
+// Whether a value is an infinity or no number.  In a product of weights and a chunk's values a token's weight for the tokens in
 // front of it is zero, which keeps it out of their sums only while its values are finite: chunks where they are not take the products
-// token by token as far as they reach.  (No branch: it stands among loads that are to be asked for together.)
-__device__ __forceinline__ bool st_odd(const float4& v) { return !((fabsf(v.x) < INFINITY) & (fabsf(v.y) < INFINITY) & (fabsf(v.z) < INFINITY) & (fabsf(v.w) < INFINITY)); }
+// token by token as far as they reach.  st_zero adds zeros of four values to z; z is zero afterwards unless one of them was odd.
+// (No branch and no comparison: it stands among loads that are to be asked for together.)
+__device__ __forceinline__ void st_zero(float& z, const float4& v) { z = fmaf(v.x, 0.f, fmaf(v.y, 0.f, fmaf(v.z, 0.f, fmaf(v.w, 0.f, z)))); }
 
 // Columns c0 .. c0 + 31 of 64 rows (tokens) into dst[column][token]; entry (column k, token t) lies at k * 64 + (t ^ 4 ((k / 4) % 8)), so
 // that neither the four stores of a thread nor the reads of four neighbouring tokens meet in a bank.

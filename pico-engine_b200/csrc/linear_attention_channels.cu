@@ -308,17 +308,17 @@ __global__ void __launch_bounds__(ST_THREADS) lc_output_kernel(LAArgs a, const f
     float* vs = smem + ST_CHUNK * ST_CHUNK;                // [64 s][64 c]
     const float* w_src = weights + ((size_t)blockIdx.x * a.H + h) * ST_CHUNK * ST_CHUNK;
     const T* v_src = (const T*)a.proj + (size_t)first * a.ld + a.v_off + h * Dv + c0;
-    bool odd = false;
+    float zero = 0.f;
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
         const int i = tid + e * ST_THREADS, s = i >> 4, c = (i & 15) * 4;
         *reinterpret_cast<float4*>(pt + 4 * i) = *reinterpret_cast<const float4*>(w_src + 4 * i);
         const float4 v = s < n ? lc_load4(v_src + (size_t)s * a.ld + c, Dv - c0 - c, vec_v) : make_float4(0.f, 0.f, 0.f, 0.f);
         const float4 u = make_float4(la_act<FAST>(v.x, a.act_v), la_act<FAST>(v.y, a.act_v), la_act<FAST>(v.z, a.act_v), la_act<FAST>(v.w, a.act_v));
-        odd |= st_odd(u);
+        st_zero(zero, u);
         *reinterpret_cast<float4*>(vs + 4 * i) = u;
     }
-    const bool guarded = __syncthreads_or(odd);
+    const bool guarded = __syncthreads_or(zero != 0.f);
     const int last = min(n, 32 + 16 * (tid >> 6) + 16);    // a warp's tokens reach this far: later ones have no weight
     st_weighted(acc, pt, vs, last, ty, tx, guarded);
 #pragma unroll

@@ -161,7 +161,9 @@ __global__ void __launch_bounds__(ST_THREADS) st_contribution_kernel(ScanArgs a,
 }
 
 // A thread an element of a sequence's state walks the sequence's chunks in order, leaves every chunk its incoming state where its own
-// contribution was, and stores the sequence's new state (whose order is that of state_space.cu's threads).
+// contribution was, and stores the sequence's new state (whose order is that of state_space.cu's threads).  ONE: the step is one slab, the
+// usual case (with the slab's bounds in the loop's the compiler keeps fewer of the eight reads in flight: 65 us instead of 32).
+template <bool ONE>
 __global__ void __launch_bounds__(256) st_carry_kernel(ScanArgs a) {
     pdl_launch_dependents();
     pdl_wait();
@@ -171,23 +173,27 @@ __global__ void __launch_bounds__(256) st_carry_kernel(ScanArgs a) {
     if (e >= per) return;
     int base = 0;
     for (int i = 0; i < b; ++i) base += (a.row_lens[i] + SS_CHUNK - 1) / SS_CHUNK;
-    // the sequence's chunks of this slab, by their places in it
-    const int begin = max(base - a.first_chunk, 0), end = min(base + (a.row_lens[b] + SS_CHUNK - 1) / SS_CHUNK - a.first_chunk, a.slab);
-    if (begin >= end) return;
+    int nc = (a.row_lens[b] + SS_CHUNK - 1) / SS_CHUNK;
+    if (!ONE) {                                           // the sequence's chunks of this slab, by their places in it
+        const int end = min(base + nc - a.first_chunk, a.slab);
+        base = max(base - a.first_chunk, 0);
+        nc = max(end - base, 0);
+    }
+    if (nc == 0) return;
     const int h = (int)(e / per_head), r = (int)(e % per_head) / a.P, p = (int)(e % per_head) % a.P;
     float* sp = a.state + (size_t)a.slots[b] * a.state_stride + (((size_t)h * a.NR + r % a.NR) * a.P + p) * a.NS + r / a.NR;
     float carry = *sp;
-    for (int c0 = begin; c0 < end; c0 += 8) {           // eight chunks' numbers in flight: they do not depend on the carry
+    for (int c0 = base; c0 < base + nc; c0 += 8) {           // eight chunks' numbers in flight: they do not depend on the carry
         float own[8], dec[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-            const bool there = c0 + u < end;
+            const bool there = c0 + u < base + nc;
             own[u] = there ? a.chunk_state[(size_t)(c0 + u) * per + e] : 0.f;
             dec[u] = there ? a.chunk_decay[(size_t)(c0 + u) * a.H + h] : 0.f;
         }
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-            if (c0 + u < end) {
+            if (c0 + u < base + nc) {
                 a.chunk_state[(size_t)(c0 + u) * per + e] = carry;
                 carry = fmaf(dec[u], carry, own[u]);
             }
@@ -256,7 +262,7 @@ __global__ void __launch_bounds__(ST_THREADS) st_output_kernel(ScanArgs a, int v
     float* xs = smem + SS_CHUNK * SS_CHUNK;                // [64 s][64 p]
     const float* scores = a.chunk_scores + ((size_t)blockIdx.x * a.G + g) * SS_CHUNK * SS_CHUNK;
     const float* x_src = a.xbc + (size_t)first * a.xbc_ld + h * P + p0;
-    bool odd = false;
+    float zero = 0.f;
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
         const int i = tid + e * ST_THREADS, s = i >> 4, t = (i & 15) * 4;
@@ -269,7 +275,7 @@ __global__ void __launch_bounds__(ST_THREADS) st_output_kernel(ScanArgs a, int v
         w.z = s <= t + 2 ? w.z * (d * expf((float)(las[t + 2] - ls))) : 0.f;
         w.w = s <= t + 3 ? w.w * (d * expf((float)(las[t + 3] - ls))) : 0.f;
         *reinterpret_cast<float4*>(pt + 4 * i) = w;
-        odd |= st_odd(x);
+        st_zero(zero, x);
         *reinterpret_cast<float4*>(xs + 4 * i) = x;
     }
 #pragma unroll
@@ -279,7 +285,7 @@ __global__ void __launch_bounds__(ST_THREADS) st_output_kernel(ScanArgs a, int v
         asm("mov.b64 %0, {%1, %2};" : "=l"(acc[i][0]) : "f"(u.x * d), "f"(u.y * d));
         asm("mov.b64 %0, {%1, %2};" : "=l"(acc[i][1]) : "f"(v.x * d), "f"(v.y * d));
     }
-    const bool guarded = __syncthreads_or(odd);
+    const bool guarded = __syncthreads_or(zero != 0.f);
     const int last = min(n, 32 + 16 * (tid >> 6) + 16);    // a warp's tokens reach this far: later ones have no weight
     st_weighted(acc, pt, xs, last, ty, tx, guarded);
     const float Dh = load_as_f(a.d_skip, a.d_dtype, h);
@@ -301,7 +307,7 @@ static int st_run(ScanArgs a, cudaStream_t s) {
     for (; a.first_chunk < a.chunks; a.first_chunk += a.slab) {      // (the carry between two slabs lies in the sequences' states)
         PE_TRY(pe_launch(st_contribution_kernel<T>, dim3(a.slab, a.H + a.G, tn * tp), ST_THREADS, 0, s, a, vec_bc, vec_x, tn));
         PE_LAUNCH_CHECK();
-        PE_TRY(pe_launch(st_carry_kernel, dim3((unsigned)(((size_t)a.H * a.N * a.P + 255) / 256), a.B), 256, 0, s, a));
+        PE_TRY(pe_launch(a.slab == a.chunks ? st_carry_kernel<true> : st_carry_kernel<false>, dim3((unsigned)(((size_t)a.H * a.N * a.P + 255) / 256), a.B), 256, 0, s, a));
         PE_LAUNCH_CHECK();
         PE_TRY(pe_launch(st_output_kernel<T>, dim3(a.slab, a.H, tp), ST_THREADS, 0, s, a, vec_bc, vec_x));
         PE_LAUNCH_CHECK();
