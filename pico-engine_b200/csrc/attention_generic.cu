@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(AG_THREADS) attention_generic_kernel(
 // 14 heads of 64, prompts of 301 and 207 tokens, on a B200: 645 us by the kernel above (a block a token and head, which read every key
 // and value once a head), 75 us here.
 #define AT_THREADS 256
-#define AG_RUN 64                                         // tokens of a run at most
+#define AG_RUN 128                                        // tokens of a run at most
 
 struct AttentionTileArgs {
     const void* q; int q_stride; void* out; const void* k_pool; const void* v_pool;
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tile_kernel(AttentionTil
     pdl_wait();
     constexpr int RT = R / 16;                             // rows a thread
     extern __shared__ __align__(16) float ag_smem[];
-    __shared__ int pos_s[R], seq_s[R];
+    __shared__ int pos_s[R], row_s[R], run_s[R], last_s;
     const int hd = a.hd, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, per4 = hd / 4;
     float* qt = ag_smem;                                   // [hd][64]: the rows' queries, turned (R of 64 places used)
     float* kt = qt + hd * 64;                              // [hd][64]: a page's keys, turned
@@ -148,7 +148,15 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tile_kernel(AttentionTil
     if (tid < R) {
         const int t = t0 + min(tid, rows - 1) / n_heads;
         pos_s[tid] = a.tok_pos[t];
-        seq_s[tid] = tid < rows ? a.tok_row[t] : -1;
+        row_s[tid] = tid < rows ? a.tok_row[t] : -1;
+    }
+    // a row's run: the first of the rows of its sequence that stand together with it
+    const bool one = a.runs || a.tokens == 1;              // (one sequence: the first row)
+    if (!one) __syncthreads();
+    if (!one && tid < (R < 32 ? 32 : R)) {
+        const unsigned begins = __ballot_sync(0xffffffffu, tid < R && (tid == 0 || row_s[tid] != row_s[tid - 1])) & (0xffffffffu >> (31 - (tid & 31)));
+        if (tid < R) run_s[tid] = begins ? (tid & ~31) + 31 - __clz(begins) : -1;
+        if (tid == 31) last_s = 31 - __clz(begins);        // (of the first 32 rows' runs: the first row always begins one)
     }
     for (int i = tid; i < R * per4; i += AT_THREADS) {
         const int r = i / per4, c = i % per4 * 4;
@@ -159,11 +167,11 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tile_kernel(AttentionTil
     __syncthreads();
     float m[RT], l[RT];
     float4 acc[RT][NJ];
-    int my_pos[RT];
+    int my_pos[RT], my_run[RT];
 #pragma unroll
     for (int i = 0; i < RT; ++i) {
         m[i] = -INFINITY; l[i] = 0.f;
-        my_pos[i] = pos_s[ty * RT + i];
+        my_pos[i] = pos_s[ty * RT + i]; my_run[i] = one ? (ty * RT + i < rows ? 0 : -1) : run_s[ty * RT + i] >= 0 ? run_s[ty * RT + i] : last_s;
 #pragma unroll
         for (int j = 0; j < NJ; ++j) acc[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
@@ -185,9 +193,9 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tile_kernel(AttentionTil
     };
     auto turn = [&](int j, int c, const float4& k) { kt[ag_turned(c, j)] = k.x; kt[ag_turned(c + 1, j)] = k.y; kt[ag_turned(c + 2, j)] = k.z; kt[ag_turned(c + 3, j)] = k.w; };
     for (int from = 0; from < rows;) {                     // the rows of one sequence that stand together, after them the next ones
-        const int seq = seq_s[from];
+        const int seq = row_s[from];
         int to = from + n_heads, lowest = pos_s[from], highest = lowest;
-        while (to < rows && seq_s[to] == seq) { lowest = min(lowest, pos_s[to]); highest = max(highest, pos_s[to]); to += n_heads; }
+        while (to < rows && row_s[to] == seq) { lowest = min(lowest, pos_s[to]); highest = max(highest, pos_s[to]); to += n_heads; }
         const int* table = a.table + (size_t)seq * a.table_stride;
         const int page_lo = a.window > 0 && lowest - a.window + 1 > 0 ? (lowest - a.window + 1) / PE_PAGE : 0;
         const int page_hi = highest / PE_PAGE;
@@ -241,8 +249,7 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tile_kernel(AttentionTil
             bool whole = true;                             // this thread's rows see the whole page
 #pragma unroll
             for (int i = 0; i < RT; ++i) {
-                const bool mine = ty * RT + i >= from && ty * RT + i < to;
-                const int hi = mine ? my_pos[i] - key0 : -1, lo = a.window > 0 ? hi - a.window + 1 : 0;      // keys lo .. hi of the four
+                const int hi = my_run[i] == from ? my_pos[i] - key0 : -1, lo = a.window > 0 ? hi - a.window + 1 : 0;      // keys lo .. hi of the four
                 s[i].x = hi >= 0 && lo <= 0 ? s[i].x * a.scale : -INFINITY;
                 s[i].y = hi >= 1 && lo <= 1 ? s[i].y * a.scale : -INFINITY;
                 s[i].z = hi >= 2 && lo <= 2 ? s[i].z * a.scale : -INFINITY;
@@ -256,14 +263,14 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tile_kernel(AttentionTil
                 float sum = (s[i].x + s[i].y) + (s[i].z + s[i].w);
 #pragma unroll
                 for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-                if (mine) {
+                if (my_run[i] == from) {
                     l[i] = l[i] * alpha + sum;
                     m[i] = m_new;
 #pragma unroll
                     for (int j = 0; j < NJ; ++j) { acc[i][j].x *= alpha; acc[i][j].y *= alpha; acc[i][j].z *= alpha; acc[i][j].w *= alpha; }
                 }
                 const int first_key = pg * PE_PAGE;
-                whole = whole && mine && my_pos[i] >= first_key + PE_PAGE - 1 && (a.window <= 0 || my_pos[i] - first_key < a.window);
+                whole = whole && my_run[i] == from && my_pos[i] >= first_key + PE_PAGE - 1 && (a.window <= 0 || my_pos[i] - first_key < a.window);
             }
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
@@ -328,19 +335,20 @@ static int attention_tile_as(AttentionTileArgs a, int n_runs, int most, cudaStre
 template <typename T>
 static int attention_tile(const AttentionTileArgs& a, int n_runs, int sequences, cudaStream_t s) {
     const int per = a.nh / a.nkv, few = per < 16 ? 16 / per : 1;      // tokens of a block of 16 rows
-    // Which blocks: 16 rows while all those run at once, else 64.  Where no runs are known a block may get tokens of several sequences, which
-    // it serves one after the other: no more of them than an eighth of what a sequence brings on average, and so single ones where they bring few.
+    // Which blocks: 16 rows while those fill half of the SMs at most, else 64 (14 heads of 64 on 2, 60 tokens alone 7.6 / 10.5 us, 20 behind
+    // 4,000 261 / 363, 100 behind 4,000 418 / 373).  Where no runs are known a block may get tokens of several sequences, which
+    // it serves one after the other: no more of them than a quarter of what a sequence brings on average, and so single ones where they bring few.
     // One prompt of 40 tokens beside 30 single tokens at 600, float32, on a B200, a block a token and head / 64 rows of neighbouring tokens
     // / runs: 14 heads of 64 on 2 255 / 506 / 69 us, 4 of 256 on one 275 / 3,801 / 138.
-    const int most = a.runs ? AG_RUN : sequences > 0 && a.T / sequences >= 16 ? a.T / sequences / 8 : 1;
+    const int most = a.runs ? AG_RUN : sequences > 0 && a.T / sequences >= 16 ? a.T / sequences / 4 : 1;
     const int blocks16 = (a.T + min(few, most) - 1) / min(few, most);
-    const bool wide = (long long)most * per > 16 && (long long)blocks16 * a.nkv * ((per + 15) / 16) > 148;
+    const bool wide = (long long)most * per > 16 && (long long)blocks16 * a.nkv * ((per + 15) / 16) > 74;
     if (a.hd <= 64) return wide ? attention_tile_as<T, 64, 1>(a, n_runs, most, s) : attention_tile_as<T, 16, 1>(a, n_runs, most, s);
     if (a.hd <= 128) return wide ? attention_tile_as<T, 64, 2>(a, n_runs, most, s) : attention_tile_as<T, 16, 2>(a, n_runs, most, s);
     return wide ? attention_tile_as<T, 64, 4>(a, n_runs, most, s) : attention_tile_as<T, 16, 4>(a, n_runs, most, s);
 }
 
-// runs: null, or [n_runs] of (batch row, first packed token, number of tokens (<= 64), ..): the step's tokens, each in one of them
+// runs: null, or [n_runs] of (batch row, first packed token, number of tokens (<= 128), ..): the step's tokens, each in one of them
 extern "C" int pe_attention_generic(const void* q, int q_stride, void* out, const void* k_pool, const void* v_pool,
                                     int dtype, const int* block_table, int table_stride, const int* tok_pos,
                                     const int* tok_row, int T, int nh, int nkv, int hd, int window, float scale, int sequences,

@@ -177,7 +177,7 @@ def attention_generic(q: torch.Tensor, q_stride: int, n_heads: int, n_kv_heads: 
                       tok_pos: torch.Tensor, tok_row: torch.Tensor, window: Optional[int], scale: float,
                       out: Optional[torch.Tensor] = None, runs: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Attention of T tokens over the cache.  ``q`` holds the query heads of token t at
-    ``t * q_stride + h * head_dim``; the result is [T, n_heads * head_dim] in q's dtype.  ``runs``: the tokens as runs of at most 64 of
+    ``t * q_stride + h * head_dim``; the result is [T, n_heads * head_dim] in q's dtype.  ``runs``: the tokens as runs of at most 128 of
     one sequence (``prefill_tiles``), for steps that bring prompts; the result does not depend on it."""
     T = tok_pos.shape[0]
     _need(q, "q"); _need(k_pool, "k_pool", q.dtype); _need(v_pool, "v_pool", q.dtype, k_pool.shape)
@@ -418,11 +418,8 @@ def attention(q: torch.Tensor, q_stride: int, n_heads: int, n_kv_heads: int, hea
         run = attention_prefill_tcgen05 if tcgen05 else attention_prefill
         return run(q, q_stride, n_heads, n_kv_heads, head_dim, k_pool, v_pool, block_table, table_stride, tiles,
                    tok_pos.shape[0], window, scale)
-    # (where every row is a prompt, blocks of neighbouring tokens cross from one to the next so seldom that the runs' last, partly filled
-    # blocks cost more: prompts of 301 and 207 tokens, two layers of 14 heads of 64, 897 us without and 909 with)
-    runs = None if all(n == 0 or n >= PREFILL_TILE for n in ctx.lens) or ctx.one_token_each else _step_tiles(ctx, PREFILL_TILE, q.device)
-    return attention_generic(q, q_stride, n_heads, n_kv_heads, head_dim, k_pool, v_pool, block_table, table_stride,
-                             tok_pos, tok_row, window, scale, runs=runs)
+    return attention_generic(q, q_stride, n_heads, n_kv_heads, head_dim, k_pool, v_pool, block_table, table_stride, tok_pos, tok_row, window, scale,
+                             runs=None if ctx.one_token_each else _step_tiles(ctx, PREFILL_TILE_TCGEN05, q.device))
 
 
 # ---------------------------------------------------------------------------- fused decode products (bfloat16, up to 16 rows)

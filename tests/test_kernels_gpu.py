@@ -1042,7 +1042,7 @@ def test_product_choice_is_made_once_and_both_ways_agree(K):
 @pytest.mark.parametrize("nh,nkv,hd,window", [(14, 2, 64, None), (3, 3, 40, 70), (20, 1, 16, None), (4, 1, 256, None)])
 @pytest.mark.parametrize("new,before", [([40] + [1] * 9, [0] + [200] * 9), ([5], [130]), ([200, 1, 129, 64], [0, 300, 7, 64])])
 def test_attention_generic_in_runs_of_one_sequence(K, nh, nkv, hd, window, new, before):
-    """Steps that bring prompts beside single tokens, as runs of one sequence each (16 and 64 rows a block, runs of one token up to 64):
+    """Steps that bring prompts beside single tokens, as runs of one sequence each (16 and 64 rows a block, runs of one token up to 128):
     the same bits as token by token."""
     lens = [n + b for n, b in zip(new, before)]
     paged = Paged(lens, nkv, hd, torch.float32, seed=hd)
@@ -1052,7 +1052,7 @@ def test_attention_generic_in_runs_of_one_sequence(K, nh, nkv, hd, window, new, 
     i32 = lambda v: dev(torch.tensor(v, dtype=torch.int32))                          # noqa: E731
     run = lambda i, runs: K.attention_generic(dev(q[i].contiguous()), nh * hd, nh, nkv, hd, kp, vp, table, table.shape[1], i32([pos[j] for j in i]),
                                               i32([row[j] for j in i]), window, hd ** -0.5, runs=runs)
-    whole = run(list(range(len(row))), K.prefill_tiles(new, before, "cuda"))
+    whole = run(list(range(len(row))), K.prefill_tiles(new, before, "cuda", K.PREFILL_TILE_TCGEN05))
     for j in sorted({0, len(row) - 1, len(row) // 2, new[0] - 1, new[0] % len(row)}):
         assert torch.equal(run([j], None)[0], whole[j]), j
     assert torch.equal(run(list(range(len(row))), None), whole)
