@@ -7,6 +7,7 @@
 // one and one, plus 64 a token and entry of q and v.  All sums are float32 multiply-adds; the powers of a are worked out in float64.
 // Queries, keys (and values, in float32) go through their activation and scale while they are brought to shared memory.
 #include "linear_attention.cuh"
+#include "chunk_tiles.cuh"
 
 #define LT_THREADS 256
 
@@ -177,7 +178,10 @@ __global__ void __launch_bounds__(LT_THREADS, 2) lt_output_kernel(LAArgs a, int 
         kt[(d + 0) * C + t] = k.x; kt[(d + 1) * C + t] = k.y; kt[(d + 2) * C + t] = k.z; kt[(d + 3) * C + t] = k.w;
     }
     v_rows.template store<FAST>(vs, a.act_v, [](int) { return 1.f; });
-    __syncthreads();
+    float zero = 0.f;
+#pragma unroll
+    for (int e = 0; e < LTRows<T, TV>::N; ++e) st_zero(zero, v_rows.v[e]);
+    const bool guarded = __syncthreads_or(zero != 0.f);
     {
         float4 w[4];
 #pragma unroll
@@ -245,7 +249,7 @@ __global__ void __launch_bounds__(LT_THREADS, 2) lt_output_kernel(LAArgs a, int 
     }
     const int last = min(n, 16 * (warp >> 1) + 16);       // a warp's tokens are sixteen neighbours: later keys have no weight
 #pragma unroll 4
-    for (int s = 0; s < last; ++s) {
+    for (int s = 0; s < (guarded ? 0 : last); ++s) {
         const float4 p = *reinterpret_cast<const float4*>(pt + s * C + ty * 4);
 #pragma unroll
         for (int j = 0; j < RV / 4; ++j) {
@@ -253,6 +257,14 @@ __global__ void __launch_bounds__(LT_THREADS, 2) lt_output_kernel(LAArgs a, int 
             lt_fma4(acc[0][j], p.x, v); lt_fma4(acc[1][j], p.y, v); lt_fma4(acc[2][j], p.z, v); lt_fma4(acc[3][j], p.w, v);
         }
     }
+#pragma unroll 1
+    for (int s = 0; s < (guarded ? last : 0); ++s)        // some value is no finite number: a token joins the sums of none in front of it
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (s <= ty * 4 + i) {
+#pragma unroll
+                for (int j = 0; j < RV / 4; ++j) lt_fma4(acc[i][j], pt[s * C + ty * 4 + i], *reinterpret_cast<const float4*>(vs + s * TV + tx * 4 + 64 * j));
+            }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int t = ty * 4 + i;

@@ -598,3 +598,23 @@ def test_chunks_in_slabs(per_channel):
     for walk, chunks in zip(*got):
         # float32 sums of the same products in another order (the bound of the tests above)
         assert (walk - chunks).abs().max() < 2e-5 * max(1.0, float(walk.abs().max()))
+
+
+@pytest.mark.parametrize("odd", [float("nan"), float("inf")])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("which", ["q", "k", "v"])
+def test_a_token_that_is_no_number_does_not_reach_back_with_a_decay_per_head(which, dtype, odd):
+    """The same with one decay a head."""
+    dt, H, D, Dv, lens = DTYPES[dtype], 2, 24, 70, [130, 40]
+    g = torch.Generator().manual_seed(8)
+    T = sum(lens)
+    ins = {n: torch.randn(T, H, d, generator=g).to(dt).float() for n, d in (("q", D), ("k", D), ("v", Dv))}
+    run = lambda t, chunked: run_recurrence(t["q"], t["k"], t["v"], dt, lens, head_decay=[0.95, 0.99], chunked=chunked)
+    clean = run(ins, True)[0]
+    for at in (5, 63, 100):
+        bad = dict(ins, **{which: ins[which].clone()})
+        bad[which][at, 0, ::3] = odd
+        (o, s), (o_walk, s_walk) = run(bad, True), run(bad, False)
+        assert torch.equal(o[:at], clean[:at]) and torch.equal(o[lens[0]:], clean[lens[0]:]), at
+        assert torch.equal(o.isfinite(), o_walk.isfinite()) and torch.equal(s.isfinite(), s_walk.isfinite()), at
+
