@@ -605,8 +605,9 @@ extern "C" void pe_attention_decode_set_max_splits(int n) { ad_split_limit() = n
 //                  8.1 us; 1 sequence: 4.9 against 5.3, 64 sequences 24 against 27 where the rule does not hold)
 //                  4 warps where a range is 1 or 2 pages long, the merge of fewer warps being most of what is left (1 sequence of
 //                  600 tokens 4.1 against 3.8 us, 8 of 2,000 7.2 against 6.5; with 3 pages a range they lose: 12 of 2,000 6.9, 7.2), but
-//                  not two ranges of a page, nor ranges of 2 pages, where every CTA has an SM to itself (1 of 128 tokens 4.0, 4.2; 1
-//                  of 2,000 4.6, 4.9), nor whole sequences of 2 pages that run at once (128 of 128 tokens 4.6, 4.8)
+//                  not two ranges of a page with less than three CTAs on two SMs (1 of 128 tokens 4.0, 4.2, 40 of 128 4.9, 5.0; 64 of
+//                  128 5.6, 5.3), nor ranges of 2 pages where every CTA has an SM to itself (1 of 2,000 4.6, 4.9), nor whole
+//                  sequences of 2 pages that run at once (128 of 128 tokens 4.6, 4.8)
 //   head size 128  4 warps, two CTAs an SM, where one CTA an SM leaves the triples whole but two allow three ranges (19
 //                  sequences of 4,000 tokens and 4 kv heads 37.5 against 26.6 us, of 1,000 12.3 against 11.3; of 640 equal), and
 //                  where all triples of short sequences then run in one turn instead of two (64 sequences of 500 tokens 15.4
@@ -628,7 +629,7 @@ static AdShape ad_choose(int T, int nh, int nkv, int max_context) {
     if constexpr (AD_HD <= 128) {                            // larger heads leave room for one page only
         AdShape n = {4, 1, 1};
         n.splits = AdVariant<4>::shape(ctas, pages, limit, &n.stages);
-        if (AD_HD <= 64 ? range(n.splits) == 1 ? n.splits != 2 || 2 * ctas > 148 : range(n.splits) == 2 && n.splits * ctas > (n.splits == 1 ? 2 : 1) * 148
+        if (AD_HD <= 64 ? range(n.splits) == 1 ? n.splits != 2 || 2 * ctas > 222 : range(n.splits) == 2 && n.splits * ctas > (n.splits == 1 ? 2 : 1) * 148
                         : (c.splits == 1 && n.splits >= 3 && pages >= 16) || (ctas > 148 && ctas <= 2 * 148 && pages <= (ctas < 192 ? 8 : 12)))
             return n;
     }
