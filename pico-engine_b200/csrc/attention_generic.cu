@@ -339,7 +339,7 @@ static int attention_tile(const AttentionTileArgs& a, int n_runs, int sequences,
     // 4,000 261 / 363, 100 behind 4,000 418 / 373).  Where no runs are known a block may get tokens of several sequences, which
     // it serves one after the other: no more of them than a quarter of what a sequence brings on average, and so single ones where they bring few.
     // One prompt of 40 tokens beside 30 single tokens at 600, float32, on a B200, a block a token and head / 64 rows of neighbouring tokens
-    // / runs: 14 heads of 64 on 2 255 / 506 / 69 us, 4 of 256 on one 275 / 3,801 / 138.
+    // / runs: 14 heads of 64 on 2 255 / 506 / 71 us, 4 of 256 on one 275 / 3,801 / 173.
     const int most = a.runs ? AG_RUN : sequences > 0 && a.T / sequences >= 16 ? a.T / sequences / 4 : 1;
     const int blocks16 = (a.T + min(few, most) - 1) / min(few, most);
     const bool wide = (long long)most * per > 16 && (long long)blocks16 * a.nkv * ((per + 15) / 16) > 74;

@@ -17,7 +17,7 @@
 //
 // Tensor memory has 256 columns for S and 256 for O: two value heads of 128 or four of 64 a CTA; more are further CTAs, which make S again.
 // Bound by a step's chain (scores, maximum, exponentials, P) rather than by the tensor cores.
-// Measured on a B200, 1,024 tokens, 16 heads of 128 on four key/value heads: 40 + 15 us, where the mma.sync kernel and its merge
+// Measured on a B200, 1,024 tokens, 16 heads of 128 on four key/value heads: 40 + 7 us, where the mma.sync kernel and its merge
 // (attention_headmix_flash.cu) take 198 + 83.
 // Head sizes: D a multiple of 16, Dv of 16.  Every mbarrier wait is bounded by the clock; a wait that runs out sets *status to 5, the
 // roles leave their loops, tensor memory is freed and the CTA returns (status 6: shared memory did not start on a 1024-byte boundary).

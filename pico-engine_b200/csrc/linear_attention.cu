@@ -22,8 +22,8 @@
 //  * chunked (prompts): a sequence's tokens are cut into chunks of LA_CHUNK.  The recurrence is linear in S,
 //    S_end = diag(A) S_in + L with A the product of the chunk's decays and L the chunk's own contribution, so
 //    pass 1 computes (A, L) of every chunk from S_in = 0, pass 2 walks a sequence's chunks in order (an element
-//    a thread), leaves each chunk's S_in where its L was and stores the sequence's new state, and pass 3 runs
-//    every chunk again from its S_in and writes the outputs.  Passes 1 and 3 are products of tiles (a decay per head:
+//    a thread), leaves each chunk's S_in where its L was and stores the sequence's new state, and pass 3 works
+//    out every chunk's outputs from its S_in.  Passes 1 and 3 are products of tiles (a decay per head:
 //    linear_attention_tiles.cu, per channel: linear_attention_channels.cu).  Chunks never cross sequences: chunk c of the step
 //    is found from the rows' lengths on the device, so the grid depends on (T, B) only.
 #include "linear_attention.cuh"

@@ -933,7 +933,8 @@ def attention_latent_prompt(q: torch.Tensor, q_stride: int, n_heads: int, width:
     """Attention of a step that brings prompts over low-rank rows (``pool`` [pages, 1, PAGE, width], whose first ``rank`` entries are the
     values) on the tcgen05 tensor cores: [T, n_heads * rank], head h of token t times sigmoid(gate[t, gate_offset + h]) where ``gate``
     [T, ld] is given; or None for what that kernel does not take (single tokens, other dtypes and sizes).  Measured on a B200 at 2,048
-    tokens, 16 heads on rows of 192 + 64: 44 us against 667 us of the mma.sync kernel, so it runs wherever it takes the sizes."""
+    tokens, 16 heads on rows of 192 + 64: 44 us against 667 us of the mma.sync kernel; the callers ask ``flashmix_prompts_pay`` whether
+    a step is one of the few that are shorter there."""
     if q.dtype != torch.bfloat16 or ctx.one_token_each or scale <= 0 or q_stride % 8 or HEADMIX_TENSOR_CORES != "1":
         return None
     from .library import state_space
@@ -1025,7 +1026,7 @@ def attention_headmix(q: torch.Tensor, q_stride: int, n_heads: int, n_kv: int, h
             and lib.pe_attention_headmix_tcgen05_takes(n_heads, n_kv, head_dim, v_head_dim)
             and not flashmix_prompts_pay(ctx, n_heads, n_kv, head_dim, v_head_dim, window)):
         # prompts whose weights are mixed: both products on tcgen05, the mixing behind them (1,024 tokens, 16
-        # heads of 128 on four key/value heads on a B200: 55 us against 281 us of the mma.sync kernel and its merge)
+        # heads of 128 on four key/value heads on a B200: 47 us against 281 us of the mma.sync kernel and its merge)
         runs = _step_tiles(ctx, PREFILL_TILE_TCGEN05, q.device)
         ws = scratch("attention_headmix", 4 * T * n_heads * n_kv * v_head_dim, q.device)
         check(lib.pe_attention_headmix_tcgen05(q.data_ptr(), q_stride, out.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), k_pool.shape[0],

@@ -316,7 +316,7 @@ SHAPE_CASES = [                       # (nh, nkv, hd, sequences, longest, bound 
     (14, 2, 64, 24, 128, 128), (2, 1, 16, 8, 300, 300),
     (16, 4, 128, 19, 1024, 1024), (16, 4, 128, 19, 960, 960),         # three ranges instead of none, from 16 pages on
     (16, 4, 128, 40, 500, 512), (16, 4, 128, 37, 500, 513),           # more triples than SMs: 4 warps up to 8 pages, then 8
-    (8, 2, 80, 74, 400, 512), (8, 2, 80, 75, 800, 833),               # as many as SMs, then the longest first
+    (8, 2, 80, 74, 400, 512), (8, 2, 80, 75, 800, 833),               # as many as SMs, then more
     (4, 4, 128, 40, 833, 833), (1, 1, 128, 256, 900, 900), (1, 1, 128, 257, 900, 900),
 ]
 
