@@ -44,7 +44,7 @@ __device__ __forceinline__ void hn_weights8(const void* w, int dtype, int at, fl
 // holds eight entries; else a head is a warp and a lane holds every 32nd entry.  Normed rows meet in shared memory as float32 for the
 // rotation.  A block a token (VEC: or gridDim.y blocks, each with its share of the heads, where the tokens are few); a pass's entries are
 // asked for before the pass in front of it, and the first one's before the angles, are worked out.
-template <typename T, bool VEC>
+template <typename T, bool VEC, bool LANES>
 __global__ void __launch_bounds__(HN_THREADS, 4) heads_norm_store_kernel(HeadsNormArgs a) {
     pdl_launch_dependents();
     __shared__ float s_cos[HN_MAX_D / 2], s_sin[HN_MAX_D / 2];
@@ -79,17 +79,21 @@ __global__ void __launch_bounds__(HN_THREADS, 4) heads_norm_store_kernel(HeadsNo
             }
         }
         __syncthreads();
-        // Where half a rotation is whole lanes, entry e turns with entry e of the lane `turn` further on (or back), by angles that the lane
+        // LANES: half a rotation is whole lanes, and entry e turns with entry e of the lane `turn` further on (or back), by angles that the lane
         // keeps: no exchange through shared memory, whose reads eight entries apart met on four banks.  2,000 tokens of 32 + 8 heads of 64 that turn
         // 48 entries: 17.8 to 16.3 us, and 13.6 with eight blocks of 128 threads an SM instead of six (64 registers a thread).
-        const int turn = half % 8 == 0 ? half / 8 : 0;
-        const bool front = l < turn, turns = turn && l < 2 * turn;
+        // An instance of its own, because other rotations paid for the angles that they do not keep: one token of 16 + 4 heads of 32 that
+        // turn 24 entries, 3.3 us with them and 2.9 without; 6,000 such tokens, 22.3 and 20.5.  (6,000 of 32 + 8 heads of 64 that turn 48: 28.9 and 27.3.)
+        const int turn = LANES ? half / 8 : 0;
+        const bool front = l < turn, turns = l < 2 * turn;
         const int partner = front ? lane + turn : lane - turn;
         float cs[8], sn[8];
+        if constexpr (LANES) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const int d = front ? l * 8 + e : l * 8 + e - half;
-            cs[e] = turns ? s_cos[d] : 1.f; sn[e] = turns ? s_sin[d] : 0.f;
+            for (int e = 0; e < 8; ++e) {
+                const int d = front ? l * 8 + e : l * 8 + e - half;
+                cs[e] = turns ? s_cos[d] : 1.f; sn[e] = turns ? s_sin[d] : 0.f;
+            }
         }
         for (int h_first = h - sub; h_first < n_heads; h_first += step, h += step) {      // (the whole warp together)
             const bool live = on && h < n_heads;
@@ -111,7 +115,7 @@ __global__ void __launch_bounds__(HN_THREADS, 4) heads_norm_store_kernel(HeadsNo
 #pragma unroll
                 for (int e = 0; e < 8; ++e) f[e] *= rstd * (query ? qw[e] : kw[e]);
             }
-            if (turn) {
+            if constexpr (LANES) {
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
                     const float other = __shfl_sync(0xffffffffu, f[e], turns ? partner : lane);
@@ -193,10 +197,10 @@ extern "C" int pe_heads_norm_store(void* proj, int dtype, int ld, int T, int H, 
     while (p < D / 8) p <<= 1;
     const int per_pass = (HN_THREADS / 32) * (32 / p), passes = (H + G + per_pass - 1) / per_pass;
     const bool few = T * passes <= 4 * 148;
-    if (dtype == PE_F32) PE_TRY(pe_launch(heads_norm_store_kernel<float, false>, T, HN_THREADS, 0, s, a));
+    if (dtype == PE_F32) PE_TRY(pe_launch(heads_norm_store_kernel<float, false, false>, T, HN_THREADS, 0, s, a));
     else if (dtype != PE_BF16) return PE_ERR_UNSUPPORTED;
-    else if (vec) PE_TRY(pe_launch(heads_norm_store_kernel<bf16, true>, dim3(T, few ? passes : 1), few ? HN_THREADS : 128, 0, s, a));
-    else PE_TRY(pe_launch(heads_norm_store_kernel<bf16, false>, T, HN_THREADS, 0, s, a));
+    else if (vec) PE_TRY(pe_launch(rot && rot % 16 == 0 ? heads_norm_store_kernel<bf16, true, true> : heads_norm_store_kernel<bf16, true, false>, dim3(T, few ? passes : 1), few ? HN_THREADS : 128, 0, s, a));
+    else PE_TRY(pe_launch(heads_norm_store_kernel<bf16, false, false>, T, HN_THREADS, 0, s, a));
     PE_LAUNCH_CHECK();
     return 0;
 }
