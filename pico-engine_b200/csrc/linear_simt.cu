@@ -1,7 +1,7 @@
 // out[M, N] = A[M, K] . W[N, K]^T (+ bias[N]) on the CUDA cores: float32 multiply-add for
-// every product, whatever the storage dtype of A and W.  This is the matrix product of the
-// true 32-bit path (no tensor-core or reduced-precision mode is involved) and the fallback
-// for operand dtypes that the tensor-core kernels do not take.
+// every product, whatever the storage dtype of A and W.  This is the matrix product of operands
+// that are not stored alike, of small float32 matrices and of a K that is no multiple of eight;
+// other float32 products are linear_split.cu's.
 //
 // K is cut into ranges whose number depends on N and K only.  The sum over k of one output element
 // runs in increasing k inside a range, one fused multiply-add per k, and the ranges' sums are added in

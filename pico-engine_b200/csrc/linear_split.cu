@@ -1,0 +1,498 @@
+// out[M, N] = A[M, K] . W[N, K]^T (+ bias[N]) for float32 operands on the 5th-generation tensor cores, at float32 accuracy.
+//
+// Every operand is cut in two, x = hi + lo: hi the eleven leading bits, rounded to nearest, and lo what is left, of which the tensor core
+// takes another eleven.  hi hi, hi lo and lo hi are multiplied on tcgen05.mma (kind::tf32, products exact in float32); what is left out
+// is of either sign and below 2^-23 of a product.  The tensor core's own sums are not rounded to nearest, so they are kept short: 32
+// entries of K, the small products first, into an accumulator that starts at zero; the sums of these chunks are added in registers, in
+// float32 to nearest.  Relative error (2-norm) against float64, beside that of a chain of multiply-adds (linear_simt.cu): 896 entries of
+// K 1.5e-7 (2.7e-7 to 3.8e-7), 3,584 1.6e-7 (7.6e-7), 4,864 1.6e-7 (4.4e-7); all entries positive 1.4e-7 (1.2e-7), 1.4e-7 (4.6e-7) and
+// 1.4e-7 (1.4e-7).  With 64 entries an accumulator the products took a twentieth less time, but positive ones were 2.8e-7 off.
+//
+// K is cut into ranges whose number depends on N and K only, a CTA each; the ranges of a tile are a cluster that adds its sums up in
+// their order (up to 64 rows of A each CTA sends the others their rows' sums, and none waits for another to read them: 0.7 to 1.1 us less
+// than reading them between two cluster barriers).  How many rows of A a tile has depends on M but changes no sum: a row's result does not depend on the rows beside it.
+//
+// A CTA: 128 rows of W (the accumulator's lanes) x up to 128 rows of A (its columns).
+//   warps 0-7  two groups that take the chunks in turn: a thread reads its row of W from the ring in shared memory, cuts it and stores
+//              both parts to tensor memory, where the products read them (an operand in shared memory would be read twelve times a chunk:
+//              with W there the tensor core waited for shared memory, 1,450 to 2,000 cycles a chunk of 112 rows of A); up to 64
+//              rows of A are cut here too and go to shared memory
+//   warp 8     issues a chunk's twelve products
+//   warp 9     brings W (float32) by TMA, before the kernel waits for its predecessor as far as the ring goes; more than 64 rows of A
+//              have been cut by a kernel before this one and come by TMA as well
+//   warps 10-  take the sums out of tensor memory
+// Bound by the tensor core and the hand-over of its sums: a chunk of 112 rows of A takes 1,150 cycles, its products alone 980.
+//
+// One B200, W read from memory, us, here / in linear_simt.cu (the only way before): rows of A 1 12 60 130 508
+//   1,152 x 896   4.8 / 5.5     5.1 / 7.7    7.1 / 12.2   10.0 / 21.7   20.9 / 34.8
+//     896 x 896   4.8 / 5.0     5.1 / 6.9    6.9 / 12.2    9.7 / 19.2   13.3 / 28.5
+//   9,728 x 896  12.2 / 12.8   13.4 / 27.2  16.4 / 51.0   40.0 / 84.3   68.1 / 208
+//     896 x 4864  9.2 / 11.4    9.9 / 20.4  12.0 / 29.9   19.0 / 64.5   42.9 / 111
+//   3,584 x 3584 20.2 / 28.7   22.4 / 50.3  27.9 / 77.3   56.2 / 176.8  108 / 316
+//
+// Infinities, values that are no number and sums beyond float32 leave results that are not finite; those are worked out again with plain
+// multiply-adds.
+//
+// Every wait is bounded by the clock; one that runs out sets *status to 9 and a flag that lets every other role leave its loop.
+//
+// pico-engine leaves these products to cuBLAS (src/pico_engine/model.py:177, 213, 223, 235, 164).
+#include "tcgen05_attention.cuh"
+
+#define SP_KC 32                                           // entries of K of a chunk: one row of the 128-byte swizzle
+#define SP_ROWS 128                                        // rows of W of a tile
+#define SP_BOX (SP_ROWS * SP_KC * 4)
+#define SP_CUTTERS 8
+#define SP_SLOTS 4                                         // chunks whose parts are in tensor memory and, of A, in shared memory
+#define SP_MANY 128                                        // NT of the form for many rows of A
+#define SP_TMEM 512
+
+// W in shared memory, chunks; sums in tensor memory, chunks; warps that take them
+template <int NT> constexpr int sp_ring() { return NT == SP_MANY ? 5 : NT == 64 ? 6 : 8; }
+template <int NT> constexpr int sp_sums() { return NT == SP_MANY ? 2 : 4; }
+template <int NT> constexpr int sp_takers() { return NT == SP_MANY ? 16 : 4; }
+template <int NT> constexpr int sp_threads() { return 32 * (SP_CUTTERS + 2 + sp_takers<NT>()); }
+// (few rows of A: a place of its own for the sums that the other CTAs of a cluster send, up to 8 x ceil(NT / 8) rows)
+template <int NT> constexpr int sp_sent_bytes() { return NT == SP_MANY ? 0 : (NT + 8) * SP_ROWS * 4; }
+template <int NT> constexpr int sp_smem_bytes() { return sp_ring<NT>() * SP_BOX + SP_SLOTS * 2 * NT * SP_KC * 4 + sp_sent_bytes<NT>() + 1024; }
+
+// A CTA an SM where few rows of A stream the weights, and ranges of seven chunks at least: what a CTA does once (its first loads, the sum
+// over the cluster) takes as long as about six chunks.
+static int sp_ranges(int N, int K) {
+    const int tiles = (N + SP_ROWS - 1) / SP_ROWS, chunks = (K + SP_KC - 1) / SP_KC;
+    int r = 148 / tiles;
+    if (r > chunks / 7) r = chunks / 7;
+    r = r > 8 ? 8 : r < 1 ? 1 : r;
+    const int each = (chunks + r - 1) / r;
+    return (chunks + each - 1) / each;                     // (no range without a chunk)
+}
+
+__device__ __forceinline__ void sp_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ float4 sp_peer_four(unsigned at, int rank) {
+    unsigned peer;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(at), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(peer) : "memory");
+    return v;
+}
+__device__ __forceinline__ float4 sp_shared_four(unsigned at) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
+    return v;
+}
+__device__ __forceinline__ void sp_put_four(unsigned at, const float* v) {
+    asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(at), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
+}
+__device__ __forceinline__ void sp_load8(float (&v)[8], const float* p) {
+    asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "l"(p) : "memory");
+}
+// (of an infinity or no number a lo is left that is no number)
+__device__ __forceinline__ float sp_hi(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u); }
+
+__device__ __forceinline__ unsigned sp_elect() {
+    unsigned r;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(r));
+    return r;
+}
+// The twelve products of a chunk, four steps of eight entries each: lo hi and hi lo, then hi hi, into an accumulator that starts at zero.
+// w: columns of tensor memory, 32 of hi and 32 of lo; a, a_lo: descriptors.  The whole warp calls; the elected thread issues.
+__device__ __forceinline__ void sp_products(unsigned elected, unsigned d, unsigned w, unsigned long long a, unsigned long long a_lo, unsigned idesc) {
+#define SP_MMA(wt, ad, p) " @e tcgen05.mma.cta_group::1.kind::tf32 [%1], [" wt "], " ad ", %10, " p ";\n"
+    asm volatile("{\n .reg .pred yes, no, e;\n .reg .b32 h1, h2, h3, l0, l1, l2, l3;\n"
+                 " setp.eq.u32 yes, 0, 0;\n setp.ne.u32 no, 0, 0;\n setp.ne.u32 e, %0, 0;\n"
+                 " add.u32 h1, %11, 8;\n add.u32 h2, %11, 16;\n add.u32 h3, %11, 24;\n add.u32 l0, %11, 32;\n add.u32 l1, %11, 40;\n add.u32 l2, %11, 48;\n add.u32 l3, %11, 56;\n"
+                 SP_MMA("l0", "%2", "no") SP_MMA("l1", "%3", "yes") SP_MMA("l2", "%4", "yes") SP_MMA("l3", "%5", "yes")
+                 SP_MMA("%11", "%6", "yes") SP_MMA("h1", "%7", "yes") SP_MMA("h2", "%8", "yes") SP_MMA("h3", "%9", "yes")
+                 SP_MMA("%11", "%2", "yes") SP_MMA("h1", "%3", "yes") SP_MMA("h2", "%4", "yes") SP_MMA("h3", "%5", "yes")
+                 "}"
+                 ::"r"(elected), "r"(d), "l"(a), "l"(a + 2), "l"(a + 4), "l"(a + 6), "l"(a_lo), "l"(a_lo + 2), "l"(a_lo + 4), "l"(a_lo + 6), "r"(idesc), "r"(w) : "memory");
+#undef SP_MMA
+}
+__device__ __forceinline__ unsigned long long sp_pair(unsigned a, unsigned b) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ void sp_st16(unsigned taddr, const float (&v)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+                 ::"r"(taddr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]), "f"(v[9]), "f"(v[10]), "f"(v[11]), "f"(v[12]),
+                   "f"(v[13]), "f"(v[14]), "f"(v[15]) : "memory");
+}
+// acc (pairs of columns) += the first `columns` columns (a multiple of eight) of this thread's lane
+template <int COLS>
+__device__ __forceinline__ void sp_add_columns(unsigned long long (&acc)[COLS / 2], unsigned taddr, int columns) {
+    constexpr int STEP = COLS < 32 ? COLS : 32;
+#pragma unroll
+    for (int c0 = 0; c0 < COLS; c0 += STEP) {
+        unsigned r[STEP];
+#pragma unroll
+        for (int c = 0; c < STEP; c += 8)
+            if (c0 + c < columns)
+                asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(r[c]), "=r"(r[c + 1]), "=r"(r[c + 2]), "=r"(r[c + 3]), "=r"(r[c + 4]), "=r"(r[c + 5]), "=r"(r[c + 6]), "=r"(r[c + 7]) : "r"(taddr + c0 + c) : "memory");
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int c = 0; c < STEP; c += 8)                  // (not before the wait)
+            asm volatile("" : "+r"(r[c]), "+r"(r[c + 1]), "+r"(r[c + 2]), "+r"(r[c + 3]), "+r"(r[c + 4]), "+r"(r[c + 5]), "+r"(r[c + 6]), "+r"(r[c + 7]) :: "memory");
+#pragma unroll
+        for (int c = 0; c < STEP; c += 2) asm("add.rn.f32x2 %0, %0, %1;" : "+l"(acc[(c0 + c) / 2]) : "l"(sp_pair(r[c], r[c + 1])));
+    }
+}
+// epilogue: 0 store float32, 1 store bfloat16, 2 add into float32 (the residual stream)
+__device__ __forceinline__ void sp_finish(float v, void* out, size_t at, const void* bias, int bias_dtype, int n, int epilogue) {
+    if (bias) v += load_as_f(bias, bias_dtype, n);
+    if (epilogue == 0) ((float*)out)[at] = v;
+    else if (epilogue == 1) ((bf16*)out)[at] = __float2bfloat16_rn(v);
+    else ((float*)out)[at] += v;
+}
+// true when the phase with this parity has completed; false when the wait ran out or another role gave up
+__device__ __forceinline__ bool sp_wait(unsigned bar, unsigned parity, volatile int* abort_flag, int* status) {
+    unsigned done;
+    asm volatile("{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    if (done) return true;
+    const long long deadline = clock64() + AT_WAIT_CYCLES;
+    for (;;) {
+        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+        if (done) return true;
+        if (*abort_flag) return false;
+        if (clock64() > deadline) {
+            *abort_flag = 1;
+            if (status) atomicExch(status, 9);
+            return false;
+        }
+    }
+}
+__device__ __forceinline__ bool sp_wait_warp(unsigned bar, unsigned parity, volatile int* abort_flag, int* status) {
+    return __all_sync(0xffffffffu, sp_wait(bar, parity, abort_flag, status));
+}
+
+// Rows of A as their parts, [2][M][K], for tiles of many rows.
+__global__ void __launch_bounds__(256) split_rows_kernel(const float* A, float* parts, long long entries, int vec_a) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const long long at = ((long long)blockIdx.x * 256 + threadIdx.x) * 4;
+    if (at >= entries) return;
+    const float4 v = vec_a ? *reinterpret_cast<const float4*>(A + at) : make_float4(A[at], A[at + 1], A[at + 2], A[at + 3]);
+    const float4 hi = make_float4(sp_hi(v.x), sp_hi(v.y), sp_hi(v.z), sp_hi(v.w));
+    *reinterpret_cast<float4*>(parts + at) = hi;
+    *reinterpret_cast<float4*>(parts + entries + at) = make_float4(v.x - hi.x, v.y - hi.y, v.z - hi.z, v.w - hi.w);
+}
+
+// NT rows of A a tile: 16, 32 or 64; or (SP_MANY) up to 128, `nt` of them, whose parts come by TMA.
+template <int NT>
+__global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const float* A,
+                                                                           const float* W, const void* bias, int bias_dtype, void* out, int epilogue, int M, int N, int K,
+                                                                           int ranges, int nt, int vec_a, int* status) {
+    constexpr bool MANY = NT == SP_MANY;
+    constexpr int RING = sp_ring<NT>(), SUMS = sp_sums<NT>(), TAKER = SP_CUTTERS + 2, COLS = NT * 4 / sp_takers<NT>();
+    constexpr int TPT = NT >= 32 ? NT / 32 : 1, GROUPS = SP_CUTTERS / 4;      // TPT: runs of eight entries of A a thread cuts
+    if (!MANY) nt = NT;
+    const int part_bytes = nt * SP_KC * 4;
+    extern __shared__ unsigned char sp_raw[];
+    __shared__ __align__(8) unsigned long long bars[2 * RING + 2 * SP_SLOTS + 2 * SUMS + 1];
+    __shared__ unsigned tmem_base_s;
+    __shared__ int abort_s;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned smem = (at_smem(sp_raw) + 1023u) & ~1023u, a_parts = smem + RING * SP_BOX;
+    const int rank = blockIdx.x % ranges, n0 = blockIdx.x / ranges * SP_ROWS, m0 = blockIdx.y * nt;
+    const int all = (K + SP_KC - 1) / SP_KC, each = (all + ranges - 1) / ranges;
+    const int k_begin = rank * each * SP_KC, k_end = min(K, k_begin + each * SP_KC), chunks = (k_end - k_begin + SP_KC - 1) / SP_KC;
+    const unsigned w_full = at_smem(bars), w_empty = w_full + 8 * RING, full = w_empty + 8 * RING, empty = full + 8 * SP_SLOTS, sum_full = empty + 8 * SP_SLOTS,
+                   sum_empty = sum_full + 8 * SUMS, sent = sum_empty + 8 * SUMS;
+    // the rows of A whose sums over the cluster this CTA finishes
+    const int slice = (nt + ranges - 1) / ranges, first_row = rank * slice, rows = max(0, min(min(nt, first_row + slice), M - m0) - first_row);
+
+    if (warp == SP_CUTTERS) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(at_smem(&tmem_base_s)), "r"((unsigned)SP_TMEM) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 32 * (SP_CUTTERS + 1)) {
+        const auto init = [](unsigned bar, int count, unsigned arrivals) {
+            for (int i = 0; i < count; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar + 8 * i), "r"(arrivals) : "memory");
+        };
+        init(w_full, RING, 1); init(w_empty, RING, 4); init(full, SP_SLOTS, MANY ? 5 : 4); init(empty, SP_SLOTS, 1); init(sum_full, SUMS, 1); init(sum_empty, SUMS, sp_takers<NT>());
+        if (!MANY) {
+            init(sent, 1, 1);
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sent), "r"((unsigned)((ranges - 1) * rows * SP_ROWS * 4)) : "memory");
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;\n\tfence.proxy.async.shared::cta;" ::: "memory");
+        abort_s = 0;
+    }
+    const auto bring_w = [&](int c) {                      // rows and entries behind the last are zeros
+        const int s = c % RING;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(w_full + 8 * s), "r"((unsigned)SP_BOX) : "memory");
+        at_tma_2d(smem + s * SP_BOX, &map_w, k_begin + c * SP_KC, n0, w_full + 8 * s);
+    };
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (!MANY && ranges > 1) asm volatile("barrier.cluster.arrive.release;" ::: "memory");      // this CTA can be sent to
+    const unsigned tmem = tmem_base_s, sums = tmem + SP_SLOTS * 2 * SP_KC;
+    pdl_launch_dependents();                               // (behind the allocation of tensor memory: a later kernel must not take it first)
+    if (tid == 32 * (SP_CUTTERS + 1))
+        for (int c = 0; c < min(RING, chunks); ++c) bring_w(c);      // weights: no kernel writes them
+    pdl_wait();
+
+    unsigned long long acc[COLS / 2];                      // pairs of columns
+    const int column0 = MANY ? ((warp - TAKER) >> 2) * COLS : 0, columns = MANY ? max(0, min(COLS, nt - column0)) : NT;
+    if (warp < SP_CUTTERS) {
+        const int row = tid & 127, lr = row >> 2, lk = (tid & 3) * 8;
+        const unsigned lanes = (unsigned)((warp & 3) * 32) << 16;
+        // entry k of a row: 16-byte groups exchanged by the row's place in its run of eight
+        const unsigned first = lr * 128 + ((((unsigned)lk >> 2) ^ (lr & 7)) << 4), second = first ^ 16u;
+        float ra[TPT][8];
+        auto fetch_a = [&](int c) {                        // rows behind the last are read as the last and not stored (K is a multiple of eight)
+            const int k = k_begin + c * SP_KC + lk;
+#pragma unroll
+            for (int e = 0; e < TPT; ++e) {
+                const float* p = A + (size_t)min(m0 + lr + 32 * e, M - 1) * K + k;
+                if (k < k_end && vec_a) sp_load8(ra[e], p);
+                else {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) ra[e][i] = k < k_end ? p[i] : 0.f;
+                }
+            }
+        };
+        if (!MANY && (warp >> 2) < chunks) fetch_a(warp >> 2);
+        for (int c = warp >> 2; c < chunks; c += GROUPS) {
+            const int r = c % RING, s = c % SP_SLOTS;
+            if (!sp_wait_warp(w_full + 8 * r, (c / RING) & 1, &abort_s, status)) break;
+            if (c >= SP_SLOTS && !sp_wait_warp(empty + 8 * s, (c / SP_SLOTS - 1) & 1, &abort_s, status)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                float hi[SP_KC / 2], lo[SP_KC / 2];
+#pragma unroll
+                for (int j = 0; j < SP_KC / 8; ++j) {
+                    const float4 v = sp_shared_four(smem + r * SP_BOX + row * 128 + (((4 * half + j) ^ (row & 7)) << 4));
+                    hi[4 * j] = sp_hi(v.x); hi[4 * j + 1] = sp_hi(v.y); hi[4 * j + 2] = sp_hi(v.z); hi[4 * j + 3] = sp_hi(v.w);
+                    lo[4 * j] = v.x - hi[4 * j]; lo[4 * j + 1] = v.y - hi[4 * j + 1]; lo[4 * j + 2] = v.z - hi[4 * j + 2]; lo[4 * j + 3] = v.w - hi[4 * j + 3];
+                }
+                sp_st16(tmem + lanes + s * 2 * SP_KC + 16 * half, hi);
+                sp_st16(tmem + lanes + s * 2 * SP_KC + SP_KC + 16 * half, lo);
+            }
+            __syncwarp();
+            if (lane == 0) at_arrive(w_empty + 8 * r);
+            if (!MANY) {
+#pragma unroll
+                for (int e = 0; e < TPT; ++e)
+                    if (NT >= 32 || lr < NT) {
+                        const unsigned at = a_parts + s * 2 * part_bytes + e * 32 * 128;
+                        float h[8], l[8];
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) { h[i] = sp_hi(ra[e][i]); l[i] = ra[e][i] - h[i]; }
+                        sp_put_four(at + first, h); sp_put_four(at + second, h + 4);
+                        sp_put_four(at + part_bytes + first, l); sp_put_four(at + part_bytes + second, l + 4);
+                    }
+                if (c + GROUPS < chunks) fetch_a(c + GROUPS);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) at_arrive(full + 8 * s);
+        }
+    } else if (warp == SP_CUTTERS) {
+        const unsigned idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((unsigned)(nt / 8) << 17) | ((unsigned)(SP_ROWS / 16) << 24);
+        const unsigned elected = sp_elect();
+        for (int c = 0; c < chunks; ++c) {
+            const int s = c % SP_SLOTS, b = c % SUMS;
+            if (c >= SUMS && !sp_wait_warp(sum_empty + 8 * b, (c / SUMS - 1) & 1, &abort_s, status)) break;
+            if (!sp_wait_warp(full + 8 * s, (c / SP_SLOTS) & 1, &abort_s, status)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const unsigned long long a = at_desc(a_parts + s * 2 * part_bytes, 16, 1024);
+            sp_products(elected, sums + b * NT, tmem + s * 2 * SP_KC, a, a + (part_bytes >> 4), idesc);
+            if (elected) {
+                at_commit(empty + 8 * s);
+                at_commit(sum_full + 8 * b);
+            }
+            __syncwarp();
+        }
+    } else if (warp == SP_CUTTERS + 1) {
+        if (lane == 0) {
+            for (int c = 0; c < chunks; ++c) {
+                const int s = c % SP_SLOTS, r = c % RING;
+                if (MANY) {
+                    if (c >= SP_SLOTS && !sp_wait(empty + 8 * s, (c / SP_SLOTS - 1) & 1, &abort_s, status)) break;
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full + 8 * s), "r"((unsigned)(2 * part_bytes)) : "memory");
+                    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+                                 ::"r"(a_parts + s * 2 * part_bytes), "l"(&map_a), "r"(full + 8 * s), "r"(k_begin + c * SP_KC), "r"(m0), "r"(0) : "memory");
+                }
+                if (c + RING < chunks) {
+                    if (!sp_wait(w_empty + 8 * r, (c / RING) & 1, &abort_s, status)) break;
+                    bring_w(c + RING);
+                }
+            }
+        }
+        __syncwarp();
+    } else {
+        const unsigned mine = sums + ((unsigned)((warp & 3) * 32) << 16) + column0;
+#pragma unroll
+        for (int i = 0; i < COLS / 2; ++i) acc[i] = 0ull;
+        for (int c = 0; c < chunks; ++c) {
+            const int b = c % SUMS;
+            if (!sp_wait_warp(sum_full + 8 * b, (c / SUMS) & 1, &abort_s, status)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            sp_add_columns<COLS>(acc, mine + b * NT, columns);
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) at_arrive(sum_empty + 8 * b);
+        }
+    }
+    __syncthreads();                                       // all products have ended, all copies have landed
+    if (warp >= TAKER) {                                   // [nt][128] sums where the operands were
+        const int row = (warp & 3) * 32 + lane, n = n0 + row;
+        float zero = 0.f;                                  // no number if one of the sums is not finite
+#pragma unroll
+        for (int i = 0; i < COLS; ++i)
+            if (i < columns) {
+                const float v = __uint_as_float((unsigned)(acc[i / 2] >> (32 * (i & 1))));
+                zero = fmaf(v, 0.f, zero);
+                asm volatile("st.shared.f32 [%0], %1;" ::"r"(smem + ((column0 + i) * SP_ROWS + row) * 4), "f"(v) : "memory");
+            }
+#pragma unroll 1
+        for (int i = 0; i < (zero != 0.f && n < N ? min(columns, M - m0 - column0) : 0); ++i) {
+            const unsigned at = smem + ((column0 + i) * SP_ROWS + row) * 4;
+            float v;
+            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
+            if (isfinite(v)) continue;
+            v = 0.f;
+            for (int k = k_begin; k < k_end; ++k) v = fmaf(A[(size_t)(m0 + column0 + i) * K + k], W[(size_t)n * K + k], v);
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(at), "f"(v) : "memory");
+        }
+    }
+    const unsigned sums_sent = a_parts + SP_SLOTS * 2 * part_bytes;       // [rank][slice][128]
+    if (MANY) {
+        if (ranges > 1) sp_cluster_sync(); else __syncthreads();
+    } else {
+        __syncthreads();
+        if (ranges > 1) {
+            asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+            for (int i = tid; i < min(nt, M - m0) * (SP_ROWS / 4); i += sp_threads<NT>()) {
+                const int t = i / (SP_ROWS / 4), col = i % (SP_ROWS / 4) * 4, to = t / slice;
+                if (to == rank) continue;
+                const float4 v = sp_shared_four(smem + (t * SP_ROWS + col) * 4);
+                asm volatile("{\n .reg .b32 at, bar;\n mapa.shared::cluster.u32 at, %0, %2;\n mapa.shared::cluster.u32 bar, %1, %2;\n"
+                             " st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [at], {%3, %4, %5, %6}, [bar];\n}"
+                             ::"r"(sums_sent + ((rank * slice + t - to * slice) * SP_ROWS + col) * 4), "r"(sent), "r"(to), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+            }
+            if (rows > 0) sp_wait(sent, 0, &abort_s, status);
+        }
+    }
+#pragma unroll 1
+    for (int i = tid; i < rows * (SP_ROWS / 4); i += sp_threads<NT>()) {
+        const int t = i / (SP_ROWS / 4), col = i % (SP_ROWS / 4) * 4, n = n0 + col;
+        if (n >= N) continue;
+        const unsigned at = smem + ((first_row + t) * SP_ROWS + col) * 4;
+        float4 part[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            if (c >= ranges) part[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+            else if (MANY) part[c] = sp_peer_four(at, c);
+            else part[c] = sp_shared_four(c == rank ? at : sums_sent + ((c * slice + t) * SP_ROWS + col) * 4);
+        }
+        float4 v = part[0];
+#pragma unroll
+        for (int c = 1; c < 8; ++c)
+            if (c < ranges) { v.x += part[c].x; v.y += part[c].y; v.z += part[c].z; v.w += part[c].w; }
+        const float four[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (n + e < N) sp_finish(four[e], out, (size_t)(m0 + first_row + t) * N + n + e, bias, bias_dtype, n + e, epilogue);
+    }
+    if (MANY && ranges > 1) sp_cluster_sync();             // nobody leaves while its sums are being read
+    if (warp == SP_CUTTERS) {
+        __syncwarp();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((unsigned)SP_TMEM) : "memory");
+    }
+}
+
+// Boxes of 32 entries x `rows` rows x `planes` of a float32 [planes][R][K] array; what lies outside reads as zero.
+static int sp_map(CUtensorMap* map, const void* base, int K, int R, int planes, int rows) {
+    at_encode_fn enc = at_encoder();
+    if (!enc) return PE_ERR_UNSUPPORTED;
+    const cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)R, (cuuint64_t)planes}, strides[2] = {(cuuint64_t)K * 4, (cuuint64_t)K * R * 4};
+    const cuuint32_t box[3] = {SP_KC, (cuuint32_t)rows, (cuuint32_t)planes}, elem[3] = {1, 1, 1};
+    const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, planes > 1 ? 3 : 2, const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? 0 : 20000 + (int)r;
+}
+
+template <int NT>
+static int sp_go(const CUtensorMap& map_w, const CUtensorMap& map_a, int nt, const float* A, const float* W, const void* bias, int bias_dtype, void* out, int epilogue,
+                 int M, int N, int K, int* status, cudaStream_t s) {
+    auto kernel = linear_split_kernel<NT>;
+    const int mt = (M + nt - 1) / nt, ranges = sp_ranges(N, K);
+    if (mt > 65535) return PE_ERR_UNSUPPORTED;
+    PE_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sp_smem_bytes<NT>()));
+    PE_TRY(pe_launch_cluster(kernel, dim3((N + SP_ROWS - 1) / SP_ROWS * ranges, mt), sp_threads<NT>(), sp_smem_bytes<NT>(), s, ranges, map_w, map_a, A, W, bias, bias_dtype,
+                             out, epilogue, M, N, K, ranges, nt, (int)((uintptr_t)A % 32 == 0), status));
+    PE_LAUNCH_CHECK();
+    return 0;
+}
+
+// How many clusters of `ranges` CTAs of the form for many rows run at once on this device.
+static int sp_resident_clusters(int ranges, int& n) {
+    static int known[64][9];                               // (the same number whoever writes it)
+    int device = 0;
+    PE_TRY(cudaGetDevice(&device));
+    if (device < 64 && known[device][ranges] > 0) { n = known[device][ranges]; return 0; }
+    auto kernel = linear_split_kernel<SP_MANY>;
+    PE_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sp_smem_bytes<SP_MANY>()));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ranges); cfg.blockDim = dim3(sp_threads<SP_MANY>()); cfg.dynamicSmemBytes = sp_smem_bytes<SP_MANY>();
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ranges; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    PE_TRY(cudaOccupancyMaxActiveClusters(&n, kernel, &cfg));
+    if (n < 1) return PE_ERR_UNSUPPORTED;
+    if (device < 64) known[device][ranges] = n;
+    return 0;
+}
+
+// Whether a product of float32 operands comes here: by N, K and the place of W alone, so that a row's result is the same in every step.
+// Smaller products of one to 16 rows are what their launch takes (512 x 512 here / as multiply-adds 5.3 / 3.3 us at one row, 6.0 / 8.5 at 17).
+extern "C" int pe_linear_split_takes(const void* W, int N, int K) { return N >= 256 && K >= 256 && (long long)N * K >= 800000 && K % 8 == 0 && (uintptr_t)W % 16 == 0; }
+
+// Rows of A that are cut at a time, so that their parts take 256 MB at most; and the bytes of scratch a product of M rows needs.
+static int sp_slab(int K) { return (int)((256ll << 20) / (8ll * K) > SP_MANY ? (256ll << 20) / (8ll * K) / SP_MANY * SP_MANY : SP_MANY); }
+extern "C" long long pe_linear_split_scratch(int M, int K) { return M <= 64 ? 0 : 8ll * K * (M < sp_slab(K) ? M : sp_slab(K)); }
+
+extern "C" int pe_linear_split(const void* A, const void* W, const void* bias, int bias_dtype, void* out, int epilogue, int M, int N, int K, void* scratch, void* status, void* stream) {
+    if (M <= 0) return 0;
+    if (!pe_linear_split_takes(W, N, K) || epilogue < 0 || epilogue > 2) return PE_ERR_UNSUPPORTED;
+    CUtensorMap map_w = {}, map_a = {};
+    const cudaStream_t s = (cudaStream_t)stream;
+    if (const int e = sp_map(&map_w, W, K, N, 1, SP_ROWS)) return e;
+#define SP_GO(NT, nt, A, out, M) sp_go<NT>(map_w, map_a, nt, (const float*)(A), (const float*)W, bias, bias_dtype, out, epilogue, M, N, K, (int*)status, s)
+    if (M <= 16) return SP_GO(16, 16, A, out, M);
+    if (M <= 32) return SP_GO(32, 32, A, out, M);
+    if (M <= 64) return SP_GO(64, 64, A, out, M);
+    int clusters = 0;
+    if (const int e = sp_resident_clusters(sp_ranges(N, K), clusters)) return e;
+    const long long tiles = (N + SP_ROWS - 1) / SP_ROWS;
+    for (int first = 0; first < M; first += sp_slab(K)) {
+        const int rows = M - first < sp_slab(K) ? M - first : sp_slab(K);
+        // Rows of A a tile: the fewest turns of clusters, each as long as its rows and as what it does whatever their number (508 rows, 9,728 x
+        // 896, three turns of 112 rows 66 us; 896 x 896, one of 128 13 us, two of 112 22).
+        int nt = SP_MANY;
+        long long least = -1;
+        for (int t = SP_MANY; t >= 64; t -= 16) {
+            const long long cost = ((rows + t - 1) / t * tiles + clusters - 1) / clusters * (t + 96);
+            if (least < 0 || cost < least) { least = cost; nt = t; }
+        }
+        const float* a = (const float*)A + (size_t)first * K;
+        void* o = (char*)out + (size_t)first * N * (epilogue == 1 ? 2 : 4);
+        const long long entries = (long long)rows * K;
+        PE_TRY(pe_launch(split_rows_kernel, dim3((unsigned)((entries / 4 + 255) / 256)), 256, 0, s, a, (float*)scratch, entries, (int)((uintptr_t)a % 16 == 0)));
+        PE_LAUNCH_CHECK();
+        if (const int e = sp_map(&map_a, scratch, K, rows, 2, nt)) return e;
+        if (const int e = SP_GO(SP_MANY, nt, a, o, rows)) return e;
+    }
+#undef SP_GO
+    return 0;
+}

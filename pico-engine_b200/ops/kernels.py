@@ -151,7 +151,7 @@ _EPILOGUE_STORE = {torch.float32: 0, torch.bfloat16: 1}
 def linear_simt(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
                 out_dtype: Optional[torch.dtype] = None, accumulate_into: Optional[torch.Tensor] = None,
                 out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """a [M, K] . w [N, K]^T (+ bias) with float32 multiply-adds.  Either stored as
+    """a [M, K] . w [N, K]^T (+ bias) in float32, whatever the operands are stored as.  Either stored as
     ``out_dtype`` or added into the float32 tensor ``accumulate_into`` [M, N]."""
     M, K = a.shape
     N = w.shape[0]
@@ -166,6 +166,13 @@ def linear_simt(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] =
             out = torch.empty(M, N, dtype=out_dtype or a.dtype, device=a.device)
         _need(out, "out", None, (M, N))
         epilogue = _EPILOGUE_STORE[out.dtype]
+    if a.dtype == w.dtype == torch.float32 and core().pe_linear_split_takes(w.data_ptr(), N, K):
+        # on the tensor cores, each operand in two parts: as exact as multiply-adds (csrc/linear_split.cu has the figures)
+        nbytes = core().pe_linear_split_scratch(M, K)
+        parts = torch.empty(nbytes, dtype=torch.uint8, device=a.device) if nbytes else None
+        check(core().pe_linear_split(a.data_ptr(), w.data_ptr(), _ptr(bias), 0 if bias is None else _code(bias, "bias"), out.data_ptr(), epilogue,
+                                     M, N, K, _ptr(parts), _status_ptr_or_none(a.device), stream_ptr()), "linear_split")
+        return out
     check(core().pe_linear_simt(a.data_ptr(), _code(a, "a"), w.data_ptr(), _code(w, "w"), _ptr(bias),
                                 0 if bias is None else _code(bias, "bias"), out.data_ptr(), epilogue, M, N, K,
                                 stream_ptr()), "linear_simt")
@@ -449,6 +456,11 @@ def status_ptr(device) -> int:
     if ptr is None:
         ptr = status_word(device).data_ptr()
     return ptr
+
+
+def _status_ptr_or_none(device) -> Optional[int]:
+    """The same for a kernel that does without: no word is made while a graph is being captured."""
+    return None if device not in _status_ptrs and torch.cuda.is_current_stream_capturing() else status_ptr(device)
 
 
 def check_status(device) -> None:

@@ -11,7 +11,7 @@ from ..csrc import build
 
 P, I, F, LL, ULL = c_void_p, c_int, c_float, c_longlong, c_ulonglong
 
-CORE_SOURCES = ("elementwise.cu", "linear_simt.cu", "attention_generic.cu", "sampling.cu", "linear_fused.cu", "gemm_tcgen05.cu")
+CORE_SOURCES = ("elementwise.cu", "linear_simt.cu", "attention_generic.cu", "sampling.cu", "linear_fused.cu", "gemm_tcgen05.cu", "linear_split.cu")
 # Kernels that no model needs unless it is asked for them: the allocation-free entry point and the split-K product it
 # is built on (linear_mma.cu), and the two kernels for decode steps of 17 to 64 rows that the library's products with
 # this library's small kernels between them still beat (linear_batch.cu: mma.sync with fused prologue and epilogues;
@@ -44,6 +44,8 @@ _SIGNATURES = {
     "pe_bias_add": [P, I, P, I, I, I, P],
     "pe_rope_store": [P, I, I, I, I, I, P, P, P, P, P, P, P, I, I, P],
     "pe_linear_simt": [P, I, P, I, P, I, P, I, I, I, I, P],
+    "pe_linear_split_takes": [P, I, I],
+    "pe_linear_split": [P, P, P, I, P, I, I, I, I, P, P, P],
     "pe_attention_generic": [P, I, P, P, P, I, P, I, P, P, I, I, I, I, I, F, I, P, I, P],
     "pe_argmax": [P, P, I, I, P, P],
     "pe_sample": [P, P, I, I, F, I, F, ULL, P, P, P, P, P],
@@ -160,6 +162,8 @@ def core() -> ctypes.CDLL:
         lib.pe_set_pdl(0 if os.environ.get("PICO_ENGINE_PDL", "1") == "0" else 1)
         lib.pe_draw_uniform.argtypes = [ULL, ULL, ULL]
         lib.pe_draw_uniform.restype = c_float
+        lib.pe_linear_split_scratch.argtypes = [I, I]
+        lib.pe_linear_split_scratch.restype = c_longlong
         lib.pe_argmax_scratch_bytes.argtypes = [I, I]
         lib.pe_argmax_scratch_bytes.restype = c_longlong
         lib.pe_sample_scratch_bytes.argtypes = [I, I]

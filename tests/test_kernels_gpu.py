@@ -608,6 +608,48 @@ def test_linear_simt_rows_do_not_depend_on_their_neighbours(K):
         assert torch.equal(K.linear_simt(dev(a[r:r + 1]), dev(w), out_dtype=torch.float32)[0], whole[r])
 
 
+SPLIT_SIZES = [(3200, 256), (1100, 744), (896, 896), (257, 3128), (9728, 320), (896, 4864), (19000, 264)]
+
+
+@pytest.mark.parametrize("N,K_", SPLIT_SIZES)
+def test_linear_float32_in_parts(K, N, K_):
+    """Float32 products on the tensor cores: rows beside the tiles, one to eight ranges of K, every epilogue, against float64; a row's
+    sums are the same alone and among others, and where its operand starts beside a 32-byte border."""
+    a, w, bias = rnd(301, K_, seed=1), rnd(N, K_, seed=2), rnd(N, seed=3)
+    want = a.double() @ w.double().T
+    A, W, B = dev(a), dev(w), dev(bias)
+    whole = K.linear_simt(A, W, B)
+    # K products of about unit size in float32: sqrt(K) * 2^-24 * sqrt(K) a few times over, as for the plain multiply-adds
+    assert float((whole.cpu().double() - want - bias.double()).abs().max()) <= 8 * (K_ + 1) * 2.0 ** -24
+    for M in (1, 16, 17, 33, 64, 65, 127, 129, 300):
+        assert torch.equal(K.linear_simt(A[:M], W, B), whole[:M]), M
+    for M in (5, 70):
+        odd = torch.empty(M * K_ + 1, device="cuda")[1:].view(M, K_).copy_(A[:M])
+        assert torch.equal(K.linear_simt(odd, W, B), whole[:M]), M
+        x = dev(torch.ones(M, N))
+        K.linear_simt(A[:M], W, accumulate_into=x)
+        assert float((x.cpu().double() - want[:M] - 1).abs().max()) <= 8 * (K_ + 1) * 2.0 ** -24
+        assert torch.equal(K.linear_simt(A[:M], W, B, out_dtype=torch.bfloat16), whole[:M].to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("M", [7, 60, 200])
+@pytest.mark.parametrize("N,K_", [(4100, 264), (896, 896)])
+def test_linear_float32_in_parts_of_values_that_are_not_finite(K, M, N, K_):
+    """Infinities, values that are no number and sums beyond float32, in either operand: as multiply-adds have them, and no other result moves."""
+    a, w = rnd(M, K_, seed=1), rnd(N, K_, seed=2)
+    clean = K.linear_simt(dev(a), dev(w)).cpu()
+    a[0, 5], a[3, K_ - 1], a[4, 0], a[5, 1] = float("inf"), float("nan"), 3.4e38, float("-inf")
+    w[7, 5], w[N - 1, 2], w[9, 0] = 0.0, float("-inf"), 4.0
+    got = K.linear_simt(dev(a), dev(w)).cpu()
+    want = (a.double() @ w.double().T).float()
+    got[4, N - 1] = want[4, N - 1]                         # (an infinity in float64; in float32 also that of 3.4e38 times a weight, so either)
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf()) and torch.equal(got[want.isinf()], want[want.isinf()])
+    same = torch.ones(M, N, dtype=torch.bool)
+    same[[0, 3, 4, 5]] = False
+    same[:, [7, N - 1, 9]] = False
+    assert torch.equal(got[same], clean[same])
+
+
 @pytest.mark.parametrize("M", [1, 8, 13, 64])
 @pytest.mark.parametrize("N,K_", [(100, 96), (896, 896), (1152, 896), (896, 4864), (9728, 896), (70, 160), (4000, 3584)])
 def test_linear_mma(K, M, N, K_):
