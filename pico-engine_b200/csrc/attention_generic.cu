@@ -84,11 +84,15 @@ __global__ void __launch_bounds__(AG_THREADS) attention_generic_kernel(
 // R / 16 rows and hd / 16 columns of the outputs.  Tokens of several sequences in a block are served one after the other, each run of
 // neighbouring tokens of one sequence by itself (tokens of two sequences may come in any order).
 // Whatever R is, a row's scores are sums over the entries in order, its weights are added in the same tree, its outputs in the order of
-// the keys: R = 16 (single tokens) and R = 64 (prompts) give the same bits.  A key that a row does not see adds nothing to it, not even
-// a value that is no number.  Bound by float32 multiply-adds and the reads from shared memory that feed them.  Two layers' attention of
-// 14 heads of 64, prompts of 301 and 207 tokens, on a B200: 645 us by the kernel above (a block a token and head, which read every key
-// and value once a head), 75 us here.
+// the keys of a segment (AG_SEGMENT pages, counted from the sequence's start), and the segments are joined in their order: R = 16 (single
+// tokens) and R = 64 (prompts) give the same bits, and so do blocks of one sequence whose segments are dealt out to a cluster
+// of CTAs, which join them in shared memory (few rows over a long context, which one CTA walks at 2 to 4 us a page).  A key that a row does not see adds nothing to it, not even
+// a value that is no number.  Bound by float32 multiply-adds and the reads from shared memory that feed them.  14 heads of 64 on 2, prompts
+// of 301 and 207 tokens, on a B200: 322 us by the kernel above (a block a token and head, which read every key and value once a head), 35 us
+// here (34 without segments).  One token behind 700 / 4,000 others 47 / 258 us in one CTA, 12 / 39 as segments over a cluster; twelve
+// tokens behind 50 to 1,500 99 and 27; segments of 4 pages 19 / 35 and 30.
 #define AT_THREADS 256
+#define AG_SEGMENT 2                                      // pages whose sums have a maximum of their own
 #define AG_RUN 128                                        // tokens of a run at most
 
 struct AttentionTileArgs {
@@ -96,6 +100,7 @@ struct AttentionTileArgs {
     const int* table; int table_stride; const int* tok_pos; const int* tok_row;
     int T, nh, nkv, hd, window; float scale;
     int heads, slices, tokens;                     // query heads and tokens of a block's rows; blocks that share a key/value head's heads
+    int cluster, buffers;                          // CTAs that share a block's segments; places for a segment's sums
     const int4* runs; int parts;                   // null: blocks of neighbouring packed tokens; else runs (row, first packed token, tokens, ..), `parts` blocks each
 };
 
@@ -120,11 +125,39 @@ __device__ __forceinline__ void ag_fma4(float4& acc, float a, const float4& b) {
 }
 // entry d of key (or row) j in a turned tile [hd][64]: neither a thread's four stores nor the reads of four neighbours meet in a bank
 __device__ __forceinline__ int ag_turned(int d, int j) { return d * 64 + (j ^ (((d >> 2) & 7) << 2)); }
+// (m, l) of what came before joined with the (ms, ls) of a segment; before and now: what the outputs of either are multiplied by.  Nothing
+// seen (a maximum of -infinity) changes no bit of the other.
+__device__ __forceinline__ void ag_join(float& m, float& l, float ms, float ls, float& before, float& now) {
+    const float m_new = fmaxf(m, ms), less = expf(fminf(m, ms) - m_new);       // (one of the two is the new maximum)
+    before = m == m_new ? 1.f : m == -INFINITY ? 0.f : less;
+    now = ms == m_new ? 1.f : ms == -INFINITY ? 0.f : less;
+    l = fmaf(l, before, ls * now);
+    m = m_new;
+}
+__device__ __forceinline__ void ag_join4(float4& acc, float before, const float4& v, float now) {
+    acc.x = fmaf(acc.x, before, v.x * now); acc.y = fmaf(acc.y, before, v.y * now); acc.z = fmaf(acc.z, before, v.z * now); acc.w = fmaf(acc.w, before, v.w * now);
+}
+__device__ __forceinline__ void ag_cluster_sync() { asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ unsigned ag_peer(const float* mine, int rank) {
+    unsigned at = (unsigned)__cvta_generic_to_shared(mine), peer;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(at), "r"(rank));
+    return peer;
+}
+__device__ __forceinline__ float ag_peer1(const float* mine, int rank) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(ag_peer(mine, rank)) : "memory");
+    return v;
+}
+__device__ __forceinline__ float4 ag_peer4(const float* mine, int rank) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(ag_peer(mine, rank)) : "memory");
+    return v;
+}
 struct ag_yes { static constexpr bool value = true; };
 struct ag_no { static constexpr bool value = false; };
 
 template <typename T, int R, int NJ>
-__global__ void __launch_bounds__(AT_THREADS) attention_tile_kernel(AttentionTileArgs a) {
+__global__ void __launch_bounds__(AT_THREADS, R == 16 && NJ == 1 ? 2 : 1) attention_tile_kernel(AttentionTileArgs a) {
     pdl_launch_dependents();
     pdl_wait();
     constexpr int RT = R / 16;                             // rows a thread
@@ -135,11 +168,13 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tile_kernel(AttentionTil
     float* kt = qt + hd * 64;                              // [hd][64]: a page's keys, turned
     float* vs = kt + hd * 64;                              // [64][hd]
     float* ps = vs + hd * 64;                              // [64 keys][R]: weights, rows in groups of four exchanged by the key
+    float* joint = ps + 64 * R;                            // a cluster: one or two buffers of a segment's maxima [R], sums [R] and outputs [R][hd]
+    const int C = R == 16 ? a.cluster : 1, member = C > 1 ? blockIdx.x % C : 0, block = C > 1 ? blockIdx.x / C : blockIdx.x;
     const int per = a.nh / a.nkv, kvh = blockIdx.y / a.slices, h0 = kvh * per + blockIdx.y % a.slices * a.heads;
-    int t0 = blockIdx.x * a.tokens, left = a.T - t0;
+    int t0 = block * a.tokens, left = a.T - t0;
     if (a.runs) {
-        const int4 run = a.runs[blockIdx.x / a.parts];
-        const int behind = blockIdx.x % a.parts * a.tokens;
+        const int4 run = a.runs[block / a.parts];
+        const int behind = block % a.parts * a.tokens;
         t0 = run.y + behind; left = run.z - behind;
         if (left <= 0) return;
     }
@@ -165,15 +200,18 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tile_kernel(AttentionTil
         qt[ag_turned(c, r)] = v.x; qt[ag_turned(c + 1, r)] = v.y; qt[ag_turned(c + 2, r)] = v.z; qt[ag_turned(c + 3, r)] = v.w;
     }
     __syncthreads();
-    float m[RT], l[RT];
-    float4 acc[RT][NJ];
+    float m[RT], l[RT], m_all[RT], l_all[RT];              // of a segment, and of those before it
+    float4 acc[RT][NJ], all[RT][NJ];
+    float joined_m[NJ], joined_l[NJ];                      // a cluster: of the rows whose columns this thread joins
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) { joined_m[j] = -INFINITY; joined_l[j] = 0.f; }
     int my_pos[RT], my_run[RT];
 #pragma unroll
     for (int i = 0; i < RT; ++i) {
-        m[i] = -INFINITY; l[i] = 0.f;
+        m[i] = m_all[i] = -INFINITY; l[i] = l_all[i] = 0.f;
         my_pos[i] = pos_s[ty * RT + i]; my_run[i] = one ? (ty * RT + i < rows ? 0 : -1) : run_s[ty * RT + i] >= 0 ? run_s[ty * RT + i] : last_s;
 #pragma unroll
-        for (int j = 0; j < NJ; ++j) acc[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int j = 0; j < NJ; ++j) acc[i][j] = all[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     // Where a page's rows are few enough registers (PRE: a thread's share of up to PU vectors of keys and of values), the next page
     // travels while this one is used.  A thread's vectors are AT_THREADS apart: their (key, entry) advance by fixed steps.
@@ -199,16 +237,9 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tile_kernel(AttentionTil
         const int* table = a.table + (size_t)seq * a.table_stride;
         const int page_lo = a.window > 0 && lowest - a.window + 1 > 0 ? (lowest - a.window + 1) / PE_PAGE : 0;
         const int page_hi = highest / PE_PAGE;
-        int page = table[page_lo];
         const auto base_of = [&](int pg) { return ((size_t)pg * a.nkv + kvh) * PE_PAGE * hd; };
-        if (PRE && page >= 0) fetch(base_of(page));
-        for (int pg = page_lo; pg <= page_hi; ++pg) {
-            const int here = page;
-            page = pg < page_hi ? table[pg + 1] : -1;
-            if (here < 0) {
-                if (PRE && page >= 0) fetch(base_of(page));
-                continue;
-            }
+        int page = -1;                                     // the one whose keys and values are on their way (PRE)
+        const auto visit = [&](int pg, int here) {         // a page's keys
             __syncthreads();                               // the page before has been used
             int j = j_first, c = c_first;
             if constexpr (PRE) {
@@ -249,11 +280,21 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tile_kernel(AttentionTil
             bool whole = true;                             // this thread's rows see the whole page
 #pragma unroll
             for (int i = 0; i < RT; ++i) {
+                const int first_key = pg * PE_PAGE;
+                whole = whole && my_run[i] == from && my_pos[i] >= first_key + PE_PAGE - 1 && (a.window <= 0 || my_pos[i] - first_key < a.window);
+            }
+#pragma unroll
+            for (int i = 0; i < RT; ++i) {
+                s[i].x *= a.scale; s[i].y *= a.scale; s[i].z *= a.scale; s[i].w *= a.scale;
+                if (whole) continue;
                 const int hi = my_run[i] == from ? my_pos[i] - key0 : -1, lo = a.window > 0 ? hi - a.window + 1 : 0;      // keys lo .. hi of the four
-                s[i].x = hi >= 0 && lo <= 0 ? s[i].x * a.scale : -INFINITY;
-                s[i].y = hi >= 1 && lo <= 1 ? s[i].y * a.scale : -INFINITY;
-                s[i].z = hi >= 2 && lo <= 2 ? s[i].z * a.scale : -INFINITY;
-                s[i].w = hi >= 3 && lo <= 3 ? s[i].w * a.scale : -INFINITY;
+                s[i].x = hi >= 0 && lo <= 0 ? s[i].x : -INFINITY;
+                s[i].y = hi >= 1 && lo <= 1 ? s[i].y : -INFINITY;
+                s[i].z = hi >= 2 && lo <= 2 ? s[i].z : -INFINITY;
+                s[i].w = hi >= 3 && lo <= 3 ? s[i].w : -INFINITY;
+            }
+#pragma unroll
+            for (int i = 0; i < RT; ++i) {
                 float mx = fmaxf(fmaxf(s[i].x, s[i].y), fmaxf(s[i].z, s[i].w));
 #pragma unroll
                 for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
@@ -269,8 +310,6 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tile_kernel(AttentionTil
 #pragma unroll
                     for (int j = 0; j < NJ; ++j) { acc[i][j].x *= alpha; acc[i][j].y *= alpha; acc[i][j].z *= alpha; acc[i][j].w *= alpha; }
                 }
-                const int first_key = pg * PE_PAGE;
-                whole = whole && my_run[i] == from && my_pos[i] >= first_key + PE_PAGE - 1 && (a.window <= 0 || my_pos[i] - first_key < a.window);
             }
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
@@ -299,20 +338,110 @@ __global__ void __launch_bounds__(AT_THREADS) attention_tile_kernel(AttentionTil
             };
             if (__all_sync(0xffffffffu, whole)) add_values(PE_PAGE, ag_no());
             else add_values(min(PE_PAGE, highest - pg * PE_PAGE + 1), ag_yes());
+        };
+        const auto fresh = [&]() {
+#pragma unroll
+            for (int i = 0; i < RT; ++i) {
+                if (my_run[i] != from) continue;
+                m[i] = -INFINITY; l[i] = 0.f;
+#pragma unroll
+                for (int j = 0; j < NJ; ++j) acc[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        };
+        if (C == 1) {
+            int segment = -1;
+            const auto join = [&]() {                      // the segment joins those before it
+#pragma unroll
+                for (int i = 0; i < RT; ++i) {
+                    float before, now;
+                    if (my_run[i] != from) continue;
+                    ag_join(m_all[i], l_all[i], m[i], l[i], before, now);
+#pragma unroll
+                    for (int j = 0; j < NJ; ++j) ag_join4(all[i][j], before, acc[i][j], now);
+                }
+                fresh();
+            };
+            page = table[page_lo];
+            if (PRE && page >= 0) fetch(base_of(page));
+            for (int pg = page_lo; pg <= page_hi; ++pg) {
+                const int here = page;
+                page = pg < page_hi ? table[pg + 1] : -1;
+                if (here < 0) {
+                    if (PRE && page >= 0) fetch(base_of(page));
+                    continue;
+                }
+                if (pg / AG_SEGMENT != segment) {
+                    if (segment >= 0) join();
+                    segment = pg / AG_SEGMENT;
+                }
+                visit(pg, here);
+            }
+            join();
+        } else {
+            // a member of a cluster has every C-th segment; all of them take as many turns
+            const auto following = [&](int pg) { return ++pg % AG_SEGMENT ? pg : pg + (C - 1) * AG_SEGMENT; };
+            const auto page_at = [&](int pg) { return pg >= page_lo && pg <= page_hi ? table[pg] : -1; };
+            const int past = (page_hi / AG_SEGMENT + 1 + member) * AG_SEGMENT;
+            int pg = (page_lo / AG_SEGMENT + member) * AG_SEGMENT, turns = 0;
+            page = page_at(pg);
+            if (PRE && page >= 0) fetch(base_of(page));
+            for (; pg < past; pg = following(pg)) {
+                const int here = page;
+                page = page_at(following(pg));
+                if (here >= 0) visit(pg, here);
+                else if (PRE && page >= 0) fetch(base_of(page));
+                if (pg % AG_SEGMENT != AG_SEGMENT - 1) continue;
+                // C segments join those before them, each of its CTA: a thread four columns of a row
+                float* mine = joint + (turns & (a.buffers - 1)) * R * (hd + 2);
+                if (tx == 0) { mine[ty] = m[0]; mine[R + ty] = l[0]; }
+    #pragma unroll
+                for (int j = 0; j < NJ; ++j)
+                    if (tx * 4 + 64 * j < hd) *reinterpret_cast<float4*>(mine + 2 * R + ty * hd + tx * 4 + 64 * j) = acc[0][j];
+                ag_cluster_sync();
+    #pragma unroll
+                for (int j = 0; j < NJ; ++j) {
+                    const int i = member + C * (tid + j * AT_THREADS), r = i / per4, c = i % per4 * 4;
+                    if (r >= rows) break;
+    #pragma unroll 1
+                    for (int p0 = 0; p0 < C; p0 += 2) {        // (C is a power of two)
+                        float ms[2], ls[2], before, now;
+                        float4 vs2[2];
+    #pragma unroll
+                        for (int p = 0; p < 2; ++p) { ms[p] = ag_peer1(mine + r, p0 + p); ls[p] = ag_peer1(mine + R + r, p0 + p); vs2[p] = ag_peer4(mine + 2 * R + r * hd + c, p0 + p); }
+    #pragma unroll
+                        for (int p = 0; p < 2; ++p) {
+                            ag_join(joined_m[j], joined_l[j], ms[p], ls[p], before, now);
+                            ag_join4(all[0][j], before, vs2[p], now);
+                        }
+                    }
+                }
+                if (a.buffers == 1) ag_cluster_sync();         // (with two, nobody is two turns ahead of a reader)
+                ++turns;
+                fresh();
+            }
         }
         from = to;
+    }
+    const auto store = [&](int r, int c, const float4& v, float sum) {
+        const float inv = sum > 0.f ? 1.0f / sum : 0.f;
+        ag_store4((T*)a.out + ((size_t)(t0 + r / n_heads) * a.nh + h0 + r % n_heads) * hd + c, make_float4(v.x * inv, v.y * inv, v.z * inv, v.w * inv));
+    };
+    if (C > 1) {
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+            const int i = member + C * (tid + j * AT_THREADS);
+            if (i / per4 < rows) store(i / per4, i % per4 * 4, all[0][j], joined_l[j]);
+        }
+        ag_cluster_sync();                                 // nobody leaves while its sums are being read
+        return;
     }
 #pragma unroll
     for (int i = 0; i < RT; ++i) {
         const int r = ty * RT + i;
         if (r >= rows) continue;
-        const float inv = l[i] > 0.f ? 1.0f / l[i] : 0.f;
-        T* o = (T*)a.out + ((size_t)(t0 + r / n_heads) * a.nh + h0 + r % n_heads) * hd;
 #pragma unroll
-        for (int j = 0; j < NJ; ++j) {
-            const int c = tx * 4 + 64 * j;
-            if (c < hd) ag_store4(o + c, make_float4(acc[i][j].x * inv, acc[i][j].y * inv, acc[i][j].z * inv, acc[i][j].w * inv));
-        }
+        for (int j = 0; j < NJ; ++j)
+            if (tx * 4 + 64 * j < hd) store(r, tx * 4 + 64 * j, all[i][j], l_all[i]);
     }
 }
 
@@ -325,18 +454,23 @@ static int attention_tile_as(AttentionTileArgs a, int n_runs, int most, cudaStre
     a.parts = (AG_RUN + a.tokens - 1) / a.tokens;
     if (a.runs) a.tokens = (AG_RUN + a.parts - 1) / a.parts;          // a whole run in equal parts
     const int blocks = a.runs ? n_runs * a.parts : (a.T + a.tokens - 1) / a.tokens;
-    const size_t smem = sizeof(float) * ((size_t)3 * a.hd * 64 + 64 * R);
+    // A cluster for each block of one sequence's rows where those leave SMs idle: as many CTAs as the longest context has segments.
+    a.cluster = 1;
+    if (R == 16 && (a.runs || a.tokens == 1))
+        while (a.cluster < 8 && (long long)2 * a.cluster * blocks * a.nkv * a.slices <= 2 * 148 && a.cluster * AG_SEGMENT < a.table_stride) a.cluster *= 2;
+    a.buffers = a.hd > 192 ? 1 : 2;
+    const size_t smem = sizeof(float) * ((size_t)3 * a.hd * 64 + 64 * R + (a.cluster > 1 ? a.buffers * R * (a.hd + 2) : 0));
     auto kernel = attention_tile_kernel<T, R, NJ>;
     PE_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    PE_TRY(pe_launch(kernel, dim3(blocks, a.nkv * a.slices), AT_THREADS, smem, s, a));
+    PE_TRY(pe_launch_cluster(kernel, dim3(blocks * a.cluster, a.nkv * a.slices), AT_THREADS, smem, s, a.cluster, a));
     PE_LAUNCH_CHECK();
     return 0;
 }
 template <typename T>
 static int attention_tile(const AttentionTileArgs& a, int n_runs, int sequences, cudaStream_t s) {
     const int per = a.nh / a.nkv, few = per < 16 ? 16 / per : 1;      // tokens of a block of 16 rows
-    // Which blocks: 16 rows while those fill half of the SMs at most, else 64 (14 heads of 64 on 2, 60 tokens alone 7.6 / 10.5 us, 20 behind
-    // 4,000 261 / 363, 100 behind 4,000 418 / 373).  Where no runs are known a block may get tokens of several sequences, which
+    // Which blocks: 16 rows while those fill half of the SMs at most, else 64 (14 heads of 64 on 2, before rows of few blocks were dealt out to clusters: 60
+    // tokens alone 7.6 / 10.5 us, 20 behind 4,000 261 / 363, 100 behind 4,000 418 / 373).  Where no runs are known a block may get tokens of several sequences, which
     // it serves one after the other: no more of them than a quarter of what a sequence brings on average, and so single ones where they bring few.
     // One prompt of 40 tokens beside 30 single tokens at 600, float32, on a B200, a block a token and head / 64 rows of neighbouring tokens
     // / runs: 14 heads of 64 on 2 255 / 506 / 71 us, 4 of 256 on one 275 / 3,801 / 173.
@@ -359,7 +493,7 @@ extern "C" int pe_attention_generic(const void* q, int q_stride, void* out, cons
     const size_t size = dtype == PE_F32 ? 4 : 2;
     if ((dtype == PE_F32 || dtype == PE_BF16) && hd % 4 == 0 && q_stride % 4 == 0 && !(((uintptr_t)q | (uintptr_t)out | (uintptr_t)k_pool | (uintptr_t)v_pool) % (4 * size))) {
         // rows of four entries that can be read at once: tiles of rows
-        const AttentionTileArgs a = {q, q_stride, out, k_pool, v_pool, block_table, table_stride, tok_pos, tok_row, T, nh, nkv, hd, window, scale, 0, 0, 0,
+        const AttentionTileArgs a = {q, q_stride, out, k_pool, v_pool, block_table, table_stride, tok_pos, tok_row, T, nh, nkv, hd, window, scale, 0, 0, 0, 1, 1,
                                      (const int4*)runs, 0};
         return dtype == PE_F32 ? attention_tile<float>(a, n_runs, sequences, s) : attention_tile<bf16>(a, n_runs, sequences, s);
     }

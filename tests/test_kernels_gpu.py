@@ -234,6 +234,28 @@ def test_attention_generic_alone_and_among_others(K, nh, nkv, hd, lens, window):
         assert torch.equal(run([j])[0], whole[j]), j
 
 
+@pytest.mark.parametrize("nh,nkv,hd,window", [(14, 2, 64, None), (4, 4, 128, 300), (3, 1, 256, None), (6, 2, 20, 129)])
+def test_attention_generic_over_a_long_context(K, nh, nkv, hd, window):
+    """Single tokens whose pages are dealt out to a cluster, one and several turns of it, first and last places of pages and of segments:
+    against the plain attention, and the same bits as in a step of all tokens."""
+    lens = [1100, 70]
+    paged = Paged(lens, nkv, hd, torch.float32, seed=hd)
+    tok_row = [b for b, n in enumerate(lens) for _ in range(n)]
+    tok_pos = [p for n in lens for p in range(n)]
+    q = rnd(len(tok_row), nh, hd, seed=nh)
+    kp, vp, table = paged.cuda()
+    run = lambda i: K.attention_generic(dev(q[i].reshape(len(i), -1).contiguous()), nh * hd, nh, nkv, hd, kp, vp, table, table.shape[1],
+                                        dev(torch.tensor([tok_pos[j] for j in i], dtype=torch.int32)),
+                                        dev(torch.tensor([tok_row[j] for j in i], dtype=torch.int32)), window, hd ** -0.5)
+    whole = run(list(range(len(tok_row))))
+    some = [0, 63, 64, 127, 128, 255, 256, 700, 1023, 1024, 1099, 1100, 1169]
+    want = reference_attention(q[some], paged, [tok_row[j] for j in some], [tok_pos[j] for j in some], nh, window)
+    assert torch.allclose(whole[some].cpu(), want.reshape(len(some), -1), atol=2e-5, rtol=2e-5)
+    for j in some:
+        assert torch.equal(run([j])[0], whole[j]), j
+    assert torch.equal(run(some[5:]), whole[some[5:]])
+
+
 @pytest.mark.parametrize("nh,nkv,hd,lens,window", CASES)
 @pytest.mark.parametrize("max_context", [None, 4096])
 def test_attention_decode(K, nh, nkv, hd, lens, window, max_context):
