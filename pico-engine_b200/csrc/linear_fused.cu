@@ -29,6 +29,8 @@
 // SWIGLU the matching gate and up rows, for ROPE the two halves of a head that rotate
 // together, so the epilogue finds its pairs in one CTA.
 //
+// Larger products go to linear_stream.cuh's kernel, which keeps a ring of W full over several tiles (ls_takes).
+//
 // Waiting on an mbarrier is bounded: a wait that runs out sets *status to 1 and the CTA
 // returns, leaving its outputs unwritten; the host reads the status word with its results.
 //
@@ -492,9 +494,12 @@ extern "C" void pe_linear_fused_set_two_tiles(int on) { lf_two_tiles() = on ? 1 
 static int& lf_ksplit_limit() { static int limit = 8; return limit; }
 extern "C" void pe_linear_fused_set_max_ksplit(int n) { lf_ksplit_limit() = n < 1 ? 1 : (n > 8 ? 8 : n); }
 
+#include "linear_stream.cuh"
+
 template <int PRO, int EPI>
 static int lf_launch(LfArgs& a, int tiles, int* status, cudaStream_t s) {
     if (!status) return PE_ERR_UNSUPPORTED;
+    if (ls_takes(a, PRO == LF_RMSNORM, EPI)) return ls_launch<PRO, EPI>(a, status, s);
     // A long K with few tiles (fewer CTAs than the GPU has SMs): cut K into ranges, one CTA each, up to
     // 8 to a cluster, while the grid stays within two to three CTAs an SM.
     a.ksplit = 1;

@@ -472,10 +472,9 @@ def check_status(device) -> None:
         raise KernelError(f"a kernel gave up a bounded wait (status {code}); its results are incomplete")
 
 
-# A weight this large streams faster through the library's product even for a few rows: measured on a B200 at
-# 8 rows, 37888 x 3584 (271 MB): 46 us (5.9 TB/s) against 61 us; 3584 x 18944 (136 MB): 28 us against 33 us;
-# 151936 x 896 (272 MB, into float32): 52 us against 72 us.  The fused kernel's CTAs restart their pipeline
-# for every tile; smaller weights are faster there, with what precedes and follows the product fused in.
+# A weight this large streams faster through the library's product even for a few rows where a CTA of the fused kernels would end with every
+# tile: measured on a B200 at 8 rows, 151936 x 896 (272 MB, into float32): 52 us against 72 us; 152064 x 3584: 178 us against 189 in the kernel that
+# keeps its ring full.  _streams names those that are faster here.
 FUSED_MAX_WEIGHT_BYTES = int(os.environ.get("PICO_ENGINE_FUSED_MAX_MB", "100")) << 20
 
 
@@ -483,7 +482,16 @@ def fused_takes(rows: int, w: torch.Tensor, *others: torch.Tensor, max_rows: int
     """Whether the fused decode kernels take a product with ``rows`` rows and weight ``w``."""
     return (rows <= max_rows and w.dtype == torch.bfloat16 and w.shape[1] % 8 == 0 and w.is_contiguous()
             and w.data_ptr() % 16 == 0 and all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in others)
-            and w.numel() * 2 <= FUSED_MAX_WEIGHT_BYTES)
+            and (w.numel() * 2 <= FUSED_MAX_WEIGHT_BYTES or (rows <= FUSED_MAX_ROWS and _streams(w, others))))
+
+
+def _streams(w: torch.Tensor, others) -> bool:
+    """Larger weights whose rings stay full (csrc/linear_stream.cuh): of normed float32 rows that fit shared memory, and of bfloat16 rows where
+    a CTA has one group of rows."""
+    N, K = w.shape
+    if others and others[0].dtype == torch.float32:
+        return 1024 <= K <= 4096
+    return 1280 <= N <= 4736
 
 
 # The same fused products for 17 to 64 rows are another kernel (csrc/linear_batch.cu: 64 rows of the weight a CTA

@@ -790,6 +790,49 @@ def test_linear_fused_rows_do_not_depend_on_their_neighbours(K):
         assert torch.equal(K.linear_fused(dev(a[rows].to(torch.bfloat16)), W, out_dtype=torch.float32), whole[rows])
 
 
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+@pytest.mark.parametrize("N,K_", [(1333, 520), (2073, 1544), (4736, 584),      # one group a CTA: a box, two, the most rows; K ends inside 64 columns
+                                  (9500, 648), (14000, 520),                   # several groups a CTA, the last one in part
+                                  (2048, 4096)])                               # the longest normed rows
+def test_linear_fused_streams(K, M, N, K_):
+    """Products whose rings stay full over several groups of rows: stored, summed, of normed rows, alone and among others."""
+    a, w, b = bf(rnd(16, K_, seed=1)), bf(rnd(N, K_, seed=2, scale=K_ ** -0.5)), bf(rnd(N, seed=3))
+    want = a[:M].double() @ w.double().T
+    A, W = dev(a.to(torch.bfloat16)), dev(w.to(torch.bfloat16))
+    got = K.linear_fused(A[:M], W, out_dtype=torch.float32)
+    assert torch.allclose(got.cpu().double(), want, atol=1e-4, rtol=1e-4), float((got.cpu().double() - want).abs().max())
+    assert torch.equal(got, K.linear_fused(A, W, out_dtype=torch.float32)[:M])
+    got = K.linear_fused(A[:M], W, dev(b), out_dtype=torch.bfloat16)
+    assert torch.allclose(got.float().cpu().double(), want + b.double(), atol=4e-2, rtol=1e-2)
+    x = rnd(M, N, seed=4)
+    got = K.linear_fused(A[:M], W, dev(b.to(torch.bfloat16)), accumulate_into=dev(x.clone()))
+    assert torch.allclose(got.cpu().double(), x.double() + want + b.double(), atol=1e-4, rtol=1e-4)
+    xs, nw = rnd(16, K_, seed=5, scale=2.0), bf(1 + rnd(K_, seed=6) * 0.1)
+    h = plain.rms_norm(xs, nw, 1e-5).to(torch.bfloat16).double()
+    for nw_dtype in (torch.bfloat16, torch.float32):
+        run = lambda m: K.linear_fused(None, W, out_dtype=torch.float32, norm_of=dev(xs[:m]), norm_weight=dev(nw.to(nw_dtype)), eps=1e-5)
+        got = run(M)
+        assert torch.allclose(got.cpu().double(), (h @ w.double().T)[:M], atol=3e-2, rtol=1e-2)   # a bfloat16 rounding of h may flip
+        assert torch.equal(got, run(16)[:M])
+    K.check_status("cuda")
+
+
+@pytest.mark.parametrize("M", [1, 8, 13])
+@pytest.mark.parametrize("H,I", [(1032, 5000), (2048, 150), (4096, 2368), (600, 2300)])
+def test_gate_up_streams(K, M, H, I):
+    """Gate and up rows in boxes of up to 16, whole and partial last groups, of normed and of bfloat16 rows."""
+    x, nw = rnd(M, H, seed=1, scale=2.0), bf(1 + rnd(H, seed=2) * 0.1)
+    w = bf(rnd(2 * I // 16 * 16, H, seed=3, scale=H ** -0.5))
+    I = w.shape[0] // 2
+    h = plain.rms_norm(x, nw, 1e-6).to(torch.bfloat16).float()
+    gu = (h @ w.T).to(torch.bfloat16).float()
+    got = K.norm_gate_up_swiglu(dev(x), dev(nw.to(torch.bfloat16)), 1e-6, dev(w.to(torch.bfloat16)))
+    assert got.shape == (M, I) and torch.allclose(got.float().cpu(), plain.swiglu(gu[:, :I], gu[:, I:]), atol=3e-2, rtol=3e-2)
+    got = K.gate_up_act(dev(h.to(torch.bfloat16)), dev(w.to(torch.bfloat16)), "relu")
+    assert torch.allclose(got.float().cpu(), gu[:, :I].relu() * gu[:, I:], atol=3e-2, rtol=3e-2)
+    K.check_status("cuda")
+
+
 @pytest.mark.parametrize("M,H,I", [(1, 64, 160), (8, 896, 4864), (16, 96, 352), (5, 3584, 1000), (13, 512, 2504),
                                    (16, 896, 4864)])           # the last three take two row tiles a CTA; 2504 / 8 is odd
 def test_norm_gate_up_swiglu(K, M, H, I):
@@ -835,6 +878,13 @@ def test_norm_qkv_rope_store(K, nq, nkv, hd, H, theta, rotate):
     K.norm_qkv_rope_store(dev(x), dev(nw.to(torch.bfloat16)), 1e-6, dev(w.to(torch.bfloat16)), None, nq, nkv, hd,
                           None, None, dev(pos), dev(row), None, None, dev(table), 3)
     assert float(kp.abs().sum()) == 0.0
+
+
+@pytest.mark.parametrize("nq,nkv,hd,H,theta,rotate", [(7, 1, 128, 1032, 1e6, True), (12, 12, 48, 520, 1e4, True), (60, 4, 16, 520, 1e4, True),
+                                                       (28, 4, 128, 3584, 1e6, True), (14, 2, 128, 3624, 1e6, True)])
+def test_norm_qkv_rope_store_streams(K, nq, nkv, hd, H, theta, rotate):
+    """The same in boxes of 16 and 8 rows of a head's half, one and several groups a CTA."""
+    test_norm_qkv_rope_store(K, nq, nkv, hd, H, theta, rotate)
 
 
 # ---------------------------------------------------------------------------- the same for 17 to 64 rows (csrc/linear_batch.cu)
