@@ -15,6 +15,8 @@
 //
 // Head sizes that are multiples of 8: D up to 64 (a key row's 64-column box is filled with zeros beyond D, so what the query box holds
 // there does not count), Dv up to 128.  Every mbarrier wait is bounded (*status 5), as in attention_prefill_tcgen05.cu.
+// Bound by a step's chain (scores, maximum, exponentials, P).  Prompts of 1,500 and 500 tokens, 8 heads of 2 x 64, window 1,024, on a B200:
+// 51.7 us with a chain of comparisons a score, single sums and rows stored by their own lanes, 47.4 us here.
 #include "tcgen05_attention.cuh"
 
 #define DT_QTILE 128
@@ -57,6 +59,31 @@ __global__ void __launch_bounds__(DT_THREADS, 1) attention_diff_tcgen05_kernel(c
         if (threadIdx.x == 0) atomicExch(status, 6);
         return;
     }
+    // (the step's description and the page table: no kernel writes them)
+    const int4 info = p.tiles[blockIdx.y];                          // heads vary fastest: the runs that see the most keys start first
+    const int brow = info.x, tok0 = info.y, n = info.z, pos0 = info.w;
+    const int per = p.H / p.G, h = blockIdx.x, g_kv = h / per;
+    const int first_key = (p.window > 0 && pos0 - p.window + 1 > 0) ? pos0 - p.window + 1 : 0;
+    const int page_lo = first_key / DT_KTILE, page_hi = (pos0 + n - 1) / DT_KTILE;
+    const int n_pages = page_hi - page_lo + 1, n_steps = (n_pages + 1) / 2, n_its = 2 * n_steps;      // an iteration: one step of one map
+    const int* table = p.block_table + (size_t)brow * p.table_stride;
+    auto bring = [&](int s, const int (&page)[2]) {                  // a stage: two pages
+        const unsigned bar = at_smem(&kv_full[s]), k_dst = kv_s + s * DT_STAGE_BYTES(VP), v_dst = k_dst + 2 * DT_PANEL;
+        stage_flags[s] = (page[0] >= 0 ? 1u : 0u) | (page[1] >= 0 ? 2u : 0u);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((unsigned)DT_STAGE_BYTES(VP)) : "memory");
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+            // a page that is not there is read from beyond the pool's end, which gives zeros: its scores are masked and its
+            // values add nothing
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+                at_tma_2d(k_dst + m * DT_PANEL + g * (DT_KTILE * 128), &map_k, 0,
+                          page[g] >= 0 ? ((page[g] * p.G + g_kv) * 2 + m) * DT_KTILE : p.k_rows, bar);
+#pragma unroll
+            for (int c = 0; c < VP; ++c)
+                at_tma_2d(v_dst + c * DT_PANEL + g * (DT_KTILE * 128), &map_v, 64 * c, page[g] >= 0 ? (page[g] * p.G + g_kv) * DT_KTILE : p.v_rows, bar);
+        }
+    };
     if (threadIdx.x == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(at_smem(&q_full)) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 8;" ::"r"(at_smem(&p_full)) : "memory");          // the eight softmax warps
@@ -70,7 +97,14 @@ __global__ void __launch_bounds__(DT_THREADS, 1) attention_diff_tcgen05_kernel(c
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 8;" ::"r"(at_smem(&s_free[b])) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(at_smem(&pv_done[b])) : "memory");
         }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;\n\tfence.proxy.async.shared::cta;" ::: "memory");
+        // the queries and the first step are asked for before the block meets
+        const int first[2] = {table[page_lo], 1 < n_pages ? table[page_lo + 1] : -1};
+        pdl_wait();
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(at_smem(&q_full)), "r"((unsigned)(2 * DT_PANEL)) : "memory");
+#pragma unroll
+        for (int m = 0; m < 2; ++m) at_tma_2d(q_s + m * DT_PANEL, &map_q, ((2 * g_kv + m) * per + h % per) * p.D, tok0, at_smem(&q_full));
+        bring(0, first);
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(at_smem(&tmem_base_s)), "r"((unsigned)DT_TMEM_COLS) : "memory");
@@ -84,41 +118,16 @@ __global__ void __launch_bounds__(DT_THREADS, 1) attention_diff_tcgen05_kernel(c
     pdl_launch_dependents();
     pdl_wait();
 
-    const int4 info = p.tiles[blockIdx.y];                          // heads vary fastest: the runs that see the most keys start first
-    const int brow = info.x, tok0 = info.y, n = info.z, pos0 = info.w;
-    const int per = p.H / p.G, h = blockIdx.x, g_kv = h / per;
-    const int first_key = (p.window > 0 && pos0 - p.window + 1 > 0) ? pos0 - p.window + 1 : 0;
-    const int page_lo = first_key / DT_KTILE, page_hi = (pos0 + n - 1) / DT_KTILE;
-    const int n_pages = page_hi - page_lo + 1, n_steps = (n_pages + 1) / 2, n_its = 2 * n_steps;      // an iteration: one step of one map
-
     if (warp == 0) {
         if (lane == 0) {                                            // ---------------- loader
-            const int* table = p.block_table + (size_t)brow * p.table_stride;
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(at_smem(&q_full)), "r"((unsigned)(2 * DT_PANEL)) : "memory");
-#pragma unroll
-            for (int m = 0; m < 2; ++m) at_tma_2d(q_s + m * DT_PANEL, &map_q, ((2 * g_kv + m) * per + h % per) * p.D, tok0, at_smem(&q_full));
-            int page[2] = {table[page_lo], 1 < n_pages ? table[page_lo + 1] : -1};
-            for (int st = 0; st < n_steps; ++st) {
+            int page[2] = {2 < n_pages ? table[page_lo + 2] : -1, 3 < n_pages ? table[page_lo + 3] : -1};
+            for (int st = 1; st < n_steps; ++st) {
                 const int s = st % DT_STAGES;
                 int next[2] = {-1, -1};                             // the step after this one: its entries travel during the wait
                 if (2 * st + 2 < n_pages) next[0] = table[page_lo + 2 * st + 2];
                 if (2 * st + 3 < n_pages) next[1] = table[page_lo + 2 * st + 3];
                 if (st >= DT_STAGES && !at_wait(at_smem(&kv_empty[s]), (unsigned)((st / DT_STAGES) - 1) & 1u)) { atomicExch(status, 5); break; }
-                const unsigned bar = at_smem(&kv_full[s]), k_dst = kv_s + s * DT_STAGE_BYTES(VP), v_dst = k_dst + 2 * DT_PANEL;
-                stage_flags[s] = (page[0] >= 0 ? 1u : 0u) | (page[1] >= 0 ? 2u : 0u);
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((unsigned)DT_STAGE_BYTES(VP)) : "memory");
-#pragma unroll
-                for (int g = 0; g < 2; ++g) {
-                    // a page that is not there is read from beyond the pool's end, which gives zeros: its scores are masked and its
-                    // values add nothing
-#pragma unroll
-                    for (int m = 0; m < 2; ++m)
-                        at_tma_2d(k_dst + m * DT_PANEL + g * (DT_KTILE * 128), &map_k, 0,
-                                  page[g] >= 0 ? ((page[g] * p.G + g_kv) * 2 + m) * DT_KTILE : p.k_rows, bar);
-#pragma unroll
-                    for (int c = 0; c < VP; ++c)
-                        at_tma_2d(v_dst + c * DT_PANEL + g * (DT_KTILE * 128), &map_v, 64 * c, page[g] >= 0 ? (page[g] * p.G + g_kv) * DT_KTILE : p.v_rows, bar);
-                }
+                bring(s, page);
                 page[0] = next[0]; page[1] = next[1];
             }
         }
@@ -169,6 +178,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) attention_diff_tcgen05_kernel(c
         const unsigned lane_addr = tmem + ((unsigned)(quarter * 32) << 16);
         const unsigned o_addr = lane_addr + DT_O_COL + g * (VP * 32);
         const unsigned pair = at_smem(&pair_bar[quarter]);
+        const unsigned long long scale2 = at_two(p.scale_log2e, p.scale_log2e);
         float m_run = -INFINITY, l_run = 0.f, m_alt = -INFINITY, l_alt = 0.f;      // of this iteration's map and of the other
         bool ok = true;
         int it = 0, met = 0;                                        // met: how often the row's two threads have met
@@ -203,13 +213,13 @@ __global__ void __launch_bounds__(DT_THREADS, 1) attention_diff_tcgen05_kernel(c
             float s[DT_KTILE];
 #pragma unroll
             for (int c = 0; c < DT_KTILE; ++c) s[c] = __uint_as_float(raw[c]);
-            const bool whole = there && key0 + DT_KTILE - 1 <= p_r && (p.window <= 0 || key0 > p_r - p.window);
-            if (!whole) {
+            const int hi = there ? p_r - key0 : -1;                 // the last of the page's keys that the row sees
+            if (p.window <= 0) {
+                if (hi < DT_KTILE - 1) at_mask_behind<DT_KTILE>(s, hi);
+            } else if (const int lo = p_r - p.window + 1 - key0; hi < DT_KTILE - 1 || lo > 0) {      // lo: the window's first one
 #pragma unroll
-                for (int c = 0; c < DT_KTILE; ++c) {
-                    const int key = key0 + c;
-                    if (!there || key > p_r || (p.window > 0 && key <= p_r - p.window)) s[c] = -INFINITY;
-                }
+                for (int c = 0; c < DT_KTILE; ++c)
+                    if (c > hi || c < lo) s[c] = -INFINITY;
             }
             float mx[4] = {s[0], s[1], s[2], s[3]};
 #pragma unroll
@@ -223,15 +233,12 @@ __global__ void __launch_bounds__(DT_THREADS, 1) attention_diff_tcgen05_kernel(c
             const float m_use = m_new == -INFINITY ? 0.f : m_new;
             const float alpha = m_run == -INFINITY ? 1.0f : at_exp2(m_run - m_use);
             m_run = m_new;
-            float sum[4] = {0.f, 0.f, 0.f, 0.f};
+            unsigned long long sum[2] = {0ull, 0ull};
+            const unsigned long long off = at_two(-m_use, -m_use);
             unsigned packed[DT_KTILE / 2];
 #pragma unroll
-            for (int c = 0; c < DT_KTILE; c += 2) {
-                const float e0 = at_exp2(fmaf(s[c], p.scale_log2e, -m_use)), e1 = at_exp2(fmaf(s[c + 1], p.scale_log2e, -m_use));
-                sum[c & 3] += e0; sum[(c + 1) & 3] += e1;
-                packed[c >> 1] = at_pack(e0, e1);
-            }
-            l_run = l_run * alpha + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
+            for (int c = 0; c < DT_KTILE; c += 2) packed[c >> 1] = at_exp2_pair(s[c], s[c + 1], scale2, off, sum[(c >> 1) & 1]);
+            l_run = l_run * alpha + at_sum_four(sum[0], sum[1]);
             // the map's P tile is free, and its O holds every earlier step, once P.V of the iteration before last is done
             if (it >= 2) {
                 if (!at_wait_warp(at_smem(&pv_done[b]), (unsigned)((it >> 1) - 1) & 1u)) { ok = false; break; }
@@ -287,14 +294,13 @@ __global__ void __launch_bounds__(DT_THREADS, 1) attention_diff_tcgen05_kernel(c
             }
             float ss_theirs;
             if (!swap(ss, ss_theirs)) ok = false;
-            else if (r < n) {
+            else {                                                  // through the queries' place: the last products have read them
                 const float f = 1.0f / sqrtf((g == 0 ? ss + ss_theirs : ss_theirs + ss) / (float)p.Dv + p.eps) * p.out_scale;
-                bf16* o_row = p.out + (size_t)(tok0 + r) * p.out_ld + p.out_col + (size_t)h * p.Dv + col0;
+                unsigned packed[VP * 16];
 #pragma unroll
-                for (int i = 0; i < VP * 32; i += 8)
-                    if (col0 + i < p.Dv)
-                        *reinterpret_cast<uint4*>(o_row + i) = make_uint4(at_pack(d[i] * f, d[i + 1] * f), at_pack(d[i + 2] * f, d[i + 3] * f),
-                                                                          at_pack(d[i + 4] * f, d[i + 5] * f), at_pack(d[i + 6] * f, d[i + 7] * f));
+                for (int i = 0; i < VP * 16; ++i) packed[i] = at_pack(d[2 * i] * f, d[2 * i + 1] * f);
+                at_put_row<VP * 32>(q_s, VP * 128, r, g * (VP * 4), packed);
+                at_store_rows<VP * 32>(q_s, VP * 128, quarter * 32, g * (VP * 4), n, p.out + (size_t)tok0 * p.out_ld + p.out_col + (size_t)h * p.Dv + col0, (size_t)p.out_ld, lane, p.Dv - col0);
             }
         }
         if (!ok) atomicExch(status, 5);

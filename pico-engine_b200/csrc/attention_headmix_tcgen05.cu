@@ -17,7 +17,8 @@
 //
 // Tensor memory has 256 columns for S and 256 for O: two value heads of 128 or four of 64 a CTA; more are further CTAs, which make S again.
 // Bound by a step's chain (scores, maximum, exponentials, P) rather than by the tensor cores.
-// Measured on a B200, 1,024 tokens, 16 heads of 128 on four key/value heads: 40 + 7 us, where the mma.sync kernel and its merge
+// Measured on a B200, 1,024 tokens, 16 heads of 128 on four key/value heads: 33 + 6 us (40 + 7 with rows of O stored by their own lanes, 32
+// lines an instruction, a chain of comparisons a score and the first loads behind the block's meeting), where the mma.sync kernel and its merge
 // (attention_headmix_flash.cu) take 198 + 83.
 // Head sizes: D a multiple of 16, Dv of 16.  Every mbarrier wait is bounded by the clock; a wait that runs out sets *status to 5, the
 // roles leave their loops, tensor memory is freed and the CTA returns (status 6: shared memory did not start on a 1024-byte boundary).
@@ -63,6 +64,30 @@ __global__ void __launch_bounds__(HT_THREADS, 1) attention_headmix_tcgen05_kerne
         if (threadIdx.x == 0) atomicExch(status, 6);
         return;
     }
+    // (the step's description and the page table: no kernel writes them)
+    const int4 info = p.tiles[blockIdx.y];                          // heads vary fastest: the runs that see the most keys start first
+    const int brow = info.x, tok0 = info.y, n = info.z, pos0 = info.w;
+    const int groups = p.G / p.cg, h = blockIdx.x / groups, c_lo = blockIdx.x % groups * p.cg, kvh = h / (p.H / p.G);
+    const int first_key = (p.window > 0 && pos0 - p.window + 1 > 0) ? pos0 - p.window + 1 : 0;
+    const int page_lo = first_key / HT_KTILE, page_hi = (pos0 + n - 1) / HT_KTILE;
+    const int n_pages = page_hi - page_lo + 1, n_steps = (n_pages + 1) / 2;
+    const int* table = p.block_table + (size_t)brow * p.table_stride;
+    auto bring = [&](int s, const int (&page)[2]) {                  // a stage: two pages
+        const unsigned bar = at_smem(&kv_full[s]), k_dst = kv_s + s * stage_bytes, v_dst = k_dst + p.qp * HT_PANEL;
+        stage_flags[s] = (page[0] >= 0 ? 1u : 0u) | (page[1] >= 0 ? 2u : 0u);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(stage_bytes) : "memory");
+        for (int g = 0; g < 2; ++g) {
+            // a page that is not there is read from beyond the pool's end, which gives zeros: its scores are masked and its
+            // values add nothing; so are a row's entries behind its size (the queries hold the next head's there)
+            const unsigned at = g * (HT_KTILE * 128);
+            for (int c = 0; c < p.qp; ++c)
+                at_tma_2d(k_dst + c * HT_PANEL + at, &map_k, 64 * c, page[g] >= 0 ? (page[g] * p.G + kvh) * HT_KTILE : p.pool_rows, bar);
+            for (int v = 0; v < p.cg; ++v)
+                for (int c = 0; c < p.vp; ++c)
+                    at_tma_2d(v_dst + (v * p.vp + c) * HT_PANEL + at, &map_v, 64 * c,
+                              page[g] >= 0 ? (page[g] * p.G + c_lo + v) * HT_KTILE : p.pool_rows, bar);
+        }
+    };
     if (threadIdx.x == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(at_smem(&q_full)) : "memory");
         for (int q = 0; q < 4; ++q) asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;" ::"r"(at_smem(&pair_bar[q])) : "memory");
@@ -75,7 +100,13 @@ __global__ void __launch_bounds__(HT_THREADS, 1) attention_headmix_tcgen05_kerne
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 8;" ::"r"(at_smem(&p_full[b])) : "memory");      // the eight softmax warps
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(at_smem(&pv_done[b])) : "memory");
         }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;\n\tfence.proxy.async.shared::cta;" ::: "memory");
+        // the queries and the first step are asked for before the block meets
+        const int first[2] = {table[page_lo], 1 < n_pages ? table[page_lo + 1] : -1};
+        pdl_wait();
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(at_smem(&q_full)), "r"((unsigned)(p.qp * HT_PANEL)) : "memory");
+        for (int c = 0; c < p.qp; ++c) at_tma_2d(q_s + c * HT_PANEL, &map_q, h * p.D + 64 * c, tok0, at_smem(&q_full));
+        bring(0, first);
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(at_smem(&tmem_base_s)), "r"((unsigned)HT_TMEM_COLS) : "memory");
@@ -89,40 +120,17 @@ __global__ void __launch_bounds__(HT_THREADS, 1) attention_headmix_tcgen05_kerne
     pdl_launch_dependents();
     pdl_wait();
 
-    const int4 info = p.tiles[blockIdx.y];                          // heads vary fastest: the runs that see the most keys start first
-    const int brow = info.x, tok0 = info.y, n = info.z, pos0 = info.w;
-    const int groups = p.G / p.cg, h = blockIdx.x / groups, c_lo = blockIdx.x % groups * p.cg, kvh = h / (p.H / p.G);
-    const int first_key = (p.window > 0 && pos0 - p.window + 1 > 0) ? pos0 - p.window + 1 : 0;
-    const int page_lo = first_key / HT_KTILE, page_hi = (pos0 + n - 1) / HT_KTILE;
-    const int n_pages = page_hi - page_lo + 1, n_steps = (n_pages + 1) / 2;
-
     if (warp == 0) {
         if (lane == 0) {                                            // ---------------- loader
-            const int* table = p.block_table + (size_t)brow * p.table_stride;
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(at_smem(&q_full)), "r"((unsigned)(p.qp * HT_PANEL)) : "memory");
-            for (int c = 0; c < p.qp; ++c) at_tma_2d(q_s + c * HT_PANEL, &map_q, h * p.D + 64 * c, tok0, at_smem(&q_full));
-            int page[2] = {table[page_lo], 1 < n_pages ? table[page_lo + 1] : -1};
-            int s = 0;
-            unsigned round = 0;                                     // how often the ring has been filled
-            for (int it = 0; it < n_steps; ++it) {
+            int page[2] = {2 < n_pages ? table[page_lo + 2] : -1, 3 < n_pages ? table[page_lo + 3] : -1};
+            int s = p.stages > 1 ? 1 : 0;
+            unsigned round = p.stages > 1 ? 0 : 1;                                     // how often the ring has been filled
+            for (int it = 1; it < n_steps; ++it) {
                 int next[2] = {-1, -1};                             // the step after this one: its entries travel during the wait
                 if (2 * it + 2 < n_pages) next[0] = table[page_lo + 2 * it + 2];
                 if (2 * it + 3 < n_pages) next[1] = table[page_lo + 2 * it + 3];
                 if (round > 0 && !at_wait(at_smem(&kv_empty[s]), (round - 1) & 1u)) { atomicExch(status, 5); break; }
-                const unsigned bar = at_smem(&kv_full[s]), k_dst = kv_s + s * stage_bytes, v_dst = k_dst + p.qp * HT_PANEL;
-                stage_flags[s] = (page[0] >= 0 ? 1u : 0u) | (page[1] >= 0 ? 2u : 0u);
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(stage_bytes) : "memory");
-                for (int g = 0; g < 2; ++g) {
-                    // a page that is not there is read from beyond the pool's end, which gives zeros: its scores are masked and its
-                    // values add nothing; so are a row's entries behind its size (the queries hold the next head's there)
-                    const unsigned at = g * (HT_KTILE * 128);
-                    for (int c = 0; c < p.qp; ++c)
-                        at_tma_2d(k_dst + c * HT_PANEL + at, &map_k, 64 * c, page[g] >= 0 ? (page[g] * p.G + kvh) * HT_KTILE : p.pool_rows, bar);
-                    for (int v = 0; v < p.cg; ++v)
-                        for (int c = 0; c < p.vp; ++c)
-                            at_tma_2d(v_dst + (v * p.vp + c) * HT_PANEL + at, &map_v, 64 * c,
-                                      page[g] >= 0 ? (page[g] * p.G + c_lo + v) * HT_KTILE : p.pool_rows, bar);
-                }
+                bring(s, page);
                 page[0] = next[0]; page[1] = next[1];
                 if (++s == p.stages) { s = 0; ++round; }
             }
@@ -180,6 +188,7 @@ __global__ void __launch_bounds__(HT_THREADS, 1) attention_headmix_tcgen05_kerne
         const int half = p.cg * p.Dv / 2;
         const unsigned o_addr = lane_addr + HT_O_COL + g * half;
         const unsigned pair = at_smem(&pair_bar[quarter]);
+        const unsigned long long scale2 = at_two(p.scale_log2e, p.scale_log2e);
         float m_run = -INFINITY, l_run = 0.f;
         bool ok = true;
         int it = 0, met = 0, st = 0;                                // met: how often the row's two threads have met; st: the step's stage
@@ -214,12 +223,13 @@ __global__ void __launch_bounds__(HT_THREADS, 1) attention_headmix_tcgen05_kerne
             float s[HT_KTILE];
 #pragma unroll
             for (int c = 0; c < HT_KTILE; ++c) s[c] = __uint_as_float(raw[c]);
-            if (!(there && key0 + HT_KTILE - 1 <= p_r && (p.window <= 0 || key0 > p_r - p.window))) {
+            const int hi = there ? p_r - key0 : -1;                 // the last of the page's keys that the row sees
+            if (p.window <= 0) {
+                if (hi < HT_KTILE - 1) at_mask_behind<HT_KTILE>(s, hi);
+            } else if (const int lo = p_r - p.window + 1 - key0; hi < HT_KTILE - 1 || lo > 0) {      // lo: the window's first one
 #pragma unroll
-                for (int c = 0; c < HT_KTILE; ++c) {
-                    const int key = key0 + c;
-                    if (!there || key > p_r || (p.window > 0 && key <= p_r - p.window)) s[c] = -INFINITY;
-                }
+                for (int c = 0; c < HT_KTILE; ++c)
+                    if (c > hi || c < lo) s[c] = -INFINITY;
             }
             float mx[4] = {s[0], s[1], s[2], s[3]};                 // four chains: a warp has little else to hide their latency
 #pragma unroll
@@ -236,15 +246,12 @@ __global__ void __launch_bounds__(HT_THREADS, 1) attention_headmix_tcgen05_kerne
             const float m_use = m_new == -INFINITY ? 0.f : m_new;
             const float alpha = m_run == -INFINITY ? 1.0f : at_exp2(m_run - m_use);
             m_run = m_new;
-            float sum[4] = {0.f, 0.f, 0.f, 0.f};
+            unsigned long long sum[2] = {0ull, 0ull};
+            const unsigned long long off = at_two(-m_use, -m_use);
             float packed[HT_KTILE / 2];
 #pragma unroll
-            for (int c = 0; c < HT_KTILE; c += 2) {
-                const float e0 = at_exp2(fmaf(s[c], p.scale_log2e, -m_use)), e1 = at_exp2(fmaf(s[c + 1], p.scale_log2e, -m_use));
-                sum[c & 3] += e0; sum[(c + 1) & 3] += e1;
-                packed[c >> 1] = __uint_as_float(at_pack(e0, e1));
-            }
-            l_run = l_run * alpha + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
+            for (int c = 0; c < HT_KTILE; c += 2) packed[c >> 1] = __uint_as_float(at_exp2_pair(s[c], s[c + 1], scale2, off, sum[(c >> 1) & 1]));
+            l_run = l_run * alpha + at_sum_four(sum[0], sum[1]);
             at_st32(lane_addr + b * (2 * HT_KTILE) + g * (HT_KTILE / 2), packed);
             if (it > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) { // a row's reference point moved: rescale this half of the warp's rows of O
                 if (!at_wait_warp(at_smem(&pv_done[b ^ 1]), (unsigned)((it - 1) >> 1) & 1u)) { ok = false; break; }
@@ -272,15 +279,20 @@ __global__ void __launch_bounds__(HT_THREADS, 1) attention_headmix_tcgen05_kerne
             float l = g == 0 ? l_run + l_theirs : l_theirs + l_run;         // the same sum in both threads
             if (p.sink) l += at_exp2(fmaf(p.sink[h], 1.4426950408889634f, -m_run));       // (a row that saw no key: 2^inf, and 1 / l = 0)
             const float inv = l > 0.f ? 1.0f / l : 0.f;
-            float* o_row = p.o + (((size_t)(tok0 + r) * p.H + h) * p.G + c_lo) * p.Dv + g * half;      // the group's heads lie side by side
+            // the group's heads lie side by side; through the place of the queries and stages (the last products have read them), 4 KB a warp
+            const unsigned tile = q_s + (warp - 2) * 4096;
+            const size_t row_floats = (size_t)p.H * p.G * p.Dv;
+            float* out = p.o + (size_t)(tok0 + quarter * 32) * row_floats + ((size_t)h * p.G + c_lo) * p.Dv + g * half;
 #pragma unroll 1
             for (int c = 0; c < half; c += 32) {
                 float o[32];
+                unsigned bits[32];
                 at_ld32(o_addr + c, o);
-                if (r < n) {
 #pragma unroll
-                    for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(o_row + c + i) = make_float4(o[i] * inv, o[i + 1] * inv, o[i + 2] * inv, o[i + 3] * inv);
-                }
+                for (int i = 0; i < 32; ++i) bits[i] = __float_as_uint(o[i] * inv);
+                at_put_row<64>(tile, 128, lane, 0, bits);           // 32 numbers of 4 bytes
+                at_store_rows<64>(tile, 128, 0, 0, n - quarter * 32, reinterpret_cast<bf16*>(out + c), 2 * row_floats, lane);
+                __syncwarp();
             }
         }
         if (!ok) atomicExch(status, 5);

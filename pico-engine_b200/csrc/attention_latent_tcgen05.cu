@@ -15,7 +15,8 @@
 //
 // Rows of up to 256 entries, a multiple of 16, values of 64, 128 or 192 of them.  At 16 heads of 192 + 64 a step is 1,024 tensor-core
 // cycles for Q K^T and 768 for P V against 1,024 of the special-function units for its exponentials: the tensor core bounds it.
-// Measured on a B200, 2,048 tokens, 16 heads of 192 + 64: 44 us, where the mma.sync kernel (attention_headmix_flash.cu) takes 667.
+// Measured on a B200, 2,048 tokens, 16 heads of 192 + 64: 40 us (45 before the first loads went out ahead of the block's meeting, the mask
+// became one comparison a score, sums took two numbers at a time and rows left through shared memory), where the mma.sync kernel (attention_headmix_flash.cu) takes 667.
 // A head's gate is one number a token and commutes with the product behind this kernel: it joins the division by the row's sum.
 // Every mbarrier wait is bounded by the clock; a wait that runs out sets *status to 5, the roles leave their loops, tensor memory is
 // freed and the CTA returns (status 6: shared memory did not start on a 1024-byte boundary, nothing was done).
@@ -60,6 +61,26 @@ __global__ void __launch_bounds__(LT_THREADS, 1) attention_latent_tcgen05_kernel
         if (threadIdx.x == 0) atomicExch(status, 6);
         return;
     }
+    // (the step's description and the page table: no kernel writes them)
+    const int4 info = p.tiles[blockIdx.y];                          // heads vary fastest: the runs that see the most keys start first
+    const int brow = info.x, tok0 = info.y, n = info.z, pos0 = info.w, h = blockIdx.x;
+    const int first_key = (p.window > 0 && pos0 - p.window + 1 > 0) ? pos0 - p.window + 1 : 0;
+    const int page_lo = first_key / LT_KTILE, page_hi = (pos0 + n - 1) / LT_KTILE;
+    const int n_pages = page_hi - page_lo + 1, n_steps = (n_pages + 1) / 2;
+    const int* table = p.block_table + (size_t)brow * p.table_stride;
+    auto bring = [&](int s, const int (&page)[2]) {                  // a stage: two pages
+        const unsigned bar = at_smem(&kv_full[s]), dst = kv_s + s * STAGE;
+        stage_flags[s] = (page[0] >= 0 ? 1u : 0u) | (page[1] >= 0 ? 2u : 0u);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((unsigned)STAGE) : "memory");
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+            // a page that is not there is read from beyond the pool's end, which gives zeros: its scores are masked and its
+            // values add nothing; so are a row's entries behind its width (the queries hold the next head's there)
+            const int y = page[g] >= 0 ? page[g] * LT_KTILE : p.pool_rows;
+#pragma unroll
+            for (int c = 0; c < KP; ++c) at_tma_2d(dst + c * LT_PANEL + g * (LT_KTILE * 128), &map_k, 64 * c, y, bar);
+        }
+    };
     if (threadIdx.x == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(at_smem(&q_full)) : "memory");
         for (int q = 0; q < 4; ++q) asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;" ::"r"(at_smem(&pair_bar[q])) : "memory");
@@ -72,7 +93,14 @@ __global__ void __launch_bounds__(LT_THREADS, 1) attention_latent_tcgen05_kernel
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 8;" ::"r"(at_smem(&p_full[b])) : "memory");      // the eight softmax warps
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(at_smem(&pv_done[b])) : "memory");
         }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;\n\tfence.proxy.async.shared::cta;" ::: "memory");
+        // the queries and the first step are asked for before the block meets
+        const int first[2] = {table[page_lo], 1 < n_pages ? table[page_lo + 1] : -1};
+        pdl_wait();
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(at_smem(&q_full)), "r"((unsigned)STAGE) : "memory");
+#pragma unroll
+        for (int c = 0; c < KP; ++c) at_tma_2d(q_s + c * LT_PANEL, &map_q, h * p.width + 64 * c, tok0, at_smem(&q_full));
+        bring(0, first);
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(at_smem(&tmem_base_s)), "r"((unsigned)LT_TMEM_COLS) : "memory");
@@ -86,36 +114,16 @@ __global__ void __launch_bounds__(LT_THREADS, 1) attention_latent_tcgen05_kernel
     pdl_launch_dependents();
     pdl_wait();
 
-    const int4 info = p.tiles[blockIdx.y];                          // heads vary fastest: the runs that see the most keys start first
-    const int brow = info.x, tok0 = info.y, n = info.z, pos0 = info.w, h = blockIdx.x;
-    const int first_key = (p.window > 0 && pos0 - p.window + 1 > 0) ? pos0 - p.window + 1 : 0;
-    const int page_lo = first_key / LT_KTILE, page_hi = (pos0 + n - 1) / LT_KTILE;
-    const int n_pages = page_hi - page_lo + 1, n_steps = (n_pages + 1) / 2;
-
     if (warp == 0) {
         if (lane == 0) {                                            // ---------------- loader
-            const int* table = p.block_table + (size_t)brow * p.table_stride;
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(at_smem(&q_full)), "r"((unsigned)STAGE) : "memory");
-#pragma unroll
-            for (int c = 0; c < KP; ++c) at_tma_2d(q_s + c * LT_PANEL, &map_q, h * p.width + 64 * c, tok0, at_smem(&q_full));
-            int page[2] = {table[page_lo], 1 < n_pages ? table[page_lo + 1] : -1};
-            for (int it = 0; it < n_steps; ++it) {
+            int page[2] = {2 < n_pages ? table[page_lo + 2] : -1, 3 < n_pages ? table[page_lo + 3] : -1};
+            for (int it = 1; it < n_steps; ++it) {
                 const int s = it % LT_STAGES;
                 int next[2] = {-1, -1};                             // the step after this one: its entries travel during the wait
                 if (2 * it + 2 < n_pages) next[0] = table[page_lo + 2 * it + 2];
                 if (2 * it + 3 < n_pages) next[1] = table[page_lo + 2 * it + 3];
                 if (it >= LT_STAGES && !at_wait(at_smem(&kv_empty[s]), (unsigned)((it / LT_STAGES) - 1) & 1u)) { atomicExch(status, 5); break; }
-                const unsigned bar = at_smem(&kv_full[s]), dst = kv_s + s * STAGE;
-                stage_flags[s] = (page[0] >= 0 ? 1u : 0u) | (page[1] >= 0 ? 2u : 0u);
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((unsigned)STAGE) : "memory");
-#pragma unroll
-                for (int g = 0; g < 2; ++g) {
-                    // a page that is not there is read from beyond the pool's end, which gives zeros: its scores are masked and its
-                    // values add nothing; so are a row's entries behind its width (the queries hold the next head's there)
-                    const int y = page[g] >= 0 ? page[g] * LT_KTILE : p.pool_rows;
-#pragma unroll
-                    for (int c = 0; c < KP; ++c) at_tma_2d(dst + c * LT_PANEL + g * (LT_KTILE * 128), &map_k, 64 * c, y, bar);
-                }
+                bring(s, page);
                 page[0] = next[0]; page[1] = next[1];
             }
         }
@@ -166,6 +174,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) attention_latent_tcgen05_kernel
         const int half = p.rank / 2;
         const unsigned o_addr = lane_addr + LT_O_COL + g * half;
         const unsigned pair = at_smem(&pair_bar[quarter]);
+        const unsigned long long scale2 = at_two(p.scale_log2e, p.scale_log2e);
         float m_run = -INFINITY, l_run = 0.f;
         bool ok = true;
         int it = 0, met = 0;                                        // met: how often the row's two threads have met
@@ -198,12 +207,13 @@ __global__ void __launch_bounds__(LT_THREADS, 1) attention_latent_tcgen05_kernel
             float s[LT_KTILE];
 #pragma unroll
             for (int c = 0; c < LT_KTILE; ++c) s[c] = __uint_as_float(raw[c]);
-            if (!(there && key0 + LT_KTILE - 1 <= p_r && (p.window <= 0 || key0 > p_r - p.window))) {
+            const int hi = there ? p_r - key0 : -1;                 // the last of the page's keys that the row sees
+            if (p.window <= 0) {
+                if (hi < LT_KTILE - 1) at_mask_behind<LT_KTILE>(s, hi);
+            } else if (const int lo = p_r - p.window + 1 - key0; hi < LT_KTILE - 1 || lo > 0) {      // lo: the window's first one
 #pragma unroll
-                for (int c = 0; c < LT_KTILE; ++c) {
-                    const int key = key0 + c;
-                    if (!there || key > p_r || (p.window > 0 && key <= p_r - p.window)) s[c] = -INFINITY;
-                }
+                for (int c = 0; c < LT_KTILE; ++c)
+                    if (c > hi || c < lo) s[c] = -INFINITY;
             }
             float mx[4] = {s[0], s[1], s[2], s[3]};                 // four chains: a warp has little else to hide their latency
 #pragma unroll
@@ -220,15 +230,12 @@ __global__ void __launch_bounds__(LT_THREADS, 1) attention_latent_tcgen05_kernel
             const float m_use = m_new == -INFINITY ? 0.f : m_new;
             const float alpha = m_run == -INFINITY ? 1.0f : at_exp2(m_run - m_use);
             m_run = m_new;
-            float sum[4] = {0.f, 0.f, 0.f, 0.f};
+            unsigned long long sum[2] = {0ull, 0ull};
+            const unsigned long long off = at_two(-m_use, -m_use);
             float packed[LT_KTILE / 2];
 #pragma unroll
-            for (int c = 0; c < LT_KTILE; c += 2) {
-                const float e0 = at_exp2(fmaf(s[c], p.scale_log2e, -m_use)), e1 = at_exp2(fmaf(s[c + 1], p.scale_log2e, -m_use));
-                sum[c & 3] += e0; sum[(c + 1) & 3] += e1;
-                packed[c >> 1] = __uint_as_float(at_pack(e0, e1));
-            }
-            l_run = l_run * alpha + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
+            for (int c = 0; c < LT_KTILE; c += 2) packed[c >> 1] = __uint_as_float(at_exp2_pair(s[c], s[c + 1], scale2, off, sum[(c >> 1) & 1]));
+            l_run = l_run * alpha + at_sum_four(sum[0], sum[1]);
             at_st32(lane_addr + b * (2 * LT_KTILE) + g * (LT_KTILE / 2), packed);
             if (it > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) { // a row's reference point moved: rescale this half of the warp's rows of O
                 if (!at_wait_warp(at_smem(&pv_done[b ^ 1]), (unsigned)((it - 1) >> 1) & 1u)) { ok = false; break; }
@@ -256,17 +263,18 @@ __global__ void __launch_bounds__(LT_THREADS, 1) attention_latent_tcgen05_kernel
             const float l = g == 0 ? l_run + l_theirs : l_theirs + l_run;   // the same sum in both threads
             float inv = l > 0.f ? 1.0f / l : 0.f;
             if (p.gate && r < n) inv *= 1.0f / (1.0f + expf(-to_f(p.gate[(size_t)(tok0 + r) * p.gate_ld + h])));
-            bf16* o_row = p.out + ((size_t)(tok0 + r) * p.H + h) * p.rank + g * half;
+            // through the queries' place (the last products have read them), 32 columns at a time
+            const int row_bytes = p.rank * 2, group0 = g * (half / 8);
+            bf16* out = p.out + ((size_t)tok0 * p.H + h) * p.rank + g * half;
 #pragma unroll 1
             for (int c = 0; c < half; c += 32) {
                 float o[32];
+                unsigned packed[16];
                 at_ld32(o_addr + c, o);
-                if (r < n) {
 #pragma unroll
-                    for (int i = 0; i < 32; i += 8)
-                        *reinterpret_cast<uint4*>(o_row + c + i) = make_uint4(at_pack(o[i] * inv, o[i + 1] * inv), at_pack(o[i + 2] * inv, o[i + 3] * inv),
-                                                                              at_pack(o[i + 4] * inv, o[i + 5] * inv), at_pack(o[i + 6] * inv, o[i + 7] * inv));
-                }
+                for (int i = 0; i < 16; ++i) packed[i] = at_pack(o[2 * i] * inv, o[2 * i + 1] * inv);
+                at_put_row<32>(q_s, row_bytes, r, group0 + c / 8, packed);
+                at_store_rows<32>(q_s, row_bytes, quarter * 32, group0 + c / 8, n, out + c, (size_t)p.H * p.rank, lane);
             }
         }
         if (!ok) atomicExch(status, 5);

@@ -22,8 +22,12 @@
 // What bounds a step: its 16,384 exponentials take 1,024 cycles of the special-function units.  With all
 // eight warps on one step (two threads a row that told each other their maxima) a step was a chain of
 // 2,480 cycles (clock stamps: waits 370, maxima 430, exponentials 1,100, P through shared memory 350);
-// with the warpgroups in turn it is 1,500 (head size 64).  2,048 tokens, 14 heads of 64, on a B200: 30 us before,
-// 26 us here; 28 heads of 128, prompts of 5,001 / 1,807 / 700 / 33 tokens: 341 us before, 278 us here.
+// with the warpgroups in turn it is 1,430 (head size 64; 1,560 with 128).  Beside the steps a CTA has about 8,000 cycles: barriers, tensor
+// memory and the first loads (asked for before the block meets), the first step's chain, the end of the row.  What the softmax
+// warps do besides exponentials counts: scale and sums go two numbers at a time (fma / add .f32x2), a page's mask is one comparison
+// a score against the last key the row sees, and rows leave through shared memory (at_store_rows).  2,048 tokens, 14 heads of 64,
+// on a B200: 26.0 us with a chain of comparisons a score, single sums and rows stored by their own lanes, 21.6 us here; 28 heads of 128,
+// prompts of 5,001 / 1,807 / 700 / 33 tokens: 273 us, 237 us here.
 //
 // Values lie in the cache as [key][head size], which is the MN-major form of the B operand of
 // P.V: its shared-memory descriptor steps 8 keys by 1024 bytes and 64 columns by one panel.
@@ -89,28 +93,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_prefill_tcgen05_kerne
         return;
     }
 
-    if (threadIdx.x == 0) {
-        auto init = [](unsigned long long* bar, unsigned count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(at_smem(bar)), "r"(count) : "memory"); };
-        init(&q_full, 1);
-        for (int s = 0; s < AT_STAGES; ++s) { init(&k_full[s], 1); init(&v_full[s], 1); init(&k_empty[s], 1); init(&v_empty[s], 1); }
-        for (int b = 0; b < AT_BUFFERS; ++b) { init(&s_full[b], 1); init(&p_full[b], 4); init(&pv_done[b], 1); }     // p_full: a warpgroup's four warps
-        for (int w = 0; w < 8; ++w) init(&told[w], 1);
-        for (int q = 0; q < 4; ++q) init(&met[q], 2);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(at_smem(&tmem_base_s)), "r"((unsigned)AT_TMEM_COLS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const unsigned tmem = tmem_base_s;
-    // Only now may the next kernel of the stream be scheduled: if it came earlier, took tensor memory on this SM
-    // and then waited for this grid to end, a CTA of this grid that still had to allocate would wait for it in turn.
-    pdl_launch_dependents();
-    pdl_wait();
-
+    // (the step's description: no kernel writes it)
     const int4 info = p.tiles[blockIdx.y];                          // heads vary fastest: the runs that see the most keys start first
     const int brow = info.x, tok0 = info.y, n = info.z, pos0 = info.w;
     const int h = blockIdx.x, kvh = h / (p.nh / p.nkv);
@@ -126,35 +109,61 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_prefill_tcgen05_kerne
     const int n_pages = kept + page_hi - page_lo + 1, n_steps = (n_pages + 1) / 2;
     auto page_at = [&](int j) { return j < kept ? j : page_lo + j - kept; };     // the j-th page the run reads, j < n_pages
 
+    const int* table = p.block_table + (size_t)brow * p.table_stride;
+    auto bring = [&](const CUtensorMap* map, unsigned dst, const int (&y)[2], unsigned bar) {      // two pages' keys or values of a head
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((unsigned)AT_STAGE_BYTES / 2) : "memory");
+#pragma unroll
+        for (int g = 0; g < 2; ++g)
+#pragma unroll
+            for (int c = 0; c < AT_PANELS; ++c) at_tma_2d(dst + c * (2 * AT_KTILE * 128) + g * (AT_KTILE * 128), map, 64 * c, y[g], bar);
+    };
+    // a page that is not there (beyond the run's last page, or left behind by the window) is read from
+    // beyond the pool's end, which gives zeros: its scores are masked and its values add nothing
+    auto rows_of = [&](int page) { return page >= 0 ? (page * p.nkv + kvh) * AT_KTILE : p.pool_rows; };
+    if (threadIdx.x == 0) {
+        auto init = [](unsigned long long* bar, unsigned count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(at_smem(bar)), "r"(count) : "memory"); };
+        init(&q_full, 1);
+        for (int s = 0; s < AT_STAGES; ++s) { init(&k_full[s], 1); init(&v_full[s], 1); init(&k_empty[s], 1); init(&v_empty[s], 1); }
+        for (int b = 0; b < AT_BUFFERS; ++b) { init(&s_full[b], 1); init(&p_full[b], 4); init(&pv_done[b], 1); }     // p_full: a warpgroup's four warps
+        for (int w = 0; w < 8; ++w) init(&told[w], 1);
+        for (int q = 0; q < 4; ++q) init(&met[q], 2);
+        asm volatile("fence.mbarrier_init.release.cluster;\n\tfence.proxy.async.shared::cta;" ::: "memory");
+        // the queries and the first step are asked for before the block meets
+        const int y[2] = {rows_of(table[page_at(0)]), rows_of(1 < n_pages ? table[page_at(1)] : -1)};
+        pdl_wait();
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(at_smem(&q_full)), "r"((unsigned)AT_Q_BYTES) : "memory");
+#pragma unroll
+        for (int c = 0; c < AT_PANELS; ++c) at_tma_2d(q_s + c * (AT_QTILE * 128), &map_q, h * AT_HD + 64 * c, tok0, at_smem(&q_full));
+        bring(&map_k, kv_s, y, at_smem(&k_full[0]));
+        bring(&map_v, kv_s + AT_STAGE_BYTES / 2, y, at_smem(&v_full[0]));
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(at_smem(&tmem_base_s)), "r"((unsigned)AT_TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const unsigned tmem = tmem_base_s;
+    // Only now may the next kernel of the stream be scheduled: if it came earlier, took tensor memory on this SM
+    // and then waited for this grid to end, a CTA of this grid that still had to allocate would wait for it in turn.
+    pdl_launch_dependents();
+    pdl_wait();
+
     if (warp == 0) {
         if (lane == 0) {                                            // ---------------- loader
-            const int* table = p.block_table + (size_t)brow * p.table_stride;
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(at_smem(&q_full)), "r"((unsigned)AT_Q_BYTES) : "memory");
-#pragma unroll
-            for (int c = 0; c < AT_PANELS; ++c) at_tma_2d(q_s + c * (AT_QTILE * 128), &map_q, h * AT_HD + 64 * c, tok0, at_smem(&q_full));
-            int page[2] = {table[page_at(0)], 1 < n_pages ? table[page_at(1)] : -1};
-            for (int it = 0; it < n_steps; ++it) {
+            int page[2] = {2 < n_pages ? table[page_at(2)] : -1, 3 < n_pages ? table[page_at(3)] : -1};
+            for (int it = 1; it < n_steps; ++it) {
                 const int s = it % AT_STAGES;
                 int next[2] = {-1, -1};                             // the step after this one: its entries travel during the wait
                 if (2 * it + 2 < n_pages) next[0] = table[page_at(2 * it + 2)];
                 if (2 * it + 3 < n_pages) next[1] = table[page_at(2 * it + 3)];
                 const unsigned k_dst = kv_s + s * AT_STAGE_BYTES, v_dst = k_dst + AT_STAGE_BYTES / 2, round = (unsigned)((it / AT_STAGES) - 1) & 1u;
-                // a page that is not there (beyond the run's last page, or left behind by the window) is read from
-                // beyond the pool's end, which gives zeros: its scores are masked and its values add nothing
-                int y[2];
-#pragma unroll
-                for (int g = 0; g < 2; ++g) y[g] = page[g] >= 0 ? (page[g] * p.nkv + kvh) * AT_KTILE : p.pool_rows;
-                auto bring = [&](const CUtensorMap* map, unsigned dst, unsigned bar) {
-                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((unsigned)AT_STAGE_BYTES / 2) : "memory");
-#pragma unroll
-                    for (int g = 0; g < 2; ++g)
-#pragma unroll
-                        for (int c = 0; c < AT_PANELS; ++c) at_tma_2d(dst + c * (2 * AT_KTILE * 128) + g * (AT_KTILE * 128), map, 64 * c, y[g], bar);
-                };
+                const int y[2] = {rows_of(page[0]), rows_of(page[1])};
                 if (it >= AT_STAGES && !at_wait(at_smem(&k_empty[s]), round)) { atomicExch(status, 5); break; }
-                bring(&map_k, k_dst, at_smem(&k_full[s]));
+                bring(&map_k, k_dst, y, at_smem(&k_full[s]));
                 if (it >= AT_STAGES && !at_wait(at_smem(&v_empty[s]), round)) { atomicExch(status, 5); break; }
-                bring(&map_v, v_dst, at_smem(&v_full[s]));
+                bring(&map_v, v_dst, y, at_smem(&v_full[s]));
                 page[0] = next[0]; page[1] = next[1];
             }
         }
@@ -205,8 +214,8 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_prefill_tcgen05_kerne
         const int r = quarter * 32 + lane;                          // this thread's query row
         const int p_r = pos0 + r;
         const unsigned lane_addr = tmem + ((unsigned)(quarter * 32) << 16);
-        const int* table = p.block_table + (size_t)brow * p.table_stride;
         const float slope = p.slopes ? p.slopes[h] * p.inv_scale : 0.f;     // in units of the unscaled score
+        const unsigned long long scale2 = at_two(p.scale_log2e, p.scale_log2e);
         float m_mine = -INFINITY, l_mine = 0.f;                     // the reference point of this group's last step; its share of the row's sum
         bool ok = true;
         int entry[2];                                               // the page table's entries of the next step of this group
@@ -239,12 +248,14 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_prefill_tcgen05_kerne
             for (int x = 0; x < 2; ++x) {
                 const int key0 = page_at(2 * it + x) * AT_KTILE;
                 float* sx = s + x * AT_KTILE;
-                if (!(there[x] && key0 + AT_KTILE - 1 <= p_r && (p.window <= 0 || key0 > p_r - p.window || key0 + AT_KTILE - 1 < p.keep_first))) {
+                const int hi = there[x] ? p_r - key0 : -1;          // the last of the page's keys that the row sees
+                if (p.window <= 0) {
+                    if (hi < AT_KTILE - 1) at_mask_behind<AT_KTILE>(sx, hi);
+                } else if (hi < AT_KTILE - 1 || (key0 <= p_r - p.window && key0 + AT_KTILE - 1 >= p.keep_first)) {
+                    const int lo = p_r - p.window + 1 - key0, kept_here = p.keep_first - key0;      // the window's first one, and how many are kept
 #pragma unroll
-                    for (int c = 0; c < AT_KTILE; ++c) {
-                        const int key = key0 + c;
-                        if (!there[x] || key > p_r || (p.window > 0 && key <= p_r - p.window && key >= p.keep_first)) sx[c] = -INFINITY;
-                    }
+                    for (int c = 0; c < AT_KTILE; ++c)
+                        if (c > hi || (c < lo && c >= kept_here)) sx[c] = -INFINITY;
                 }
                 // the distance's share of the score, slope * (key - row): the part that grows along the page is added here, the
                 // page's own part (`base`, one number a page) joins the maximum and the exponent's offset
@@ -283,20 +294,16 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_prefill_tcgen05_kerne
             const float alpha = m_run == -INFINITY ? 1.0f : at_exp2(m_run - m_use);          // for O
             l_mine *= m_mine == -INFINITY ? 1.0f : at_exp2(m_mine - m_use);                  // (no sum yet: it is zero)
             m_mine = m_new;
-            float sum[4] = {0.f, 0.f, 0.f, 0.f};
+            unsigned long long sum[2] = {0ull, 0ull};
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
                 float packed[AT_KTILE / 2];
                 const float off = fmaf(base[x], p.scale_log2e, -m_use);
 #pragma unroll
-                for (int c = 0; c < AT_KTILE; c += 2) {
-                    const float e0 = at_exp2(fmaf(s[x * AT_KTILE + c], p.scale_log2e, off)), e1 = at_exp2(fmaf(s[x * AT_KTILE + c + 1], p.scale_log2e, off));
-                    sum[c & 3] += e0; sum[(c + 1) & 3] += e1;
-                    packed[c >> 1] = __uint_as_float(at_pack(e0, e1));
-                }
+                for (int c = 0; c < AT_KTILE; c += 2) packed[c >> 1] = __uint_as_float(at_exp2_pair(s[x * AT_KTILE + c], s[x * AT_KTILE + c + 1], scale2, at_two(off, off), sum[(c >> 1) & 1]));
                 at_st32(s_addr + x * (AT_KTILE / 2), packed);       // P over the scores, two keys a column
             }
-            l_mine += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+            l_mine += at_sum_four(sum[0], sum[1]);
             if (it > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) { // a row's reference point moved: rescale the warp's rows of O
                 if (!at_wait_warp(at_smem(&pv_done[(it - 1) % AT_BUFFERS]), (unsigned)((it - 1) / AT_BUFFERS) & 1u)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -333,19 +340,19 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_prefill_tcgen05_kerne
             }
             if (p.sinks) l += at_exp2(fmaf(p.sinks[h], 1.4426950408889634f, -m_run));   // (a row that saw no key: 2^inf, and 1 / l = 0)
             const float inv = l > 0.f ? 1.0f / l : 0.f;
+            // through the queries' place: the last products have read them
             const unsigned o_addr = lane_addr + AT_O_COL + g * (AT_HD / 2);
-            bf16* o_row = p.out + ((size_t)(tok0 + r) * p.nh + h) * AT_HD + g * (AT_HD / 2);
-#pragma unroll 1
+            constexpr int GROUPS = AT_HD / 16;                      // 16-byte groups of a warpgroup's half of a row
+#pragma unroll
             for (int c = 0; c < AT_HD / 2; c += 32) {
                 float o[32];
+                unsigned packed[16];
                 at_ld32(o_addr + c, o);
-                if (r < n) {
 #pragma unroll
-                    for (int i = 0; i < 32; i += 8)
-                        *reinterpret_cast<uint4*>(o_row + c + i) = make_uint4(at_pack(o[i] * inv, o[i + 1] * inv), at_pack(o[i + 2] * inv, o[i + 3] * inv),
-                                                                              at_pack(o[i + 4] * inv, o[i + 5] * inv), at_pack(o[i + 6] * inv, o[i + 7] * inv));
-                }
+                for (int i = 0; i < 16; ++i) packed[i] = at_pack(o[2 * i] * inv, o[2 * i + 1] * inv);
+                at_put_row<32>(q_s, AT_HD * 2, r, g * GROUPS + c / 8, packed);
             }
+            at_store_rows<AT_HD / 2>(q_s, AT_HD * 2, quarter * 32, g * GROUPS, n, p.out + ((size_t)tok0 * p.nh + h) * AT_HD + g * (AT_HD / 2), (size_t)p.nh * AT_HD, lane);
         }
         if (!ok) atomicExch(status, 5);
     }

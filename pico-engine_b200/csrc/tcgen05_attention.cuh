@@ -118,6 +118,59 @@ __device__ __forceinline__ unsigned at_pack(float lo, float hi) {
     return *reinterpret_cast<unsigned*>(&v);
 }
 
+// Two numbers for the multiply-adds that take two at a time (each half rounds as a plain one does).
+__device__ __forceinline__ unsigned long long at_two(float a, float b) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 at_both(unsigned long long v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+// 2^(a * scale + off) and 2^(b * scale + off) as two bfloat16 numbers, and both (unrounded) into `sum`
+__device__ __forceinline__ unsigned at_exp2_pair(float a, float b, unsigned long long scale, unsigned long long off, unsigned long long& sum) {
+    unsigned long long x = at_two(a, b);
+    asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(x) : "l"(scale), "l"(off));
+    const float2 v = at_both(x);
+    const float e0 = at_exp2(v.x), e1 = at_exp2(v.y);
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum) : "l"(at_two(e0, e1)));
+    return at_pack(e0, e1);
+}
+__device__ __forceinline__ float at_sum_four(unsigned long long a, unsigned long long b) {
+    const float2 x = at_both(a), y = at_both(b);
+    return (x.x + x.y) + (y.x + y.y);
+}
+// COLS bfloat16 columns of 32 rows (a row a lane, `packed` pairs) to global memory through shared memory: `tile` holds rows of `row_bytes` (128 or
+// more), this warp's from `row0` on, its columns from 16-byte group `group0` on; groups are exchanged by the row inside a run of eight.  A lane
+// storing its own row touched 32 lines an instruction: 3,700 cycles for 128 columns of eight warps, 700 here.
+template <int COLS>
+__device__ __forceinline__ void at_put_row(unsigned tile, int row_bytes, int row, int group0, const unsigned* packed) {
+#pragma unroll
+    for (int j = 0; j < COLS / 8; ++j)
+        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(tile + row * row_bytes + (((group0 + j) ^ (row & 7)) << 4)), "r"(packed[4 * j]), "r"(packed[4 * j + 1]),
+                     "r"(packed[4 * j + 2]), "r"(packed[4 * j + 3]) : "memory");
+}
+template <int COLS>
+__device__ __forceinline__ void at_store_rows(unsigned tile, int row_bytes, int row0, int group0, int rows, bf16* out, size_t stride, int lane, int cols = COLS) {
+    constexpr int LANES = COLS / 8, ROWS = 32 / LANES;     // lanes a row, rows at a time
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 32; i += ROWS) {
+        const int row = row0 + i + lane / LANES, j = lane % LANES;
+        uint4 v;
+        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(tile + row * row_bytes + (((group0 + j) ^ (row & 7)) << 4)) : "memory");
+        if (row < rows && j * 8 < cols) *reinterpret_cast<uint4*>(out + (size_t)row * stride + j * 8) = v;
+    }
+}
+// scores behind the last one a row sees do not count
+template <int N>
+__device__ __forceinline__ void at_mask_behind(float* s, int last) {
+#pragma unroll
+    for (int c = 0; c < N; ++c) s[c] = c <= last ? s[c] : -INFINITY;
+}
+
 // ---------------------------------------------------------------- host side
 namespace {
 
