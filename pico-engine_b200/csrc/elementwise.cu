@@ -116,69 +116,103 @@ __device__ __forceinline__ float4 load4_as_f(const bf16* p) {
     return make_float4(lo.x, lo.y, hi.x, hi.y);
 }
 
-// With ADD the row of y is first added to the row of x, which is written back: the residual sum
-// that precedes the norm, in the same pass.  A thread keeps up to RN_KEEP groups of four elements in
-// registers between the two passes and fetches their weights before the block-wide sum, so that
-// the sum's latency hides the fetch; longer rows are read again.
-#define RN_KEEP 4
+// Four weights; `whole`: they start on an 8-byte (bfloat16) or 16-byte boundary.
+__device__ __forceinline__ float4 rn_weights(const void* w, int w_dtype, int i, bool whole) {
+    if (!whole) return make_float4(load_as_f(w, w_dtype, i), load_as_f(w, w_dtype, i + 1), load_as_f(w, w_dtype, i + 2), load_as_f(w, w_dtype, i + 3));
+    return w_dtype == PE_BF16 ? load4_as_f((const bf16*)w + i) : load4_as_f((const float*)w + i);
+}
 
-template <typename TO, typename TY, bool ADD>
-__global__ void rmsnorm_kernel(float* x, const TY* y, const int* rows_index,
-                               const void* w, int w_dtype, float eps, TO* out, int H) {
-    pdl_launch_dependents();
-    pdl_wait();
-    __shared__ float scratch[33];
-    const int r = blockIdx.x;
-    const size_t src = rows_index ? rows_index[r] : r;
-    float* xr = x + src * H;
-    TO* o = out + (size_t)r * H;
-    float ss = 0.f;
-    if ((H & 3) == 0) {                                       // rows start on 16-byte boundaries
-        float4* x4 = reinterpret_cast<float4*>(xr);
-        const int n4 = H / 4;
-        float4 v[RN_KEEP], wv[RN_KEEP];
+// Up to KEEP groups of four elements of a row, `step` groups apart from group `i0` on: four groups' loads go out together (x is written back
+// in the same pass: a load behind a store that might touch its place would wait for that store's own operands), then, with ADD, the
+// sums x + y go back to x.  Returns the squares' sum.
+template <int KEEP, typename TY, bool ADD>
+__device__ __forceinline__ float rn_take(float4* x4, const TY* y, int i0, int step, int n4, float4* v, float ss) {
+    if constexpr (KEEP > 4) {
+        return rn_take<KEEP - 4, TY, ADD>(x4, y, i0 + 4 * step, step, n4, v + 4, rn_take<4, TY, ADD>(x4, y, i0, step, n4, v, ss));
+    } else {
+        float4 a[KEEP];
 #pragma unroll
-        for (int k = 0; k < RN_KEEP; ++k) {
-            const int i = threadIdx.x + k * blockDim.x;
+        for (int k = 0; k < KEEP; ++k) {
+            const int i = i0 + k * step;
             if (i < n4) {
                 v[k] = x4[i];
+                if (ADD) a[k] = load4_as_f(y + 4 * i);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k) {
+            const int i = i0 + k * step;
+            if (i < n4) {
                 if (ADD) {
-                    const float4 a = load4_as_f(y + src * H + 4 * i);
-                    v[k].x += a.x; v[k].y += a.y; v[k].z += a.z; v[k].w += a.w;
+                    v[k].x += a[k].x; v[k].y += a[k].y; v[k].z += a[k].z; v[k].w += a[k].w;
                     x4[i] = v[k];
                 }
                 ss = fmaf(v[k].x, v[k].x, ss); ss = fmaf(v[k].y, v[k].y, ss); ss = fmaf(v[k].z, v[k].z, ss); ss = fmaf(v[k].w, v[k].w, ss);
             }
         }
-        for (int i = threadIdx.x + RN_KEEP * blockDim.x; i < n4; i += blockDim.x) {
-            float4 u = x4[i];
-            if (ADD) {
-                const float4 a = load4_as_f(y + src * H + 4 * i);
-                u.x += a.x; u.y += a.y; u.z += a.z; u.w += a.w;
-                x4[i] = u;
-            }
-            ss = fmaf(u.x, u.x, ss); ss = fmaf(u.y, u.y, ss); ss = fmaf(u.z, u.z, ss); ss = fmaf(u.w, u.w, ss);
-        }
+        return ss;
+    }
+}
+
+// With ADD the row of y is first added to the row of x, which is written back: the residual sum
+// that precedes the norm, in the same pass.  A thread keeps up to KEEP groups of four elements in
+// registers between the two passes; longer rows are read again.  Weights are fetched while the kernel before still runs (WB: bfloat16 on an
+// 8-byte boundary, two registers for four of them), or, where that would take registers from the blocks beside this one, before the block meets.
+template <typename TO, typename TY, bool ADD, int KEEP, bool WB>
+__global__ void __launch_bounds__(512, 2) rmsnorm_kernel(float* x, const TY* y, const int* rows_index,
+                                                         const void* w, int w_dtype, float eps, TO* out, int H) {
+    pdl_launch_dependents();
+    __shared__ float scratch[33];
+    const int r = blockIdx.x;
+    TO* o = out + (size_t)r * H;
+    if ((H & 3) == 0) {                                       // rows start on 16-byte boundaries
+        const int n4 = H / 4;
+        const bool whole = ((uintptr_t)w & (w_dtype == PE_BF16 ? 7 : 15)) == 0;
+        float4 v[KEEP], wv[KEEP];
+        uint2 wr[KEEP];
+        auto weights = [&]() {
 #pragma unroll
-        for (int k = 0; k < RN_KEEP; ++k) {
-            const int i = threadIdx.x + k * blockDim.x;
-            if (i < n4) wv[k] = make_float4(load_as_f(w, w_dtype, 4 * i), load_as_f(w, w_dtype, 4 * i + 1),
-                                            load_as_f(w, w_dtype, 4 * i + 2), load_as_f(w, w_dtype, 4 * i + 3));
+            for (int k = 0; k < KEEP; ++k) {
+                const int i = threadIdx.x + k * blockDim.x;
+                if (i >= n4) continue;
+                if (WB) wr[k] = *reinterpret_cast<const uint2*>((const bf16*)w + 4 * i);
+                else wv[k] = rn_weights(w, w_dtype, 4 * i, whole);
+            }
+        };
+        constexpr bool early = WB || KEEP <= 2 || !ADD;
+        if (early) weights();
+        pdl_wait();
+        const size_t src = rows_index ? rows_index[r] : r;
+        float4* x4 = reinterpret_cast<float4*>(x + src * H);
+        float ss = rn_take<KEEP, TY, ADD>(x4, y + src * H, threadIdx.x, blockDim.x, n4, v, 0.f);
+        for (int i = threadIdx.x + KEEP * blockDim.x; i < n4; i += blockDim.x) {
+            float4 u[1];
+            ss = rn_take<1, TY, ADD>(x4, y + src * H, i, 1, n4, u, ss);
         }
-        ss = block_sum(ss, scratch);
+        ss = warp_sum(ss);                                    // one meeting: every thread adds the warps' sums itself
+        if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = ss;
+        if (!early) weights();
+        __syncthreads();
+        ss = scratch[0];
+        for (int i = 1; i < (int)(blockDim.x >> 5); ++i) ss += scratch[i];
         const float rstd = 1.0f / sqrtf(ss / (float)H + eps);
 #pragma unroll
-        for (int k = 0; k < RN_KEEP; ++k) {
+        for (int k = 0; k < KEEP; ++k) {
             const int i = threadIdx.x + k * blockDim.x;
-            if (i < n4) store4(o + 4 * i, v[k].x * rstd * wv[k].x, v[k].y * rstd * wv[k].y, v[k].z * rstd * wv[k].z, v[k].w * rstd * wv[k].w);
+            if (i >= n4) continue;
+            const float4 g = WB ? load4_as_f(reinterpret_cast<const bf16*>(&wr[k])) : wv[k];
+            store4(o + 4 * i, v[k].x * rstd * g.x, v[k].y * rstd * g.y, v[k].z * rstd * g.z, v[k].w * rstd * g.w);
         }
-        for (int i = threadIdx.x + RN_KEEP * blockDim.x; i < n4; i += blockDim.x) {
-            const float4 u = x4[i];                           // this thread wrote it, if anyone did
-            store4(o + 4 * i, u.x * rstd * load_as_f(w, w_dtype, 4 * i), u.y * rstd * load_as_f(w, w_dtype, 4 * i + 1),
-                   u.z * rstd * load_as_f(w, w_dtype, 4 * i + 2), u.w * rstd * load_as_f(w, w_dtype, 4 * i + 3));
+        for (int i = threadIdx.x + KEEP * blockDim.x; i < n4; i += blockDim.x) {
+            const float4 u = x4[i], g = rn_weights(w, w_dtype, 4 * i, whole);      // this thread wrote it, if anyone did
+            store4(o + 4 * i, u.x * rstd * g.x, u.y * rstd * g.y, u.z * rstd * g.z, u.w * rstd * g.w);
         }
         return;
     }
+    pdl_wait();
+    const size_t src = rows_index ? rows_index[r] : r;
+    float* xr = x + src * H;
+    float ss = 0.f;
     for (int i = threadIdx.x; i < H; i += blockDim.x) {
         float u = xr[i];
         if (ADD) { u += to_f(y[src * H + i]); xr[i] = u; }
@@ -189,78 +223,61 @@ __global__ void rmsnorm_kernel(float* x, const TY* y, const int* rows_index,
     for (int i = threadIdx.x; i < H; i += blockDim.x) o[i] = from_f<TO>(xr[i] * rstd * load_as_f(w, w_dtype, i));
 }
 
-// The same for many rows: a warp to a row, eight rows to a block, so that a step of thousands of rows is a few hundred
-// blocks that never wait at a block-wide barrier (the sum of a row's squares is a warp's shuffle).  A lane keeps up
-// to RW_KEEP groups of four elements between the two passes; a longer row is read again (from L2).
-#define RW_KEEP 8
+// The same for many rows of up to 1,024 elements (128 * KEEP): a warp to a row, eight rows to a block, so that a step of thousands of rows is a
+// few hundred blocks that never wait at a block-wide barrier (the sum of a row's squares is a warp's shuffle).
 #define RW_WARPS 8
 
-template <typename TO, typename TY, bool ADD>
-__global__ void __launch_bounds__(32 * RW_WARPS) rmsnorm_rows_kernel(float* x, const TY* y, const void* w, int w_dtype, float eps,
-                                                                     TO* out, int rows, int H) {
+template <typename TO, typename TY, bool ADD, int KEEP>
+__global__ void __launch_bounds__(32 * RW_WARPS, 4) rmsnorm_rows_kernel(float* x, const TY* y, const void* w, int w_dtype, float eps,
+                                                                        TO* out, int rows, int H) {
     pdl_launch_dependents();
     pdl_wait();
     const int lane = threadIdx.x & 31, r = blockIdx.x * RW_WARPS + (threadIdx.x >> 5);
     if (r >= rows) return;
-    float4* x4 = reinterpret_cast<float4*>(x + (size_t)r * H);
     TO* o = out + (size_t)r * H;
     const int n4 = H / 4;
-    float4 v[RW_KEEP];
-    float ss = 0.f;
-#pragma unroll
-    for (int k = 0; k < RW_KEEP; ++k) {
-        const int i = lane + 32 * k;
-        if (i < n4) {
-            v[k] = x4[i];
-            if (ADD) {
-                const float4 a = load4_as_f(y + (size_t)r * H + 4 * i);
-                v[k].x += a.x; v[k].y += a.y; v[k].z += a.z; v[k].w += a.w;
-                x4[i] = v[k];
-            }
-            ss = fmaf(v[k].x, v[k].x, ss); ss = fmaf(v[k].y, v[k].y, ss); ss = fmaf(v[k].z, v[k].z, ss); ss = fmaf(v[k].w, v[k].w, ss);
-        }
-    }
-    for (int i = lane + 32 * RW_KEEP; i < n4; i += 32) {
-        float4 u = x4[i];
-        if (ADD) {
-            const float4 a = load4_as_f(y + (size_t)r * H + 4 * i);
-            u.x += a.x; u.y += a.y; u.z += a.z; u.w += a.w;
-            x4[i] = u;
-        }
-        ss = fmaf(u.x, u.x, ss); ss = fmaf(u.y, u.y, ss); ss = fmaf(u.z, u.z, ss); ss = fmaf(u.w, u.w, ss);
-    }
-    ss = warp_sum(ss);
+    const bool whole = ((uintptr_t)w & (w_dtype == PE_BF16 ? 7 : 15)) == 0;
+    float4 v[KEEP];
+    const float ss = warp_sum(rn_take<KEEP, TY, ADD>(reinterpret_cast<float4*>(x + (size_t)r * H), y + (size_t)r * H, lane, 32, n4, v, 0.f));
     const float rstd = 1.0f / sqrtf(ss / (float)H + eps);
 #pragma unroll
-    for (int k = 0; k < RW_KEEP; ++k) {
+    for (int k = 0; k < KEEP; ++k) {
         const int i = lane + 32 * k;
-        if (i < n4) store4(o + 4 * i, v[k].x * rstd * load_as_f(w, w_dtype, 4 * i), v[k].y * rstd * load_as_f(w, w_dtype, 4 * i + 1),
-                           v[k].z * rstd * load_as_f(w, w_dtype, 4 * i + 2), v[k].w * rstd * load_as_f(w, w_dtype, 4 * i + 3));
-    }
-    for (int i = lane + 32 * RW_KEEP; i < n4; i += 32) {
-        const float4 u = x4[i];                               // this lane wrote it, if anyone did
-        store4(o + 4 * i, u.x * rstd * load_as_f(w, w_dtype, 4 * i), u.y * rstd * load_as_f(w, w_dtype, 4 * i + 1),
-               u.z * rstd * load_as_f(w, w_dtype, 4 * i + 2), u.w * rstd * load_as_f(w, w_dtype, 4 * i + 3));
+        if (i < n4) {
+            const float4 g = rn_weights(w, w_dtype, 4 * i, whole);
+            store4(o + 4 * i, v[k].x * rstd * g.x, v[k].y * rstd * g.y, v[k].z * rstd * g.z, v[k].w * rstd * g.w);
+        }
     }
 }
 
 template <typename TY, bool ADD>
 static int rmsnorm_launch(float* x, const TY* y, const int* rows_index, const void* w, int w_dtype, float eps, void* out,
                           int out_dtype, int rows, int H, cudaStream_t s) {
-    // many whole rows: a warp a row.  Measured inside a graph at 896 columns: level with a block a row at 2,048 rows
-    // (3.7 against 4.2 us, with the residual sum 6.0 against 5.3 us), ahead at 8,192 (10.0 against 12.6, 17.5 against 19.2 us)
-    if (!rows_index && rows >= 4096 && (H & 3) == 0 && H <= 8192) {
-        const int blocks = (rows + RW_WARPS - 1) / RW_WARPS;
-        if (out_dtype == PE_F32) PE_TRY(pe_launch(rmsnorm_rows_kernel<float, TY, ADD>, blocks, 32 * RW_WARPS, 0, s, x, y, w, w_dtype, eps, (float*)out, rows, H));
-        else if (out_dtype == PE_BF16) PE_TRY(pe_launch(rmsnorm_rows_kernel<bf16, TY, ADD>, blocks, 32 * RW_WARPS, 0, s, x, y, w, w_dtype, eps, (bf16*)out, rows, H));
-        else return PE_ERR_UNSUPPORTED;
-        PE_LAUNCH_CHECK();
+    // All loads of a thread go out before its first store and one block-wide meeting is left of three: inside a graph, bfloat16 y, before and
+    // now, us with / without the residual sum: 1 row of 896 2.2 / 1.8 and 1.3 / 1.1; 2,048 rows of 896 5.3 / 4.2 and 3.7 / 3.1; 7,541 rows of
+    // 3,584 71 / 42 (a warp a row, read twice) and 52 / 29, 6.3 TB/s.
+    // Many rows of up to 1,024 columns: a warp a row.  4,096 rows against 4,095 in blocks: 64 columns 2.0 against 4.7, 896 columns without
+    // the sum 3.4 against 5.4, with it level (7.5, 7.2).  Wider rows stay in blocks: 7,541 of 2,048 columns 29 against 39 a warp a row.
+    // Two groups of four a thread up to 1,024 columns, four beyond: 7,541 rows of 3,584 52 / 29 against 62 / 50 with two.
+    // Four groups' weights ahead of the wait cost residency: with the sum, 1 row of 3,584 1.9 against 2.2, 2,048 rows 17.3 against 16.2.
+    auto run = [&](auto* o) -> int {
+        using TO = std::remove_pointer_t<decltype(o)>;
+        if (!rows_index && rows >= 4096 && (H & 3) == 0 && H <= 1024) {
+            const int blocks = (rows + RW_WARPS - 1) / RW_WARPS;
+            if (H <= 256) PE_TRY(pe_launch(rmsnorm_rows_kernel<TO, TY, ADD, 2>, blocks, 32 * RW_WARPS, 0, s, x, y, w, w_dtype, eps, o, rows, H));
+            else PE_TRY(pe_launch(rmsnorm_rows_kernel<TO, TY, ADD, 8>, blocks, 32 * RW_WARPS, 0, s, x, y, w, w_dtype, eps, o, rows, H));
+            return 0;
+        }
+        const int keep = H <= 1024 ? 2 : 4;
+        const int threads = H >= 8192 ? 512 : H <= 512 ? 64 : (H + 128 * keep - 1) / (128 * keep) * 32;
+        const bool wb = w_dtype == PE_BF16 && ((uintptr_t)w & 7) == 0 && (keep == 2 || !ADD || rows < 1024);
+        auto* kernel = keep == 2 ? (wb ? rmsnorm_kernel<TO, TY, ADD, 2, true> : rmsnorm_kernel<TO, TY, ADD, 2, false>)
+                                 : (wb ? rmsnorm_kernel<TO, TY, ADD, 4, true> : rmsnorm_kernel<TO, TY, ADD, 4, false>);
+        PE_TRY(pe_launch(kernel, rows, threads, 0, s, x, y, rows_index, w, w_dtype, eps, o, H));
         return 0;
-    }
-    const int threads = H >= 4096 ? 512 : (H >= 1024 ? 256 : 128);
-    if (out_dtype == PE_F32) PE_TRY(pe_launch(rmsnorm_kernel<float, TY, ADD>, rows, threads, 0, s, x, y, rows_index, w, w_dtype, eps, (float*)out, H));
-    else if (out_dtype == PE_BF16) PE_TRY(pe_launch(rmsnorm_kernel<bf16, TY, ADD>, rows, threads, 0, s, x, y, rows_index, w, w_dtype, eps, (bf16*)out, H));
-    else return PE_ERR_UNSUPPORTED;
+    };
+    const int rc = out_dtype == PE_F32 ? run((float*)out) : out_dtype == PE_BF16 ? run((bf16*)out) : PE_ERR_UNSUPPORTED;
+    if (rc) return rc;
     PE_LAUNCH_CHECK();
     return 0;
 }

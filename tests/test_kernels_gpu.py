@@ -84,6 +84,27 @@ def test_rmsnorm_of_many_rows(K, H, rows):
     assert torch.allclose(got.float().cpu(), plain.rms_norm(x + y, w, 1e-6), atol=2e-2, rtol=2e-2)
 
 
+@pytest.mark.parametrize("H", [4, 256, 260, 512, 516, 1024, 1028, 3584, 4100, 8188, 8192, 12004])
+@pytest.mark.parametrize("rows,shift", [(3, 0), (3, 1), (4099, 0), (4099, 3)])
+def test_rmsnorm_at_the_edges_of_its_shapes(K, H, rows, shift):
+    """At the column counts where a thread's groups, the block's size or the kernel change, and with weights off the boundary that four of them
+    are read from, against float64: a thread adds up to 24 squares, then 5 shuffles and up to 16 warps' sums, which the root halves;
+    four more roundings make the result (2^-24 each, all with one sign at worst)."""
+    if rows > 1000 and H > 4100:
+        pytest.skip("the same kernels as with few rows")
+    x, y = rnd(rows, H, seed=1, scale=3.0), bf(rnd(rows, H, seed=4))
+    for wdtype in ("f32", "bf16"):
+        w = bf(1 + rnd(H + shift, seed=2) * 0.1)
+        wd = dev(w.to(DT[wdtype]))[shift:]
+        for with_y in (False, True):
+            total = x + y if with_y else x                       # one addition in float32: the kernel's is the same
+            want = total.double() / (total.double().pow(2).mean(-1, keepdim=True) + 1e-6).sqrt() * w[shift:].double()
+            xd = dev(x.clone())
+            got = K.add_rmsnorm(xd, dev(y.to(torch.bfloat16)), wd, 1e-6, torch.float32) if with_y else K.rmsnorm(xd, wd, 1e-6, torch.float32)
+            assert torch.equal(xd.cpu(), total)
+            assert ((got.double().cpu() - want).abs() <= (45 / 2 + 4) * 2.0 ** -24 * want.abs()).all()
+
+
 def test_rmsnorm_eps_matters(K):
     x, w = torch.full((1, 64), 1e-3), torch.ones(64)
     for eps in (1e-6, 1e-2):
