@@ -178,7 +178,7 @@ extern "C" long long pe_state_space_elems(int H, int P, int N) {
 // full (64 heads of 64 columns, 128 state rows: 125 chunks, 8,000 blocks a launch), and batches of prompts need no more scratch than it.
 #define SS_SCRATCH_FLOATS (64ll << 20)
 extern "C" int pe_state_space_chunks(int T, int B) { return (T + SS_CHUNK - 1) / SS_CHUNK + B; }
-static long long ss_chunk_floats(int H, int P, int N, int G) { return (long long)G * SS_CHUNK * SS_CHUNK + (long long)H * P * N + H; }
+static long long ss_chunk_floats(int H, int P, int N, int G) { return (long long)G * SS_CHUNK * SS_CHUNK + (long long)H * (P * N + SS_STEP_FLOATS + 1) + 4; }
 static int ss_slab(int chunks, int H, int P, int N, int G) {
     const long long floats = ss_chunk_floats(H, P, N, G), most = floats >= SS_SCRATCH_FLOATS ? 1 : SS_SCRATCH_FLOATS / floats;
     const long long slabs = (chunks + most - 1) / most;
@@ -284,13 +284,15 @@ extern "C" int pe_state_space_scan(const float* xbc, int xbc_ld, const void* pro
     if (PT > P) PT = P;
     int threads = ((PT * NS + 31) / 32) * 32;
     ScanArgs a = {xbc, xbc_ld, proj, proj_ld, dt_off, dt_bias, dtb_dtype, a_log, al_dtype, d_skip, d_dtype, state, state_stride,
-                  row_first, row_lens, slots, y, B, H, P, N, G, NS, NR, NRP, PT, nullptr, nullptr, nullptr, 0, 0, 0};
+                  row_first, row_lens, slots, y, B, H, P, N, G, NS, NR, NRP, PT, nullptr, nullptr, nullptr, nullptr, nullptr, 0, 0, 0};
     if (dtype != PE_F32 && dtype != PE_BF16) return PE_ERR_UNSUPPORTED;
     if (chunked) {
         a.chunks = pe_state_space_chunks(T, B);
         a.slab = ss_slab(a.chunks, H, P, N, G);
-        a.chunk_scores = scratch;
-        a.chunk_state = scratch + (size_t)a.slab * G * SS_CHUNK * SS_CHUNK;
+        a.chunk_steps = scratch;                                  // (64-bit entries and vectors first; four floats for a chunk's place)
+        a.chunk_rows = reinterpret_cast<int2*>(scratch + (size_t)a.slab * H * SS_STEP_FLOATS);
+        a.chunk_scores = scratch + (size_t)a.slab * (H * SS_STEP_FLOATS + 4);
+        a.chunk_state = a.chunk_scores + (size_t)a.slab * G * SS_CHUNK * SS_CHUNK;
         a.chunk_decay = a.chunk_state + (size_t)a.slab * H * P * N;
         return ss_tiles(a, dtype, (cudaStream_t)stream);
     }

@@ -4,6 +4,8 @@
 
 #define SS_CHUNK 64          // tokens of a chunk of a prompt
 
+#define SS_STEP_FLOATS (4 * 64)               // of a chunk of 64 tokens and a head
+
 struct ScanArgs {
     const float* xbc; int xbc_ld;             // [T, inner + 2 G N] float32: x | B | C after the convolution
     const void* proj; int proj_ld, dt_off;    // dt_raw at columns dt_off .. dt_off + H - 1 of proj (the step's dtype)
@@ -15,6 +17,8 @@ struct ScanArgs {
     float* chunk_state;                       // [chunks][H][N][P]: a chunk's own contribution, then its incoming state
     float* chunk_decay;                       // [chunks][H]: the product of a chunk's decays
     float* chunk_scores;                      // [chunks][G][64 s][64 t]: C_t . B_s
+    float* chunk_steps;                       // [chunks][H][SS_STEP_FLOATS]: 64 x (dt, dt * the decays behind it), then 64 running sums (float64)
+    int2* chunk_rows;                         // [chunks]: first packed token and number of tokens
     int chunks;                               // of the step, at most
     int first_chunk, slab;                    // those that a launch takes: from first_chunk on, `slab` of them at most
 };

@@ -9,8 +9,8 @@
 //
 // Bound by float32 multiply-adds (fma.rn.f32x2: two an instruction, each half rounds as a plain one does).  Decays between two tokens
 // are exp of the difference of running sums of -exp(A_log) dt in float64, which costs no digits however long the chunk's sum.
-// Measured on a B200, 64 heads of 64 columns, 128 state rows, rows of 1,400 and 647 tokens: 1,028 us as a walk, 195 us here
-// (contributions 70, carry 32, outputs 93: 28 float32 TFLOP/s).
+// Measured on a B200, 64 heads of 64 columns, 128 state rows, rows of 1,400 and 647 tokens: 1,028 us as a walk, 190 us here (steps 3.5,
+// contributions 61, 70 before the steps had a launch of their own, carry 32, outputs 94: 28 float32 TFLOP/s).
 #include "state_space.cuh"
 #include "chunk_tiles.cuh"
 
@@ -24,39 +24,47 @@ __device__ __forceinline__ void st_find_chunk(const ScanArgs& a, int c, int& fir
     }
 }
 
-// The chunk's step sizes dts[64] and running sums las[64] of -exp(A_log) dt (zero steps behind its tokens); the block synchronises after.
+// Four heads of a chunk: its place in the packed tokens, its steps' sizes dt and weights in the state's contribution dt_s a(s, n-1), and
+// the running sums of -exp(A_log) dt (zero steps behind its tokens).  Once a chunk and head: worked out by every tile of contributions and
+// again by every tile of outputs, in front of their products, they cost both kernels a chain of searches, logarithms and sums in float64.
 template <typename T>
-__device__ __forceinline__ void st_steps(const ScanArgs& a, int h, int first, int n, float* dts, double* las, double* half) {
-    const int t = threadIdx.x, lane = t & 31;
-    double la = 0.0;
-    if (t < SS_CHUNK) {
-        const float A = expf(load_as_f(a.a_log, a.al_dtype, h)), bias = load_as_f(a.dt_bias, a.dtb_dtype, h);
-        const float dt = t < n ? ss_softplus(to_f(((const T*)a.proj)[(size_t)(first + t) * a.proj_ld + a.dt_off + h]) + bias) : 0.f;
-        la = fmax(-(double)A * (double)dt, -1e4);          // (exp of it is zero in float32 long before; a sum with an infinity has no differences)
+__global__ void __launch_bounds__(4 * SS_CHUNK) st_steps_kernel(ScanArgs a) {
+    pdl_launch_dependents();
+    pdl_wait();
+    __shared__ double sums[4][2];
+    int first, n;
+    st_find_chunk(a, a.first_chunk + blockIdx.x, first, n);
+    if (threadIdx.x == 0 && blockIdx.y == 0) a.chunk_rows[blockIdx.x] = make_int2(first, n);
+    if (n <= 0) return;
+    const int hh = threadIdx.x / SS_CHUNK, t = threadIdx.x % SS_CHUNK, lane = t & 31, h = blockIdx.y * 4 + hh;
+    const bool on = h < a.H;
+    const float A = on ? expf(load_as_f(a.a_log, a.al_dtype, h)) : 0.f, bias = on ? load_as_f(a.dt_bias, a.dtb_dtype, h) : 0.f;
+    const float dt = on && t < n ? ss_softplus(to_f(((const T*)a.proj)[(size_t)(first + t) * a.proj_ld + a.dt_off + h]) + bias) : 0.f;
+    double la = fmax(-(double)A * (double)dt, -1e4);       // (exp of it is zero in float32 long before; a sum with an infinity has no differences)
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const double below = __shfl_up_sync(0xffffffffu, la, o);
-            if (lane >= o) la += below;
-        }
-        if (t == 31) *half = la;
-        dts[t] = dt;
+    for (int o = 1; o < 32; o <<= 1) {
+        const double below = __shfl_up_sync(0xffffffffu, la, o);
+        if (lane >= o) la += below;
     }
+    if (lane == 31) sums[hh][t >> 5] = la;
     __syncthreads();
-    if (t < SS_CHUNK) las[t] = t < 32 ? la : la + *half;
-    __syncthreads();
+    if (!on) return;
+    const double end = sums[hh][1] + sums[hh][0];
+    if (t >= 32) la += sums[hh][0];
+    float* dst = a.chunk_steps + ((size_t)blockIdx.x * a.H + h) * SS_STEP_FLOATS;
+    reinterpret_cast<float2*>(dst)[t] = make_float2(dt, dt * expf((float)(end - la)));
+    reinterpret_cast<double*>(dst + 2 * SS_CHUNK)[t] = la;
+    if (t == 0) a.chunk_decay[(size_t)blockIdx.x * a.H + h] = expf((float)end);
 }
 
 // blockIdx.y < H: chunk and head, 128 state rows x 64 columns of L (blockIdx.z: which).  From H on: the scores of a chunk and group.
-template <typename T>
 __global__ void __launch_bounds__(ST_THREADS) st_contribution_kernel(ScanArgs a, int vec_bc, int vec_x, int tiles_n) {
     pdl_launch_dependents();
     pdl_wait();
     __shared__ __align__(16) float smem[SS_CHUNK * 128 / 2 + SS_CHUNK * 64 / 2];         // 32 tokens of B and of x; or two slices
-    __shared__ float dts[SS_CHUNK];
-    __shared__ double las[SS_CHUNK], half;
+    __shared__ float ws[SS_CHUNK];
     const int tid = threadIdx.x, H = a.H, N = a.N, P = a.P, inner = H * P;
-    int first, n;
-    st_find_chunk(a, a.first_chunk + blockIdx.x, first, n);
+    const int first = a.chunk_rows[blockIdx.x].x, n = a.chunk_rows[blockIdx.x].y;
     if (n <= 0) return;
     if ((int)blockIdx.y >= H) {
         if (blockIdx.z) return;
@@ -116,8 +124,7 @@ __global__ void __launch_bounds__(ST_THREADS) st_contribution_kernel(ScanArgs a,
         }
     };
     fetch(0);
-    st_steps<T>(a, h, first, n, dts, las, &half);
-    const double end = las[SS_CHUNK - 1];
+    if (tid < SS_CHUNK) ws[tid] = reinterpret_cast<const float2*>(a.chunk_steps + ((size_t)blockIdx.x * H + h) * SS_STEP_FLOATS)[tid].y;
     const int lane = tid & 31, warp = tid >> 5, ty = warp * 4 + (lane >> 3), tx = lane & 7;       // 16 x 8 threads: rows ty * 4 + 64 i, columns tx * 4 + 32 j
     st_pair acc[8][4];
 #pragma unroll
@@ -125,13 +132,13 @@ __global__ void __launch_bounds__(ST_THREADS) st_contribution_kernel(ScanArgs a,
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
     for (int s0 = 0; s0 < n; s0 += 32) {
-        if (s0) __syncthreads();
+        __syncthreads();
 #pragma unroll
         for (int e = 0; e < 8; ++e) *reinterpret_cast<float4*>(bs + 4 * (tid + e * ST_THREADS)) = rb[e];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int i = tid + e * ST_THREADS, s = s0 + (i >> 4);
-            const float w = dts[s] * expf((float)(end - las[s]));
+            const float w = ws[s];
             *reinterpret_cast<float4*>(xs + 4 * i) = make_float4(rx[e].x * w, rx[e].y * w, rx[e].z * w, rx[e].w * w);
         }
         if (s0 + 32 < n) fetch(s0 + 32);
@@ -157,7 +164,6 @@ __global__ void __launch_bounds__(ST_THREADS) st_contribution_kernel(ScanArgs a,
         st_store4(row, P - p0 - tx * 4, vec, st_four(acc[i][0], acc[i][1]));
         st_store4(row + 32, P - p0 - tx * 4 - 32, vec, st_four(acc[i][2], acc[i][3]));
     }
-    if (blockIdx.z == 0 && tid == 0) a.chunk_decay[(size_t)blockIdx.x * H + h] = expf((float)end);
 }
 
 // A thread an element of a sequence's state walks the sequence's chunks in order, leaves every chunk its incoming state where its own
@@ -203,16 +209,14 @@ __global__ void __launch_bounds__(256) st_carry_kernel(ScanArgs a) {
 }
 
 // Chunk, head and 64 columns of its outputs.
-template <typename T>
 __global__ void __launch_bounds__(ST_THREADS) st_output_kernel(ScanArgs a, int vec_bc, int vec_x) {
     pdl_launch_dependents();
     pdl_wait();
     __shared__ __align__(16) float smem[2 * SS_CHUNK * SS_CHUNK];       // two buffers of a slice of C and of S; then weights and x
     __shared__ float dts[SS_CHUNK];
-    __shared__ double las[SS_CHUNK], half;
+    __shared__ double las[SS_CHUNK];
     const int tid = threadIdx.x, H = a.H, N = a.N, P = a.P, inner = H * P, h = blockIdx.y, g = h / (H / a.G), p0 = blockIdx.z * 64;
-    int first, n;
-    st_find_chunk(a, a.first_chunk + blockIdx.x, first, n);
+    const int first = a.chunk_rows[blockIdx.x].x, n = a.chunk_rows[blockIdx.x].y;
     if (n <= 0) return;
     int ty, tx;
     st_place(ty, tx);
@@ -235,7 +239,11 @@ __global__ void __launch_bounds__(ST_THREADS) st_output_kernel(ScanArgs a, int v
         for (int e = 0; e < 4; ++e) *reinterpret_cast<float4*>(to + ST_SLICE * SS_CHUNK + 4 * (tid + e * ST_THREADS)) = rs[e];
     };
     fetch(0);
-    st_steps<T>(a, h, first, n, dts, las, &half);
+    if (tid < SS_CHUNK) {
+        const float* steps = a.chunk_steps + ((size_t)blockIdx.x * H + h) * SS_STEP_FLOATS;
+        dts[tid] = reinterpret_cast<const float2*>(steps)[tid].x;
+        las[tid] = reinterpret_cast<const double*>(steps + 2 * SS_CHUNK)[tid];
+    }
     put(smem);
     __syncthreads();
     st_pair acc[8][2];
@@ -305,11 +313,13 @@ static int st_run(ScanArgs a, cudaStream_t s) {
     const int vec_x = rows && a.P % 4 == 0, vec_bc = rows && (a.H * a.P) % 4 == 0 && a.N % 4 == 0;
     const int tn = (a.N + 127) / 128, tp = (a.P + 63) / 64;
     for (; a.first_chunk < a.chunks; a.first_chunk += a.slab) {      // (the carry between two slabs lies in the sequences' states)
-        PE_TRY(pe_launch(st_contribution_kernel<T>, dim3(a.slab, a.H + a.G, tn * tp), ST_THREADS, 0, s, a, vec_bc, vec_x, tn));
+        PE_TRY(pe_launch(st_steps_kernel<T>, dim3(a.slab, (a.H + 3) / 4), 4 * SS_CHUNK, 0, s, a));
+        PE_LAUNCH_CHECK();
+        PE_TRY(pe_launch(st_contribution_kernel, dim3(a.slab, a.H + a.G, tn * tp), ST_THREADS, 0, s, a, vec_bc, vec_x, tn));
         PE_LAUNCH_CHECK();
         PE_TRY(pe_launch(a.slab == a.chunks ? st_carry_kernel<true> : st_carry_kernel<false>, dim3((unsigned)(((size_t)a.H * a.N * a.P + 255) / 256), a.B), 256, 0, s, a));
         PE_LAUNCH_CHECK();
-        PE_TRY(pe_launch(st_output_kernel<T>, dim3(a.slab, a.H, tp), ST_THREADS, 0, s, a, vec_bc, vec_x));
+        PE_TRY(pe_launch(st_output_kernel, dim3(a.slab, a.H, tp), ST_THREADS, 0, s, a, vec_bc, vec_x));
         PE_LAUNCH_CHECK();
     }
     return 0;

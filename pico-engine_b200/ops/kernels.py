@@ -1377,7 +1377,7 @@ def state_space_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_offset: int, dt_b
     """y float32 [T, H * P] of S_t = exp(-exp(A_log) dt) S_(t-1) + dt B_t x_t^T, y_t = S_t^T C_t + D x_t with dt = softplus(raw + bias):
     x | B | C are the columns of ``xbc`` float32 [T, H*P + 2 G N], the raw step sizes columns ``dt_offset`` .. of proj.  The states
     come from and return to the sequences' float32 state at ``state_offset``.  ``chunked``: prompts, as products of tiles over chunks of 64
-    tokens (in slabs of chunks, three launches each: every chunk's contribution to the state, a carry pass, the outputs) instead of one walk a sequence; both give
+    tokens (in slabs of chunks, four launches each: the chunks' step sizes and decays, every chunk's contribution to the state, a carry pass, the outputs) instead of one walk a sequence; both give
     the same numbers up to float32 rounding."""
     from .library import state_space
     T = xbc.shape[0]
@@ -1397,7 +1397,7 @@ def state_space_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_offset: int, dt_b
                                             dt_bias.data_ptr(), _code(dt_bias, "dt_bias"), a_log.data_ptr(), _code(a_log, "a_log"),
                                             d_skip.data_ptr(), _code(d_skip, "d_skip"), sp, stride, row_first.data_ptr(),
                                             row_lens.data_ptr(), slots.data_ptr(), y.data_ptr(), T, slots.shape[0], H, P, N, G,
-                                            1 if chunked else 0, ws, stream_ptr()), "state_space_scan", 3 * slabs if chunked else 1)
+                                            1 if chunked else 0, ws, stream_ptr()), "state_space_scan", 4 * slabs if chunked else 1)
     return y
 
 

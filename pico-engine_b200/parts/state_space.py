@@ -77,7 +77,7 @@ class StateSpace(Mixer):
         token after token; either way gives the same numbers up to float32 rounding.
 
         A walk takes as long as the longest row, and as all rows' tokens take where there are more blocks (a row, head and as many columns as
-        256 threads hold) than run side by side; tiles cost three launches, every chunk its products whatever it holds, and every row the
+        256 threads hold) than run side by side; tiles cost four launches, every chunk its products whatever it holds, and every row the
         pass that carries its state.  The numbers (for microseconds on a B200) are fitted to 339 steps of 1 to 64 rows of 8 to 2,048 tokens, 16
         to 256 state rows and 8 to 112 heads; the worst choice among them costs a third more than the better way.  64
         heads of 64 columns, 128 state rows, walk / tiles: 1 x 17 tokens 17 / 36 us, 1 x 64 53 / 43, 1 x 2,048 1,583 / 179; 8 x 32 86 / 97,
