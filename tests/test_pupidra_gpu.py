@@ -379,6 +379,38 @@ def run_state_space(proj, m, conv_w, conv_b, dt_bias, a_log, d_skip, norm_w, eps
     return out
 
 
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("taps", [2, 3, 4])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_convolution_of_runs_where_rows_meet(dtype, taps, shift):
+    """Rows that begin and end at every place of a run of eight tokens, one to nine tokens long and longer, from a state that is not zero, with
+    weights off the boundary that four of them are read from: against float64.  A sum has taps + 1 roundings of at most the sum of its
+    terms' magnitudes (2^-24 each), which silu passes on at most 1.1-fold and rounds to a few 2^-24 of itself."""
+    from pico_engine.ops import kernels
+    dt, C, ld, off = DTYPES[dtype], 1280, 1288, 4
+    lens = [1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 3, 1, 1, 13, 300, 64, 27]
+    T, B = sum(lens), len(lens)
+    assert T * C >= 500000 and T >= 8 * B                        # the sizes that runs take
+    g = torch.Generator().manual_seed(taps)
+    proj = torch.randn(T, ld, generator=g).to(dt)
+    w, bias = (torch.randn(*n, generator=g).to(dt).cuda().view(-1)[shift:] for n in ((C * taps + shift,), (C + shift,)))
+    state = torch.randn(B + 1, (taps - 1) * C, generator=g).cuda()
+    slots = torch.arange(B, 0, -1, dtype=torch.int32).cuda()
+    first = np.concatenate([[0], np.cumsum(lens)])
+    old = state.double().cpu()
+    got = kernels.conv_silu(proj.cuda(), off, C, w.view(C, taps), bias, state, 0, torch.tensor(np.repeat(np.arange(B), lens), dtype=torch.int32).cuda(),
+                            torch.tensor(first, dtype=torch.int32).cuda(), torch.tensor(lens, dtype=torch.int32).cuda(), slots).double().cpu()
+    w64, b64 = w.view(C, taps).double().cpu(), bias.double().cpu()
+    for b, n in enumerate(lens):
+        rows = proj[first[b]: first[b] + n, off: off + C].double()
+        u = torch.cat([old[B - b].view(taps - 1, C).flip(0), rows])          # entry k of a state: the input k + 1 places before the step
+        terms = torch.stack([w64[:, j] * u[j: j + n] for j in range(taps)])
+        v = terms.sum(0) + b64
+        err = (got[first[b]: first[b] + n] - v * torch.sigmoid(v)).abs()
+        assert (err <= 2.0 ** -24 * (1.1 * (taps + 1) * (terms.abs().sum(0) + b64.abs()) + 8 * v.abs())).all(), (b, n)
+        assert torch.equal(state[B - b].double().cpu().view(taps - 1, C), u.flip(0)[: taps - 1])
+
+
 def plain_state_space(proj, m, conv_w, conv_b, dt_bias, a_log, d_skip, norm_w, eps, lens):
     H, P, N, G = m["heads"], m["vdim"], m["state"], m["groups"]
     inner = H * P
