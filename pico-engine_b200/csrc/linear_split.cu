@@ -33,7 +33,10 @@
 // Infinities, values that are no number and sums beyond float32 leave results that are not finite; those are worked out again with plain
 // multiply-adds.
 //
-// Every wait is bounded by the clock; one that runs out sets *status to 9 and a flag that lets every other role leave its loop.
+// Every wait is bounded by the clock; one that runs out sets *status to 9 and a flag that lets every other role leave its loop.  The CTA
+// then waits (with a limit again) for the copies and products it has under way, stores nothing, and takes the same steps with its cluster as
+// every other CTA: none leaves before all have sent their sums, and the wait for these does not look at the flag, since
+// every CTA sends them whatever became of its loops.
 //
 // pico-engine leaves these products to cuBLAS (src/pico_engine/model.py:177, 213, 223, 235, 164).
 #include "tcgen05_attention.cuh"
@@ -164,6 +167,8 @@ __device__ __forceinline__ bool sp_wait(unsigned bar, unsigned parity, volatile 
         }
     }
 }
+// The wait for what the cluster's other CTAs send: whatever happened here they send it, at the latest when their own waits have run out.
+__device__ __forceinline__ bool sp_wait_sent(unsigned bar) { return at_wait(bar, 0) || at_wait(bar, 0) || at_wait(bar, 0); }
 __device__ __forceinline__ bool sp_wait_warp(unsigned bar, unsigned parity, volatile int* abort_flag, int* status) {
     return __all_sync(0xffffffffu, sp_wait(bar, parity, abort_flag, status));
 }
@@ -191,7 +196,7 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
     if (!MANY) nt = NT;
     const int part_bytes = nt * SP_KC * 4;
     extern __shared__ unsigned char sp_raw[];
-    __shared__ __align__(8) unsigned long long bars[2 * RING + 2 * SP_SLOTS + 2 * SUMS + 1];
+    __shared__ __align__(8) unsigned long long bars[2 * RING + 3 * SP_SLOTS + 2 * SUMS + 1];
     __shared__ unsigned tmem_base_s;
     __shared__ int abort_s;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -200,7 +205,7 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
     const int all = (K + SP_KC - 1) / SP_KC, each = (all + ranges - 1) / ranges;
     const int k_begin = rank * each * SP_KC, k_end = min(K, k_begin + each * SP_KC), chunks = (k_end - k_begin + SP_KC - 1) / SP_KC;
     const unsigned w_full = at_smem(bars), w_empty = w_full + 8 * RING, full = w_empty + 8 * RING, empty = full + 8 * SP_SLOTS, sum_full = empty + 8 * SP_SLOTS,
-                   sum_empty = sum_full + 8 * SUMS, sent = sum_empty + 8 * SUMS;
+                   sum_empty = sum_full + 8 * SUMS, sent = sum_empty + 8 * SUMS, a_full = sent + 8;
     // the rows of A whose sums over the cluster this CTA finishes
     const int slice = (nt + ranges - 1) / ranges, first_row = rank * slice, rows = max(0, min(min(nt, first_row + slice), M - m0) - first_row);
 
@@ -212,7 +217,7 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
         const auto init = [](unsigned bar, int count, unsigned arrivals) {
             for (int i = 0; i < count; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar + 8 * i), "r"(arrivals) : "memory");
         };
-        init(w_full, RING, 1); init(w_empty, RING, 4); init(full, SP_SLOTS, MANY ? 5 : 4); init(empty, SP_SLOTS, 1); init(sum_full, SUMS, 1); init(sum_empty, SUMS, sp_takers<NT>());
+        init(w_full, RING, 1); init(w_empty, RING, 4); init(full, SP_SLOTS, 4); if (MANY) init(a_full, SP_SLOTS, 1); init(empty, SP_SLOTS, 1); init(sum_full, SUMS, 1); init(sum_empty, SUMS, sp_takers<NT>());
         if (!MANY) {
             init(sent, 1, 1);
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sent), "r"((unsigned)((ranges - 1) * rows * SP_ROWS * 4)) : "memory");
@@ -297,10 +302,12 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
     } else if (warp == SP_CUTTERS) {
         const unsigned idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((unsigned)(nt / 8) << 17) | ((unsigned)(SP_ROWS / 16) << 24);
         const unsigned elected = sp_elect();
+        int issued = 0;
         for (int c = 0; c < chunks; ++c) {
             const int s = c % SP_SLOTS, b = c % SUMS;
             if (c >= SUMS && !sp_wait_warp(sum_empty + 8 * b, (c / SUMS - 1) & 1, &abort_s, status)) break;
             if (!sp_wait_warp(full + 8 * s, (c / SP_SLOTS) & 1, &abort_s, status)) break;
+            if (MANY && !sp_wait_warp(a_full + 8 * s, (c / SP_SLOTS) & 1, &abort_s, status)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const unsigned long long a = at_desc(a_parts + s * 2 * part_bytes, 16, 1024);
             sp_products(elected, sums + b * NT, tmem + s * 2 * SP_KC, a, a + (part_bytes >> 4), idesc);
@@ -309,22 +316,30 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
                 at_commit(sum_full + 8 * b);
             }
             __syncwarp();
+            issued = c + 1;
         }
+        if (issued > 0) at_wait_warp(sum_full + 8 * ((issued - 1) % SUMS), ((issued - 1) / SUMS) & 1);      // nothing stays under way
     } else if (warp == SP_CUTTERS + 1) {
         if (lane == 0) {
+            int brought = min(RING, chunks), brought_a = 0;
             for (int c = 0; c < chunks; ++c) {
                 const int s = c % SP_SLOTS, r = c % RING;
                 if (MANY) {
                     if (c >= SP_SLOTS && !sp_wait(empty + 8 * s, (c / SP_SLOTS - 1) & 1, &abort_s, status)) break;
-                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full + 8 * s), "r"((unsigned)(2 * part_bytes)) : "memory");
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(a_full + 8 * s), "r"((unsigned)(2 * part_bytes)) : "memory");
                     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-                                 ::"r"(a_parts + s * 2 * part_bytes), "l"(&map_a), "r"(full + 8 * s), "r"(k_begin + c * SP_KC), "r"(m0), "r"(0) : "memory");
+                                 ::"r"(a_parts + s * 2 * part_bytes), "l"(&map_a), "r"(a_full + 8 * s), "r"(k_begin + c * SP_KC), "r"(m0), "r"(0) : "memory");
+                    brought_a = c + 1;
                 }
                 if (c + RING < chunks) {
                     if (!sp_wait(w_empty + 8 * r, (c / RING) & 1, &abort_s, status)) break;
                     bring_w(c + RING);
+                    brought = c + RING + 1;
                 }
             }
+            // (each of them has landed long ago unless a role gave up)
+            for (int c = max(0, brought - RING); c < brought; ++c) at_wait(w_full + 8 * (c % RING), (c / RING) & 1);
+            for (int c = max(0, brought_a - SP_SLOTS); c < brought_a; ++c) at_wait(a_full + 8 * (c % SP_SLOTS), (c / SP_SLOTS) & 1);
         }
         __syncwarp();
     } else {
@@ -342,6 +357,7 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
         }
     }
     __syncthreads();                                       // all products have ended, all copies have landed
+    bool whole = *(volatile int*)&abort_s == 0;
     if (warp >= TAKER) {                                   // [nt][128] sums where the operands were
         const int row = (warp & 3) * 32 + lane, n = n0 + row;
         float zero = 0.f;                                  // no number if one of the sums is not finite
@@ -378,11 +394,15 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
                              " st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [at], {%3, %4, %5, %6}, [bar];\n}"
                              ::"r"(sums_sent + ((rank * slice + t - to * slice) * SP_ROWS + col) * 4), "r"(sent), "r"(to), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
             }
-            if (rows > 0) sp_wait(sent, 0, &abort_s, status);
+            asm volatile("barrier.cluster.arrive.release;" ::: "memory");      // this CTA has sent
+            if (rows > 0 && !sp_wait_sent(sent)) {
+                whole = false;
+                if (status) atomicExch(status, 9);
+            }
         }
     }
 #pragma unroll 1
-    for (int i = tid; i < rows * (SP_ROWS / 4); i += sp_threads<NT>()) {
+    for (int i = tid; i < (whole ? rows * (SP_ROWS / 4) : 0); i += sp_threads<NT>()) {
         const int t = i / (SP_ROWS / 4), col = i % (SP_ROWS / 4) * 4, n = n0 + col;
         if (n >= N) continue;
         const unsigned at = smem + ((first_row + t) * SP_ROWS + col) * 4;
@@ -403,6 +423,10 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
             if (n + e < N) sp_finish(four[e], out, (size_t)(m0 + first_row + t) * N + n + e, bias, bias_dtype, n + e, epilogue);
     }
     if (MANY && ranges > 1) sp_cluster_sync();             // nobody leaves while its sums are being read
+    if (!MANY && ranges > 1) {
+        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");           // or before all have sent
+        if (!whole && rows > 0) sp_wait_sent(sent);
+    }
     if (warp == SP_CUTTERS) {
         __syncwarp();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");

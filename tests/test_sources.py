@@ -15,3 +15,17 @@ def test_cluster_barriers_are_of_the_form_that_lanes_may_reach_apart(name):
     with open(os.path.join(CSRC, name + ".cu")) as f:
         lines = [line for line in f if "barrier.cluster" in line]
     assert lines and not any(".aligned" in line for line in lines)
+
+
+def test_float32_products_leave_their_cluster_together():
+    """Up to 64 rows, the CTAs of linear_split.cu write sums into each other's shared memory, so none may end before all have sent, not even
+    one whose waits ran out: no way out of the kernel but its end, a cluster barrier between the last sum sent and that end in
+    every form, and a wait for the others' sums that the CTA's own give-up flag does not cut short."""
+    with open(os.path.join(CSRC, "linear_split.cu")) as f:
+        text = f.read()
+    body = text[text.index("linear_split_kernel(const __grid_constant__"):text.index("static int sp_map")]
+    behind = body[body.index("st.async"):]
+    assert "return;" not in body
+    arrive, finish = behind.index("barrier.cluster.arrive"), behind.index("sp_finish(")
+    assert arrive < finish < behind.index("barrier.cluster.wait")
+    assert not any("(sent" in line and "abort" in line for line in body.splitlines())
