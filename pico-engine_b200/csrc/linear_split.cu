@@ -18,7 +18,7 @@
 //              with W there the tensor core waited for shared memory, 1,450 to 2,000 cycles a chunk of 112 rows of A); up to 64
 //              rows of A are cut here too and go to shared memory
 //   warp 8     issues a chunk's twelve products
-//   warp 9     brings W (float32) by TMA, before the kernel waits for its predecessor as far as the ring goes; more than 64 rows of A
+//   warp 9     brings W (float32) by TMA, into L2 as far as the ring goes before the kernel waits for its predecessor; more than 64 rows of A
 //              have been cut by a kernel before this one and come by TMA as well
 //   warps 10-  take the sums out of tensor memory
 // Bound by the tensor core and the hand-over of its sums: a chunk of 112 rows of A takes 1,150 cycles, its products alone 980.
@@ -236,9 +236,13 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
     if (!MANY && ranges > 1) asm volatile("barrier.cluster.arrive.release;" ::: "memory");      // this CTA can be sent to
     const unsigned tmem = tmem_base_s, sums = tmem + SP_SLOTS * 2 * SP_KC;
     pdl_launch_dependents();                               // (behind the allocation of tensor memory: a later kernel must not take it first)
+    // W may be what the kernel in front writes: until that has ended it is only brought as far as L2, where its writes arrive too
     if (tid == 32 * (SP_CUTTERS + 1))
-        for (int c = 0; c < min(RING, chunks); ++c) bring_w(c);      // weights: no kernel writes them
+        for (int c = 0; c < min(RING, chunks); ++c)
+            asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(&map_w), "r"(k_begin + c * SP_KC), "r"(n0) : "memory");
     pdl_wait();
+    if (tid == 32 * (SP_CUTTERS + 1))
+        for (int c = 0; c < min(RING, chunks); ++c) bring_w(c);
 
     unsigned long long acc[COLS / 2];                      // pairs of columns
     const int column0 = MANY ? ((warp - TAKER) >> 2) * COLS : 0, columns = MANY ? max(0, min(COLS, nt - column0)) : NT;

@@ -675,6 +675,18 @@ def test_linear_float32_in_parts(K, N, K_):
         assert torch.equal(K.linear_simt(A[:M], W, B, out_dtype=torch.bfloat16), whole[:M].to(torch.bfloat16))
 
 
+@pytest.mark.parametrize("M", [3, 100])
+def test_linear_float32_of_a_weight_just_written(K, M):
+    """A weight that the kernel in front writes: no entry is read before it is there."""
+    a, ids = dev(rnd(M, 896, seed=1)), dev(torch.arange(1024, dtype=torch.int32).flip(0))
+    tables = [dev(rnd(1024, 896, seed=2 + i)) for i in range(8)]
+    want = [K.linear_simt(a, t.flip(0)) for t in tables]
+    w = torch.zeros(1024, 896, device="cuda")
+    torch.cuda.synchronize()
+    got = [K.linear_simt(a, K.embed(t, ids, out=w)) for t in tables]
+    assert all(torch.equal(g, x) for g, x in zip(got, want))
+
+
 @pytest.mark.parametrize("M", [7, 60, 200])
 @pytest.mark.parametrize("N,K_", [(4100, 264), (896, 896)])
 def test_linear_float32_in_parts_of_values_that_are_not_finite(K, M, N, K_):
