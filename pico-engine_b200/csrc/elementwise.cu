@@ -156,8 +156,9 @@ __device__ __forceinline__ float rn_take(float4* x4, const TY* y, int i0, int st
 
 // With ADD the row of y is first added to the row of x, which is written back: the residual sum
 // that precedes the norm, in the same pass.  A thread keeps up to KEEP groups of four elements in
-// registers between the two passes; longer rows are read again.  Weights are fetched while the kernel before still runs (WB: bfloat16 on an
-// 8-byte boundary, two registers for four of them), or, where that would take registers from the blocks beside this one, before the block meets.
+// registers between the two passes; longer rows are read again.  Weights come as far as L2 while the kernel before still runs (it may be
+// writing them) and are asked for with the row (WB: bfloat16 on an 8-byte boundary, two registers for four of them), or, where that would take
+// registers from the blocks beside this one, before the block meets.
 template <typename TO, typename TY, bool ADD, int KEEP, bool WB>
 __global__ void __launch_bounds__(512, 2) rmsnorm_kernel(float* x, const TY* y, const int* rows_index,
                                                          const void* w, int w_dtype, float eps, TO* out, int H) {
@@ -180,8 +181,10 @@ __global__ void __launch_bounds__(512, 2) rmsnorm_kernel(float* x, const TY* y, 
             }
         };
         constexpr bool early = WB || KEEP <= 2 || !ADD;
-        if (early) weights();
+        for (unsigned at = threadIdx.x * 128u, end = (unsigned)H * (w_dtype == PE_BF16 ? 2u : 4u); at < end; at += blockDim.x * 128u)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"((const char*)w + at) : "memory");
         pdl_wait();
+        if (early) weights();
         const size_t src = rows_index ? rows_index[r] : r;
         float4* x4 = reinterpret_cast<float4*>(x + src * H);
         float ss = rn_take<KEEP, TY, ADD>(x4, y + src * H, threadIdx.x, blockDim.x, n4, v, 0.f);

@@ -105,6 +105,22 @@ def test_rmsnorm_at_the_edges_of_its_shapes(K, H, rows, shift):
             assert ((got.double().cpu() - want).abs() <= (45 / 2 + 4) * 2.0 ** -24 * want.abs()).all()
 
 
+@pytest.mark.parametrize("rows,H", [(1, 896), (5, 3584), (5000, 128)])
+@pytest.mark.parametrize("add", [False, True])
+def test_rmsnorm_of_a_weight_just_written(K, rows, H, add):
+    """A weight that the kernel in front writes, in the last of its rows: no entry is read before it is there."""
+    x, y, ids = dev(rnd(rows, H, seed=1)), dev(rnd(rows, H, seed=2)), dev(torch.arange(300, dtype=torch.int32).flip(0))
+    run = lambda w: K.add_rmsnorm(x.clone(), y, w, 1e-6, torch.float32) if add else K.rmsnorm(x, w, 1e-6, torch.float32)
+    tables = [dev(rnd(300, H, seed=3 + i)) for i in range(8)]
+    want = [run(t[0].clone()) for t in tables]
+    buf = torch.zeros(300, H, device="cuda")
+    xs = [x.clone() for _ in tables]
+    torch.cuda.synchronize()
+    got = [K.add_rmsnorm(xc, y, K.embed(t, ids, out=buf)[299], 1e-6, torch.float32) if add else K.rmsnorm(x, K.embed(t, ids, out=buf)[299], 1e-6, torch.float32)
+           for t, xc in zip(tables, xs)]
+    assert all(torch.equal(g, v) for g, v in zip(got, want))
+
+
 def test_rmsnorm_eps_matters(K):
     x, w = torch.full((1, 64), 1e-3), torch.ones(64)
     for eps in (1e-6, 1e-2):
