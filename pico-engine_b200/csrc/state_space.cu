@@ -47,7 +47,7 @@ __global__ void conv_silu_kernel(const T* proj, int ld, int c_off, int C, int ta
 // to the next ones, so that an input is read once (and `taps` - 1 times more at the front of a run) where the kernel above reads it
 // `taps` times, with a division an element to find its place.  The sums run in the same order.  Where the run and the inputs in front of
 // it lie in one row, those are asked for together with the run's own: places and states, three reads one behind the other, are
-// looked up only where a row begins.  Weights come four at a time and before the wait for the kernel in front.  2,047 tokens of
+// looked up only where a row begins.  Weights come four at a time, as far as L2 before the wait for the kernel in front (which may be writing them).  2,047 tokens of
 // 4,608 channels, bfloat16, on a B200: 79 us by the kernel above, 23.3 with the look-up for each run and single weights, 20.1 here.
 #define CONV_TOKENS 8
 __device__ __forceinline__ float4 ss_read4(const float* p) { return *reinterpret_cast<const float4*>(p); }
@@ -68,11 +68,14 @@ __global__ void __launch_bounds__(128) conv_silu_vec_kernel(const T* proj, int l
     pdl_launch_dependents();
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 4, t0 = blockIdx.y * CONV_TOKENS, m = min(CONV_TOKENS, n_tok - t0);
     if (c >= C) return;
+    const unsigned w_size = w_dtype == PE_BF16 ? 2 : 4, b_size = b_dtype == PE_BF16 ? 2 : 4;
+    asm volatile("prefetch.global.L2 [%0];" ::"l"((const char*)w + (size_t)c * TAPS * w_size) : "memory");
+    if (bias) asm volatile("prefetch.global.L2 [%0];" ::"l"((const char*)bias + (size_t)c * b_size) : "memory");
+    pdl_wait();
     __align__(16) float flat[4 * TAPS], b4[4];                   // channel c + e, weight j: flat[e * TAPS + j]
 #pragma unroll
     for (int q = 0; q < TAPS; ++q) *reinterpret_cast<float4*>(flat + 4 * q) = ss_weights4(w, w_dtype, (size_t)c * TAPS + 4 * q);
     *reinterpret_cast<float4*>(b4) = bias ? ss_weights4(bias, b_dtype, c) : make_float4(0.f, 0.f, 0.f, 0.f);
-    pdl_wait();
     const T* src = proj + (size_t)t0 * ld + c_off + c;
     float4 in[CONV_TOKENS], past[TAPS];                          // past[k]: the input k + 1 places back
     const int front = t0 - (TAPS - 1), last = tok_row[t0 + m - 1];

@@ -411,6 +411,24 @@ def test_convolution_of_runs_where_rows_meet(dtype, taps, shift):
         assert torch.equal(state[B - b].double().cpu().view(taps - 1, C), u.flip(0)[: taps - 1])
 
 
+def test_convolution_of_weights_just_written():
+    """Weights that the kernel in front writes: none is read before it is there."""
+    from pico_engine.ops import kernels
+    T, C, taps = 1000, 1024, 4
+    g = torch.Generator().manual_seed(1)
+    rnd = lambda *n: torch.randn(*n, generator=g)
+    proj, state, ids = rnd(T, C).cuda(), torch.zeros(1, (taps - 1) * C, device="cuda"), torch.arange(C, dtype=torch.int32).flip(0).cuda()
+    bias, zeros, one = rnd(C).cuda(), torch.zeros(T, dtype=torch.int32, device="cuda"), torch.tensor([0, T], dtype=torch.int32, device="cuda")
+    run = lambda w: kernels.conv_silu(proj, 0, C, w, bias, torch.zeros_like(state), 0, zeros, one, one[1:], zeros[:1])
+    tables = [rnd(C, taps).cuda() for _ in range(8)]
+    want = [run(t.flip(0)) for t in tables]
+    w = torch.zeros(C, taps, device="cuda")
+    states = [state.clone() for _ in tables]
+    torch.cuda.synchronize()
+    got = [kernels.conv_silu(proj, 0, C, kernels.embed(t, ids, out=w), bias, s, 0, zeros, one, one[1:], zeros[:1]) for t, s in zip(tables, states)]
+    assert all(torch.equal(g, v) for g, v in zip(got, want))
+
+
 def plain_state_space(proj, m, conv_w, conv_b, dt_bias, a_log, d_skip, norm_w, eps, lens):
     H, P, N, G = m["heads"], m["vdim"], m["state"], m["groups"]
     inner = H * P
