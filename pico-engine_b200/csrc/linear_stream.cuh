@@ -13,6 +13,9 @@
 // (the row's 1/rms is applied to the sums); of bfloat16 rows 64 columns come with each pair of boxes.
 //
 // A row's sums do not depend on its neighbours: columns are added in the order of the warps that have them, whatever M is.
+//
+// A wait that runs out sets *status to 10.  The whole CTA leaves before it writes anything of that group or of a later one, when what it has
+// under way has landed (a wait with a limit again).
 #pragma once
 #include "tcgen05_attention.cuh"
 
@@ -122,6 +125,7 @@ __global__ void __launch_bounds__(32 * LS_WARPS, 1) linear_stream_kernel(const _
 
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
     int used = 0;
+    bool late = false;                                      // a box of this warp's has not come
     for (int group = blockIdx.x; group < a.groups; group += gridDim.x) {
         // ROPE: what the epilogue needs of the step's description and of the rotation tables is asked for now
         const int ep_r = (lane >> 2) + 8 * ((warp >> 1) & 1), ep_m = (warp >> 2) * 8 + 2 * (lane & 3) + (warp & 1);      // this thread's row and token (256 threads: two tokens' groups)
@@ -140,10 +144,7 @@ __global__ void __launch_bounds__(32 * LS_WARPS, 1) linear_stream_kernel(const _
             for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.f;
         for (int c = warp; c < chunks; c += LS_WARPS) {
             const unsigned s = used % SLOTS, w_at = ring + s * SLOT;
-            if (!lf_bar_wait(bar + 8 * s, (used / SLOTS) & 1)) {
-                atomicExch(status, 10);                     // the copies did not arrive: what this warp has is wrong, and said to be
-                break;
-            }
+            const bool here = lf_bar_wait(bar + 8 * s, (used / SLOTS) & 1);
             ++used;
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
@@ -160,7 +161,7 @@ __global__ void __launch_bounds__(32 * LS_WARPS, 1) linear_stream_kernel(const _
                     lf_mma(acc[1][j], h0.z, h1.z, h0.w, h1.w, v.z, v.w);
                 }
             }
-            __syncwarp();
+            if ((late = __any_sync(0xffffffffu, !here))) break;
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");             // the slot's reads precede its refill
             send();
         }
@@ -171,7 +172,11 @@ __global__ void __launch_bounds__(32 * LS_WARPS, 1) linear_stream_kernel(const _
             for (int j = 0; j < NT; ++j)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) red[warp][(i * NT + j) * 4 + e][lane] = acc[i][j][e];
-        __syncthreads();
+        if (__syncthreads_or(late)) {
+            if (late && lane == 0) atomicExch(status, 10);
+            for (int s = max(0, used - 1); s < sent; ++s) at_wait(bar + 8 * (s % SLOTS), (s / SLOTS) & 1);
+            break;
+        }
         if (tid < NT * 128 && ep_m < M && ep_r < a.height) {
             float lo = 0.f, hi = 0.f;
 #pragma unroll
