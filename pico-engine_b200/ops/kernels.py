@@ -474,15 +474,16 @@ def check_status(device) -> None:
 
 # A weight this large streams faster through the library's product even for a few rows where a CTA of the fused kernels would end with every
 # tile: measured on a B200 at 8 rows, 151936 x 896 (272 MB, into float32): 52 us against 72 us; 152064 x 3584: 178 us against 189 in the kernel that
-# keeps its ring full.  _streams names those that are faster here.
+# keeps its ring full.  _streams names those that are faster here.  PICO_ENGINE_FUSED_MAX_MB, where it is set, is the limit for all weights.
 FUSED_MAX_WEIGHT_BYTES = int(os.environ.get("PICO_ENGINE_FUSED_MAX_MB", "100")) << 20
+FUSED_MAX_IS_SET = "PICO_ENGINE_FUSED_MAX_MB" in os.environ
 
 
 def fused_takes(rows: int, w: torch.Tensor, *others: torch.Tensor, max_rows: int = FUSED_MAX_ROWS) -> bool:
     """Whether the fused decode kernels take a product with ``rows`` rows and weight ``w``."""
     return (rows <= max_rows and w.dtype == torch.bfloat16 and w.shape[1] % 8 == 0 and w.is_contiguous()
             and w.data_ptr() % 16 == 0 and all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in others)
-            and (w.numel() * 2 <= FUSED_MAX_WEIGHT_BYTES or (rows <= FUSED_MAX_ROWS and _streams(w, others))))
+            and (w.numel() * 2 <= FUSED_MAX_WEIGHT_BYTES or (not FUSED_MAX_IS_SET and rows <= FUSED_MAX_ROWS and _streams(w, others))))
 
 
 def _streams(w: torch.Tensor, others) -> bool:

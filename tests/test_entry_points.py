@@ -141,6 +141,22 @@ def test_command_line_generates_the_plain_tokens(tmp_path):
     assert [len(o["prompt"]) for o in outs] == [5, 9, 13] and all(len(o["output"]) == 8 for o in outs)
 
 
+@pytest.mark.parametrize("limit,want", [(None, [True, True, False, True]), ("100", [False, False, False, True]), ("8", [False] * 4),
+                                        ("600", [True] * 4)])
+def test_a_limit_on_fused_weights_holds_for_all_of_them(limit, want):
+    """PICO_ENGINE_FUSED_MAX_MB, where it is set, keeps every larger weight off the fused decode products; where it is not, weights of more than
+    100 MB are taken by the widths that stream."""
+    code = ("import torch\nfrom pico_engine.ops.kernels import fused_takes\n"
+            "m = lambda *n, dtype=torch.bfloat16: torch.empty(*n, dtype=dtype, device='meta')\n"
+            "print([fused_takes(8, m(37888, 3584), m(8, 3584, dtype=torch.float32)), fused_takes(8, m(3584, 18944), m(8, 18944)),"
+            " fused_takes(8, m(151936, 896), m(8, 896)), fused_takes(8, m(9728, 896), m(8, 896, dtype=torch.float32))])")
+    env = {k: v for k, v in os.environ.items() if k != "PICO_ENGINE_FUSED_MAX_MB"}
+    if limit is not None:
+        env["PICO_ENGINE_FUSED_MAX_MB"] = limit
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, env=env, capture_output=True, text=True)
+    assert r.returncode == 0 and json.loads(r.stdout.lower()) == want, r.stderr[-2000:]
+
+
 @pytest.mark.gpu
 def test_benchmark_command_line_writes_its_record(tmp_path):
     out = tmp_path / "record.json"
