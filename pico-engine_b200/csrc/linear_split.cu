@@ -58,6 +58,9 @@ template <int NT> constexpr int sp_threads() { return 32 * (SP_CUTTERS + 2 + sp_
 template <int NT> constexpr int sp_sent_bytes() { return NT == SP_MANY ? 0 : (NT + 8) * SP_ROWS * 4; }
 template <int NT> constexpr int sp_smem_bytes() { return sp_ring<NT>() * SP_BOX + SP_SLOTS * 2 * NT * SP_KC * 4 + sp_sent_bytes<NT>() + 1024; }
 
+// The status word of products captured into a graph before their device had one (pe_linear_split_gave_up reads it).
+static __device__ int sp_gave_up;
+
 // A CTA an SM where few rows of A stream the weights, and ranges of seven chunks at least: what a CTA does once (its first loads, the sum
 // over the cluster) takes as long as about six chunks.
 static int sp_ranges(int N, int K) {
@@ -162,7 +165,7 @@ __device__ __forceinline__ bool sp_wait(unsigned bar, unsigned parity, volatile 
         if (*abort_flag) return false;
         if (clock64() > deadline) {
             *abort_flag = 1;
-            if (status) atomicExch(status, 9);
+            atomicExch(status, 9);
             return false;
         }
     }
@@ -200,6 +203,7 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
     __shared__ unsigned tmem_base_s;
     __shared__ int abort_s;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (!status) status = &sp_gave_up;
     const unsigned smem = (at_smem(sp_raw) + 1023u) & ~1023u, a_parts = smem + RING * SP_BOX;
     const int rank = blockIdx.x % ranges, n0 = blockIdx.x / ranges * SP_ROWS, m0 = blockIdx.y * nt;
     const int all = (K + SP_KC - 1) / SP_KC, each = (all + ranges - 1) / ranges;
@@ -401,7 +405,7 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
             asm volatile("barrier.cluster.arrive.release;" ::: "memory");      // this CTA has sent
             if (rows > 0 && !sp_wait_sent(sent)) {
                 whole = false;
-                if (status) atomicExch(status, 9);
+                atomicExch(status, 9);
             }
         }
     }
@@ -489,6 +493,14 @@ extern "C" int pe_linear_split_takes(const void* W, int N, int K) { return N >= 
 // Rows of A that are cut at a time, so that their parts take 256 MB at most; and the bytes of scratch a product of M rows needs.
 static int sp_slab(int K) { return (int)((256ll << 20) / (8ll * K) > SP_MANY ? (256ll << 20) / (8ll * K) / SP_MANY * SP_MANY : SP_MANY); }
 extern "C" long long pe_linear_split_scratch(int M, int K) { return M <= 64 ? 0 : 8ll * K * (M < sp_slab(K) ? M : sp_slab(K)); }
+
+// What the word of products without one holds on the current device; it is zero again behind this.  Synchronises.
+extern "C" int pe_linear_split_gave_up(int* code) {
+    const int zero = 0;
+    PE_TRY(cudaMemcpyFromSymbol(code, sp_gave_up, sizeof(int)));
+    if (*code) PE_TRY(cudaMemcpyToSymbol(sp_gave_up, &zero, sizeof(int)));
+    return 0;
+}
 
 extern "C" int pe_linear_split(const void* A, const void* W, const void* bias, int bias_dtype, void* out, int epilogue, int M, int N, int K, void* scratch, void* status, void* stream) {
     if (M <= 0) return 0;

@@ -4,6 +4,7 @@ here with torch's allocator.  There is no other implementation behind these func
 """
 from __future__ import annotations
 
+import ctypes
 import os
 from dataclasses import dataclass
 from typing import Optional
@@ -458,9 +459,17 @@ def status_ptr(device) -> int:
     return ptr
 
 
+_captured_without_word = set()                            # devices
+
+
 def _status_ptr_or_none(device) -> Optional[int]:
-    """The same for a kernel that does without: no word is made while a graph is being captured."""
-    return None if device not in _status_ptrs and torch.cuda.is_current_stream_capturing() else status_ptr(device)
+    """The same for a kernel that has a word of its own: none is made while a graph is being captured."""
+    if device not in _status_ptrs and torch.cuda.is_current_stream_capturing():
+        from .workspace import has_scratch
+        if not has_scratch("status", torch.device(device)):
+            _captured_without_word.add(torch.device(device).index or 0)
+            return None
+    return status_ptr(device)
 
 
 def check_status(device) -> None:
@@ -469,6 +478,11 @@ def check_status(device) -> None:
     code = int(word.item())
     if code:
         word.zero_()
+    if (torch.device(device).index or 0) in _captured_without_word:
+        own = ctypes.c_int(0)
+        check(core().pe_linear_split_gave_up(ctypes.addressof(own)), "linear_split_gave_up", 0)
+        code = code or own.value
+    if code:
         raise KernelError(f"a kernel gave up a bounded wait (status {code}); its results are incomplete")
 
 

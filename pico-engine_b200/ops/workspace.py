@@ -29,3 +29,8 @@ def scratch(purpose: str, nbytes: int, device: torch.device, zeroed: bool = Fals
         torch.empty(size, dtype=torch.uint8, device=device)
     have.append(buf)
     return buf
+
+
+def has_scratch(purpose: str, device: torch.device) -> bool:
+    """Whether a buffer for ``purpose`` has been made on the device."""
+    return bool(_buffers.get((purpose, device.index or 0)))

@@ -2,6 +2,8 @@
 import math
 import os
 import random
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -689,6 +691,16 @@ def test_linear_float32_in_parts(K, N, K_):
         K.linear_simt(A[:M], W, accumulate_into=x)
         assert float((x.cpu().double() - want[:M] - 1).abs().max()) <= 8 * (K_ + 1) * 2.0 ** -24
         assert torch.equal(K.linear_simt(A[:M], W, B, out_dtype=torch.bfloat16), whole[:M].to(torch.bfloat16))
+
+
+def test_linear_float32_captured_first_of_all(K):
+    """A product whose capture is the first thing a process does runs, and its status can be asked for."""
+    code = ("import torch\nfrom pico_engine.ops import kernels as K\na, w = torch.randn(5, 896, device='cuda'), torch.randn(1024, 896, device='cuda')\n"
+            "g = torch.cuda.CUDAGraph()\nwith torch.cuda.graph(g):\n    out = K.linear_simt(a, w)\n"
+            "g.replay(); K.check_status('cuda'); K.check_status('cuda:0')\n"
+            "assert torch.allclose(out.double(), a.double() @ w.double().T, atol=1e-3)\nprint('fine')")
+    r = subprocess.run([sys.executable, "-c", code], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0 and "fine" in r.stdout, r.stderr[-2000:]
 
 
 @pytest.mark.parametrize("M", [3, 100])

@@ -194,3 +194,33 @@ def test_a_padded_step_is_described_with_idle_rows_and_a_fixed_number_of_runs():
         st.describe([b], [200], None, None, n_tiles=(2, 1))
     with pytest.raises(StepError, match="brings no token"):
         st.describe([b], [0], None, None)
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_a_wait_that_ran_out_in_a_graph_without_a_status_word_is_reported(monkeypatch, captured):
+    """A float32 product captured before its device has a status word records in a word of the library's own, which check_status reads too."""
+    import ctypes
+    own = [9]
+
+    class Core:
+        @staticmethod
+        def pe_linear_split_gave_up(at):
+            ctypes.c_int.from_address(at).value, own[0] = own[0], 0
+            return 0
+    monkeypatch.setattr(kernels, "core", Core)
+    monkeypatch.setattr(kernels, "_status_words", {})
+    monkeypatch.setattr(kernels, "_status_ptrs", {})
+    monkeypatch.setattr(kernels, "_captured_without_word", set())
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: captured)
+    monkeypatch.setattr("pico_engine.ops.workspace._buffers", {})
+    cpu = torch.device("cpu")
+    assert (kernels._status_ptr_or_none(cpu) is None) == captured
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    if captured:
+        with pytest.raises(kernels.KernelError, match="status 9"):
+            kernels.check_status("cpu")
+    kernels.check_status("cpu")
+    assert own == [0 if captured else 9]
+    # the word that exists is found under every name of its device
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+    assert kernels._status_ptr_or_none("cpu") == kernels._status_ptr_or_none(cpu) == kernels.status_word(cpu).data_ptr()
