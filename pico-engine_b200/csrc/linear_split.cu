@@ -493,6 +493,8 @@ extern "C" int pe_linear_split_takes(const void* W, int N, int K) { return N >= 
 // Rows of A that are cut at a time, so that their parts take 256 MB at most; and the bytes of scratch a product of M rows needs.
 static int sp_slab(int K) { return (int)((256ll << 20) / (8ll * K) > SP_MANY ? (256ll << 20) / (8ll * K) / SP_MANY * SP_MANY : SP_MANY); }
 extern "C" long long pe_linear_split_scratch(int M, int K) { return M <= 64 ? 0 : 8ll * K * (M < sp_slab(K) ? M : sp_slab(K)); }
+// The kernels that a product of M rows launches.
+extern "C" int pe_linear_split_launches(int M, int K) { return M <= 0 ? 0 : M <= 64 ? 1 : 2 * ((M + sp_slab(K) - 1) / sp_slab(K)); }
 
 // What the word of products without one holds on the current device; it is zero again behind this.  Synchronises.
 extern "C" int pe_linear_split_gave_up(int* code) {

@@ -172,7 +172,8 @@ def linear_simt(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] =
         nbytes = core().pe_linear_split_scratch(M, K)
         parts = torch.empty(nbytes, dtype=torch.uint8, device=a.device) if nbytes else None
         check(core().pe_linear_split(a.data_ptr(), w.data_ptr(), _ptr(bias), 0 if bias is None else _code(bias, "bias"), out.data_ptr(), epilogue,
-                                     M, N, K, _ptr(parts), _status_ptr_or_none(a.device), stream_ptr()), "linear_split")
+                                     M, N, K, _ptr(parts), _status_ptr_or_none(a.device), stream_ptr()), "linear_split",
+              core().pe_linear_split_launches(M, K))
         return out
     check(core().pe_linear_simt(a.data_ptr(), _code(a, "a"), w.data_ptr(), _code(w, "w"), _ptr(bias),
                                 0 if bias is None else _code(bias, "bias"), out.data_ptr(), epilogue, M, N, K,

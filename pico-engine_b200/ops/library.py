@@ -46,6 +46,7 @@ _SIGNATURES = {
     "pe_linear_simt": [P, I, P, I, P, I, P, I, I, I, I, P],
     "pe_linear_split_takes": [P, I, I],
     "pe_linear_split_gave_up": [P],
+    "pe_linear_split_launches": [I, I],
     "pe_linear_split": [P, P, P, I, P, I, I, I, I, P, P, P],
     "pe_attention_generic": [P, I, P, P, P, I, P, I, P, P, I, I, I, I, I, F, I, P, I, P],
     "pe_argmax": [P, P, I, I, P, P],

@@ -693,6 +693,16 @@ def test_linear_float32_in_parts(K, N, K_):
         assert torch.equal(K.linear_simt(A[:M], W, B, out_dtype=torch.bfloat16), whole[:M].to(torch.bfloat16))
 
 
+@pytest.mark.parametrize("M,kernels", [(1, 1), (64, 1), (65, 2), (130, 2), (200 * 1024 + 5, 4)])
+def test_linear_float32_counts_its_launches(K, M, kernels):
+    """One kernel for up to 64 rows; beyond, one that cuts the rows and one of products for every slab of them."""
+    from pico_engine.ops import library
+    a, w = torch.zeros(M, 256, device="cuda"), torch.zeros(3128, 256, device="cuda")
+    before = library.LAUNCHES[0]
+    K.linear_simt(a, w)
+    assert library.LAUNCHES[0] - before == kernels
+
+
 def test_linear_float32_captured_first_of_all(K):
     """A product whose capture is the first thing a process does runs, and its status can be asked for."""
     code = ("import torch\nfrom pico_engine.ops import kernels as K\na, w = torch.randn(5, 896, device='cuda'), torch.randn(1024, 896, device='cuda')\n"
