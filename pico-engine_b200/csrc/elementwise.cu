@@ -272,7 +272,8 @@ static int rmsnorm_launch(float* x, const TY* y, const int* rows_index, const vo
             return 0;
         }
         const int keep = H <= 1024 ? 2 : 4;
-        const int threads = H >= 8192 ? 512 : H <= 512 ? 64 : (H + 128 * keep - 1) / (128 * keep) * 32;
+        // Widths that are no multiple of four are read an element at a time: as many threads as such rows can use.
+        const int threads = (H & 3) ? (H >= 4096 ? 512 : H >= 1024 ? 256 : 128) : H >= 8192 ? 512 : H <= 512 ? 64 : (H + 128 * keep - 1) / (128 * keep) * 32;
         const bool wb = w_dtype == PE_BF16 && ((uintptr_t)w & 7) == 0 && (keep == 2 || !ADD || rows < 1024);
         auto* kernel = keep == 2 ? (wb ? rmsnorm_kernel<TO, TY, ADD, 2, true> : rmsnorm_kernel<TO, TY, ADD, 2, false>)
                                  : (wb ? rmsnorm_kernel<TO, TY, ADD, 4, true> : rmsnorm_kernel<TO, TY, ADD, 4, false>);
