@@ -144,7 +144,10 @@ __global__ void __launch_bounds__(32 * LS_WARPS, 1) linear_stream_kernel(const _
             for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.f;
         for (int c = warp; c < chunks; c += LS_WARPS) {
             const unsigned s = used % SLOTS, w_at = ring + s * SLOT;
-            const bool here = lf_bar_wait(bar + 8 * s, (used / SLOTS) & 1);
+            if (!lf_bar_wait(bar + 8 * s, (used / SLOTS) & 1)) {      // (the warp asks as one: a vote here costs a twentieth of the time)
+                late = true;
+                break;
+            }
             ++used;
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
@@ -161,7 +164,7 @@ __global__ void __launch_bounds__(32 * LS_WARPS, 1) linear_stream_kernel(const _
                     lf_mma(acc[1][j], h0.z, h1.z, h0.w, h1.w, v.z, v.w);
                 }
             }
-            if ((late = __any_sync(0xffffffffu, !here))) break;
+            __syncwarp();
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");             // the slot's reads precede its refill
             send();
         }
@@ -174,7 +177,7 @@ __global__ void __launch_bounds__(32 * LS_WARPS, 1) linear_stream_kernel(const _
                 for (int e = 0; e < 4; ++e) red[warp][(i * NT + j) * 4 + e][lane] = acc[i][j][e];
         if (__syncthreads_or(late)) {
             if (late && lane == 0) atomicExch(status, 10);
-            for (int s = max(0, used - 1); s < sent; ++s) at_wait(bar + 8 * (s % SLOTS), (s / SLOTS) & 1);
+            for (int s = used; s < sent; ++s) at_wait(bar + 8 * (s % SLOTS), (s / SLOTS) & 1);
             break;
         }
         if (tid < NT * 128 && ep_m < M && ep_r < a.height) {
