@@ -181,8 +181,9 @@ __global__ void __launch_bounds__(512, 2) rmsnorm_kernel(float* x, const TY* y, 
             }
         };
         constexpr bool early = WB || KEEP <= 2 || !ADD;
-        for (unsigned at = threadIdx.x * 128u, end = (unsigned)H * (w_dtype == PE_BF16 ? 2u : 4u); at < end; at += blockDim.x * 128u)
-            asm volatile("prefetch.global.L2 [%0];" ::"l"((const char*)w + at) : "memory");
+        if (blockIdx.x == 0)                                  // (by every block: 2,048 rows of 896 5.4 us, 3.3 so)
+            for (unsigned at = threadIdx.x * 128u, end = (unsigned)H * (w_dtype == PE_BF16 ? 2u : 4u); at < end; at += blockDim.x * 128u)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"((const char*)w + at) : "memory");
         pdl_wait();
         if (early) weights();
         const size_t src = rows_index ? rows_index[r] : r;
