@@ -260,13 +260,18 @@ static int ls_launch_nt(const CUtensorMap& map, const CUtensorMap& map_a, const 
 //                      gate/up 9728 x 1536  7.8 7.8 8.9 / 8.9 8.9 10.5           gate/up 16384 x 2048  20.0 19.8 22.3 / 13.5 14.0 16.5
 // and of more than 100 MB, the library's product with the passes around it / here: gate/up 37888 x 3584 51.9 52.3 52.6 / 44.0 45.4 49.8,
 // 3584 x 18944 30.4 30.9 30.9 / 22.9 23.2 30.9.
+// The lines of the rule lie where a grid of 152 shapes changes sides: normed rows, 33 rows of W a CTA or more (a second group of few rows keeps
+// too little under way), 6144 x 512 5.1 6.1 4.4 / 5.0 5.2 6.1, x 768 6.5 7.6 6.1 / 6.5 6.7 7.7, x 1024 7.6 8.8 7.3 / 7.3 7.4 8.4, x 3072 16.0 17.1 18.4 /
+// 15.7 16.4 18.4; fewer rows a CTA win from 1024 x 512 (3.2 3.6 3.8 / 2.6 2.7 3.5) to 4608 x 1024 (6.9 8.2 6.7 / 4.2 4.3 5.2).  bfloat16 rows: gate/up 4736 x 1024
+// 2.8 3.5 3.8 / 3.5 3.4 3.7, 2368 x 2048 3.9 4.0 4.9 / 4.6 4.5 5.2, 4736 x 1536 5.3 5.1 6.1 / 4.6 4.5 5.1; stored, 1280 x 512 2.6 2.3 2.5 / 1.8 1.7 1.8 to 4736 x 512
+// 3.1 3.2 3.0 / 2.3 2.3 2.4.  Taken although one row is slower: 4736 x 1024 2.9 3.0 4.3 / 3.5 3.4 3.7, 9500 x 512 3.7 3.7 5.7 / 4.5 4.4 5.0.
 static bool ls_takes(const LfArgs& p, bool norm, int epi) {
     const bool pairs = epi == LF_SWIGLU || epi == LF_ROPE;
     const long long entries = (long long)p.N * p.K;
     if (p.K < 512 || (norm && p.K > 4096) || (epi == LF_ROPE && p.hd % 8)) return false;
     const int rows = ((pairs ? p.N / 2 : p.N) + 147) / 148 * (pairs ? 2 : 1);      // of W, a CTA: up to 32 are one group
-    if (epi == LF_SWIGLU) return norm ? p.K >= 1024 || rows <= 32 : entries >= 25000000 || (rows <= 32 && entries >= 4000000);
-    if (norm) return p.N >= 1024;
+    if (epi == LF_SWIGLU) return norm ? p.K >= 1024 || rows <= 32 : entries >= 25000000 || (rows <= 32 && entries >= 6000000);
+    if (norm) return p.N >= 1024 && (rows <= 32 || p.K >= 1024);
     return rows >= 9 && (rows <= 32 || rows >= 64);        // (two groups of few rows keep too little under way)
 }
 
