@@ -179,6 +179,11 @@ __global__ void __launch_bounds__(AT_THREADS, R == 16 && NJ == 1 ? 2 : 1) attent
         if (left <= 0) return;
     }
     const int n_heads = min(a.heads, kvh * per + per - h0), n_tok = min(a.tokens, left);
+    if (member > 0) {                                      // one segment is the first member's: nobody waits for anybody
+        int lowest = a.tok_pos[t0], highest = lowest;
+        for (int t = 1; t < n_tok; ++t) { lowest = min(lowest, a.tok_pos[t0 + t]); highest = max(highest, a.tok_pos[t0 + t]); }
+        if ((a.window > 0 ? max(lowest - a.window + 1, 0) : 0) / (PE_PAGE * AG_SEGMENT) == highest / (PE_PAGE * AG_SEGMENT)) return;
+    }
     const int rows = n_heads * n_tok;                      // row r: token t0 + r / n_heads, head h0 + r % n_heads
     if (tid < R) {
         const int t = t0 + min(tid, rows - 1) / n_heads;
@@ -230,6 +235,7 @@ __global__ void __launch_bounds__(AT_THREADS, R == 16 && NJ == 1 ? 2 : 1) attent
         }
     };
     auto turn = [&](int j, int c, const float4& k) { kt[ag_turned(c, j)] = k.x; kt[ag_turned(c + 1, j)] = k.y; kt[ag_turned(c + 2, j)] = k.z; kt[ag_turned(c + 3, j)] = k.w; };
+    bool alone = true;                                     // no other CTA has a part in this block's rows
     for (int from = 0; from < rows;) {                     // the rows of one sequence that stand together, after them the next ones
         const int seq = row_s[from];
         int to = from + n_heads, lowest = pos_s[from], highest = lowest;
@@ -348,7 +354,8 @@ __global__ void __launch_bounds__(AT_THREADS, R == 16 && NJ == 1 ? 2 : 1) attent
                 for (int j = 0; j < NJ; ++j) acc[i][j] = make_float4(0.f, 0.f, 0.f, 0.f);
             }
         };
-        if (C == 1) {
+        alone = C == 1 || page_lo / AG_SEGMENT == page_hi / AG_SEGMENT;
+        if (alone) {
             int segment = -1;
             const auto join = [&]() {                      // the segment joins those before it
 #pragma unroll
@@ -398,12 +405,13 @@ __global__ void __launch_bounds__(AT_THREADS, R == 16 && NJ == 1 ? 2 : 1) attent
                 for (int j = 0; j < NJ; ++j)
                     if (tx * 4 + 64 * j < hd) *reinterpret_cast<float4*>(mine + 2 * R + ty * hd + tx * 4 + 64 * j) = acc[0][j];
                 ag_cluster_sync();
+                const int here_now = min(C, page_hi / AG_SEGMENT - page_lo / AG_SEGMENT + 1 - turns * C);
     #pragma unroll
                 for (int j = 0; j < NJ; ++j) {
                     const int i = member + C * (tid + j * AT_THREADS), r = i / per4, c = i % per4 * 4;
                     if (r >= rows) break;
     #pragma unroll 1
-                    for (int p0 = 0; p0 < C; p0 += 2) {        // (C is a power of two)
+                    for (int p0 = 0; p0 < here_now; p0 += 2) {     // (C is a power of two; who has no segment has seen nothing)
                         float ms[2], ls[2], before, now;
                         float4 vs2[2];
     #pragma unroll
@@ -426,7 +434,7 @@ __global__ void __launch_bounds__(AT_THREADS, R == 16 && NJ == 1 ? 2 : 1) attent
         const float inv = sum > 0.f ? 1.0f / sum : 0.f;
         ag_store4((T*)a.out + ((size_t)(t0 + r / n_heads) * a.nh + h0 + r % n_heads) * hd + c, make_float4(v.x * inv, v.y * inv, v.z * inv, v.w * inv));
     };
-    if (C > 1) {
+    if (!alone) {
 #pragma unroll
         for (int j = 0; j < NJ; ++j) {
             const int i = member + C * (tid + j * AT_THREADS);
@@ -454,10 +462,13 @@ static int attention_tile_as(AttentionTileArgs a, int n_runs, int most, cudaStre
     a.parts = (AG_RUN + a.tokens - 1) / a.tokens;
     if (a.runs) a.tokens = (AG_RUN + a.parts - 1) / a.parts;          // a whole run in equal parts
     const int blocks = a.runs ? n_runs * a.parts : (a.T + a.tokens - 1) / a.tokens;
-    // A cluster for each block of one sequence's rows where those leave SMs idle: as many CTAs as the longest context has segments.
+    // A cluster for each block of one sequence's rows where those leave SMs idle: as many CTAs as a context that fills its row of the page table
+    // has segments (how long contexts are is on the device; a captured step's tables are as wide as contexts may become).
+    // All of them fit at once, two an SM of heads of up to 64 and one of larger ones: eight tokens behind 200, 16 heads of 128 on 4, 46 us with clusters
+    // of eight, which do not.
     a.cluster = 1;
     if (R == 16 && (a.runs || a.tokens == 1))
-        while (a.cluster < 8 && (long long)2 * a.cluster * blocks * a.nkv * a.slices <= 2 * 148 && a.cluster * AG_SEGMENT < a.table_stride) a.cluster *= 2;
+        while (a.cluster < 8 && (long long)2 * a.cluster * blocks * a.nkv * a.slices <= (NJ == 1 ? 2 * 148 : 148) && a.cluster * AG_SEGMENT < a.table_stride) a.cluster *= 2;
     a.buffers = a.hd > 192 ? 1 : 2;
     const size_t smem = sizeof(float) * ((size_t)3 * a.hd * 64 + 64 * R + (a.cluster > 1 ? a.buffers * R * (a.hd + 2) : 0));
     auto kernel = attention_tile_kernel<T, R, NJ>;
