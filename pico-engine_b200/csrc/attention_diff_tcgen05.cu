@@ -59,7 +59,8 @@ __global__ void __launch_bounds__(DT_THREADS, 1) attention_diff_tcgen05_kernel(c
         if (threadIdx.x == 0) atomicExch(status, 6);
         return;
     }
-    // (the step's description and the page table: no kernel writes them)
+    // (the step's description and the page table are inputs like any other: the kernel in front may have written them)
+    pdl_wait();
     const int4 info = p.tiles[blockIdx.y];                          // heads vary fastest: the runs that see the most keys start first
     const int brow = info.x, tok0 = info.y, n = info.z, pos0 = info.w;
     const int per = p.H / p.G, h = blockIdx.x, g_kv = h / per;
@@ -100,7 +101,6 @@ __global__ void __launch_bounds__(DT_THREADS, 1) attention_diff_tcgen05_kernel(c
         asm volatile("fence.mbarrier_init.release.cluster;\n\tfence.proxy.async.shared::cta;" ::: "memory");
         // the queries and the first step are asked for before the block meets
         const int first[2] = {table[page_lo], 1 < n_pages ? table[page_lo + 1] : -1};
-        pdl_wait();
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(at_smem(&q_full)), "r"((unsigned)(2 * DT_PANEL)) : "memory");
 #pragma unroll
         for (int m = 0; m < 2; ++m) at_tma_2d(q_s + m * DT_PANEL, &map_q, ((2 * g_kv + m) * per + h % per) * p.D, tok0, at_smem(&q_full));
@@ -116,7 +116,6 @@ __global__ void __launch_bounds__(DT_THREADS, 1) attention_diff_tcgen05_kernel(c
     const unsigned tmem = tmem_base_s;
     // only now may the next kernel of the stream be scheduled: it could take tensor memory that a CTA of this grid still waits for
     pdl_launch_dependents();
-    pdl_wait();
 
     if (warp == 0) {
         if (lane == 0) {                                            // ---------------- loader

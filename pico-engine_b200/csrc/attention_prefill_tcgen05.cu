@@ -93,7 +93,8 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_prefill_tcgen05_kerne
         return;
     }
 
-    // (the step's description: no kernel writes it)
+    // (the step's description and the page table are inputs like any other: the kernel in front may have written them)
+    pdl_wait();
     const int4 info = p.tiles[blockIdx.y];                          // heads vary fastest: the runs that see the most keys start first
     const int brow = info.x, tok0 = info.y, n = info.z, pos0 = info.w;
     const int h = blockIdx.x, kvh = h / (p.nh / p.nkv);
@@ -130,7 +131,6 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_prefill_tcgen05_kerne
         asm volatile("fence.mbarrier_init.release.cluster;\n\tfence.proxy.async.shared::cta;" ::: "memory");
         // the queries and the first step are asked for before the block meets
         const int y[2] = {rows_of(table[page_at(0)]), rows_of(1 < n_pages ? table[page_at(1)] : -1)};
-        pdl_wait();
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(at_smem(&q_full)), "r"((unsigned)AT_Q_BYTES) : "memory");
 #pragma unroll
         for (int c = 0; c < AT_PANELS; ++c) at_tma_2d(q_s + c * (AT_QTILE * 128), &map_q, h * AT_HD + 64 * c, tok0, at_smem(&q_full));
@@ -148,7 +148,6 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_prefill_tcgen05_kerne
     // Only now may the next kernel of the stream be scheduled: if it came earlier, took tensor memory on this SM
     // and then waited for this grid to end, a CTA of this grid that still had to allocate would wait for it in turn.
     pdl_launch_dependents();
-    pdl_wait();
 
     if (warp == 0) {
         if (lane == 0) {                                            // ---------------- loader

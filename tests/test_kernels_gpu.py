@@ -595,6 +595,25 @@ def test_attention_causal_edge_inside_a_run(K, kernel, j):
     assert hit == [p >= j for p in range(n)], (kernel, j, [p for p in range(n) if hit[p] != (p >= j)][:6])
 
 
+def test_prefill_tcgen05_of_a_page_table_just_written(K):
+    """Pages and runs that the kernel in front writes: no entry is read before it is there."""
+    nh, nkv, hd, n = 4, 2, 64, 300
+    q, kp, vp = (dev(rnd(*s, seed=i).to(torch.bfloat16)) for i, s in enumerate([(n, nh * hd), (40, nkv, PAGE, hd), (40, nkv, PAGE, hd)]))
+    g = torch.Generator().manual_seed(9)
+    tables = [dev(torch.randperm(40, generator=g)[:5].to(torch.int32)) for _ in range(8)]
+    runs = K.prefill_tiles([n], [0], "cuda", K.PREFILL_TILE_TCGEN05)
+    src, all_runs = dev(torch.arange(5, dtype=torch.int32)), dev(torch.arange(runs.numel(), dtype=torch.int32))
+    run = lambda t, r: K.attention_prefill_tcgen05(q, nh * hd, nh, nkv, hd, kp, vp, t.view(1, 5), 5, r, n, None, hd ** -0.5)
+    want = [run(t, runs) for t in tables]
+    table, tiles = torch.zeros_like(tables[0]), torch.zeros_like(runs)
+    torch.cuda.synchronize()
+    got = [run(K.select_tokens(table, t, src), runs) for t in tables]
+    K.select_tokens(tiles.view(-1), runs.view(-1), all_runs)
+    got.append(run(tables[0], tiles))
+    assert all(torch.equal(a, b) for a, b in zip(got, want + want[:1]))
+    K.check_status("cuda")
+
+
 # ---------------------------------------------------------------------------- rotary encoding and the cache write
 
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])

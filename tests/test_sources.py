@@ -40,3 +40,11 @@ def test_streamed_decode_products_write_nothing_of_a_group_that_did_not_come():
     waits, told, writes = body.index("lf_bar_wait(bar"), body.index("__syncthreads_or("), body.index("p.out")
     assert waits < told < writes and "break;" in body[told:writes]
     assert body[waits:told].count("break;") == 1 and "late = true" in body[waits:told]
+
+
+@pytest.mark.parametrize("name", ["prefill", "diff", "headmix", "latent"])
+def test_prompt_kernels_read_nothing_before_the_kernel_in_front_has_ended(name):
+    """The step's runs and the page table are inputs like any other: a kernel in front may be writing them."""
+    with open(os.path.join(CSRC, f"attention_{name}_tcgen05.cu")) as f:
+        body = f.read().split("__global__", 1)[1]
+    assert body.index("pdl_wait();") < min(body.index(what) for what in ("p.tiles[", "p.block_table", "table["))
