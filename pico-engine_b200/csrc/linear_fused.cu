@@ -579,7 +579,7 @@ extern "C" int pe_linear_fused_scaled(const void* a, const float* x_norm, const 
                                       const void* W, const void* bias, int bias_dtype, void* out, int epilogue, float out_scale,
                                       int M, int N, int K, int* status, void* stream) {
     if (M <= 0 || N <= 0) return 0;
-    if (M > 16 || K <= 0 || K % 8 || epilogue < 0 || epilogue > 2 || !lf_aligned(W) || !lf_aligned(x_norm ? (const void*)x_norm : a))
+    if (M > 16 || K <= 0 || K % 8 || epilogue < 0 || epilogue > 2 || !lf_aligned(W) || !lf_aligned(x_norm ? (const void*)x_norm : a) || (x_norm && !lf_aligned(norm_w)))
         return PE_ERR_UNSUPPORTED;
     LfArgs p = {};
     p.A = (const bf16*)a; p.X = x_norm; p.norm_w = norm_w; p.norm_w_dtype = norm_w_dtype; p.eps = eps;
@@ -608,7 +608,7 @@ extern "C" int pe_linear_fused(const void* a, const float* x_norm, const void* n
 extern "C" int pe_norm_gate_up_swiglu(const float* x, const void* norm_w, int norm_w_dtype, float eps, const void* W,
                                       void* act, int M, int I, int K, int* status, void* stream) {
     if (M <= 0 || I <= 0) return 0;
-    if (M > 16 || K <= 0 || K % 8 || I % 8 || !lf_aligned(W) || !lf_aligned(x)) return PE_ERR_UNSUPPORTED;
+    if (M > 16 || K <= 0 || K % 8 || I % 8 || !lf_aligned(W) || !lf_aligned(x) || !lf_aligned(norm_w)) return PE_ERR_UNSUPPORTED;
     LfArgs p = {};
     p.X = x; p.norm_w = norm_w; p.norm_w_dtype = norm_w_dtype; p.eps = eps; p.W = (const bf16*)W; p.out = act;
     p.M = M; p.N = 2 * I; p.K = K; p.I = I; p.rows = 16;
@@ -634,7 +634,7 @@ extern "C" int pe_norm_qkv_rope_store(const void* a, const float* x, const void*
                                       const int* tok_pos, const int* tok_row, void* k_pool, void* v_pool,
                                       const int* block_table, int table_stride, int store, int* status, void* stream) {
     if (M <= 0) return 0;
-    if (M > 16 || K <= 0 || K % 8 || hd % 16 || !lf_aligned(W) || !lf_aligned(x ? (const void*)x : a)) return PE_ERR_UNSUPPORTED;
+    if (M > 16 || K <= 0 || K % 8 || hd % 16 || !lf_aligned(W) || !lf_aligned(x ? (const void*)x : a) || (x && !lf_aligned(norm_w))) return PE_ERR_UNSUPPORTED;
     LfArgs p = {};
     p.A = (const bf16*)a; p.X = x; p.norm_w = norm_w; p.norm_w_dtype = norm_w_dtype; p.eps = eps;
     p.W = (const bf16*)W; p.bias = bias; p.bias_dtype = bias_dtype; p.out = q_out; p.M = M; p.N = (n_q + 2 * n_kv) * hd;

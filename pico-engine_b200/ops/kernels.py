@@ -495,7 +495,7 @@ FUSED_MAX_IS_SET = "PICO_ENGINE_FUSED_MAX_MB" in os.environ
 
 
 def fused_takes(rows: int, w: torch.Tensor, *others: torch.Tensor, max_rows: int = FUSED_MAX_ROWS) -> bool:
-    """Whether the fused decode kernels take a product with ``rows`` rows and weight ``w``."""
+    """Whether the fused decode kernels take a product with ``rows`` rows and weight ``w``; ``others``: the rows, and the weights of their norm."""
     return (rows <= max_rows and w.dtype == torch.bfloat16 and w.shape[1] % 8 == 0 and w.is_contiguous()
             and w.data_ptr() % 16 == 0 and all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in others)
             and (w.numel() * 2 <= FUSED_MAX_WEIGHT_BYTES or (not FUSED_MAX_IS_SET and rows <= FUSED_MAX_ROWS and _streams(w, others))))

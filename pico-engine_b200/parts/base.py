@@ -172,7 +172,7 @@ def normed_rows(h, x_norm, ctx, w):
     from ..ops import kernels
     from .norm import RMSNorm
     x, norm = x_norm
-    if ctx.dtype == torch.bfloat16 and type(norm) is RMSNorm and kernels.fused_takes(x.shape[0], w, x):
+    if ctx.dtype == torch.bfloat16 and type(norm) is RMSNorm and kernels.fused_takes(x.shape[0], w, x, norm.weight):
         return None, x, norm.weight, norm.eps
     return norm.forward(x, ctx.dtype), None, None, 0.0
 

@@ -224,3 +224,21 @@ def test_a_wait_that_ran_out_in_a_graph_without_a_status_word_is_reported(monkey
     # the word that exists is found under every name of its device
     monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
     assert kernels._status_ptr_or_none("cpu") == kernels._status_ptr_or_none(cpu) == kernels.status_word(cpu).data_ptr()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_norm_weights_that_do_not_start_on_a_boundary_stay_out_of_the_fused_products(dtype):
+    """The fused decode products read sixteen bytes of the norm's weights at a time: a view that starts beside a boundary is normed apart, and the
+    entry points refuse it before they launch anything."""
+    from pico_engine.ops.library import core
+    w, x = torch.empty(2048, 1024, dtype=torch.bfloat16), torch.empty(4, 1024)
+    buf = torch.empty(1040, dtype=dtype)
+    assert w.data_ptr() % 16 == x.data_ptr() % 16 == buf.data_ptr() % 16 == 0
+    assert kernels.fused_takes(4, w, x, buf[:1024]) and not kernels.fused_takes(4, w, x, buf[1:1025])
+    word, code = torch.zeros(4, dtype=torch.int32), 0 if dtype == torch.float32 else 1
+    odd = buf[1:1025].data_ptr()
+    args = (4, 2048, 1024, word.data_ptr(), None)
+    assert core().pe_linear_fused(None, x.data_ptr(), odd, code, 1e-6, w.data_ptr(), None, 0, x.data_ptr(), 0, *args) == 10001
+    assert core().pe_norm_gate_up_swiglu(x.data_ptr(), odd, code, 1e-6, w.data_ptr(), x.data_ptr(), 4, 1024, 1024, word.data_ptr(), None) == 10001
+    assert core().pe_norm_qkv_rope_store(None, x.data_ptr(), odd, code, 1e-6, w.data_ptr(), None, 0, x.data_ptr(), 4, 1024, 14, 1, 128, None, None, None, None,
+                                         None, None, None, 0, 0, word.data_ptr(), None) == 10001
