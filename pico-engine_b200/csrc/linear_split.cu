@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
     extern __shared__ unsigned char sp_raw[];
     __shared__ __align__(8) unsigned long long bars[2 * RING + 3 * SP_SLOTS + 2 * SUMS + 1];
     __shared__ unsigned tmem_base_s;
-    __shared__ int abort_s;
+    __shared__ int abort_s, odd_s;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (!status) status = &sp_gave_up;
     const unsigned smem = (at_smem(sp_raw) + 1023u) & ~1023u, a_parts = smem + RING * SP_BOX;
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sent), "r"((unsigned)((ranges - 1) * rows * SP_ROWS * 4)) : "memory");
         }
         asm volatile("fence.mbarrier_init.release.cluster;\n\tfence.proxy.async.shared::cta;" ::: "memory");
-        abort_s = 0;
+        abort_s = odd_s = 0;
     }
     const auto bring_w = [&](int c) {                      // rows and entries behind the last are zeros
         const int s = c % RING;
@@ -376,15 +376,26 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
                 zero = fmaf(v, 0.f, zero);
                 asm volatile("st.shared.f32 [%0], %1;" ::"r"(smem + ((column0 + i) * SP_ROWS + row) * 4), "f"(v) : "memory");
             }
+        if (zero != 0.f && n < N) odd_s = 1;
+    }
+    __syncthreads();
+    if (odd_s) {                                           // sums that are not finite, a warp each, all warps a share
 #pragma unroll 1
-        for (int i = 0; i < (zero != 0.f && n < N ? min(columns, M - m0 - column0) : 0); ++i) {
-            const unsigned at = smem + ((column0 + i) * SP_ROWS + row) * 4;
+        for (int i = warp; i < 4 * min(nt, M - m0); i += sp_threads<NT>() / 32) {
+            const unsigned at = smem + ((i >> 2) * SP_ROWS + (i & 3) * 32 + lane) * 4;
+            const float* a = A + (size_t)(m0 + (i >> 2)) * K;
             float v;
             asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
-            if (isfinite(v)) continue;
-            v = 0.f;
-            for (int k = k_begin; k < k_end; ++k) v = fmaf(A[(size_t)(m0 + column0 + i) * K + k], W[(size_t)n * K + k], v);
-            asm volatile("st.shared.f32 [%0], %1;" ::"r"(at), "f"(v) : "memory");
+            unsigned odd = __ballot_sync(0xffffffffu, !isfinite(v) && n0 + (i & 3) * 32 + lane < N);
+#pragma unroll 1
+            for (; odd; odd &= odd - 1) {
+                const float* w = W + (size_t)(n0 + (i & 3) * 32 + __ffs(odd) - 1) * K;
+                float sum = 0.f;
+#pragma unroll 4
+                for (int k = k_begin + lane; k < k_end; k += 32) sum = fmaf(a[k], w[k], sum);
+                sum = warp_sum(sum);
+                if (lane == __ffs(odd) - 1) asm volatile("st.shared.f32 [%0], %1;" ::"r"(at), "f"(sum) : "memory");
+            }
         }
     }
     const unsigned sums_sent = a_parts + SP_SLOTS * 2 * part_bytes;       // [rank][slice][128]
