@@ -1,37 +1,44 @@
 // out[M, N] = A[M, K] . W[N, K]^T (+ bias[N]) for float32 operands on the 5th-generation tensor cores, at float32 accuracy.
 //
-// Every operand is cut in two, x = hi + lo: hi the eleven leading bits, rounded to nearest, and lo what is left, of which the tensor core
-// takes another eleven.  hi hi, hi lo and lo hi are multiplied on tcgen05.mma (kind::tf32, products exact in float32); what is left out
-// is of either sign and below 2^-23 of a product.  The tensor core's own sums are not rounded to nearest, so they are kept short: 32
-// entries of K, the small products first, into an accumulator that starts at zero; the sums of these chunks are added in registers, in
-// float32 to nearest.  Relative error (2-norm) against float64, beside that of a chain of multiply-adds (linear_simt.cu): 896 entries of
-// K 1.5e-7 (2.7e-7 to 3.8e-7), 3,584 1.6e-7 (7.6e-7), 4,864 1.6e-7 (4.4e-7); all entries positive 1.4e-7 (1.2e-7), 1.4e-7 (4.6e-7) and
-// 1.4e-7 (1.4e-7).  With 64 entries an accumulator the products took a twentieth less time, but positive ones were 2.8e-7 off.
+// Every operand is cut in three bfloat16 numbers, x = hi + mid + lo, which together hold its 24 bits.  Six of the nine products of parts are
+// multiplied on tcgen05.mma (kind::f16, products exact in float32); mid lo, lo mid and lo lo are left out, of either sign and together at
+// most 2^-24 of a product (2^-28 as a root mean square).  The tensor core's sums are not rounded to nearest: addends lose what lies 2^-25
+// below the largest, results are cut to 24 bits.  So hi hi, 16 bits a product, is summed over 32 entries of K at a time into an accumulator that
+// starts at zero, and these sums are added in registers, in float32 to nearest; the small products, a 256th of it, have an accumulator of
+// their own for all of a CTA's K.  The product with a power of two is exact.
+// Error against float64, here / a chain of multiply-adds (linear_simt.cu), relative 2-norm, 60 rows of A:
+//               3,200 x 256      896 x 896        9,728 x 896      896 x 4,864      3,584 x 3,584    3,584 x 18,944
+//   normal      7.3e-8 / 2.0e-7  8.1e-8 / 2.7e-7  1.1e-7 / 3.8e-7  1.1e-7 / 4.4e-7  1.1e-7 / 7.6e-7  2.2e-7 / 1.7e-6
+//   positive    6.4e-8 / 1.2e-7  5.2e-8 / 1.1e-7  8.5e-8 / 2.1e-7  6.6e-8 / 1.4e-7  6.2e-8 / 4.2e-7  8.4e-8 / 1.0e-6
+//   one term    2.6e-8 / 2.5e-8  2.6e-8 / 2.5e-8  2.6e-8 / 2.5e-8  2.6e-8 / 2.6e-8  2.6e-8 / 2.5e-8  2.6e-8 / 2.5e-8   (largest 1.7 / 1.0 x 2^-24)
+//   four terms  2.7e-8 / 4.1e-8  4.2e-8 / 4.5e-8  2.7e-8 / 4.2e-8  4.5e-8 / 4.6e-8  4.4e-8 / 4.2e-8  4.3e-8 / 4.2e-8
+// An entry below 2^-110 (7.7e-34) that is not the sum of three bfloat16 numbers is marked by a part that is no number.
 //
 // K is cut into ranges whose number depends on N and K only, a CTA each; the ranges of a tile are a cluster that adds its sums up in
 // their order (up to 64 rows of A each CTA sends the others their rows' sums, and none waits for another to read them: 0.7 to 1.1 us less
 // than reading them between two cluster barriers).  How many rows of A a tile has depends on M but changes no sum: a row's result does not depend on the rows beside it.
 //
 // A CTA: 128 rows of W (the accumulator's lanes) x up to 128 rows of A (its columns).
-//   warps 0-7  two groups that take the chunks in turn: a thread reads its row of W from the ring in shared memory, cuts it and stores
-//              both parts to tensor memory, where the products read them (an operand in shared memory would be read twelve times a chunk:
-//              with W there the tensor core waited for shared memory, 1,450 to 2,000 cycles a chunk of 112 rows of A); up to 64
-//              rows of A are cut here too and go to shared memory
-//   warp 8     issues a chunk's twelve products
-//   warp 9     brings W (float32) by TMA, into L2 as far as the ring goes before the kernel waits for its predecessor; more than 64 rows of A
-//              have been cut by a kernel before this one and come by TMA as well
-//   warps 10-  take the sums out of tensor memory
-// Bound by the tensor core and the hand-over of its sums: a chunk of 112 rows of A takes 1,150 cycles, its products alone 980.
+//   cutting    two groups of four warps, or four, that take the chunks in turn: a thread reads its row of W from the ring in shared memory, cuts it
+//              and stores the parts to tensor memory, where the products read them (an operand in shared memory would be read twelve times a
+//              chunk); up to 64 rows of A are cut here too and go to shared memory
+//   products   a warp issues a chunk's twelve
+//   loads      a warp brings W (float32) by TMA, into L2 as far as the ring goes before the kernel waits for its predecessor; more than 64 rows of
+//              A have been cut by a kernel before this one and come by TMA as well
+//   sums       4 or 16 warps take the sums of hi hi out of tensor memory
+// Bound by the hand-overs between them: 508 rows, 9,728 x 896, a chunk of 112 rows of A takes 1,700 cycles, the tensor pipe is busy for a third
+// of it, the issue slots for half.  Leaving out two thirds of the products, the cutting or the reading of sums saves 3 to 7 % each.
 //
 // One B200, W read from memory, us, here / in linear_simt.cu (the only way before): rows of A 1 12 60 130 508
-//   1,152 x 896   4.8 / 5.5     5.1 / 7.7    7.1 / 12.2   10.0 / 21.7   20.9 / 34.8
-//     896 x 896   4.8 / 5.0     5.1 / 6.9    6.9 / 12.2    9.7 / 19.2   13.3 / 28.5
-//   9,728 x 896  12.2 / 12.8   13.4 / 27.2  16.4 / 51.0   40.0 / 84.3   68.1 / 208
-//     896 x 4864  9.2 / 11.4    9.9 / 20.4  12.0 / 29.9   19.0 / 64.5   42.9 / 111
-//   3,584 x 3584 20.2 / 28.7   22.4 / 50.3  27.9 / 77.3   56.2 / 176.8  108 / 316
+//   1,152 x 896   5.4 / 5.5     5.6 / 7.7    7.9 / 12.2   11.1 / 21.7   24.5 / 34.8
+//     896 x 896   5.4 / 5.8     5.6 / 7.6    7.9 / 13.1   10.8 / 25.5   15.1 / 28.0
+//   9,728 x 896  13.8 / 12.8   14.1 / 27.2  19.0 / 51.0   46.9 / 84.3   76.8 / 208
+//     896 x 4864 10.0 / 11.4   10.2 / 20.4  13.5 / 29.9   21.4 / 64.5   50.2 / 111
+//   3,584 x 3584 24.6 / 28.7   25.0 / 50.3  32.3 / 77.3   65.1 / 176.8  133 / 316
 //
-// Infinities, values that are no number and sums beyond float32 leave results that are not finite; those are worked out again with plain
-// multiply-adds.
+// Infinities, values that are no number, marked entries and sums beyond float32 leave results that are not finite; those are worked out again with
+// plain multiply-adds, a warp a result (one thread a result, down the columns of W, took 812 us where 60 rows meet an infinity in a weight of 9,728 x
+// 896, and 30 ms where 508 rows hold no number; 36 us and 2.8 ms so).
 //
 // Every wait is bounded by the clock; one that runs out sets *status to 9 and a flag that lets every other role leave its loop.  The CTA
 // then waits (with a limit again) for the copies and products it has under way, stores nothing, and takes the same steps with its cluster as
@@ -41,22 +48,33 @@
 // pico-engine leaves these products to cuBLAS (src/pico_engine/model.py:177, 213, 223, 235, 164).
 #include "tcgen05_attention.cuh"
 
-#define SP_KC 32                                           // entries of K of a chunk: one row of the 128-byte swizzle
+#define SP_KC 32                                           // entries of K of a chunk: as float32 a row of the 128-byte swizzle, as bfloat16 one of the 64-byte one
+#define SP_PARTS 3
+#define SP_W_COLS (SP_PARTS * SP_KC / 2)                   // columns of tensor memory of a chunk's parts of W
 #define SP_ROWS 128                                        // rows of W of a tile
 #define SP_BOX (SP_ROWS * SP_KC * 4)
-#define SP_CUTTERS 8
-#define SP_SLOTS 4                                         // chunks whose parts are in tensor memory and, of A, in shared memory
+#define SP_SLOTS 4                                         // chunks at most whose parts are in tensor memory and, of A, in shared memory
 #define SP_MANY 128                                        // NT of the form for many rows of A
 #define SP_TMEM 512
 
 // W in shared memory, chunks; sums in tensor memory, chunks; warps that take them
-template <int NT> constexpr int sp_ring() { return NT == SP_MANY ? 5 : NT == 64 ? 6 : 8; }
+template <int NT> constexpr int sp_ring() { return 8; }
 template <int NT> constexpr int sp_sums() { return NT == SP_MANY ? 2 : 4; }
 template <int NT> constexpr int sp_takers() { return NT == SP_MANY ? 16 : 4; }
-template <int NT> constexpr int sp_threads() { return 32 * (SP_CUTTERS + 2 + sp_takers<NT>()); }
+// Warps that cut, four a chunk, in turns of two groups or four (few rows of A wait for W to be cut: 12 rows, 3,584 x 3584 27.0 us with two groups, 24.4;
+// 60 rows, whose sums take more registers, 31.5 and with three groups 35.2).
+template <int NT> constexpr int sp_cutters() { return NT <= 32 ? 16 : 8; }
+template <int NT> constexpr int sp_threads() { return 32 * (sp_cutters<NT>() + 2 + sp_takers<NT>()); }
 // (few rows of A: a place of its own for the sums that the other CTAs of a cluster send, up to 8 x ceil(NT / 8) rows)
 template <int NT> constexpr int sp_sent_bytes() { return NT == SP_MANY ? 0 : (NT + 8) * SP_ROWS * 4; }
-template <int NT> constexpr int sp_smem_bytes() { return sp_ring<NT>() * SP_BOX + SP_SLOTS * 2 * NT * SP_KC * 4 + sp_sent_bytes<NT>() + 1024; }
+// Parts of W, two accumulators of the large products and one of the small ones share 512 columns.
+__host__ __device__ constexpr int sp_slots(int nt) { return nt > 112 ? 2 : nt > 96 ? 3 : SP_SLOTS; }
+template <int NT> constexpr int sp_smem_bytes() { return sp_ring<NT>() * SP_BOX + (NT == SP_MANY ? SP_SLOTS * 96 : SP_SLOTS * NT) * SP_PARTS * SP_KC * 2 + sp_sent_bytes<NT>() + 1024; }
+static_assert(sp_slots(128) * SP_W_COLS + 3 * 128 <= SP_TMEM && sp_slots(112) * SP_W_COLS + 3 * 112 <= SP_TMEM && SP_SLOTS * SP_W_COLS + 3 * 96 <= SP_TMEM &&
+              SP_SLOTS * SP_W_COLS + 5 * 64 <= SP_TMEM && sp_slots(128) * 128 <= SP_SLOTS * 96 && sp_slots(112) * 112 <= SP_SLOTS * 96, "room for the parts and the sums");
+// A group that waits for a slot's n-th products knows that those before them have ended (or the parity would not tell them apart) from its own
+// turn before: groups must not outnumber slots.
+static_assert(sp_cutters<SP_MANY>() / 4 <= sp_slots(128) && sp_cutters<64>() / 4 <= SP_SLOTS && sp_cutters<16>() / 4 <= SP_SLOTS, "a slot for every group");
 
 // The status word of products captured into a graph before their device had one (pe_linear_split_gave_up reads it).
 static __device__ int sp_gave_up;
@@ -87,44 +105,71 @@ __device__ __forceinline__ float4 sp_shared_four(unsigned at) {
     asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
     return v;
 }
-__device__ __forceinline__ void sp_put_four(unsigned at, const float* v) {
-    asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(at), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
+__device__ __forceinline__ void sp_put_four(unsigned at, const unsigned* v) {
+    asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(at), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
 }
 __device__ __forceinline__ void sp_load8(float (&v)[8], const float* p) {
     asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "l"(p) : "memory");
-}
-// (of an infinity or no number a lo is left that is no number)
-__device__ __forceinline__ float sp_hi(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u); }
-
-__device__ __forceinline__ unsigned sp_elect() {
-    unsigned r;
-    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(r));
-    return r;
-}
-// The twelve products of a chunk, four steps of eight entries each: lo hi and hi lo, then hi hi, into an accumulator that starts at zero.
-// w: columns of tensor memory, 32 of hi and 32 of lo; a, a_lo: descriptors.  The whole warp calls; the elected thread issues.
-__device__ __forceinline__ void sp_products(unsigned elected, unsigned d, unsigned w, unsigned long long a, unsigned long long a_lo, unsigned idesc) {
-#define SP_MMA(wt, ad, p) " @e tcgen05.mma.cta_group::1.kind::tf32 [%1], [" wt "], " ad ", %10, " p ";\n"
-    asm volatile("{\n .reg .pred yes, no, e;\n .reg .b32 h1, h2, h3, l0, l1, l2, l3;\n"
-                 " setp.eq.u32 yes, 0, 0;\n setp.ne.u32 no, 0, 0;\n setp.ne.u32 e, %0, 0;\n"
-                 " add.u32 h1, %11, 8;\n add.u32 h2, %11, 16;\n add.u32 h3, %11, 24;\n add.u32 l0, %11, 32;\n add.u32 l1, %11, 40;\n add.u32 l2, %11, 48;\n add.u32 l3, %11, 56;\n"
-                 SP_MMA("l0", "%2", "no") SP_MMA("l1", "%3", "yes") SP_MMA("l2", "%4", "yes") SP_MMA("l3", "%5", "yes")
-                 SP_MMA("%11", "%6", "yes") SP_MMA("h1", "%7", "yes") SP_MMA("h2", "%8", "yes") SP_MMA("h3", "%9", "yes")
-                 SP_MMA("%11", "%2", "yes") SP_MMA("h1", "%3", "yes") SP_MMA("h2", "%4", "yes") SP_MMA("h3", "%5", "yes")
-                 "}"
-                 ::"r"(elected), "r"(d), "l"(a), "l"(a + 2), "l"(a + 4), "l"(a + 6), "l"(a_lo), "l"(a_lo + 2), "l"(a_lo + 4), "l"(a_lo + 6), "r"(idesc), "r"(w) : "memory");
-#undef SP_MMA
 }
 __device__ __forceinline__ unsigned long long sp_pair(unsigned a, unsigned b) {
     unsigned long long r;
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b));
     return r;
 }
-__device__ __forceinline__ void sp_st16(unsigned taddr, const float (&v)[16]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-                 ::"r"(taddr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]), "f"(v[9]), "f"(v[10]), "f"(v[11]), "f"(v[12]),
-                   "f"(v[13]), "f"(v[14]), "f"(v[15]) : "memory");
+// Two neighbouring entries as their parts (of an infinity or no number, parts that are no numbers are left).
+__device__ __forceinline__ void sp_cut(float x, float y, unsigned& hi, unsigned& mid, unsigned& lo) {
+    unsigned long long rest = at_two(x, y);
+    const unsigned long long minus = at_two(-1.f, -1.f);
+    hi = at_pack(x, y);
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(rest) : "l"(sp_pair(hi << 16, hi & 0xffff0000u)), "l"(minus));      // (exact)
+    float2 r = at_both(rest);
+    mid = at_pack(r.x, r.y);
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(rest) : "l"(sp_pair(mid << 16, mid & 0xffff0000u)), "l"(minus));
+    r = at_both(rest);
+    lo = at_pack(r.x, r.y);
+}
+// Entries below this may not be the sum of three bfloat16 numbers (the last would lie below 2^-133).
+#define SP_SMALL 0x1p-110f
+// The first parts of a pair in which an entry that its parts are not the sum of is marked by one that is no number, so that its results are
+// not finite and are worked out again with multiply-adds.
+__device__ __noinline__ unsigned sp_marked(float x, float y) {
+    unsigned hi, mid, lo;
+    sp_cut(x, y, hi, mid, lo);
+    const float a = (__uint_as_float(hi << 16) + __uint_as_float(mid << 16)) + __uint_as_float(lo << 16);
+    const float b = (__uint_as_float(hi & 0xffff0000u) + __uint_as_float(mid & 0xffff0000u)) + __uint_as_float(lo & 0xffff0000u);
+    return (a == x ? hi & 0xffffu : 0x7fffu) | (b == y ? hi & 0xffff0000u : 0x7fff0000u);
+}
+__device__ __forceinline__ void sp_least(float& least, float x, float y) { asm("min.abs.f32 %0, %0, %1, %2;" : "+f"(least) : "f"(x), "f"(y)); }
+// operand descriptor of the 64-byte swizzle: rows of 64 bytes, eight of them every 512
+__device__ __forceinline__ unsigned long long sp_desc(unsigned at) {
+    return (unsigned long long)((at >> 4) & 0x3FFFu) | (1ull << 16) | ((unsigned long long)(512 >> 4) << 32) | (1ull << 46) | (4ull << 61);
+}
+
+__device__ __forceinline__ unsigned sp_elect() {
+    unsigned r;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(r));
+    return r;
+}
+// The twelve products of a chunk, two steps of sixteen entries each.  hi hi go to `large`, an accumulator that starts at zero with every chunk, the
+// small ones to `small`, which starts with the first chunk (`more`: this is a later one).
+// w: columns of tensor memory, 16 of hi, of mid and of lo; a, a_mid, a_lo: descriptors.  The whole warp calls; the elected thread issues.
+__device__ __forceinline__ void sp_products(unsigned elected, unsigned large, unsigned small, unsigned w, unsigned long long a, unsigned long long a_mid, unsigned long long a_lo,
+                                            unsigned idesc, unsigned more) {
+#define SP_MMA(d, wt, ad, p) " @e tcgen05.mma.cta_group::1.kind::f16 [" d "], [" wt "], " ad ", %10, " p ";\n"
+    asm volatile("{\n .reg .pred yes, no, e, f;\n .reg .b32 h1, m0, m1, l0, l1;\n"
+                 " setp.eq.u32 yes, 0, 0;\n setp.ne.u32 no, 0, 0;\n setp.ne.u32 e, %0, 0;\n setp.ne.u32 f, %11, 0;\n"
+                 " add.u32 h1, %3, 8;\n add.u32 m0, %3, 16;\n add.u32 m1, %3, 24;\n add.u32 l0, %3, 32;\n add.u32 l1, %3, 40;\n"
+                 SP_MMA("%2", "l0", "%4", "f") SP_MMA("%2", "l1", "%5", "yes") SP_MMA("%2", "%3", "%8", "yes") SP_MMA("%2", "h1", "%9", "yes")
+                 SP_MMA("%2", "m0", "%6", "yes") SP_MMA("%2", "m1", "%7", "yes") SP_MMA("%2", "m0", "%4", "yes") SP_MMA("%2", "m1", "%5", "yes")
+                 SP_MMA("%2", "%3", "%6", "yes") SP_MMA("%2", "h1", "%7", "yes") SP_MMA("%1", "%3", "%4", "no") SP_MMA("%1", "h1", "%5", "yes")
+                 "}"
+                 ::"r"(elected), "r"(large), "r"(small), "r"(w), "l"(a), "l"(a + 2), "l"(a_mid), "l"(a_mid + 2), "l"(a_lo), "l"(a_lo + 2), "r"(idesc), "r"(more) : "memory");
+#undef SP_MMA
+}
+__device__ __forceinline__ void sp_st8(unsigned taddr, const unsigned (&v)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                 ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
 }
 // acc (pairs of columns) += the first `columns` columns (a multiple of eight) of this thread's lane
 template <int COLS>
@@ -176,16 +221,28 @@ __device__ __forceinline__ bool sp_wait_warp(unsigned bar, unsigned parity, vola
     return __all_sync(0xffffffffu, sp_wait(bar, parity, abort_flag, status));
 }
 
-// Rows of A as their parts, [2][M][K], for tiles of many rows.
-__global__ void __launch_bounds__(256) split_rows_kernel(const float* A, float* parts, long long entries, int vec_a) {
+// Rows of A as their parts, [3][M][K], for tiles of many rows.
+__global__ void __launch_bounds__(256) split_rows_kernel(const float* A, bf16* parts, long long entries, int vec_a) {
     pdl_launch_dependents();
     pdl_wait();
-    const long long at = ((long long)blockIdx.x * 256 + threadIdx.x) * 4;
+    const long long at = ((long long)blockIdx.x * 256 + threadIdx.x) * 8;
     if (at >= entries) return;
-    const float4 v = vec_a ? *reinterpret_cast<const float4*>(A + at) : make_float4(A[at], A[at + 1], A[at + 2], A[at + 3]);
-    const float4 hi = make_float4(sp_hi(v.x), sp_hi(v.y), sp_hi(v.z), sp_hi(v.w));
-    *reinterpret_cast<float4*>(parts + at) = hi;
-    *reinterpret_cast<float4*>(parts + entries + at) = make_float4(v.x - hi.x, v.y - hi.y, v.z - hi.z, v.w - hi.w);
+    float v[8];
+    if (vec_a) {
+        const float4 lo = *reinterpret_cast<const float4*>(A + at), hi = *reinterpret_cast<const float4*>(A + at + 4);
+        v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w; v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = A[at + i];
+    }
+    unsigned part[SP_PARTS][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        sp_cut(v[2 * i], v[2 * i + 1], part[0][i], part[1][i], part[2][i]);
+        if (fminf(fabsf(v[2 * i]), fabsf(v[2 * i + 1])) < SP_SMALL) part[0][i] = sp_marked(v[2 * i], v[2 * i + 1]);
+    }
+#pragma unroll
+    for (int q = 0; q < SP_PARTS; ++q) *reinterpret_cast<uint4*>(parts + q * entries + at) = make_uint4(part[q][0], part[q][1], part[q][2], part[q][3]);
 }
 
 // NT rows of A a tile: 16, 32 or 64; or (SP_MANY) up to 128, `nt` of them, whose parts come by TMA.
@@ -194,10 +251,10 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
                                                                            const float* W, const void* bias, int bias_dtype, void* out, int epilogue, int M, int N, int K,
                                                                            int ranges, int nt, int vec_a, int* status) {
     constexpr bool MANY = NT == SP_MANY;
-    constexpr int RING = sp_ring<NT>(), SUMS = sp_sums<NT>(), TAKER = SP_CUTTERS + 2, COLS = NT * 4 / sp_takers<NT>();
-    constexpr int TPT = NT >= 32 ? NT / 32 : 1, GROUPS = SP_CUTTERS / 4;      // TPT: runs of eight entries of A a thread cuts
+    constexpr int RING = sp_ring<NT>(), SUMS = sp_sums<NT>(), CUTTERS = sp_cutters<NT>(), TAKER = CUTTERS + 2, COLS = NT * 4 / sp_takers<NT>();
+    constexpr int TPT = NT >= 32 ? NT / 32 : 1, GROUPS = CUTTERS / 4;      // TPT: runs of eight entries of A a thread cuts
     if (!MANY) nt = NT;
-    const int part_bytes = nt * SP_KC * 4;
+    const int part_bytes = nt * SP_KC * 2, slots = MANY ? sp_slots(nt) : SP_SLOTS;
     extern __shared__ unsigned char sp_raw[];
     __shared__ __align__(8) unsigned long long bars[2 * RING + 3 * SP_SLOTS + 2 * SUMS + 1];
     __shared__ unsigned tmem_base_s;
@@ -213,15 +270,15 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
     // the rows of A whose sums over the cluster this CTA finishes
     const int slice = (nt + ranges - 1) / ranges, first_row = rank * slice, rows = max(0, min(min(nt, first_row + slice), M - m0) - first_row);
 
-    if (warp == SP_CUTTERS) {
+    if (warp == CUTTERS) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(at_smem(&tmem_base_s)), "r"((unsigned)SP_TMEM) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    if (tid == 32 * (SP_CUTTERS + 1)) {
+    if (tid == 32 * (CUTTERS + 1)) {
         const auto init = [](unsigned bar, int count, unsigned arrivals) {
             for (int i = 0; i < count; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar + 8 * i), "r"(arrivals) : "memory");
         };
-        init(w_full, RING, 1); init(w_empty, RING, 4); init(full, SP_SLOTS, 4); if (MANY) init(a_full, SP_SLOTS, 1); init(empty, SP_SLOTS, 1); init(sum_full, SUMS, 1); init(sum_empty, SUMS, sp_takers<NT>());
+        init(w_full, RING, 1); init(w_empty, RING, 4); init(full, SP_SLOTS, 4); init(a_full, SP_SLOTS, 1); init(empty, SP_SLOTS, 1); init(sum_full, SUMS, 1); init(sum_empty, SUMS, sp_takers<NT>());
         if (!MANY) {
             init(sent, 1, 1);
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sent), "r"((unsigned)((ranges - 1) * rows * SP_ROWS * 4)) : "memory");
@@ -238,23 +295,23 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (!MANY && ranges > 1) asm volatile("barrier.cluster.arrive.release;" ::: "memory");      // this CTA can be sent to
-    const unsigned tmem = tmem_base_s, sums = tmem + SP_SLOTS * 2 * SP_KC;
+    const unsigned tmem = tmem_base_s, sums = tmem + slots * SP_W_COLS, small = sums + SUMS * nt;
     pdl_launch_dependents();                               // (behind the allocation of tensor memory: a later kernel must not take it first)
     // W may be what the kernel in front writes: until that has ended it is only brought as far as L2, where its writes arrive too
-    if (tid == 32 * (SP_CUTTERS + 1))
+    if (tid == 32 * (CUTTERS + 1))
         for (int c = 0; c < min(RING, chunks); ++c)
             asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(&map_w), "r"(k_begin + c * SP_KC), "r"(n0) : "memory");
     pdl_wait();
-    if (tid == 32 * (SP_CUTTERS + 1))
+    if (tid == 32 * (CUTTERS + 1))
         for (int c = 0; c < min(RING, chunks); ++c) bring_w(c);
 
     unsigned long long acc[COLS / 2];                      // pairs of columns
     const int column0 = MANY ? ((warp - TAKER) >> 2) * COLS : 0, columns = MANY ? max(0, min(COLS, nt - column0)) : NT;
-    if (warp < SP_CUTTERS) {
+    if (warp < CUTTERS) {
         const int row = tid & 127, lr = row >> 2, lk = (tid & 3) * 8;
         const unsigned lanes = (unsigned)((warp & 3) * 32) << 16;
-        // entry k of a row: 16-byte groups exchanged by the row's place in its run of eight
-        const unsigned first = lr * 128 + ((((unsigned)lk >> 2) ^ (lr & 7)) << 4), second = first ^ 16u;
+        // entries k .. k + 7 of a row are 16 bytes; the four groups of a row are exchanged by half its place in a run of eight
+        const unsigned group = lr * 64 + ((((unsigned)lk >> 3) ^ ((lr >> 1) & 3)) << 4);
         float ra[TPT][8];
         auto fetch_a = [&](int c) {                        // rows behind the last are read as the last and not stored (K is a multiple of eight)
             const int k = k_begin + c * SP_KC + lk;
@@ -270,55 +327,89 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
         };
         if (!MANY && (warp >> 2) < chunks) fetch_a(warp >> 2);
         for (int c = warp >> 2; c < chunks; c += GROUPS) {
-            const int r = c % RING, s = c % SP_SLOTS;
+            const int r = c % RING, s = c % slots;
             if (!sp_wait_warp(w_full + 8 * r, (c / RING) & 1, &abort_s, status)) break;
-            if (c >= SP_SLOTS && !sp_wait_warp(empty + 8 * s, (c / SP_SLOTS - 1) & 1, &abort_s, status)) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            bool ok = true;
+            float least = INFINITY;                        // the smallest of the entries cut here
+            const auto four = [&](int j) { return sp_shared_four(smem + r * SP_BOX + row * 128 + ((j ^ (row & 7)) << 4)); };
+            const unsigned to = tmem + lanes + s * SP_W_COLS, a_to = a_parts + s * SP_PARTS * part_bytes + group;
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
-                float hi[SP_KC / 2], lo[SP_KC / 2];
+                unsigned hi[SP_KC / 4], mid[SP_KC / 4], lo[SP_KC / 4];
 #pragma unroll
                 for (int j = 0; j < SP_KC / 8; ++j) {
-                    const float4 v = sp_shared_four(smem + r * SP_BOX + row * 128 + (((4 * half + j) ^ (row & 7)) << 4));
-                    hi[4 * j] = sp_hi(v.x); hi[4 * j + 1] = sp_hi(v.y); hi[4 * j + 2] = sp_hi(v.z); hi[4 * j + 3] = sp_hi(v.w);
-                    lo[4 * j] = v.x - hi[4 * j]; lo[4 * j + 1] = v.y - hi[4 * j + 1]; lo[4 * j + 2] = v.z - hi[4 * j + 2]; lo[4 * j + 3] = v.w - hi[4 * j + 3];
+                    const float4 v = four(4 * half + j);
+                    sp_least(least, v.x, v.y); sp_least(least, v.z, v.w);
+                    sp_cut(v.x, v.y, hi[2 * j], mid[2 * j], lo[2 * j]);
+                    sp_cut(v.z, v.w, hi[2 * j + 1], mid[2 * j + 1], lo[2 * j + 1]);
                 }
-                sp_st16(tmem + lanes + s * 2 * SP_KC + 16 * half, hi);
-                sp_st16(tmem + lanes + s * 2 * SP_KC + SP_KC + 16 * half, lo);
+                if (half == 0) {                           // (the first half is cut while the slot's last products end)
+                    if (c >= slots && !(ok = sp_wait_warp(empty + 8 * s, (c / slots - 1) & 1, &abort_s, status))) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                }
+                sp_st8(to + 8 * half, hi); sp_st8(to + 8 * half + SP_KC / 2, mid); sp_st8(to + 8 * half + SP_KC, lo);
             }
-            __syncwarp();
-            if (lane == 0) at_arrive(w_empty + 8 * r);
+            if (!ok) break;
             if (!MANY) {
 #pragma unroll
                 for (int e = 0; e < TPT; ++e)
                     if (NT >= 32 || lr < NT) {
-                        const unsigned at = a_parts + s * 2 * part_bytes + e * 32 * 128;
-                        float h[8], l[8];
+                        unsigned part[SP_PARTS][4];
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) { h[i] = sp_hi(ra[e][i]); l[i] = ra[e][i] - h[i]; }
-                        sp_put_four(at + first, h); sp_put_four(at + second, h + 4);
-                        sp_put_four(at + part_bytes + first, l); sp_put_four(at + part_bytes + second, l + 4);
+                        for (int i = 0; i < 4; ++i) {
+                            sp_least(least, ra[e][2 * i], ra[e][2 * i + 1]);
+                            sp_cut(ra[e][2 * i], ra[e][2 * i + 1], part[0][i], part[1][i], part[2][i]);
+                        }
+#pragma unroll
+                        for (int q = 0; q < SP_PARTS; ++q) sp_put_four(a_to + e * 32 * 64 + q * part_bytes, part[q]);
                     }
+            }
+            if (__any_sync(0xffffffffu, least < SP_SMALL)) {      // (zeros, as a rule)
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+#pragma unroll 1
+                for (int half = 0; half < 2; ++half) {
+                    unsigned hi[SP_KC / 4];
+#pragma unroll
+                    for (int j = 0; j < SP_KC / 8; ++j) {
+                        const float4 v = four(4 * half + j);
+                        hi[2 * j] = sp_marked(v.x, v.y); hi[2 * j + 1] = sp_marked(v.z, v.w);
+                    }
+                    __syncwarp();
+                    sp_st8(to + 8 * half, hi);
+                }
+                if (!MANY) {
+#pragma unroll
+                    for (int e = 0; e < TPT; ++e)
+                        if (NT >= 32 || lr < NT) {
+                            unsigned part[4];
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) part[i] = sp_marked(ra[e][2 * i], ra[e][2 * i + 1]);
+                            sp_put_four(a_to + e * 32 * 64, part);
+                        }
+                }
+            }
+            __syncwarp();
+            if (lane == 0) at_arrive(w_empty + 8 * r);
+            if (!MANY) {
                 if (c + GROUPS < chunks) fetch_a(c + GROUPS);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            }
+            } else if ((warp & 3) == 0 && !sp_wait_warp(a_full + 8 * s, (c / slots) & 1, &abort_s, status)) break;
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) at_arrive(full + 8 * s);
         }
-    } else if (warp == SP_CUTTERS) {
-        const unsigned idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((unsigned)(nt / 8) << 17) | ((unsigned)(SP_ROWS / 16) << 24);
+    } else if (warp == CUTTERS) {
+        const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(nt / 8) << 17) | ((unsigned)(SP_ROWS / 16) << 24);
         const unsigned elected = sp_elect();
         int issued = 0;
         for (int c = 0; c < chunks; ++c) {
-            const int s = c % SP_SLOTS, b = c % SUMS;
+            const int s = c % slots, b = c % SUMS;
             if (c >= SUMS && !sp_wait_warp(sum_empty + 8 * b, (c / SUMS - 1) & 1, &abort_s, status)) break;
-            if (!sp_wait_warp(full + 8 * s, (c / SP_SLOTS) & 1, &abort_s, status)) break;
-            if (MANY && !sp_wait_warp(a_full + 8 * s, (c / SP_SLOTS) & 1, &abort_s, status)) break;
+            if (!sp_wait_warp(full + 8 * s, (c / slots) & 1, &abort_s, status)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const unsigned long long a = at_desc(a_parts + s * 2 * part_bytes, 16, 1024);
-            sp_products(elected, sums + b * NT, tmem + s * 2 * SP_KC, a, a + (part_bytes >> 4), idesc);
+            const unsigned long long a = sp_desc(a_parts + s * SP_PARTS * part_bytes), part = part_bytes >> 4;
+            sp_products(elected, sums + b * nt, small, tmem + s * SP_W_COLS, a, a + part, a + 2 * part, idesc, c > 0);
             if (elected) {
                 at_commit(empty + 8 * s);
                 at_commit(sum_full + 8 * b);
@@ -327,16 +418,16 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
             issued = c + 1;
         }
         if (issued > 0) at_wait_warp(sum_full + 8 * ((issued - 1) % SUMS), ((issued - 1) / SUMS) & 1);      // nothing stays under way
-    } else if (warp == SP_CUTTERS + 1) {
+    } else if (warp == CUTTERS + 1) {
         if (lane == 0) {
             int brought = min(RING, chunks), brought_a = 0;
             for (int c = 0; c < chunks; ++c) {
-                const int s = c % SP_SLOTS, r = c % RING;
+                const int s = c % slots, r = c % RING;
                 if (MANY) {
-                    if (c >= SP_SLOTS && !sp_wait(empty + 8 * s, (c / SP_SLOTS - 1) & 1, &abort_s, status)) break;
-                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(a_full + 8 * s), "r"((unsigned)(2 * part_bytes)) : "memory");
+                    if (c >= slots && !sp_wait(empty + 8 * s, (c / slots - 1) & 1, &abort_s, status)) break;
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(a_full + 8 * s), "r"((unsigned)(SP_PARTS * part_bytes)) : "memory");
                     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-                                 ::"r"(a_parts + s * 2 * part_bytes), "l"(&map_a), "r"(a_full + 8 * s), "r"(k_begin + c * SP_KC), "r"(m0), "r"(0) : "memory");
+                                 ::"r"(a_parts + s * SP_PARTS * part_bytes), "l"(&map_a), "r"(a_full + 8 * s), "r"(k_begin + c * SP_KC), "r"(m0), "r"(0) : "memory");
                     brought_a = c + 1;
                 }
                 if (c + RING < chunks) {
@@ -347,7 +438,7 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
             }
             // (each of them has landed long ago unless a role gave up)
             for (int c = max(0, brought - RING); c < brought; ++c) at_wait(w_full + 8 * (c % RING), (c / RING) & 1);
-            for (int c = max(0, brought_a - SP_SLOTS); c < brought_a; ++c) at_wait(a_full + 8 * (c % SP_SLOTS), (c / SP_SLOTS) & 1);
+            for (int c = max(0, brought_a - slots); c < brought_a; ++c) at_wait(a_full + 8 * (c % slots), (c / slots) & 1);
         }
         __syncwarp();
     } else {
@@ -358,11 +449,12 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
             const int b = c % SUMS;
             if (!sp_wait_warp(sum_full + 8 * b, (c / SUMS) & 1, &abort_s, status)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            sp_add_columns<COLS>(acc, mine + b * NT, columns);
+            sp_add_columns<COLS>(acc, mine + b * nt, columns);
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) at_arrive(sum_empty + 8 * b);
         }
+        if (chunks > 0) sp_add_columns<COLS>(acc, mine + SUMS * nt, columns);      // (the last chunk's products were these accumulators' last)
     }
     __syncthreads();                                       // all products have ended, all copies have landed
     bool whole = *(volatile int*)&abort_s == 0;
@@ -398,7 +490,7 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
             }
         }
     }
-    const unsigned sums_sent = a_parts + SP_SLOTS * 2 * part_bytes;       // [rank][slice][128]
+    const unsigned sums_sent = a_parts + SP_SLOTS * SP_PARTS * part_bytes;       // [rank][slice][128]
     if (MANY) {
         if (ranges > 1) sp_cluster_sync(); else __syncthreads();
     } else {
@@ -446,21 +538,23 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
         asm volatile("barrier.cluster.wait.acquire;" ::: "memory");           // or before all have sent
         if (!whole && rows > 0) sp_wait_sent(sent);
     }
-    if (warp == SP_CUTTERS) {
+    if (warp == CUTTERS) {
         __syncwarp();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((unsigned)SP_TMEM) : "memory");
     }
 }
 
-// Boxes of 32 entries x `rows` rows x `planes` of a float32 [planes][R][K] array; what lies outside reads as zero.
-static int sp_map(CUtensorMap* map, const void* base, int K, int R, int planes, int rows) {
+// Boxes of 32 entries x `rows` rows of float32 [R][K], or of all parts in bfloat16 [SP_PARTS][R][K]; what lies outside reads as zero.
+static int sp_map(CUtensorMap* map, const void* base, int K, int R, int rows, bool parts) {
     at_encode_fn enc = at_encoder();
     if (!enc) return PE_ERR_UNSUPPORTED;
-    const cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)R, (cuuint64_t)planes}, strides[2] = {(cuuint64_t)K * 4, (cuuint64_t)K * R * 4};
-    const cuuint32_t box[3] = {SP_KC, (cuuint32_t)rows, (cuuint32_t)planes}, elem[3] = {1, 1, 1};
-    const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, planes > 1 ? 3 : 2, const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    const unsigned size = parts ? 2 : 4;
+    const cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)R, SP_PARTS}, strides[2] = {(cuuint64_t)K * size, (cuuint64_t)K * R * size};
+    const cuuint32_t box[3] = {SP_KC, (cuuint32_t)rows, SP_PARTS}, elem[3] = {1, 1, 1};
+    const CUresult r = enc(map, parts ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, parts ? 3 : 2, const_cast<void*>(base), dims, strides, box, elem,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, parts ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? 0 : 20000 + (int)r;
 }
 
@@ -498,12 +592,14 @@ static int sp_resident_clusters(int ranges, int& n) {
 }
 
 // Whether a product of float32 operands comes here: by N, K and the place of W alone, so that a row's result is the same in every step.
-// Smaller products of one to 16 rows are what their launch takes (512 x 512 here / as multiply-adds 5.3 / 3.3 us at one row, 6.0 / 8.5 at 17).
+// 800,000 entries is where one row takes as long either way: 1, 12, 60 and 508 rows, here / as multiply-adds, 512 x 512 5.3 5.5 8.4 11.5 / 3.2 4.2 8.4 16.8,
+// 768 x 768 5.7 5.9 8.7 13.8 / 4.5 5.8 11.2 24.8, 1024 x 768 5.6 5.7 8.6 14.3 / 5.3 7.6 12.1 25.0, 832 x 960 5.5 5.7 8.3 15.7 / 5.5 7.9 13.6 31.5, 1024 x 1024 5.6 5.7 8.4
+// 16.3 / 6.3 9.4 14.9 31.4; narrow ones lose a little at one row: 3200 x 256 5.1 / 4.8, 256 x 3200 7.1 / 6.9, 1280 x 640 6.3 / 5.8.
 extern "C" int pe_linear_split_takes(const void* W, int N, int K) { return N >= 256 && K >= 256 && (long long)N * K >= 800000 && K % 8 == 0 && (uintptr_t)W % 16 == 0; }
 
 // Rows of A that are cut at a time, so that their parts take 256 MB at most; and the bytes of scratch a product of M rows needs.
-static int sp_slab(int K) { return (int)((256ll << 20) / (8ll * K) > SP_MANY ? (256ll << 20) / (8ll * K) / SP_MANY * SP_MANY : SP_MANY); }
-extern "C" long long pe_linear_split_scratch(int M, int K) { return M <= 64 ? 0 : 8ll * K * (M < sp_slab(K) ? M : sp_slab(K)); }
+static int sp_slab(int K) { return (int)((256ll << 20) / (2ll * SP_PARTS * K) > SP_MANY ? (256ll << 20) / (2ll * SP_PARTS * K) / SP_MANY * SP_MANY : SP_MANY); }
+extern "C" long long pe_linear_split_scratch(int M, int K) { return M <= 64 ? 0 : 2ll * SP_PARTS * K * (M < sp_slab(K) ? M : sp_slab(K)); }
 // The kernels that a product of M rows launches.
 extern "C" int pe_linear_split_launches(int M, int K) { return M <= 0 ? 0 : M <= 64 ? 1 : 2 * ((M + sp_slab(K) - 1) / sp_slab(K)); }
 
@@ -520,7 +616,7 @@ extern "C" int pe_linear_split(const void* A, const void* W, const void* bias, i
     if (!pe_linear_split_takes(W, N, K) || epilogue < 0 || epilogue > 2) return PE_ERR_UNSUPPORTED;
     CUtensorMap map_w = {}, map_a = {};
     const cudaStream_t s = (cudaStream_t)stream;
-    if (const int e = sp_map(&map_w, W, K, N, 1, SP_ROWS)) return e;
+    if (const int e = sp_map(&map_w, W, K, N, SP_ROWS, false)) return e;
 #define SP_GO(NT, nt, A, out, M) sp_go<NT>(map_w, map_a, nt, (const float*)(A), (const float*)W, bias, bias_dtype, out, epilogue, M, N, K, (int*)status, s)
     if (M <= 16) return SP_GO(16, 16, A, out, M);
     if (M <= 32) return SP_GO(32, 32, A, out, M);
@@ -541,9 +637,9 @@ extern "C" int pe_linear_split(const void* A, const void* W, const void* bias, i
         const float* a = (const float*)A + (size_t)first * K;
         void* o = (char*)out + (size_t)first * N * (epilogue == 1 ? 2 : 4);
         const long long entries = (long long)rows * K;
-        PE_TRY(pe_launch(split_rows_kernel, dim3((unsigned)((entries / 4 + 255) / 256)), 256, 0, s, a, (float*)scratch, entries, (int)((uintptr_t)a % 16 == 0)));
+        PE_TRY(pe_launch(split_rows_kernel, dim3((unsigned)((entries / 8 + 255) / 256)), 256, 0, s, a, (bf16*)scratch, entries, (int)((uintptr_t)a % 16 == 0)));
         PE_LAUNCH_CHECK();
-        if (const int e = sp_map(&map_a, scratch, K, rows, 2, nt)) return e;
+        if (const int e = sp_map(&map_a, scratch, K, rows, nt, true)) return e;
         if (const int e = SP_GO(SP_MANY, nt, a, o, rows)) return e;
     }
 #undef SP_GO

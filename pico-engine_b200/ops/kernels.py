@@ -153,7 +153,8 @@ def linear_simt(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] =
                 out_dtype: Optional[torch.dtype] = None, accumulate_into: Optional[torch.Tensor] = None,
                 out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """a [M, K] . w [N, K]^T (+ bias) in float32, whatever the operands are stored as.  Either stored as
-    ``out_dtype`` or added into the float32 tensor ``accumulate_into`` [M, N]."""
+    ``out_dtype`` or added into the float32 tensor ``accumulate_into`` [M, N].  All bits of
+    float32 operands count, and results are no further from exact ones than a chain of multiply-adds has them."""
     M, K = a.shape
     N = w.shape[0]
     _need(a, "a"); _need(w, "w", None, (N, K))
@@ -168,7 +169,7 @@ def linear_simt(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] =
         _need(out, "out", None, (M, N))
         epilogue = _EPILOGUE_STORE[out.dtype]
     if a.dtype == w.dtype == torch.float32 and core().pe_linear_split_takes(w.data_ptr(), N, K):
-        # on the tensor cores, each operand in two parts: as exact as multiply-adds (csrc/linear_split.cu has the figures)
+        # on the tensor cores, each operand in three parts that hold all its bits (csrc/linear_split.cu: errors beside those of multiply-adds)
         nbytes = core().pe_linear_split_scratch(M, K)
         parts = torch.empty(nbytes, dtype=torch.uint8, device=a.device) if nbytes else None
         check(core().pe_linear_split(a.data_ptr(), w.data_ptr(), _ptr(bias), 0 if bias is None else _code(bias, "bias"), out.data_ptr(), epilogue,
@@ -541,7 +542,9 @@ def linear_fused(a: Optional[torch.Tensor], w: torch.Tensor, bias: Optional[torc
                  eps: float = 0.0, scale: float = 1.0) -> torch.Tensor:
     """a [M <= 64, K] . w [N, K]^T (+ bias); with ``norm_of`` (float32 [M, K]) the operand is
     RMSNorm(norm_of) with ``norm_weight`` instead of ``a``.  (More than 16 rows: bfloat16 or accumulated results.)
-    ``scale`` (up to 16 rows, with ``accumulate_into``): accumulate_into += scale * product."""
+    ``scale`` (up to 16 rows, with ``accumulate_into``): accumulate_into += scale * product.
+    ``w`` and ``norm_weight`` are read while the kernel in front may still run: no kernel may have written them just before.  (The same
+    holds for the weights of the other fused decode products, and so for a bfloat16 ``linear`` of up to 16 rows.)"""
     src = norm_of if norm_of is not None else a
     M, K = src.shape
     N = w.shape[0]

@@ -12,8 +12,8 @@ follows it in a layer: the choice of kernel for a matrix product.
   so the first time a product of some shape is asked for, both are timed on the device, a few replays of
   a captured CUDA graph each, and the faster one is remembered (``Choice``).  ``PICO_ENGINE_GEMM=tcgen05``
   or ``=library`` fixes the choice instead.
-* float32 activations and weights (the float32 engine): the tensor cores with each operand in two
-  parts, at float32 accuracy, ``csrc/linear_split.cu``; matrices of less than 800,000 entries, and
+* float32 activations and weights (the float32 engine): the tensor cores with each operand in three
+  parts that hold all its bits, at float32 accuracy, ``csrc/linear_split.cu``; matrices of less than 800,000 entries, and
   anything else (weights that were stored in float32 beside bfloat16 rows): float32 multiply-adds on
   the CUDA cores, ``csrc/linear_simt.cu``.
 """

@@ -744,6 +744,66 @@ def test_linear_float32_of_a_weight_just_written(K, M):
     assert all(torch.equal(g, x) for g, x in zip(got, want))
 
 
+def multiply_adds(a, w):
+    """The same product by the kernel of multiply-adds, whatever the sizes."""
+    from pico_engine.ops.library import check, core, stream_ptr
+    out = torch.empty(a.shape[0], w.shape[0], device="cuda")
+    check(core().pe_linear_simt(a.data_ptr(), 0, w.data_ptr(), 0, None, 0, out.data_ptr(), 0, a.shape[0], w.shape[0], a.shape[1], stream_ptr()), "linear_simt")
+    return out
+
+
+def _entries(kind, M, K_):
+    """Rows of A: random ones, or such that one or a few of their products make a result."""
+    g = torch.Generator().manual_seed(7)
+    rows, some = torch.arange(M), lambda: torch.randint(0, K_, (M,), generator=g)
+    a = {"normal": rnd(M, K_, seed=1), "positive": torch.rand(M, K_, generator=g), "dominant": rnd(M, K_, seed=1, scale=1e-4)}.get(kind, torch.zeros(M, K_))
+    for _ in range({"one": 1, "four": 4, "dominant": 1}.get(kind, 0)):
+        a[rows, some()] = torch.randn(M, generator=g)
+    return a
+
+
+@pytest.mark.parametrize("M", [60, 200])
+@pytest.mark.parametrize("N,K_", SPLIT_SIZES)
+@pytest.mark.parametrize("kind", ["normal", "positive", "one", "four", "dominant"])
+def test_linear_float32_is_as_exact_as_multiply_adds(K, kind, M, N, K_):
+    """Full float32 operands against float64, in the 2-norm.  A result adds up to 28 sums of 32 entries, each rounded to 24 bits: their roundings
+    are a quarter of 2^-23 of the running sum, which grows as the root of their number, 9e-8 for 28; the cuts within a sum of 32 are 0.6 x 2^-23 =
+    7e-8 of it.  1.2e-7 in all for random signs, 2e-7 allowed (sums with one less bit an operand, or over 64 entries at a time, of positive
+    entries would be above it).  One to four terms: what is left out and the roundings, 2^-24 each at most."""
+    a, w = dev(_entries(kind, M, K_)), dev(torch.rand(N, K_, generator=torch.Generator().manual_seed(2)) if kind == "positive" else rnd(N, K_, seed=2))
+    want = a.double() @ w.double().T
+    err = lambda got: float((got.double() - want).norm() / want.norm())
+    here, plain_ = err(K.linear_simt(a, w)), err(multiply_adds(a, w))
+    assert here <= (2 ** -24 if kind in ("one", "four") else 2e-7), (here, plain_)
+    assert here <= 1.25 * plain_, (here, plain_)          # (of one term: the two parts of the sum are rounded one after the other)
+    if kind == "one":
+        assert ((K.linear_simt(a, w).double() - want).abs() <= (2 + 2 ** -9) * 2.0 ** -24 * want.abs()).all()
+    K.check_status("cuda")
+
+
+@pytest.mark.parametrize("M", [5, 60, 200])
+@pytest.mark.parametrize("N,K_", SPLIT_SIZES)
+def test_linear_float32_of_unit_vectors_and_small_numbers(K, M, N, K_):
+    """A row that picks one entry, or a power of two times it, gives that entry in all its bits.  Entries too small to be the sum of three bfloat16
+    numbers count in full, alone and among others: a result is off by at most 40 x 2^-24 of its terms' magnitudes (2 cuts of 2^-23 in each sum
+    of 32, 28 additions)."""
+    w = dev(rnd(N, K_, seed=2))
+    col = torch.randint(0, K_, (M,), generator=torch.Generator().manual_seed(3))
+    a = torch.zeros(M, K_)
+    a[torch.arange(M), col] = torch.tensor([1.0, -2.0, 2.0 ** -30, 4.0, 1.0])[torch.arange(M) % 5]
+    assert torch.equal(K.linear_simt(dev(a), w), w.T[dev(col)] * dev(a).sum(1, keepdim=True))
+    for small in (1e-30, 1e-33, 1e-36, 1e-39, 3e-45):
+        x = dev(rnd(M, K_, seed=4) * small)
+        x[M // 2:, K_ // 2:] = 0                               # zeros are no such entries
+        x[0, 1:] = 0
+        for scale in (1.0, 2.0 ** 100):
+            for b, c in ((x, w * scale), (dev(rnd(M, K_, seed=5)) * scale, torch.cat([x, w])[:N].contiguous())):
+                want = b.double() @ c.double().T
+                bound = 40 * 2.0 ** -24 * (b.double().abs() @ c.double().abs().T) + K_ * 2.0 ** -149
+                assert ((K.linear_simt(b, c).double() - want).abs() <= bound).all(), (small, scale)
+    K.check_status("cuda")
+
+
 @pytest.mark.parametrize("M", [7, 60, 200])
 @pytest.mark.parametrize("N,K_", [(4100, 264), (896, 896)])
 def test_linear_float32_in_parts_of_values_that_are_not_finite(K, M, N, K_):

@@ -46,6 +46,33 @@ def test_real_layer_sizes_every_way_of_cutting(name, layers, seed):
         gc.collect(); torch.cuda.empty_cache()
 
 
+@pytest.mark.parametrize("name", ["qwen2.5-0.5b", "qwen2.5-7b"])
+def test_float32_weights_with_all_their_bits(tmp_path, name):
+    """Weights stored in float32 whose low bits are not zero, as a bfloat16 draw's are, through the float32 engine."""
+    from conftest import write_model
+    from pico_engine.config import config_from_dict
+    from pico_engine.config.registry import architecture
+    from pico_engine.config.shapes import shape
+    from pico_engine.engine.engine import Engine
+    from pico_engine.weights import random_tensor
+    d = shape(name)
+    d["num_hidden_layers"], d["vocab_size"] = 1, 2048
+    cfg = config_from_dict(d)
+    expected = architecture(cfg.ARCHITECTURE).build_model(cfg, torch.float32, "meta").expected_tensors()
+    weights = {n: random_tensor(n, spec, 6, torch.float32, "cuda") for n, spec in expected.items()}
+    assert all((t.view(torch.int32) & 0xFFFF).ne(0).any() for t in weights.values())
+    g = torch.Generator().manual_seed(6)
+    reqs = {f"r{i}": torch.randint(0, 2048, (n,), generator=g).tolist() for i, n in enumerate(LENGTHS)}
+    want = replay.plain_logits(d, weights, reqs)
+    folder = write_model(tmp_path, d, weights, store=torch.float32)
+    del weights
+    eng = Engine(folder, device="cuda", dtype="float32")
+    replay.compare(replay.run_in_process(eng, replay.whole(reqs)), want, "float32", f"{name} whole")
+    replay.compare(replay.run_in_process(eng, replay.tail(reqs, 8)), want, "float32", f"{name} tail")
+    del eng
+    gc.collect(); torch.cuda.empty_cache()
+
+
 @pytest.mark.parametrize("name,layers,seed", SHAPES[:2], ids=[s[0] for s in SHAPES[:2]])
 def test_real_layer_sizes_generation_with_graphs(name, layers, seed):
     """Greedy generation in bfloat16 through the entry point at head sizes 64 and 128, with the decode graphs and one
