@@ -26,8 +26,8 @@
 // memory and the first loads (asked for before the block meets), the first step's chain, the end of the row.  What the softmax
 // warps do besides exponentials counts: scale and sums go two numbers at a time (fma / add .f32x2), a page's mask is one comparison
 // a score against the last key the row sees, and rows leave through shared memory (at_store_rows).  2,048 tokens, 14 heads of 64,
-// on a B200: 26.0 us with a chain of comparisons a score, single sums and rows stored by their own lanes, 21.6 us here; 28 heads of 128,
-// prompts of 5,001 / 1,807 / 700 / 33 tokens: 273 us, 237 us here.
+// on a B200, in a graph of nothing else: 23.8 us with a chain of comparisons a score, single sums and rows stored by their own lanes, 19.3 us here (18.9 if runs and
+// page table were read before the kernel in front has ended); 28 heads of 128, prompts of 5,001 / 1,807 / 700 / 33 tokens: 271 us, 228 us here.
 //
 // Values lie in the cache as [key][head size], which is the MN-major form of the B operand of
 // P.V: its shared-memory descriptor steps 8 keys by 1024 bytes and 64 columns by one panel.

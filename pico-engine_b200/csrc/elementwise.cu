@@ -258,12 +258,13 @@ template <typename TY, bool ADD>
 static int rmsnorm_launch(float* x, const TY* y, const int* rows_index, const void* w, int w_dtype, float eps, void* out,
                           int out_dtype, int rows, int H, cudaStream_t s) {
     // All loads of a thread go out before its first store and one block-wide meeting is left of three: inside a graph, bfloat16 y, before and
-    // now, us with / without the residual sum: 1 row of 896 2.2 / 1.8 and 1.3 / 1.1; 2,048 rows of 896 5.3 / 4.2 and 3.7 / 3.1; 7,541 rows of
-    // 3,584 71 / 42 (a warp a row, read twice) and 52 / 29, 6.3 TB/s.
+    // now, us with / without the residual sum: 1 row of 896 2.2 / 1.8 and 1.3 / 1.2; 2,048 rows of 896 5.3 / 4.2 and 3.6 / 3.3; 7,541 rows of
+    // 3,584 71 / 42 (a warp a row, read twice) and 49 / 29, 6.3 TB/s.  A width of 1,027 2.8 us a row, with 96 threads instead of 256 4.7; 4,099 4.2, 288
+    // threads instead of 512 6.2.
     // Many rows of up to 1,024 columns: a warp a row.  4,096 rows against 4,095 in blocks: 64 columns 2.0 against 4.7, 896 columns without
     // the sum 3.4 against 5.4, with it level (7.5, 7.2).  Wider rows stay in blocks: 7,541 of 2,048 columns 29 against 39 a warp a row.
     // Two groups of four a thread up to 1,024 columns, four beyond: 7,541 rows of 3,584 52 / 29 against 62 / 50 with two.
-    // Four groups' weights ahead of the wait cost residency: with the sum, 1 row of 3,584 1.9 against 2.2, 2,048 rows 17.3 against 16.2.
+    // Four groups' weights asked for with the row cost residency: with the sum, 1 row of 3,584 1.9 against 2.2, 2,048 rows 17.3 against 16.2.
     auto run = [&](auto* o) -> int {
         using TO = std::remove_pointer_t<decltype(o)>;
         if (!rows_index && rows >= 4096 && (H & 3) == 0 && H <= 1024) {
