@@ -1,0 +1,186 @@
+// Float32 products over chunks of 64 tokens on the tensor cores, every float32 number in three bfloat16 parts that hold all of its bits:
+// hi = round(v), mid = round(v - hi), lo = round(v - hi - mid).  Of the nine products of two numbers six are made (the other three are
+// below 2^-25 of theirs).  The tensor cores cut their sums to 24 bits, so hi hi is summed over 32 entries at a time and these sums are
+// added as float32 numbers are; the small products, 2^-8 of it at most, are summed first.
+//
+// What three parts cannot hold is infinities, numbers that are none, numbers that round to an infinity, and tiles of nothing but numbers
+// below 2^-90, whose small parts fall out of bfloat16's range: cm_watch finds them on the way, and the results that they reach are worked
+// out with multiply-adds.  (A token that is no number reaches none in front of it: cm_mend puts zeros in its place, and those keep their bits.)
+//
+// A plane is 64 rows (tokens) of 64 bfloat16 numbers, a part each: rows of 128 bytes whose eight 16-byte groups are exchanged by the row's
+// place in a run of eight, which is what the 128-byte swizzle of an operand in shared memory is, along a row (K-major) or across rows.
+#pragma once
+#include "tcgen05_attention.cuh"
+
+#define CM_CHUNK 64                                       // tokens of a chunk
+#define CM_PLANE (CM_CHUNK * 128)                         // bytes
+#define CM_PARTS 3
+
+__device__ __forceinline__ unsigned cm_at(int row, int group) { return row * 128 + ((group ^ (row & 7)) << 4); }      // eight numbers of a row in a plane
+
+// Two neighbouring numbers' parts, packed.
+__device__ __forceinline__ unsigned long long cm_pair(unsigned a, unsigned b) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ void cm_cut(float a, float b, unsigned& hi, unsigned& mid, unsigned& lo) {
+    unsigned long long rest = at_two(a, b);
+    const unsigned long long minus = at_two(-1.f, -1.f);
+    hi = at_pack(a, b);
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(rest) : "l"(cm_pair(hi << 16, hi & 0xffff0000u)), "l"(minus));      // (exact)
+    float2 r = at_both(rest);
+    mid = at_pack(r.x, r.y);
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(rest) : "l"(cm_pair(mid << 16, mid & 0xffff0000u)), "l"(minus));
+    r = at_both(rest);
+    lo = at_pack(r.x, r.y);
+}
+// The largest upper part that was seen (no number beats every number); its bits in a block's word, for up to five tiles of a block: something that its
+// parts do not hold, something of a usual size, something tiny.
+__device__ __forceinline__ void cm_watch(unsigned& most, unsigned hi) {
+    asm("{\n\t.reg .b32 t;\n\tabs.bf16x2 t, %1;\n\tmax.NaN.bf16x2 %0, %0, t;\n\t}" : "+r"(most) : "r"(hi));
+}
+__device__ __forceinline__ unsigned cm_seen(unsigned most, int tile) {
+    const unsigned a = most & 0x7fffu, b = (most >> 16) & 0x7fffu, m = a > b ? a : b;
+    return (m >= 0x7f80u ? 1u : m >= 0x1280u ? 2u : m ? 4u : 0u) << (3 * tile);      // 0x1280: 2^-90
+}
+#define CM_TILES 0x1249u                                  // the first bits of five tiles
+__device__ __forceinline__ bool cm_odd(unsigned seen) { return (seen & CM_TILES) != 0; }
+__device__ __forceinline__ bool cm_odd_tile(unsigned seen, int tile) { return (seen >> (3 * tile)) & 1u; }
+__device__ __forceinline__ bool cm_tiny(unsigned seen) { return ((seen >> 2) & ~(seen >> 1) & ~seen & CM_TILES) != 0; }      // some tile of nothing but tiny numbers
+__device__ __forceinline__ void cm_report(unsigned* seen, unsigned mine) {         // (a block's word in shared memory)
+    const unsigned all = __reduce_or_sync(0xffffffffu, mine);
+    if ((threadIdx.x & 31) == 0 && all) atomicOr(seen, all);
+}
+// Eight numbers' parts into planes that lie `stride` bytes apart, at `to` in the first.
+__device__ __forceinline__ void cm_put(unsigned char* to, int stride, const float4& a, const float4& b, unsigned& most) {
+    unsigned part[CM_PARTS][4];
+    cm_cut(a.x, a.y, part[0][0], part[1][0], part[2][0]); cm_cut(a.z, a.w, part[0][1], part[1][1], part[2][1]);
+    cm_cut(b.x, b.y, part[0][2], part[1][2], part[2][2]); cm_cut(b.z, b.w, part[0][3], part[1][3], part[2][3]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) cm_watch(most, part[0][i]);
+#pragma unroll
+    for (int p = 0; p < CM_PARTS; ++p) *reinterpret_cast<uint4*>(to + p * stride) = make_uint4(part[p][0], part[p][1], part[p][2], part[p][3]);
+}
+// A plane of upper parts of which some is no finite number: zeros for such entries in all of its parts, `stride` bytes apart; `first` becomes the first
+// row that has one.  All threads.
+__device__ __forceinline__ void cm_mend(unsigned char* plane, int stride, unsigned* first) {
+#pragma unroll 1
+    for (int i = threadIdx.x; i < CM_PLANE / 4; i += blockDim.x) {
+        unsigned* at = reinterpret_cast<unsigned*>(plane) + i;
+        const unsigned v = *at, keep = ((v & 0x7f80u) == 0x7f80u ? 0u : 0xffffu) | ((v & 0x7f800000u) == 0x7f800000u ? 0u : 0xffff0000u);
+        if (keep == 0xffffffffu) continue;
+        for (int p = 0; p < CM_PARTS; ++p) at[p * stride / 4] &= keep;
+        atomicMin(first, (unsigned)(i / 32));
+    }
+}
+// `bytes` (a multiple of 16, both addresses too) into shared memory, all threads of the block; cm_landed waits for all that were asked for.
+__device__ __forceinline__ void cm_bring(unsigned char* dst, const void* src, int bytes) {
+    for (int i = threadIdx.x * 16; i < bytes; i += blockDim.x * 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(at_smem(dst + i)), "l"((const char*)src + i) : "memory");
+}
+__device__ __forceinline__ void cm_landed() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// ---------------------------------------------------------------- products by tcgen05 (one warp calls, its elected thread issues)
+// An operand of 64 entries of K: descriptors of its parts (`stride` bytes apart), and how far 16 entries of K are in 16-byte units.
+struct CMOperand { unsigned long long hi, mid, lo; unsigned step; };
+__device__ __forceinline__ CMOperand cm_along(unsigned at, int stride) {                     // K along the rows of the planes
+    const unsigned long long d = at_desc(at, 0, 1024);
+    return {d, d + (stride >> 4), d + 2 * (stride >> 4), 2u};
+}
+// K across the rows; the operand's second 64 columns are the plane `second` bytes behind
+__device__ __forceinline__ CMOperand cm_across(unsigned at, int stride, int second) {
+    const unsigned long long d = at_desc(at, second, 1024);
+    return {d, d + (stride >> 4), d + 2 * (stride >> 4), 128u};
+}
+__device__ __forceinline__ unsigned cm_elect() {
+    unsigned r;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cm_issue(unsigned elected, unsigned sums, unsigned long long a, unsigned long long b, unsigned idesc, bool add) {
+    asm volatile("{\n .reg .pred e, p;\n setp.ne.u32 e, %0, 0;\n setp.ne.u32 p, %5, 0;\n"
+                 " @e tcgen05.mma.cta_group::1.kind::f16 [%1], %2, %3, %4, p;\n}"
+                 ::"r"(elected), "r"(sums), "l"(a), "l"(b), "r"(idesc), "r"((unsigned)add) : "memory");
+}
+// [128 x N] products over 64 entries: hi hi of the first 32 in `first`; the small ones and then hi hi of the other 32 in `rest` (so that either sum is
+// cut twice at its full size).  The whole warp goes through it, with the same operands (in a branch of one thread each instruction waits for
+// its operands to be moved: 150 cycles apiece).
+__device__ __forceinline__ void cm_products(unsigned elected, unsigned first, unsigned rest, const CMOperand& a, const CMOperand& b, unsigned idesc) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const unsigned ka = k * a.step, kb = k * b.step;
+        cm_issue(elected, rest, a.lo + ka, b.hi + kb, idesc, k);
+        cm_issue(elected, rest, a.hi + ka, b.lo + kb, idesc, true);
+        cm_issue(elected, rest, a.mid + ka, b.mid + kb, idesc, true);
+        cm_issue(elected, rest, a.mid + ka, b.hi + kb, idesc, true);
+        cm_issue(elected, rest, a.hi + ka, b.mid + kb, idesc, true);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) cm_issue(elected, k < 2 ? first : rest, a.hi + k * a.step, b.hi + k * b.step, idesc, k != 0);
+}
+// idesc: float32 sums of bfloat16 products, 128 rows, n columns, either operand across the rows of its planes or along them
+__device__ __forceinline__ constexpr unsigned cm_idesc(int n, bool a_across, bool b_across) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((a_across ? 1u : 0u) << 15) | ((b_across ? 1u : 0u) << 16) | ((unsigned)(n >> 3) << 17) | ((unsigned)(128 >> 4) << 24);
+}
+// 16 or 32 columns of this thread's row, and acc += them
+__device__ __forceinline__ void cm_read(float (&v)[16], unsigned taddr) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\ttcgen05.wait::ld.sync.aligned;"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]),
+                   "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]) : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void cm_read(float (&v)[32], unsigned taddr) { at_ld32(taddr, v); }
+template <int N>
+__device__ __forceinline__ void cm_take(float (&acc)[N], unsigned taddr) {
+    float v[N];
+    cm_read(v, taddr);
+#pragma unroll
+    for (int i = 0; i < N; ++i) acc[i] += v[i];
+}
+
+// ---------------------------------------------------------------- products by mma.sync (scores of a chunk's tokens over its keys)
+__device__ __forceinline__ void cm_ldmatrix(unsigned& a, unsigned& b, unsigned& c, unsigned& d, unsigned at) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "r"(at) : "memory");
+}
+__device__ __forceinline__ void cm_mma(float (&c)[4], const unsigned (&a)[4], const unsigned (&b)[2]) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+// A warp's 16 tokens x 32 keys of [t][s], over 64 entries of queries and keys: planes of parts, `stride` bytes apart.  A thread holds tokens
+// lane / 4 and lane / 4 + 8, keys 2 (lane % 4) and the one behind it of each run of eight.
+struct CMScores {
+    float sum[4][4], small[4][4];
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) sum[j][e] = small[j][e] = 0.f;
+    }
+    __device__ __forceinline__ void add(unsigned q, unsigned k, int stride, int t0, int s0) {
+        const int lane = threadIdx.x & 31;
+#pragma unroll 1
+        for (int ks = 0; ks < 4; ++ks) {
+            unsigned a[CM_PARTS][4];
+#pragma unroll
+            for (int p = 0; p < CM_PARTS; ++p) cm_ldmatrix(a[p][0], a[p][1], a[p][2], a[p][3], q + p * stride + cm_at(t0 + (lane & 15), 2 * ks + (lane >> 4)));
+#pragma unroll
+            for (int y = CM_PARTS - 1; y >= 0; --y) {
+                unsigned b[4][2];
+#pragma unroll
+                for (int j = 0; j < 4; j += 2)
+                    cm_ldmatrix(b[j][0], b[j][1], b[j + 1][0], b[j + 1][1], k + y * stride + cm_at(s0 + 8 * j + (lane & 7) + (lane >> 4) * 8, 2 * ks + ((lane >> 3) & 1)));
+#pragma unroll
+                for (int x = CM_PARTS - 1 - y; x >= 0; --x)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        if (x + y) { cm_mma(small[j], a[x], b[j]); continue; }
+                        float t[4] = {0.f, 0.f, 0.f, 0.f};
+                        cm_mma(t, a[0], b[j]);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) sum[j][e] += t[e];
+                    }
+            }
+        }
+    }
+    __device__ __forceinline__ float get(int j, int e) const { return sum[j][e] + small[j][e]; }
+};

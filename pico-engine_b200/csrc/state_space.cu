@@ -190,7 +190,11 @@ extern "C" long long pe_state_space_elems(int H, int P, int N) {
 // full (64 heads of 64 columns, 128 state rows: 125 chunks, 8,000 blocks a launch), and batches of prompts need no more scratch than it.
 #define SS_SCRATCH_FLOATS (64ll << 20)
 extern "C" int pe_state_space_chunks(int T, int B) { return (T + SS_CHUNK - 1) / SS_CHUNK + B; }
-static long long ss_chunk_floats(int H, int P, int N, int G) { return (long long)G * SS_CHUNK * SS_CHUNK + (long long)H * (P * N + SS_STEP_FLOATS + 1) + 4; }
+static int ss_step_floats(int H, int P, int N, int G) { return ss_on_tensor_cores(H, P, N, G) ? SS_MATRIX_STEP_FLOATS : SS_STEP_FLOATS; }
+static long long ss_chunk_floats(int H, int P, int N, int G) {
+    const long long parts = ss_on_tensor_cores(H, P, N, G) ? (long long)G * (2 * ss_plane_bytes(N) / 4 + 1) : 0;
+    return (long long)G * SS_CHUNK * SS_CHUNK + (long long)H * (P * N + ss_step_floats(H, P, N, G) + 1) + 8 + parts;
+}
 static int ss_slab(int chunks, int H, int P, int N, int G) {
     const long long floats = ss_chunk_floats(H, P, N, G), most = floats >= SS_SCRATCH_FLOATS ? 1 : SS_SCRATCH_FLOATS / floats;
     const long long slabs = (chunks + most - 1) / most;
@@ -287,7 +291,7 @@ static int scan_run(const ScanArgs& a, int threads, size_t smem, cudaStream_t s)
 extern "C" int pe_state_space_scan(const float* xbc, int xbc_ld, const void* proj, int dtype, int proj_ld, int dt_off, const void* dt_bias,
                                    int dtb_dtype, const void* a_log, int al_dtype, const void* d_skip, int d_dtype, float* state,
                                    long long state_stride, const int* row_first, const int* row_lens, const int* slots, float* y,
-                                   int T, int B, int H, int P, int N, int G, int chunked, float* scratch, void* stream) {
+                                   int T, int B, int H, int P, int N, int G, int chunked, float* scratch, int* status, void* stream) {
     if (B <= 0 || T <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G || P <= 0 || N <= 0 || N > 512) return PE_ERR_UNSUPPORTED;
     if (chunked && !scratch) return PE_ERR_UNSUPPORTED;
@@ -296,16 +300,24 @@ extern "C" int pe_state_space_scan(const float* xbc, int xbc_ld, const void* pro
     if (PT > P) PT = P;
     int threads = ((PT * NS + 31) / 32) * 32;
     ScanArgs a = {xbc, xbc_ld, proj, proj_ld, dt_off, dt_bias, dtb_dtype, a_log, al_dtype, d_skip, d_dtype, state, state_stride,
-                  row_first, row_lens, slots, y, B, H, P, N, G, NS, NR, NRP, PT, nullptr, nullptr, nullptr, nullptr, nullptr, 0, 0, 0};
+                  row_first, row_lens, slots, y, B, H, P, N, G, NS, NR, NRP, PT, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, 0, 0};
     if (dtype != PE_F32 && dtype != PE_BF16) return PE_ERR_UNSUPPORTED;
     if (chunked) {
         a.chunks = pe_state_space_chunks(T, B);
         a.slab = ss_slab(a.chunks, H, P, N, G);
-        a.chunk_steps = scratch;                                  // (64-bit entries and vectors first; four floats for a chunk's place)
-        a.chunk_rows = reinterpret_cast<int2*>(scratch + (size_t)a.slab * H * SS_STEP_FLOATS);
-        a.chunk_scores = scratch + (size_t)a.slab * (H * SS_STEP_FLOATS + 4);
+        a.chunk_steps = scratch;                                  // (64-bit entries and vectors of eight first; eight floats for a chunk's place)
+        const int step_floats = ss_step_floats(H, P, N, G);
+        a.chunk_rows = reinterpret_cast<int2*>(scratch + (size_t)a.slab * H * step_floats);
+        a.chunk_scores = scratch + (size_t)a.slab * (H * step_floats + 8);
         a.chunk_state = a.chunk_scores + (size_t)a.slab * G * SS_CHUNK * SS_CHUNK;
         a.chunk_decay = a.chunk_state + (size_t)a.slab * H * P * N;
+        if (ss_on_tensor_cores(H, P, N, G)) {
+            if (!status) return PE_ERR_UNSUPPORTED;
+            a.chunk_planes = reinterpret_cast<unsigned char*>(a.chunk_decay);                                     // (vectors first)
+            a.chunk_decay = reinterpret_cast<float*>(a.chunk_planes + (size_t)a.slab * G * 2 * ss_plane_bytes(N));
+            a.chunk_seen = reinterpret_cast<unsigned*>(a.chunk_decay + (size_t)a.slab * H);
+            return ss_tensor_tiles(a, dtype, status, (cudaStream_t)stream);
+        }
         return ss_tiles(a, dtype, (cudaStream_t)stream);
     }
     const size_t smem = sizeof(float) * ((size_t)SS_TOKENS * (2 * NS * NRP + PT) + 2 * SS_TOKENS);

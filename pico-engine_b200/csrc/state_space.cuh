@@ -5,6 +5,11 @@
 #define SS_CHUNK 64          // tokens of a chunk of a prompt
 
 #define SS_STEP_FLOATS (4 * 64)               // of a chunk of 64 tokens and a head
+#define SS_MATRIX_STEP_FLOATS (20 * 64)       // the same for products on the tensor cores
+
+// Whether prompts' products run on the tensor cores (state_space_tcgen05.cu), and the bytes of a chunk's and group's parts of B (and of C) there.
+inline bool ss_on_tensor_cores(int H, int P, int N, int G) { return P == 64 && (N == 64 || N == 128) && H / G % 2 == 0; }
+__host__ __device__ __forceinline__ size_t ss_plane_bytes(int N) { return (size_t)(N / 64) * 3 * 8192; }
 
 struct ScanArgs {
     const float* xbc; int xbc_ld;             // [T, inner + 2 G N] float32: x | B | C after the convolution
@@ -18,6 +23,8 @@ struct ScanArgs {
     float* chunk_decay;                       // [chunks][H]: the product of a chunk's decays
     float* chunk_scores;                      // [chunks][G][64 s][64 t]: C_t . B_s
     float* chunk_steps;                       // [chunks][H][SS_STEP_FLOATS]: 64 x (dt, dt * the decays behind it), then 64 running sums (float64)
+    unsigned char* chunk_planes;              // tensor cores: [chunks][G][B, C][64 state rows at a time]: their bfloat16 parts (chunk_mma.cuh)
+    unsigned* chunk_seen;                     // [chunks][G]: what cm_watch saw of them (tile 0: B, 1: C), and from bit 16 on the first token with an entry that parts do not hold (64: none)
     int2* chunk_rows;                         // [chunks]: first packed token and number of tokens
     int chunks;                               // of the step, at most
     int first_chunk, slab;                    // those that a launch takes: from first_chunk on, `slab` of them at most
@@ -26,4 +33,15 @@ struct ScanArgs {
 __device__ __forceinline__ float ss_silu(float v) { return v / (1.0f + expf(-v)); }
 __device__ __forceinline__ float ss_softplus(float v) { return fmaxf(v, 0.f) + log1pf(expf(-fabsf(v))); }
 
+// Which sequence chunk `c` belongs to, its first packed token and its number of tokens (0: no such chunk).
+__device__ __forceinline__ void ss_find_chunk(const ScanArgs& a, int c, int& first, int& count) {
+    first = count = 0;
+    for (int b = 0; b < a.B; ++b) {
+        const int n = a.row_lens[b], nc = (n + SS_CHUNK - 1) / SS_CHUNK;
+        if (c < nc) { first = a.row_first[b] + c * SS_CHUNK; count = min(SS_CHUNK, n - c * SS_CHUNK); return; }
+        c -= nc;
+    }
+}
+
+int ss_tensor_tiles(const ScanArgs& a, int dtype, int* status, cudaStream_t s);
 int ss_tiles(const ScanArgs& a, int dtype, cudaStream_t s);     // prompts: contributions, carry, outputs

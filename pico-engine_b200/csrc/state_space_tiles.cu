@@ -14,16 +14,6 @@
 #include "state_space.cuh"
 #include "chunk_tiles.cuh"
 
-// Which sequence chunk `c` belongs to, its first packed token and its number of tokens (0: no such chunk).
-__device__ __forceinline__ void st_find_chunk(const ScanArgs& a, int c, int& first, int& count) {
-    first = count = 0;
-    for (int b = 0; b < a.B; ++b) {
-        const int n = a.row_lens[b], nc = (n + SS_CHUNK - 1) / SS_CHUNK;
-        if (c < nc) { first = a.row_first[b] + c * SS_CHUNK; count = min(SS_CHUNK, n - c * SS_CHUNK); return; }
-        c -= nc;
-    }
-}
-
 // Four heads of a chunk: its place in the packed tokens, its steps' sizes dt and weights in the state's contribution dt_s a(s, n-1), and
 // the running sums of -exp(A_log) dt (zero steps behind its tokens).  Once a chunk and head: worked out by every tile of contributions and
 // again by every tile of outputs, in front of their products, they cost both kernels a chain of searches, logarithms and sums in float64.
@@ -33,7 +23,7 @@ __global__ void __launch_bounds__(4 * SS_CHUNK) st_steps_kernel(ScanArgs a) {
     pdl_wait();
     __shared__ double sums[4][2];
     int first, n;
-    st_find_chunk(a, a.first_chunk + blockIdx.x, first, n);
+    ss_find_chunk(a, a.first_chunk + blockIdx.x, first, n);
     if (threadIdx.x == 0 && blockIdx.y == 0) a.chunk_rows[blockIdx.x] = make_int2(first, n);
     if (n <= 0) return;
     const int hh = threadIdx.x / SS_CHUNK, t = threadIdx.x % SS_CHUNK, lane = t & 31, h = blockIdx.y * 4 + hh;

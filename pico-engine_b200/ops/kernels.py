@@ -1416,7 +1416,7 @@ def state_space_scan(xbc: torch.Tensor, proj: torch.Tensor, dt_offset: int, dt_b
                                             dt_bias.data_ptr(), _code(dt_bias, "dt_bias"), a_log.data_ptr(), _code(a_log, "a_log"),
                                             d_skip.data_ptr(), _code(d_skip, "d_skip"), sp, stride, row_first.data_ptr(),
                                             row_lens.data_ptr(), slots.data_ptr(), y.data_ptr(), T, slots.shape[0], H, P, N, G,
-                                            1 if chunked else 0, ws, stream_ptr()), "state_space_scan", 4 * slabs if chunked else 1)
+                                            1 if chunked else 0, ws, status_ptr(xbc.device) if chunked else None, stream_ptr()), "state_space_scan", 4 * slabs if chunked else 1)
     return y
 
 

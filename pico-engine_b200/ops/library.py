@@ -27,7 +27,7 @@ MIXER_SOURCES = ("layernorm_conv.cu", "attention_headmix.cu", "attention_headmix
 GATED_SOURCES = ("linear_attention.cu", "linear_attention_tiles.cu", "linear_attention_channels.cu", "gated_ops.cu", "branch_ops.cu")
 # The kernels of the state-space mixer (short convolution with silu, the recurrence with a scalar decay, gate then norm) and of
 # attention over one low-rank row per position.
-STATE_SOURCES = ("state_space.cu", "state_space_tiles.cu", "latent_ops.cu", "attention_latent_tcgen05.cu")
+STATE_SOURCES = ("state_space.cu", "state_space_tiles.cu", "state_space_tcgen05.cu", "latent_ops.cu", "attention_latent_tcgen05.cu")
 # The kernels of sublayers that read the same rows and share their first and last product, of heads with several maps, and of routers
 # that read normed rows.
 JOINED_SOURCES = ("joined_ops.cu", "attention_diff.cu", "attention_diff_tcgen05.cu")
@@ -102,7 +102,7 @@ _STATE_SIGNATURES = {
     "pe_conv_silu": [P, I, I, I, I, I, P, I, P, I, P, LL, P, P, P, P, P, I, I, P],
     "pe_attention_latent_tcgen05_takes": [I, I],
     "pe_attention_latent_tcgen05": [P, I, P, P, LL, P, I, P, I, I, I, I, I, I, F, P, I, P, P],
-    "pe_state_space_scan": [P, I, P, I, I, I, P, I, P, I, P, I, P, LL, P, P, P, P, I, I, I, I, I, I, I, P, P],
+    "pe_state_space_scan": [P, I, P, I, I, I, P, I, P, I, P, I, P, LL, P, P, P, P, I, I, I, I, I, I, I, P, P, P],
     "pe_gate_norm": [P, I, I, I, P, I, I, I, P, I, F, P, P],
     "pe_latent_prepare": [P, I, I, I, I, I, I, I, I, P, I, F, P, I, P, P, P, P, P, P, I, I, I, P, I, P],
     "pe_rmsnorm_cols": [P, I, I, I, I, P, I, F, P, I, P],

@@ -708,3 +708,58 @@ def test_convolution_in_runs_of_channels(dtype, taps, C, lens):
             assert (got[at: at + n] - want).abs().max() < 1e-5, (step, b)
             past[b], at = u[-(taps - 1):], at + n
 
+
+def tensor_core_case(H, N, G, lens, seed, offset=0):
+    """Inputs of the state-space recurrence at sizes whose prompts run on the tensor cores; rows that start ``offset`` numbers off a vector."""
+    g = torch.Generator("cuda").manual_seed(seed)
+    T, width = sum(lens), H * 64 + 2 * G * N
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    xbc = torch.empty(T * width + offset, device="cuda")[offset:].view(T, width)
+    xbc.copy_(r(T, width))
+    first, rows, slots = (torch.tensor(v, dtype=torch.int32).cuda() for v in (np.concatenate([[0], np.cumsum(lens)]), lens, range(len(lens))))
+    steps = r(T, H), r(H) - 1.0, 0.7 * r(H) - 0.5, 1 + 0.3 * r(H)
+
+    def run(rows_in, chunked):
+        from pico_engine.ops import kernels
+        state = torch.full((len(lens), kernels.state_space_elems(H, 64, N)), 0.5, device="cuda")
+        y = kernels.state_space_scan(rows_in, steps[0], 0, *steps[1:], state, 0, first, rows, slots, H, 64, N, G, chunked=chunked)
+        kernels.check_status(torch.device("cuda", torch.cuda.current_device()))
+        return y, state
+    return xbc, run
+
+
+@pytest.mark.parametrize("H,N,G,offset", [(2, 64, 1, 0), (2, 128, 1, 0), (12, 128, 2, 1), (10, 64, 5, 0), (6, 64, 3, 3)])
+def test_state_space_products_on_the_tensor_cores(H, N, G, offset):
+    """Chunks that end on, before and behind their 64 tokens, more units than blocks, rows off a vector: products in bfloat16 parts against the walk."""
+    lens = [1, 63, 64, 65, 128, 1000, 700, 7] + [64] * (40 if H > 6 else 1)
+    xbc, run = tensor_core_case(H, N, G, lens, H + N, offset)
+    for walk, chunks in zip(run(xbc, False), run(xbc, True)):
+        # float32 sums of the same products in another order (the bound of the tests above)
+        assert (walk - chunks).abs().max() < 3e-5 * max(1.0, float(walk.abs().max()))
+
+
+@pytest.mark.parametrize("odd", [float("nan"), float("-inf"), 3.4e38])
+@pytest.mark.parametrize("N,which", [(64, "x"), (128, "B"), (128, "C")])
+def test_numbers_that_parts_do_not_hold_stay_where_they_are(odd, N, which):
+    """A number that is none, an infinity, and one that rounds to an infinity: tokens in front keep their bits, and the places that are lost are the walk's."""
+    H, G, lens = 4, 2, [130, 40]
+    xbc, run = tensor_core_case(H, N, G, lens, N)
+    clean = run(xbc, True)[0]
+    column = {"x": 70, "B": H * 64 + 1, "C": H * 64 + G * N + 1}[which]
+    for at in (0, 5, 63, 100):
+        bad = xbc.clone()
+        bad[at, column] = odd
+        (y, s), (y_walk, s_walk) = run(bad, True), run(bad, False)
+        assert torch.equal(y[:at], clean[:at]) and torch.equal(y[lens[0]:], clean[lens[0]:]), at
+        if odd != 3.4e38:                                     # (products of it may or may not leave float32, by their order)
+            assert torch.equal(y.isfinite(), y_walk.isfinite()) and torch.equal(s.isfinite(), s_walk.isfinite()), at
+
+
+@pytest.mark.parametrize("scale", [1e-36, 1e-30, 1e30])
+def test_state_space_products_at_the_ends_of_the_range(scale):
+    """x far below and far above one: errors as large, beside the results, as at one (numbers below 2^-90 are multiplied as they are)."""
+    xbc, run = tensor_core_case(4, 128, 2, [200], 3)
+    xbc[:, :256] *= scale
+    walk, chunks = run(xbc, False)[0], run(xbc, True)[0]
+    # the state begins at 0.5: at 1e-36 nothing of x is left beside it
+    assert (walk - chunks).abs().max() < 3e-5 * float(walk.abs().max())
