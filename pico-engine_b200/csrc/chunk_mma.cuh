@@ -62,15 +62,15 @@ __device__ __forceinline__ void cm_put(unsigned char* to, int stride, const floa
 #pragma unroll
     for (int p = 0; p < CM_PARTS; ++p) *reinterpret_cast<uint4*>(to + p * stride) = make_uint4(part[p][0], part[p][1], part[p][2], part[p][3]);
 }
-// A plane of upper parts of which some is no finite number: zeros for such entries in all of its parts, `stride` bytes apart; `first` becomes the first
+// A plane of upper parts of which some is no finite number: zeros for such entries in all of its `parts`, `stride` bytes apart; `first` becomes the first
 // row that has one.  All threads.
-__device__ __forceinline__ void cm_mend(unsigned char* plane, int stride, unsigned* first) {
+__device__ __forceinline__ void cm_mend(unsigned char* plane, int stride, int parts, unsigned* first) {
 #pragma unroll 1
     for (int i = threadIdx.x; i < CM_PLANE / 4; i += blockDim.x) {
         unsigned* at = reinterpret_cast<unsigned*>(plane) + i;
         const unsigned v = *at, keep = ((v & 0x7f80u) == 0x7f80u ? 0u : 0xffffu) | ((v & 0x7f800000u) == 0x7f800000u ? 0u : 0xffff0000u);
         if (keep == 0xffffffffu) continue;
-        for (int p = 0; p < CM_PARTS; ++p) at[p * stride / 4] &= keep;
+        for (int p = 0; p < parts; ++p) at[p * stride / 4] &= keep;
         atomicMin(first, (unsigned)(i / 32));
     }
 }
@@ -81,6 +81,12 @@ __device__ __forceinline__ void cm_bring(unsigned char* dst, const void* src, in
 }
 __device__ __forceinline__ void cm_landed() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+__device__ __forceinline__ void cm_load8(float4& a, float4& b, const float* p) {
+    asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];" : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void cm_store8(float* p, const float (&v)[8]) {
+    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
+}
 // ---------------------------------------------------------------- products by tcgen05 (one warp calls, its elected thread issues)
 // An operand of 64 entries of K: descriptors of its parts (`stride` bytes apart), and how far 16 entries of K are in 16-byte units.
 struct CMOperand { unsigned long long hi, mid, lo; unsigned step; };
@@ -119,6 +125,16 @@ __device__ __forceinline__ void cm_products(unsigned elected, unsigned first, un
 #pragma unroll
     for (int k = 0; k < 4; ++k) cm_issue(elected, k < 2 ? first : rest, a.hi + k * a.step, b.hi + k * b.step, idesc, k != 0);
 }
+// The same for an A of one part (numbers that are bfloat16 already): three products.
+__device__ __forceinline__ void cm_products_one(unsigned elected, unsigned first, unsigned rest, unsigned long long a, unsigned step, const CMOperand& b, unsigned idesc) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        cm_issue(elected, rest, a + k * step, b.lo + k * b.step, idesc, k);
+        cm_issue(elected, rest, a + k * step, b.mid + k * b.step, idesc, true);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) cm_issue(elected, k < 2 ? first : rest, a + k * step, b.hi + k * b.step, idesc, k != 0);
+}
 // idesc: float32 sums of bfloat16 products, 128 rows, n columns, either operand across the rows of its planes or along them
 __device__ __forceinline__ constexpr unsigned cm_idesc(int n, bool a_across, bool b_across) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((a_across ? 1u : 0u) << 15) | ((b_across ? 1u : 0u) << 16) | ((unsigned)(n >> 3) << 17) | ((unsigned)(128 >> 4) << 24);
@@ -138,6 +154,44 @@ __device__ __forceinline__ void cm_take(float (&acc)[N], unsigned taddr) {
     for (int i = 0; i < N; ++i) acc[i] += v[i];
 }
 
+#define CM_TMEM 256                                       // columns of tensor memory a block: the two sums of 128 columns, or of two times 64
+// A block's tensor memory and the barrier that its products arrive at.
+__device__ __forceinline__ unsigned cm_begin(unsigned* tmem, unsigned long long* bar) {
+    if (threadIdx.x == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(at_smem(bar)) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (threadIdx.x < 32) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(at_smem(tmem)), "r"((unsigned)CM_TMEM) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    pdl_launch_dependents();                               // (behind the allocation: a later kernel must not take tensor memory first)
+    return *tmem;
+}
+__device__ __forceinline__ void cm_end(unsigned tmem) {
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (threadIdx.x < 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((unsigned)CM_TMEM) : "memory");
+}
+// What the block wrote to shared memory is there for the tensor core, and what it read of tensor memory has been read.
+__device__ __forceinline__ void cm_ready() {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+}
+// The block's next products have ended: one warp waits for them, the others for it (eight warps that ask the barrier again and again take the
+// other block's issue slots).  A wait that runs out leaves a status, and every later one is bounded too.
+__device__ __forceinline__ void cm_done(unsigned long long* bar, unsigned& phase, int* status) {
+    if (threadIdx.x < 32 && !at_wait_warp(at_smem(bar), phase) && threadIdx.x == 0) atomicExch(status, 11);
+    phase ^= 1;
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+}
 // ---------------------------------------------------------------- products by mma.sync (scores of a chunk's tokens over its keys)
 __device__ __forceinline__ void cm_ldmatrix(unsigned& a, unsigned& b, unsigned& c, unsigned& d, unsigned at) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "r"(at) : "memory");

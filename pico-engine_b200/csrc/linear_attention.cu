@@ -214,6 +214,10 @@ static int la_run(LAArgs a, int chunked, cudaStream_t s) {
     const dim3 carry((unsigned)((per + 255) / 256), a.B);
     constexpr int types = sizeof(T) == 4 ? 0 : sizeof(TQ) == 2 ? 1 : 2;
     for (; a.first_chunk < a.chunks; a.first_chunk += a.slab) {      // (the carry between two slabs lies in the sequences' states)
+        if (a.chunk_planes) {
+            if (const int e = la_tensor_chunks(a, types, sizeof(TZ) == 4 ? 0 : 1, s)) return e;
+            continue;
+        }
         if constexpr (PC) { if (const int e = la_channels_contributions(a, sizeof(T) == 4, sizeof(TZ) == 4, a.channel_scratch, s)) return e; }
         else if (const int e = la_tiles_contributions(a, types, s)) return e;
         PE_TRY(pe_launch(la_carry_kernel, carry, 256, 0, s, a));
@@ -241,8 +245,18 @@ extern "C" int pe_linear_attention_chunks(int T, int B) { return (T + LA_CHUNK -
 // sizes that fill it keeps the GPU full (16 heads of 128 x 128 with a decay per channel: 109 chunks, 1,744 blocks a launch), and batches of
 // prompts need no more scratch than it.
 #define LA_SCRATCH_FLOATS (64ll << 20)
+// Sizes, and then rows, whose prompts run on the tensor cores (linear_attention_tcgen05.cu): every chunked step of theirs, down to a chunk of one token.
+static bool la_tensor_sizes(int H, int D, int Dv) { return D == Dv && (D == 128 || (D == 64 && H % 2 == 0)) && H <= 65535; }
+extern "C" int pe_linear_attention_on_tensor_cores(const void* proj, int dtype, int ld, int v_off, int H, int D, int Dv) {
+    return la_tensor_sizes(H, D, Dv) && dtype == PE_BF16 && ld % 8 == 0 && v_off % 8 == 0 && (uintptr_t)proj % 16 == 0;
+}
+// Floats of scratch that a chunk takes, whichever way its step goes.
+static long long la_chunk_floats(int H, int D, int Dv, int per_channel) {
+    const long long adds = per_channel ? la_channels_scratch_floats(1, H, D) : 0, parts = la_tensor_sizes(H, D, Dv) ? la_tensor_chunk_floats(H, D) : 0;
+    return (long long)H * D * ((long long)Dv + 1) + (adds > parts ? adds : parts);
+}
 static int la_slab(int chunks, int H, int D, int Dv, int per_channel) {
-    const long long floats = (long long)H * D * ((long long)Dv + 1) + (per_channel ? la_channels_scratch_floats(1, H, D) : 0);
+    const long long floats = la_chunk_floats(H, D, Dv, per_channel);
     const long long most = floats >= LA_SCRATCH_FLOATS ? 1 : LA_SCRATCH_FLOATS / floats, slabs = (chunks + most - 1) / most;
     return (int)((chunks + slabs - 1) / slabs);
 }
@@ -252,15 +266,14 @@ extern "C" int pe_linear_attention_slabs(int T, int B, int H, int D, int Dv, int
 }
 // Floats of scratch the chunked way needs.
 extern "C" long long pe_linear_attention_scratch_floats(int T, int B, int H, int D, int Dv, int per_channel) {
-    const int slab = la_slab(pe_linear_attention_chunks(T, B), H, D, Dv, per_channel);
-    return (long long)slab * H * D * ((long long)Dv + 1) + (per_channel ? 3 + la_channels_scratch_floats(slab, H, D) : 0);
+    return la_slab(pe_linear_attention_chunks(T, B), H, D, Dv, per_channel) * la_chunk_floats(H, D, Dv, per_channel) + 8;
 }
 
 extern "C" int pe_linear_attention(const void* proj, int dtype, int ld, int q_off, int k_off, int v_off, const void* z, int z_dtype,
                                    int z_ld, const float* head_decay, float inv_tau, float q_scale, int act_qk, int act_v,
                                    float* state, long long state_stride, const int* row_first, const int* row_lens,
                                    const int* slots, float* out, int T, int B, int H, int D, int Dv, int chunked, float* scratch,
-                                   const float* qk, int qk_ld, void* stream) {
+                                   const float* qk, int qk_ld, int* status, void* stream) {
     if (T <= 0 || B <= 0) return 0;
     if ((z == nullptr) == (head_decay == nullptr) || D <= 0 || Dv <= 0 || H <= 0) return PE_ERR_UNSUPPORTED;
     if (chunked && !scratch) return PE_ERR_UNSUPPORTED;
@@ -278,6 +291,17 @@ extern "C" int pe_linear_attention(const void* proj, int dtype, int ld, int q_of
     a.chunk_state = scratch;
     a.chunk_decay = scratch ? scratch + (size_t)a.slab * H * D * Dv : nullptr;
     a.channel_scratch = scratch ? scratch + ((size_t)a.slab * H * D * ((size_t)Dv + 1) + 3) / 4 * 4 : nullptr;      // (read in vectors)
+    a.chunk_planes = nullptr;
+    if (chunked && status && pe_linear_attention_on_tensor_cores(proj, dtype, ld, v_off, H, D, Dv)) {
+        a.chunk_planes = reinterpret_cast<unsigned char*>(scratch);                                    // (vectors first)
+        a.chunk_seen = reinterpret_cast<unsigned*>(scratch + (size_t)a.slab * (la_tensor_chunk_floats(H, D) - H - 2));
+        a.chunk_rows = reinterpret_cast<int2*>(a.chunk_seen + (size_t)a.slab * H);
+        float* rest = reinterpret_cast<float*>(a.chunk_rows + a.slab);
+        a.chunk_state = scratch + ((rest - scratch) + 7) / 8 * 8;
+        a.chunk_decay = a.chunk_state + (size_t)a.slab * H * D * Dv;
+        a.status = status;
+        a.qk_f32 = qk != nullptr || dtype == PE_F32; a.z_f32 = z_dtype == PE_F32;
+    }
     cudaStream_t s = (cudaStream_t)stream;
     if (dtype == PE_F32) {
         if (!pc) return la_by_rows<float, float, float, false>(a, chunked, s);

@@ -21,6 +21,12 @@ struct LAArgs {
     int chunks;              // of the step, at most
     int first_chunk, slab;   // those that this launch takes: from first_chunk on, `slab` of them at most
     float* channel_scratch;  // with a decay per channel: weights, decayed queries and keys of every chunk
+    // on the tensor cores (linear_attention_tcgen05.cu):
+    unsigned char* chunk_planes;   // the units' queries, keys and weights as bfloat16 parts
+    unsigned* chunk_seen;          // [chunks][H]: what cm_watch saw of them
+    int2* chunk_rows;              // [chunks]: first packed token and number of tokens
+    int* status;
+    int qk_f32, z_f32;
 };
 
 // silu of a projection.  FAST (the bfloat16 engine, whose projections carry 8 bits): 2^x and the reciprocal from the
@@ -36,6 +42,16 @@ __device__ __forceinline__ float la_act(float v, int act) {
         return v * r;
     }
     return v / (1.0f + expf(-v));
+}
+
+// pw[i] = a^i for i <= 64 (a^0 = 1, also for a = 0)
+__device__ __forceinline__ void la_powers(float* pw, float a) {
+    const int i = threadIdx.x;
+    if (i <= LA_CHUNK) {
+        double r = 1.0, b = (double)a;
+        for (int e = i; e; e >>= 1) { if (e & 1) r *= b; b *= b; }
+        pw[i] = (float)r;
+    }
 }
 
 // Which sequence chunk `c` of the step belongs to, its first packed token and its number of tokens (0: no such chunk).
@@ -63,3 +79,8 @@ int la_tiles_outputs(const LAArgs& a, int types, cudaStream_t s);
 long long la_channels_scratch_floats(int chunks, int H, int D);
 int la_channels_contributions(const LAArgs& a, bool f32, bool z_f32, float* scratch, cudaStream_t s);
 int la_channels_outputs(const LAArgs& a, bool f32, float* scratch, cudaStream_t s);
+// Both on the tensor cores (linear_attention_tcgen05.cu), all of a slab's launches; the floats of scratch that a chunk takes beside its states and decays;
+// and the kernel that works out queries, keys and weights with a decay per channel.
+int la_tensor_chunks(const LAArgs& a, int types, int z_types, cudaStream_t s);
+long long la_tensor_chunk_floats(int H, int D);
+int la_channels_prepare(const LAArgs& a, bool z_f32, bool two, cudaStream_t s);

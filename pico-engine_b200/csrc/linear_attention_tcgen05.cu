@@ -1,0 +1,407 @@
+// Linear attention of prompts as products of tiles on the 5th-generation tensor cores (linear_attention_tiles.cu and
+// linear_attention_channels.cu have the same with multiply-adds, and the sums that are worked out; chunk_mma.cuh how float32 numbers are
+// multiplied).  bfloat16 rows, heads of 128 x 128, or an even number of heads of 64 x 64.
+//
+// A first kernel a kind of decay works out what does not depend on the state and leaves it as bfloat16 parts: the chunk's queries (times their decays
+// from the chunk's start, where those are a channel's), its keys times their decays to the chunk's end, and its weights q_t . A(s, t) k_s.
+// A unit is a chunk and 128 value columns, one head's or two heads', which stand on the accumulator's lanes:
+//   contributions  L^T [v][d] = v^T K          K: the chunk's tokens
+//   outputs        o^T [v][t] = S^T Q^T (times the decay to t, where it is a head's) + v^T W^T      K: the state's rows, 64 at a time; then the tokens
+// Values that no activation is applied to are bfloat16 numbers as they are: one part, half of the products.  Of two heads the products hold what either's
+// columns give with the other's rows too, which is left.
+//
+// A state in scratch is [half of the unit's columns][D / 8][64 v][8 d], so that a thread writes and reads runs of 32 bytes and a warp whole lines.
+//
+// Contributions and outputs only copy, multiply and store (outputs cut the state): what bounds them is the parts' way from L2.  Measured on a B200, 2,048
+// tokens, 16 heads of 128 x 128, us: a decay a head and silu on queries, keys and values 122 as multiply-adds, 92 here (operands 35,
+// contributions 15, carry 10, outputs 29); a decay a channel 175 and 128 (79, 12, 10, 23).  14 heads of 64: 57 and 43, 76 and 63; 200 tokens of those 34 and
+// 26, 43 and 36; three prompts of 300, 500 and 33, 16 heads 67 and 48, 92 and 67: these sizes always come here.  Errors against 64 bits, of the
+// outputs' norm: 2.1e-7 as multiply-adds and 6.3e-8 here, with a decay a channel 2.0e-7 and 1.6e-7 (its weights are the same sums); of the states 1.0e-7 and 6.1e-8,
+// 1.44e-7 and 1.28e-7.
+#include "linear_attention_parts.cuh"
+
+#define LM_THREADS 256
+#define LM_SMEM (12 * CM_PLANE + 1024)                    // parts of Q (or of W) and of S (or the values), both halves
+
+// A chunk's inputs, for what is worked out number by number.
+struct LMInputs {
+    const LAArgs& a; int first, n, pc;
+    __device__ __forceinline__ float decay(int t, int h, int d) const {
+        if (!pc) return a.head_decay[h];
+        const float u = -load_as_f(a.z, a.z_f32 ? PE_F32 : PE_BF16, (size_t)(first + t) * a.z_ld + h * a.D + d);
+        return expf(-(fmaxf(u, 0.f) + log1pf(expf(-fabsf(u)))) * a.inv_tau);
+    }
+    __device__ __forceinline__ float qk(int off, int t, int h, int d) const { return la_act<true>(load_as_f(a.qk, a.qk_f32 ? PE_F32 : PE_BF16, (size_t)(first + t) * a.qk_ld + off + h * a.D + d), a.act_qk); }
+    __device__ __forceinline__ float v(int t, int col) const { return la_act<true>(__bfloat162float(((const bf16*)a.proj)[(size_t)(first + t) * a.ld + a.v_off + col]), a.act_v); }
+};
+// With one decay a head, a chunk and head: queries and keys through their activation, k_s a^(n-1-s), and weights q_t . k_s a^(t-s), from scores by mma.sync.
+template <typename TQ, bool TWO>
+__global__ void __launch_bounds__(512, 2) lm_prepare_kernel(LAArgs a, int vec_q) {
+    pdl_launch_dependents();
+    extern __shared__ __align__(16) unsigned char lm_mem[];
+    unsigned char *qs = lm_mem, *ks = lm_mem + 3 * CM_PLANE;          // 64 channels at a time; in the end the weights
+    __shared__ float pw[LA_CHUNK + 1];
+    __shared__ unsigned seen, from;
+    using Unit = LMUnit<TWO>;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, row = tid >> 3, group = tid & 7, h = blockIdx.y, D = a.D;
+    if (tid == 0) { seen = 0; from = LA_CHUNK; }
+    pdl_wait();
+    int seq, first, n;
+    la_find_chunk(a.row_first, a.row_lens, a.B, a.first_chunk + blockIdx.x, seq, first, n);
+    if (tid == 0 && h == 0) a.chunk_rows[blockIdx.x] = make_int2(first, n);
+    if (n <= 0) return;
+    la_powers(pw, a.head_decay[h]);
+    unsigned char* unit = Unit::of(a, blockIdx.x, h);
+    const int t0 = (warp & 3) * 16, s0 = warp < 8 ? (warp >> 2) * 32 : LA_CHUNK;
+    const bool there = row < n;
+    const TQ* src = (const TQ*)a.qk + (size_t)(first + (there ? row : 0)) * a.qk_ld + h * D + 8 * group;
+    CMScores acc;
+    acc.clear();
+    unsigned most_w = 0, most_v = 0;
+    __syncthreads();
+    const float follow = there ? pw[n - 1 - row] : 0.f;
+    for (int j = 0; j < D / 64; ++j) {
+        float q[8], k[8];
+        unsigned most[3] = {0, 0, 0};
+        lm_eight(q, src + a.q_off + 64 * j, there, vec_q);
+        lm_eight(k, src + a.k_off + 64 * j, there, vec_q);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) { q[i] = la_act<true>(q[i], a.act_qk) * a.q_scale; k[i] = la_act<true>(k[i], a.act_qk); }
+        if (j) __syncthreads();
+        lm_put(qs + cm_at(row, group), CM_PLANE, q, most[0]);
+        lm_put(ks + cm_at(row, group), CM_PLANE, k, most[1]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) k[i] *= follow;
+        const int half = (TWO ? h & 1 : j) * CM_PLANE;
+        lm_put(unit + Unit::KEYS + half + cm_at(row, group), 2 * CM_PLANE, k, most[2]);
+        cm_report(&seen, cm_seen(most[0], 0) | cm_seen(most[1], 1) | cm_seen(most[2], 4));
+        __syncthreads();
+        if (cm_odd(seen)) {
+            cm_mend(qs, CM_PLANE, CM_PARTS, &from);
+            cm_mend(ks, CM_PLANE, CM_PARTS, &from);
+            __syncthreads();
+        }
+#pragma unroll
+        for (int p = 0; p < CM_PARTS; ++p)
+            *reinterpret_cast<uint4*>(unit + Unit::QUERIES + p * 2 * CM_PLANE + half + tid * 16) = *reinterpret_cast<const uint4*>(qs + p * CM_PLANE + tid * 16);
+        if (s0 <= t0) acc.add(at_smem(qs), at_smem(ks), CM_PLANE, t0, s0);
+        lm_values(a, unit + Unit::VALUES + half + cm_at(row, group), (const bf16*)a.proj + (size_t)(first + row) * a.ld + a.v_off + h * a.Dv + 64 * j + 8 * group, there, row, &from, most_v);
+    }
+    __syncthreads();
+    if (warp < 8) {                                        // (later keys have no weight)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; e += 2) {
+                const int t = t0 + lane / 4 + 4 * e, s = s0 + 8 * j + lane % 4 * 2;
+                unsigned hi, mid, lo;
+                cm_cut(s <= t ? acc.get(j, e) * pw[t - s] : 0.f, s + 1 <= t ? acc.get(j, e + 1) * pw[t - s - 1] : 0.f, hi, mid, lo);
+                cm_watch(most_w, hi);
+                unsigned char* to = qs + cm_at(t, s >> 3) + (s & 7) * 2;
+                *reinterpret_cast<unsigned*>(to) = hi;
+                *reinterpret_cast<unsigned*>(to + CM_PLANE) = mid;
+                *reinterpret_cast<unsigned*>(to + 2 * CM_PLANE) = lo;
+            }
+    }
+    cm_report(&seen, cm_seen(most_w, 2) | lm_value_seen(most_v, a.act_v));
+    __syncthreads();
+    if (cm_odd_tile(seen, 2)) {
+        cm_mend(qs, CM_PLANE, CM_PARTS, &from);
+        __syncthreads();
+    }
+#pragma unroll
+    for (int p = 0; p < CM_PARTS; ++p)
+        *reinterpret_cast<uint4*>(unit + Unit::WEIGHTS + (p * Unit::W_HEADS + (TWO ? h & 1 : 0)) * CM_PLANE + tid * 16) = *reinterpret_cast<const uint4*>(qs + p * CM_PLANE + tid * 16);
+    if (tid == 0) a.chunk_seen[(size_t)blockIdx.x * a.H + h] = seen | from << 16;
+    if (tid < D) a.chunk_decay[((size_t)blockIdx.x * a.H + h) * D + tid] = pw[n];
+}
+
+// What stands in the words of a unit's heads (bits from 16 on: the first token that parts do not hold).
+template <bool TWO>
+__device__ __forceinline__ unsigned lm_known(const LAArgs& a, int c, int h0) {
+    const unsigned x = a.chunk_seen[(size_t)c * a.H + h0];
+    if (!TWO) return x;
+    const unsigned y = a.chunk_seen[(size_t)c * a.H + h0 + 1];
+    return ((x | y) & 0xffffu) | (min(x >> 16, y >> 16) << 16);
+}
+// The values of a unit, [half][64 tokens][64 columns], zeros behind its tokens.
+__device__ __forceinline__ void lm_bring_values(unsigned char* dst, const LAArgs& a, int first, int n, int col0) {
+    const bf16* src = (const bf16*)a.proj + (size_t)first * a.ld + a.v_off + col0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const int u = threadIdx.x + e * LM_THREADS, s = u >> 4, g = u & 15;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(at_smem(dst + (g >> 3) * CM_PLANE + cm_at(s, g & 7))), "l"(src + (size_t)min(s, n - 1) * a.ld + 8 * g), "r"(s < n ? 16 : 0) : "memory");
+    }
+}
+
+// Chunks of a unit's heads, contributions.  Nothing is cut here: the parts and values of the next unit come while this one's sums leave.
+template <bool TWO, int VALUE_PARTS>
+__global__ void __launch_bounds__(LM_THREADS, 2) lm_contribution_kernel(LAArgs a, int units) {
+    extern __shared__ unsigned char lm_raw[];
+    __shared__ __align__(8) unsigned long long bar;
+    __shared__ unsigned tmem_s;
+    using Unit = LMUnit<TWO>;
+    constexpr int ND = Unit::ND;
+    unsigned char* ks = lm_raw + (-at_smem(lm_raw) & 1023u);          // [part][two][64 s][64 d]
+    unsigned char* vs = ks + 6 * CM_PLANE;                            // [part][half][64 s][64 v]
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), per = TWO ? a.H / 2 : a.H;
+    const int q = warp & 3, hh = q >> 1, p = (q & 1) * 32 + lane;
+    const unsigned tmem = cm_begin(&tmem_s, &bar);
+    const unsigned elected = warp == 0 ? cm_elect() : 0u;
+    pdl_wait();
+    unsigned phase = 0;
+    int2 place = a.chunk_rows[blockIdx.x / per];
+    unsigned known = 0;
+    auto bring = [&](int unit) {
+        const int c = unit / per, h0 = unit % per * (TWO ? 2 : 1);
+        cm_bring(ks, Unit::of(a, c, h0) + Unit::KEYS, 6 * CM_PLANE);
+        if constexpr (VALUE_PARTS == 1) lm_bring_values(vs, a, place.x, place.y, h0 * a.Dv);
+        else cm_bring(vs, Unit::of(a, c, h0) + Unit::VALUES, 6 * CM_PLANE);
+        known = lm_known<TWO>(a, c, h0);
+    };
+    if (place.y > 0) bring(blockIdx.x);
+    for (int unit = blockIdx.x; unit < units && place.y > 0; unit += gridDim.x) {
+        const int h0 = unit % per * (TWO ? 2 : 1), next = unit + gridDim.x, first = place.x, n = place.y;
+        if (next < units) place = a.chunk_rows[next / per];
+        cm_landed();
+        cm_ready();
+        const unsigned mine = known & 0xffffu;
+        const bool parts = !cm_odd(mine) && !cm_tiny(mine);           // (every thread has read the same words)
+        if (parts) {
+            if (warp == 0) {
+                if constexpr (VALUE_PARTS == 1) cm_products_one(elected, tmem, tmem + 128, at_desc(at_smem(vs), CM_PLANE, 1024), 128u, cm_across(at_smem(ks), 2 * CM_PLANE, CM_PLANE), cm_idesc(128, true, true));
+                else cm_products(elected, tmem, tmem + 128, cm_across(at_smem(vs), 2 * CM_PLANE, CM_PLANE), cm_across(at_smem(ks), 2 * CM_PLANE, CM_PLANE), cm_idesc(128, true, true));
+                if (elected) at_commit(at_smem(&bar));
+                __syncwarp();
+            }
+            cm_done(&bar, phase, a.status);
+        } else __syncthreads();
+        if (next < units && place.y > 0) bring(next);
+        float* state = a.chunk_state + (size_t)unit * 128 * ND;
+        if (parts) {
+            const int column0 = TWO ? hh * 64 + (warp >> 2) * 32 : (warp >> 2) * 64;
+#pragma unroll
+            for (int j = 0; j < (TWO ? 2 : 4); ++j) {
+                const int column = column0 + 16 * j;
+                const unsigned at = tmem + ((unsigned)(q * 32) << 16) + column;
+                float acc[16];
+                cm_read(acc, at + 128);
+                cm_take(acc, at);
+                float* to = state + (size_t)hh * ND * 64 + ((size_t)((TWO ? column & 63 : column) / 8) * 64 + p) * 8;
+                cm_store8(to, *reinterpret_cast<const float (*)[8]>(acc));
+                cm_store8(to + 512, *reinterpret_cast<const float (*)[8]>(acc + 8));
+            }
+        } else {
+            const LMInputs in = {a, first, n, a.z != nullptr};
+#pragma unroll 1
+            for (int i = tid; i < 128 * ND; i += LM_THREADS) {
+                const int half = i / (64 * ND), d = i % (64 * ND) / 512 * 8 + i % 8, v = half * 64 + i / 8 % 64, h = TWO ? h0 + half : h0;
+                float sum = 0.f;
+                for (int t = 0; t < n; ++t) sum = fmaf(in.decay(t, h, d), sum, in.qk(a.k_off, t, h, d) * in.v(t, h0 * a.Dv + v));
+                state[i] = sum;
+            }
+        }
+    }
+    cm_end(tmem);
+}
+
+// A block eight columns of a head's state, 2 D threads: a thread four rows of a column walks the sequence's chunks in order, leaves every chunk its
+// incoming state where its own contribution was, and stores the sequence's new state.  Reads in whole runs of eight chunks and what is left apart
+// (one loop whose reads ask whether there is a chunk took twice as long in state_space_tcgen05.cu's pass of the same kind).
+__global__ void __launch_bounds__(256) lm_carry_kernel(LAArgs a) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int b = blockIdx.y, tid = threadIdx.x, D = a.D, eights = a.Dv / 8, h = blockIdx.x / eights, v = blockIdx.x % eights * 8 + tid / 2 % 8, d0 = tid / 16 * 8 + tid % 2 * 4;
+    int base = 0;
+    for (int i = 0; i < b; ++i) base += (a.row_lens[i] + LA_CHUNK - 1) / LA_CHUNK;
+    int nc = (a.row_lens[b] + LA_CHUNK - 1) / LA_CHUNK;
+    const int end = min(base + nc - a.first_chunk, a.slab);           // the sequence's chunks of this slab, by their places in it
+    base = max(base - a.first_chunk, 0);
+    nc = end - base;
+    if (nc <= 0) return;
+    const size_t per = (size_t)a.H * D * a.Dv / 4;
+    float4* chunks = reinterpret_cast<float4*>(a.chunk_state + ((size_t)h * a.Dv + v / 64 * 64) * D + ((size_t)(d0 / 8) * 64 + v % 64) * 8 + d0 % 8) + (size_t)base * per;
+    const float4* decay = reinterpret_cast<const float4*>(a.chunk_decay + ((size_t)base * a.H + h) * D + d0);
+    const size_t per_decay = (size_t)a.H * D / 4;
+    float4 own[8], dec[8];
+    auto ask = [&](int m) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (u < m) { own[u] = chunks[u * per]; dec[u] = decay[u * per_decay]; }
+    };
+    if (nc >= 8) ask(8);
+    else ask(nc);
+    float* sp = a.state + (size_t)a.slots[b] * a.state_stride + ((size_t)h * D + d0) * a.Dv + v;
+    float4 carry = make_float4(sp[0], sp[a.Dv], sp[2 * a.Dv], sp[3 * a.Dv]);
+    auto step = [&](int m) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (u < m) {
+                chunks[u * per] = carry;
+                carry = make_float4(fmaf(dec[u].x, carry.x, own[u].x), fmaf(dec[u].y, carry.y, own[u].y), fmaf(dec[u].z, carry.z, own[u].z), fmaf(dec[u].w, carry.w, own[u].w));
+            }
+    };
+    while (nc >= 8) {
+        step(8);
+        nc -= 8; chunks += 8 * per; decay += 8 * per_decay;
+        if (nc >= 8) ask(8);
+        else ask(nc);
+    }
+    step(nc);
+    sp[0] = carry.x; sp[a.Dv] = carry.y; sp[2 * a.Dv] = carry.z; sp[3 * a.Dv] = carry.w;
+}
+
+// Chunks of a unit's heads, outputs: the next unit's first rows of the state are asked for while this one's last products run, its queries come when
+// these have ended.
+template <bool TWO, int VALUE_PARTS>
+__global__ void __launch_bounds__(LM_THREADS, 2) lm_output_kernel(LAArgs a, int units) {
+    extern __shared__ unsigned char lm_raw[];
+    __shared__ __align__(8) unsigned long long bar;
+    __shared__ unsigned tmem_s, odd_state, from_s;
+    __shared__ __align__(16) float es[TWO ? 2 : 1][LA_CHUNK];
+    using Unit = LMUnit<TWO>;
+    constexpr int ND = Unit::ND, SLABS = TWO ? 1 : 2;
+    unsigned char* ss = lm_raw + (-at_smem(lm_raw) & 1023u);          // [part][half][64 v][64 d] of the state; then the values, [part][half][64 s][64 v]
+    unsigned char* qs = ss + 6 * CM_PLANE;                            // [part][two][64 t][64 d]; then the weights, [part][heads][64 t][64 s]
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), per = TWO ? a.H / 2 : a.H, ld_out = a.H * a.Dv;
+    const int q = warp & 3, hh = q >> 1, p = (q & 1) * 32 + lane, column = (warp >> 2) * 32;
+    const bool scaled = a.z == nullptr;                               // one decay a head: the decay to a token behind the products
+    const unsigned tmem = cm_begin(&tmem_s, &bar), mine = tmem + ((unsigned)(q * 32) << 16) + column + (TWO ? hh * 64 : 0);
+    const unsigned elected = warp == 0 ? cm_elect() : 0u;
+    pdl_wait();
+    unsigned phase = 0, known = 0;
+    int2 place = a.chunk_rows[blockIdx.x / per];
+    float4 v[4][2];
+    auto fetch_state = [&](int unit, int slab) {
+        const float* state = a.chunk_state + (size_t)unit * 128 * ND + ((size_t)(slab * 8 + (tid >> 6)) * 64 + (tid & 63)) * 8;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) cm_load8(v[e][0], v[e][1], state + (size_t)(e >> 1) * ND * 64 + (e & 1) * 4 * 512);
+    };
+    auto bring_queries = [&](int unit) {
+        const int c = unit / per, h0 = unit % per * (TWO ? 2 : 1);
+        cm_bring(qs, Unit::of(a, c, h0) + Unit::QUERIES, 6 * CM_PLANE);
+        known = lm_known<TWO>(a, c, h0);
+    };
+    fetch_state(blockIdx.x, 0);
+    if (place.y > 0) bring_queries(blockIdx.x);
+    for (int unit = blockIdx.x; unit < units && place.y > 0; unit += gridDim.x) {
+        const int c = unit / per, h0 = unit % per * (TWO ? 2 : 1), next = unit + gridDim.x, first = place.x, n = place.y;
+        if (next < units) place = a.chunk_rows[next / per];
+        const unsigned seen = known & 0xffffu, from = known >> 16;
+        if (tid == 0) { odd_state = 0; from_s = from; }
+        if (scaled && tid < (TWO ? 2 : 1) * LA_CHUNK) {
+            double r = 1.0, by = (double)a.head_decay[h0 + (tid >> 6)];
+            for (int e = (tid & 63) + 1; e; e >>= 1) { if (e & 1) r *= by; by *= by; }
+            es[tid >> 6][tid & 63] = (float)r;
+        }
+        unsigned most = 0;
+        for (int slab = 0; slab < SLABS; ++slab) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) cm_put(ss + (e >> 1) * CM_PLANE + cm_at(tid & 63, (e & 1) * 4 + (tid >> 6)), 2 * CM_PLANE, v[e][0], v[e][1], most);
+            if (slab == 0) cm_landed();
+            cm_ready();
+            if (warp == 0) {
+                if constexpr (TWO) cm_products(elected, tmem, tmem + 128, cm_along(at_smem(ss), 2 * CM_PLANE), cm_along(at_smem(qs), 2 * CM_PLANE), cm_idesc(128, false, false));
+                else cm_products(elected, tmem + 128 * slab, tmem + 128 * slab + 64, cm_along(at_smem(ss), 2 * CM_PLANE), cm_along(at_smem(qs) + slab * CM_PLANE, 2 * CM_PLANE), cm_idesc(64, false, false));
+                if (elected) at_commit(at_smem(&bar));
+                __syncwarp();
+            }
+            if (slab + 1 < SLABS) fetch_state(unit, 1);
+            cm_done(&bar, phase, a.status);
+        }
+        cm_report(&odd_state, cm_seen(most, 0));
+        if constexpr (VALUE_PARTS == 1) lm_bring_values(ss, a, first, n, h0 * a.Dv);
+        else cm_bring(ss, Unit::of(a, c, h0) + Unit::VALUES, 6 * CM_PLANE);
+        cm_bring(qs, Unit::of(a, c, h0) + Unit::WEIGHTS, 3 * Unit::W_HEADS * CM_PLANE);
+        float acc[32];
+        cm_read(acc, mine + (TWO ? 128 : 64));
+        cm_take(acc, mine);
+        if constexpr (!TWO) { cm_take(acc, mine + 192); cm_take(acc, mine + 128); }
+        if (scaled) {
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) {
+                const float4 d = *reinterpret_cast<const float4*>(&es[TWO ? hh : 0][column + i]);
+                acc[i] *= d.x; acc[i + 1] *= d.y; acc[i + 2] *= d.z; acc[i + 3] *= d.w;
+            }
+        }
+        cm_landed();
+        cm_ready();
+        const int exact = cm_odd(odd_state) || cm_tiny(odd_state) || cm_tiny(seen & ~(7u << 12)) ? 0 : min(n, (int)from);      // tokens in front of it have their outputs from the parts
+        if (cm_odd_tile(seen, 3)) {
+            cm_mend(ss, 2 * CM_PLANE, VALUE_PARTS, &from_s);
+            cm_mend(ss + CM_PLANE, 2 * CM_PLANE, VALUE_PARTS, &from_s);
+            cm_ready();
+        }
+        if (warp == 0) {
+            constexpr int SUM = TWO ? 128 : 64;
+            const CMOperand weights = cm_along(at_smem(qs), Unit::W_HEADS * CM_PLANE);
+            if constexpr (VALUE_PARTS == 1) cm_products_one(elected, tmem, tmem + SUM, at_desc(at_smem(ss), CM_PLANE, 1024), 128u, weights, cm_idesc(SUM, true, false));
+            else cm_products(elected, tmem, tmem + SUM, cm_across(at_smem(ss), 2 * CM_PLANE, CM_PLANE), weights, cm_idesc(SUM, true, false));
+            if (elected) at_commit(at_smem(&bar));
+            __syncwarp();
+        }
+        if (next < units) fetch_state(next, 0);
+        cm_done(&bar, phase, a.status);
+        if (next < units && place.y > 0) bring_queries(next);
+        cm_take(acc, mine + (TWO ? 128 : 64));
+        cm_take(acc, mine);
+        float* out = a.out + (size_t)(first + column) * ld_out + h0 * a.Dv + hh * 64 + p;
+        if (exact == LA_CHUNK) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) out[i * ld_out] = acc[i];
+        } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+                if (column + i < exact) out[i * ld_out] = acc[i];
+            if (exact < n && tid < 128) {                  // a column a thread: the walk over the chunk's tokens, row by row of the state
+                const int h = TWO ? h0 + (tid >> 6) : h0;
+                const LMInputs in = {a, first, n, a.z != nullptr};
+                const float* state = a.chunk_state + (size_t)unit * 128 * ND + (size_t)(tid >> 6) * ND * 64 + (tid & 63) * 8;
+                float* to = a.out + (size_t)first * ld_out + h0 * a.Dv + tid;
+                for (int t = exact; t < n; ++t) to[(size_t)t * ld_out] = 0.f;
+#pragma unroll 1
+                for (int d = 0; d < ND; ++d) {
+                    float s = state[(size_t)(d / 8) * 512 + d % 8];
+#pragma unroll 1
+                    for (int t = 0; t < n; ++t) {
+                        s = fmaf(in.decay(t, h, d), s, in.qk(a.k_off, t, h, d) * in.v(t, h0 * a.Dv + tid));
+                        if (t >= exact) to[(size_t)t * ld_out] = fmaf(s, in.qk(a.q_off, t, h, d) * a.q_scale, to[(size_t)t * ld_out]);
+                    }
+                }
+            }
+        }
+    }
+    cm_end(tmem);
+}
+
+template <bool TWO, int VP>
+static int lm_run(LAArgs a, int types, int z_types, cudaStream_t s) {
+    const int units = a.slab * (TWO ? a.H / 2 : a.H), blocks = units < 2 * 148 ? units : 2 * 148;
+    PE_TRY(cudaFuncSetAttribute(lm_contribution_kernel<TWO, VP>, cudaFuncAttributeMaxDynamicSharedMemorySize, LM_SMEM));
+    PE_TRY(cudaFuncSetAttribute(lm_output_kernel<TWO, VP>, cudaFuncAttributeMaxDynamicSharedMemorySize, LM_SMEM));
+    if (a.z) { if (const int e = la_channels_prepare(a, z_types == 0, TWO, s)) return e; }
+    else {
+        const int size = types == 2 ? 4 : 2;
+        const int vec_q = (uintptr_t)a.qk % 16 == 0 && a.qk_ld * size % 16 == 0 && a.q_off * size % 16 == 0 && a.k_off * size % 16 == 0;
+        auto kernel = types == 2 ? lm_prepare_kernel<float, TWO> : lm_prepare_kernel<bf16, TWO>;
+        PE_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 6 * CM_PLANE));
+        PE_TRY(pe_launch(kernel, dim3(a.slab, a.H), 512, 6 * CM_PLANE, s, a, vec_q));
+        PE_LAUNCH_CHECK();
+    }
+    PE_TRY(pe_launch(lm_contribution_kernel<TWO, VP>, blocks, LM_THREADS, LM_SMEM, s, a, units));
+    PE_LAUNCH_CHECK();
+    PE_TRY(pe_launch(lm_carry_kernel, dim3(a.H * a.Dv / 8, a.B), 2 * a.D, 0, s, a));
+    PE_LAUNCH_CHECK();
+    PE_TRY(pe_launch(lm_output_kernel<TWO, VP>, blocks, LM_THREADS, LM_SMEM, s, a, units));
+    PE_LAUNCH_CHECK();
+    return 0;
+}
+
+long long la_tensor_chunk_floats(int H, int D) {                      // a chunk's parts, words and place
+    const long long parts = D == 128 ? (long long)H * LMUnit<false>::BYTES : (long long)H / 2 * LMUnit<true>::BYTES;
+    return parts / 4 + H + 2;
+}
+int la_tensor_chunks(const LAArgs& a, int types, int z_types, cudaStream_t s) {
+    if (a.act_v) return a.D == 64 ? lm_run<true, 3>(a, types, z_types, s) : lm_run<false, 3>(a, types, z_types, s);
+    return a.D == 64 ? lm_run<true, 1>(a, types, z_types, s) : lm_run<false, 1>(a, types, z_types, s);
+}

@@ -37,16 +37,6 @@ __device__ __forceinline__ void lt_fma4(float4& acc, float a, const float4& b) {
         : "+f"(acc.x), "+f"(acc.y), "+f"(acc.z), "+f"(acc.w) : "f"(a), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w));
 }
 
-// pw[i] = a^i for i <= 64 (a^0 = 1, also for a = 0)
-__device__ __forceinline__ void lt_powers(float* pw, float a) {
-    const int i = threadIdx.x;
-    if (i <= LA_CHUNK) {
-        double r = 1.0, b = (double)a;
-        for (int e = i; e; e >>= 1) { if (e & 1) r *= b; b *= b; }
-        pw[i] = (float)r;
-    }
-}
-
 // A thread's share of [64][TW] entries of a chunk (columns c0 .. of every token's run at `src`), zeros behind its tokens and behind the
 // head's columns: all of it is asked for before any of it is used.
 template <typename T, int TW>
@@ -97,7 +87,7 @@ __global__ void __launch_bounds__(LT_THREADS) lt_contribution_kernel(LAArgs a, i
     LTRows<T, TV> v_rows;
     k_rows.load((const TQ*)a.qk + (size_t)first * a.qk_ld + a.k_off + h * a.D + d0, a.qk_ld, n, a.D - d0, vec_q);
     v_rows.load((const T*)a.proj + (size_t)first * a.ld + a.v_off + h * a.Dv + c0, a.ld, n, a.Dv - c0, vec_v);
-    lt_powers(pw, a.head_decay[h]);
+    la_powers(pw, a.head_decay[h]);
     __syncthreads();
     k_rows.template store<FAST>(ks, a.act_qk, [&](int t) { return t < n ? pw[n - 1 - t] : 0.f; });
     v_rows.template store<FAST>(vs, a.act_v, [](int) { return 1.f; });
@@ -163,7 +153,7 @@ __global__ void __launch_bounds__(LT_THREADS, 2) lt_output_kernel(LAArgs a, int 
     if (n <= 0) return;
     LTRows<T, TV> v_rows;
     v_rows.load((const T*)a.proj + (size_t)first * a.ld + a.v_off + h * a.Dv + c0, a.ld, n, a.Dv - c0, vec_v);
-    lt_powers(pw, a.head_decay[h]);
+    la_powers(pw, a.head_decay[h]);
     // a lane a token: four entries are read as a run and stored to four columns, neighbouring lanes side by side
 #pragma unroll 4
     for (int u = warp; u < 2 * (DP / 4); u += LT_THREADS / 32) {

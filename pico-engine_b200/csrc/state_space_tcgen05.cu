@@ -31,16 +31,9 @@
 #define SM_FACTOR 128
 #define SM_RUNS 256
 #define SM_INSIDE (256 + 8 * SS_CHUNK)
-#define SM_TMEM 256                                       // the two sums of 128 columns, or of two slabs of 64
 #define SM_CONTRIBUTION_SMEM (4 * SM_SLAB + 1024)
 #define SM_OUTPUT_SMEM (4 * SM_SLAB + 1024)
 
-__device__ __forceinline__ void sm_load8(float4& a, float4& b, const float* p) {
-    asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];" : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w) : "l"(p) : "memory");
-}
-__device__ __forceinline__ void sm_store8(float* p, const float (&v)[8]) {
-    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
-}
 __device__ __forceinline__ float4 sm_times(const float4& v, float w) { return make_float4(v.x * w, v.y * w, v.z * w, v.w * w); }
 
 // A chunk's place and where its numbers are read: those of two heads from h on, and their group's B and C.
@@ -95,8 +88,8 @@ __global__ void __launch_bounds__(SM_THREADS) sm_steps_kernel(ScanArgs a, int ve
             cm_report(&seen, cm_seen(most[0], 0) | cm_seen(most[1], 1));
             __syncthreads();
             if (cm_odd(seen)) {
-                cm_mend(sm_mem, CM_PLANE, &from);
-                cm_mend(sm_mem + SM_SLAB, CM_PLANE, &from);
+                cm_mend(sm_mem, CM_PLANE, CM_PARTS, &from);
+                cm_mend(sm_mem + SM_SLAB, CM_PLANE, CM_PARTS, &from);
                 __syncthreads();
             }
             unsigned char* to = planes + (size_t)(k0 / 64) * SM_SLAB;
@@ -156,48 +149,11 @@ __global__ void __launch_bounds__(SM_THREADS) sm_steps_kernel(ScanArgs a, int ve
         runs[i] = i < t >> 3 ? expf((float)(la - las[hh][8 * i + 7])) : 0.f;
         inside[i] = s <= t ? dts[hh][s] * expf((float)(la - las[hh][s])) : 0.f;
     }
-    sm_store8(dst + SM_RUNS + 8 * t, runs);
-    sm_store8(dst + SM_INSIDE + 8 * t, inside);
+    cm_store8(dst + SM_RUNS + 8 * t, runs);
+    cm_store8(dst + SM_INSIDE + 8 * t, inside);
     if (t == 0) a.chunk_decay[(size_t)blockIdx.x * a.H + h] = expf((float)end);
 }
 
-// A block's tensor memory and the barrier that its products arrive at.
-__device__ __forceinline__ unsigned sm_begin(unsigned* tmem, unsigned long long* bar) {
-    if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(at_smem(bar)) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (threadIdx.x < 32) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(at_smem(tmem)), "r"((unsigned)SM_TMEM) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    pdl_launch_dependents();                               // (behind the allocation: a later kernel must not take tensor memory first)
-    return *tmem;
-}
-__device__ __forceinline__ void sm_end(unsigned tmem) {
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (threadIdx.x < 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((unsigned)SM_TMEM) : "memory");
-}
-// What the block wrote to shared memory is there for the tensor core, and what it read of tensor memory has been read.
-__device__ __forceinline__ void sm_ready() {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-// The block's next products have ended: one warp waits for them, the others for it (eight warps that ask the barrier again and again take the
-// other block's issue slots).  A wait that runs out leaves a status, and every later one is bounded too.
-__device__ __forceinline__ void sm_done(unsigned long long* bar, unsigned& phase, int* status) {
-    if (threadIdx.x < 32 && !at_wait_warp(at_smem(bar), phase) && threadIdx.x == 0) atomicExch(status, 11);
-    phase ^= 1;
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
 // Chunks and two heads at a time, contributions: the next unit's x is asked for while this one's products run.
 __global__ void __launch_bounds__(SM_FEW, 2) sm_contribution_kernel(ScanArgs a, int vec, int units, int* status) {
     extern __shared__ unsigned char sm_raw[];
@@ -208,7 +164,7 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_contribution_kernel(ScanArgs a, 
     unsigned char* bs = xs + 2 * SM_SLAB;                             // [slab][part][64 s][64 n]
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), H = a.H, N = a.N, pairs = H / 2, slabs = N / 64;
     const int q = warp & 3, hh = q >> 1, p = (q & 1) * 32 + lane, row = tid >> 3, group = tid & 7;      // a thread's runs of eight: this row and the one 32 behind, of either head
-    const unsigned tmem = sm_begin(&tmem_s, &bar);
+    const unsigned tmem = cm_begin(&tmem_s, &bar);
     const unsigned elected = warp == 0 ? cm_elect() : 0u;
     pdl_wait();
     unsigned phase = 0, known = 0;
@@ -241,7 +197,7 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_contribution_kernel(ScanArgs a, 
         }
         cm_report(&seen, cm_seen(most, 2));
         cm_landed();
-        sm_ready();
+        cm_ready();
         const bool parts = !cm_odd(seen) && !cm_tiny(seen);
         if (parts && warp == 0) {
             cm_products(elected, tmem, tmem + N, cm_across(at_smem(xs), 2 * CM_PLANE, CM_PLANE), cm_across(at_smem(bs), CM_PLANE, SM_SLAB), cm_idesc(N, true, true));
@@ -251,7 +207,7 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_contribution_kernel(ScanArgs a, 
         if (next < units && place.y > 0) fetch(next, place);
         float* state = a.chunk_state + ((size_t)c * H + h0) * N * 64;
         if (parts) {
-            sm_done(&bar, phase, status);
+            cm_done(&bar, phase, status);
             for (int j = 0; j < 2 * slabs; ++j) {
                 const int column = (warp >> 2) * (N / 2) + 16 * j;
                 const unsigned mine = tmem + ((unsigned)(q * 32) << 16) + column;
@@ -259,8 +215,8 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_contribution_kernel(ScanArgs a, 
                 cm_read(acc, mine + N);
                 cm_take(acc, mine);
                 float* to = state + (size_t)hh * N * 64 + ((size_t)(column / 8) * 64 + p) * 8;
-                sm_store8(to, *reinterpret_cast<const float (*)[8]>(acc));
-                sm_store8(to + 512, *reinterpret_cast<const float (*)[8]>(acc + 8));
+                cm_store8(to, *reinterpret_cast<const float (*)[8]>(acc));
+                cm_store8(to + 512, *reinterpret_cast<const float (*)[8]>(acc + 8));
             }
         } else {
 #pragma unroll 1
@@ -273,7 +229,7 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_contribution_kernel(ScanArgs a, 
             __syncthreads();                               // (the weights have been read)
         }
     }
-    sm_end(tmem);
+    cm_end(tmem);
 }
 
 // A block eight columns of a head's state, 2 N threads: a thread four entries (rows r .. r + 3 of a column) walks the sequence's chunks in order, leaves
@@ -351,7 +307,7 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_output_kernel(ScanArgs a, int ve
     unsigned char* wgt = mem + 2 * SM_SLAB;                           // [part][head][64 t][64 s]
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), H = a.H, N = a.N, inner = H * 64, pairs = H / 2, slabs = N / 64;
     const int q = warp & 3, hh = q >> 1, p = (q & 1) * 32 + lane, column = (warp >> 2) * 32, row = tid >> 3, group = tid & 7;
-    const unsigned tmem = sm_begin(&tmem_s, &bar), mine = tmem + ((unsigned)(q * 32) << 16) + column;
+    const unsigned tmem = cm_begin(&tmem_s, &bar), mine = tmem + ((unsigned)(q * 32) << 16) + column;
     const unsigned elected = warp == 0 ? cm_elect() : 0u;
     pdl_wait();
     unsigned phase = 0, known = 0;
@@ -361,7 +317,7 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_output_kernel(ScanArgs a, int ve
     auto fetch_state = [&](int unit, int slab) {
         const float* state = a.chunk_state + ((size_t)(unit / pairs) * H + unit % pairs * 2) * N * 64 + ((size_t)(slab * 8 + (tid >> 6)) * 64 + (tid & 63)) * 8;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) sm_load8(v[e][0], v[e][1], state + (size_t)(e >> 1) * N * 64 + (e & 1) * 4 * 512);
+        for (int e = 0; e < 4; ++e) cm_load8(v[e][0], v[e][1], state + (size_t)(e >> 1) * N * 64 + (e & 1) * 4 * 512);
     };
     auto fetch = [&](int unit) {                           // what a unit begins with
         fetch_state(unit, 0);
@@ -384,7 +340,7 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_output_kernel(ScanArgs a, int ve
 #pragma unroll
             for (int e = 0; e < 4; ++e) cm_put(ss + (e >> 1) * CM_PLANE + cm_at(tid & 63, (e & 1) * 4 + (tid >> 6)), 2 * CM_PLANE, v[e][0], v[e][1], most_s);
             if (slab == 0) cm_landed();
-            sm_ready();
+            cm_ready();
             if (warp == 0) {
                 cm_products(elected, tmem + 128 * slab, tmem + 128 * slab + 64, cm_along(at_smem(ss), 2 * CM_PLANE), cm_along(at_smem(cs) + slab * SM_SLAB, CM_PLANE), cm_idesc(64, false, false));
                 if (elected) at_commit(at_smem(&bar));
@@ -395,7 +351,7 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_output_kernel(ScanArgs a, int ve
 #pragma unroll
                 for (int e = 0; e < 4; ++e) chunk.eight(v[e][0], v[e][1], chunk.x + (e >> 1) * 64, row + (e & 1) * 32, 8 * group);
             }
-            sm_done(&bar, phase, status);
+            cm_done(&bar, phase, status);
         }
         float4 score[2][2];                                // (both heads')
 #pragma unroll
@@ -439,14 +395,14 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_output_kernel(ScanArgs a, int ve
             cm_put(wgt + k * CM_PLANE + cm_at(t, group), 2 * CM_PLANE, make_float4(w[0], w[1], w[2], w[3]), make_float4(w[4], w[5], w[6], w[7]), most_w);
         }
         cm_report(&seen, cm_seen(most_s, 2) | cm_seen(most_x, 3) | cm_seen(most_w, 4));
-        sm_ready();
+        cm_ready();
         if (cm_odd(seen)) {
 #pragma unroll 1
             for (int k = 0; k < 2; ++k) {
-                cm_mend(xs + k * CM_PLANE, 2 * CM_PLANE, &from);
-                cm_mend(wgt + k * CM_PLANE, 2 * CM_PLANE, &from);
+                cm_mend(xs + k * CM_PLANE, 2 * CM_PLANE, CM_PARTS, &from);
+                cm_mend(wgt + k * CM_PLANE, 2 * CM_PLANE, CM_PARTS, &from);
             }
-            sm_ready();
+            cm_ready();
         }
         if (warp == 0) {
             cm_products(elected, tmem, tmem + 128, cm_across(at_smem(xs), 2 * CM_PLANE, CM_PLANE), cm_along(at_smem(wgt), 2 * CM_PLANE), cm_idesc(128, true, false));
@@ -456,7 +412,7 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_output_kernel(ScanArgs a, int ve
         float* y = a.y + (size_t)(first + column) * inner + (h0 + hh) * 64 + p;
         const int exact = cm_odd_tile(seen, 2) || cm_tiny(seen) ? 0 : min(n, (int)from);      // tokens in front of it have their outputs from the parts
         if (next < units) fetch(next);
-        sm_done(&bar, phase, status);
+        cm_done(&bar, phase, status);
         cm_take(acc, mine + hh * 64);
         cm_take(acc, mine + hh * 64 + 128);
         if (exact == SS_CHUNK) {
@@ -486,7 +442,7 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_output_kernel(ScanArgs a, int ve
             __syncthreads();                               // (the steps have been read)
         }
     }
-    sm_end(tmem);
+    cm_end(tmem);
 }
 
 template <typename T>

@@ -1140,7 +1140,7 @@ def linear_attention(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, n_h
     ``q_off``, ``k_off``, ``v_off`` of proj [T, ld] (packed sequences).  The decay is ``head_decay`` [H] float32 (one constant
     a head) or sigmoid(``decay_logits`` [T, H * D], float32 or of proj's dtype)^``inv_tau`` (a number per key channel and token).  S [H, D, Dv] comes from
     and returns to the sequences' float32 state at ``state_offset``.  ``chunked``: prompts, in slabs of chunks of the sequences, three
-    launches a slab (four with a decay per channel); else token after token in one launch.  ``qk`` (float32 [T, ld2], with a decay per head): q and k are the columns
+    launches a slab (four with a decay per channel, and on the tensor cores); else token after token in one launch.  ``qk`` (float32 [T, ld2], with a decay per head): q and k are the columns
     ``q_off`` and ``k_off`` of these rows instead (rotated ones, that are not rounded on their way into the recurrence)."""
     T, ld = proj.shape
     H, D, Dv = n_heads, head_dim, v_head_dim
@@ -1167,18 +1167,19 @@ def linear_attention(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, n_h
     B = slots.shape[0]
     out = torch.empty(T, H * Dv, dtype=torch.float32, device=proj.device)
     lib = gated()
-    ws = None
+    ws, launches = None, 1
     if chunked:
         from .workspace import scratch
         sizes = (T, B, H, D, Dv, 0 if decay_logits is None else 1)
-        slabs = lib.pe_linear_attention_slabs(*sizes)
+        tensor_cores = lib.pe_linear_attention_on_tensor_cores(proj.data_ptr(), _code(proj, "proj"), ld, v_off, H, D, Dv)
+        launches = (4 if tensor_cores or decay_logits is not None else 3) * lib.pe_linear_attention_slabs(*sizes)
         ws = scratch("linear_attention", 4 * lib.pe_linear_attention_scratch_floats(*sizes), proj.device).data_ptr()
     check(lib.pe_linear_attention(proj.data_ptr(), _code(proj, "proj"), ld, q_off, k_off, v_off, _ptr(decay_logits),
                                   0 if decay_logits is None else _code(decay_logits, "decay_logits"), H * D, _ptr(head_decay),
                                   float(inv_tau), float(q_scale), LA_ACTIVATIONS[qk_activation], LA_ACTIVATIONS[v_activation],
                                   sp, stride, row_first.data_ptr(), row_lens.data_ptr(), slots.data_ptr(), out.data_ptr(),
-                                  T, B, H, D, Dv, 1 if chunked else 0, ws, _ptr(qk), qk_ld, stream_ptr()),
-          "linear_attention", (3 if decay_logits is None else 4) * slabs if chunked else 1)
+                                  T, B, H, D, Dv, 1 if chunked else 0, ws, _ptr(qk), qk_ld, status_ptr(proj.device) if chunked else None, stream_ptr()),
+          "linear_attention", launches)
     return out
 
 

@@ -24,7 +24,7 @@ MIXER_SOURCES = ("layernorm_conv.cu", "attention_headmix.cu", "attention_headmix
 # The kernels of gated mixers and routed feed-forwards (the linear-attention recurrence, rotation of pairs with unit norm and
 # cache write, norms over groups of channels with a gate, sums of normed branches, gated activations, the choice of experts;
 # branches that share their first and last product, and residuals of several streams).
-GATED_SOURCES = ("linear_attention.cu", "linear_attention_tiles.cu", "linear_attention_channels.cu", "gated_ops.cu", "branch_ops.cu")
+GATED_SOURCES = ("linear_attention.cu", "linear_attention_tiles.cu", "linear_attention_channels.cu", "linear_attention_tcgen05.cu", "gated_ops.cu", "branch_ops.cu")
 # The kernels of the state-space mixer (short convolution with silu, the recurrence with a scalar decay, gate then norm) and of
 # attention over one low-rank row per position.
 STATE_SOURCES = ("state_space.cu", "state_space_tiles.cu", "state_space_tcgen05.cu", "latent_ops.cu", "attention_latent_tcgen05.cu")
@@ -80,7 +80,8 @@ _MIXER_SIGNATURES = {
 }
 
 _GATED_SIGNATURES = {
-    "pe_linear_attention": [P, I, I, I, I, I, P, I, I, P, F, F, I, I, P, LL, P, P, P, P, I, I, I, I, I, I, P, P, I, P],
+    "pe_linear_attention": [P, I, I, I, I, I, P, I, I, P, F, F, I, I, P, LL, P, P, P, P, I, I, I, I, I, I, P, P, I, P, P],
+    "pe_linear_attention_on_tensor_cores": [P, I, I, I, I, I, I],
     "pe_rotary_norm_store": [P, I, I, I, I, I, I, I, P, I, I, F, P, P, P, P, P, I, I, P],
     "pe_gated_norm": [P, I, I, I, I, P, I, F, P, I, I, I, P, I, P],
     "pe_normed_sum_add": [P, P, P, P, P, I, P, P, P, P, I, I, I, I, F, F, P],

@@ -618,3 +618,62 @@ def test_a_token_that_is_no_number_does_not_reach_back_with_a_decay_per_head(whi
         assert torch.equal(o[:at], clean[:at]) and torch.equal(o[lens[0]:], clean[lens[0]:]), at
         assert torch.equal(o.isfinite(), o_walk.isfinite()) and torch.equal(s.isfinite(), s_walk.isfinite()), at
 
+
+
+def tensor_core_rows(H, D, lens, per_channel, seed, logits=torch.bfloat16):
+    """Inputs of linear attention at sizes whose prompts run on the tensor cores, and a run of them."""
+    from pico_engine.ops import kernels
+    g = torch.Generator("cuda").manual_seed(seed)
+    T, B = sum(lens), len(lens)
+    proj = torch.randn(T, 3 * H * D, generator=g, device="cuda").bfloat16()
+    decay = {"decay_logits": (2 + 2 * torch.randn(T, H * D, generator=g, device="cuda")).to(logits)} if per_channel else {"head_decay": torch.linspace(0.2, 0.999, H, device="cuda")}
+    first, rows, slots = (torch.tensor(v, dtype=torch.int32).cuda() for v in (np.concatenate([[0], np.cumsum(lens)]), lens, range(B)))
+
+    def run(proj, chunked, **more):
+        state = torch.full((B, H * D * D + 3), 0.5, device="cuda")
+        o = kernels.linear_attention(proj, 0, H * D, 2 * H * D, H, D, D, state, 3, first, rows, slots, chunked, inv_tau=1 / 16, q_scale=D ** -0.5,
+                                     qk_activation="none" if per_channel else "silu", **decay, **more)
+        kernels.check_status(torch.device("cuda", torch.cuda.current_device()))
+        return o, state[:, 3:]
+    return proj, run
+
+
+@pytest.mark.parametrize("per_channel,logits", [(False, None), (True, torch.bfloat16), (True, torch.float32)])
+@pytest.mark.parametrize("H,D", [(1, 128), (5, 128), (2, 64), (6, 64)])
+def test_linear_attention_products_on_the_tensor_cores(H, D, per_channel, logits):
+    """Chunks that end on, before and behind their 64 tokens, more units than blocks: products in bfloat16 parts against the walk."""
+    lens = [1, 63, 64, 65, 128, 1000, 700, 7] + [64] * (60 if H > 4 else 1)
+    proj, run = tensor_core_rows(H, D, lens, per_channel, H + D, logits)
+    for act in ("none", "silu"):                             # values in one part, and in three
+        for walk, chunks in zip(run(proj, False, v_activation=act), run(proj, True, v_activation=act)):
+            # float32 sums of the same products in another order (the bound of the tests above)
+            assert (walk - chunks).abs().max() < 2e-5 * max(1.0, float(walk.abs().max())), act
+
+
+def test_float32_queries_and_keys_on_the_tensor_cores():
+    """Queries and keys in float32 rows of their own, which start anywhere."""
+    H, D, lens = 2, 128, [200, 65]
+    proj, run = tensor_core_rows(H, D, lens, False, 3)
+    for pad in (0, 1):
+        qk = torch.empty(sum(lens) * 2 * H * D + pad, device="cuda")[pad:].view(sum(lens), 2 * H * D)
+        qk.copy_(torch.randn(sum(lens), 2 * H * D, generator=torch.Generator("cuda").manual_seed(5), device="cuda"))
+        for walk, chunks in zip(run(proj, False, qk=qk), run(proj, True, qk=qk)):
+            assert (walk - chunks).abs().max() < 2e-5 * max(1.0, float(walk.abs().max()))
+
+
+@pytest.mark.parametrize("odd", [float("nan"), float("inf")])
+@pytest.mark.parametrize("which", ["q", "k", "v"])
+@pytest.mark.parametrize("H,D,per_channel", [(2, 128, False), (4, 64, False), (2, 128, True), (4, 64, True)])
+def test_a_token_that_is_no_number_stays_where_it_is_on_the_tensor_cores(H, D, per_channel, which, odd):
+    """Tokens in front of it and other sequences keep their bits, and the places that are lost are the walk's."""
+    lens = [130, 40]
+    proj, run = tensor_core_rows(H, D, lens, per_channel, 8)
+    for act in ("none", "silu"):
+        clean = run(proj, True, v_activation=act)[0]
+        column = "qkv".index(which) * H * D
+        for at in (0, 5, 63, 100):
+            bad = proj.clone()
+            bad[at, column: column + D: 3] = odd
+            (o, s), (o_walk, s_walk) = run(bad, True, v_activation=act), run(bad, False, v_activation=act)
+            assert torch.equal(o[:at], clean[:at]) and torch.equal(o[lens[0]:], clean[lens[0]:]), (at, act)
+            assert torch.equal(o.isfinite(), o_walk.isfinite()) and torch.equal(s.isfinite(), s_walk.isfinite()), (at, act)
