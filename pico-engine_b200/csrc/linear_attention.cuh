@@ -79,8 +79,6 @@ int la_tiles_outputs(const LAArgs& a, int types, cudaStream_t s);
 long long la_channels_scratch_floats(int chunks, int H, int D);
 int la_channels_contributions(const LAArgs& a, bool f32, bool z_f32, float* scratch, cudaStream_t s);
 int la_channels_outputs(const LAArgs& a, bool f32, float* scratch, cudaStream_t s);
-// Both on the tensor cores (linear_attention_tcgen05.cu), all of a slab's launches; the floats of scratch that a chunk takes beside its states and decays;
-// and the kernel that works out queries, keys and weights with a decay per channel.
+// Both on the tensor cores (linear_attention_tcgen05.cu), all of a slab's launches; and the floats of scratch that a chunk takes beside its states and decays.
 int la_tensor_chunks(const LAArgs& a, int types, int z_types, cudaStream_t s);
 long long la_tensor_chunk_floats(int H, int D);
-int la_channels_prepare(const LAArgs& a, bool z_f32, bool two, cudaStream_t s);

@@ -11,11 +11,10 @@
 //
 // Bound by float32 multiply-adds (fma.rn.f32x2) and, in the first kernel, by the decays' exponentials and logarithms.  2,048 tokens, 16
 // heads of 128 x 128, on a B200: 258 us as two walks of every chunk, 160 us here (weights 71, contributions 39, outputs 50); the
-// logits come as the product before wrote them (as float32 they were converted first, 10.5 us).  bfloat16 rows of heads of 64 x 64 and 128 x 128 take
-// their products to the tensor cores (linear_attention_tcgen05.cu) and come here for queries, keys and weights only: with 512 threads a block, the parts included, 79 us.
+// logits come as the product before wrote them (as float32 they were converted first, 10.5 us).  bfloat16 rows of heads of 64 x 64 and 128 x 128 go
+// another way (linear_attention_tcgen05.cu).
 #include "linear_attention.cuh"
 #include "chunk_tiles.cuh"
-#include "linear_attention_parts.cuh"
 
 #define LC_THREADS 256
 #define LC_RUN 16
@@ -48,81 +47,24 @@ __device__ __forceinline__ void lc_write16(float* p, const float (&v)[LC_RUN]) {
     for (int t = 0; t < LC_RUN; t += 4) *reinterpret_cast<float4*>(p + t) = *reinterpret_cast<const float4*>(v + t);
 }
 
-// The end of lc_prepare_kernel for the tensor cores, 64 channels at a time: 512 threads, a token's run of eight each.  `planes`: 24 KB of shared
-// memory; lead: [4][D], what a run's queries are multiplied by; follow: its keys.
-template <int HEADS>
-__device__ __forceinline__ void lc_parts(const LAArgs& a, const float* qt, const float* kt, const float* whole, const float* lead, const float* follow, unsigned char* planes,
-                                         const float* weights, unsigned* seen, unsigned* from, int first, int n, int h) {
-    using Unit = LMUnit<HEADS == 2>;
-    const int tid = threadIdx.x, D = a.D, half = HEADS == 2 ? h & 1 : 0, t = tid & 63, group = tid >> 6;
-    unsigned char* unit = Unit::of(a, blockIdx.x, h);
-    auto leave = [&](unsigned char* to, int stride) {     // (whole planes, as lines)
-#pragma unroll
-        for (int p = 0; p < CM_PARTS; ++p) *reinterpret_cast<uint4*>(to + p * stride + tid * 16) = *reinterpret_cast<const uint4*>(planes + p * CM_PLANE + tid * 16);
-    };
-    unsigned most_v = 0;
-    for (int j = 0; j < D / 64; ++j) {
-        const int place = (HEADS == 2 ? half : j) * CM_PLANE;
-        for (int which = 0; which < 2; ++which) {         // queries times all decays from the chunk's start, keys times all to its end
-            unsigned most = 0;
-            float v[8];
-            const float* rows = (which ? kt : qt) + (64 * j + 8 * group) * LC_LD + t;
-            const float* by = (which ? follow : lead) + (t >> 4) * D + 64 * j + 8 * group;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = rows[i * LC_LD] * by[i];
-            lm_put(planes + cm_at(t, group), CM_PLANE, v, most);
-            cm_report(seen, cm_seen(most, which ? 4 : 0));
-            __syncthreads();
-            if (which == 0 && cm_odd_tile(*seen, 0)) {
-                cm_mend(planes, CM_PLANE, CM_PARTS, from);
-                __syncthreads();
-            }
-            leave(unit + (which ? Unit::KEYS : Unit::QUERIES) + place, 2 * CM_PLANE);
-            __syncthreads();
-        }
-        const int row = tid >> 3;
-        lm_values(a, unit + Unit::VALUES + place + cm_at(row, tid & 7), (const bf16*)a.proj + (size_t)(first + row) * a.ld + a.v_off + h * a.Dv + 64 * j + 8 * (tid & 7), row < n, row, from, most_v);
-    }
-    unsigned most = 0;
-    float v[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = 8 * group + i <= t ? weights[(8 * group + i) * ST_CHUNK + t] : 0.f;
-    lm_put(planes + cm_at(t, group), CM_PLANE, v, most);
-    cm_report(seen, cm_seen(most, 2) | lm_value_seen(most_v, a.act_v));
-    __syncthreads();
-    if (cm_odd_tile(*seen, 2)) {
-        cm_mend(planes, CM_PLANE, CM_PARTS, from);
-        __syncthreads();
-    }
-    leave(unit + Unit::WEIGHTS + half * CM_PLANE, Unit::W_HEADS * CM_PLANE);
-    if (tid == 0) a.chunk_seen[(size_t)blockIdx.x * a.H + h] = *seen | *from << 16;
-    if (tid < D) a.chunk_decay[((size_t)blockIdx.x * a.H + h) * D + tid] = ((whole[3 * D + tid] * whole[2 * D + tid]) * whole[D + tid]) * whole[tid];
-}
-
-// A chunk and head: weights [64 s][64 t], decayed queries and keys [64][D], and the product of the chunk's decays.  HEADS: 0, as float32 numbers; 1 or 2, for
-// the tensor cores: as bfloat16 parts where linear_attention_tcgen05.cu reads them, units of one or two heads (the weights lie as
-// float32 numbers where the chunk's contribution will be, until all of them are there).
-template <typename T, typename TZ, int HEADS>
-__global__ void __launch_bounds__(HEADS ? 2 * LC_THREADS : LC_THREADS, 2) lc_prepare_kernel(LAArgs a, float* weights, float* queries, float* keys, int vec_q, int vec_z) {
+// A chunk and head: weights [64 s][64 t], decayed queries and keys [64][D], and the product of the chunk's decays.
+template <typename T, typename TZ>
+__global__ void __launch_bounds__(LC_THREADS) lc_prepare_kernel(LAArgs a, float* weights, float* queries, float* keys, int vec_q, int vec_z) {
     pdl_launch_dependents();
     pdl_wait();
     constexpr bool FAST = sizeof(T) == 2;
-    constexpr int TH = HEADS ? 2 * LC_THREADS : LC_THREADS, PARTS = TH / 64;       // threads that share a run's token, and a token of the runs behind it
     extern __shared__ __align__(16) float lc_smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h = blockIdx.y, D = a.D, DP = (D + 3) / 4 * 4;
     float* qt = lc_smem;                                  // [DP][64 + 4]: queries, channel by channel
     float* kt = qt + DP * LC_LD;                          // keys
     float* at = kt + DP * LC_LD;                          // decays; one behind the chunk's tokens
     float* whole = at + DP * LC_LD;                       // [4][DP]: the product of each run's decays
-    __shared__ unsigned seen, from;
-    if (HEADS && tid == 0) { seen = 0; from = LA_CHUNK; }
     int row, first, n;
     la_find_chunk(a.row_first, a.row_lens, a.B, a.first_chunk + blockIdx.x, row, first, n);
-    if (HEADS && tid == 0 && h == 0) a.chunk_rows[blockIdx.x] = make_int2(first, n);
     if (n <= 0) return;
     // a lane a token: four channels are read as a run and stored to four rows, neighbouring lanes side by side
 #pragma unroll 2
-    for (int u = warp; u < 2 * (DP / 4); u += TH / 32) {
+    for (int u = warp; u < 2 * (DP / 4); u += LC_THREADS / 32) {
         const int t = (u & 1) * 32 + lane, d = (u >> 1) * 4;
         float4 q = make_float4(0.f, 0.f, 0.f, 0.f), k = q, z = make_float4(1.f, 1.f, 1.f, 1.f);
         if (t < n) {
@@ -142,14 +84,14 @@ __global__ void __launch_bounds__(HEADS ? 2 * LC_THREADS : LC_THREADS, 2) lc_pre
         p[0] = z.x; p[LC_LD] = z.y; p[2 * LC_LD] = z.z; p[3 * LC_LD] = z.w;
     }
     __syncthreads();
-    float* out = HEADS ? a.chunk_state + ((size_t)blockIdx.x * a.H + h) * D * a.Dv : weights + ((size_t)blockIdx.x * a.H + h) * ST_CHUNK * ST_CHUNK;
-    // inside a run: thread (run, s, a quarter or an eighth of the channels) walks the decays from s on; four or eight neighbours add up their channels
+    float* out = weights + ((size_t)blockIdx.x * a.H + h) * ST_CHUNK * ST_CHUNK;
+    // inside a run: thread (run, s, quarter of the channels) walks the decays from s on; four neighbours add up their channels
     {
-        const int u = tid / PARTS, run = u >> 4, s = u & 15, part = tid % PARTS;
+        const int run = warp >> 1, s = (warp & 1) * 8 + (lane >> 2), part = lane & 3;
         float w[LC_RUN];
 #pragma unroll
         for (int t = 0; t < LC_RUN; ++t) w[t] = 0.f;
-        for (int d = part; d < DP; d += PARTS) {
+        for (int d = part; d < DP; d += 4) {
             float q[LC_RUN], c[LC_RUN];
 #pragma unroll
             for (int t = 0; t < LC_RUN; t += 4) {
@@ -165,20 +107,22 @@ __global__ void __launch_bounds__(HEADS ? 2 * LC_THREADS : LC_THREADS, 2) lc_pre
             }
         }
 #pragma unroll
-        for (int o = 1; o < PARTS; o <<= 1)
+        for (int t = 0; t < LC_RUN; ++t) {
+            w[t] += __shfl_xor_sync(0xffffffffu, w[t], 1);
+            w[t] += __shfl_xor_sync(0xffffffffu, w[t], 2);
+        }
+        float* dst = out + (run * LC_RUN + s) * ST_CHUNK + run * LC_RUN + 4 * part;
+        float4 mine = make_float4(w[0], w[1], w[2], w[3]);
 #pragma unroll
-            for (int t = 0; t < LC_RUN; ++t) w[t] += __shfl_xor_sync(0xffffffffu, w[t], o);
-        float* dst = out + (run * LC_RUN + s) * ST_CHUNK + run * LC_RUN;
-#pragma unroll
-        for (int p = 0; p < 4; ++p)
-            if (part == p) *reinterpret_cast<float4*>(dst + 4 * p) = make_float4(w[4 * p], w[4 * p + 1], w[4 * p + 2], w[4 * p + 3]);
+        for (int p = 1; p < 4; ++p)
+            if (part == p) mine = make_float4(w[4 * p], w[4 * p + 1], w[4 * p + 2], w[4 * p + 3]);
+        *reinterpret_cast<float4*>(dst) = mine;
         // runs that s does not reach back to: no weight
-        if (!HEADS)
-            for (int t = part * 4; t < run * LC_RUN; t += 16) *reinterpret_cast<float4*>(out + (run * LC_RUN + s) * ST_CHUNK + t) = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int t = part * 4; t < run * LC_RUN; t += 16) *reinterpret_cast<float4*>(out + (run * LC_RUN + s) * ST_CHUNK + t) = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     __syncthreads();
     // queries times what leads to them in their run, keys times what follows them there; thread (channel, run)
-    for (int i = tid; i < 4 * DP; i += TH) {
+    for (int i = tid; i < 4 * DP; i += LC_THREADS) {
         const int d = i % DP, run = i / DP;
         const int at_run = d * LC_LD + run * LC_RUN;
         float q[LC_RUN], k[LC_RUN], c[LC_RUN];
@@ -193,17 +137,16 @@ __global__ void __launch_bounds__(HEADS ? 2 * LC_THREADS : LC_THREADS, 2) lc_pre
         lc_write16(qt + at_run, q); lc_write16(kt + at_run, k);
     }
     __syncthreads();
-    // between runs j < i: 16 threads of 4 x 4 weights for each of the six pairs, two or four of them sharing the channels
-    constexpr int SHARE = TH / 128;
-    if (tid < 6 * 16 * SHARE) {
-        const int half = tid % SHARE, u = (tid / SHARE) & 15, pair = tid / (16 * SHARE);
+    // between runs j < i: 16 threads of 4 x 4 weights for each of the six pairs, two of them sharing the channels
+    if (tid < 6 * 16 * 2) {
+        const int half = tid & 1, u = (tid >> 1) & 15, pair = tid >> 5;
         const int i = pair < 3 ? pair + 1 : pair < 5 ? pair - 1 : 3, j = pair < 3 ? pair : pair < 5 ? pair - 3 : 0;      // (1,0) (2,1) (3,2) (2,0) (3,1) (3,0)
         const int s0 = j * LC_RUN + (u >> 2) * 4, t0 = i * LC_RUN + (u & 3) * 4;
         float4 w[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) w[e] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
-        for (int d = half; d < DP; d += SHARE) {
+        for (int d = half; d < DP; d += 2) {
             const float4 q = *reinterpret_cast<const float4*>(qt + d * LC_LD + t0), k = *reinterpret_cast<const float4*>(kt + d * LC_LD + s0);
             float between = 1.f;
             if (i - j > 1) between = whole[(j + 1) * DP + d];
@@ -217,24 +160,10 @@ __global__ void __launch_bounds__(HEADS ? 2 * LC_THREADS : LC_THREADS, 2) lc_pre
         }
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-#pragma unroll
-            for (int o = 1; o < SHARE; o <<= 1) {
-                w[e].x += __shfl_xor_sync(0xffffffffu, w[e].x, o); w[e].y += __shfl_xor_sync(0xffffffffu, w[e].y, o);
-                w[e].z += __shfl_xor_sync(0xffffffffu, w[e].z, o); w[e].w += __shfl_xor_sync(0xffffffffu, w[e].w, o);
-            }
-            if (e * SHARE / 4 == half) *reinterpret_cast<float4*>(out + (s0 + e) * ST_CHUNK + t0) = w[e];
+            w[e].x += __shfl_xor_sync(0xffffffffu, w[e].x, 1); w[e].y += __shfl_xor_sync(0xffffffffu, w[e].y, 1);
+            w[e].z += __shfl_xor_sync(0xffffffffu, w[e].z, 1); w[e].w += __shfl_xor_sync(0xffffffffu, w[e].w, 1);
+            if (e >> 1 == half) *reinterpret_cast<float4*>(out + (s0 + e) * ST_CHUNK + t0) = w[e];
         }
-    }
-    if constexpr (HEADS > 0) {
-        float *lead = whole + 4 * DP, *follow = lead + 4 * DP;
-        for (int d = tid; d < DP; d += TH) {
-            const float w[4] = {whole[d], whole[DP + d], whole[2 * DP + d], whole[3 * DP + d]};
-            lead[d] = 1.f; lead[DP + d] = w[0]; lead[2 * DP + d] = w[0] * w[1]; lead[3 * DP + d] = (w[0] * w[1]) * w[2];
-            follow[3 * DP + d] = 1.f; follow[2 * DP + d] = w[3]; follow[DP + d] = w[3] * w[2]; follow[d] = (w[3] * w[2]) * w[1];
-        }
-        __syncthreads();                                  // (the weights are written, the decays read)
-        lc_parts<HEADS>(a, qt, kt, whole, lead, follow, reinterpret_cast<unsigned char*>(HEADS == 2 ? follow + 4 * DP : at), out, &seen, &from, first, n, h);
-        return;
     }
     // queries times all decays from the chunk's start, keys times all to its end, channels side by side
     float* q_out = queries + ((size_t)blockIdx.x * a.H + h) * ST_CHUNK * D;
@@ -412,8 +341,8 @@ static int lc_prepare_and_contribute(const LAArgs& a, float* scratch, cudaStream
     const int vec_z = (uintptr_t)a.z % (4 * sizeof(TZ)) == 0 && a.z_ld % 4 == 0 && a.D % 4 == 0;
     const int vec_v = (uintptr_t)a.proj % (4 * size) == 0 && a.ld % 4 == 0 && a.v_off % 4 == 0 && a.Dv % 4 == 0;
     const size_t smem = sizeof(float) * ((size_t)3 * DP * LC_LD + 4 * DP);
-    PE_TRY(cudaFuncSetAttribute(lc_prepare_kernel<T, TZ, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    PE_TRY(pe_launch(lc_prepare_kernel<T, TZ, 0>, dim3(a.slab, a.H), LC_THREADS, smem, s, a, weights, queries, keys, vec_q, vec_z));
+    PE_TRY(cudaFuncSetAttribute(lc_prepare_kernel<T, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PE_TRY(pe_launch(lc_prepare_kernel<T, TZ>, dim3(a.slab, a.H), LC_THREADS, smem, s, a, weights, queries, keys, vec_q, vec_z));
     PE_LAUNCH_CHECK();
     const int td = (a.D + 127) / 128, tv = (a.Dv + 63) / 64;
     PE_TRY(pe_launch(lc_contribution_kernel<T>, dim3(a.slab, a.H, td * tv), ST_THREADS, 0, s, a, (const float*)keys, vec_v, td));
@@ -435,19 +364,3 @@ int la_channels_contributions(const LAArgs& a, bool f32, bool z_f32, float* scra
     return z_f32 ? lc_prepare_and_contribute<bf16, float>(a, scratch, s) : lc_prepare_and_contribute<bf16, bf16>(a, scratch, s);
 }
 int la_channels_outputs(const LAArgs& a, bool f32, float* scratch, cudaStream_t s) { return f32 ? lc_outputs<float>(a, scratch, s) : lc_outputs<bf16>(a, scratch, s); }
-
-template <typename TZ, int HEADS>
-static int lc_prepare_parts(const LAArgs& a, cudaStream_t s) {
-    const int vec_q = (uintptr_t)a.qk % 8 == 0 && a.qk_ld % 4 == 0 && a.q_off % 4 == 0 && a.k_off % 4 == 0;
-    const int vec_z = (uintptr_t)a.z % (4 * sizeof(TZ)) == 0 && a.z_ld % 4 == 0;
-    const size_t smem = sizeof(float) * ((size_t)3 * a.D * LC_LD + 12 * a.D) + (HEADS == 2 ? CM_PARTS * CM_PLANE : 0);      // (64 channels' decays leave no room for the planes)
-    PE_TRY(cudaFuncSetAttribute(lc_prepare_kernel<bf16, TZ, HEADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    PE_TRY(pe_launch(lc_prepare_kernel<bf16, TZ, HEADS>, dim3(a.slab, a.H), 2 * LC_THREADS, smem, s, a, (float*)nullptr, (float*)nullptr, (float*)nullptr, vec_q, vec_z));
-    PE_LAUNCH_CHECK();
-    return 0;
-}
-int la_channels_prepare(const LAArgs& a, bool z_f32, bool two, cudaStream_t s) {
-    if (a.H > 65535) return PE_ERR_UNSUPPORTED;
-    if (two) return z_f32 ? lc_prepare_parts<float, 2>(a, s) : lc_prepare_parts<bf16, 2>(a, s);
-    return z_f32 ? lc_prepare_parts<float, 1>(a, s) : lc_prepare_parts<bf16, 1>(a, s);
-}

@@ -13,15 +13,83 @@
 // A state in scratch is [half of the unit's columns][D / 8][64 v][8 d], so that a thread writes and reads runs of 32 bytes and a warp whole lines.
 //
 // Contributions and outputs only copy, multiply and store (outputs cut the state): what bounds them is the parts' way from L2.  Measured on a B200, 2,048
-// tokens, 16 heads of 128 x 128, us: a decay a head and silu on queries, keys and values 122 as multiply-adds, 92 here (operands 35,
-// contributions 15, carry 10, outputs 29); a decay a channel 175 and 128 (79, 12, 10, 23).  14 heads of 64: 57 and 43, 76 and 63; 200 tokens of those 34 and
-// 26, 43 and 36; three prompts of 300, 500 and 33, 16 heads 67 and 48, 92 and 67: these sizes always come here.  Errors against 64 bits, of the
+// tokens, 16 heads of 128 x 128, us: a decay a head and silu on queries, keys and values 122 as multiply-adds, 93 here (operands 36,
+// contributions 15, carry 10, outputs 29); a decay a channel 175 and 103 (54, 12, 10, 23).  14 heads of 64: 57 and 43, 76 and 49; 200 tokens of those 34 and
+// 26, 43 and 29; three prompts of 300, 500 and 33, 16 heads 67 and 48, 92 and 54: these sizes always come here.  Errors against 64 bits, of the
 // outputs' norm: 2.1e-7 as multiply-adds and 6.3e-8 here, with a decay a channel 2.0e-7 and 1.6e-7 (its weights are the same sums); of the states 1.0e-7 and 6.1e-8,
 // 1.44e-7 and 1.28e-7.
-#include "linear_attention_parts.cuh"
+#include "linear_attention.cuh"
+#include "chunk_mma.cuh"
 
 #define LM_THREADS 256
 #define LM_SMEM (12 * CM_PLANE + 1024)                    // parts of Q (or of W) and of S (or the values), both halves
+
+// A unit's parts in scratch: queries and keys, [part][two][64 tokens][64 channels] each (two: the channels' halves, or the heads), and weights
+// [part][heads][64 t][64 s]; and values behind their activation, [part][half][64 s][64 columns].
+template <bool TWO> struct LMUnit {
+    static constexpr int ND = TWO ? 64 : 128;             // rows of a head's state
+    static constexpr int QUERIES = 0, KEYS = 6 * CM_PLANE, WEIGHTS = 12 * CM_PLANE, W_HEADS = TWO ? 2 : 1, VALUES = (12 + 3 * W_HEADS) * CM_PLANE, BYTES = VALUES + 6 * CM_PLANE;
+    // of a head h
+    static __device__ __forceinline__ unsigned char* of(const LAArgs& a, int c, int h) { return a.chunk_planes + ((size_t)c * (TWO ? a.H / 2 : a.H) + (TWO ? h / 2 : h)) * BYTES; }
+};
+
+// Tiles of a chunk's and head's word: 0 queries, 1 keys (with one decay a head), 2 weights, 3 values, 4 keys times their decays.
+// From bit 16 on the first token with an entry that parts do not hold.
+
+// Eight neighbouring numbers of a row, zeros behind the chunk's tokens.
+template <typename TQ>
+__device__ __forceinline__ void lm_eight(float (&v)[8], const TQ* p, bool there, bool vec) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = 0.f;
+    if (!there) return;
+    if (vec) {
+        if constexpr (sizeof(TQ) == 4) {
+            *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(p);
+            *reinterpret_cast<float4*>(v + 4) = *reinterpret_cast<const float4*>(p + 4);
+        } else {
+            const uint4 r = *reinterpret_cast<const uint4*>(p);
+            const unsigned w[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { v[2 * i] = __uint_as_float(w[i] << 16); v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = to_f(p[i]);
+    }
+}
+__device__ __forceinline__ void lm_put(unsigned char* to, int stride, const float (&v)[8], unsigned& most) {
+    cm_put(to, stride, make_float4(v[0], v[1], v[2], v[3]), make_float4(v[4], v[5], v[6], v[7]), most);
+}
+// The same with zeros for what parts do not hold; first: the first row that has such a number.
+__device__ __noinline__ void lm_mend(unsigned char* to, int stride, float4 a, float4 b, int row, unsigned* first) {
+    atomicMin(first, (unsigned)row);
+    const auto fit = [](float v) { unsigned one = 0; cm_watch(one, at_pack(v, 0.f)); return cm_odd(cm_seen(one, 0)) ? 0.f : v; };
+    unsigned most = 0;
+    cm_put(to, stride, make_float4(fit(a.x), fit(a.y), fit(a.z), fit(a.w)), make_float4(fit(b.x), fit(b.y), fit(b.z), fit(b.w)), most);
+}
+__device__ __forceinline__ void lm_put_mended(unsigned char* to, int stride, const float (&v)[8], unsigned& most, int row, unsigned* first) {
+    unsigned mine = 0;
+    lm_put(to, stride, v, mine);
+    cm_watch(most, mine);
+    if (cm_odd(cm_seen(mine, 0))) lm_mend(to, stride, make_float4(v[0], v[1], v[2], v[3]), make_float4(v[4], v[5], v[6], v[7]), row, first);
+}
+__device__ __forceinline__ unsigned lm_value_seen(unsigned most, int act) { return act ? cm_seen(most, 3) : cm_odd(cm_seen(most, 0)) ? 1u << 9 : 2u << 9; }      // (one part holds any finite value)
+// Eight values of a token: parts behind their activation; without one they are only looked at.
+__device__ __forceinline__ void lm_values(const LAArgs& a, unsigned char* to, const bf16* from, bool there, int row, unsigned* first_odd, unsigned& most) {
+    unsigned mine = 0;
+    if (a.act_v) {
+        float v[8];
+        lm_eight(v, from, there, true);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = la_act<true>(v[i], a.act_v);
+        lm_put(to, 2 * CM_PLANE, v, mine);
+    } else if (there) {
+        const uint4 r = *reinterpret_cast<const uint4*>(from);
+        cm_watch(mine, r.x); cm_watch(mine, r.y); cm_watch(mine, r.z); cm_watch(mine, r.w);
+    }
+    if (cm_odd(cm_seen(mine, 0))) atomicMin(first_odd, (unsigned)row);
+    cm_watch(most, mine);
+}
 
 // A chunk's inputs, for what is worked out number by number.
 struct LMInputs {
@@ -68,22 +136,17 @@ __global__ void __launch_bounds__(512, 2) lm_prepare_kernel(LAArgs a, int vec_q)
 #pragma unroll
         for (int i = 0; i < 8; ++i) { q[i] = la_act<true>(q[i], a.act_qk) * a.q_scale; k[i] = la_act<true>(k[i], a.act_qk); }
         if (j) __syncthreads();
-        lm_put(qs + cm_at(row, group), CM_PLANE, q, most[0]);
-        lm_put(ks + cm_at(row, group), CM_PLANE, k, most[1]);
+        lm_put_mended(qs + cm_at(row, group), CM_PLANE, q, most[0], row, &from);
+        lm_put_mended(ks + cm_at(row, group), CM_PLANE, k, most[1], row, &from);
+        const int half = (TWO ? h & 1 : j) * CM_PLANE;
+#pragma unroll
+        for (int p = 0; p < CM_PARTS; ++p)                 // (the thread's own run, a line by eight neighbours)
+            *reinterpret_cast<uint4*>(unit + Unit::QUERIES + p * 2 * CM_PLANE + half + cm_at(row, group)) = *reinterpret_cast<const uint4*>(qs + p * CM_PLANE + cm_at(row, group));
 #pragma unroll
         for (int i = 0; i < 8; ++i) k[i] *= follow;
-        const int half = (TWO ? h & 1 : j) * CM_PLANE;
         lm_put(unit + Unit::KEYS + half + cm_at(row, group), 2 * CM_PLANE, k, most[2]);
         cm_report(&seen, cm_seen(most[0], 0) | cm_seen(most[1], 1) | cm_seen(most[2], 4));
         __syncthreads();
-        if (cm_odd(seen)) {
-            cm_mend(qs, CM_PLANE, CM_PARTS, &from);
-            cm_mend(ks, CM_PLANE, CM_PARTS, &from);
-            __syncthreads();
-        }
-#pragma unroll
-        for (int p = 0; p < CM_PARTS; ++p)
-            *reinterpret_cast<uint4*>(unit + Unit::QUERIES + p * 2 * CM_PLANE + half + tid * 16) = *reinterpret_cast<const uint4*>(qs + p * CM_PLANE + tid * 16);
         if (s0 <= t0) acc.add(at_smem(qs), at_smem(ks), CM_PLANE, t0, s0);
         lm_values(a, unit + Unit::VALUES + half + cm_at(row, group), (const bf16*)a.proj + (size_t)(first + row) * a.ld + a.v_off + h * a.Dv + 64 * j + 8 * group, there, row, &from, most_v);
     }
@@ -114,6 +177,186 @@ __global__ void __launch_bounds__(512, 2) lm_prepare_kernel(LAArgs a, int vec_q)
         *reinterpret_cast<uint4*>(unit + Unit::WEIGHTS + (p * Unit::W_HEADS + (TWO ? h & 1 : 0)) * CM_PLANE + tid * 16) = *reinterpret_cast<const uint4*>(qs + p * CM_PLANE + tid * 16);
     if (tid == 0) a.chunk_seen[(size_t)blockIdx.x * a.H + h] = seen | from << 16;
     if (tid < D) a.chunk_decay[((size_t)blockIdx.x * a.H + h) * D + tid] = pw[n];
+}
+
+// With one decay a channel, a chunk and head: queries times all decays from the chunk's start, keys times all to its end, and weights q_t . A(s, t) k_s.
+// Every product of decays is formed forwards, from factors of at most one (linear_attention_channels.cu): a chunk is four runs of 16; inside a run the
+// decays are walked, between two runs they are what follows s in its run, the whole runs between, and what leads to t in its own.
+// Numbers lie channel by channel, [D][64], rows of 68 with four more every eight channels: a token's run of eight channels and a channel's run of tokens
+// both meet every bank once.  What bounds it: issue slots, half of them the logarithms and exponentials of the decays and what surrounds the walks.  2,048 tokens, 16
+// heads of 128: 54 us; 79 with rows of 68 read a token a lane, walks over whole runs for every key, and parts turned through shared memory.
+#define LMC_RUN 16
+__device__ __forceinline__ int lmc_row(int d) { return d * 68 + (d >> 3) * 4; }
+__host__ __device__ constexpr int lmc_floats(int D) { return D * 68 + D / 8 * 4; }
+// a = sigmoid(z)^(inv_tau), through the logarithm: -softplus(-z) * inv_tau (as the walk has it)
+__device__ __forceinline__ float lmc_decay(float z, float inv_tau) {
+    const float u = -z;
+    return expf(-(fmaxf(u, 0.f) + log1pf(expf(-fabsf(u)))) * inv_tau);
+}
+__device__ __forceinline__ void lmc_read16(float (&v)[LMC_RUN], const float* p) {
+#pragma unroll
+    for (int t = 0; t < LMC_RUN; t += 4) *reinterpret_cast<float4*>(v + t) = *reinterpret_cast<const float4*>(p + t);
+}
+// Sums over 16 neighbouring lanes of N (16 or 8) numbers each: lane l is left with number l % N.
+template <int N>
+__device__ __forceinline__ float lmc_sums(float (&w)[N], int lane) {
+#pragma unroll
+    for (int o = N / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < o; ++i) {
+            const bool upper = lane & o;
+            const float keep = upper ? w[i + o] : w[i], give = upper ? w[i] : w[i + o];
+            w[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    if (N == 8) w[0] += __shfl_xor_sync(0xffffffffu, w[0], 8);
+    return w[0];
+}
+template <typename TZ, bool TWO>
+__global__ void __launch_bounds__(512, 2) lm_channels_kernel(LAArgs a, int vec_q, int vec_z) {
+    pdl_launch_dependents();
+    extern __shared__ __align__(16) float lmc_smem[];
+    __shared__ unsigned seen, from;
+    using Unit = LMUnit<TWO>;
+    constexpr int D = Unit::ND;
+    const int tid = threadIdx.x, lane = tid & 31, row = tid >> 3, group = tid & 7, h = blockIdx.y;
+    float *qt = lmc_smem, *kt = qt + lmc_floats(D), *at = kt + lmc_floats(D);
+    float *whole = at + lmc_floats(D), *lead = whole + 4 * D, *follow = lead + 4 * D;                       // [4][D]: a run's decays; what leads to it; what follows it
+    if (tid == 0) { seen = 0; from = LA_CHUNK; }
+    pdl_wait();
+    int seq, first, n;
+    la_find_chunk(a.row_first, a.row_lens, a.B, a.first_chunk + blockIdx.x, seq, first, n);
+    if (tid == 0 && h == 0) a.chunk_rows[blockIdx.x] = make_int2(first, n);
+    if (n <= 0) return;
+    const bool there = row < n;
+    const size_t token = first + (there ? row : 0);
+    unsigned char* unit = Unit::of(a, blockIdx.x, h);
+    unsigned most_q = 0, most_k = 0, most_w = 0, most_v = 0;
+#pragma unroll 1
+    for (int j = 0; j < D / 64; ++j) {
+        const int d = 64 * j + 8 * group;
+        float q[8], k[8], z[8];
+        lm_eight(q, (const bf16*)a.qk + token * a.qk_ld + a.q_off + h * D + d, there, vec_q);
+        lm_eight(k, (const bf16*)a.qk + token * a.qk_ld + a.k_off + h * D + d, there, vec_q);
+        lm_eight(z, (const TZ*)a.z + token * a.z_ld + h * D + d, there, vec_z);
+        lm_values(a, unit + Unit::VALUES + (TWO ? h & 1 : j) * CM_PLANE + cm_at(row, group), (const bf16*)a.proj + token * a.ld + a.v_off + h * a.Dv + d, there, row, &from, most_v);
+        float* to = qt + lmc_row(d) + row;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            to[i * 68] = la_act<true>(q[i], a.act_qk) * a.q_scale;
+            to[i * 68 + lmc_floats(D)] = la_act<true>(k[i], a.act_qk);
+            to[i * 68 + 2 * lmc_floats(D)] = there ? lmc_decay(z[i], a.inv_tau) : 1.f;
+        }
+    }
+    __syncthreads();
+    float* weights = a.chunk_state + ((size_t)blockIdx.x * a.H + h) * D * a.Dv;      // [64 s][64 t], until the contribution takes the place
+    // inside a run: 16 neighbours share the channels of keys s and s + 8 of a run
+    {
+        const int part = tid & 15, run = tid >> 7, s = (tid >> 4) & 7;
+        float w[16], late[8];                              // weights of s over the run, of s + 8 over its second half
+#pragma unroll
+        for (int t = 0; t < 16; ++t) w[t] = 0.f;
+#pragma unroll
+        for (int t = 0; t < 8; ++t) late[t] = 0.f;
+#pragma unroll 1
+        for (int d = part; d < D; d += 16) {
+            float q[LMC_RUN], c[LMC_RUN];
+            const float* p = qt + lmc_row(d) + run * LMC_RUN;
+            lmc_read16(q, p);
+            lmc_read16(c, p + 2 * lmc_floats(D));
+            const float k = p[lmc_floats(D) + s], k_late = p[lmc_floats(D) + 8 + s];
+            float x = 0.f, y = 0.f;                        // (tokens in front of s: whatever comes of them is not read)
+#pragma unroll
+            for (int t = 0; t < 8; ++t) { x = t == s ? k : x * c[t]; w[t] = fmaf(q[t], x, w[t]); }
+#pragma unroll
+            for (int t = 8; t < 16; ++t) {
+                x *= c[t]; w[t] = fmaf(q[t], x, w[t]);
+                y = t == s + 8 ? k_late : y * c[t]; late[t - 8] = fmaf(q[t], y, late[t - 8]);
+            }
+        }
+        float* to = weights + (run * LMC_RUN + s) * LA_CHUNK + run * LMC_RUN;
+        to[part] = lmc_sums(w, lane);
+        const float v = lmc_sums(late, lane);
+        if (part < 8) to[8 * LA_CHUNK + 8 + part] = v;
+    }
+    __syncthreads();
+    // queries times what leads to them in their run, keys times what follows them there; thread (channel, run)
+    if (tid < 4 * D) {
+        const int d = tid % D, run = tid / D;
+        float q[LMC_RUN], k[LMC_RUN], c[LMC_RUN];
+        float* p = qt + lmc_row(d) + run * LMC_RUN;
+        lmc_read16(q, p); lmc_read16(k, p + lmc_floats(D)); lmc_read16(c, p + 2 * lmc_floats(D));
+        float x = 1.f;
+#pragma unroll
+        for (int t = 0; t < LMC_RUN; ++t) { x *= c[t]; q[t] *= x; }
+        whole[run * D + d] = x;
+        x = 1.f;
+#pragma unroll
+        for (int t = LMC_RUN - 1; t >= 0; --t) { k[t] *= x; x *= c[t]; }
+#pragma unroll
+        for (int t = 0; t < LMC_RUN; t += 4) {
+            *reinterpret_cast<float4*>(p + t) = make_float4(q[t], q[t + 1], q[t + 2], q[t + 3]);
+            *reinterpret_cast<float4*>(p + lmc_floats(D) + t) = make_float4(k[t], k[t + 1], k[t + 2], k[t + 3]);
+        }
+    }
+    __syncthreads();
+    if (tid < D) {
+        const int d = tid;
+        const float w[4] = {whole[d], whole[D + d], whole[2 * D + d], whole[3 * D + d]};
+        lead[d] = 1.f; lead[D + d] = w[0]; lead[2 * D + d] = w[0] * w[1]; lead[3 * D + d] = (w[0] * w[1]) * w[2];
+        follow[3 * D + d] = 1.f; follow[2 * D + d] = w[3]; follow[D + d] = w[3] * w[2]; follow[d] = (w[3] * w[2]) * w[1];
+        a.chunk_decay[((size_t)blockIdx.x * a.H + h) * D + d] = ((w[3] * w[2]) * w[1]) * w[0];
+    }
+    // between runs j < i: 16 threads of 4 x 4 weights for each of the six pairs, four of them sharing the channels
+    if (tid < 6 * 16 * 4) {
+        const int quarter = tid & 3, u = (tid >> 2) & 15, pair = tid >> 6;
+        const int i = pair < 3 ? pair + 1 : pair < 5 ? pair - 1 : 3, j = pair < 3 ? pair : pair < 5 ? pair - 3 : 0;      // (1,0) (2,1) (3,2) (2,0) (3,1) (3,0)
+        const int s0 = j * LMC_RUN + (u >> 2) * 4, t0 = i * LMC_RUN + (u & 3) * 4;
+        float4 w[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) w[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+        for (int d = quarter; d < D; d += 4) {
+            const float4 q = *reinterpret_cast<const float4*>(qt + lmc_row(d) + t0), k = *reinterpret_cast<const float4*>(kt + lmc_row(d) + s0);
+            float between = 1.f;
+            if (i - j > 1) between = whole[(j + 1) * D + d];
+            if (i - j > 2) between *= whole[(j + 2) * D + d];
+            const float ks[4] = {k.x * between, k.y * between, k.z * between, k.w * between};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                w[e].x = fmaf(ks[e], q.x, w[e].x); w[e].y = fmaf(ks[e], q.y, w[e].y);
+                w[e].z = fmaf(ks[e], q.z, w[e].z); w[e].w = fmaf(ks[e], q.w, w[e].w);
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+#pragma unroll
+            for (int o = 1; o < 4; o <<= 1) {
+                w[e].x += __shfl_xor_sync(0xffffffffu, w[e].x, o); w[e].y += __shfl_xor_sync(0xffffffffu, w[e].y, o);
+                w[e].z += __shfl_xor_sync(0xffffffffu, w[e].z, o); w[e].w += __shfl_xor_sync(0xffffffffu, w[e].w, o);
+            }
+            if (e == quarter) *reinterpret_cast<float4*>(weights + (s0 + e) * LA_CHUNK + t0) = w[e];
+        }
+    }
+    __syncthreads();                                       // (the weights are written, what leads and follows too)
+    float weight[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) weight[i] = 8 * group + i <= row ? weights[(8 * group + i) * LA_CHUNK + row] : 0.f;
+#pragma unroll 1
+    for (int j = 0; j < D / 64; ++j) {
+        const int d = 64 * j + 8 * group, place = (TWO ? h & 1 : j) * CM_PLANE + cm_at(row, group), run = row >> 4;
+        const float* p = qt + lmc_row(d) + row;
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = p[i * 68] * lead[run * D + d + i];
+        lm_put_mended(unit + Unit::QUERIES + place, 2 * CM_PLANE, v, most_q, row, &from);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = p[i * 68 + lmc_floats(D)] * follow[run * D + d + i];
+        lm_put(unit + Unit::KEYS + place, 2 * CM_PLANE, v, most_k);
+    }
+    lm_put_mended(unit + Unit::WEIGHTS + (TWO ? h & 1 : 0) * CM_PLANE + cm_at(row, group), Unit::W_HEADS * CM_PLANE, weight, most_w, row, &from);
+    cm_report(&seen, cm_seen(most_q, 0) | cm_seen(most_k, 4) | cm_seen(most_w, 2) | lm_value_seen(most_v, a.act_v));
+    __syncthreads();
+    if (tid == 0) a.chunk_seen[(size_t)blockIdx.x * a.H + h] = seen | from << 16;
 }
 
 // What stands in the words of a unit's heads (bits from 16 on: the first token that parts do not hold).
@@ -379,9 +622,15 @@ static int lm_run(LAArgs a, int types, int z_types, cudaStream_t s) {
     const int units = a.slab * (TWO ? a.H / 2 : a.H), blocks = units < 2 * 148 ? units : 2 * 148;
     PE_TRY(cudaFuncSetAttribute(lm_contribution_kernel<TWO, VP>, cudaFuncAttributeMaxDynamicSharedMemorySize, LM_SMEM));
     PE_TRY(cudaFuncSetAttribute(lm_output_kernel<TWO, VP>, cudaFuncAttributeMaxDynamicSharedMemorySize, LM_SMEM));
-    if (a.z) { if (const int e = la_channels_prepare(a, z_types == 0, TWO, s)) return e; }
-    else {
-        const int size = types == 2 ? 4 : 2;
+    const int size = types == 2 ? 4 : 2;
+    if (a.z) {
+        const int z_size = z_types == 0 ? 4 : 2, smem = 4 * (3 * lmc_floats(a.D) + 12 * a.D);
+        const int vec_q = (uintptr_t)a.qk % 16 == 0 && a.qk_ld % 8 == 0 && a.q_off % 8 == 0 && a.k_off % 8 == 0, vec_z = (uintptr_t)a.z % 16 == 0 && a.z_ld * z_size % 16 == 0;
+        auto kernel = z_types == 0 ? lm_channels_kernel<float, TWO> : lm_channels_kernel<bf16, TWO>;
+        PE_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        PE_TRY(pe_launch(kernel, dim3(a.slab, a.H), 512, smem, s, a, vec_q, vec_z));
+        PE_LAUNCH_CHECK();
+    } else {
         const int vec_q = (uintptr_t)a.qk % 16 == 0 && a.qk_ld * size % 16 == 0 && a.q_off * size % 16 == 0 && a.k_off * size % 16 == 0;
         auto kernel = types == 2 ? lm_prepare_kernel<float, TWO> : lm_prepare_kernel<bf16, TWO>;
         PE_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 6 * CM_PLANE));
