@@ -47,6 +47,7 @@ struct GtArgs {
     int M, N, K;           // M rows of A; N rows of W (SWIGLU: N = 2 I)
     int I, relu;           // SWIGLU: columns of the result; relu != 0: max(gate, 0) in place of silu
     int tiles_m, tiles;    // tiles along the rows of A; all tiles (tile t: m = t % tiles_m, n = t / tiles_m)
+    int whole, parts;      // SWIGLU: the tiles from `whole` on are `parts` pieces of work each (then `tiles` counts pieces)
     // ROPE
     int n_q, n_kv, hd;
     const float* cos_t; const float* sin_t;
@@ -206,16 +207,16 @@ __device__ __forceinline__ void gt_rope_scatter(const GtArgs& p, const unsigned 
 template <bool SWAP, int BN, int EPI>
 __device__ __forceinline__ void gt_epilogue_tile(const GtArgs& p, const CUtensorMap* map_out, unsigned taddr, int m0, int n0,
                                                  int quarter, int turn, int lane, unsigned char* staging, unsigned char* box,
-                                                 int& staged) {
+                                                 int& staged, int width) {
     if (!SWAP) {
         const int row = m0 + quarter * 32 + lane;           // this lane's token
         if (EPI == GT_SWIGLU) {
 #pragma unroll 1
-            for (int c = 32 * turn; c < 128; c += 32 * (GT_EPI_WARPS / 4)) {
+            for (int c = 32 * turn; c < width; c += 32 * (GT_EPI_WARPS / 4)) {
                 if (n0 + c >= p.I) break;
                 float gate[32], up[32];
                 gt_ld32(taddr + c, gate);
-                gt_ld32(taddr + 128 + c, up);
+                gt_ld32(taddr + width + c, up);
                 if (row < p.M) {
                     bf16* o = (bf16*)p.out + (size_t)row * p.I + n0 + c;
 #pragma unroll
@@ -349,7 +350,9 @@ template <bool SWAP, int BN, int EPI>
 __global__ void __launch_bounds__(GT_THREADS) gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_act,
                                                                   const __grid_constant__ CUtensorMap map_w,
                                                                   const __grid_constant__ CUtensorMap map_out,
+                                                                  const __grid_constant__ CUtensorMap map_w_part,
                                                                   const GtArgs p, int* status) {
+    constexpr bool PARTS = !SWAP && EPI == GT_SWIGLU;                      // tiles behind the last whole turn are cut in columns
     constexpr int NA = (SWAP && EPI == GT_SWIGLU) ? 2 : 1;                 // accumulators (tiles of W) of a tile
     constexpr unsigned A_BYTES = NA * 128 * GT_BK * 2, B_BYTES = BN * GT_BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
     constexpr int STAGES = gt_stages(STAGE_BYTES, EPI);
@@ -393,56 +396,81 @@ __global__ void __launch_bounds__(GT_THREADS) gemm_tcgen05_kernel(const __grid_c
     // tile t of this CTA: first row of A and first row of W (SWIGLU: of the gate rows)
     auto tile_m0 = [&](int t) { return (t % p.tiles_m) * (SWAP ? BN : 128); };
     auto tile_n0 = [&](int t) { return (t / p.tiles_m) * (SWAP ? 128 : OUT_COLS); };
+    // the t-th piece of work: its tile, and (PARTS) its gate columns (and as many up columns) and how far in the tile they begin
+    auto piece = [&](int t, int& first) {
+        first = 0;
+        if (!PARTS || t < p.whole) return 128;
+        first = (t - p.whole) % p.parts * (128 / p.parts);
+        return 128 / p.parts;
+    };
+    auto tile_of = [&](int t) { return !PARTS || t < p.whole ? t : p.whole + (t - p.whole) / p.parts; };
 
     if (warp == 0) {
         if (lane == 0) {                                            // ---------------- producer
             const int my_tiles = ((int)blockIdx.x < p.tiles) ? (p.tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
             const long long total = (long long)my_tiles * k_blocks;
-            auto load_w = [&](long long it) {
-                const int t = (int)blockIdx.x + (int)(it / k_blocks) * (int)gridDim.x, kb = (int)(it % k_blocks), s = (int)(it % STAGES);
+            // The next k block of W and of the activations: their piece of work and where it lies, worked out once a piece.  (With the piece, the k block and
+            // the stage divided out of one running number for every load, this thread was what everybody waited for: 2,048 rows of 896 x 9,728
+            // 36.3 us for 31.7, 64 of 18,944 x 3,584 132 for 90, 4,096 of 3,584 x 4,608 on pairs 104 for 88.)
+            int w_t = blockIdx.x, w_k = 0, w_n0 = 0, w_width = 128, a_t = blockIdx.x, a_k = 0, a_m0 = 0;
+            auto w_piece = [&]() { int begins; w_width = piece(w_t, begins); w_n0 = tile_n0(tile_of(w_t)) + begins; };
+            auto a_piece = [&]() { a_m0 = tile_m0(tile_of(a_t)); };
+            auto load_w = [&](int s) {
+                if (w_k == 0) w_piece();
                 const unsigned bar = gt_smem(&full_bar[s]), dst = stage0 + s * STAGE_BYTES;
-                const int n0 = tile_n0(t);
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(STAGE_BYTES) : "memory");
-                if (SWAP) {
-                    gt_tma_2d(dst, &map_w, kb * GT_BK, n0, bar);
-                    if (NA == 2) gt_tma_2d(dst + 128 * GT_BK * 2, &map_w, kb * GT_BK, p.I + n0, bar);
-                } else if (EPI == GT_SWIGLU) {
-                    gt_tma_2d(dst + A_BYTES, &map_w, kb * GT_BK, n0, bar);                         // gate rows
-                    gt_tma_2d(dst + A_BYTES + 128 * GT_BK * 2, &map_w, kb * GT_BK, p.I + n0, bar);   // the matching up rows
+                const int k = w_k * GT_BK, n0 = w_n0;
+                if (PARTS && w_width != 128) {
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(A_BYTES + 2 * w_width * GT_BK * 2) : "memory");
+                    gt_tma_2d(dst + A_BYTES, &map_w_part, k, n0, bar);
+                    gt_tma_2d(dst + A_BYTES + w_width * GT_BK * 2, &map_w_part, k, p.I + n0, bar);
                 } else {
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(STAGE_BYTES) : "memory");
+                    if (SWAP) {
+                        gt_tma_2d(dst, &map_w, k, n0, bar);
+                        if (NA == 2) gt_tma_2d(dst + 128 * GT_BK * 2, &map_w, k, p.I + n0, bar);
+                    } else if (EPI == GT_SWIGLU) {
+                        gt_tma_2d(dst + A_BYTES, &map_w, k, n0, bar);                              // gate rows
+                        gt_tma_2d(dst + A_BYTES + 128 * GT_BK * 2, &map_w, k, p.I + n0, bar);        // the matching up rows
+                    } else {
 #pragma unroll
-                    for (int r = 0; r < BN; r += 128) gt_tma_2d(dst + A_BYTES + r * GT_BK * 2, &map_w, kb * GT_BK, n0 + r, bar);
+                        for (int r = 0; r < BN; r += 128) gt_tma_2d(dst + A_BYTES + r * GT_BK * 2, &map_w, k, n0 + r, bar);
+                    }
                 }
+                if (++w_k == k_blocks) { w_k = 0; w_t += gridDim.x; }
             };
-            auto load_act = [&](long long it) {
-                const int t = (int)blockIdx.x + (int)(it / k_blocks) * (int)gridDim.x, kb = (int)(it % k_blocks), s = (int)(it % STAGES);
-                gt_tma_2d(stage0 + s * STAGE_BYTES + (SWAP ? A_BYTES : 0u), &map_act, kb * GT_BK, tile_m0(t), gt_smem(&full_bar[s]));
+            auto load_act = [&](int s) {
+                if (a_k == 0) a_piece();
+                gt_tma_2d(stage0 + s * STAGE_BYTES + (SWAP ? A_BYTES : 0u), &map_act, a_k * GT_BK, a_m0, gt_smem(&full_bar[s]));
+                if (++a_k == k_blocks) { a_k = 0; a_t += gridDim.x; }
             };
-            const long long ahead = total < STAGES ? total : STAGES;
-            for (long long it = 0; it < ahead; ++it) load_w(it);     // weights: nothing to wait for
+            const int ahead = total < STAGES ? (int)total : STAGES;
+            for (int s = 0; s < ahead; ++s) load_w(s);               // weights: nothing to wait for
             pdl_wait();
-            for (long long it = 0; it < ahead; ++it) load_act(it);
+            for (int s = 0; s < ahead; ++s) load_act(s);
+            int s = ahead % STAGES;
+            unsigned round = 0;                                      // parity of the stage's last use
             for (long long it = ahead; it < total; ++it) {
-                const int s = (int)(it % STAGES);
-                if (!gt_wait(gt_smem(&empty_bar[s]), (unsigned)((it / STAGES) - 1) & 1u, abort_flag)) { atomicExch(status, 2); abort_s = 1; break; }
-                load_w(it);
-                load_act(it);
+                if (!gt_wait(gt_smem(&empty_bar[s]), round, abort_flag)) { atomicExch(status, 2); abort_s = 1; break; }
+                load_w(s);
+                load_act(s);
+                if (++s == STAGES) { s = 0; round ^= 1u; }
             }
         }
     } else if (warp == 1) {
         if (lane == 0) {                                            // ---------------- MMA issuer
-            // instruction descriptor: float32 accumulator, bfloat16 A and B, both K-major, N = BN, M = 128
-            const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) | ((unsigned)(128 >> 4) << 24);
-            long long it = 0;
+            // instruction descriptor: float32 accumulator, bfloat16 A and B, both K-major, N = BN (or a part's columns), M = 128
+            int s = 0;
+            unsigned round = 0;
             bool ok = true;
             for (int t = blockIdx.x, lt = 0; t < p.tiles && ok; t += gridDim.x, ++lt) {
                 const int buf = lt & 1;
+                int begins;
+                const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)((PARTS ? 2 * piece(t, begins) : BN) >> 3) << 17) | ((unsigned)(128 >> 4) << 24);
                 if (!gt_wait(gt_smem(&acc_empty[buf]), (unsigned)((lt >> 1) & 1) ^ 1u, abort_flag)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const unsigned acc = tmem + (unsigned)(buf * ACC_COLS);
-                for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-                    const int s = (int)(it % STAGES);
-                    if (!gt_wait(gt_smem(&full_bar[s]), (unsigned)(it / STAGES) & 1u, abort_flag)) { ok = false; break; }
+                for (int kb = 0; kb < k_blocks; ++kb) {
+                    if (!gt_wait(gt_smem(&full_bar[s]), round, abort_flag)) { ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const unsigned base = stage0 + s * STAGE_BYTES;
                     const unsigned long long db = gt_desc(base + A_BYTES);
@@ -454,6 +482,7 @@ __global__ void __launch_bounds__(GT_THREADS) gemm_tcgen05_kernel(const __grid_c
                             gt_mma(acc + a * BN, da + 2ull * kk, db + 2ull * kk, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
                     }
                     gt_commit(gt_smem(&empty_bar[s]));               // the stage is free once these MMAs have read it
+                    if (++s == STAGES) { s = 0; round ^= 1u; }
                 }
                 if (ok) gt_commit(gt_smem(&acc_full[buf]));          // all MMAs of the tile done: the accumulator is complete
             }
@@ -467,14 +496,15 @@ __global__ void __launch_bounds__(GT_THREADS) gemm_tcgen05_kernel(const __grid_c
         int staged = 0;                                             // ACCUM: boxes this warp has sent
         pdl_wait();
         for (int t = blockIdx.x, lt = 0; t < p.tiles; t += gridDim.x, ++lt) {
-            const int buf = lt & 1, m0 = tile_m0(t), n0 = tile_n0(t);
+            int begins;
+            const int width = piece(t, begins), buf = lt & 1, m0 = tile_m0(tile_of(t)), n0 = tile_n0(tile_of(t)) + begins;
             bool ok = gt_wait(gt_smem(&acc_full[buf]), (unsigned)((lt >> 1) & 1), abort_flag);
             if (EPI == GT_ROPE) ok = gt_epilogue_all(ok);           // (also: the last tile's scatter is over, the staging is free)
             if (!ok) { atomicExch(status, 2); abort_s = 1; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const unsigned taddr = tmem + ((unsigned)(quarter * 32) << 16) + (unsigned)(buf * ACC_COLS);
 
-            gt_epilogue_tile<SWAP, BN, EPI>(p, &map_out, taddr, m0, n0, quarter, turn, lane, staging, box, staged);
+            gt_epilogue_tile<SWAP, BN, EPI>(p, &map_out, taddr, m0, n0, quarter, turn, lane, staging, box, staged, width);
             // the accumulator has been read: the tensor core may fill it again
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
@@ -580,29 +610,34 @@ __global__ void __launch_bounds__(GT_THREADS) gemm_tcgen05_pair_kernel(const __g
     if (warp == 0) {
         if (lane == 0) {                                            // ---------------- producer (both CTAs)
             const long long total = (long long)my_tiles * k_blocks;
-            auto load_w = [&](long long it) {
-                const int t = pair + (int)(it / k_blocks) * pairs, kb = (int)(it % k_blocks), s = (int)(it % STAGES);
+            // the next k block of W and of the activations: their tile's rows (worked out once a tile)
+            int w_t = pair, w_k = 0, w_n0 = 0, a_t = pair, a_k = 0, a_m0 = 0;
+            auto load_w = [&](int s) {
+                if (w_k == 0) w_n0 = tile_n0(w_t);
                 const unsigned bar = gt_map_to_rank(gt_smem(&full_bar[s]), 0u), dst = stage0 + s * STAGE_BYTES + A_BYTES;
-                const int n0 = tile_n0(t);
                 if (rank == 0)                                       // the even CTA's barrier counts the bytes of both
                     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(gt_smem(&full_bar[s])), "r"(2u * STAGE_BYTES) : "memory");
-                if (EPI == GT_SWIGLU) gt_tma_2d_pair(dst, &map_w, kb * GT_BK, rank == 0 ? n0 : p.I + n0, bar);
-                else gt_tma_2d_pair(dst, &map_w, kb * GT_BK, n0 + (int)rank * (BN / 2), bar);
+                if (EPI == GT_SWIGLU) gt_tma_2d_pair(dst, &map_w, w_k * GT_BK, rank == 0 ? w_n0 : p.I + w_n0, bar);
+                else gt_tma_2d_pair(dst, &map_w, w_k * GT_BK, w_n0 + (int)rank * (BN / 2), bar);
+                if (++w_k == k_blocks) { w_k = 0; w_t += pairs; }
             };
-            auto load_act = [&](long long it) {
-                const int t = pair + (int)(it / k_blocks) * pairs, kb = (int)(it % k_blocks), s = (int)(it % STAGES);
-                gt_tma_2d_pair(stage0 + s * STAGE_BYTES, &map_act, kb * GT_BK, tile_m0(t), gt_map_to_rank(gt_smem(&full_bar[s]), 0u));
+            auto load_act = [&](int s) {
+                if (a_k == 0) a_m0 = tile_m0(a_t);
+                gt_tma_2d_pair(stage0 + s * STAGE_BYTES, &map_act, a_k * GT_BK, a_m0, gt_map_to_rank(gt_smem(&full_bar[s]), 0u));
+                if (++a_k == k_blocks) { a_k = 0; a_t += pairs; }
             };
-            const long long ahead = total < STAGES ? total : STAGES;
-            for (long long it = 0; it < ahead; ++it) load_w(it);
+            const int ahead = total < STAGES ? (int)total : STAGES;
+            for (int s = 0; s < ahead; ++s) load_w(s);
             pdl_wait();
-            for (long long it = 0; it < ahead; ++it) load_act(it);
+            for (int s = 0; s < ahead; ++s) load_act(s);
             bool ok = true;
+            int s = ahead % STAGES;
+            unsigned round = 0;                                      // parity of the stage's last use
             for (long long it = ahead; it < total; ++it) {
-                const int s = (int)(it % STAGES);
-                if (!gt_wait(gt_smem(&empty_bar[s]), (unsigned)((it / STAGES) - 1) & 1u, abort_flag)) { ok = false; break; }
-                load_w(it);
-                load_act(it);
+                if (!gt_wait(gt_smem(&empty_bar[s]), round, abort_flag)) { ok = false; break; }
+                load_w(s);
+                load_act(s);
+                if (++s == STAGES) { s = 0; round ^= 1u; }
             }
             // before this CTA may end, the commits that the even CTA sends to its "empty" barriers must have arrived
             for (long long it = total > STAGES ? total - STAGES : 0; ok && it < total; ++it)
@@ -613,16 +648,16 @@ __global__ void __launch_bounds__(GT_THREADS) gemm_tcgen05_pair_kernel(const __g
         if (lane == 0 && rank == 0) {                               // ---------------- MMA issuer (even CTA)
             // instruction descriptor: float32 accumulator, bfloat16 A and B, both K-major, N = BN, M = 256 over the pair
             const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) | ((unsigned)(256 >> 4) << 24);
-            long long it = 0;
+            int s = 0;
+            unsigned round = 0;
             bool ok = true;
             for (int lt = 0; lt < my_tiles && ok; ++lt) {
                 const int buf = lt & 1;
                 if (!gt_wait(gt_smem(&acc_empty[buf]), (unsigned)((lt >> 1) & 1) ^ 1u, abort_flag)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const unsigned acc = tmem + (unsigned)(buf * BN);
-                for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-                    const int s = (int)(it % STAGES);
-                    if (!gt_wait(gt_smem(&full_bar[s]), (unsigned)(it / STAGES) & 1u, abort_flag)) { ok = false; break; }
+                for (int kb = 0; kb < k_blocks; ++kb) {
+                    if (!gt_wait(gt_smem(&full_bar[s]), round, abort_flag)) { ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const unsigned base = stage0 + s * STAGE_BYTES;
                     const unsigned long long da = gt_desc(base), db = gt_desc(base + A_BYTES);
@@ -630,6 +665,7 @@ __global__ void __launch_bounds__(GT_THREADS) gemm_tcgen05_pair_kernel(const __g
                     for (int kk = 0; kk < GT_BK / 16; ++kk)
                         gt_mma_pair(acc, da + 2ull * kk, db + 2ull * kk, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
                     gt_commit_pair(gt_smem(&empty_bar[s]));
+                    if (++s == STAGES) { s = 0; round ^= 1u; }
                 }
                 if (ok) gt_commit_pair(gt_smem(&acc_full[buf]));
             }
@@ -647,7 +683,7 @@ __global__ void __launch_bounds__(GT_THREADS) gemm_tcgen05_pair_kernel(const __g
             if (!ok) { atomicExch(status, 2); abort_s = 1; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const unsigned taddr = tmem + ((unsigned)(quarter * 32) << 16) + (unsigned)(buf * BN);
-            gt_epilogue_tile<false, BN, EPI>(p, &map_out, taddr, m0, n0, quarter, turn, lane, staging, box, staged);
+            gt_epilogue_tile<false, BN, EPI>(p, &map_out, taddr, m0, n0, quarter, turn, lane, staging, box, staged, 128);
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0)                                          // both CTAs' warps count on the even CTA's barrier
@@ -707,8 +743,22 @@ static int gt_launch(const void* A, const void* W, GtArgs& p, int* status, cudaS
         PE_TRY(cudaFuncSetAttribute(gemm_tcgen05_kernel<SWAP, BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         attr_set = true;
     }
+    // What is left behind the last turn that keeps every SM busy would take a turn of its own with most of them idle: where there is room those tiles are
+    // cut into two or four pieces of 64 or 32 gate columns and as many up columns, a CTA each, half to two thirds of a tile's time.  2,048 rows of
+    // 896 x 9,728 are 608 tiles, 16 more than four turns: 31.7 us, 30.2 with them in quarters; 512 rows, 152 tiles, 14.4 and 12.5.  (Every sum stays the same.)
+    p.whole = p.tiles; p.parts = 1;
+    CUtensorMap mp = mw;
+    if (EPI == GT_SWIGLU && !SWAP) {
+        const int sms = gt_sm_count(), rest = p.tiles % sms;
+        p.parts = rest == 0 ? 1 : 4 * rest <= sms ? 4 : 2 * rest <= sms ? 2 : 1;
+        if (p.parts > 1) {
+            p.whole = p.tiles - rest; p.tiles = p.whole + rest * p.parts;
+            rc = gt_make_map(&mp, W, p.N, p.K, 128 / p.parts, GT_BK, false);
+            if (rc) return rc;
+        }
+    }
     const int ctas = p.tiles < gt_sm_count() ? p.tiles : gt_sm_count();
-    PE_TRY(pe_launch(gemm_tcgen05_kernel<SWAP, BN, EPI>, dim3(ctas), GT_THREADS, smem, s, ma, mw, mo, p, status));
+    PE_TRY(pe_launch(gemm_tcgen05_kernel<SWAP, BN, EPI>, dim3(ctas), GT_THREADS, smem, s, ma, mw, mo, mp, p, status));
     return 0;
 }
 

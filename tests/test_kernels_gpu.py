@@ -1338,3 +1338,19 @@ def test_linear_simt_with_a_short_k(K, N, K_, ta, tw):
         assert float((x.cpu().double() - want - 1).abs().max()) <= 8 * (K_ + 1) * 2.0 ** -24
         assert torch.equal(got, K.linear_simt(dev(a), dev(w), dev(bias), out_dtype=torch.float32)[:M])
 
+
+@pytest.mark.parametrize("M,I,K", [(130, 8, 64), (200, 328, 200), (300, 2104, 136), (1300, 2000, 64), (1300, 4000, 72), (128, 18944, 64)])
+def test_gate_up_tiles_behind_the_last_whole_turn(M, I, K):
+    """Tiles that are left behind the turns that keep every SM busy are cut into two or four pieces of their columns: the same bits as CTA
+    pairs give, which have no pieces, and the product within bfloat16's rounding."""
+    from pico_engine.ops import kernels
+    g = torch.Generator("cuda").manual_seed(M + I)
+    a = torch.randn(M, K, generator=g, device="cuda").bfloat16()
+    w = (torch.randn(2 * I, K, generator=g, device="cuda") * K ** -0.5).bfloat16()
+    got, pairs = (kernels.gemm_tcgen05(a, w, swiglu=True, orientation=o) for o in ("rows", "pairs"))
+    kernels.check_status(torch.device("cuda", torch.cuda.current_device()))
+    assert torch.equal(got, pairs)
+    gate, up = (a.float() @ w.float().t()).bfloat16().float().split(I, dim=1)
+    want = torch.nn.functional.silu(gate) * up
+    # gate and up may round to the neighbouring bfloat16 number (2^-8 of each), the result rounds once more
+    assert ((got.float() - want).abs() <= 2 ** -6 * (want.abs() + gate.abs() * 2 ** -7 + up.abs() * 2 ** -7) + 1e-6).all()
