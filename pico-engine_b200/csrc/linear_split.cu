@@ -326,8 +326,9 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
             }
         };
         if (!MANY && (warp >> 2) < chunks) fetch_a(warp >> 2);
+        int s = warp >> 2, turn = 0;                       // the chunk's slot, and how often it was taken before (parity): stepped, not divided out of c
         for (int c = warp >> 2; c < chunks; c += GROUPS) {
-            const int r = c % RING, s = c % slots;
+            const int r = c % RING;
             if (!sp_wait_warp(w_full + 8 * r, (c / RING) & 1, &abort_s, status)) break;
             bool ok = true;
             float least = INFINITY;                        // the smallest of the entries cut here
@@ -344,7 +345,7 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
                     sp_cut(v.z, v.w, hi[2 * j + 1], mid[2 * j + 1], lo[2 * j + 1]);
                 }
                 if (half == 0) {                           // (the first half is cut while the slot's last products end)
-                    if (c >= slots && !(ok = sp_wait_warp(empty + 8 * s, (c / slots - 1) & 1, &abort_s, status))) break;
+                    if (c >= slots && !(ok = sp_wait_warp(empty + 8 * s, turn ^ 1, &abort_s, status))) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 }
                 sp_st8(to + 8 * half, hi); sp_st8(to + 8 * half + SP_KC / 2, mid); sp_st8(to + 8 * half + SP_KC, lo);
@@ -393,20 +394,22 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
             if (!MANY) {
                 if (c + GROUPS < chunks) fetch_a(c + GROUPS);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            } else if ((warp & 3) == 0 && !sp_wait_warp(a_full + 8 * s, (c / slots) & 1, &abort_s, status)) break;
+            } else if ((warp & 3) == 0 && !sp_wait_warp(a_full + 8 * s, turn, &abort_s, status)) break;
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) at_arrive(full + 8 * s);
+            s += GROUPS;                                   // (no more groups than slots)
+            if (s >= slots) { s -= slots; turn ^= 1; }
         }
     } else if (warp == CUTTERS) {
         const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(nt / 8) << 17) | ((unsigned)(SP_ROWS / 16) << 24);
         const unsigned elected = sp_elect();
-        int issued = 0;
+        int issued = 0, s = 0, turn = 0;
         for (int c = 0; c < chunks; ++c) {
-            const int s = c % slots, b = c % SUMS;
+            const int b = c % SUMS;
             if (c >= SUMS && !sp_wait_warp(sum_empty + 8 * b, (c / SUMS - 1) & 1, &abort_s, status)) break;
-            if (!sp_wait_warp(full + 8 * s, (c / slots) & 1, &abort_s, status)) break;
+            if (!sp_wait_warp(full + 8 * s, turn, &abort_s, status)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const unsigned long long a = sp_desc(a_parts + s * SP_PARTS * part_bytes), part = part_bytes >> 4;
             sp_products(elected, sums + b * nt, small, tmem + s * SP_W_COLS, a, a + part, a + 2 * part, idesc, c > 0);
@@ -416,19 +419,21 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
             }
             __syncwarp();
             issued = c + 1;
+            if (++s == slots) { s = 0; turn ^= 1; }
         }
         if (issued > 0) at_wait_warp(sum_full + 8 * ((issued - 1) % SUMS), ((issued - 1) / SUMS) & 1);      // nothing stays under way
     } else if (warp == CUTTERS + 1) {
         if (lane == 0) {
-            int brought = min(RING, chunks), brought_a = 0;
+            int brought = min(RING, chunks), brought_a = 0, s = 0, turn = 0;
             for (int c = 0; c < chunks; ++c) {
-                const int s = c % slots, r = c % RING;
+                const int r = c % RING;
                 if (MANY) {
-                    if (c >= slots && !sp_wait(empty + 8 * s, (c / slots - 1) & 1, &abort_s, status)) break;
+                    if (c >= slots && !sp_wait(empty + 8 * s, turn ^ 1, &abort_s, status)) break;
                     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(a_full + 8 * s), "r"((unsigned)(SP_PARTS * part_bytes)) : "memory");
                     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
                                  ::"r"(a_parts + s * SP_PARTS * part_bytes), "l"(&map_a), "r"(a_full + 8 * s), "r"(k_begin + c * SP_KC), "r"(m0), "r"(0) : "memory");
                     brought_a = c + 1;
+                    if (++s == slots) { s = 0; turn ^= 1; }
                 }
                 if (c + RING < chunks) {
                     if (!sp_wait(w_empty + 8 * r, (c / RING) & 1, &abort_s, status)) break;
