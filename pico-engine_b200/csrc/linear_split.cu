@@ -26,14 +26,14 @@
 //   loads      a warp brings W (float32) by TMA, into L2 as far as the ring goes before the kernel waits for its predecessor; more than 64 rows of
 //              A have been cut by a kernel before this one and come by TMA as well
 //   sums       4 or 16 warps take the sums of hi hi out of tensor memory
-// Bound by the hand-overs between them: 508 rows, 9,728 x 896, a chunk of 112 rows of A takes 1,700 cycles, the tensor pipe is busy for a third
+// Bound by the hand-overs between them: 508 rows, 9,728 x 896, a chunk of 112 rows of A takes 1,600 cycles, the tensor pipe is busy for a third
 // of it, the issue slots for half.  Leaving out two thirds of the products, the cutting or the reading of sums saves 3 to 7 % each.
 //
 // One B200, W read from memory, us, here / in linear_simt.cu (the only way before): rows of A 1 12 60 130 508
-//   1,152 x 896   5.4 / 5.5     5.6 / 7.7    7.9 / 12.2   11.1 / 21.7   24.5 / 34.8
-//     896 x 896   5.4 / 5.8     5.6 / 7.6    7.9 / 13.1   10.8 / 25.5   15.1 / 28.0
-//   9,728 x 896  13.8 / 12.8   14.1 / 27.2  19.0 / 51.0   46.9 / 84.3   76.8 / 208
-//     896 x 4864 10.0 / 11.4   10.2 / 20.4  13.5 / 29.9   21.4 / 64.5   50.2 / 111
+//   1,152 x 896   5.4 / 5.5     5.6 / 7.7    7.9 / 12.2   11.1 / 21.7   24.0 / 34.8
+//     896 x 896   5.4 / 5.8     5.6 / 7.6    7.9 / 13.1   10.8 / 25.5   15.4 / 28.0
+//   9,728 x 896  13.8 / 12.8   14.1 / 27.2  19.0 / 51.0   44.5 / 84.3   70.5 / 208
+//     896 x 4864 10.0 / 11.4   10.2 / 20.4  13.5 / 29.9   20.4 / 64.5   49.6 / 111
 //   3,584 x 3584 24.6 / 28.7   25.0 / 50.3  32.3 / 77.3   65.1 / 176.8  133 / 316
 //
 // Infinities, values that are no number, marked entries and sums beyond float32 leave results that are not finite; those are worked out again with

@@ -763,3 +763,30 @@ def test_state_space_products_at_the_ends_of_the_range(scale):
     walk, chunks = run(xbc, False)[0], run(xbc, True)[0]
     # the state begins at 0.5: at 1e-36 nothing of x is left beside it
     assert (walk - chunks).abs().max() < 3e-5 * float(walk.abs().max())
+
+
+@pytest.mark.parametrize("T", [1, 3, 130])
+@pytest.mark.parametrize("H,D,R,rank,rot,rows,absorbed", [(1, 8, 8, 8, 8, False, True), (16, 128, 64, 192, 64, False, False), (5, 16, 24, 256, 16, True, True), (3, 8, 16, 40, 0, False, True),
+                                                          (60, 8, 64, 64, 64, True, False)])
+def test_low_rank_rows_in_runs_of_eight(T, H, D, R, rank, rot, rows, absorbed):
+    """The kernel that takes eight entries a thread against the general one, which takes the same numbers from a place one entry further on."""
+    from pico_engine.ops import kernels
+    g = torch.Generator("cuda").manual_seed(rank + T)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    width, W = H * (D + R), rank + R
+    proj, q_rows, qa, weight = r(T, width + W), r(T, width) if rows else None, r(H, T, rank) if absorbed else None, 1 + 0.1 * r(rank)
+    freq = 10000.0 ** (-torch.arange(max(rot // 2, 1), device="cuda") / max(rot // 2, 1))
+    pos = torch.randperm(5000, generator=g, device="cuda")[:T].int().sort().values       # (no place of the cache twice)
+    pages = int(pos.max()) // 64 + 1
+    table = torch.randperm(pages, generator=g, device="cuda").int().view(1, pages)
+    got = []
+    for shift in (0, 1):
+        put = lambda t: None if t is None else torch.empty(t.numel() + shift, dtype=t.dtype, device="cuda")[shift:].view(t.shape).copy_(t)
+        pool, out = torch.zeros(pages, 1, 64, W, dtype=torch.bfloat16, device="cuda"), torch.zeros(T, H * W, dtype=torch.bfloat16, device="cuda")
+        q = kernels.latent_prepare(put(proj), H, D, R, rank, width, weight, 1e-5, freq, rot, put(qa), pos, torch.zeros(T, dtype=torch.int32, device="cuda"), pool, table, pages,
+                                   q_rows=put(q_rows), q_out=None if absorbed else out)
+        got.append((q.float(), pool.float()))
+    # the same arithmetic up to float32 rounding (squares in another order; which of a rotation's two products the multiply-add keeps unrounded), then
+    # one rounding to bfloat16: a neighbouring number at most, and 2^-22 of entries of up to 6 where a rotation cancels
+    for a, b in zip(*got):
+        assert ((a - b).abs() <= 2 ** -7 * b.abs() + 6 * 2 ** -22).all()
