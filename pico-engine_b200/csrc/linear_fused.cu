@@ -207,13 +207,13 @@ __global__ void __launch_bounds__(32 * LF_WARPS, LF_MIN_CTAS(NT, RT, EPI)) linea
     const int cp_row = cp_r < 0 ? -1 : cp_l < 8 ? lo_base + cp_rt * rt_step + cp_l : (hi_base < 0 ? -1 : hi_base + cp_rt * rt_step + cp_l - 8);
     const bool cp_ok = cp_r >= 0 && cp_r < tile_rows && cp_row >= 0 && cp_row < p.N && (EPI != LF_SWIGLU || cp_l >= 8 || cp_row < p.I);
     const unsigned n_ok = __popc(__ballot_sync(0xffffffffu, my_row_ok));
-    auto issue = [&](int c) {
+    auto issue = [&](int c, int slot) {                      // slot = c % stages, stepped by the caller: a division is some forty cycles
         const int k0 = c * chunk, cols = min(chunk, K - k0);
-        const unsigned bar = bar0 + 8u * (c % stages);
+        const unsigned bar = bar0 + 8u * slot;
         if (threadIdx.x == 0) lf_bar_expect(bar, n_ok * (unsigned)cols * 2u);
         if (cp_ok) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // earlier reads of the stage precede its refill
-            lf_bulk_copy(smem0 + (c % stages) * stage_bytes + cp_r * row_bytes, p.W + (size_t)cp_row * p.K + k_begin + k0,
+            lf_bulk_copy(smem0 + slot * stage_bytes + cp_r * row_bytes, p.W + (size_t)cp_row * p.K + k_begin + k0,
                          (unsigned)cols * 2u, bar);
         }
     };
@@ -222,19 +222,19 @@ __global__ void __launch_bounds__(32 * LF_WARPS, LF_MIN_CTAS(NT, RT, EPI)) linea
     const int cp_a = (lane == 4 || lane == 5) ? warp * 2 + lane - 4 : -1;
     const bool cp_a_ok = cp_a >= 0 && cp_a < a_rows && cp_a < M;
     const unsigned n_a_ok = __popc(__ballot_sync(0xffffffffu, my_a_ok));
-    auto issue_a = [&](int c) {
+    auto issue_a = [&](int c, int slot) {
         const int k0 = c * chunk, cols = min(chunk, K - k0);
-        const unsigned bar = bar_a0 + 8u * (c % stages);
+        const unsigned bar = bar_a0 + 8u * slot;
         if (threadIdx.x == 0) lf_bar_expect(bar, n_a_ok * (unsigned)cols * 2u);
         if (cp_a_ok) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            lf_bulk_copy(smem0 + (c % stages) * stage_bytes + (tile_rows + cp_a) * row_bytes, p.A + (size_t)cp_a * p.K + k_begin + k0,
+            lf_bulk_copy(smem0 + slot * stage_bytes + (tile_rows + cp_a) * row_bytes, p.A + (size_t)cp_a * p.K + k_begin + k0,
                          (unsigned)cols * 2u, bar);
         }
     };
 
     pdl_launch_dependents();
-    for (int c = 0; c < n_chunks && c < stages; ++c) issue(c);      // W first: no kernel writes it, so it need not wait
+    for (int c = 0; c < n_chunks && c < stages; ++c) issue(c, c);      // W first: no kernel writes it, so it need not wait
     // The norm's weights too, into L1: a step streams more weights than L2 holds, so that they come from DRAM, and behind the wait
     // they would be as long on their way as everything else the kernel does there (clock stamps: 1.9 us from the wait to the first product;
     // with this and waits that are not slept over, a step of 24 layers of the Qwen2.5-0.5B widths 724 -> 706 us at 8 rows).
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(32 * LF_WARPS, LF_MIN_CTAS(NT, RT, EPI)) linea
     }
     pdl_wait();                                              // from here on the preceding kernel's results may be read
     if (PRO == LF_PLAIN)
-        for (int c = 0; c < n_chunks && c < stages; ++c) issue_a(c);
+        for (int c = 0; c < n_chunks && c < stages; ++c) issue_a(c, c);
 
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
     // RMSNORM: the operand is bfloat16(x * w); the row's 1/rms is applied to the sums at the end (the
@@ -316,14 +316,15 @@ __global__ void __launch_bounds__(32 * LF_WARPS, LF_MIN_CTAS(NT, RT, EPI)) linea
 
     uint4 a_cur[LF_UNROLL(NT)][NT], a_next[LF_UNROLL(NT)][NT];
     if (PRO == LF_RMSNORM) load_a(0, a_cur);
+    int slot = 0;                                            // c % stages and the parity of c / stages
+    unsigned parity = 0u;
     for (int c = 0; c < n_chunks; ++c) {
         const int k0 = c * chunk, cols = min(chunk, K - k0), steps = (cols + 31) / 32;
-        const unsigned stage = smem0 + (c % stages) * stage_bytes;
+        const unsigned stage = smem0 + slot * stage_bytes;
         if (PRO == LF_RMSNORM) load_a(c + 1, a_next);        // in flight while this chunk's W is awaited and used
-        const unsigned parity = (unsigned)(c / stages) & 1u;
         const int first = (warp - k0 / 32) & (LF_WARPS - 1);     // this warp's k steps: those of the range that are = warp mod 8,
-        if (first < steps && !(lf_bar_wait(bar0 + 8u * (c % stages), parity) &&
-                              (PRO != LF_PLAIN || lf_bar_wait(bar_a0 + 8u * (c % stages), parity)))) {
+        if (first < steps && !(lf_bar_wait(bar0 + 8u * slot, parity) &&
+                              (PRO != LF_PLAIN || lf_bar_wait(bar_a0 + 8u * slot, parity)))) {
             atomicExch(status, 1);                           // the copies did not arrive: give up, loudly
             return;
         }
@@ -358,9 +359,10 @@ __global__ void __launch_bounds__(32 * LF_WARPS, LF_MIN_CTAS(NT, RT, EPI)) linea
         }
         if (c + stages < n_chunks) {                         // the stage is free again: refill it
             __syncthreads();
-            issue(c + stages);
-            if (PRO == LF_PLAIN) issue_a(c + stages);
+            issue(c + stages, slot);
+            if (PRO == LF_PLAIN) issue_a(c + stages, slot);
         }
+        if (++slot == stages) { slot = 0; parity ^= 1u; }
     }
 
     // acc[rt][j][e] of lane (g, t): MMA row g (+8 if e & 2) of tile rt, sequence j*8 + 2t + (e & 1)
