@@ -362,6 +362,28 @@ __global__ void swiglu_bf16x8_kernel(const bf16* gu, bf16* out, int I, size_t gr
     }
 }
 
+// float32, I a multiple of 4: two runs of four a thread, 16-byte accesses; each entry by the same arithmetic as above.  Runs are counted in
+// `Index`, 32 bits where they fit: an entry a thread at a time spent itself on a division and a remainder of 64 bits by a number known only now.
+// 508 tokens of 4,864 (30 MB, two thirds of them left in L2 by the product in front): 9.3 us with an entry at a time, 5.2 so.
+template <typename Index>
+__global__ void __launch_bounds__(256) swiglu_f32x4_kernel(const float* gu, float* out, int I, Index groups) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const Index per_row = I / 4;
+    const Index stride = (Index)gridDim.x * blockDim.x;
+    for (Index idx = (Index)blockIdx.x * blockDim.x + threadIdx.x; idx < groups; idx += 2 * stride) {
+        const Index idx1 = idx + stride;
+        const bool two = idx1 < groups;
+        const Index r0 = idx / per_row, r1 = two ? idx1 / per_row : r0;
+        const size_t t0 = r0, i0 = (size_t)(idx - r0 * per_row) * 4, t1 = r1, i1 = two ? (size_t)(idx1 - r1 * per_row) * 4 : i0;
+        const float4 g0 = *reinterpret_cast<const float4*>(gu + t0 * 2 * I + i0), u0 = *reinterpret_cast<const float4*>(gu + t0 * 2 * I + I + i0);
+        const float4 g1 = *reinterpret_cast<const float4*>(gu + t1 * 2 * I + i1), u1 = *reinterpret_cast<const float4*>(gu + t1 * 2 * I + I + i1);
+        *reinterpret_cast<float4*>(out + t0 * I + i0) = make_float4(silu_mul(g0.x, u0.x), silu_mul(g0.y, u0.y), silu_mul(g0.z, u0.z), silu_mul(g0.w, u0.w));
+        if (two)
+            *reinterpret_cast<float4*>(out + t1 * I + i1) = make_float4(silu_mul(g1.x, u1.x), silu_mul(g1.y, u1.y), silu_mul(g1.z, u1.z), silu_mul(g1.w, u1.w));
+    }
+}
+
 extern "C" int pe_swiglu(const void* gu, void* out, int dtype, int T, int I, void* stream) {
     if (T <= 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
@@ -370,6 +392,14 @@ extern "C" int pe_swiglu(const void* gu, void* out, int dtype, int T, int I, voi
         const size_t groups = total / 8, want = (groups + 511) / 512;      // two groups a thread
         const int blocks = (int)(want < 148 * 16 ? want : 148 * 16);
         PE_TRY(pe_launch(swiglu_bf16x8_kernel, blocks, 256, 0, s, (const bf16*)gu, (bf16*)out, I, groups));
+        PE_LAUNCH_CHECK();
+        return 0;
+    }
+    if (dtype == PE_F32 && I % 4 == 0 && !(((uintptr_t)gu | (uintptr_t)out) & 15)) {
+        const size_t groups = total / 4, want = (groups + 511) / 512;
+        const int blocks = (int)(want < 148 * 16 ? want : 148 * 16);
+        if (groups < (1u << 31)) PE_TRY(pe_launch(swiglu_f32x4_kernel<unsigned>, blocks, 256, 0, s, (const float*)gu, (float*)out, I, (unsigned)groups));
+        else PE_TRY(pe_launch(swiglu_f32x4_kernel<size_t>, blocks, 256, 0, s, (const float*)gu, (float*)out, I, groups));
         PE_LAUNCH_CHECK();
         return 0;
     }
@@ -550,13 +580,61 @@ __global__ void rope_store_bf16x8_kernel(bf16* qkv, int n_q, int n_kv, int hd, c
     }
 }
 
+// The same for float32 with head sizes that are multiples of 8: four pairs a thread, 16-byte accesses.
+// 508 tokens of 14 + 2 heads of 64: 4.1 us with a pair a thread, 3.6 so.
+__global__ void __launch_bounds__(128) rope_store_f32x4_kernel(float* qkv, int n_q, int n_kv, int hd, const float* cos_t, const float* sin_t,
+                                                               const int* tok_pos, const int* tok_row, float* k_pool, float* v_pool,
+                                                               const int* block_table, int table_stride, int store) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int t = blockIdx.x;
+    const int pos = tok_pos[t];
+    const int half = hd >> 1, groups = half >> 2;               // groups of 4 pairs per head
+    float* row = qkv + (size_t)t * (n_q + 2 * n_kv) * hd;
+    size_t cache_base = 0;
+    bool do_store = false;
+    if (store) {
+        const int page = block_table[(size_t)tok_row[t] * table_stride + pos / PE_PAGE];
+        do_store = page >= 0;
+        cache_base = (size_t)page * n_kv * PE_PAGE * hd + (size_t)(pos % PE_PAGE) * hd;
+    }
+    for (int idx = threadIdx.x; idx < (n_q + n_kv) * groups; idx += blockDim.x) {
+        const int head = idx / groups, j = (idx - head * groups) * 4;
+        float* p = row + (size_t)head * hd;
+        float4 a = *reinterpret_cast<const float4*>(p + j), b = *reinterpret_cast<const float4*>(p + j + half);
+        if (cos_t) {
+            const float4 c = *reinterpret_cast<const float4*>(cos_t + (size_t)pos * half + j), s = *reinterpret_cast<const float4*>(sin_t + (size_t)pos * half + j);
+            const float4 ra = make_float4(a.x * c.x - b.x * s.x, a.y * c.y - b.y * s.y, a.z * c.z - b.z * s.z, a.w * c.w - b.w * s.w);
+            b = make_float4(a.x * s.x + b.x * c.x, a.y * s.y + b.y * c.y, a.z * s.z + b.z * c.z, a.w * s.w + b.w * c.w);
+            a = ra;
+            *reinterpret_cast<float4*>(p + j) = a;
+            *reinterpret_cast<float4*>(p + j + half) = b;
+        }
+        if (do_store && head >= n_q) {
+            float* dst = k_pool + cache_base + (size_t)(head - n_q) * PE_PAGE * hd;
+            *reinterpret_cast<float4*>(dst + j) = a;
+            *reinterpret_cast<float4*>(dst + j + half) = b;
+        }
+    }
+    if (do_store) {
+        const float* v = row + (size_t)(n_q + n_kv) * hd;
+        for (int idx = threadIdx.x * 4; idx < n_kv * hd; idx += blockDim.x * 4) {
+            const int head = idx / hd, d = idx - head * hd;
+            *reinterpret_cast<float4*>(v_pool + cache_base + (size_t)head * PE_PAGE * hd + d) = *reinterpret_cast<const float4*>(v + idx);
+        }
+    }
+}
+
 extern "C" int pe_rope_store(void* qkv, int dtype, int T, int n_q, int n_kv, int hd, const float* cos_t,
                              const float* sin_t, const int* tok_pos, const int* tok_row, void* k_pool, void* v_pool,
                              const int* block_table, int table_stride, int store, void* stream) {
     if (T <= 0) return 0;
     if (hd % 2) return PE_ERR_UNSUPPORTED;
     cudaStream_t s = (cudaStream_t)stream;
-    if (dtype == PE_F32)
+    if (dtype == PE_F32 && hd % 8 == 0 && !(((uintptr_t)qkv | (uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)cos_t | (uintptr_t)sin_t) & 15))
+        PE_TRY(pe_launch(rope_store_f32x4_kernel, T, 128, 0, s, (float*)qkv, n_q, n_kv, hd, cos_t, sin_t, tok_pos, tok_row,
+                         (float*)k_pool, (float*)v_pool, block_table, table_stride, store));
+    else if (dtype == PE_F32)
         PE_TRY(pe_launch(rope_store_kernel<float>, T, 256, 0, s, (float*)qkv, n_q, n_kv, hd, cos_t, sin_t, tok_pos, tok_row,
                                                     (float*)k_pool, (float*)v_pool, block_table, table_stride, store));
     else if (dtype == PE_BF16 && hd % 16 == 0 && !(((uintptr_t)qkv | (uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)cos_t | (uintptr_t)sin_t) & 15))

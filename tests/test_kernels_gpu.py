@@ -139,6 +139,32 @@ def test_swiglu(K, dtype, T, I):
     assert torch.allclose(got.float().cpu(), want, atol=1e-5 if dtype == "f32" else 3e-2, rtol=1e-5 if dtype == "f32" else 1e-2)
 
 
+@pytest.mark.parametrize("T,I", [(1, 4), (1, 2044), (3, 340), (257, 2052), (2400, 4096)])      # one run; a run short of, and past, a block; several turns
+def test_swiglu_float32_in_runs_of_four(K, T, I):
+    gu = rnd(T, 2 * I, seed=5, scale=3.0)
+    got = K.swiglu(dev(gu))
+    # the same arithmetic an entry at a time, where the rows do not begin on 16 bytes: the same bits
+    shifted = torch.empty(T * 2 * I + 1, device="cuda")[1:].view(T, 2 * I).copy_(gu)
+    assert torch.equal(got, K.swiglu(shifted))
+    assert torch.allclose(got.cpu(), plain.swiglu(gu[:, :I], gu[:, I:]), atol=1e-5, rtol=1e-5)
+
+
+@pytest.mark.parametrize("nq,nkv,hd", [(1, 1, 8), (5, 3, 24), (33, 4, 128)])      # a run a half; halves of three runs; more runs than threads
+def test_rope_store_float32_in_runs_of_four(K, nq, nkv, hd):
+    T, W = 67, (nq + 2 * nkv) * hd
+    qkv, (cos, sin) = rnd(T, W, seed=6), plain.rope_angles(torch.arange(T), hd, 1e4)
+    place = [dev(torch.arange(T, dtype=torch.int32)), dev(torch.zeros(T, dtype=torch.int32))]
+    table, out = dev(torch.tensor([[1, 0]], dtype=torch.int32)), []
+    for skip in (0, 1):                                        # at 1 the rows do not begin on 16 bytes: a pair at a time
+        buf = torch.empty(T * W + skip, device="cuda")[skip:].view(T, W).copy_(qkv)
+        kp, vp = (torch.zeros(2, nkv, PAGE, hd, device="cuda") for _ in range(2))
+        K.rope_store(buf, nq, nkv, hd, dev(cos), dev(sin), *place, kp, vp, table, 2)
+        out.append((buf, kp, vp))
+    # a product and a sum of two products, contracted or not: two roundings of values below 2 |x| <= 10
+    assert all(torch.allclose(a, b, rtol=0, atol=2 * 10 * 2.0 ** -24) for a, b in zip(*out))
+    assert torch.equal(out[0][2], out[1][2]) and torch.equal(out[0][0][:, (nq + nkv) * hd:].cpu(), qkv[:, (nq + nkv) * hd:])
+
+
 def test_residual_and_bias_add(K):
     x, y, b = rnd(6, 50, seed=1), bf(rnd(6, 50, seed=2)), rnd(50, seed=3)
     got = K.residual_add(dev(x.clone()), dev(y.to(torch.bfloat16)))
