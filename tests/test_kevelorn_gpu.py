@@ -403,6 +403,25 @@ def test_a_window_of_one_sees_only_the_token_itself(dtype, D):
 
 # ------------------------------------------------------------------ norms with gates, sums of branches, the stream
 
+@pytest.mark.parametrize("act", ["silu", "sigmoid"])
+@pytest.mark.parametrize("T,H,Dv", [(8193, 1, 4), (2731, 3, 20), (1171, 7, 64), (5462, 3, 68), (1261, 13, 128)])   # one lane a run to all of them; a last warp that is not full
+def test_gated_norm_many_short_runs(T, H, Dv, act):
+    """Many short runs share a warp; few have one each: the same rows through both."""
+    from pico_engine.ops import kernels
+    C = H * Dv
+    g = torch.Generator("cpu").manual_seed(Dv)
+    o, gate = torch.randn(T, C, generator=g), torch.randn(T, C + 8, generator=g).to(torch.bfloat16)
+    o[5] = 0.0
+    for w in (torch.randn(Dv, generator=g), torch.randn(Dv, generator=g).to(torch.bfloat16), torch.randn(Dv + 1, generator=g)[1:], None):
+        w = None if w is None else torch.empty(Dv + 1, dtype=w.dtype, device="cuda")[1:].copy_(w) if w.storage_offset() else w.cuda()
+        for gt in (gate.cuda(), None):
+            run = lambda a, b: kernels.gated_norm(o[a:b].cuda(), Dv, w, 1e-5, None if gt is None else gt[a:b].contiguous(), 4 if gt is not None else 0, act,   # noqa: E731
+                                                  torch.bfloat16)
+            few = torch.cat([run(a, min(a + 4000 // H, T)) for a in range(0, T, 4000 // H)])
+            # float32 sums that differ in their last places, then one rounding to bfloat16: at most a neighbour, 2^-7 of the value
+            assert torch.allclose(run(0, T).float(), few.float(), rtol=2.0 ** -7, atol=1e-30)
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("T,H,Dv,off", [(9, 3, 40, 7), (9, 3, 40, 8), (5, 6, 128, 0), (3, 1, 4100, 4), (4, 5, 6, 3)])
 def test_gated_norm_kernel(dtype, T, H, Dv, off):
