@@ -6,6 +6,8 @@
 // Walking the tokens costs two multiply-adds an element of the state and token in the first and three in the second; as products it is
 // one and one, plus 64 a token and entry of q and v.  All sums are float32 multiply-adds; the powers of a are worked out in float64.
 // Queries, keys (and values, in float32) go through their activation and scale while they are brought to shared memory.
+// bfloat16 rows with heads of 128 x 128, or an even number of heads of 64 x 64, go another way (linear_attention_tcgen05.cu); these kernels have
+// float32 rows and the other sizes.
 #include "linear_attention.cuh"
 #include "chunk_tiles.cuh"
 

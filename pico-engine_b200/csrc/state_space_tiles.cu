@@ -10,7 +10,8 @@
 // Bound by float32 multiply-adds (fma.rn.f32x2: two an instruction, each half rounds as a plain one does).  Decays between two tokens
 // are exp of the difference of running sums of -exp(A_log) dt in float64, which costs no digits however long the chunk's sum.
 // Measured on a B200, 64 heads of 64 columns, 128 state rows, rows of 1,400 and 647 tokens: 1,028 us as a walk, 190 us here (steps 3.5,
-// contributions 61, 70 before the steps had a launch of their own, carry 32, outputs 94: 28 float32 TFLOP/s).
+// contributions 61, 70 before the steps had a launch of their own, carry 32, outputs 94: 28 float32 TFLOP/s).  Heads of 64 columns, an even
+// number of them a group, with 64 or 128 state rows go another way (state_space_tcgen05.cu: 132 us); these kernels have the other sizes.
 #include "state_space.cuh"
 #include "chunk_tiles.cuh"
 
