@@ -9,7 +9,7 @@
 //   warp 0     producer: TMA tiled loads (cp.async.bulk.tensor.2d, 128-byte swizzle) of the two operand
 //              tiles of a 64-wide k block into a ring of stages; the tiles of W of the first stages are
 //              asked for before the kernel waits for its predecessor (no kernel writes weights)
-//   warp 1     allocates tensor memory; one lane issues the tcgen05.mma of a stage (K = 16 each) and commits
+//   warp 1     allocates tensor memory; its elected thread issues the tcgen05.mma of a stage (K = 16 each) and commits
 //              them to the stage's "empty" barrier, the last of a tile to the accumulator's "full" barrier
 //   warps 2-17 epilogue: four warps to each quarter of the accumulator's lanes, taking its 32-column chunks in turn
 //              (a warp issues an instruction every 6 to 8 cycles here, so a scheduler needs several of them to
@@ -85,11 +85,28 @@ __device__ __forceinline__ unsigned long long gt_desc(unsigned smem_addr) {
     return (unsigned long long)((smem_addr >> 4) & 0x3FFFu) | ((unsigned long long)(1024u >> 4) << 32) |
            (1ull << 46) | (2ull << 61);
 }
-__device__ __forceinline__ void gt_mma(unsigned tmem_d, unsigned long long a, unsigned long long b, unsigned idesc, unsigned accumulate) {
-    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                 " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n}"
-                 ::"r"(tmem_d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+__device__ __forceinline__ unsigned gt_elect() {
+    unsigned r;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(r));
+    return r;
 }
+// The four products of a stage (16 columns of K each, 32 bytes further inside the swizzle atom) by the elected thread; the whole warp calls, so
+// that descriptors and addresses are the warp's and not one lane's.  Issued by one lane in a branch of its own, a stage of 128 x 128 x 64 took 560 cycles, its bytes
+// 500 and its products 256; this way q/k/v of 2,048 rows (896 x 1,152) 10.3 -> 8.8 us, 4,864 -> 896 27.0 -> 22.5, 896 -> 896 8.7 -> 7.5; 8,192 rows 25.8 -> 22.1, 98 -> 89,
+// 22.9 -> 20.5.  Products of 256 columns, 512 cycles a stage, do not wait for it (gate/up of 2,048 rows 30.1 -> 29.9).
+template <int CTAS>
+__device__ __forceinline__ void gt_products(unsigned elected, unsigned d, unsigned long long a, unsigned long long b, unsigned idesc, unsigned more) {
+#define GT_MMA(group, x, y, p) " @e tcgen05.mma.cta_group::" group ".kind::f16 [%1], " x ", " y ", %10, " p ";\n"
+#define GT_FOUR(group) \
+    asm volatile("{\n .reg .pred e, f, yes;\n setp.ne.u32 e, %0, 0;\n setp.ne.u32 f, %11, 0;\n setp.eq.u32 yes, 0, 0;\n" \
+                 GT_MMA(group, "%2", "%6", "f") GT_MMA(group, "%3", "%7", "yes") GT_MMA(group, "%4", "%8", "yes") GT_MMA(group, "%5", "%9", "yes") "}" \
+                 ::"r"(elected), "r"(d), "l"(a), "l"(a + 2), "l"(a + 4), "l"(a + 6), "l"(b), "l"(b + 2), "l"(b + 4), "l"(b + 6), "r"(idesc), "r"(more) : "memory")
+    if constexpr (CTAS == 1) GT_FOUR("1");
+    else GT_FOUR("2");
+#undef GT_FOUR
+#undef GT_MMA
+}
+static_assert(GT_BK == 64, "four products a stage");
 __device__ __forceinline__ void gt_commit(unsigned bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -457,7 +474,8 @@ __global__ void __launch_bounds__(GT_THREADS) gemm_tcgen05_kernel(const __grid_c
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {                                            // ---------------- MMA issuer
+        {                                                           // ---------------- MMA issuer: the warp waits, one thread issues
+            const unsigned elected = gt_elect();
             // instruction descriptor: float32 accumulator, bfloat16 A and B, both K-major, N = BN (or a part's columns), M = 128
             int s = 0;
             unsigned round = 0;
@@ -466,25 +484,25 @@ __global__ void __launch_bounds__(GT_THREADS) gemm_tcgen05_kernel(const __grid_c
                 const int buf = lt & 1;
                 int begins;
                 const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)((PARTS ? 2 * piece(t, begins) : BN) >> 3) << 17) | ((unsigned)(128 >> 4) << 24);
-                if (!gt_wait(gt_smem(&acc_empty[buf]), (unsigned)((lt >> 1) & 1) ^ 1u, abort_flag)) { ok = false; break; }
+                if (!__all_sync(0xffffffffu, gt_wait(gt_smem(&acc_empty[buf]), (unsigned)((lt >> 1) & 1) ^ 1u, abort_flag))) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const unsigned acc = tmem + (unsigned)(buf * ACC_COLS);
                 for (int kb = 0; kb < k_blocks; ++kb) {
-                    if (!gt_wait(gt_smem(&full_bar[s]), round, abort_flag)) { ok = false; break; }
+                    if (!__all_sync(0xffffffffu, gt_wait(gt_smem(&full_bar[s]), round, abort_flag))) { ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const unsigned base = stage0 + s * STAGE_BYTES;
                     const unsigned long long db = gt_desc(base + A_BYTES);
 #pragma unroll
                     for (int a = 0; a < NA; ++a) {
                         const unsigned long long da = gt_desc(base + a * 128 * GT_BK * 2);
-#pragma unroll
-                        for (int kk = 0; kk < GT_BK / 16; ++kk)      // 16 columns = 32 bytes further inside the swizzle atom
-                            gt_mma(acc + a * BN, da + 2ull * kk, db + 2ull * kk, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+                        gt_products<1>(elected, acc + a * BN, da, db, idesc, kb > 0);
                     }
-                    gt_commit(gt_smem(&empty_bar[s]));               // the stage is free once these MMAs have read it
+                    if (elected) gt_commit(gt_smem(&empty_bar[s]));   // the stage is free once these MMAs have read it
+                    __syncwarp();
                     if (++s == STAGES) { s = 0; round ^= 1u; }
                 }
-                if (ok) gt_commit(gt_smem(&acc_full[buf]));          // all MMAs of the tile done: the accumulator is complete
+                if (ok && elected) gt_commit(gt_smem(&acc_full[buf]));   // all MMAs of the tile done: the accumulator is complete
+                __syncwarp();
             }
             if (!ok) { atomicExch(status, 2); abort_s = 1; }
         }
@@ -542,11 +560,6 @@ __device__ __forceinline__ unsigned gt_map_to_rank(unsigned local_addr, unsigned
 __device__ __forceinline__ void gt_tma_2d_pair(unsigned dst, const CUtensorMap* map, int x, int y, unsigned cluster_bar) {
     asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                  ::"r"(dst), "l"(map), "r"(cluster_bar), "r"(x), "r"(y) : "memory");
-}
-__device__ __forceinline__ void gt_mma_pair(unsigned tmem_d, unsigned long long a, unsigned long long b, unsigned idesc, unsigned accumulate) {
-    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                 " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n}"
-                 ::"r"(tmem_d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
 }
 // arrives on the barrier at this address in both CTAs of the pair once the MMAs issued so far are done
 __device__ __forceinline__ void gt_commit_pair(unsigned bar) {
@@ -645,7 +658,8 @@ __global__ void __launch_bounds__(GT_THREADS) gemm_tcgen05_pair_kernel(const __g
             if (!ok) { atomicExch(status, 2); abort_s = 1; }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {                               // ---------------- MMA issuer (even CTA)
+        if (rank == 0) {                                            // ---------------- MMA issuer (even CTA): the warp waits, one thread issues
+            const unsigned elected = gt_elect();
             // instruction descriptor: float32 accumulator, bfloat16 A and B, both K-major, N = BN, M = 256 over the pair
             const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) | ((unsigned)(256 >> 4) << 24);
             int s = 0;
@@ -653,21 +667,21 @@ __global__ void __launch_bounds__(GT_THREADS) gemm_tcgen05_pair_kernel(const __g
             bool ok = true;
             for (int lt = 0; lt < my_tiles && ok; ++lt) {
                 const int buf = lt & 1;
-                if (!gt_wait(gt_smem(&acc_empty[buf]), (unsigned)((lt >> 1) & 1) ^ 1u, abort_flag)) { ok = false; break; }
+                if (!__all_sync(0xffffffffu, gt_wait(gt_smem(&acc_empty[buf]), (unsigned)((lt >> 1) & 1) ^ 1u, abort_flag))) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const unsigned acc = tmem + (unsigned)(buf * BN);
                 for (int kb = 0; kb < k_blocks; ++kb) {
-                    if (!gt_wait(gt_smem(&full_bar[s]), round, abort_flag)) { ok = false; break; }
+                    if (!__all_sync(0xffffffffu, gt_wait(gt_smem(&full_bar[s]), round, abort_flag))) { ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const unsigned base = stage0 + s * STAGE_BYTES;
                     const unsigned long long da = gt_desc(base), db = gt_desc(base + A_BYTES);
-#pragma unroll
-                    for (int kk = 0; kk < GT_BK / 16; ++kk)
-                        gt_mma_pair(acc, da + 2ull * kk, db + 2ull * kk, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
-                    gt_commit_pair(gt_smem(&empty_bar[s]));
+                    gt_products<2>(elected, acc, da, db, idesc, kb > 0);
+                    if (elected) gt_commit_pair(gt_smem(&empty_bar[s]));
+                    __syncwarp();
                     if (++s == STAGES) { s = 0; round ^= 1u; }
                 }
-                if (ok) gt_commit_pair(gt_smem(&acc_full[buf]));
+                if (ok && elected) gt_commit_pair(gt_smem(&acc_full[buf]));
+                __syncwarp();
             }
             if (!ok) { atomicExch(status, 2); abort_s = 1; }
         }
