@@ -131,7 +131,8 @@ __global__ void __launch_bounds__(DT_THREADS, 1) attention_diff_tcgen05_kernel(c
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {                                            // ---------------- MMA issuer
+        {                                                           // ---------------- MMA issuer: the warp waits, one thread issues
+            const unsigned elected = at_elect();
             // instruction descriptors: float32 accumulator, bfloat16 operands, M = 128; S: A and B K-major, N = 128 keys;
             // O: B MN-major (bit 16), N = Dv rounded up to 16
             const unsigned idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)((2 * DT_KTILE) >> 3) << 17) | ((unsigned)(DT_QTILE >> 4) << 24);
@@ -139,33 +140,33 @@ __global__ void __launch_bounds__(DT_THREADS, 1) attention_diff_tcgen05_kernel(c
             const unsigned long long dq = at_desc(q_s, 0, 1024), dk = at_desc(kv_s, 0, 1024), dp = at_desc(p_s, 0, 1024);
             const unsigned long long dv = at_desc(kv_s + 2 * DT_PANEL, DT_PANEL, 1024);
             const int k_steps = (p.D + 15) >> 4;
-            bool ok = at_wait(at_smem(&q_full), 0u);
+            bool ok = at_wait_warp(at_smem(&q_full), 0u);
             auto issue_s = [&](int it) -> bool {                    // S of iteration `it` (map it & 1) into S buffer it & 1
                 const int st = it >> 1, s = st % DT_STAGES, b = it & 1;
-                if (!at_wait(at_smem(&kv_full[s]), (unsigned)(st / DT_STAGES) & 1u)) return false;
-                if (it >= 2 && !at_wait(at_smem(&s_free[b]), (unsigned)((it >> 1) - 1) & 1u)) return false;
+                if (!at_wait_warp(at_smem(&kv_full[s]), (unsigned)(st / DT_STAGES) & 1u)) return false;
+                if (it >= 2 && !at_wait_warp(at_smem(&s_free[b]), (unsigned)((it >> 1) - 1) & 1u)) return false;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const unsigned long long dqs = dq + (unsigned long long)(b * (DT_PANEL >> 4));
                 const unsigned long long dks = dk + (unsigned long long)(s * (DT_STAGE_BYTES(VP) >> 4) + b * (DT_PANEL >> 4));
                 for (int kk = 0; kk < k_steps; ++kk)                // 16 columns = 32 bytes inside the swizzle atom
-                    at_mma(tmem + b * (2 * DT_KTILE), dqs + kk * 2, dks + kk * 2, idesc_s, kk > 0 ? 1u : 0u);
-                at_commit(at_smem(&s_full[b]));
+                    at_mma(elected, tmem + b * (2 * DT_KTILE), dqs + kk * 2, dks + kk * 2, idesc_s, kk > 0 ? 1u : 0u);
+                at_commit_by(elected, at_smem(&s_full[b]));
                 return true;
             };
             if (ok) ok = issue_s(0);
             for (int it = 0; it < n_its && ok; ++it) {
                 if (it + 1 < n_its && !issue_s(it + 1)) { ok = false; break; }
                 const int s = (it >> 1) % DT_STAGES, b = it & 1;
-                if (!at_wait(at_smem(&p_full), (unsigned)it & 1u)) { ok = false; break; }
+                if (!at_wait_warp(at_smem(&p_full), (unsigned)it & 1u)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const unsigned long long dps = dp + (unsigned long long)(b * (2 * DT_PANEL >> 4)), dvs = dv + (unsigned long long)(s * (DT_STAGE_BYTES(VP) >> 4));
 #pragma unroll
                 for (int kk = 0; kk < 2 * DT_KTILE / 16; ++kk) {    // 16 keys: 32 bytes further in P's rows (64 keys a panel), 16 rows further in V
                     const unsigned off_p = ((kk / 4) * DT_PANEL + (kk % 4) * 32) >> 4, off_v = (kk * 16 * 128) >> 4;
-                    at_mma(tmem + DT_O_COL + b * 128, dps + off_p, dvs + off_v, idesc_o, (it > 1 || kk > 0) ? 1u : 0u);
+                    at_mma(elected, tmem + DT_O_COL + b * 128, dps + off_p, dvs + off_v, idesc_o, (it > 1 || kk > 0) ? 1u : 0u);
                 }
-                if (it & 1) at_commit(at_smem(&kv_empty[s]));       // both maps have read the stage
-                at_commit(at_smem(&pv_done[b]));                    // and O of this map holds this step's share
+                if (it & 1) at_commit_by(elected, at_smem(&kv_empty[s]));       // both maps have read the stage
+                at_commit_by(elected, at_smem(&pv_done[b]));   // and O of this map holds this step's share
             }
             if (!ok) atomicExch(status, 5);
         }

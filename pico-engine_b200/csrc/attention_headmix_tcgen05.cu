@@ -10,7 +10,7 @@
 //   a step    = two pages of the cache (128 keys)
 //   warp 0      loader: TMA tiled loads (128-byte swizzle) of the run's queries and of the pages' keys and the group's values into a ring
 //               of stages; it alone reads the page table and tells the others through flags which pages are there
-//   warp 1      allocates tensor memory; one lane issues S = Q K^T (128 x 128) into one of two buffers and O_c += P V_c for the group's
+//   warp 1      allocates tensor memory; an elected thread issues S = Q K^T (128 x 128) into one of two buffers and O_c += P V_c for the group's
 //               heads: S of the next step before P V of this one
 //   warps 2-9   softmax, two threads a query row, one for each page of the step; P goes as bfloat16 back into the S buffer's own columns,
 //               from where it is the A operand of P V.  O is rescaled only when a row's reference point has moved by more than 2^8.
@@ -135,27 +135,28 @@ __global__ void __launch_bounds__(HT_THREADS, 1) attention_headmix_tcgen05_kerne
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {                                            // ---------------- MMA issuer
+        {                                                           // ---------------- MMA issuer: the warp waits, one thread issues
+            const unsigned elected = at_elect();
             // instruction descriptors: float32 accumulator, bfloat16 operands, M = 128; S: A and B K-major, N = 128 keys;
             // O: A from tensor memory, B MN-major (bit 16), N = Dv
             const unsigned idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)((2 * HT_KTILE) >> 3) << 17) | ((unsigned)(HT_QTILE >> 4) << 24);
             const unsigned idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((unsigned)(p.Dv >> 3) << 17) | ((unsigned)(HT_QTILE >> 4) << 24);
             const unsigned long long dq = at_desc(q_s, 0, 1024), dk = at_desc(kv_s, 0, 1024), dv = at_desc(kv_s + p.qp * HT_PANEL, HT_PANEL, 1024);
             const int k_steps = p.D / 16;
-            bool ok = at_wait(at_smem(&q_full), 0u);
+            bool ok = at_wait_warp(at_smem(&q_full), 0u);
             int s_next = 0, s_here = 0;                             // the stages of the S issued next and of the P V issued next
             unsigned s_round = 0;
             auto issue_s = [&](int it) -> bool {                    // S of step `it` into buffer it & 1, when P V has read the P that lay there
                 const int b = it & 1;
-                if (it >= 2 && !at_wait(at_smem(&pv_done[b]), (unsigned)((it >> 1) - 1) & 1u)) return false;
-                if (!at_wait(at_smem(&kv_full[s_next]), s_round & 1u)) return false;
+                if (it >= 2 && !at_wait_warp(at_smem(&pv_done[b]), (unsigned)((it >> 1) - 1) & 1u)) return false;
+                if (!at_wait_warp(at_smem(&kv_full[s_next]), s_round & 1u)) return false;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const unsigned long long dks = dk + (unsigned long long)(s_next * (stage_bytes >> 4));
                 for (int kk = 0; kk < k_steps; ++kk) {              // 16 columns = 32 bytes inside the swizzle atom; 64 columns = one panel
                     const unsigned off = ((kk / 4) * HT_PANEL + (kk % 4) * 32) >> 4;
-                    at_mma(tmem + b * (2 * HT_KTILE), dq + off, dks + off, idesc_s, kk > 0 ? 1u : 0u);
+                    at_mma(elected, tmem + b * (2 * HT_KTILE), dq + off, dks + off, idesc_s, kk > 0 ? 1u : 0u);
                 }
-                at_commit(at_smem(&s_full[b]));
+                at_commit_by(elected, at_smem(&s_full[b]));
                 if (++s_next == p.stages) { s_next = 0; ++s_round; }
                 return true;
             };
@@ -163,16 +164,16 @@ __global__ void __launch_bounds__(HT_THREADS, 1) attention_headmix_tcgen05_kerne
             for (int it = 0; it < n_steps && ok; ++it) {
                 if (it + 1 < n_steps && !issue_s(it + 1)) { ok = false; break; }
                 const int b = it & 1;
-                if (!at_wait(at_smem(&p_full[b]), (unsigned)(it >> 1) & 1u)) { ok = false; break; }
+                if (!at_wait_warp(at_smem(&p_full[b]), (unsigned)(it >> 1) & 1u)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 for (int v = 0; v < p.cg; ++v) {
                     const unsigned long long dvs = dv + (unsigned long long)(s_here * (stage_bytes >> 4) + v * p.vp * (HT_PANEL >> 4));
 #pragma unroll
                     for (int kk = 0; kk < 2 * HT_KTILE / 16; ++kk)  // 16 keys: 8 columns further in P, 16 rows further in the panels
-                        at_mma_ts(tmem + HT_O_COL + v * p.Dv, tmem + b * (2 * HT_KTILE) + kk * 8, dvs + ((kk * 16 * 128) >> 4), idesc_o, (it > 0 || kk > 0) ? 1u : 0u);
+                        at_mma_ts(elected, tmem + HT_O_COL + v * p.Dv, tmem + b * (2 * HT_KTILE) + kk * 8, dvs + ((kk * 16 * 128) >> 4), idesc_o, (it > 0 || kk > 0) ? 1u : 0u);
                 }
-                at_commit(at_smem(&kv_empty[s_here]));              // the stage's keys and values have been read
-                at_commit(at_smem(&pv_done[b]));                    // and O holds this step's share
+                at_commit_by(elected, at_smem(&kv_empty[s_here]));   // the stage's keys and values have been read
+                at_commit_by(elected, at_smem(&pv_done[b]));   // and O holds this step's share
                 if (++s_here == p.stages) s_here = 0;
             }
             if (!ok) atomicExch(status, 5);

@@ -7,7 +7,7 @@
 //               64-column panels, as values (MN-major)
 //   warp 0      loader: TMA tiled loads (128-byte swizzle) of the run's queries and of the pages' rows into a ring of two stages; it
 //               alone reads the page table and tells the others through flags which pages are there
-//   warp 1      allocates tensor memory; one lane issues S = Q K^T (128 x 128) into one of two buffers and O += P V: S of the next step
+//   warp 1      allocates tensor memory; an elected thread issues S = Q K^T (128 x 128) into one of two buffers and O += P V: S of the next step
 //               before P V of this one
 //   warps 2-9   softmax, two threads a query row, one for each page of the step.  P goes as bfloat16 back into the S buffer's own
 //               columns, from where it is the A operand of P V: with queries of 64 KB and two stages of 64 KB there is no room for it
@@ -127,39 +127,40 @@ __global__ void __launch_bounds__(LT_THREADS, 1) attention_latent_tcgen05_kernel
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {                                            // ---------------- MMA issuer
+        {                                                           // ---------------- MMA issuer: the warp waits, one thread issues
+            const unsigned elected = at_elect();
             // instruction descriptors: float32 accumulator, bfloat16 operands, M = 128; S: A and B K-major, N = 128 keys;
             // O: A from tensor memory, B MN-major (bit 16), N = rank
             const unsigned idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)((2 * LT_KTILE) >> 3) << 17) | ((unsigned)(LT_QTILE >> 4) << 24);
             const unsigned idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((unsigned)(p.rank >> 3) << 17) | ((unsigned)(LT_QTILE >> 4) << 24);
             const unsigned long long dq = at_desc(q_s, 0, 1024), dk = at_desc(kv_s, 0, 1024), dv = at_desc(kv_s, LT_PANEL, 1024);
             const int k_steps = p.width / 16;
-            bool ok = at_wait(at_smem(&q_full), 0u);
+            bool ok = at_wait_warp(at_smem(&q_full), 0u);
             auto issue_s = [&](int it) -> bool {                    // S of step `it` into buffer it & 1, when P V has read the P that lay there
                 const int s = it % LT_STAGES, b = it & 1;
-                if (it >= 2 && !at_wait(at_smem(&pv_done[b]), (unsigned)((it >> 1) - 1) & 1u)) return false;
-                if (!at_wait(at_smem(&kv_full[s]), (unsigned)(it / LT_STAGES) & 1u)) return false;
+                if (it >= 2 && !at_wait_warp(at_smem(&pv_done[b]), (unsigned)((it >> 1) - 1) & 1u)) return false;
+                if (!at_wait_warp(at_smem(&kv_full[s]), (unsigned)(it / LT_STAGES) & 1u)) return false;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const unsigned long long dks = dk + (unsigned long long)(s * (STAGE >> 4));
                 for (int kk = 0; kk < k_steps; ++kk) {              // 16 columns = 32 bytes inside the swizzle atom; 64 columns = one panel
                     const unsigned off = ((kk / 4) * LT_PANEL + (kk % 4) * 32) >> 4;
-                    at_mma(tmem + b * (2 * LT_KTILE), dq + off, dks + off, idesc_s, kk > 0 ? 1u : 0u);
+                    at_mma(elected, tmem + b * (2 * LT_KTILE), dq + off, dks + off, idesc_s, kk > 0 ? 1u : 0u);
                 }
-                at_commit(at_smem(&s_full[b]));
+                at_commit_by(elected, at_smem(&s_full[b]));
                 return true;
             };
             if (ok) ok = issue_s(0);
             for (int it = 0; it < n_steps && ok; ++it) {
                 if (it + 1 < n_steps && !issue_s(it + 1)) { ok = false; break; }
                 const int s = it % LT_STAGES, b = it & 1;
-                if (!at_wait(at_smem(&p_full[b]), (unsigned)(it >> 1) & 1u)) { ok = false; break; }
+                if (!at_wait_warp(at_smem(&p_full[b]), (unsigned)(it >> 1) & 1u)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const unsigned long long dvs = dv + (unsigned long long)(s * (STAGE >> 4));
 #pragma unroll
                 for (int kk = 0; kk < 2 * LT_KTILE / 16; ++kk)      // 16 keys: 8 columns further in P, 16 rows further in the panels
-                    at_mma_ts(tmem + LT_O_COL, tmem + b * (2 * LT_KTILE) + kk * 8, dvs + ((kk * 16 * 128) >> 4), idesc_o, (it > 0 || kk > 0) ? 1u : 0u);
-                at_commit(at_smem(&kv_empty[s]));                   // the stage's rows have been read
-                at_commit(at_smem(&pv_done[b]));                    // and O holds this step's share
+                    at_mma_ts(elected, tmem + LT_O_COL, tmem + b * (2 * LT_KTILE) + kk * 8, dvs + ((kk * 16 * 128) >> 4), idesc_o, (it > 0 || kk > 0) ? 1u : 0u);
+                at_commit_by(elected, at_smem(&kv_empty[s]));   // the stage's rows have been read
+                at_commit_by(elected, at_smem(&pv_done[b]));   // and O holds this step's share
             }
             if (!ok) atomicExch(status, 5);
         }

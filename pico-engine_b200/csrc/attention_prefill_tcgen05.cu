@@ -7,7 +7,7 @@
 //               fixed latency than in work, so fewer and larger ones are issued
 //   warp 0      loader: TMA tiled loads (cp.async.bulk.tensor.2d, 128-byte swizzle) of the run's
 //               queries and, step after step, of the pages' keys and values into a ring
-//   warp 1      allocates tensor memory; one lane issues S = Q.K^T (128 x 128, K = head size) into
+//   warp 1      allocates tensor memory; an elected thread issues S = Q.K^T (128 x 128, K = head size) into
 //               one of three S buffers and O += P.V (128 x head size, K = 128 keys); S runs three
 //               steps ahead of P.V.  A stage's keys are free for the next ones when S has read them,
 //               its values when P.V has
@@ -167,7 +167,8 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_prefill_tcgen05_kerne
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {                                            // ---------------- MMA issuer
+        {                                                           // ---------------- MMA issuer: the warp waits, one thread issues
+            const unsigned elected = at_elect();
             // instruction descriptors: float32 accumulator, bfloat16 operands, M = 128;
             // S: A and B K-major, N = 128 keys;  O: B MN-major (bit 16), N = head size
             const unsigned idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)((2 * AT_KTILE) >> 3) << 17) | ((unsigned)(AT_QTILE >> 4) << 24);
@@ -175,34 +176,34 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_prefill_tcgen05_kerne
             // operand descriptors of stage 0; a stage further on adds its offset in 16-byte units
             const unsigned long long dq = at_desc(q_s, 0, 1024), dk = at_desc(kv_s, 0, 1024);
             const unsigned long long dv = at_desc(kv_s + AT_STAGE_BYTES / 2, 2 * AT_KTILE * 128, 1024);
-            bool ok = at_wait(at_smem(&q_full), 0u);
+            bool ok = at_wait_warp(at_smem(&q_full), 0u);
             auto issue_s = [&](int it) -> bool {                    // S = Q . K^T of step `it`, when P.V has read the P that lay in its buffer
                 const int s = it % AT_STAGES, b = it % AT_BUFFERS;
-                if (it >= AT_BUFFERS && !at_wait(at_smem(&pv_done[b]), (unsigned)(it / AT_BUFFERS - 1) & 1u)) return false;
-                if (!at_wait(at_smem(&k_full[s]), (unsigned)(it / AT_STAGES) & 1u)) return false;
+                if (it >= AT_BUFFERS && !at_wait_warp(at_smem(&pv_done[b]), (unsigned)(it / AT_BUFFERS - 1) & 1u)) return false;
+                if (!at_wait_warp(at_smem(&k_full[s]), (unsigned)(it / AT_STAGES) & 1u)) return false;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const unsigned long long dks = dk + (unsigned long long)(s * (AT_STAGE_BYTES >> 4));
 #pragma unroll
                 for (int kk = 0; kk < AT_HD / 16; ++kk) {           // 16 columns = 32 bytes inside the swizzle atom; 64 columns = one panel
                     const unsigned off_q = ((kk / 4) * (AT_QTILE * 128) + (kk % 4) * 32) >> 4, off_k = ((kk / 4) * (2 * AT_KTILE * 128) + (kk % 4) * 32) >> 4;
-                    at_mma(tmem + b * (2 * AT_KTILE), dq + off_q, dks + off_k, idesc_s, kk > 0 ? 1u : 0u);
+                    at_mma(elected, tmem + b * (2 * AT_KTILE), dq + off_q, dks + off_k, idesc_s, kk > 0 ? 1u : 0u);
                 }
-                at_commit(at_smem(&k_empty[s]));                    // the stage's keys have been read
-                at_commit(at_smem(&s_full[b]));
+                at_commit_by(elected, at_smem(&k_empty[s]));   // the stage's keys have been read
+                at_commit_by(elected, at_smem(&s_full[b]));
                 return true;
             };
             for (int it = 0; it < min(AT_AHEAD, n_steps) && ok; ++it) ok = issue_s(it);
             for (int it = 0; it < n_steps && ok; ++it) {
                 const int s = it % AT_STAGES, b = it % AT_BUFFERS;
-                if (!at_wait(at_smem(&v_full[s]), (unsigned)(it / AT_STAGES) & 1u)) { ok = false; break; }
-                if (!at_wait(at_smem(&p_full[b]), (unsigned)(it / AT_BUFFERS) & 1u)) { ok = false; break; }
+                if (!at_wait_warp(at_smem(&v_full[s]), (unsigned)(it / AT_STAGES) & 1u)) { ok = false; break; }
+                if (!at_wait_warp(at_smem(&p_full[b]), (unsigned)(it / AT_BUFFERS) & 1u)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const unsigned long long dvs = dv + (unsigned long long)(s * (AT_STAGE_BYTES >> 4));
 #pragma unroll
                 for (int kk = 0; kk < 2 * AT_KTILE / 16; ++kk)      // 16 keys: 8 columns further in P, 16 rows further in V
-                    at_mma_ts(tmem + AT_O_COL, tmem + b * (2 * AT_KTILE) + kk * 8, dvs + ((kk * 16 * 128) >> 4), idesc_o, (it > 0 || kk > 0) ? 1u : 0u);
-                at_commit(at_smem(&v_empty[s]));                    // the stage's values have been read
-                at_commit(at_smem(&pv_done[b]));                    // and O holds this step's share
+                    at_mma_ts(elected, tmem + AT_O_COL, tmem + b * (2 * AT_KTILE) + kk * 8, dvs + ((kk * 16 * 128) >> 4), idesc_o, (it > 0 || kk > 0) ? 1u : 0u);
+                at_commit_by(elected, at_smem(&v_empty[s]));   // the stage's values have been read
+                at_commit_by(elected, at_smem(&pv_done[b]));   // and O holds this step's share
                 if (it + AT_AHEAD < n_steps && !issue_s(it + AT_AHEAD)) ok = false;
             }
             if (!ok) atomicExch(status, 5);
