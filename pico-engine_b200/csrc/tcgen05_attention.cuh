@@ -37,8 +37,8 @@ __device__ __forceinline__ unsigned long long at_desc(unsigned smem_addr, unsign
            ((unsigned long long)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46) | (2ull << 61);
 }
 // The thread of a warp that issues products and their commits.  The warp goes through the loop that issues them as one, waits included: in a branch
-// of one lane's own a product took about 90 cycles to issue, and a step's twelve to sixteen stood in its chain.  A prompt of 2,048 tokens through 24 layers of the
-// Qwen2.5-0.5B widths 2,342 -> 2,297 us, the mixer with latent rows 98.2 -> 95.9, with mixed heads 71.5 -> 69.9, differential attention's layer 228 -> 226.
+// of one lane's own a product took about 90 cycles to issue.  The kernels themselves gain little (2,048 tokens, 14 heads of 64: 21.9 -> 21.6 us; differential attention 47.9 -> 47.1;
+// latent rows and mixed heads the same), in a chain of kernels the mixer with latent rows 98.2 -> 95.9 us, with mixed heads 71.5 -> 69.9.
 __device__ __forceinline__ unsigned at_elect() {
     unsigned r;
     asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(r));
