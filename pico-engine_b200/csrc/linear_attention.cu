@@ -255,6 +255,19 @@ static long long la_chunk_floats(int H, int D, int Dv, int per_channel) {
     const long long adds = per_channel ? la_channels_scratch_floats(1, H, D) : 0, parts = la_tensor_sizes(H, D, Dv) ? la_tensor_chunk_floats(H, D) : 0;
     return (long long)H * D * ((long long)Dv + 1) + (adds > parts ? adds : parts);
 }
+// Where a slab's arrays lie in scratch on the tensor cores, in bytes: the widest accesses first.  Parts are read in 16 bytes, places as int2, words as they
+// are, states in runs of 32 bytes, decays as float4 (four floats of a head, whose D is 64 or 128).
+struct LATensorScratch {
+    long long rows, seen, state, decay, end;
+    LATensorScratch(int slab, int H, int D, int Dv) {
+        rows = 4 * (long long)slab * (la_tensor_chunk_floats(H, D) - H - 2);
+        seen = rows + 8ll * slab;
+        state = (seen + 4ll * slab * H + 31) / 32 * 32;
+        decay = state + 4ll * slab * H * D * Dv;
+        end = decay + 4ll * slab * H * D;
+    }
+    bool aligned() const { return rows % 16 == 0 && seen % 4 == 0 && state % 32 == 0 && decay % 16 == 0; }
+};
 static int la_slab(int chunks, int H, int D, int Dv, int per_channel) {
     const long long floats = la_chunk_floats(H, D, Dv, per_channel);
     const long long most = floats >= LA_SCRATCH_FLOATS ? 1 : LA_SCRATCH_FLOATS / floats, slabs = (chunks + most - 1) / most;
@@ -267,6 +280,14 @@ extern "C" int pe_linear_attention_slabs(int T, int B, int H, int D, int Dv, int
 // Floats of scratch the chunked way needs.
 extern "C" long long pe_linear_attention_scratch_floats(int T, int B, int H, int D, int Dv, int per_channel) {
     return la_slab(pe_linear_attention_chunks(T, B), H, D, Dv, per_channel) * la_chunk_floats(H, D, Dv, per_channel) + 8;
+}
+
+// The same places, for whoever checks them without a GPU (places: those of the struct, in its order); 0 where a call of these sizes has none.
+extern "C" int pe_linear_attention_scratch_places(int T, int B, int H, int D, int Dv, int per_channel, long long* places) {
+    if (!la_tensor_sizes(H, D, Dv)) return 0;
+    const LATensorScratch at(la_slab(pe_linear_attention_chunks(T, B), H, D, Dv, per_channel), H, D, Dv);
+    places[0] = at.rows; places[1] = at.seen; places[2] = at.state; places[3] = at.decay; places[4] = at.end;
+    return 1;
 }
 
 extern "C" int pe_linear_attention(const void* proj, int dtype, int ld, int q_off, int k_off, int v_off, const void* z, int z_dtype,
@@ -293,12 +314,14 @@ extern "C" int pe_linear_attention(const void* proj, int dtype, int ld, int q_of
     a.channel_scratch = scratch ? scratch + ((size_t)a.slab * H * D * ((size_t)Dv + 1) + 3) / 4 * 4 : nullptr;      // (read in vectors)
     a.chunk_planes = nullptr;
     if (chunked && status && pe_linear_attention_on_tensor_cores(proj, dtype, ld, v_off, H, D, Dv)) {
-        a.chunk_planes = reinterpret_cast<unsigned char*>(scratch);                                    // (vectors first)
-        a.chunk_seen = reinterpret_cast<unsigned*>(scratch + (size_t)a.slab * (la_tensor_chunk_floats(H, D) - H - 2));
-        a.chunk_rows = reinterpret_cast<int2*>(a.chunk_seen + (size_t)a.slab * H);
-        float* rest = reinterpret_cast<float*>(a.chunk_rows + a.slab);
-        a.chunk_state = scratch + ((rest - scratch) + 7) / 8 * 8;
-        a.chunk_decay = a.chunk_state + (size_t)a.slab * H * D * Dv;
+        const LATensorScratch at(a.slab, H, D, Dv);
+        if (!at.aligned()) return PE_ERR_UNSUPPORTED;
+        char* base = reinterpret_cast<char*>(scratch);
+        a.chunk_planes = reinterpret_cast<unsigned char*>(base);
+        a.chunk_rows = reinterpret_cast<int2*>(base + at.rows);
+        a.chunk_seen = reinterpret_cast<unsigned*>(base + at.seen);
+        a.chunk_state = reinterpret_cast<float*>(base + at.state);
+        a.chunk_decay = reinterpret_cast<float*>(base + at.decay);
         a.status = status;
         a.qk_f32 = qk != nullptr || dtype == PE_F32; a.z_f32 = z_dtype == PE_F32;
     }

@@ -82,6 +82,7 @@ _MIXER_SIGNATURES = {
 _GATED_SIGNATURES = {
     "pe_linear_attention": [P, I, I, I, I, I, P, I, I, P, F, F, I, I, P, LL, P, P, P, P, I, I, I, I, I, I, P, P, I, P, P],
     "pe_linear_attention_on_tensor_cores": [P, I, I, I, I, I, I],
+    "pe_linear_attention_scratch_places": [I, I, I, I, I, I, P],
     "pe_rotary_norm_store": [P, I, I, I, I, I, I, I, P, I, I, F, P, P, P, P, P, I, I, P],
     "pe_gated_norm": [P, I, I, I, I, P, I, F, P, I, I, I, P, I, P],
     "pe_normed_sum_add": [P, P, P, P, P, I, P, P, P, P, I, I, I, I, F, F, P],

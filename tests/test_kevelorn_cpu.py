@@ -149,6 +149,29 @@ def test_scratch_of_a_batch_of_prompts_is_bounded(per_channel):
     assert state_space().pe_state_space_slabs(2048, 1, 64, 64, 128, 2) == 1
 
 
+@pytest.mark.parametrize("per_channel", [0, 1])
+@pytest.mark.parametrize("D", [64, 128])
+def test_scratch_of_the_tensor_cores_is_aligned_for_what_reads_it(D, per_channel):
+    """Any number of heads and chunks, odd ones too: parts and states start where 16 and 32 bytes are read at once, a chunk's place where 8 are,
+    nothing overlaps and all of it lies in the scratch."""
+    import ctypes
+    from pico_engine.ops.library import gated
+    lib, places = gated(), (ctypes.c_longlong * 5)()
+    for H in range(1, 17):
+        for chunks in range(2, 200):
+            T = 64 * (chunks - 1)
+            sizes = (T, 1, H, D, D, per_channel)
+            if not lib.pe_linear_attention_scratch_places(*sizes, ctypes.addressof(places)):
+                assert D == 64 and H % 2
+                continue
+            rows, seen, state, decay, end = places
+            slab = -(-chunks // lib.pe_linear_attention_slabs(*sizes))
+            assert rows % 16 == 0 and seen % 4 == 0 and state % 32 == 0 and decay % 16 == 0, (H, chunks)
+            planes = (12 + 3 * (1 if D == 128 else 2) + 6) * 8192 * (H if D == 128 else H // 2)
+            assert rows >= slab * planes and seen - rows >= 8 * slab and state - seen >= 4 * slab * H and decay - state >= 4 * slab * H * D * D
+            assert end - decay >= 4 * slab * H * D and end <= 4 * lib.pe_linear_attention_scratch_floats(*sizes), (H, chunks)
+
+
 ONES = [1] * 63
 
 

@@ -669,6 +669,18 @@ def test_linear_attention_products_on_the_tensor_cores(H, D, per_channel, logits
             assert (walk - chunks).abs().max() < 2e-5 * max(1.0, float(walk.abs().max())), act
 
 
+@pytest.mark.parametrize("per_channel", [False, True])
+@pytest.mark.parametrize("H,lens", [(1, [65]), (5, [200]), (7, [2048]), (3, [130, 3])])
+def test_odd_heads_and_odd_chunks_on_the_tensor_cores(H, lens, per_channel):
+    """An odd number of heads times an odd number of chunks: whatever lies behind their words in scratch starts on its own boundary."""
+    D = 128
+    proj, run = tensor_core_rows(H, D, lens, per_channel, H)
+    for act in ("none", "silu"):
+        for walk, chunks in zip(run(proj, False, v_activation=act), run(proj, True, v_activation=act)):
+            # float32 sums of the same products in another order (the bound of the tests above)
+            assert (walk - chunks).abs().max() < 2e-5 * max(1.0, float(walk.abs().max())), act
+
+
 def test_float32_queries_and_keys_on_the_tensor_cores():
     """Queries and keys in float32 rows of their own, which start anywhere."""
     H, D, lens = 2, 128, [200, 65]
