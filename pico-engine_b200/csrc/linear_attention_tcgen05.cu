@@ -227,6 +227,7 @@ __global__ void __launch_bounds__(512, 2) lm_channels_kernel(LAArgs a, int vec_q
     la_find_chunk(a.row_first, a.row_lens, a.B, a.first_chunk + blockIdx.x, seq, first, n);
     if (tid == 0 && h == 0) a.chunk_rows[blockIdx.x] = make_int2(first, n);
     if (n <= 0) return;
+    __syncthreads();                                       // (the words stand before a value that is no number lowers one)
     const bool there = row < n;
     const size_t token = first + (there ? row : 0);
     unsigned char* unit = Unit::of(a, blockIdx.x, h);

@@ -48,3 +48,14 @@ def test_prompt_kernels_read_nothing_before_the_kernel_in_front_has_ended(name):
     with open(os.path.join(CSRC, f"attention_{name}_tcgen05.cu")) as f:
         body = f.read().split("__global__", 1)[1]
     assert body.index("pdl_wait();") < min(body.index(what) for what in ("p.tiles[", "p.block_table", "table["))
+
+
+@pytest.mark.parametrize("name,kernel", [("linear_attention_tcgen05", "lm_prepare_kernel"), ("linear_attention_tcgen05", "lm_channels_kernel"), ("state_space_tcgen05", "sm_steps_kernel")])
+def test_words_that_a_block_lowers_stand_before_any_thread_does(name, kernel):
+    """One thread sets the words that tell of entries which are no numbers; the block meets before any other may change them, or its store
+    could come behind theirs and forget a token."""
+    with open(os.path.join(CSRC, name + ".cu")) as f:
+        body = f.read().split(kernel + "(", 1)[1].split("__global__", 1)[0]
+    body = body[body.index("seen = 0;"):]
+    first = min(body.index(what) for what in ("lm_values(", "lm_put_mended(", "cm_report(", "cm_mend(", "atomicMin(") if what in body)
+    assert "__syncthreads();" in body[:first]
