@@ -10,8 +10,9 @@ follows it in a layer: the choice of kernel for a matrix product.
   this library's kernel for that step.  Which of the two is faster depends on the sizes (the library
   has tile shapes and TMA multicast that this kernel has not; this kernel saves a pass over the product),
   so the first time a product of some shape is asked for, both are timed on the device, a few replays of
-  a captured CUDA graph each, and the faster one is remembered (``Choice``).  ``PICO_ENGINE_GEMM=tcgen05``
-  or ``=library`` fixes the choice instead.
+  a captured CUDA graph each, and the faster one is remembered (``Choice``; the library's where the two are
+  nearly as fast, so that a result's last bits do not hang on a clock's noise).  A sum into the stream that may wait
+  for the norm behind it is timed with that norm.  ``PICO_ENGINE_GEMM=tcgen05`` or ``=library`` fixes the choice instead.
 * float32 activations and weights (the float32 engine): the tensor cores with each operand in three
   parts that hold all its bits, at float32 accuracy, ``csrc/linear_split.cu``; matrices of less than 800,000 entries, and
   anything else (weights that were stored in float32 beside bfloat16 rows): float32 multiply-adds on
@@ -71,11 +72,14 @@ class Choice:
     # to CAPTURED_ROWS rows are decode steps, replayed from a graph, where only device time counts.
     HOST_US_PER_LAUNCH = 6.0
     CAPTURED_ROWS = 128
+    # The two ways round differently, so a decision must not depend on the noise of one timing (1 to 2 % from process to process on a B200; 4 % for
+    # products of a millisecond under the power cap): the fused kernel is taken where it is faster by more than this share.
+    NEAR = 0.04
 
     @classmethod
-    def pick(cls, key: Tuple, own: Callable[[], object], library: Callable[[], object], launches_saved: int = 0) -> str:
-        """"tcgen05" or "library" for ``key``; the two callables run the product on scratch operands
-        of the key's sizes; ``launches_saved``: how many launches fewer the fused kernel is.  While a CUDA
+    def pick(cls, key: Tuple, sides: Callable[[], Tuple[Callable[[], object], Callable[[], object]]], launches_saved: int = 0) -> str:
+        """"tcgen05" or "library" for ``key``; ``sides`` makes the two callables, this library's and the other, that run the product
+        on scratch operands of the key's sizes; ``launches_saved``: how many launches fewer the fused kernel is.  While a CUDA
         graph is being captured nothing can be timed: the library product runs, and the question is asked
         again outside a capture."""
         got = cls.table.get(key)
@@ -86,10 +90,11 @@ class Choice:
             return _FORCED
         if torch.cuda.is_current_stream_capturing():
             return "library"
+        own, library = sides()
         t_own, t_lib = _device_time(own), _device_time(library)
         cls.timings[key] = (t_own, t_lib)
         host = cls.HOST_US_PER_LAUNCH * launches_saved if key[1] > cls.CAPTURED_ROWS else 0.0
-        cls.table[key] = "tcgen05" if t_own < t_lib + host else "library"
+        cls.table[key] = "tcgen05" if t_own < (1.0 - cls.NEAR) * (t_lib + host) else "library"
         return cls.table[key]
 
 
@@ -131,7 +136,9 @@ def _device_time(fn: Callable[[], object], calls: int = 6, replays: int = 3) -> 
 
 
 def _scratch_rows(rows: int, cols: int, dtype, device) -> torch.Tensor:
-    return torch.zeros(rows, cols, dtype=dtype, device=device)
+    """Operands to time with: numbers, not zeros, which a large product multiplies at a higher clock (8,192 rows of 18,944 x 3,584 with the norm
+    behind it, this library's kernel / the other: 738 / 717 us of zeros, 883 / 831 of numbers)."""
+    return torch.randn(rows, cols, generator=torch.Generator(device).manual_seed(0), dtype=dtype, device=device)
 
 
 def _takes_tcgen05(a: torch.Tensor, w: torch.Tensor) -> bool:
@@ -151,12 +158,20 @@ def linear(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
         if bias is None and accumulate_into is None and out_dtype == torch.float32:
             return torch.mm(a, w.t(), out_dtype=torch.float32)   # the logits: the library's float32 accumulator as it is
         if accumulate_into is not None and bias is None and _takes_tcgen05(a, w):
-            key = ("accumulate", Choice.bucket(M), w.shape[0], w.shape[1])
+            # A sum that may wait costs the norm that follows a part of its pass only, so each side is timed with that norm: 2,048 rows of
+            # 896 x 896 7.7 / 8.4 us with a pass for the sum, 11.4 / 10.1 as they run; 8,192 of 3,584 x 3,584 151 / 174 and 190 / 183.
+            key = ("accumulate" if defer_add is None else "accumulate_normed", Choice.bucket(M), w.shape[0], w.shape[1])
+
+            def sides():
+                rows, cols = Choice.bucket(M), w.shape[0]
+                sa, sx = _scratch_rows(rows, a.shape[1], a.dtype, a.device), _scratch_rows(rows, cols, torch.float32, a.device)
+                if defer_add is None:
+                    return (lambda: kernels.gemm_tcgen05(sa, w, accumulate_into=sx)), (lambda: kernels.residual_add(sx, torch.mm(sa, w.t())))
+                weight = torch.ones(cols, dtype=a.dtype, device=a.device)
+                return (lambda: kernels.rmsnorm(kernels.gemm_tcgen05(sa, w, accumulate_into=sx), weight, 1e-6, a.dtype)), \
+                       (lambda: kernels.add_rmsnorm(sx, torch.mm(sa, w.t()), weight, 1e-6, a.dtype))
             if key not in Choice.table:
-                rows = Choice.bucket(M)
-                sa, sx = _scratch_rows(rows, a.shape[1], a.dtype, a.device), _scratch_rows(rows, w.shape[0], torch.float32, a.device)
-                Choice.pick(key, lambda: kernels.gemm_tcgen05(sa, w, accumulate_into=sx),
-                            lambda: kernels.residual_add(sx, torch.mm(sa, w.t())))
+                Choice.pick(key, sides)
             if Choice.table.get(key) == "tcgen05":
                 return kernels.gemm_tcgen05(a, w, accumulate_into=accumulate_into)
         if bias is not None and bias.dtype == a.dtype:
@@ -186,10 +201,12 @@ def gate_up_act(h: torch.Tensor, w_gate_up: torch.Tensor, activation: str = "sil
         if _takes_tcgen05(h, w_gate_up):
             fused = True if activation == "silu" else activation
             key = ("swiglu" if activation == "silu" else activation + "_gate", Choice.bucket(M), w_gate_up.shape[0], w_gate_up.shape[1])
-            if key not in Choice.table:
+
+            def sides():
                 sh = _scratch_rows(Choice.bucket(M), h.shape[1], h.dtype, h.device)
-                Choice.pick(key, lambda: kernels.gemm_tcgen05(sh, w_gate_up, swiglu=fused), lambda: after(torch.mm(sh, w_gate_up.t())),
-                            launches_saved=1)
+                return (lambda: kernels.gemm_tcgen05(sh, w_gate_up, swiglu=fused)), (lambda: after(torch.mm(sh, w_gate_up.t())))
+            if key not in Choice.table:
+                Choice.pick(key, sides, launches_saved=1)
             if Choice.table.get(key) == "tcgen05":
                 return kernels.gemm_tcgen05(h, w_gate_up, swiglu=fused)
     return after(linear(h, w_gate_up, out_dtype=h.dtype))
@@ -213,17 +230,19 @@ def qkv_rope_store(h: torch.Tensor, w_qkv: torch.Tensor, b_qkv: Optional[torch.T
     kernel; or None where the product followed by the rotation kernel is faster (the caller then runs those)."""
     M = h.shape[0]
     key = ("rope", Choice.bucket(M), w_qkv.shape[0], w_qkv.shape[1], head_dim)
-    if key not in Choice.table:
+
+    def sides():
         rows = Choice.bucket(M)
         sh = _scratch_rows(rows, h.shape[1], h.dtype, h.device)
         pos = torch.zeros(rows, dtype=torch.int32, device=h.device)
-        # timed without the cache write on both sides (a scratch cache would have to be as large as the real one)
-        own = lambda: kernels.gemm_qkv_rope_store(sh, w_qkv, b_qkv, n_q, n_kv, head_dim, cos, sin, pos, pos, None, None, None, 0)
 
         def library():
             y = linear(sh, w_qkv, b_qkv, out_dtype=h.dtype)
             kernels.rope_store(y, n_q, n_kv, head_dim, cos, sin, pos, pos, None, None, None, 0)
-        Choice.pick(key, own, library, launches_saved=1)
+        # timed without the cache write on both sides (a scratch cache would have to be as large as the real one)
+        return (lambda: kernels.gemm_qkv_rope_store(sh, w_qkv, b_qkv, n_q, n_kv, head_dim, cos, sin, pos, pos, None, None, None, 0)), library
+    if key not in Choice.table:
+        Choice.pick(key, sides, launches_saved=1)
     if Choice.table.get(key) != "tcgen05":
         return None
     return kernels.gemm_qkv_rope_store(h, w_qkv, b_qkv, n_q, n_kv, head_dim, cos, sin, tok_pos, tok_row, k_pool, v_pool,
