@@ -111,12 +111,23 @@ __global__ void __launch_bounds__(1024) latent_prepare_vec_kernel(const bf16* pr
 #pragma unroll
     for (int e = 0; e < 4; ++e) { f[2 * e] = __uint_as_float(w4[e] << 16); f[2 * e + 1] = __uint_as_float(w4[e] & 0xffff0000u); }
     if (latent) {
-        float ss = 0.f;
+        // the sum in the order of the kernel above, where a thread has one entry: over the 32 of a warp, then over its warps, halves first; the same bits
+        float sq[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) ss = fmaf(f[e], f[e], ss);
-        const float rstd = 1.0f / sqrtf(warp_sum(ss) / (float)rank + eps);
+        for (int e = 0; e < 8; ++e) sq[e] = f[e] * f[e];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) f[e] *= rstd * (on ? load_as_f(norm_w, nw_dtype, i + e) : 0.f);
+        for (int o = 2; o > 0; o >>= 1)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) sq[e] += __shfl_xor_sync(0xffffffffu, sq[e], o);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+            for (int e = 0; e < o; ++e) sq[e] += sq[e + o];
+#pragma unroll
+        for (int o = 16; o > 2; o >>= 1) sq[0] += __shfl_xor_sync(0xffffffffu, sq[0], o);
+        const float rstd = 1.0f / sqrtf(sq[0] / (float)rank + eps);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] = f[e] * rstd * (on ? load_as_f(norm_w, nw_dtype, i + e) : 0.f);
     }
     __syncthreads();
     if (!latent && on) {
@@ -124,8 +135,8 @@ __global__ void __launch_bounds__(1024) latent_prepare_vec_kernel(const bf16* pr
         for (int e = 0; e < 8; e += 2)
             if (i + e + 1 < rot_dims) {
                 const float2 c = turn[(i + e) / 2];
-                const float a0 = f[e], a1 = f[e + 1];
-                f[e] = a0 * c.x - a1 * c.y; f[e + 1] = a1 * c.x + a0 * c.y;
+                const float a0 = f[e], a1 = f[e + 1];                   // (which product stays unrounded as the compiler has it above: the same bits)
+                f[e] = fmaf(a0, c.x, -__fmul_rn(a1, c.y)); f[e + 1] = fmaf(a1, c.x, __fmul_rn(a0, c.y));
             }
     }
     bf16* to = latent ? (dst ? dst + i : nullptr) : who == 0 ? (dst ? dst + rank + i : nullptr) : q_out + ((size_t)t * H + who - 1) * W + rank + i;
