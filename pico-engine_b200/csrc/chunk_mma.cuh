@@ -3,9 +3,10 @@
 // below 2^-25 of theirs).  The tensor cores cut their sums to 24 bits, so hi hi is summed over 32 entries at a time and these sums are
 // added as float32 numbers are; the small products, 2^-8 of it at most, are summed first.
 //
-// What three parts cannot hold is infinities, numbers that are none, numbers that round to an infinity, and tiles of nothing but numbers
-// below 2^-90, whose small parts fall out of bfloat16's range: cm_watch finds them on the way, and the results that they reach are worked
-// out with multiply-adds.  (A token that is no number reaches none in front of it: cm_mend puts zeros in its place, and those keep their bits.)
+// Numbers are cut times 2^24, so that the lowest part of the smallest of them is still a bfloat16 number, and results are brought back: a power of two
+// changes no bits.  What parts are not made of is numbers of 2^35 and more (sums of products of smaller ones stay inside float32), infinities and numbers that are
+// none: cm_watch finds them on the way, and the results that they reach are worked out with multiply-adds.  (A token with such a number reaches none in
+// front of it: cm_mend puts zeros in its place, and those keep their bits.)
 //
 // A plane is 64 rows (tokens) of 64 bfloat16 numbers, a part each: rows of 128 bytes whose eight 16-byte groups are exchanged by the row's
 // place in a run of eight, which is what the 128-byte swizzle of an operand in shared memory is, along a row (K-major) or across rows.
@@ -15,6 +16,10 @@
 #define CM_CHUNK 64                                       // tokens of a chunk
 #define CM_PLANE (CM_CHUNK * 128)                         // bytes
 #define CM_PARTS 3
+#define CM_UP 0x1p24f
+#define CM_DOWN 0x1p-24f                                  // for each operand that was cut
+#define CM_MOST 0x5d00u                                   // 2^59 as bfloat16: 2^35 times 2^24
+#define CM_MOST_PLAIN 0x5100u                             // 2^35, of numbers that are bfloat16 already
 
 __device__ __forceinline__ unsigned cm_at(int row, int group) { return row * 128 + ((group ^ (row & 7)) << 4); }      // eight numbers of a row in a plane
 
@@ -24,35 +29,40 @@ __device__ __forceinline__ unsigned long long cm_pair(unsigned a, unsigned b) {
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b));
     return r;
 }
+__device__ __forceinline__ float2 cm_scaled(float a, float b, float by) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(at_two(a, b)), "l"(at_two(by, by)));
+    return at_both(r);
+}
+template <int N>
+__device__ __forceinline__ void cm_scale(float (&v)[N], float by) {
+#pragma unroll
+    for (int i = 0; i < N; i += 2) { const float2 r = cm_scaled(v[i], v[i + 1], by); v[i] = r.x; v[i + 1] = r.y; }
+}
+// (numbers times CM_UP)
 __device__ __forceinline__ void cm_cut(float a, float b, unsigned& hi, unsigned& mid, unsigned& lo) {
     unsigned long long rest = at_two(a, b);
     const unsigned long long minus = at_two(-1.f, -1.f);
+    float2 r;
     hi = at_pack(a, b);
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(rest) : "l"(cm_pair(hi << 16, hi & 0xffff0000u)), "l"(minus));      // (exact)
-    float2 r = at_both(rest);
+    r = at_both(rest);
     mid = at_pack(r.x, r.y);
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(rest) : "l"(cm_pair(mid << 16, mid & 0xffff0000u)), "l"(minus));
     r = at_both(rest);
     lo = at_pack(r.x, r.y);
 }
-// The largest upper part that was seen (no number beats every number); its bits in a block's word, for up to five tiles of a block: something that its
-// parts do not hold, something of a usual size, something tiny.
+// The largest upper part that was seen (no number beats every number); whether it is more than parts are made of, as a tile's bit of a word.
 __device__ __forceinline__ void cm_watch(unsigned& most, unsigned hi) {
     asm("{\n\t.reg .b32 t;\n\tabs.bf16x2 t, %1;\n\tmax.NaN.bf16x2 %0, %0, t;\n\t}" : "+r"(most) : "r"(hi));
 }
-__device__ __forceinline__ unsigned cm_seen(unsigned most, int tile) {
-    const unsigned a = most & 0x7fffu, b = (most >> 16) & 0x7fffu, m = a > b ? a : b;
-    return (m >= 0x7f80u ? 1u : m >= 0x1280u ? 2u : m ? 4u : 0u) << (3 * tile);      // 0x1280: 2^-90
-}
-#define CM_TILES 0x1249u                                  // the first bits of five tiles
-__device__ __forceinline__ bool cm_odd(unsigned seen) { return (seen & CM_TILES) != 0; }
-__device__ __forceinline__ bool cm_odd_tile(unsigned seen, int tile) { return (seen >> (3 * tile)) & 1u; }
-__device__ __forceinline__ bool cm_tiny(unsigned seen) { return ((seen >> 2) & ~(seen >> 1) & ~seen & CM_TILES) != 0; }      // some tile of nothing but tiny numbers
+__device__ __forceinline__ bool cm_odd(unsigned most, unsigned limit = CM_MOST) { return (most & 0x7fffu) >= limit || ((most >> 16) & 0x7fffu) >= limit; }
+__device__ __forceinline__ unsigned cm_seen(unsigned most, int tile, unsigned limit = CM_MOST) { return (cm_odd(most, limit) ? 1u : 0u) << tile; }
 __device__ __forceinline__ void cm_report(unsigned* seen, unsigned mine) {         // (a block's word in shared memory)
     const unsigned all = __reduce_or_sync(0xffffffffu, mine);
     if ((threadIdx.x & 31) == 0 && all) atomicOr(seen, all);
 }
-// Eight numbers' parts into planes that lie `stride` bytes apart, at `to` in the first.
+// Eight numbers' parts into planes that lie `stride` bytes apart, at `to` in the first (numbers times CM_UP).
 __device__ __forceinline__ void cm_put(unsigned char* to, int stride, const float4& a, const float4& b, unsigned& most) {
     unsigned part[CM_PARTS][4];
     cm_cut(a.x, a.y, part[0][0], part[1][0], part[2][0]); cm_cut(a.z, a.w, part[0][1], part[1][1], part[2][1]);
@@ -62,13 +72,13 @@ __device__ __forceinline__ void cm_put(unsigned char* to, int stride, const floa
 #pragma unroll
     for (int p = 0; p < CM_PARTS; ++p) *reinterpret_cast<uint4*>(to + p * stride) = make_uint4(part[p][0], part[p][1], part[p][2], part[p][3]);
 }
-// A plane of upper parts of which some is no finite number: zeros for such entries in all of its `parts`, `stride` bytes apart; `first` becomes the first
-// row that has one.  All threads.
-__device__ __forceinline__ void cm_mend(unsigned char* plane, int stride, int parts, unsigned* first) {
+// A plane of upper parts of which some are more than parts are made of: zeros for such entries in all of its `parts`, `stride` bytes apart; `first` becomes
+// the first row that has one.  All threads.
+__device__ __forceinline__ void cm_mend(unsigned char* plane, int stride, int parts, unsigned* first, unsigned limit = CM_MOST) {
 #pragma unroll 1
     for (int i = threadIdx.x; i < CM_PLANE / 4; i += blockDim.x) {
         unsigned* at = reinterpret_cast<unsigned*>(plane) + i;
-        const unsigned v = *at, keep = ((v & 0x7f80u) == 0x7f80u ? 0u : 0xffffu) | ((v & 0x7f800000u) == 0x7f800000u ? 0u : 0xffff0000u);
+        const unsigned v = *at, keep = ((v & 0x7fffu) >= limit ? 0u : 0xffffu) | (((v >> 16) & 0x7fffu) >= limit ? 0u : 0xffff0000u);
         if (keep == 0xffffffffu) continue;
         for (int p = 0; p < parts; ++p) at[p * stride / 4] &= keep;
         atomicMin(first, (unsigned)(i / 32));
@@ -236,5 +246,5 @@ struct CMScores {
             }
         }
     }
-    __device__ __forceinline__ float get(int j, int e) const { return sum[j][e] + small[j][e]; }
+    __device__ __forceinline__ float get(int j, int e) const { return sum[j][e] + small[j][e]; }      // (times CM_UP twice)
 };

@@ -63,7 +63,7 @@ __device__ __forceinline__ void lm_put(unsigned char* to, int stride, const floa
 // The same with zeros for what parts do not hold; first: the first row that has such a number.
 __device__ __noinline__ void lm_mend(unsigned char* to, int stride, float4 a, float4 b, int row, unsigned* first) {
     atomicMin(first, (unsigned)row);
-    const auto fit = [](float v) { unsigned one = 0; cm_watch(one, at_pack(v, 0.f)); return cm_odd(cm_seen(one, 0)) ? 0.f : v; };
+    const auto fit = [](float v) { return fabsf(v) < 0x1p59f ? v : 0.f; };
     unsigned most = 0;
     cm_put(to, stride, make_float4(fit(a.x), fit(a.y), fit(a.z), fit(a.w)), make_float4(fit(b.x), fit(b.y), fit(b.z), fit(b.w)), most);
 }
@@ -71,9 +71,8 @@ __device__ __forceinline__ void lm_put_mended(unsigned char* to, int stride, con
     unsigned mine = 0;
     lm_put(to, stride, v, mine);
     cm_watch(most, mine);
-    if (cm_odd(cm_seen(mine, 0))) lm_mend(to, stride, make_float4(v[0], v[1], v[2], v[3]), make_float4(v[4], v[5], v[6], v[7]), row, first);
+    if (cm_odd(mine)) lm_mend(to, stride, make_float4(v[0], v[1], v[2], v[3]), make_float4(v[4], v[5], v[6], v[7]), row, first);
 }
-__device__ __forceinline__ unsigned lm_value_seen(unsigned most, int act) { return act ? cm_seen(most, 3) : cm_odd(cm_seen(most, 0)) ? 1u << 9 : 2u << 9; }      // (one part holds any finite value)
 // Eight values of a token: parts behind their activation; without one they are only looked at.
 __device__ __forceinline__ void lm_values(const LAArgs& a, unsigned char* to, const bf16* from, bool there, int row, unsigned* first_odd, unsigned& most) {
     unsigned mine = 0;
@@ -82,12 +81,13 @@ __device__ __forceinline__ void lm_values(const LAArgs& a, unsigned char* to, co
         lm_eight(v, from, there, true);
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = la_act<true>(v[i], a.act_v);
+        cm_scale(v, CM_UP);
         lm_put(to, 2 * CM_PLANE, v, mine);
     } else if (there) {
         const uint4 r = *reinterpret_cast<const uint4*>(from);
         cm_watch(mine, r.x); cm_watch(mine, r.y); cm_watch(mine, r.z); cm_watch(mine, r.w);
     }
-    if (cm_odd(cm_seen(mine, 0))) atomicMin(first_odd, (unsigned)row);
+    if (cm_odd(mine, a.act_v ? CM_MOST : CM_MOST_PLAIN)) atomicMin(first_odd, (unsigned)row);
     cm_watch(most, mine);
 }
 
@@ -135,6 +135,8 @@ __global__ void __launch_bounds__(512, 2) lm_prepare_kernel(LAArgs a, int vec_q)
         lm_eight(k, src + a.k_off + 64 * j, there, vec_q);
 #pragma unroll
         for (int i = 0; i < 8; ++i) { q[i] = la_act<true>(q[i], a.act_qk) * a.q_scale; k[i] = la_act<true>(k[i], a.act_qk); }
+        cm_scale(q, CM_UP);
+        cm_scale(k, CM_UP);
         if (j) __syncthreads();
         lm_put_mended(qs + cm_at(row, group), CM_PLANE, q, most[0], row, &from);
         lm_put_mended(ks + cm_at(row, group), CM_PLANE, k, most[1], row, &from);
@@ -158,7 +160,8 @@ __global__ void __launch_bounds__(512, 2) lm_prepare_kernel(LAArgs a, int vec_q)
             for (int e = 0; e < 4; e += 2) {
                 const int t = t0 + lane / 4 + 4 * e, s = s0 + 8 * j + lane % 4 * 2;
                 unsigned hi, mid, lo;
-                cm_cut(s <= t ? acc.get(j, e) * pw[t - s] : 0.f, s + 1 <= t ? acc.get(j, e + 1) * pw[t - s - 1] : 0.f, hi, mid, lo);
+                const float2 scores = cm_scaled(acc.get(j, e), acc.get(j, e + 1), CM_DOWN);      // (times CM_UP once)
+                cm_cut(s <= t ? scores.x * pw[t - s] : 0.f, s + 1 <= t ? scores.y * pw[t - s - 1] : 0.f, hi, mid, lo);
                 cm_watch(most_w, hi);
                 unsigned char* to = qs + cm_at(t, s >> 3) + (s & 7) * 2;
                 *reinterpret_cast<unsigned*>(to) = hi;
@@ -166,9 +169,9 @@ __global__ void __launch_bounds__(512, 2) lm_prepare_kernel(LAArgs a, int vec_q)
                 *reinterpret_cast<unsigned*>(to + 2 * CM_PLANE) = lo;
             }
     }
-    cm_report(&seen, cm_seen(most_w, 2) | lm_value_seen(most_v, a.act_v));
+    cm_report(&seen, cm_seen(most_w, 2) | cm_seen(most_v, 3, a.act_v ? CM_MOST : CM_MOST_PLAIN));
     __syncthreads();
-    if (cm_odd_tile(seen, 2)) {
+    if (seen >> 2 & 1u) {
         cm_mend(qs, CM_PLANE, CM_PARTS, &from);
         __syncthreads();
     }
@@ -349,13 +352,16 @@ __global__ void __launch_bounds__(512, 2) lm_channels_kernel(LAArgs a, int vec_q
         float v[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = p[i * 68] * lead[run * D + d + i];
+        cm_scale(v, CM_UP);
         lm_put_mended(unit + Unit::QUERIES + place, 2 * CM_PLANE, v, most_q, row, &from);
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = p[i * 68 + lmc_floats(D)] * follow[run * D + d + i];
+        cm_scale(v, CM_UP);
         lm_put(unit + Unit::KEYS + place, 2 * CM_PLANE, v, most_k);
     }
+    cm_scale(weight, CM_UP);
     lm_put_mended(unit + Unit::WEIGHTS + (TWO ? h & 1 : 0) * CM_PLANE + cm_at(row, group), Unit::W_HEADS * CM_PLANE, weight, most_w, row, &from);
-    cm_report(&seen, cm_seen(most_q, 0) | cm_seen(most_k, 4) | cm_seen(most_w, 2) | lm_value_seen(most_v, a.act_v));
+    cm_report(&seen, cm_seen(most_q, 0) | cm_seen(most_k, 4) | cm_seen(most_w, 2) | cm_seen(most_v, 3, a.act_v ? CM_MOST : CM_MOST_PLAIN));
     __syncthreads();
     if (tid == 0) a.chunk_seen[(size_t)blockIdx.x * a.H + h] = seen | from << 16;
 }
@@ -409,8 +415,7 @@ __global__ void __launch_bounds__(LM_THREADS, 2) lm_contribution_kernel(LAArgs a
         if (next < units) place = a.chunk_rows[next / per];
         cm_landed();
         cm_ready();
-        const unsigned mine = known & 0xffffu;
-        const bool parts = !cm_odd(mine) && !cm_tiny(mine);           // (every thread has read the same words)
+        const bool parts = !(known & (1u << 3 | 1u << 4));            // (every thread has read the same words)
         if (parts) {
             if (warp == 0) {
                 if constexpr (VALUE_PARTS == 1) cm_products_one(elected, tmem, tmem + 128, at_desc(at_smem(vs), CM_PLANE, 1024), 128u, cm_across(at_smem(ks), 2 * CM_PLANE, CM_PLANE), cm_idesc(128, true, true));
@@ -431,6 +436,7 @@ __global__ void __launch_bounds__(LM_THREADS, 2) lm_contribution_kernel(LAArgs a
                 float acc[16];
                 cm_read(acc, at + 128);
                 cm_take(acc, at);
+                cm_scale(acc, VALUE_PARTS == 1 ? CM_DOWN : CM_DOWN * CM_DOWN);
                 float* to = state + (size_t)hh * ND * 64 + ((size_t)((TWO ? column & 63 : column) / 8) * 64 + p) * 8;
                 cm_store8(to, *reinterpret_cast<const float (*)[8]>(acc));
                 cm_store8(to + 512, *reinterpret_cast<const float (*)[8]>(acc + 8));
@@ -531,7 +537,8 @@ __global__ void __launch_bounds__(LM_THREADS, 2) lm_output_kernel(LAArgs a, int 
     for (int unit = blockIdx.x; unit < units && place.y > 0; unit += gridDim.x) {
         const int c = unit / per, h0 = unit % per * (TWO ? 2 : 1), next = unit + gridDim.x, first = place.x, n = place.y;
         if (next < units) place = a.chunk_rows[next / per];
-        const unsigned seen = known & 0xffffu, from = known >> 16;
+        const unsigned from = known >> 16;
+        const bool odd_values = known >> 3 & 1u;
         if (tid == 0) { odd_state = 0; from_s = from; }
         if (scaled && tid < (TWO ? 2 : 1) * LA_CHUNK) {
             double r = 1.0, by = (double)a.head_decay[h0 + (tid >> 6)];
@@ -541,7 +548,11 @@ __global__ void __launch_bounds__(LM_THREADS, 2) lm_output_kernel(LAArgs a, int 
         unsigned most = 0;
         for (int slab = 0; slab < SLABS; ++slab) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) cm_put(ss + (e >> 1) * CM_PLANE + cm_at(tid & 63, (e & 1) * 4 + (tid >> 6)), 2 * CM_PLANE, v[e][0], v[e][1], most);
+            for (int e = 0; e < 4; ++e) {
+                float s[8] = {v[e][0].x, v[e][0].y, v[e][0].z, v[e][0].w, v[e][1].x, v[e][1].y, v[e][1].z, v[e][1].w};
+                cm_scale(s, CM_UP);
+                lm_put(ss + (e >> 1) * CM_PLANE + cm_at(tid & 63, (e & 1) * 4 + (tid >> 6)), 2 * CM_PLANE, s, most);
+            }
             if (slab == 0) cm_landed();
             cm_ready();
             if (warp == 0) {
@@ -561,6 +572,7 @@ __global__ void __launch_bounds__(LM_THREADS, 2) lm_output_kernel(LAArgs a, int 
         cm_read(acc, mine + (TWO ? 128 : 64));
         cm_take(acc, mine);
         if constexpr (!TWO) { cm_take(acc, mine + 192); cm_take(acc, mine + 128); }
+        if constexpr (VALUE_PARTS == 1) cm_scale(acc, CM_DOWN);       // (as the sums over the values come: one of their operands is cut)
         if (scaled) {
 #pragma unroll
             for (int i = 0; i < 32; i += 4) {
@@ -570,10 +582,11 @@ __global__ void __launch_bounds__(LM_THREADS, 2) lm_output_kernel(LAArgs a, int 
         }
         cm_landed();
         cm_ready();
-        const int exact = cm_odd(odd_state) || cm_tiny(odd_state) || cm_tiny(seen & ~(7u << 12)) ? 0 : min(n, (int)from);      // tokens in front of it have their outputs from the parts
-        if (cm_odd_tile(seen, 3)) {
-            cm_mend(ss, 2 * CM_PLANE, VALUE_PARTS, &from_s);
-            cm_mend(ss + CM_PLANE, 2 * CM_PLANE, VALUE_PARTS, &from_s);
+        const int exact = odd_state ? 0 : min(n, (int)from);      // tokens in front of it have their outputs from the parts
+        if (odd_values) {
+            constexpr unsigned LIMIT = VALUE_PARTS == 1 ? CM_MOST_PLAIN : CM_MOST;
+            cm_mend(ss, 2 * CM_PLANE, VALUE_PARTS, &from_s, LIMIT);
+            cm_mend(ss + CM_PLANE, 2 * CM_PLANE, VALUE_PARTS, &from_s, LIMIT);
             cm_ready();
         }
         if (warp == 0) {
@@ -589,6 +602,7 @@ __global__ void __launch_bounds__(LM_THREADS, 2) lm_output_kernel(LAArgs a, int 
         if (next < units && place.y > 0) bring_queries(next);
         cm_take(acc, mine + (TWO ? 128 : 64));
         cm_take(acc, mine);
+        cm_scale(acc, VALUE_PARTS == 1 ? CM_DOWN : CM_DOWN * CM_DOWN);
         float* out = a.out + (size_t)(first + column) * ld_out + h0 * a.Dv + hh * 64 + p;
         if (exact == LA_CHUNK) {
 #pragma unroll

@@ -34,7 +34,10 @@
 #define SM_CONTRIBUTION_SMEM (4 * SM_SLAB + 1024)
 #define SM_OUTPUT_SMEM (4 * SM_SLAB + 1024)
 
-__device__ __forceinline__ float4 sm_times(const float4& v, float w) { return make_float4(v.x * w, v.y * w, v.z * w, v.w * w); }
+__device__ __forceinline__ float4 sm_times(const float4& v, float w) {
+    const float2 a = cm_scaled(v.x, v.y, w), b = cm_scaled(v.z, v.w, w);
+    return make_float4(a.x, a.y, b.x, b.y);
+}
 
 // A chunk's place and where its numbers are read: those of two heads from h on, and their group's B and C.
 struct SMChunk {
@@ -84,10 +87,10 @@ __global__ void __launch_bounds__(SM_THREADS) sm_steps_kernel(ScanArgs a, int ve
             for (int e = 0; e < 2; ++e) chunk.eight(v[e][0], v[e][1], e ? chunk.c : chunk.b, row, k0 + 8 * group);
             __syncthreads();
 #pragma unroll
-            for (int e = 0; e < 2; ++e) cm_put(sm_mem + e * SM_SLAB + cm_at(row, group), CM_PLANE, v[e][0], v[e][1], most[e]);
+            for (int e = 0; e < 2; ++e) cm_put(sm_mem + e * SM_SLAB + cm_at(row, group), CM_PLANE, sm_times(v[e][0], CM_UP), sm_times(v[e][1], CM_UP), most[e]);
             cm_report(&seen, cm_seen(most[0], 0) | cm_seen(most[1], 1));
             __syncthreads();
-            if (cm_odd(seen)) {
+            if (seen) {
                 cm_mend(sm_mem, CM_PLANE, CM_PARTS, &from);
                 cm_mend(sm_mem + SM_SLAB, CM_PLANE, CM_PARTS, &from);
                 __syncthreads();
@@ -101,7 +104,7 @@ __global__ void __launch_bounds__(SM_THREADS) sm_steps_kernel(ScanArgs a, int ve
         }
         if (tid == 0) a.chunk_seen[(size_t)blockIdx.x * a.G + g] = seen | from << 16;
         float* dst = a.chunk_scores + ((size_t)blockIdx.x * a.G + g) * SS_CHUNK * SS_CHUNK;
-        const int exact = cm_tiny(seen) ? 0 : (int)from;   // tokens in front of it have their scores from the parts
+        const int exact = from;                            // tokens in front of it have their scores from the parts
 #pragma unroll 1
         for (int i = exact * SS_CHUNK + tid; i < n * SS_CHUNK; i += SM_THREADS) {
             const int t = i / SS_CHUNK, s = i % SS_CHUNK;
@@ -116,7 +119,7 @@ __global__ void __launch_bounds__(SM_THREADS) sm_steps_kernel(ScanArgs a, int ve
             const int t = t0 + lane / 4 + 4 * e;
             if (t >= exact) continue;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) *reinterpret_cast<float2*>(dst + t * SS_CHUNK + s0 + 8 * j + lane % 4 * 2) = make_float2(acc.get(j, e), acc.get(j, e + 1));
+            for (int j = 0; j < 4; ++j) *reinterpret_cast<float2*>(dst + t * SS_CHUNK + s0 + 8 * j + lane % 4 * 2) = cm_scaled(acc.get(j, e), acc.get(j, e + 1), CM_DOWN * CM_DOWN);
         }
         return;
     }
@@ -177,7 +180,7 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_contribution_kernel(ScanArgs a, 
 #pragma unroll
         for (int e = 0; e < 4; ++e) chunk.eight(v[e][0], v[e][1], chunk.x + (e >> 1) * 64, row + (e & 1) * 32, 8 * group);
         if (tid < 2 * SS_CHUNK) w = a.chunk_steps[((size_t)(unit / pairs) * H + h0 + (tid >> 6)) * SS_MATRIX_STEP_FLOATS + SM_WS + (tid & 63)];
-        if (tid == 0) known = a.chunk_seen[(size_t)(unit / pairs) * a.G + h0 / (H / a.G)] & 0xffffu;
+        if (tid == 0) known = a.chunk_seen[(size_t)(unit / pairs) * a.G + h0 / (H / a.G)] & 1u;      // (B)
     };
     if (place.y > 0) fetch(blockIdx.x, place);
     for (int unit = blockIdx.x; unit < units && place.y > 0; unit += gridDim.x) {
@@ -192,13 +195,13 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_contribution_kernel(ScanArgs a, 
         unsigned most = 0;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            const float by = ws[e >> 1][row + (e & 1) * 32];
-            cm_put(xs + (e >> 1) * CM_PLANE + cm_at(row + (e & 1) * 32, group), 2 * CM_PLANE, sm_times(v[e][0], by), sm_times(v[e][1], by), most);
+            const float by = ws[e >> 1][row + (e & 1) * 32];          // (times x before the power of two: either product alone stays in range)
+            cm_put(xs + (e >> 1) * CM_PLANE + cm_at(row + (e & 1) * 32, group), 2 * CM_PLANE, sm_times(sm_times(v[e][0], by), CM_UP), sm_times(sm_times(v[e][1], by), CM_UP), most);
         }
         cm_report(&seen, cm_seen(most, 2));
         cm_landed();
         cm_ready();
-        const bool parts = !cm_odd(seen) && !cm_tiny(seen);
+        const bool parts = !seen;
         if (parts && warp == 0) {
             cm_products(elected, tmem, tmem + N, cm_across(at_smem(xs), 2 * CM_PLANE, CM_PLANE), cm_across(at_smem(bs), CM_PLANE, SM_SLAB), cm_idesc(N, true, true));
             if (elected) at_commit(at_smem(&bar));
@@ -214,6 +217,7 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_contribution_kernel(ScanArgs a, 
                 float acc[16];
                 cm_read(acc, mine + N);
                 cm_take(acc, mine);
+                cm_scale(acc, CM_DOWN * CM_DOWN);
                 float* to = state + (size_t)hh * N * 64 + ((size_t)(column / 8) * 64 + p) * 8;
                 cm_store8(to, *reinterpret_cast<const float (*)[8]>(acc));
                 cm_store8(to + 512, *reinterpret_cast<const float (*)[8]>(acc + 8));
@@ -338,7 +342,7 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_output_kernel(ScanArgs a, int ve
         const float skip[2] = {load_as_f(a.d_skip, a.d_dtype, h0), load_as_f(a.d_skip, a.d_dtype, h0 + 1)};
         for (int slab = 0; slab < slabs; ++slab) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) cm_put(ss + (e >> 1) * CM_PLANE + cm_at(tid & 63, (e & 1) * 4 + (tid >> 6)), 2 * CM_PLANE, v[e][0], v[e][1], most_s);
+            for (int e = 0; e < 4; ++e) cm_put(ss + (e >> 1) * CM_PLANE + cm_at(tid & 63, (e & 1) * 4 + (tid >> 6)), 2 * CM_PLANE, sm_times(v[e][0], CM_UP), sm_times(v[e][1], CM_UP), most_s);
             if (slab == 0) cm_landed();
             cm_ready();
             if (warp == 0) {
@@ -373,7 +377,7 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_output_kernel(ScanArgs a, int ve
             acc[i] *= d.x; acc[i + 1] *= d.y; acc[i + 2] *= d.z; acc[i + 3] *= d.w;
         }
 #pragma unroll
-        for (int e = 0; e < 4; ++e) cm_put(xs + (e >> 1) * CM_PLANE + cm_at(row + (e & 1) * 32, group), 2 * CM_PLANE, v[e][0], v[e][1], most_x);
+        for (int e = 0; e < 4; ++e) cm_put(xs + (e >> 1) * CM_PLANE + cm_at(row + (e & 1) * 32, group), 2 * CM_PLANE, sm_times(v[e][0], CM_UP), sm_times(v[e][1], CM_UP), most_x);
         // weights: scores times a factor of s and one of its run of eight and t, or (t's own run) one of both; D x_t joins as a weight of the token itself
         float by[4];
 #pragma unroll
@@ -392,11 +396,11 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_output_kernel(ScanArgs a, int ve
             const float factor[8] = {v[e][0].x, v[e][0].y, v[e][0].z, v[e][0].w, v[e][1].x, v[e][1].y, v[e][1].z, v[e][1].w};
 #pragma unroll
             for (int i = 0; i < 8; ++i) w[i] = 8 * group + i > t ? 0.f : fmaf(w[i], factor[i] * by[e], 8 * group + i == t ? skip[k] : 0.f);
-            cm_put(wgt + k * CM_PLANE + cm_at(t, group), 2 * CM_PLANE, make_float4(w[0], w[1], w[2], w[3]), make_float4(w[4], w[5], w[6], w[7]), most_w);
+            cm_put(wgt + k * CM_PLANE + cm_at(t, group), 2 * CM_PLANE, sm_times(make_float4(w[0], w[1], w[2], w[3]), CM_UP), sm_times(make_float4(w[4], w[5], w[6], w[7]), CM_UP), most_w);
         }
         cm_report(&seen, cm_seen(most_s, 2) | cm_seen(most_x, 3) | cm_seen(most_w, 4));
         cm_ready();
-        if (cm_odd(seen)) {
+        if (seen) {
 #pragma unroll 1
             for (int k = 0; k < 2; ++k) {
                 cm_mend(xs + k * CM_PLANE, 2 * CM_PLANE, CM_PARTS, &from);
@@ -410,11 +414,12 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_output_kernel(ScanArgs a, int ve
             __syncwarp();
         }
         float* y = a.y + (size_t)(first + column) * inner + (h0 + hh) * 64 + p;
-        const int exact = cm_odd_tile(seen, 2) || cm_tiny(seen) ? 0 : min(n, (int)from);      // tokens in front of it have their outputs from the parts
+        const int exact = seen >> 2 & 1u ? 0 : min(n, (int)from);      // tokens in front of it have their outputs from the parts
         if (next < units) fetch(next);
         cm_done(&bar, phase, status);
         cm_take(acc, mine + hh * 64);
         cm_take(acc, mine + hh * 64 + 128);
+        cm_scale(acc, CM_DOWN * CM_DOWN);
         if (exact == SS_CHUNK) {
 #pragma unroll
             for (int i = 0; i < 32; ++i) y[i * inner] = acc[i];

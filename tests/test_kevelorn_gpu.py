@@ -648,8 +648,8 @@ def tensor_core_rows(H, D, lens, per_channel, seed, logits=torch.bfloat16):
     decay = {"decay_logits": (2 + 2 * torch.randn(T, H * D, generator=g, device="cuda")).to(logits)} if per_channel else {"head_decay": torch.linspace(0.2, 0.999, H, device="cuda")}
     first, rows, slots = (torch.tensor(v, dtype=torch.int32).cuda() for v in (np.concatenate([[0], np.cumsum(lens)]), lens, range(B)))
 
-    def run(proj, chunked, **more):
-        state = torch.full((B, H * D * D + 3), 0.5, device="cuda")
+    def run(proj, chunked, start=0.5, **more):
+        state = torch.full((B, H * D * D + 3), start, device="cuda")
         o = kernels.linear_attention(proj, 0, H * D, 2 * H * D, H, D, D, state, 3, first, rows, slots, chunked, inv_tau=1 / 16, q_scale=D ** -0.5,
                                      qk_activation="none" if per_channel else "silu", **decay, **more)
         kernels.check_status(torch.device("cuda", torch.cuda.current_device()))
@@ -679,6 +679,29 @@ def test_odd_heads_and_odd_chunks_on_the_tensor_cores(H, lens, per_channel):
         for walk, chunks in zip(run(proj, False, v_activation=act), run(proj, True, v_activation=act)):
             # float32 sums of the same products in another order (the bound of the tests above)
             assert (walk - chunks).abs().max() < 2e-5 * max(1.0, float(walk.abs().max())), act
+
+
+@pytest.mark.parametrize("size", [2.0 ** -122, 2.0 ** 60])
+@pytest.mark.parametrize("which,what", [("v", "a head"), ("v", "some columns"), ("k", "a head"), ("q", "a token")])
+@pytest.mark.parametrize("H,D,per_channel", [(2, 64, False), (2, 64, True), (3, 128, False), (3, 128, True)])
+def test_numbers_of_another_size_beside_others_keep_their_digits(H, D, per_channel, which, what, size):
+    """A head, some columns or a token 2^-122 or 2^60 beside numbers near one: each result to float32 of its own size."""
+    lens = [130, 65]
+    proj, run = tensor_core_rows(H, D, lens, per_channel, 11)
+    at = "qkv".index(which) * H * D
+    rows, cols = slice(None), slice(at + D, at + 2 * D)
+    if what == "some columns":
+        cols = slice(at + D, at + 2 * D, 3)
+    if what == "a token":
+        rows, cols = slice(70, 71), slice(at, at + H * D)
+    proj[rows, cols] *= size
+    for act in ("none", "silu") if which == "v" and size < 1 else ("none",):
+        (o_walk, s_walk), (o, s) = (run(proj, chunked, 0.0, v_activation=act) for chunked in (False, True))
+        o_walk, o, s_walk, s = o_walk.view(-1, H, D), o.view(-1, H, D), s_walk.view(2, H, D, D), s.view(2, H, D, D)
+        # float32 sums of the same products in another order, beside the largest number of the token (of the head) and of the columns of one size
+        for c in (slice(0, None, 3), slice(1, None, 3), slice(2, None, 3)):
+            for walk, chunks, over in ((o_walk[..., c], o[..., c], 2), (s_walk[..., c], s[..., c], (2, 3))):
+                assert ((walk - chunks).abs() <= 6e-5 * walk.abs().amax(dim=over, keepdim=True)).all(), act
 
 
 def test_float32_queries_and_keys_on_the_tensor_cores():

@@ -719,9 +719,9 @@ def tensor_core_case(H, N, G, lens, seed, offset=0):
     first, rows, slots = (torch.tensor(v, dtype=torch.int32).cuda() for v in (np.concatenate([[0], np.cumsum(lens)]), lens, range(len(lens))))
     steps = r(T, H), r(H) - 1.0, 0.7 * r(H) - 0.5, 1 + 0.3 * r(H)
 
-    def run(rows_in, chunked):
+    def run(rows_in, chunked, start=0.5):
         from pico_engine.ops import kernels
-        state = torch.full((len(lens), kernels.state_space_elems(H, 64, N)), 0.5, device="cuda")
+        state = torch.full((len(lens), kernels.state_space_elems(H, 64, N)), start, device="cuda")
         y = kernels.state_space_scan(rows_in, steps[0], 0, *steps[1:], state, 0, first, rows, slots, H, 64, N, G, chunked=chunked)
         kernels.check_status(torch.device("cuda", torch.cuda.current_device()))
         return y, state
@@ -757,12 +757,44 @@ def test_numbers_that_parts_do_not_hold_stay_where_they_are(odd, N, which):
 
 @pytest.mark.parametrize("scale", [1e-36, 1e-30, 1e30])
 def test_state_space_products_at_the_ends_of_the_range(scale):
-    """x far below and far above one: errors as large, beside the results, as at one (numbers below 2^-90 are multiplied as they are)."""
+    """x far below and far above one: errors as large, beside the results, as at one (numbers of 2^35 and more are multiplied as they are)."""
     xbc, run = tensor_core_case(4, 128, 2, [200], 3)
     xbc[:, :256] *= scale
     walk, chunks = run(xbc, False)[0], run(xbc, True)[0]
     # the state begins at 0.5: at 1e-36 nothing of x is left beside it
     assert (walk - chunks).abs().max() < 3e-5 * float(walk.abs().max())
+
+
+@pytest.mark.parametrize("what", ["a head", "a column", "B", "C", "all"])
+@pytest.mark.parametrize("N", [64, 128])
+def test_tiny_numbers_beside_others_keep_their_digits(N, what):
+    """One head's x, one column of it, a token's B or C, and everything, 2^-122 beside numbers near one: each result to float32 of its own size."""
+    H, G, lens, tiny = 4, 2, [200, 65], 2.0 ** -122
+    xbc, run = tensor_core_case(H, N, G, lens, 7)
+    inner = H * 64
+    if what == "a head":
+        xbc[:, 64:128] *= tiny
+    elif what == "a column":
+        xbc[:, 130] *= tiny
+    elif what == "B":
+        xbc[:, inner: inner + G * N] *= tiny
+    elif what == "C":
+        xbc[70, inner + G * N:] *= tiny
+        xbc[70, :inner] = 0.0                                 # (the token's own x joins its output as it is)
+    else:
+        xbc[:, :inner] *= tiny
+    for walk, chunks in zip(run(xbc, False, 0.0), run(xbc, True, 0.0)):
+        if walk.shape[0] == len(lens):                        # states: [sequence][head][rows and columns]
+            walk, chunks = (s.view(len(lens), H, -1) for s in (walk, chunks))
+        else:                                                 # outputs: a column a result of its own
+            walk, chunks = (y.view(-1, H, 64).permute(0, 1, 2) for y in (walk, chunks))
+            rows = [70] if what == "C" else list(range(65))   # (from the first sequence: the second begins anew)
+            walk, chunks = walk[rows], chunks[rows]
+            if what == "a column":
+                walk, chunks = walk[:, :, 2:3], chunks[:, :, 2:3]
+        # float32 sums of the same products in another order, beside the largest of the head (the bound of the tests above)
+        size = walk.abs().amax(dim=(0, 2), keepdim=True)
+        assert ((walk - chunks).abs() <= 3e-5 * size).all()
 
 
 @pytest.mark.parametrize("T", [1, 3, 130])
