@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(SM_THREADS) sm_steps_kernel(ScanArgs a, int ve
     }
     cm_store8(dst + SM_RUNS + 8 * t, runs);
     cm_store8(dst + SM_INSIDE + 8 * t, inside);
-    if (t == 0) a.chunk_decay[(size_t)blockIdx.x * a.H + h] = expf((float)end);
+    if (t == 0) a.chunk_decay[(size_t)blockIdx.x * a.H + h] = (float)exp(end);      // (a state hands its errors on from chunk to chunk)
 }
 
 // Chunks and two heads at a time, contributions: the next unit's x is asked for while this one's products run.
@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_output_kernel(ScanArgs a, int ve
         if (tid == 0) { seen = known & 0xffffu; from = known >> 16; }
         const float* scores = a.chunk_scores + ((size_t)c * a.G + g) * SS_CHUNK * SS_CHUNK;
         unsigned most_s = 0, most_x = 0, most_w = 0;
-        const float skip[2] = {load_as_f(a.d_skip, a.d_dtype, h0), load_as_f(a.d_skip, a.d_dtype, h0 + 1)};
+        const float skips[2] = {load_as_f(a.d_skip, a.d_dtype, h0), load_as_f(a.d_skip, a.d_dtype, h0 + 1)}, skip = skips[hh];
         for (int slab = 0; slab < slabs; ++slab) {
 #pragma unroll
             for (int e = 0; e < 4; ++e) cm_put(ss + (e >> 1) * CM_PLANE + cm_at(tid & 63, (e & 1) * 4 + (tid >> 6)), 2 * CM_PLANE, sm_times(v[e][0], CM_UP), sm_times(v[e][1], CM_UP), most_s);
@@ -378,7 +378,9 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_output_kernel(ScanArgs a, int ve
         }
 #pragma unroll
         for (int e = 0; e < 4; ++e) cm_put(xs + (e >> 1) * CM_PLANE + cm_at(row + (e & 1) * 32, group), 2 * CM_PLANE, sm_times(v[e][0], CM_UP), sm_times(v[e][1], CM_UP), most_x);
-        // weights: scores times a factor of s and one of its run of eight and t, or (t's own run) one of both; D x_t joins as a weight of the token itself
+        // weights: scores times a factor of s and one of its run of eight and t, or (t's own run) one of both.  With 128 state rows D x_t joins as a weight of the
+        // token itself; with 64 it is most of many outputs and comes as a multiply-add at the end: cut with the others' products it left errors of 6.4 to 6.8e-8 of the
+        // outputs' norm where multiply-adds have 4.7 to 5.8 (with 128 rows 7.8e-8 for 1.15e-7)
         float by[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -395,7 +397,7 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_output_kernel(ScanArgs a, int ve
             float w[8] = {sc[0].x, sc[0].y, sc[0].z, sc[0].w, sc[1].x, sc[1].y, sc[1].z, sc[1].w};
             const float factor[8] = {v[e][0].x, v[e][0].y, v[e][0].z, v[e][0].w, v[e][1].x, v[e][1].y, v[e][1].z, v[e][1].w};
 #pragma unroll
-            for (int i = 0; i < 8; ++i) w[i] = 8 * group + i > t ? 0.f : fmaf(w[i], factor[i] * by[e], 8 * group + i == t ? skip[k] : 0.f);
+            for (int i = 0; i < 8; ++i) w[i] = 8 * group + i > t ? 0.f : fmaf(w[i], factor[i] * by[e], 8 * group + i == t && slabs > 1 ? skips[k] : 0.f);
             cm_put(wgt + k * CM_PLANE + cm_at(t, group), 2 * CM_PLANE, sm_times(make_float4(w[0], w[1], w[2], w[3]), CM_UP), sm_times(make_float4(w[4], w[5], w[6], w[7]), CM_UP), most_w);
         }
         cm_report(&seen, cm_seen(most_s, 2) | cm_seen(most_x, 3) | cm_seen(most_w, 4));
@@ -420,6 +422,15 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_output_kernel(ScanArgs a, int ve
         cm_take(acc, mine + hh * 64);
         cm_take(acc, mine + hh * 64 + 128);
         cm_scale(acc, CM_DOWN * CM_DOWN);
+        if (slabs == 1) {                                  // D x_t, from its parts
+            const unsigned char* xt = xs + hh * CM_PLANE + column * 128 + (p & 7) * 2;
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+                const unsigned char* at = xt + cm_at(i, p >> 3);
+                const auto part = [&](int q) { return __uint_as_float((unsigned)*reinterpret_cast<const unsigned short*>(at + q * 2 * CM_PLANE) << 16); };
+                acc[i] = fmaf(skip, ((part(2) + part(1)) + part(0)) * CM_DOWN, acc[i]);
+            }
+        }
         if (exact == SS_CHUNK) {
 #pragma unroll
             for (int i = 0; i < 32; ++i) y[i * inner] = acc[i];

@@ -765,6 +765,39 @@ def test_state_space_products_at_the_ends_of_the_range(scale):
     assert (walk - chunks).abs().max() < 3e-5 * float(walk.abs().max())
 
 
+@pytest.mark.parametrize("H,N,G,lens,most_y,most_state", [(8, 64, 1, [65, 1], 5.7e-8, 9.6e-8), (28, 64, 2, [300, 100], 6.3e-8, 1.04e-7), (28, 128, 2, [300, 100], 1.04e-7, 1.06e-7)])
+def test_state_space_errors_are_no_larger_than_multiply_adds(H, N, G, lens, most_y, most_state):
+    """Outputs and states against 64 bits, beside their norms, means over eight inputs; the bounds are what the multiply-add tiles leave of such inputs."""
+    from pico_engine.ops import kernels
+    errors = []
+    for seed in range(8):
+        g = torch.Generator("cuda").manual_seed(seed)
+        r = lambda *s: torch.randn(*s, device="cuda", generator=g)                       # noqa: E731
+        T, split = sum(lens), kernels.state_space_split(N)
+        xbc, dt_raw = torch.nn.functional.silu(r(T, H * 64 + 2 * G * N)), r(T, H)
+        dt0 = torch.exp(torch.rand(H, device="cuda", generator=g) * 4.6 - 6.9)           # steps of 0.001 to 0.1, decay rates of 1 to 16
+        bias, a_log, skip = dt0 + torch.log(-torch.expm1(-dt0)), torch.log(1 + 15 * torch.rand(H, device="cuda", generator=g)), 1 + 0.05 * r(H)
+        first, rows, slots = (torch.tensor(v, dtype=torch.int32).cuda() for v in (np.concatenate([[0], np.cumsum(lens)]), lens, range(len(lens))))
+        state = torch.zeros(len(lens), kernels.state_space_elems(H, 64, N), device="cuda")
+        y = kernels.state_space_scan(xbc, dt_raw, 0, bias, a_log, skip, state, 0, first, rows, slots, H, 64, N, G, chunked=True)
+        got = state.view(len(lens), H, N // split, 64, split).permute(0, 1, 4, 2, 3).reshape(len(lens), H, N, 64)
+        x, b, c = (t.double() for t in xbc.split([H * 64, G * N, G * N], 1))
+        x, (b, c) = x.view(T, H, 64), (t.view(T, G, N).repeat_interleave(H // G, 1) for t in (b, c))
+        dt = torch.nn.functional.softplus(dt_raw.double() + bias.double(), threshold=100.0)
+        decay, want, ends, at = torch.exp(-torch.exp(a_log.double()) * dt), torch.empty_like(x), [], 0
+        for n in lens:
+            S = torch.zeros(H, N, 64, dtype=torch.float64, device="cuda")
+            for t in range(at, at + n):
+                S = decay[t][:, None, None] * S + (dt[t][:, None] * b[t])[:, :, None] * x[t][:, None]
+                want[t] = (c[t][:, None] @ S)[:, 0] + skip.double()[:, None] * x[t]
+            ends.append(S)
+            at += n
+        ends = torch.stack(ends)
+        errors.append([float((y.view(T, H, 64) - want).norm() / want.norm()), float((got - ends).norm() / ends.norm())])
+    e_y, e_state = np.mean(errors, 0)
+    assert e_y < most_y and e_state < most_state, (e_y, e_state)
+
+
 @pytest.mark.parametrize("what", ["a head", "a column", "B", "C", "all"])
 @pytest.mark.parametrize("N", [64, 128])
 def test_tiny_numbers_beside_others_keep_their_digits(N, what):
