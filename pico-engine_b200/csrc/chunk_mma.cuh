@@ -39,6 +39,83 @@ __device__ __forceinline__ void cm_scale(float (&v)[N], float by) {
 #pragma unroll
     for (int i = 0; i < N; i += 2) { const float2 r = cm_scaled(v[i], v[i + 1], by); v[i] = r.x; v[i + 1] = r.y; }
 }
+// Two numbers at a time, each half as a plain multiply or multiply-add.
+__device__ __forceinline__ unsigned long long cm_mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long cm_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// A walk over a chunk's tokens with multiply-adds, for what parts are not made of: 256 threads, 128 columns.  Eight neighbouring lanes share four columns; a
+// lane has their rows 32 j + 4 (lane % 8) .. + 3 of a state that lies [ND / 8][64 columns][8] (with a column a lane a token's reads of shared memory took 1,500 cycles).
+template <int ND>
+struct CMWalk {
+    static constexpr int RUNS = ND / 32;
+    unsigned long long s[4][2 * RUNS];
+    static __device__ __forceinline__ int column() { return (threadIdx.x >> 3) * 4; }                        // the first of the thread's four
+    static __device__ __forceinline__ int row() { return (threadIdx.x & 7) * 4; }
+    static __device__ __forceinline__ size_t place() { return (size_t)(column() >> 6) * ND * 64 + ((row() >> 3) * 64 + (column() & 63)) * 8 + (row() & 7); }
+    static __device__ __forceinline__ int written() { return column() + (threadIdx.x >> 1 & 2) + (threadIdx.x >> 1 & 1); }      // the column whose output `output` leaves
+    // (no state: zeros); whether each of the thread's columns has a row that is no number, here or in a neighbour: no output of theirs is one then
+    __device__ __forceinline__ bool begin(const float* state) {
+        unsigned lost = 0;
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int j = 0; j < RUNS; ++j) {
+                const float4 f = state ? *reinterpret_cast<const float4*>(state + place() + c * 8 + j * 2048) : make_float4(0.f, 0.f, 0.f, 0.f);
+                s[c][2 * j] = at_two(f.x, f.y); s[c][2 * j + 1] = at_two(f.z, f.w);
+                if (f.x != f.x || f.y != f.y || f.z != f.z || f.w != f.w) lost |= 1u << c;
+            }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) lost |= __shfl_xor_sync(0xffffffffu, lost, o);
+        return lost == 15u;
+    }
+    __device__ __forceinline__ void end(float* state) const {
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int j = 0; j < RUNS; ++j) *reinterpret_cast<ulonglong2*>(state + place() + c * 8 + j * 2048) = make_ulonglong2(s[c][2 * j], s[c][2 * j + 1]);
+    }
+    // s = decay s + k u: k (and decays, if there are any) a token's ND numbers in shared memory
+    __device__ __forceinline__ void step(const float* k, const float* decays, float decay, const float (&u)[4]) {
+        unsigned long long uu[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) uu[c] = at_two(u[c], u[c]);
+#pragma unroll
+        for (int j = 0; j < RUNS; ++j) {
+            const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(k + row() + 32 * j);
+            ulonglong2 d = make_ulonglong2(at_two(decay, decay), at_two(decay, decay));
+            if (decays) d = *reinterpret_cast<const ulonglong2*>(decays + row() + 32 * j);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                s[c][2 * j] = cm_fma2(d.x, s[c][2 * j], cm_mul2(x.x, uu[c]));
+                s[c][2 * j + 1] = cm_fma2(d.y, s[c][2 * j + 1], cm_mul2(x.y, uu[c]));
+            }
+        }
+    }
+    // q . s of column written(), in both lanes that have it
+    __device__ __forceinline__ float output(const float* q) const {
+        unsigned long long sum[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int j = 0; j < RUNS; ++j) {
+            const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(q + row() + 32 * j);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) sum[c] = cm_fma2(x.y, s[c][2 * j + 1], cm_fma2(x.x, s[c][2 * j], sum[c]));
+        }
+        float o[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) { const float2 v = at_both(sum[c]); o[c] = v.x + v.y; }
+        const bool upper = threadIdx.x & 4, odd = threadIdx.x & 2;
+        const float a = (upper ? o[2] : o[0]) + __shfl_xor_sync(0xffffffffu, upper ? o[0] : o[2], 4), b = (upper ? o[3] : o[1]) + __shfl_xor_sync(0xffffffffu, upper ? o[1] : o[3], 4);
+        const float r = (odd ? b : a) + __shfl_xor_sync(0xffffffffu, odd ? a : b, 2);
+        return r + __shfl_xor_sync(0xffffffffu, r, 1);
+    }
+};
 // (numbers times CM_UP)
 __device__ __forceinline__ void cm_cut(float a, float b, unsigned& hi, unsigned& mid, unsigned& lo) {
     unsigned long long rest = at_two(a, b);
@@ -56,6 +133,11 @@ __device__ __forceinline__ void cm_cut(float a, float b, unsigned& hi, unsigned&
 __device__ __forceinline__ void cm_watch(unsigned& most, unsigned hi) {
     asm("{\n\t.reg .b32 t;\n\tabs.bf16x2 t, %1;\n\tmax.NaN.bf16x2 %0, %0, t;\n\t}" : "+r"(most) : "r"(hi));
 }
+// The same of numbers alone.  Where an entry joins every sum of its row (or column) of a product, one that is no number makes them all none, here as with
+// multiply-adds, and reaches no other: nothing is left to be worked out.
+__device__ __forceinline__ void cm_watch_numbers(unsigned& most, unsigned hi) {
+    asm("{\n\t.reg .b32 t;\n\tabs.bf16x2 t, %1;\n\tmax.bf16x2 %0, %0, t;\n\t}" : "+r"(most) : "r"(hi));
+}
 __device__ __forceinline__ bool cm_odd(unsigned most, unsigned limit = CM_MOST) { return (most & 0x7fffu) >= limit || ((most >> 16) & 0x7fffu) >= limit; }
 __device__ __forceinline__ unsigned cm_seen(unsigned most, int tile, unsigned limit = CM_MOST) { return (cm_odd(most, limit) ? 1u : 0u) << tile; }
 __device__ __forceinline__ void cm_report(unsigned* seen, unsigned mine) {         // (a block's word in shared memory)
@@ -63,12 +145,16 @@ __device__ __forceinline__ void cm_report(unsigned* seen, unsigned mine) {      
     if ((threadIdx.x & 31) == 0 && all) atomicOr(seen, all);
 }
 // Eight numbers' parts into planes that lie `stride` bytes apart, at `to` in the first (numbers times CM_UP).
+template <bool NUMBERS = false>
 __device__ __forceinline__ void cm_put(unsigned char* to, int stride, const float4& a, const float4& b, unsigned& most) {
     unsigned part[CM_PARTS][4];
     cm_cut(a.x, a.y, part[0][0], part[1][0], part[2][0]); cm_cut(a.z, a.w, part[0][1], part[1][1], part[2][1]);
     cm_cut(b.x, b.y, part[0][2], part[1][2], part[2][2]); cm_cut(b.z, b.w, part[0][3], part[1][3], part[2][3]);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) cm_watch(most, part[0][i]);
+    for (int i = 0; i < 4; ++i) {
+        if constexpr (NUMBERS) cm_watch_numbers(most, part[0][i]);
+        else cm_watch(most, part[0][i]);
+    }
 #pragma unroll
     for (int p = 0; p < CM_PARTS; ++p) *reinterpret_cast<uint4*>(to + p * stride) = make_uint4(part[p][0], part[p][1], part[p][2], part[p][3]);
 }

@@ -258,11 +258,12 @@ static long long la_chunk_floats(int H, int D, int Dv, int per_channel) {
 // Where a slab's arrays lie in scratch on the tensor cores, in bytes: the widest accesses first.  Parts are read in 16 bytes, places as int2, words as they
 // are, states in runs of 32 bytes, decays as float4 (four floats of a head, whose D is 64 or 128).
 struct LATensorScratch {
-    long long rows, seen, state, decay, end;
+    long long rows, seen, exact, state, decay, end;
     LATensorScratch(int slab, int H, int D, int Dv) {
-        rows = 4 * (long long)slab * (la_tensor_chunk_floats(H, D) - H - 2);
+        rows = 4 * (long long)slab * (la_tensor_chunk_floats(H, D) - 2 * H - 2);
         seen = rows + 8ll * slab;
-        state = (seen + 4ll * slab * H + 31) / 32 * 32;
+        exact = seen + 4ll * slab * H;
+        state = (exact + 4ll * slab * H + 31) / 32 * 32;
         decay = state + 4ll * slab * H * D * Dv;
         end = decay + 4ll * slab * H * D;
     }
@@ -320,6 +321,7 @@ extern "C" int pe_linear_attention(const void* proj, int dtype, int ld, int q_of
         a.chunk_planes = reinterpret_cast<unsigned char*>(base);
         a.chunk_rows = reinterpret_cast<int2*>(base + at.rows);
         a.chunk_seen = reinterpret_cast<unsigned*>(base + at.seen);
+        a.unit_exact = reinterpret_cast<int*>(base + at.exact);
         a.chunk_state = reinterpret_cast<float*>(base + at.state);
         a.chunk_decay = reinterpret_cast<float*>(base + at.decay);
         a.status = status;

@@ -25,6 +25,7 @@ struct LAArgs {
     unsigned char* chunk_planes;   // the units' queries, keys and weights as bfloat16 parts
     unsigned* chunk_seen;          // [chunks][H]: what cm_watch saw of them
     int2* chunk_rows;              // [chunks]: first packed token and number of tokens
+    int* unit_exact;               // [chunks][units]: tokens of a unit's chunk whose outputs come from parts
     int* status;
     int qk_f32, z_f32;
 };

@@ -33,7 +33,7 @@ template <bool TWO> struct LMUnit {
     static __device__ __forceinline__ unsigned char* of(const LAArgs& a, int c, int h) { return a.chunk_planes + ((size_t)c * (TWO ? a.H / 2 : a.H) + (TWO ? h / 2 : h)) * BYTES; }
 };
 
-// Tiles of a chunk's and head's word: 0 queries, 1 keys (with one decay a head), 2 weights, 3 values, 4 keys times their decays.
+// Tiles of a chunk's and head's word: 0 queries, 1 keys (with one decay a head), 2 weights, 3 values; of numbers alone (cm_watch_numbers) 4 keys times their decays, 5 values.
 // From bit 16 on the first token with an entry that parts do not hold.
 
 // Eight neighbouring numbers of a row, zeros behind the chunk's tokens.
@@ -57,8 +57,9 @@ __device__ __forceinline__ void lm_eight(float (&v)[8], const TQ* p, bool there,
         for (int i = 0; i < 8; ++i) v[i] = to_f(p[i]);
     }
 }
+template <bool NUMBERS = false>
 __device__ __forceinline__ void lm_put(unsigned char* to, int stride, const float (&v)[8], unsigned& most) {
-    cm_put(to, stride, make_float4(v[0], v[1], v[2], v[3]), make_float4(v[4], v[5], v[6], v[7]), most);
+    cm_put<NUMBERS>(to, stride, make_float4(v[0], v[1], v[2], v[3]), make_float4(v[4], v[5], v[6], v[7]), most);
 }
 // The same with zeros for what parts do not hold; first: the first row that has such a number.
 __device__ __noinline__ void lm_mend(unsigned char* to, int stride, float4 a, float4 b, int row, unsigned* first) {
@@ -74,7 +75,7 @@ __device__ __forceinline__ void lm_put_mended(unsigned char* to, int stride, con
     if (cm_odd(mine)) lm_mend(to, stride, make_float4(v[0], v[1], v[2], v[3]), make_float4(v[4], v[5], v[6], v[7]), row, first);
 }
 // Eight values of a token: parts behind their activation; without one they are only looked at.
-__device__ __forceinline__ void lm_values(const LAArgs& a, unsigned char* to, const bf16* from, bool there, int row, unsigned* first_odd, unsigned& most) {
+__device__ __forceinline__ void lm_values(const LAArgs& a, unsigned char* to, const bf16* from, bool there, int row, unsigned* first_odd, unsigned& most, unsigned& numbers) {
     unsigned mine = 0;
     if (a.act_v) {
         float v[8];
@@ -87,21 +88,105 @@ __device__ __forceinline__ void lm_values(const LAArgs& a, unsigned char* to, co
         const uint4 r = *reinterpret_cast<const uint4*>(from);
         cm_watch(mine, r.x); cm_watch(mine, r.y); cm_watch(mine, r.z); cm_watch(mine, r.w);
     }
-    if (cm_odd(mine, a.act_v ? CM_MOST : CM_MOST_PLAIN)) atomicMin(first_odd, (unsigned)row);
     cm_watch(most, mine);
+    if (!cm_odd(mine, a.act_v ? CM_MOST : CM_MOST_PLAIN)) return;
+    atomicMin(first_odd, (unsigned)row);
+    for (int i = 0; i < 8; ++i) {                          // (seldom: which of them are numbers)
+        const float v = la_act<true>(to_f(from[i]), a.act_v);
+        if (fabsf(v) >= 0x1p34f) numbers = CM_MOST;        // (2^34: what is rounded to 2^35 counts)
+    }
 }
 
-// A chunk's inputs, for what is worked out number by number.
-struct LMInputs {
-    const LAArgs& a; int first, n, pc;
-    __device__ __forceinline__ float decay(int t, int h, int d) const {
-        if (!pc) return a.head_decay[h];
-        const float u = -load_as_f(a.z, a.z_f32 ? PE_F32 : PE_BF16, (size_t)(first + t) * a.z_ld + h * a.D + d);
-        return expf(-(fmaxf(u, 0.f) + log1pf(expf(-fabsf(u)))) * a.inv_tau);
+// a = sigmoid(z)^(inv_tau), through the logarithm: -softplus(-z) * inv_tau (as the walk of linear_attention.cu has it)
+__device__ __forceinline__ float lm_decay(float z, float inv_tau) {
+    const float u = -z;
+    return expf(-(fmaxf(u, 0.f) + log1pf(expf(-fabsf(u)))) * inv_tau);
+}
+
+// [2][64 t][64] or [64 t][128] numbers of rows, all asked for before any is stored: dst in shared memory.
+template <typename T, int ND>
+__device__ __forceinline__ void lm_fill(float* dst, const T* src, int ld, int n) {
+    float v[2][8];
+#pragma unroll 1
+    for (int r = 0; r < 4; r += 2) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int i = ((r + e) * LM_THREADS + threadIdx.x) * 8;
+            lm_eight(v[e], src + (size_t)min(i / ND % 64, n - 1) * ld + i / (64 * ND) * ND + i % ND, true, ((uintptr_t)src | ld * sizeof(T)) % 16 == 0);
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            float* to = dst + ((r + e) * LM_THREADS + threadIdx.x) * 8;
+            *reinterpret_cast<float4*>(to) = make_float4(v[e][0], v[e][1], v[e][2], v[e][3]);
+            *reinterpret_cast<float4*>(to + 4) = make_float4(v[e][4], v[e][5], v[e][6], v[e][7]);
+        }
     }
-    __device__ __forceinline__ float qk(int off, int t, int h, int d) const { return la_act<true>(load_as_f(a.qk, a.qk_f32 ? PE_F32 : PE_BF16, (size_t)(first + t) * a.qk_ld + off + h * a.D + d), a.act_qk); }
-    __device__ __forceinline__ float v(int t, int col) const { return la_act<true>(__bfloat162float(((const bf16*)a.proj)[(size_t)(first + t) * a.ld + a.v_off + col]), a.act_v); }
-};
+}
+// What parts are not made of: a unit's chunk token after token with multiply-adds, from its incoming state (none: zeros), all threads of a block.  Outputs from
+// token `exact` on; the state behind the chunk to `to_state`, if that is asked for.  Queries, keys and decays are worked out once, into the block's shared memory
+// (which nobody else uses then).  A state with infinities or huge numbers sends every unit behind it here, a token that is no number those of its chunk.  2,048 tokens with one
+// value, one head's keys, all of a token, every token that is none, us:
+//   16 heads of 128, a decay a head     144 / 145 / 148 / 164 (96 without; multiply-add tiles 125; entry by entry from memory 4,115 to 8,013)
+//   a decay a channel                   155 / 152 / 155 / 171 (110; 180; 5,276 to 9,552)
+//   14 heads of 64                      82 / 83 / 84 / 91 (49; 53; 2,000) and 88 / 84 / 89 / 90 (53; 79; 2,600)
+// Most of it is one walk's latency, 50 us.
+template <bool TWO>
+__device__ __noinline__ void lm_walk(const LAArgs& a, int first, int n, int h0, const float* state, int exact, float* to_state) {
+    extern __shared__ unsigned char lm_raw[];
+    float* smem = reinterpret_cast<float*>(lm_raw + (-at_smem(lm_raw) & 1023u));
+    constexpr int ND = LMUnit<TWO>::ND;
+    using Walk = CMWalk<ND>;
+    const int tid = threadIdx.x, ld_out = a.H * a.Dv, ld = a.ld, act_qk = a.act_qk, act_v = a.act_v, hh = TWO ? Walk::column() >> 6 : 0;
+    float *qs = smem, *ks = smem + 64 * 128, *as = smem + 2 * 64 * 128;                     // [head][64 t][ND]
+    const bool writes = !(tid & 1);
+    float* out = a.out + (size_t)first * ld_out + h0 * a.Dv + Walk::written();
+    Walk walk;
+    if (__syncthreads_and(walk.begin(state))) {            // no state that is a number: no output is one
+        if (writes)
+            for (int t = exact; t < n; ++t) out[(size_t)t * ld_out] = __int_as_float(0x7fffffff);
+        return;
+    }
+    // The numbers as they are, then each through its activation.  (Loops of few instructions: what runs here has not run before and comes from L2.)
+    const bool pc = a.z != nullptr;
+    const float q_scale = a.q_scale, inv_tau = a.inv_tau;    // (loops that store read nothing of the arguments, which they would read again each time)
+    const size_t row = (size_t)first * a.qk_ld + h0 * ND;
+    if (a.qk_f32) {
+        lm_fill<float, ND>(ks, (const float*)a.qk + row + a.k_off, a.qk_ld, n);
+        lm_fill<float, ND>(qs, (const float*)a.qk + row + a.q_off, a.qk_ld, n);
+    } else {
+        lm_fill<bf16, ND>(ks, (const bf16*)a.qk + row + a.k_off, a.qk_ld, n);
+        lm_fill<bf16, ND>(qs, (const bf16*)a.qk + row + a.q_off, a.qk_ld, n);
+    }
+    if (pc && a.z_f32) lm_fill<float, ND>(as, (const float*)a.z + (size_t)first * a.z_ld + h0 * ND, a.z_ld, n);
+    if (pc && !a.z_f32) lm_fill<bf16, ND>(as, (const bf16*)a.z + (size_t)first * a.z_ld + h0 * ND, a.z_ld, n);
+    __syncthreads();
+#pragma unroll 1
+    for (int i = tid; i < 64 * 128; i += LM_THREADS) {
+        ks[i] = la_act<true>(ks[i], act_qk);
+        qs[i] = la_act<true>(qs[i], act_qk) * q_scale;
+        if (pc) as[i] = lm_decay(as[i], inv_tau);
+    }
+    const float fixed = pc ? 0.f : a.head_decay[h0 + hh];
+    const bf16* values = (const bf16*)a.proj + (size_t)first * a.ld + a.v_off + h0 * a.Dv + Walk::column();
+    auto ask = [&](int t) { return *reinterpret_cast<const uint2*>(values + (size_t)min(t, n - 1) * ld); };
+    uint2 next = ask(0), later = ask(1);
+    __syncthreads();
+#pragma unroll 1
+    for (int t = 0; t < n; ++t) {
+        const uint2 now = next;
+        next = later;
+        later = ask(t + 2);
+        const int at = (hh * 64 + t) * ND;
+        const float v[4] = {la_act<true>(__uint_as_float(now.x << 16), act_v), la_act<true>(__uint_as_float(now.x & 0xffff0000u), act_v),
+                            la_act<true>(__uint_as_float(now.y << 16), act_v), la_act<true>(__uint_as_float(now.y & 0xffff0000u), act_v)};
+        walk.step(ks + at, pc ? as + at : nullptr, fixed, v);
+        if (t < exact) continue;
+        const float o = walk.output(qs + at);
+        if (writes) out[(size_t)t * ld_out] = o;
+    }
+    if (to_state) walk.end(to_state);
+    __syncthreads();                                       // (the shared memory has been read)
+}
 // With one decay a head, a chunk and head: queries and keys through their activation, k_s a^(n-1-s), and weights q_t . k_s a^(t-s), from scores by mma.sync.
 template <typename TQ, bool TWO>
 __global__ void __launch_bounds__(512, 2) lm_prepare_kernel(LAArgs a, int vec_q) {
@@ -125,7 +210,7 @@ __global__ void __launch_bounds__(512, 2) lm_prepare_kernel(LAArgs a, int vec_q)
     const TQ* src = (const TQ*)a.qk + (size_t)(first + (there ? row : 0)) * a.qk_ld + h * D + 8 * group;
     CMScores acc;
     acc.clear();
-    unsigned most_w = 0, most_v = 0;
+    unsigned most_w = 0, most_v = 0, numbers = 0;
     __syncthreads();
     const float follow = there ? pw[n - 1 - row] : 0.f;
     for (int j = 0; j < D / 64; ++j) {
@@ -146,11 +231,11 @@ __global__ void __launch_bounds__(512, 2) lm_prepare_kernel(LAArgs a, int vec_q)
             *reinterpret_cast<uint4*>(unit + Unit::QUERIES + p * 2 * CM_PLANE + half + cm_at(row, group)) = *reinterpret_cast<const uint4*>(qs + p * CM_PLANE + cm_at(row, group));
 #pragma unroll
         for (int i = 0; i < 8; ++i) k[i] *= follow;
-        lm_put(unit + Unit::KEYS + half + cm_at(row, group), 2 * CM_PLANE, k, most[2]);
+        lm_put<true>(unit + Unit::KEYS + half + cm_at(row, group), 2 * CM_PLANE, k, most[2]);
         cm_report(&seen, cm_seen(most[0], 0) | cm_seen(most[1], 1) | cm_seen(most[2], 4));
         __syncthreads();
         if (s0 <= t0) acc.add(at_smem(qs), at_smem(ks), CM_PLANE, t0, s0);
-        lm_values(a, unit + Unit::VALUES + half + cm_at(row, group), (const bf16*)a.proj + (size_t)(first + row) * a.ld + a.v_off + h * a.Dv + 64 * j + 8 * group, there, row, &from, most_v);
+        lm_values(a, unit + Unit::VALUES + half + cm_at(row, group), (const bf16*)a.proj + (size_t)(first + row) * a.ld + a.v_off + h * a.Dv + 64 * j + 8 * group, there, row, &from, most_v, numbers);
     }
     __syncthreads();
     if (warp < 8) {                                        // (later keys have no weight)
@@ -169,7 +254,7 @@ __global__ void __launch_bounds__(512, 2) lm_prepare_kernel(LAArgs a, int vec_q)
                 *reinterpret_cast<unsigned*>(to + 2 * CM_PLANE) = lo;
             }
     }
-    cm_report(&seen, cm_seen(most_w, 2) | cm_seen(most_v, 3, a.act_v ? CM_MOST : CM_MOST_PLAIN));
+    cm_report(&seen, cm_seen(most_w, 2) | cm_seen(most_v, 3, a.act_v ? CM_MOST : CM_MOST_PLAIN) | cm_seen(numbers, 5));
     __syncthreads();
     if (seen >> 2 & 1u) {
         cm_mend(qs, CM_PLANE, CM_PARTS, &from);
@@ -191,11 +276,6 @@ __global__ void __launch_bounds__(512, 2) lm_prepare_kernel(LAArgs a, int vec_q)
 #define LMC_RUN 16
 __device__ __forceinline__ int lmc_row(int d) { return d * 68 + (d >> 3) * 4; }
 __host__ __device__ constexpr int lmc_floats(int D) { return D * 68 + D / 8 * 4; }
-// a = sigmoid(z)^(inv_tau), through the logarithm: -softplus(-z) * inv_tau (as the walk has it)
-__device__ __forceinline__ float lmc_decay(float z, float inv_tau) {
-    const float u = -z;
-    return expf(-(fmaxf(u, 0.f) + log1pf(expf(-fabsf(u)))) * inv_tau);
-}
 __device__ __forceinline__ void lmc_read16(float (&v)[LMC_RUN], const float* p) {
 #pragma unroll
     for (int t = 0; t < LMC_RUN; t += 4) *reinterpret_cast<float4*>(v + t) = *reinterpret_cast<const float4*>(p + t);
@@ -234,7 +314,7 @@ __global__ void __launch_bounds__(512, 2) lm_channels_kernel(LAArgs a, int vec_q
     const bool there = row < n;
     const size_t token = first + (there ? row : 0);
     unsigned char* unit = Unit::of(a, blockIdx.x, h);
-    unsigned most_q = 0, most_k = 0, most_w = 0, most_v = 0;
+    unsigned most_q = 0, most_k = 0, most_w = 0, most_v = 0, numbers = 0;
 #pragma unroll 1
     for (int j = 0; j < D / 64; ++j) {
         const int d = 64 * j + 8 * group;
@@ -242,13 +322,13 @@ __global__ void __launch_bounds__(512, 2) lm_channels_kernel(LAArgs a, int vec_q
         lm_eight(q, (const bf16*)a.qk + token * a.qk_ld + a.q_off + h * D + d, there, vec_q);
         lm_eight(k, (const bf16*)a.qk + token * a.qk_ld + a.k_off + h * D + d, there, vec_q);
         lm_eight(z, (const TZ*)a.z + token * a.z_ld + h * D + d, there, vec_z);
-        lm_values(a, unit + Unit::VALUES + (TWO ? h & 1 : j) * CM_PLANE + cm_at(row, group), (const bf16*)a.proj + token * a.ld + a.v_off + h * a.Dv + d, there, row, &from, most_v);
+        lm_values(a, unit + Unit::VALUES + (TWO ? h & 1 : j) * CM_PLANE + cm_at(row, group), (const bf16*)a.proj + token * a.ld + a.v_off + h * a.Dv + d, there, row, &from, most_v, numbers);
         float* to = qt + lmc_row(d) + row;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             to[i * 68] = la_act<true>(q[i], a.act_qk) * a.q_scale;
             to[i * 68 + lmc_floats(D)] = la_act<true>(k[i], a.act_qk);
-            to[i * 68 + 2 * lmc_floats(D)] = there ? lmc_decay(z[i], a.inv_tau) : 1.f;
+            to[i * 68 + 2 * lmc_floats(D)] = there ? lm_decay(z[i], a.inv_tau) : 1.f;
         }
     }
     __syncthreads();
@@ -357,11 +437,11 @@ __global__ void __launch_bounds__(512, 2) lm_channels_kernel(LAArgs a, int vec_q
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = p[i * 68 + lmc_floats(D)] * follow[run * D + d + i];
         cm_scale(v, CM_UP);
-        lm_put(unit + Unit::KEYS + place, 2 * CM_PLANE, v, most_k);
+        lm_put<true>(unit + Unit::KEYS + place, 2 * CM_PLANE, v, most_k);
     }
     cm_scale(weight, CM_UP);
     lm_put_mended(unit + Unit::WEIGHTS + (TWO ? h & 1 : 0) * CM_PLANE + cm_at(row, group), Unit::W_HEADS * CM_PLANE, weight, most_w, row, &from);
-    cm_report(&seen, cm_seen(most_q, 0) | cm_seen(most_k, 4) | cm_seen(most_w, 2) | cm_seen(most_v, 3, a.act_v ? CM_MOST : CM_MOST_PLAIN));
+    cm_report(&seen, cm_seen(most_q, 0) | cm_seen(most_k, 4) | cm_seen(most_w, 2) | cm_seen(most_v, 3, a.act_v ? CM_MOST : CM_MOST_PLAIN) | cm_seen(numbers, 5));
     __syncthreads();
     if (tid == 0) a.chunk_seen[(size_t)blockIdx.x * a.H + h] = seen | from << 16;
 }
@@ -386,7 +466,7 @@ __device__ __forceinline__ void lm_bring_values(unsigned char* dst, const LAArgs
 
 // Chunks of a unit's heads, contributions.  Nothing is cut here: the parts and values of the next unit come while this one's sums leave.
 template <bool TWO, int VALUE_PARTS>
-__global__ void __launch_bounds__(LM_THREADS, 2) lm_contribution_kernel(LAArgs a, int units) {
+__global__ void __launch_bounds__(LM_THREADS, TWO || VALUE_PARTS == 3 ? 3 : 2) lm_contribution_kernel(LAArgs a, int units) {
     extern __shared__ unsigned char lm_raw[];
     __shared__ __align__(8) unsigned long long bar;
     __shared__ unsigned tmem_s;
@@ -402,6 +482,7 @@ __global__ void __launch_bounds__(LM_THREADS, 2) lm_contribution_kernel(LAArgs a
     unsigned phase = 0;
     int2 place = a.chunk_rows[blockIdx.x / per];
     unsigned known = 0;
+    bool odd = false;
     auto bring = [&](int unit) {
         const int c = unit / per, h0 = unit % per * (TWO ? 2 : 1);
         cm_bring(ks, Unit::of(a, c, h0) + Unit::KEYS, 6 * CM_PLANE);
@@ -411,11 +492,12 @@ __global__ void __launch_bounds__(LM_THREADS, 2) lm_contribution_kernel(LAArgs a
     };
     if (place.y > 0) bring(blockIdx.x);
     for (int unit = blockIdx.x; unit < units && place.y > 0; unit += gridDim.x) {
-        const int h0 = unit % per * (TWO ? 2 : 1), next = unit + gridDim.x, first = place.x, n = place.y;
+        const int next = unit + gridDim.x;
         if (next < units) place = a.chunk_rows[next / per];
         cm_landed();
         cm_ready();
-        const bool parts = !(known & (1u << 3 | 1u << 4));            // (every thread has read the same words)
+        const bool parts = !(known & (1u << 4 | 1u << 5));            // (every thread has read the same words)
+        odd = odd || !parts;
         if (parts) {
             if (warp == 0) {
                 if constexpr (VALUE_PARTS == 1) cm_products_one(elected, tmem, tmem + 128, at_desc(at_smem(vs), CM_PLANE, 1024), 128u, cm_across(at_smem(ks), 2 * CM_PLANE, CM_PLANE), cm_idesc(128, true, true));
@@ -424,7 +506,7 @@ __global__ void __launch_bounds__(LM_THREADS, 2) lm_contribution_kernel(LAArgs a
                 __syncwarp();
             }
             cm_done(&bar, phase, a.status);
-        } else __syncthreads();
+        }
         if (next < units && place.y > 0) bring(next);
         float* state = a.chunk_state + (size_t)unit * 128 * ND;
         if (parts) {
@@ -441,18 +523,20 @@ __global__ void __launch_bounds__(LM_THREADS, 2) lm_contribution_kernel(LAArgs a
                 cm_store8(to, *reinterpret_cast<const float (*)[8]>(acc));
                 cm_store8(to + 512, *reinterpret_cast<const float (*)[8]>(acc + 8));
             }
-        } else {
-            const LMInputs in = {a, first, n, a.z != nullptr};
-#pragma unroll 1
-            for (int i = tid; i < 128 * ND; i += LM_THREADS) {
-                const int half = i / (64 * ND), d = i % (64 * ND) / 512 * 8 + i % 8, v = half * 64 + i / 8 % 64, h = TWO ? h0 + half : h0;
-                float sum = 0.f;
-                for (int t = 0; t < n; ++t) sum = fmaf(in.decay(t, h, d), sum, in.qk(a.k_off, t, h, d) * in.v(t, h0 * a.Dv + v));
-                state[i] = sum;
-            }
         }
     }
     cm_end(tmem);
+    if (!odd) return;                                      // (the walks behind the loop: inside they cost its registers)
+    __shared__ LAArgs args;
+    if (tid == 0) args = a;
+    __syncthreads();
+#pragma unroll 1
+    for (int unit = blockIdx.x; unit < units; unit += gridDim.x) {
+        const int c = unit / per, h0 = unit % per * (TWO ? 2 : 1);
+        const int2 at = a.chunk_rows[c];
+        if (at.y <= 0) break;
+        if (lm_known<TWO>(a, c, h0) & (1u << 4 | 1u << 5)) lm_walk<TWO>(args, at.x, at.y, h0, nullptr, at.y, a.chunk_state + (size_t)unit * 128 * ND);
+    }
 }
 
 // A block eight columns of a head's state, 2 D threads: a thread four rows of a column walks the sequence's chunks in order, leaves every chunk its
@@ -507,7 +591,7 @@ template <bool TWO, int VALUE_PARTS>
 __global__ void __launch_bounds__(LM_THREADS, 2) lm_output_kernel(LAArgs a, int units) {
     extern __shared__ unsigned char lm_raw[];
     __shared__ __align__(8) unsigned long long bar;
-    __shared__ unsigned tmem_s, odd_state, from_s;
+    __shared__ unsigned tmem_s, odd_state, from_s, odd;
     __shared__ __align__(16) float es[TWO ? 2 : 1][LA_CHUNK];
     using Unit = LMUnit<TWO>;
     constexpr int ND = Unit::ND, SLABS = TWO ? 1 : 2;
@@ -516,6 +600,7 @@ __global__ void __launch_bounds__(LM_THREADS, 2) lm_output_kernel(LAArgs a, int 
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), per = TWO ? a.H / 2 : a.H, ld_out = a.H * a.Dv;
     const int q = warp & 3, hh = q >> 1, p = (q & 1) * 32 + lane, column = (warp >> 2) * 32;
     const bool scaled = a.z == nullptr;                               // one decay a head: the decay to a token behind the products
+    if (tid == 0) odd = 0;
     const unsigned tmem = cm_begin(&tmem_s, &bar), mine = tmem + ((unsigned)(q * 32) << 16) + column + (TWO ? hh * 64 : 0);
     const unsigned elected = warp == 0 ? cm_elect() : 0u;
     pdl_wait();
@@ -551,7 +636,7 @@ __global__ void __launch_bounds__(LM_THREADS, 2) lm_output_kernel(LAArgs a, int 
             for (int e = 0; e < 4; ++e) {
                 float s[8] = {v[e][0].x, v[e][0].y, v[e][0].z, v[e][0].w, v[e][1].x, v[e][1].y, v[e][1].z, v[e][1].w};
                 cm_scale(s, CM_UP);
-                lm_put(ss + (e >> 1) * CM_PLANE + cm_at(tid & 63, (e & 1) * 4 + (tid >> 6)), 2 * CM_PLANE, s, most);
+                lm_put<true>(ss + (e >> 1) * CM_PLANE + cm_at(tid & 63, (e & 1) * 4 + (tid >> 6)), 2 * CM_PLANE, s, most);
             }
             if (slab == 0) cm_landed();
             cm_ready();
@@ -611,25 +696,24 @@ __global__ void __launch_bounds__(LM_THREADS, 2) lm_output_kernel(LAArgs a, int 
 #pragma unroll
             for (int i = 0; i < 32; ++i)
                 if (column + i < exact) out[i * ld_out] = acc[i];
-            if (exact < n && tid < 128) {                  // a column a thread: the walk over the chunk's tokens, row by row of the state
-                const int h = TWO ? h0 + (tid >> 6) : h0;
-                const LMInputs in = {a, first, n, a.z != nullptr};
-                const float* state = a.chunk_state + (size_t)unit * 128 * ND + (size_t)(tid >> 6) * ND * 64 + (tid & 63) * 8;
-                float* to = a.out + (size_t)first * ld_out + h0 * a.Dv + tid;
-                for (int t = exact; t < n; ++t) to[(size_t)t * ld_out] = 0.f;
-#pragma unroll 1
-                for (int d = 0; d < ND; ++d) {
-                    float s = state[(size_t)(d / 8) * 512 + d % 8];
-#pragma unroll 1
-                    for (int t = 0; t < n; ++t) {
-                        s = fmaf(in.decay(t, h, d), s, in.qk(a.k_off, t, h, d) * in.v(t, h0 * a.Dv + tid));
-                        if (t >= exact) to[(size_t)t * ld_out] = fmaf(s, in.qk(a.q_off, t, h, d) * a.q_scale, to[(size_t)t * ld_out]);
-                    }
-                }
-            }
+        }
+        if (tid == 0) {
+            a.unit_exact[unit] = exact;
+            if (exact < n) odd = 1;
         }
     }
     cm_end(tmem);
+    if (!odd) return;                                      // (the walks behind the loop: inside they cost its registers)
+    __shared__ LAArgs args;
+    if (tid == 0) args = a;
+    __syncthreads();
+#pragma unroll 1
+    for (int unit = blockIdx.x; unit < units; unit += gridDim.x) {
+        const int2 at = a.chunk_rows[unit / per];
+        if (at.y <= 0) break;
+        const int exact = a.unit_exact[unit];
+        if (exact < at.y) lm_walk<TWO>(args, at.x, at.y, unit % per * (TWO ? 2 : 1), a.chunk_state + (size_t)unit * 128 * ND, exact, nullptr);
+    }
 }
 
 template <bool TWO, int VP>
@@ -663,7 +747,7 @@ static int lm_run(LAArgs a, int types, int z_types, cudaStream_t s) {
 
 long long la_tensor_chunk_floats(int H, int D) {                      // a chunk's parts, words and place
     const long long parts = D == 128 ? (long long)H * LMUnit<false>::BYTES : (long long)H / 2 * LMUnit<true>::BYTES;
-    return parts / 4 + H + 2;
+    return parts / 4 + 2 * H + 2;
 }
 int la_tensor_chunks(const LAArgs& a, int types, int z_types, cudaStream_t s) {
     if (a.act_v) return a.D == 64 ? lm_run<true, 3>(a, types, z_types, s) : lm_run<false, 3>(a, types, z_types, s);

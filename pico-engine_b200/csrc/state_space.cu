@@ -192,7 +192,7 @@ extern "C" long long pe_state_space_elems(int H, int P, int N) {
 extern "C" int pe_state_space_chunks(int T, int B) { return (T + SS_CHUNK - 1) / SS_CHUNK + B; }
 static int ss_step_floats(int H, int P, int N, int G) { return ss_on_tensor_cores(H, P, N, G) ? SS_MATRIX_STEP_FLOATS : SS_STEP_FLOATS; }
 static long long ss_chunk_floats(int H, int P, int N, int G) {
-    const long long parts = ss_on_tensor_cores(H, P, N, G) ? (long long)G * (2 * ss_plane_bytes(N) / 4 + 1) : 0;
+    const long long parts = ss_on_tensor_cores(H, P, N, G) ? (long long)G * (2 * ss_plane_bytes(N) / 4 + 1) + H / 2 : 0;
     return (long long)G * SS_CHUNK * SS_CHUNK + (long long)H * (P * N + ss_step_floats(H, P, N, G) + 1) + 8 + parts;
 }
 static int ss_slab(int chunks, int H, int P, int N, int G) {
@@ -300,7 +300,7 @@ extern "C" int pe_state_space_scan(const float* xbc, int xbc_ld, const void* pro
     if (PT > P) PT = P;
     int threads = ((PT * NS + 31) / 32) * 32;
     ScanArgs a = {xbc, xbc_ld, proj, proj_ld, dt_off, dt_bias, dtb_dtype, a_log, al_dtype, d_skip, d_dtype, state, state_stride,
-                  row_first, row_lens, slots, y, B, H, P, N, G, NS, NR, NRP, PT, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, 0, 0};
+                  row_first, row_lens, slots, y, B, H, P, N, G, NS, NR, NRP, PT, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, 0, 0};
     if (dtype != PE_F32 && dtype != PE_BF16) return PE_ERR_UNSUPPORTED;
     if (chunked) {
         a.chunks = pe_state_space_chunks(T, B);
@@ -316,6 +316,7 @@ extern "C" int pe_state_space_scan(const float* xbc, int xbc_ld, const void* pro
             a.chunk_planes = reinterpret_cast<unsigned char*>(a.chunk_decay);                                     // (vectors first)
             a.chunk_decay = reinterpret_cast<float*>(a.chunk_planes + (size_t)a.slab * G * 2 * ss_plane_bytes(N));
             a.chunk_seen = reinterpret_cast<unsigned*>(a.chunk_decay + (size_t)a.slab * H);
+            a.unit_exact = reinterpret_cast<int*>(a.chunk_seen + (size_t)a.slab * G);
             return ss_tensor_tiles(a, dtype, status, (cudaStream_t)stream);
         }
         return ss_tiles(a, dtype, (cudaStream_t)stream);

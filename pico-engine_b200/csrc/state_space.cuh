@@ -24,7 +24,8 @@ struct ScanArgs {
     float* chunk_scores;                      // [chunks][G][64 s][64 t]: C_t . B_s
     float* chunk_steps;                       // [chunks][H][SS_STEP_FLOATS]: 64 x (dt, dt * the decays behind it), then 64 running sums (float64)
     unsigned char* chunk_planes;              // tensor cores: [chunks][G][B, C][64 state rows at a time]: their bfloat16 parts (chunk_mma.cuh)
-    unsigned* chunk_seen;                     // [chunks][G]: what cm_watch saw of them (tile 0: B, 1: C), and from bit 16 on the first token with an entry that parts do not hold (64: none)
+    unsigned* chunk_seen;                     // [chunks][G]: whether B has numbers that parts are not made of; from bit 16 on the first token where B or C has an entry that they are not made of (64: none)
+    int* unit_exact;                          // [chunks][H / 2]: tokens of a chunk and two heads whose results come from parts
     int2* chunk_rows;                         // [chunks]: first packed token and number of tokens
     int chunks;                               // of the step, at most
     int first_chunk, slab;                    // those that a launch takes: from first_chunk on, `slab` of them at most

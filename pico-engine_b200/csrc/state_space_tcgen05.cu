@@ -29,10 +29,11 @@
 #define SM_WS 0
 #define SM_ES 64
 #define SM_FACTOR 128
+#define SM_STEP 192                                       // and each token's own decay, for the walk
 #define SM_RUNS 256
 #define SM_INSIDE (256 + 8 * SS_CHUNK)
-#define SM_CONTRIBUTION_SMEM (4 * SM_SLAB + 1024)
-#define SM_OUTPUT_SMEM (4 * SM_SLAB + 1024)
+#define SM_CONTRIBUTION_SMEM (4 * SM_SLAB + 2048)         // (1,024 to begin on a boundary, 1,024 behind for the walk's decays and steps)
+#define SM_OUTPUT_SMEM (4 * SM_SLAB + 2048)
 
 __device__ __forceinline__ float4 sm_times(const float4& v, float w) {
     const float2 a = cm_scaled(v.x, v.y, w), b = cm_scaled(v.z, v.w, w);
@@ -87,14 +88,15 @@ __global__ void __launch_bounds__(SM_THREADS) sm_steps_kernel(ScanArgs a, int ve
             for (int e = 0; e < 2; ++e) chunk.eight(v[e][0], v[e][1], e ? chunk.c : chunk.b, row, k0 + 8 * group);
             __syncthreads();
 #pragma unroll
-            for (int e = 0; e < 2; ++e) cm_put(sm_mem + e * SM_SLAB + cm_at(row, group), CM_PLANE, sm_times(v[e][0], CM_UP), sm_times(v[e][1], CM_UP), most[e]);
-            cm_report(&seen, cm_seen(most[0], 0) | cm_seen(most[1], 1));
-            __syncthreads();
-            if (seen) {
-                cm_mend(sm_mem, CM_PLANE, CM_PARTS, &from);
-                cm_mend(sm_mem + SM_SLAB, CM_PLANE, CM_PARTS, &from);
-                __syncthreads();
+            for (int e = 0; e < 2; ++e) {
+                cm_put(sm_mem + e * SM_SLAB + cm_at(row, group), CM_PLANE, sm_times(v[e][0], CM_UP), sm_times(v[e][1], CM_UP), most[e]);
+                if (!cm_odd(most[e])) continue;
+                atomicMin(&from, (unsigned)row);
+                const float w[8] = {v[e][0].x, v[e][0].y, v[e][0].z, v[e][0].w, v[e][1].x, v[e][1].y, v[e][1].z, v[e][1].w};
+                for (int i = 0; i < 8; ++i)
+                    if (e == 0 && fabsf(w[i]) >= 0x1p34f) atomicOr(&seen, 1u);          // (2^34: what is rounded to 2^35 counts)
             }
+            __syncthreads();
             unsigned char* to = planes + (size_t)(k0 / 64) * SM_SLAB;
             for (int i = tid * 16; i < SM_SLAB; i += SM_THREADS * 16) {
                 *reinterpret_cast<uint4*>(to + i) = *reinterpret_cast<const uint4*>(sm_mem + i);
@@ -105,13 +107,22 @@ __global__ void __launch_bounds__(SM_THREADS) sm_steps_kernel(ScanArgs a, int ve
         if (tid == 0) a.chunk_seen[(size_t)blockIdx.x * a.G + g] = seen | from << 16;
         float* dst = a.chunk_scores + ((size_t)blockIdx.x * a.G + g) * SS_CHUNK * SS_CHUNK;
         const int exact = from;                            // tokens in front of it have their scores from the parts
+        if (exact < n) {                                   // the others with multiply-adds, B's rows in shared memory, 68 or 132 numbers apart
+            float* rows = reinterpret_cast<float*>(sm_mem);
+            __syncthreads();
 #pragma unroll 1
-        for (int i = exact * SS_CHUNK + tid; i < n * SS_CHUNK; i += SM_THREADS) {
-            const int t = i / SS_CHUNK, s = i % SS_CHUNK;
-            if (s > t) continue;
-            float v = 0.f;
-            for (int k = 0; k < N; ++k) v = fmaf(chunk.b[(size_t)s * chunk.ld + k], chunk.c[(size_t)t * chunk.ld + k], v);
-            dst[i] = v;
+            for (int i = tid; i < n * N; i += SM_THREADS) rows[i / N * (N + 4) + i % N] = chunk.b[(size_t)(i / N) * chunk.ld + i % N];
+            __syncthreads();
+#pragma unroll 1
+            for (int i = exact * SS_CHUNK + tid; i < n * SS_CHUNK; i += SM_THREADS) {
+                const int t = i / SS_CHUNK, s = i % SS_CHUNK;
+                if (s > t) continue;
+                const float *b = rows + s * (N + 4), *c = chunk.c + (size_t)t * chunk.ld;
+                float v = 0.f;
+#pragma unroll 4
+                for (int k = 0; k < N; ++k) v = fmaf(b[k], c[k], v);
+                dst[i] = v;
+            }
         }
         if (s0 > t0) return;                               // (nobody reads the weights of later keys)
 #pragma unroll
@@ -144,6 +155,7 @@ __global__ void __launch_bounds__(SM_THREADS) sm_steps_kernel(ScanArgs a, int ve
     float* dst = a.chunk_steps + ((size_t)blockIdx.x * a.H + h) * SS_MATRIX_STEP_FLOATS;
     dst[SM_WS + t] = dt * expf((float)(end - la));
     dst[SM_ES + t] = expf((float)la);
+    dst[SM_STEP + t] = expf((float)(la - (t ? las[hh][t - 1] : 0.0)));
     dst[SM_FACTOR + t] = dt * expf((float)(las[hh][t | 7] - la));
     float runs[8], inside[8];
 #pragma unroll
@@ -157,16 +169,72 @@ __global__ void __launch_bounds__(SM_THREADS) sm_steps_kernel(ScanArgs a, int ve
     if (t == 0) a.chunk_decay[(size_t)blockIdx.x * a.H + h] = (float)exp(end);      // (a state hands its errors on from chunk to chunk)
 }
 
+// What parts are not made of: two heads' chunk token after token with multiply-adds, from its incoming state (none: zeros), all threads of a block.  Outputs from token
+// `exact` on; the state behind the chunk to `to_state`, if that is asked for.  B, C and x lie in the block's shared memory (which nobody else uses then).  A state with
+// infinities or huge numbers sends every unit behind it here, a token that is no number those of its chunk.  64 heads, 128 state rows, rows of 1,400 and 647 tokens with one
+// number of x, one of B, all of a token, every token that is none: 178 / 203 / 203 / 262 us (139 without; multiply-add tiles 191; entry by entry from memory 640 to 1,637).
+template <int N>
+__device__ __noinline__ void sm_walk(const ScanArgs& a, int c, int first, int n, int h0, int g, const float* state, int exact, float* to_state) {
+    extern __shared__ unsigned char sm_raw[];
+    float* smem = reinterpret_cast<float*>(sm_raw + (-at_smem(sm_raw) & 1023u));
+    using Walk = CMWalk<N>;
+    const SMChunk chunk(a, first, n, h0, g, 0);
+    const int tid = threadIdx.x, h = h0 + (Walk::column() >> 6), ld = chunk.ld, ld_y = a.H * 64;       // (loops that store read nothing of the arguments, which they would read again each time)
+    float *bs = smem, *cs = smem + SS_CHUNK * N, *xs = cs + SS_CHUNK * N, *turns = xs + SS_CHUNK * 128;      // [64 t][N]; [64 t][128]; [head][64 t]: decays, then steps
+    const bool writes = !(tid & 1);
+    float* y = a.y + (size_t)first * ld_y + h0 * 64 + Walk::written();
+    Walk walk;
+    if (__syncthreads_and(walk.begin(state))) {            // no state that is a number: no output is one
+        if (writes)
+            for (int t = exact; t < n; ++t) y[(size_t)t * ld_y] = __int_as_float(0x7fffffff);
+        return;
+    }
+    const auto fill = [&](float* dst, const float* src, int width) {       // eight reads in front of their stores
+#pragma unroll 1
+        for (int i = tid; i < SS_CHUNK * width; i += 8 * SM_FEW) {
+            float v[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = src[(size_t)min((i + e * SM_FEW) / width, n - 1) * ld + (i + e * SM_FEW) % width];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) dst[i + e * SM_FEW] = v[e];
+        }
+    };
+    fill(bs, chunk.b, N);
+    fill(cs, chunk.c, N);
+    fill(xs, chunk.x, 128);
+    if (tid < 2 * SS_CHUNK) {
+        const float* steps = a.chunk_steps + ((size_t)c * a.H + h0 + (tid >> 6)) * SS_MATRIX_STEP_FLOATS;
+        const int t = tid & 63;
+        turns[tid] = steps[SM_STEP + t];
+        turns[2 * SS_CHUNK + tid] = steps[SM_INSIDE + 8 * t + (t & 7)];       // (a token's weight for itself: dt)
+    }
+    const float skip = load_as_f(a.d_skip, a.d_dtype, h);
+    const float* turn = turns + (Walk::column() >> 6) * SS_CHUNK;
+    __syncthreads();
+#pragma unroll 1                                           // (few instructions: what runs here has not run before, and comes from L2 a line at a time)
+    for (int t = 0; t < n; ++t) {
+        const float4 x = *reinterpret_cast<const float4*>(xs + t * 128 + Walk::column());
+        const float dt = turn[2 * SS_CHUNK + t], u[4] = {x.x * dt, x.y * dt, x.z * dt, x.w * dt};
+        walk.step(bs + t * N, nullptr, turn[t], u);
+        if (t < exact) continue;
+        const float o = walk.output(cs + t * N);
+        if (writes) y[(size_t)t * ld_y] = fmaf(skip, xs[t * 128 + Walk::written()], o);
+    }
+    if (to_state) walk.end(to_state);
+    __syncthreads();                                       // (the shared memory has been read)
+}
+
 // Chunks and two heads at a time, contributions: the next unit's x is asked for while this one's products run.
 __global__ void __launch_bounds__(SM_FEW, 2) sm_contribution_kernel(ScanArgs a, int vec, int units, int* status) {
     extern __shared__ unsigned char sm_raw[];
     __shared__ __align__(8) unsigned long long bar;
-    __shared__ unsigned tmem_s, seen;
+    __shared__ unsigned tmem_s, seen, odd;
     __shared__ float ws[2][SS_CHUNK];
     unsigned char* xs = sm_raw + (-at_smem(sm_raw) & 1023u);          // [part][head][64 s][64 p]
     unsigned char* bs = xs + 2 * SM_SLAB;                             // [slab][part][64 s][64 n]
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), H = a.H, N = a.N, pairs = H / 2, slabs = N / 64;
     const int q = warp & 3, hh = q >> 1, p = (q & 1) * 32 + lane, row = tid >> 3, group = tid & 7;      // a thread's runs of eight: this row and the one 32 behind, of either head
+    if (tid == 0) odd = 0;
     const unsigned tmem = cm_begin(&tmem_s, &bar);
     const unsigned elected = warp == 0 ? cm_elect() : 0u;
     pdl_wait();
@@ -185,7 +253,6 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_contribution_kernel(ScanArgs a, 
     if (place.y > 0) fetch(blockIdx.x, place);
     for (int unit = blockIdx.x; unit < units && place.y > 0; unit += gridDim.x) {
         const int c = unit / pairs, h0 = unit % pairs * 2, g = h0 / (H / a.G), n = place.y;
-        const SMChunk chunk(a, place.x, n, h0, g, vec);
         cm_bring(bs, a.chunk_planes + ((size_t)c * a.G + g) * 2 * ss_plane_bytes(N), slabs * SM_SLAB);
         const int next = unit + gridDim.x;
         if (next < units) place = a.chunk_rows[next / pairs];
@@ -196,7 +263,7 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_contribution_kernel(ScanArgs a, 
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const float by = ws[e >> 1][row + (e & 1) * 32];          // (times x before the power of two: either product alone stays in range)
-            cm_put(xs + (e >> 1) * CM_PLANE + cm_at(row + (e & 1) * 32, group), 2 * CM_PLANE, sm_times(sm_times(v[e][0], by), CM_UP), sm_times(sm_times(v[e][1], by), CM_UP), most);
+            cm_put<true>(xs + (e >> 1) * CM_PLANE + cm_at(row + (e & 1) * 32, group), 2 * CM_PLANE, sm_times(sm_times(v[e][0], by), CM_UP), sm_times(sm_times(v[e][1], by), CM_UP), most);
         }
         cm_report(&seen, cm_seen(most, 2));
         cm_landed();
@@ -208,6 +275,10 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_contribution_kernel(ScanArgs a, 
             __syncwarp();
         }
         if (next < units && place.y > 0) fetch(next, place);
+        if (tid == 0) {
+            a.unit_exact[unit] = parts ? n : 0;
+            if (!parts) odd = 1;
+        }
         float* state = a.chunk_state + ((size_t)c * H + h0) * N * 64;
         if (parts) {
             cm_done(&bar, phase, status);
@@ -222,18 +293,24 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_contribution_kernel(ScanArgs a, 
                 cm_store8(to, *reinterpret_cast<const float (*)[8]>(acc));
                 cm_store8(to + 512, *reinterpret_cast<const float (*)[8]>(acc + 8));
             }
-        } else {
-#pragma unroll 1
-            for (int i = tid; i < 2 * 64 * N; i += SM_FEW) {
-                const int k = i / (64 * N), r = i % (64 * N) / 512 * 8 + i % 8, col = i / 8 % 64;
-                float sum = 0.f;
-                for (int s = 0; s < n; ++s) sum = fmaf(chunk.b[(size_t)s * chunk.ld + r], chunk.x[(size_t)s * chunk.ld + k * 64 + col] * ws[k][s], sum);
-                state[i] = sum;
-            }
-            __syncthreads();                               // (the weights have been read)
         }
     }
     cm_end(tmem);
+    if (!odd) return;                                      // (the walks behind the loop: inside they cost its registers)
+    __shared__ ScanArgs args;
+    if (tid == 0) args = a;
+    __syncthreads();
+#pragma unroll 1
+    for (int unit = blockIdx.x; unit < units; unit += gridDim.x) {
+        const int c = unit / pairs, h0 = unit % pairs * 2, g = h0 / (H / a.G);
+        const int2 at = a.chunk_rows[c];
+        if (at.y <= 0) break;
+        const int exact = a.unit_exact[unit];
+        float* state = a.chunk_state + ((size_t)c * H + h0) * N * 64;
+        if (exact >= at.y) continue;
+        if (N == 64) sm_walk<64>(args, c, at.x, at.y, h0, g, nullptr, at.y, state);
+        else sm_walk<128>(args, c, at.x, at.y, h0, g, nullptr, at.y, state);
+    }
 }
 
 // A block eight columns of a head's state, 2 N threads: a thread four entries (rows r .. r + 3 of a column) walks the sequence's chunks in order, leaves
@@ -302,7 +379,7 @@ __global__ void __launch_bounds__(256) sm_carry_kernel(ScanArgs a) {
 __global__ void __launch_bounds__(SM_FEW, 2) sm_output_kernel(ScanArgs a, int vec, int units, int* status) {
     extern __shared__ unsigned char sm_raw[];
     __shared__ __align__(8) unsigned long long bar;
-    __shared__ unsigned tmem_s, seen, from;
+    __shared__ unsigned tmem_s, seen, from, odd;
     __shared__ __align__(16) float es[2][SS_CHUNK];
     unsigned char* mem = sm_raw + (-at_smem(sm_raw) & 1023u);
     unsigned char* ss = mem;                                          // [part][head][64 p][64 n] of the state
@@ -311,6 +388,7 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_output_kernel(ScanArgs a, int ve
     unsigned char* wgt = mem + 2 * SM_SLAB;                           // [part][head][64 t][64 s]
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), H = a.H, N = a.N, inner = H * 64, pairs = H / 2, slabs = N / 64;
     const int q = warp & 3, hh = q >> 1, p = (q & 1) * 32 + lane, column = (warp >> 2) * 32, row = tid >> 3, group = tid & 7;
+    if (tid == 0) odd = 0;
     const unsigned tmem = cm_begin(&tmem_s, &bar), mine = tmem + ((unsigned)(q * 32) << 16) + column;
     const unsigned elected = warp == 0 ? cm_elect() : 0u;
     pdl_wait();
@@ -336,13 +414,13 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_output_kernel(ScanArgs a, int ve
         const int next = unit + gridDim.x;
         if (next < units) place = a.chunk_rows[next / pairs];
         if (tid < 2 * SS_CHUNK) es[tid >> 6][tid & 63] = step;
-        if (tid == 0) { seen = known & 0xffffu; from = known >> 16; }
+        if (tid == 0) { seen = 0; from = known >> 16; }
         const float* scores = a.chunk_scores + ((size_t)c * a.G + g) * SS_CHUNK * SS_CHUNK;
         unsigned most_s = 0, most_x = 0, most_w = 0;
         const float skips[2] = {load_as_f(a.d_skip, a.d_dtype, h0), load_as_f(a.d_skip, a.d_dtype, h0 + 1)}, skip = skips[hh];
         for (int slab = 0; slab < slabs; ++slab) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) cm_put(ss + (e >> 1) * CM_PLANE + cm_at(tid & 63, (e & 1) * 4 + (tid >> 6)), 2 * CM_PLANE, sm_times(v[e][0], CM_UP), sm_times(v[e][1], CM_UP), most_s);
+            for (int e = 0; e < 4; ++e) cm_put<true>(ss + (e >> 1) * CM_PLANE + cm_at(tid & 63, (e & 1) * 4 + (tid >> 6)), 2 * CM_PLANE, sm_times(v[e][0], CM_UP), sm_times(v[e][1], CM_UP), most_s);
             if (slab == 0) cm_landed();
             cm_ready();
             if (warp == 0) {
@@ -402,7 +480,7 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_output_kernel(ScanArgs a, int ve
         }
         cm_report(&seen, cm_seen(most_s, 2) | cm_seen(most_x, 3) | cm_seen(most_w, 4));
         cm_ready();
-        if (seen) {
+        if (seen & 0x18u) {
 #pragma unroll 1
             for (int k = 0; k < 2; ++k) {
                 cm_mend(xs + k * CM_PLANE, 2 * CM_PLANE, CM_PARTS, &from);
@@ -438,27 +516,28 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_output_kernel(ScanArgs a, int ve
 #pragma unroll
             for (int i = 0; i < 32; ++i)
                 if (column + i < exact) y[i * inner] = acc[i];
-            if (exact < n) {
-                const float* state = a.chunk_state + ((size_t)c * H + h0) * N * 64;
-#pragma unroll 1
-                for (int i = exact * 128 + tid; i < n * 128; i += SM_FEW) {
-                    const int t = i / 128, k = i / 64 % 2, col = i % 64;
-                    const float* xc = chunk.x + k * 64 + col;
-                    float sum = 0.f;
-                    for (int r = 0; r < N; ++r) sum = fmaf(chunk.c[(size_t)t * chunk.ld + r], state[(size_t)k * N * 64 + (size_t)(r / 8 * 64 + col) * 8 + r % 8], sum);
-                    sum *= es[k][t];
-                    const float* steps = a.chunk_steps + ((size_t)c * H + h0 + k) * SS_MATRIX_STEP_FLOATS;
-                    for (int s = 0; s <= t; ++s) {         // (a token joins the sums of none in front of it)
-                        const float by = s >> 3 < t >> 3 ? steps[SM_FACTOR + s] * steps[SM_RUNS + 8 * t + (s >> 3)] : steps[SM_INSIDE + 8 * t + s % 8];
-                        sum = fmaf(scores[t * SS_CHUNK + s] * by, xc[(size_t)s * chunk.ld], sum);
-                    }
-                    a.y[(size_t)(first + t) * inner + (h0 + k) * 64 + col] = fmaf(load_as_f(a.d_skip, a.d_dtype, h0 + k), xc[(size_t)t * chunk.ld], sum);
-                }
-            }
-            __syncthreads();                               // (the steps have been read)
+        }
+        if (tid == 0) {
+            a.unit_exact[unit] = exact;
+            if (exact < n) odd = 1;
         }
     }
     cm_end(tmem);
+    if (!odd) return;                                      // (the walks behind the loop: inside they cost its registers)
+    __shared__ ScanArgs args;
+    if (tid == 0) args = a;
+    __syncthreads();
+#pragma unroll 1
+    for (int unit = blockIdx.x; unit < units; unit += gridDim.x) {
+        const int c = unit / pairs, h0 = unit % pairs * 2, g = h0 / (H / a.G);
+        const int2 at = a.chunk_rows[c];
+        if (at.y <= 0) break;
+        const int exact = a.unit_exact[unit];
+        float* state = a.chunk_state + ((size_t)c * H + h0) * N * 64;
+        if (exact >= at.y) continue;
+        if (N == 64) sm_walk<64>(args, c, at.x, at.y, h0, g, state, exact, nullptr);
+        else sm_walk<128>(args, c, at.x, at.y, h0, g, state, exact, nullptr);
+    }
 }
 
 template <typename T>

@@ -168,7 +168,7 @@ def test_scratch_of_the_tensor_cores_is_aligned_for_what_reads_it(D, per_channel
             slab = -(-chunks // lib.pe_linear_attention_slabs(*sizes))
             assert rows % 16 == 0 and seen % 4 == 0 and state % 32 == 0 and decay % 16 == 0, (H, chunks)
             planes = (12 + 3 * (1 if D == 128 else 2) + 6) * 8192 * (H if D == 128 else H // 2)
-            assert rows >= slab * planes and seen - rows >= 8 * slab and state - seen >= 4 * slab * H and decay - state >= 4 * slab * H * D * D
+            assert rows >= slab * planes and seen - rows >= 8 * slab and state - seen >= 8 * slab * H and decay - state >= 4 * slab * H * D * D
             assert end - decay >= 4 * slab * H * D and end <= 4 * lib.pe_linear_attention_scratch_floats(*sizes), (H, chunks)
 
 

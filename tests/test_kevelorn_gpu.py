@@ -731,3 +731,56 @@ def test_a_token_that_is_no_number_stays_where_it_is_on_the_tensor_cores(H, D, p
             (o, s), (o_walk, s_walk) = run(bad, True, v_activation=act), run(bad, False, v_activation=act)
             assert torch.equal(o[:at], clean[:at]) and torch.equal(o[lens[0]:], clean[lens[0]:]), (at, act)
             assert torch.equal(o.isfinite(), o_walk.isfinite()) and torch.equal(s.isfinite(), s_walk.isfinite()), (at, act)
+
+
+@pytest.mark.parametrize("H,D", [(3, 128), (4, 64)])
+@pytest.mark.parametrize("which", ["v", "k", "z", "many"])
+def test_what_a_token_that_is_no_number_does_not_reach_is_still_worked_out(H, D, which):
+    """Behind such a token a unit's chunk is walked: the columns and sequences that it does not reach have their numbers, decay logits that are none
+    are lost where the walk loses them, and more units than blocks of them come out right."""
+    from pico_engine.ops import kernels
+    lens = [130, 40] + ([64] * 150 if which == "many" else [])
+    for per_channel in (True, False) if which != "z" else (True,):
+        proj, run = tensor_core_rows(H, D, lens, per_channel, 9)
+        if which == "z":
+            T, g = sum(lens), torch.Generator("cuda").manual_seed(4)
+            logits = (2 + 2 * torch.randn(T, H * D, generator=g, device="cuda")).bfloat16()
+            logits[70, 5: H * D: 3] = float("nan")
+            first, rows, slots = (torch.tensor(v, dtype=torch.int32).cuda() for v in (np.concatenate([[0], np.cumsum(lens)]), lens, range(len(lens))))
+
+            def run(rows_in, chunked):
+                state = torch.full((len(lens), H * D * D), 0.5, device="cuda")
+                return kernels.linear_attention(rows_in, 0, H * D, 2 * H * D, H, D, D, state, 0, first, rows, slots, chunked, inv_tau=1 / 16, q_scale=D ** -0.5,
+                                                decay_logits=logits), state
+        elif which == "many":
+            proj[5::64, 2 * H * D: 3 * H * D: 7] = float("nan")
+        else:
+            column = "qkv".index(which) * H * D
+            proj[70, column + 3: column + D: 5] = float("inf") if which == "k" else float("nan")
+        for walk, chunks in zip(run(proj, False), run(proj, True)):
+            there = walk.isfinite()
+            assert torch.equal(there, chunks.isfinite()) and there.any() and not there.all()
+            # float32 sums of the same products in another order (the bound of the tests above)
+            assert (walk - chunks)[there].abs().max() < 2e-5 * max(1.0, float(walk[there].abs().max()))
+
+
+@pytest.mark.parametrize("per_channel", [False, True])
+def test_a_sequence_that_is_no_number_does_not_hold_up_the_others(per_channel):
+    """A batch's step with one such sequence takes about as long as without it: 1.1 to 2 times where a walk from memory took 20 to 80."""
+    lens = [1024] * 4
+    proj, run = tensor_core_rows(16, 128, lens, per_channel, 2)
+    bad = proj.clone()
+    bad[5] = float("nan")
+
+    def time(rows):
+        run(rows, True)
+        best = float("inf")
+        for _ in range(5):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            run(rows, True)
+            e1.record()
+            e1.synchronize()
+            best = min(best, e0.elapsed_time(e1))
+        return best
+    assert time(bad) < 4 * time(proj)

@@ -853,3 +853,24 @@ def test_low_rank_rows_in_runs_of_eight(T, H, D, R, rank, rot, rows, absorbed):
         got.append((q.float(), pool.float()))
     for a, b in zip(*got):                                     # the same arithmetic in the same order
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("which", ["x", "B"])
+def test_a_sequence_that_is_no_number_does_not_hold_up_the_others(which):
+    """A batch's step with one such sequence takes about as long as without it: 1.3 to 1.5 times where a walk from memory took 5 to 9."""
+    xbc, run = tensor_core_case(64, 128, 2, [1400, 647], 2)
+    bad = xbc.clone()
+    bad[5, 3 if which == "x" else 64 * 64 + 3] = float("nan")
+
+    def time(rows):
+        run(rows, True)
+        best = float("inf")
+        for _ in range(5):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            run(rows, True)
+            e1.record()
+            e1.synchronize()
+            best = min(best, e0.elapsed_time(e1))
+        return best
+    assert time(bad) < 3 * time(xbc)
