@@ -242,25 +242,29 @@ static int la_by_rows(const LAArgs& a, int chunked, cudaStream_t s) {
 extern "C" int pe_linear_attention_chunks(int T, int B) { return (T + LA_CHUNK - 1) / LA_CHUNK + B; }
 
 // Chunks that are worked on at a time: as many as LA_SCRATCH_FLOATS of scratch hold (one at least), in slabs of equal size.  A slab of the
-// sizes that fill it keeps the GPU full (16 heads of 128 x 128 with a decay per channel: 109 chunks, 1,744 blocks a launch), and batches of
-// prompts need no more scratch than it.
+// sizes that fill it keeps the GPU full (16 heads of 128 x 128: 254 chunks with a decay per head, 113 with one per channel as multiply-adds; 88 on the tensor
+// cores, 1,408 units a launch, 70 where values go through an activation), and batches of prompts need no more scratch than it.
 #define LA_SCRATCH_FLOATS (64ll << 20)
 // Sizes, and then rows, whose prompts run on the tensor cores (linear_attention_tcgen05.cu): every chunked step of theirs, down to a chunk of one token.
 static bool la_tensor_sizes(int H, int D, int Dv) { return D == Dv && (D == 128 || (D == 64 && H % 2 == 0)) && H <= 65535; }
 extern "C" int pe_linear_attention_on_tensor_cores(const void* proj, int dtype, int ld, int v_off, int H, int D, int Dv) {
     return la_tensor_sizes(H, D, Dv) && dtype == PE_BF16 && ld % 8 == 0 && v_off % 8 == 0 && (uintptr_t)proj % 16 == 0;
 }
-// Floats of scratch that a chunk takes, whichever way its step goes.
-static long long la_chunk_floats(int H, int D, int Dv, int per_channel) {
-    const long long adds = per_channel ? la_channels_scratch_floats(1, H, D) : 0, parts = la_tensor_sizes(H, D, Dv) ? la_tensor_chunk_floats(H, D) : 0;
-    return (long long)H * D * ((long long)Dv + 1) + (adds > parts ? adds : parts);
+// How a step goes, for the functions below: LA_CHANNELS a decay per channel, LA_TENSOR on the tensor cores, LA_VALUES values through an activation.
+#define LA_CHANNELS 1
+#define LA_TENSOR 2
+#define LA_VALUES 4
+// Floats of scratch that a chunk takes.
+static long long la_chunk_floats(int H, int D, int Dv, int kind) {
+    const long long more = kind & LA_TENSOR ? la_tensor_chunk_floats(H, D, kind & LA_VALUES) : kind & LA_CHANNELS ? la_channels_scratch_floats(1, H, D) : 0;
+    return (long long)H * D * ((long long)Dv + 1) + more;
 }
 // Where a slab's arrays lie in scratch on the tensor cores, in bytes: the widest accesses first.  Parts are read in 16 bytes, places as int2, words as they
 // are, states in runs of 32 bytes, decays as float4 (four floats of a head, whose D is 64 or 128).
 struct LATensorScratch {
     long long rows, seen, exact, state, decay, end;
-    LATensorScratch(int slab, int H, int D, int Dv) {
-        rows = 4 * (long long)slab * (la_tensor_chunk_floats(H, D) - 2 * H - 2);
+    LATensorScratch(int slab, int H, int D, int Dv, bool values) {
+        rows = 4 * (long long)slab * (la_tensor_chunk_floats(H, D, values) - 2 * H - 2);
         seen = rows + 8ll * slab;
         exact = seen + 4ll * slab * H;
         state = (exact + 4ll * slab * H + 31) / 32 * 32;
@@ -269,24 +273,24 @@ struct LATensorScratch {
     }
     bool aligned() const { return rows % 16 == 0 && seen % 4 == 0 && state % 32 == 0 && decay % 16 == 0; }
 };
-static int la_slab(int chunks, int H, int D, int Dv, int per_channel) {
-    const long long floats = la_chunk_floats(H, D, Dv, per_channel);
+static int la_slab(int chunks, int H, int D, int Dv, int kind) {
+    const long long floats = la_chunk_floats(H, D, Dv, kind);
     const long long most = floats >= LA_SCRATCH_FLOATS ? 1 : LA_SCRATCH_FLOATS / floats, slabs = (chunks + most - 1) / most;
     return (int)((chunks + slabs - 1) / slabs);
 }
-extern "C" int pe_linear_attention_slabs(int T, int B, int H, int D, int Dv, int per_channel) {
-    const int chunks = pe_linear_attention_chunks(T, B), slab = la_slab(chunks, H, D, Dv, per_channel);
+extern "C" int pe_linear_attention_slabs(int T, int B, int H, int D, int Dv, int kind) {
+    const int chunks = pe_linear_attention_chunks(T, B), slab = la_slab(chunks, H, D, Dv, kind);
     return (chunks + slab - 1) / slab;
 }
 // Floats of scratch the chunked way needs.
-extern "C" long long pe_linear_attention_scratch_floats(int T, int B, int H, int D, int Dv, int per_channel) {
-    return la_slab(pe_linear_attention_chunks(T, B), H, D, Dv, per_channel) * la_chunk_floats(H, D, Dv, per_channel) + 8;
+extern "C" long long pe_linear_attention_scratch_floats(int T, int B, int H, int D, int Dv, int kind) {
+    return la_slab(pe_linear_attention_chunks(T, B), H, D, Dv, kind) * la_chunk_floats(H, D, Dv, kind) + 8;
 }
 
 // The same places, for whoever checks them without a GPU (places: those of the struct, in its order); 0 where a call of these sizes has none.
-extern "C" int pe_linear_attention_scratch_places(int T, int B, int H, int D, int Dv, int per_channel, long long* places) {
-    if (!la_tensor_sizes(H, D, Dv)) return 0;
-    const LATensorScratch at(la_slab(pe_linear_attention_chunks(T, B), H, D, Dv, per_channel), H, D, Dv);
+extern "C" int pe_linear_attention_scratch_places(int T, int B, int H, int D, int Dv, int kind, long long* places) {
+    if (!(kind & LA_TENSOR) || !la_tensor_sizes(H, D, Dv)) return 0;
+    const LATensorScratch at(la_slab(pe_linear_attention_chunks(T, B), H, D, Dv, kind), H, D, Dv, kind & LA_VALUES);
     places[0] = at.rows; places[1] = at.seen; places[2] = at.state; places[3] = at.decay; places[4] = at.end;
     return 1;
 }
@@ -309,13 +313,14 @@ extern "C" int pe_linear_attention(const void* proj, int dtype, int ld, int q_of
     const bool pc = z != nullptr;
     a.chunks = pe_linear_attention_chunks(T, B);
     a.first_chunk = 0;
-    a.slab = la_slab(a.chunks, H, D, Dv, pc);
+    const bool tensor = chunked && status && pe_linear_attention_on_tensor_cores(proj, dtype, ld, v_off, H, D, Dv);
+    a.slab = la_slab(a.chunks, H, D, Dv, (pc ? LA_CHANNELS : 0) | (tensor ? LA_TENSOR : 0) | (act_v ? LA_VALUES : 0));
     a.chunk_state = scratch;
     a.chunk_decay = scratch ? scratch + (size_t)a.slab * H * D * Dv : nullptr;
     a.channel_scratch = scratch ? scratch + ((size_t)a.slab * H * D * ((size_t)Dv + 1) + 3) / 4 * 4 : nullptr;      // (read in vectors)
     a.chunk_planes = nullptr;
-    if (chunked && status && pe_linear_attention_on_tensor_cores(proj, dtype, ld, v_off, H, D, Dv)) {
-        const LATensorScratch at(a.slab, H, D, Dv);
+    if (tensor) {
+        const LATensorScratch at(a.slab, H, D, Dv, act_v != 0);
         if (!at.aligned()) return PE_ERR_UNSUPPORTED;
         char* base = reinterpret_cast<char*>(scratch);
         a.chunk_planes = reinterpret_cast<unsigned char*>(base);

@@ -82,4 +82,4 @@ int la_channels_contributions(const LAArgs& a, bool f32, bool z_f32, float* scra
 int la_channels_outputs(const LAArgs& a, bool f32, float* scratch, cudaStream_t s);
 // Both on the tensor cores (linear_attention_tcgen05.cu), all of a slab's launches; and the floats of scratch that a chunk takes beside its states and decays.
 int la_tensor_chunks(const LAArgs& a, int types, int z_types, cudaStream_t s);
-long long la_tensor_chunk_floats(int H, int D);
+long long la_tensor_chunk_floats(int H, int D, bool values);      // values: they go through an activation

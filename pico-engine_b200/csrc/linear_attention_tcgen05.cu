@@ -25,12 +25,13 @@
 #define LM_SMEM (12 * CM_PLANE + 1024)                    // parts of Q (or of W) and of S (or the values), both halves
 
 // A unit's parts in scratch: queries and keys, [part][two][64 tokens][64 channels] each (two: the channels' halves, or the heads), and weights
-// [part][heads][64 t][64 s]; and values behind their activation, [part][half][64 s][64 columns].
+// [part][heads][64 t][64 s]; and values behind their activation, if there is one, [part][half][64 s][64 columns].
 template <bool TWO> struct LMUnit {
     static constexpr int ND = TWO ? 64 : 128;             // rows of a head's state
-    static constexpr int QUERIES = 0, KEYS = 6 * CM_PLANE, WEIGHTS = 12 * CM_PLANE, W_HEADS = TWO ? 2 : 1, VALUES = (12 + 3 * W_HEADS) * CM_PLANE, BYTES = VALUES + 6 * CM_PLANE;
+    static constexpr int QUERIES = 0, KEYS = 6 * CM_PLANE, WEIGHTS = 12 * CM_PLANE, W_HEADS = TWO ? 2 : 1, VALUES = (12 + 3 * W_HEADS) * CM_PLANE;
+    static __host__ __device__ __forceinline__ constexpr size_t bytes(bool values) { return VALUES + (values ? 6 * CM_PLANE : 0); }
     // of a head h
-    static __device__ __forceinline__ unsigned char* of(const LAArgs& a, int c, int h) { return a.chunk_planes + ((size_t)c * (TWO ? a.H / 2 : a.H) + (TWO ? h / 2 : h)) * BYTES; }
+    static __device__ __forceinline__ unsigned char* of(const LAArgs& a, int c, int h) { return a.chunk_planes + ((size_t)c * (TWO ? a.H / 2 : a.H) + (TWO ? h / 2 : h)) * bytes(a.act_v != 0); }
 };
 
 // Tiles of a chunk's and head's word: 0 queries, 1 keys (with one decay a head), 2 weights, 3 values; of numbers alone (cm_watch_numbers) 4 keys times their decays, 5 values.
@@ -745,8 +746,8 @@ static int lm_run(LAArgs a, int types, int z_types, cudaStream_t s) {
     return 0;
 }
 
-long long la_tensor_chunk_floats(int H, int D) {                      // a chunk's parts, words and place
-    const long long parts = D == 128 ? (long long)H * LMUnit<false>::BYTES : (long long)H / 2 * LMUnit<true>::BYTES;
+long long la_tensor_chunk_floats(int H, int D, bool values) {         // a chunk's parts, words and place
+    const long long parts = D == 128 ? (long long)H * LMUnit<false>::bytes(values) : (long long)H / 2 * LMUnit<true>::bytes(values);
     return parts / 4 + 2 * H + 2;
 }
 int la_tensor_chunks(const LAArgs& a, int types, int z_types, cudaStream_t s) {

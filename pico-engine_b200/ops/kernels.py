@@ -1170,8 +1170,8 @@ def linear_attention(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, n_h
     ws, launches = None, 1
     if chunked:
         from .workspace import scratch
-        sizes = (T, B, H, D, Dv, 0 if decay_logits is None else 1)
         tensor_cores = lib.pe_linear_attention_on_tensor_cores(proj.data_ptr(), _code(proj, "proj"), ld, v_off, H, D, Dv)
+        sizes = (T, B, H, D, Dv, (0 if decay_logits is None else 1) | (2 if tensor_cores else 0) | (4 if LA_ACTIVATIONS[v_activation] else 0))
         launches = (4 if tensor_cores or decay_logits is not None else 3) * lib.pe_linear_attention_slabs(*sizes)
         ws = scratch("linear_attention", 4 * lib.pe_linear_attention_scratch_floats(*sizes), proj.device).data_ptr()
     check(lib.pe_linear_attention(proj.data_ptr(), _code(proj, "proj"), ld, q_off, k_off, v_off, _ptr(decay_logits),

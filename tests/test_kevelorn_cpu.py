@@ -150,8 +150,22 @@ def test_scratch_of_a_batch_of_prompts_is_bounded(per_channel):
 
 
 @pytest.mark.parametrize("per_channel", [0, 1])
+def test_scratch_is_what_the_way_of_a_step_takes(per_channel):
+    """Float32 rows have no parts and rows without an activation on the values none of those: neither pays for them with smaller slabs."""
+    from pico_engine.ops.library import gated
+    lib, H, D = gated(), 16, 128
+    adds, parts, values = (lib.pe_linear_attention_scratch_floats(200, 1, H, D, D, per_channel | kind) - 8 for kind in (0, 2, 6))
+    state = 5 * H * D * (D + 1)
+    assert adds == state + per_channel * 5 * H * (64 * 64 + 2 * 64 * D)
+    assert parts == state + 5 * (H * 15 * 8192 // 4 + 2 * H + 2) and values - parts == 5 * H * 6 * 8192 // 4
+    T = 64 * (253 if per_channel == 0 else 108)
+    assert [lib.pe_linear_attention_slabs(T, 1, H, D, D, per_channel | kind) for kind in (0, 2, 6)] == ([1, 3, 4] if per_channel == 0 else [1, 2, 2])
+
+
+@pytest.mark.parametrize("values", [0, 4])
+@pytest.mark.parametrize("per_channel", [0, 1])
 @pytest.mark.parametrize("D", [64, 128])
-def test_scratch_of_the_tensor_cores_is_aligned_for_what_reads_it(D, per_channel):
+def test_scratch_of_the_tensor_cores_is_aligned_for_what_reads_it(D, per_channel, values):
     """Any number of heads and chunks, odd ones too: parts and states start where 16 and 32 bytes are read at once, a chunk's place where 8 are,
     nothing overlaps and all of it lies in the scratch."""
     import ctypes
@@ -160,14 +174,14 @@ def test_scratch_of_the_tensor_cores_is_aligned_for_what_reads_it(D, per_channel
     for H in range(1, 17):
         for chunks in range(2, 200):
             T = 64 * (chunks - 1)
-            sizes = (T, 1, H, D, D, per_channel)
+            sizes = (T, 1, H, D, D, per_channel | 2 | values)
             if not lib.pe_linear_attention_scratch_places(*sizes, ctypes.addressof(places)):
                 assert D == 64 and H % 2
                 continue
             rows, seen, state, decay, end = places
             slab = -(-chunks // lib.pe_linear_attention_slabs(*sizes))
             assert rows % 16 == 0 and seen % 4 == 0 and state % 32 == 0 and decay % 16 == 0, (H, chunks)
-            planes = (12 + 3 * (1 if D == 128 else 2) + 6) * 8192 * (H if D == 128 else H // 2)
+            planes = (12 + 3 * (1 if D == 128 else 2) + (6 if values else 0)) * 8192 * (H if D == 128 else H // 2)
             assert rows >= slab * planes and seen - rows >= 8 * slab and state - seen >= 8 * slab * H and decay - state >= 4 * slab * H * D * D
             assert end - decay >= 4 * slab * H * D and end <= 4 * lib.pe_linear_attention_scratch_floats(*sizes), (H, chunks)
 
