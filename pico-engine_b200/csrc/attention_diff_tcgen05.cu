@@ -7,8 +7,8 @@
 //               products while the softmax warps work on the other's scores
 //   warp 0      loader: TMA tiled loads (128-byte swizzle) of both maps' queries and, every second step, of two pages' keys of both
 //               maps and of the values they share into a ring of two stages; it alone reads the page table
-//   warp 1      allocates tensor memory (two S buffers and two accumulators of up to 128 columns: one of each a map); one lane
-//               issues S = Q_m K_m^T and O_m += P V, S of the next step before P V of this one
+//   warp 1      allocates tensor memory (two S buffers and two accumulators of up to 128 columns: one of each a map); an elected
+//               thread issues S = Q_m K_m^T and O_m += P V, S of the next step before P V of this one
 //   warps 2-9   softmax, two threads a query row, one for each page of the step, with a running maximum and sum a map; at the end
 //               each thread has half of both maps' rows in registers, forms the difference, meets its partner for the sum of
 //               squares and stores its half
@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) attention_diff_tcgen05_kernel(c
         }
     } else if (warp == 1) {
         {                                                           // ---------------- MMA issuer: the warp waits, one thread issues
-            const unsigned elected = at_elect();
+            const unsigned elected = pe_elect();
             // instruction descriptors: float32 accumulator, bfloat16 operands, M = 128; S: A and B K-major, N = 128 keys;
             // O: B MN-major (bit 16), N = Dv rounded up to 16
             const unsigned idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)((2 * DT_KTILE) >> 3) << 17) | ((unsigned)(DT_QTILE >> 4) << 24);

@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) attention_latent_tcgen05_kernel
         }
     } else if (warp == 1) {
         {                                                           // ---------------- MMA issuer: the warp waits, one thread issues
-            const unsigned elected = at_elect();
+            const unsigned elected = pe_elect();
             // instruction descriptors: float32 accumulator, bfloat16 operands, M = 128; S: A and B K-major, N = 128 keys;
             // O: A from tensor memory, B MN-major (bit 16), N = rank
             const unsigned idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)((2 * LT_KTILE) >> 3) << 17) | ((unsigned)(LT_QTILE >> 4) << 24);

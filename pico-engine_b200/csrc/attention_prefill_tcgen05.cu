@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attention_prefill_tcgen05_kerne
         }
     } else if (warp == 1) {
         {                                                           // ---------------- MMA issuer: the warp waits, one thread issues
-            const unsigned elected = at_elect();
+            const unsigned elected = pe_elect();
             // instruction descriptors: float32 accumulator, bfloat16 operands, M = 128;
             // S: A and B K-major, N = 128 keys;  O: B MN-major (bit 16), N = head size
             const unsigned idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)((2 * AT_KTILE) >> 3) << 17) | ((unsigned)(AT_QTILE >> 4) << 24);

@@ -195,11 +195,6 @@ __device__ __forceinline__ CMOperand cm_across(unsigned at, int stride, int seco
     const unsigned long long d = at_desc(at, second, 1024);
     return {d, d + (stride >> 4), d + 2 * (stride >> 4), 128u};
 }
-__device__ __forceinline__ unsigned cm_elect() {
-    unsigned r;
-    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(r));
-    return r;
-}
 __device__ __forceinline__ void cm_issue(unsigned elected, unsigned sums, unsigned long long a, unsigned long long b, unsigned idesc, bool add) {
     asm volatile("{\n .reg .pred e, p;\n setp.ne.u32 e, %0, 0;\n setp.ne.u32 p, %5, 0;\n"
                  " @e tcgen05.mma.cta_group::1.kind::f16 [%1], %2, %3, %4, p;\n}"

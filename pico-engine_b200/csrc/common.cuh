@@ -32,6 +32,22 @@ typedef __nv_bfloat16 bf16;
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// The thread of a warp that issues for it (products on the tensor cores and their commits); the whole warp calls.
+__device__ __forceinline__ unsigned pe_elect() {
+    unsigned r;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(r));
+    return r;
+}
+// SMs of the device, for grids whose blocks stay.
+inline int pe_sm_count() {
+    static int n = 0;
+    if (!n) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+    }
+    return n;
+}
+
 inline int& pe_pdl_enabled() { static int on = 1; return on; }
 
 template <typename... KArgs, typename... Args>

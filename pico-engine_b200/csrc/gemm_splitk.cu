@@ -365,15 +365,6 @@ __global__ void __launch_bounds__(GS_THREADS, 1) gemm_splitk_kernel(const __grid
 }
 
 // ---------------------------------------------------------------- host side
-static int gs_sm_count() {
-    static int n = 0;
-    if (!n) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-    }
-    return n;
-}
-
 static size_t gs_smem_bytes(int ksplit, int stages) {
     return 1024 + (size_t)stages * GS_STAGE + GS_TILE_BYTES + (ksplit > 1 ? (size_t)(ksplit - 1) * 2 * (64 / ksplit) * GS_BN * 4 : 0);
 }
@@ -419,7 +410,7 @@ static int gs_launch(GsArgs& a, const void* A, const void* W, int box_rows, int 
     const int blocks = (a.K + GS_BK - 1) / GS_BK;
     int split = GS_MAX_SPLIT;
     for (; split > 1; split >>= 1) {
-        if (split > blocks || tiles * split > gs_sm_count()) continue;
+        if (split > blocks || tiles * split > pe_sm_count()) continue;
         const int per = (blocks + split - 1) / split;
         if ((blocks + per - 1) / per != split) continue;     // (a range would be empty)
         const int at_once = gs_clusters_at_once<EPI>(split, gs_stages(split, per));

@@ -85,11 +85,6 @@ __device__ __forceinline__ unsigned long long gt_desc(unsigned smem_addr) {
     return (unsigned long long)((smem_addr >> 4) & 0x3FFFu) | ((unsigned long long)(1024u >> 4) << 32) |
            (1ull << 46) | (2ull << 61);
 }
-__device__ __forceinline__ unsigned gt_elect() {
-    unsigned r;
-    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(r));
-    return r;
-}
 // The four products of a stage (16 columns of K each, 32 bytes further inside the swizzle atom) by the elected thread; the whole warp calls, so
 // that descriptors and addresses are the warp's and not one lane's.  Issued by one lane in a branch of its own, a stage of 128 x 128 x 64 took 560 cycles, its bytes
 // 500 and its products 256; this way q/k/v of 2,048 rows (896 x 1,152) 10.3 -> 8.8 us, 4,864 -> 896 27.0 -> 22.5, 896 -> 896 8.7 -> 7.5; 8,192 rows 25.8 -> 22.1, 98 -> 89,
@@ -475,7 +470,7 @@ __global__ void __launch_bounds__(GT_THREADS) gemm_tcgen05_kernel(const __grid_c
         }
     } else if (warp == 1) {
         {                                                           // ---------------- MMA issuer: the warp waits, one thread issues
-            const unsigned elected = gt_elect();
+            const unsigned elected = pe_elect();
             // instruction descriptor: float32 accumulator, bfloat16 A and B, both K-major, N = BN (or a part's columns), M = 128
             int s = 0;
             unsigned round = 0;
@@ -659,7 +654,7 @@ __global__ void __launch_bounds__(GT_THREADS) gemm_tcgen05_pair_kernel(const __g
         }
     } else if (warp == 1) {
         if (rank == 0) {                                            // ---------------- MMA issuer (even CTA): the warp waits, one thread issues
-            const unsigned elected = gt_elect();
+            const unsigned elected = pe_elect();
             // instruction descriptor: float32 accumulator, bfloat16 A and B, both K-major, N = BN, M = 256 over the pair
             const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) | ((unsigned)(256 >> 4) << 24);
             int s = 0;
@@ -723,15 +718,6 @@ static int gt_make_map(CUtensorMap* map, const void* base, long long rows, long 
     return pe_tensor_map_2d(map, base, rows, cols, box_rows, box_cols, f32);
 }
 
-static int gt_sm_count() {
-    static int n = 0;
-    if (!n) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-    }
-    return n;
-}
-
 template <bool SWAP, int BN, int EPI>
 static int gt_launch(const void* A, const void* W, GtArgs& p, int* status, cudaStream_t s) {
     constexpr int NA = (SWAP && EPI == GT_SWIGLU) ? 2 : 1;
@@ -763,7 +749,7 @@ static int gt_launch(const void* A, const void* W, GtArgs& p, int* status, cudaS
     p.whole = p.tiles; p.parts = 1;
     CUtensorMap mp = mw;
     if (EPI == GT_SWIGLU && !SWAP) {
-        const int sms = gt_sm_count(), rest = p.tiles % sms;
+        const int sms = pe_sm_count(), rest = p.tiles % sms;
         p.parts = rest == 0 ? 1 : 4 * rest <= sms ? 4 : 2 * rest <= sms ? 2 : 1;
         if (p.parts > 1) {
             p.whole = p.tiles - rest; p.tiles = p.whole + rest * p.parts;
@@ -771,7 +757,7 @@ static int gt_launch(const void* A, const void* W, GtArgs& p, int* status, cudaS
             if (rc) return rc;
         }
     }
-    const int ctas = p.tiles < gt_sm_count() ? p.tiles : gt_sm_count();
+    const int ctas = p.tiles < pe_sm_count() ? p.tiles : pe_sm_count();
     PE_TRY(pe_launch(gemm_tcgen05_kernel<SWAP, BN, EPI>, dim3(ctas), GT_THREADS, smem, s, ma, mw, mo, mp, p, status));
     return 0;
 }
@@ -800,7 +786,7 @@ static int gt_launch_pair(const void* A, const void* W, GtArgs& p, int* status, 
         PE_TRY(cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         attr_set = true;
     }
-    const int max_pairs = gt_sm_count() / 2, pairs = p.tiles < max_pairs ? p.tiles : max_pairs;
+    const int max_pairs = pe_sm_count() / 2, pairs = p.tiles < max_pairs ? p.tiles : max_pairs;
     PE_TRY(pe_launch_cluster(gemm_tcgen05_pair_kernel<BN, EPI>, dim3(2 * pairs), GT_THREADS, smem, s, 2u, ma, mw, mo, p, status));
     return 0;
 }

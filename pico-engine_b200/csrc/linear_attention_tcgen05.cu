@@ -1,5 +1,5 @@
 // Linear attention of prompts as products of tiles on the 5th-generation tensor cores (linear_attention_tiles.cu and
-// linear_attention_channels.cu have the same with multiply-adds, and the sums that are worked out; chunk_mma.cuh how float32 numbers are
+// linear_attention_channels.cu have the same with multiply-adds, and the sums; chunk_mma.cuh how float32 numbers are
 // multiplied).  bfloat16 rows, heads of 128 x 128, or an even number of heads of 64 x 64.
 //
 // A first kernel a kind of decay works out what does not depend on the state and leaves it as bfloat16 parts: the chunk's queries (times their decays
@@ -13,11 +13,11 @@
 // A state in scratch is [half of the unit's columns][D / 8][64 v][8 d], so that a thread writes and reads runs of 32 bytes and a warp whole lines.
 //
 // Contributions and outputs only copy, multiply and store (outputs cut the state): what bounds them is the parts' way from L2.  Measured on a B200, 2,048
-// tokens, 16 heads of 128 x 128, us: a decay a head and silu on queries, keys and values 122 as multiply-adds, 93 here (operands 36,
-// contributions 15, carry 10, outputs 29); a decay a channel 175 and 103 (54, 12, 10, 23).  14 heads of 64: 57 and 43, 76 and 49; 200 tokens of those 34 and
-// 26, 43 and 29; three prompts of 300, 500 and 33, 16 heads 67 and 48, 92 and 54: these sizes always come here.  Errors against 64 bits, of the
-// outputs' norm: 2.1e-7 as multiply-adds and 6.3e-8 here, with a decay a channel 2.0e-7 and 1.6e-7 (its weights are the same sums); of the states 1.0e-7 and 6.1e-8,
-// 1.44e-7 and 1.28e-7.
+// tokens, 16 heads of 128 x 128, us: a decay a head and silu on queries, keys and values 121 as multiply-adds, 93 here (operands 36,
+// contributions 15, carry 10, outputs 29); a decay a channel 174 and 104 (54, 12, 10, 23).  14 heads of 64: 57 and 45, 76 and 49; 200 tokens of those 34 and
+// 26, 43 and 29; three prompts of 300, 500 and 33, 16 heads 67 and 49, 91 and 55: steps that go in chunks at all (LinearAttention.chunks_pay) are sooner here.
+// Errors against 64 bits, of the outputs' norm: 2.1e-7 as multiply-adds and 6.3e-8 here, with a decay a channel 2.0e-7 and 1.6e-7 (its weights are the same
+// sums); of the states 1.0e-7 and 6.1e-8, 1.44e-7 and 1.28e-7.
 #include "linear_attention.cuh"
 #include "chunk_mma.cuh"
 
@@ -478,7 +478,7 @@ __global__ void __launch_bounds__(LM_THREADS, TWO || VALUE_PARTS == 3 ? 3 : 2) l
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), per = TWO ? a.H / 2 : a.H;
     const int q = warp & 3, hh = q >> 1, p = (q & 1) * 32 + lane;
     const unsigned tmem = cm_begin(&tmem_s, &bar);
-    const unsigned elected = warp == 0 ? cm_elect() : 0u;
+    const unsigned elected = warp == 0 ? pe_elect() : 0u;
     pdl_wait();
     unsigned phase = 0;
     int2 place = a.chunk_rows[blockIdx.x / per];
@@ -603,7 +603,7 @@ __global__ void __launch_bounds__(LM_THREADS, 2) lm_output_kernel(LAArgs a, int 
     const bool scaled = a.z == nullptr;                               // one decay a head: the decay to a token behind the products
     if (tid == 0) odd = 0;
     const unsigned tmem = cm_begin(&tmem_s, &bar), mine = tmem + ((unsigned)(q * 32) << 16) + column + (TWO ? hh * 64 : 0);
-    const unsigned elected = warp == 0 ? cm_elect() : 0u;
+    const unsigned elected = warp == 0 ? pe_elect() : 0u;
     pdl_wait();
     unsigned phase = 0, known = 0;
     int2 place = a.chunk_rows[blockIdx.x / per];
@@ -719,7 +719,7 @@ __global__ void __launch_bounds__(LM_THREADS, 2) lm_output_kernel(LAArgs a, int 
 
 template <bool TWO, int VP>
 static int lm_run(LAArgs a, int types, int z_types, cudaStream_t s) {
-    const int units = a.slab * (TWO ? a.H / 2 : a.H), blocks = units < 2 * 148 ? units : 2 * 148;
+    const int units = a.slab * (TWO ? a.H / 2 : a.H), blocks = units < 2 * pe_sm_count() ? units : 2 * pe_sm_count();
     PE_TRY(cudaFuncSetAttribute(lm_contribution_kernel<TWO, VP>, cudaFuncAttributeMaxDynamicSharedMemorySize, LM_SMEM));
     PE_TRY(cudaFuncSetAttribute(lm_output_kernel<TWO, VP>, cudaFuncAttributeMaxDynamicSharedMemorySize, LM_SMEM));
     const int size = types == 2 ? 4 : 2;

@@ -426,15 +426,6 @@ __global__ void __launch_bounds__(LB_THREADS, 1) linear_batch_kernel(const __gri
 // ---------------------------------------------------------------- host side
 extern "C" void pe_set_pdl(int on) { pe_pdl_enabled() = on ? 1 : 0; }     // (this library's own copy of the switch)
 
-static int lb_sm_count() {
-    static int n = 0;
-    if (!n) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-    }
-    return n;
-}
-
 static size_t lb_gather_bytes(int ksplit) { return ksplit > 1 ? (size_t)(ksplit - 1) * (LB_TW * LB_TM + LB_TM) * 4 : 0; }
 static int lb_stages(int ksplit, int chunks_per_split) {
     const size_t budget = 224 * 1024;
@@ -480,8 +471,8 @@ static int lb_launch(LbArgs& a, const void* A, const void* W, int box_rows, int 
     // weights; but no more ranges than lets all clusters run at once (a GPU runs fewer CTAs in clusters than alone).
     const int chunks = (a.K + LB_KC - 1) / LB_KC;
     int split = 1;
-    if (tiles * 2 <= lb_sm_count()) {
-        split = lb_sm_count() / tiles;
+    if (tiles * 2 <= pe_sm_count()) {
+        split = pe_sm_count() / tiles;
         if (split > LB_MAX_SPLIT) split = LB_MAX_SPLIT;
         if (split > chunks) split = chunks;
         for (; split > 1; --split) {

@@ -146,11 +146,6 @@ __device__ __forceinline__ unsigned long long sp_desc(unsigned at) {
     return (unsigned long long)((at >> 4) & 0x3FFFu) | (1ull << 16) | ((unsigned long long)(512 >> 4) << 32) | (1ull << 46) | (4ull << 61);
 }
 
-__device__ __forceinline__ unsigned sp_elect() {
-    unsigned r;
-    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(r));
-    return r;
-}
 // The twelve products of a chunk, two steps of sixteen entries each.  hi hi go to `large`, an accumulator that starts at zero with every chunk, the
 // small ones to `small`, which starts with the first chunk (`more`: this is a later one).
 // w: columns of tensor memory, 16 of hi, of mid and of lo; a, a_mid, a_lo: descriptors.  The whole warp calls; the elected thread issues.
@@ -404,7 +399,7 @@ __global__ void __launch_bounds__(sp_threads<NT>(), 1) linear_split_kernel(const
         }
     } else if (warp == CUTTERS) {
         const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(nt / 8) << 17) | ((unsigned)(SP_ROWS / 16) << 24);
-        const unsigned elected = sp_elect();
+        const unsigned elected = pe_elect();
         int issued = 0, s = 0, turn = 0;
         for (int c = 0; c < chunks; ++c) {
             const int b = c % SUMS;

@@ -187,7 +187,7 @@ extern "C" long long pe_state_space_elems(int H, int P, int N) {
 }
 // Chunks a step of T tokens in B sequences can have at most; those that are worked on at a time, as many as SS_SCRATCH_FLOATS of scratch
 // hold (one at least), in slabs of equal size; and the floats of scratch that a slab needs.  A slab of the sizes that fill it keeps the GPU
-// full (64 heads of 64 columns, 128 state rows: 125 chunks, 8,000 blocks a launch), and batches of prompts need no more scratch than it.
+// full (64 heads of 64 columns, 128 state rows: 101 chunks on the tensor cores, 3,232 units of two heads a launch), and batches of prompts need no more scratch than it.
 #define SS_SCRATCH_FLOATS (64ll << 20)
 extern "C" int pe_state_space_chunks(int T, int B) { return (T + SS_CHUNK - 1) / SS_CHUNK + B; }
 static int ss_step_floats(int H, int P, int N, int G) { return ss_on_tensor_cores(H, P, N, G) ? SS_MATRIX_STEP_FLOATS : SS_STEP_FLOATS; }

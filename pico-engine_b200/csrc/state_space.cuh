@@ -21,8 +21,9 @@ struct ScanArgs {
     int B, H, P, N, G, NS, NR, NRP, PT;
     float* chunk_state;                       // [chunks][H][N][P]: a chunk's own contribution, then its incoming state
     float* chunk_decay;                       // [chunks][H]: the product of a chunk's decays
-    float* chunk_scores;                      // [chunks][G][64 s][64 t]: C_t . B_s
-    float* chunk_steps;                       // [chunks][H][SS_STEP_FLOATS]: 64 x (dt, dt * the decays behind it), then 64 running sums (float64)
+    float* chunk_scores;                      // [chunks][G][64 s][64 t]: C_t . B_s (tensor cores: [64 t][64 s])
+    float* chunk_steps;                       // [chunks][H][SS_STEP_FLOATS]: 64 x (dt, dt * the decays behind it), then 64 running sums (float64);
+                                              // tensor cores: [chunks][H][SS_MATRIX_STEP_FLOATS], SM_WS and on (state_space_tcgen05.cu)
     unsigned char* chunk_planes;              // tensor cores: [chunks][G][B, C][64 state rows at a time]: their bfloat16 parts (chunk_mma.cuh)
     unsigned* chunk_seen;                     // [chunks][G]: whether B has numbers that parts are not made of; from bit 16 on the first token where B or C has an entry that they are not made of (64: none)
     int* unit_exact;                          // [chunks][H / 2]: tokens of a chunk and two heads whose results come from parts

@@ -1,5 +1,5 @@
 // The state-space recurrence of prompts as products of tiles on the 5th-generation tensor cores (state_space_tiles.cu has the same with
-// multiply-adds, and the sums that are worked out; chunk_mma.cuh how float32 numbers are multiplied).  Heads of 64 columns, an even number of them a group, 64 or 128 state rows.
+// multiply-adds, and the sums; chunk_mma.cuh how float32 numbers are multiplied).  Heads of 64 columns, an even number of them a group, 64 or 128 state rows.
 //
 // Two heads of a group are the 128 rows of a product: their columns p stand on the accumulator's lanes, and what all heads of a group
 // share (B, C, cut into parts once a chunk and group) is the other operand:
@@ -7,14 +7,15 @@
 //   outputs        y^T [(h, p)][t] = a(-1, t) S^T C^T + x^T W_h^T      K: the state's rows, 64 at a time; then the chunk's tokens
 // W_h differs between the two heads: both heads' columns meet both heads' weights, and half of the results is left.
 //
-// A state in scratch is [N / 8][64 p][8 n], so that a thread writes and reads runs of 32 bytes and a warp whole lines.  Two CTAs of sixteen
+// A state in scratch is [N / 8][64 p][8 n], so that a thread writes and reads runs of 32 bytes and a warp whole lines.  Two CTAs of eight
 // warps an SM, 256 columns of tensor memory each: the loads, cuts and stores of one cover the waits of the other.
 //
 // What bounds it: outputs the chain of a unit (loads, cuts, products, weights: 25,000 cycles of which the products are 5,000; two blocks
 // an SM overlap), contributions and carry the state's way through L2 (5 to 10 TB/s).  Measured on a B200, 64 heads, 128 state rows,
-// rows of 1,400 and 647 tokens: 132 us (steps with parts and scores 12, contributions 27, carry 25, outputs 61) where multiply-adds take 187 (3, 61, 32, 94);
-// 28 heads, 2,500 tokens 74 (102), 8 heads, 65 tokens and one 28 (34), so these sizes always come here.  The error of the outputs against 64 bits is
-// 7.8e-8 of their norm (1.15e-7 by multiply-adds), of the states 7.8e-8 (6.9e-8; 28 heads 9.8e-8 and 1.02e-7): most of it the decays'.
+// rows of 1,400 and 647 tokens: 134.5 us (steps with parts and scores 12, contributions 27, carry 25, outputs 63) where multiply-adds take 187 (3, 61, 32, 94);
+// 28 heads, 2,500 tokens 76 (102), 8 heads, 65 tokens and one 28.7 (34.5): steps that go in chunks at all (StateSpace.chunks_pay) are sooner here whatever their size.
+// Errors against 64 bits, means over eight inputs, outputs and states of their norms (multiply-adds): 64 heads, 128 state rows, rows of 1,400 and 647 tokens 7.9e-8
+// and 9.1e-8 (1.09e-7 and 9.3e-8); 28 heads, 64 state rows, rows of 700 and 100 4.7e-8 and 1.00e-7 (6.3e-8 and 1.04e-7): most of it the decays' and the steps'.
 // With mma.sync in place of tcgen05 contributions took 50 and outputs 99 us (the fragments' loads and cuts between the products); an exponential for
 // each pair of tokens outputs 71 us; sixteen warps a block instead of eight contributions 35 and outputs 66 us.
 #include "state_space.cuh"
@@ -236,7 +237,7 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_contribution_kernel(ScanArgs a, 
     const int q = warp & 3, hh = q >> 1, p = (q & 1) * 32 + lane, row = tid >> 3, group = tid & 7;      // a thread's runs of eight: this row and the one 32 behind, of either head
     if (tid == 0) odd = 0;
     const unsigned tmem = cm_begin(&tmem_s, &bar);
-    const unsigned elected = warp == 0 ? cm_elect() : 0u;
+    const unsigned elected = warp == 0 ? pe_elect() : 0u;
     pdl_wait();
     unsigned phase = 0, known = 0;
     int2 place = a.chunk_rows[blockIdx.x / pairs];
@@ -390,7 +391,7 @@ __global__ void __launch_bounds__(SM_FEW, 2) sm_output_kernel(ScanArgs a, int ve
     const int q = warp & 3, hh = q >> 1, p = (q & 1) * 32 + lane, column = (warp >> 2) * 32, row = tid >> 3, group = tid & 7;
     if (tid == 0) odd = 0;
     const unsigned tmem = cm_begin(&tmem_s, &bar), mine = tmem + ((unsigned)(q * 32) << 16) + column;
-    const unsigned elected = warp == 0 ? cm_elect() : 0u;
+    const unsigned elected = warp == 0 ? pe_elect() : 0u;
     pdl_wait();
     unsigned phase = 0, known = 0;
     int2 place = a.chunk_rows[blockIdx.x / pairs];
@@ -546,7 +547,7 @@ static int sm_run(ScanArgs a, int* status, cudaStream_t s) {
     PE_TRY(cudaFuncSetAttribute(sm_steps_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * SM_SLAB));
     PE_TRY(cudaFuncSetAttribute(sm_contribution_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SM_CONTRIBUTION_SMEM));
     PE_TRY(cudaFuncSetAttribute(sm_output_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SM_OUTPUT_SMEM));
-    const int units = a.slab * (a.H / 2), blocks = units < 2 * 148 ? units : 2 * 148;
+    const int units = a.slab * (a.H / 2), blocks = units < 2 * pe_sm_count() ? units : 2 * pe_sm_count();
     for (; a.first_chunk < a.chunks; a.first_chunk += a.slab) {      // (the carry between two slabs lies in the sequences' states)
         PE_TRY(pe_launch(sm_steps_kernel<T>, dim3(a.slab, a.G + (a.H + 7) / 8), SM_THREADS, 2 * SM_SLAB, s, a, vec));
         PE_LAUNCH_CHECK();

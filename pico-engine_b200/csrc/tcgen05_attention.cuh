@@ -36,14 +36,9 @@ __device__ __forceinline__ unsigned long long at_desc(unsigned smem_addr, unsign
     return (unsigned long long)((smem_addr >> 4) & 0x3FFFu) | ((unsigned long long)((lbo >> 4) & 0x3FFFu) << 16) |
            ((unsigned long long)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46) | (2ull << 61);
 }
-// The thread of a warp that issues products and their commits.  The warp goes through the loop that issues them as one, waits included: in a branch
+// Products and commits are issued by a warp's elected thread (pe_elect).  The warp goes through the loop that issues them as one, waits included: in a branch
 // of one lane's own a product took about 90 cycles to issue.  The kernels themselves gain little (2,048 tokens, 14 heads of 64: 21.9 -> 21.6 us; differential attention 47.9 -> 47.1;
 // latent rows and mixed heads the same), in a chain of kernels the mixer with latent rows 98.2 -> 95.9 us, with mixed heads 71.5 -> 69.9.
-__device__ __forceinline__ unsigned at_elect() {
-    unsigned r;
-    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(r));
-    return r;
-}
 __device__ __forceinline__ void at_mma(unsigned elected, unsigned tmem_d, unsigned long long a, unsigned long long b, unsigned idesc, unsigned accumulate) {
     asm volatile("{\n .reg .pred p, e;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 e, %5, 0;\n"
                  " @e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"

@@ -1140,7 +1140,7 @@ def linear_attention(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, n_h
     ``q_off``, ``k_off``, ``v_off`` of proj [T, ld] (packed sequences).  The decay is ``head_decay`` [H] float32 (one constant
     a head) or sigmoid(``decay_logits`` [T, H * D], float32 or of proj's dtype)^``inv_tau`` (a number per key channel and token).  S [H, D, Dv] comes from
     and returns to the sequences' float32 state at ``state_offset``.  ``chunked``: prompts, in slabs of chunks of the sequences, three
-    launches a slab (four with a decay per channel, and on the tensor cores); else token after token in one launch.  ``qk`` (float32 [T, ld2], with a decay per head): q and k are the columns
+    launches a slab (four with a decay per channel, and on the tensor cores, csrc/linear_attention_tcgen05.cu); else token after token in one launch.  ``qk`` (float32 [T, ld2], with a decay per head): q and k are the columns
     ``q_off`` and ``k_off`` of these rows instead (rotated ones, that are not rounded on their way into the recurrence)."""
     T, ld = proj.shape
     H, D, Dv = n_heads, head_dim, v_head_dim

@@ -118,13 +118,16 @@ class LinearAttention(Mixer, SharedProducts):
         token after token; either way gives the same numbers up to float32 rounding.
 
         A walk is a block a row, head and 64 (or 32) columns: it takes as long as the longest row, and as all rows' tokens take where there
-        are more blocks than run side by side.  Tiles cost four launches, every chunk its products whatever it holds, and every row the pass that
-        carries its state.  The numbers (for microseconds on a B200) are fitted so that the two cross where they were measured to, for 1 to 64 rows of 8
-        to 2,048 tokens: with a decay per channel, 16 heads of 128 x 128, walk / tiles: 1 x 17 tokens 10 / 51 us, 1 x 128 53 / 61, 1 x 256
-        103 / 69, 1 x 2,048 841 / 182; 4 x 128 70 / 88, 4 x 256 137 / 103; 64 x 17 102 / 600, 64 x 256 1,250 / 1,684, 63 single tokens beside
-        2,048 1,259 / 722.  With a decay per head: 1 x 128 39 / 52, 1 x 256 74 / 53; 64 x 17 77 / 499, 63 x 1 and 2,048 906 / 591.  Of 643
-        measured steps, heads of 40 to 256 among them, one choice costs 1.7 times the better way (16 x 128, 4 heads of 256 x 256), no other more
-        than a third."""
+        are more blocks than run side by side.  Tiles cost three or four launches, every chunk its products whatever it holds, and every row the pass that
+        carries its state.  The numbers (for microseconds on a B200) are fitted so that the two cross where they were measured to with multiply-add tiles,
+        which other sizes than those below and float32 rows still take, for 643 steps of 1 to 64 rows of 8 to 2,048 tokens, heads of 40 to 256 among them.
+
+        Heads of 128 (or an even number of 64) with bfloat16 rows have chunks on the tensor cores, which are sooner than that fit says, so that steps
+        near the line walk although chunks would be done before.  Walk / chunks now, us: a decay per channel, 16 heads of 128 x 128: 1 x 17 tokens 10 / 38,
+        1 x 96 39 / 34, 1 x 128 51 / 33, 1 x 256 100 / 35, 1 x 2,048 783 / 105; 4 x 128 67 / 52, 4 x 256 131 / 59; 64 x 17 90 / 358, 64 x 256
+        1,134 / 1,146, 63 single tokens beside 2,048 1,227 / 484.  A decay per head: 1 x 128 39 / 29, 1 x 256 76 / 34; 64 x 17 77 / 400, 63 x 1 and 2,048 892 / 461.
+        Of 96 such steps of four sizes the choice costs 1.5 times the better way at worst (1 x 128) and more than a fifth in four.
+        """
         longest = max(lens, default=0)
         if longest <= 16:                                                     # (the walk wherever it was measured)
             return False

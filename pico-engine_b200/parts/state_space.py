@@ -79,9 +79,14 @@ class StateSpace(Mixer):
         A walk takes as long as the longest row, and as all rows' tokens take where there are more blocks (a row, head and as many columns as
         256 threads hold) than run side by side; tiles cost four launches, every chunk its products whatever it holds, and every row the
         pass that carries its state.  The numbers (for microseconds on a B200) are fitted to 339 steps of 1 to 64 rows of 8 to 2,048 tokens, 16
-        to 256 state rows and 8 to 112 heads; the worst choice among them costs a third more than the better way.  64
-        heads of 64 columns, 128 state rows, walk / tiles: 1 x 17 tokens 17 / 36 us, 1 x 64 53 / 43, 1 x 2,048 1,583 / 179; 8 x 32 86 / 97,
-        8 x 48 127 / 103; 64 x 17 356 / 873, 64 x 64 1,174 / 1,024; 63 single tokens beside 200 261 / 840, beside 2,048 2,036 / 982."""
+        to 256 state rows and 8 to 112 heads with multiply-add tiles, which other sizes than those below still take.
+
+        Heads of 64 columns, an even number of them a group, with 64 or 128 state rows have chunks on the tensor cores, which are sooner than that fit
+        says, so that some steps walk although chunks would be done before.  Walk / chunks now, us: 64 heads, 128 state rows: 1 x 17 tokens 16 / 30, 1 x 64 49 / 30,
+        1 x 2,048 1,522 / 142; 4 x 32 55 / 43; 64 x 17 353 / 444, 64 x 32 602 / 443, 64 x 64 1,166 / 545; 63 single tokens beside 200 254 / 449, beside 512 548 / 462,
+        beside 2,048 2,020 / 562.  16 heads, 64 state rows: 16 x 64 55 / 30, 63 single tokens beside 200 129 / 74.  Of 72 such steps of three sizes the choice
+        costs 1.9 times the better way at worst and more than a fifth in five.
+        """
         longest = max(lens, default=0)
         if longest <= 16:                                                     # (the walk wherever it was measured)
             return False
