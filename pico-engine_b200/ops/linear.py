@@ -161,16 +161,15 @@ def linear(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
             # A sum that may wait costs the norm that follows a part of its pass only, so each side is timed with that norm: 2,048 rows of
             # 896 x 896 7.7 / 8.4 us with a pass for the sum, 11.4 / 10.1 as they run; 8,192 of 3,584 x 3,584 151 / 174 and 190 / 183.
             key = ("accumulate" if defer_add is None else "accumulate_normed", Choice.bucket(M), w.shape[0], w.shape[1])
-
-            def sides():
-                rows, cols = Choice.bucket(M), w.shape[0]
-                sa, sx = _scratch_rows(rows, a.shape[1], a.dtype, a.device), _scratch_rows(rows, cols, torch.float32, a.device)
-                if defer_add is None:
-                    return (lambda: kernels.gemm_tcgen05(sa, w, accumulate_into=sx)), (lambda: kernels.residual_add(sx, torch.mm(sa, w.t())))
-                weight = torch.ones(cols, dtype=a.dtype, device=a.device)
-                return (lambda: kernels.rmsnorm(kernels.gemm_tcgen05(sa, w, accumulate_into=sx), weight, 1e-6, a.dtype)), \
-                       (lambda: kernels.add_rmsnorm(sx, torch.mm(sa, w.t()), weight, 1e-6, a.dtype))
             if key not in Choice.table:
+                def sides():
+                    rows, cols = Choice.bucket(M), w.shape[0]
+                    sa, sx = _scratch_rows(rows, a.shape[1], a.dtype, a.device), _scratch_rows(rows, cols, torch.float32, a.device)
+                    if defer_add is None:
+                        return (lambda: kernels.gemm_tcgen05(sa, w, accumulate_into=sx)), (lambda: kernels.residual_add(sx, torch.mm(sa, w.t())))
+                    weight = torch.ones(cols, dtype=a.dtype, device=a.device)
+                    return (lambda: kernels.rmsnorm(kernels.gemm_tcgen05(sa, w, accumulate_into=sx), weight, 1e-6, a.dtype)), \
+                           (lambda: kernels.add_rmsnorm(sx, torch.mm(sa, w.t()), weight, 1e-6, a.dtype))
                 Choice.pick(key, sides)
             if Choice.table.get(key) == "tcgen05":
                 return kernels.gemm_tcgen05(a, w, accumulate_into=accumulate_into)
@@ -201,11 +200,10 @@ def gate_up_act(h: torch.Tensor, w_gate_up: torch.Tensor, activation: str = "sil
         if _takes_tcgen05(h, w_gate_up):
             fused = True if activation == "silu" else activation
             key = ("swiglu" if activation == "silu" else activation + "_gate", Choice.bucket(M), w_gate_up.shape[0], w_gate_up.shape[1])
-
-            def sides():
-                sh = _scratch_rows(Choice.bucket(M), h.shape[1], h.dtype, h.device)
-                return (lambda: kernels.gemm_tcgen05(sh, w_gate_up, swiglu=fused)), (lambda: after(torch.mm(sh, w_gate_up.t())))
             if key not in Choice.table:
+                def sides():
+                    sh = _scratch_rows(Choice.bucket(M), h.shape[1], h.dtype, h.device)
+                    return (lambda: kernels.gemm_tcgen05(sh, w_gate_up, swiglu=fused)), (lambda: after(torch.mm(sh, w_gate_up.t())))
                 Choice.pick(key, sides, launches_saved=1)
             if Choice.table.get(key) == "tcgen05":
                 return kernels.gemm_tcgen05(h, w_gate_up, swiglu=fused)
@@ -230,18 +228,17 @@ def qkv_rope_store(h: torch.Tensor, w_qkv: torch.Tensor, b_qkv: Optional[torch.T
     kernel; or None where the product followed by the rotation kernel is faster (the caller then runs those)."""
     M = h.shape[0]
     key = ("rope", Choice.bucket(M), w_qkv.shape[0], w_qkv.shape[1], head_dim)
-
-    def sides():
-        rows = Choice.bucket(M)
-        sh = _scratch_rows(rows, h.shape[1], h.dtype, h.device)
-        pos = torch.zeros(rows, dtype=torch.int32, device=h.device)
-
-        def library():
-            y = linear(sh, w_qkv, b_qkv, out_dtype=h.dtype)
-            kernels.rope_store(y, n_q, n_kv, head_dim, cos, sin, pos, pos, None, None, None, 0)
-        # timed without the cache write on both sides (a scratch cache would have to be as large as the real one)
-        return (lambda: kernels.gemm_qkv_rope_store(sh, w_qkv, b_qkv, n_q, n_kv, head_dim, cos, sin, pos, pos, None, None, None, 0)), library
     if key not in Choice.table:
+        def sides():
+            rows = Choice.bucket(M)
+            sh = _scratch_rows(rows, h.shape[1], h.dtype, h.device)
+            pos = torch.zeros(rows, dtype=torch.int32, device=h.device)
+
+            def library():
+                y = linear(sh, w_qkv, b_qkv, out_dtype=h.dtype)
+                kernels.rope_store(y, n_q, n_kv, head_dim, cos, sin, pos, pos, None, None, None, 0)
+            # timed without the cache write on both sides (a scratch cache would have to be as large as the real one)
+            return (lambda: kernels.gemm_qkv_rope_store(sh, w_qkv, b_qkv, n_q, n_kv, head_dim, cos, sin, pos, pos, None, None, None, 0)), library
         Choice.pick(key, sides, launches_saved=1)
     if Choice.table.get(key) != "tcgen05":
         return None

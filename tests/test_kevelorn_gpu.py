@@ -784,3 +784,44 @@ def test_a_sequence_that_is_no_number_does_not_hold_up_the_others(per_channel):
             best = min(best, e0.elapsed_time(e1))
         return best
     assert time(bad) < 4 * time(proj)
+
+
+@pytest.mark.parametrize("per_channel", [False, True])
+def test_odd_heads_in_slabs_on_the_tensor_cores(per_channel):
+    """More chunks than the scratch holds at once, an odd number of them a slab and of heads; sequences that begin in one slab and end in the next."""
+    from pico_engine.ops.library import gated
+    H, D, lens = 5, 128, [5000, 64, 1, 5000, 4780]
+    kind = int(per_channel) | 2
+    chunks = -(-sum(lens) // 64) + len(lens)
+    assert gated().pe_linear_attention_slabs(sum(lens), len(lens), H, D, D, kind | 4) == 2 and -(-chunks // 2) % 2
+    proj, run = tensor_core_rows(H, D, lens, per_channel, 6)
+    for walk, out in zip(run(proj, False, v_activation="silu"), run(proj, True, v_activation="silu")):
+        # float32 sums of the same products in another order (the bound of the tests above)
+        assert (walk - out).abs().max() < 2e-5 * max(1.0, float(walk.abs().max()))
+
+
+@pytest.mark.parametrize("H,D,per_channel,most_o,most_state", [(14, 64, False, 1.6e-7, 1.06e-7), (14, 64, True, 1.7e-7, 1.35e-7), (3, 128, False, 2.0e-7, 1.0e-7), (3, 128, True, 2.0e-7, 1.4e-7)])
+def test_errors_are_no_larger_than_multiply_adds(H, D, per_channel, most_o, most_state):
+    """Outputs and states against 64 bits, beside their norms, means over four inputs; the bounds are what the multiply-add tiles leave of such inputs."""
+    from pico_engine.ops import kernels
+    T, errors = 200, []
+    first, rows, slots = (torch.tensor(v, dtype=torch.int32).cuda() for v in ([0, T], [T], [0]))
+    for seed in range(4):
+        g = torch.Generator("cuda").manual_seed(seed)
+        proj, z = torch.randn(T, 3 * H * D, generator=g, device="cuda").bfloat16(), (1.5 * torch.randn(T, H * D, generator=g, device="cuda")).bfloat16()
+        fixed, state = torch.tensor([1 - 2.0 ** -(3 + h % 6) for h in range(H)], device="cuda"), torch.zeros(1, H * D * D, device="cuda")
+        how = dict(decay_logits=z, inv_tau=1 / 16, q_scale=D ** -0.5) if per_channel else dict(head_decay=fixed, qk_activation="silu", v_activation="silu")
+        o = kernels.linear_attention(proj, 0, H * D, 2 * H * D, H, D, D, state, 0, first, rows, slots, True, **how)
+        q, k, v = (t.double().view(T, H, D) for t in proj.split(H * D, 1))
+        if per_channel:
+            q, decay = q * D ** -0.5, (torch.sigmoid(z.double()) ** (1 / 16)).view(T, H, D)
+        else:
+            q, k, v = (torch.nn.functional.silu(t) for t in (q, k, v))
+            decay = fixed.double().view(1, H, 1).expand(T, H, D)
+        S, want = torch.zeros(H, D, D, dtype=torch.float64, device="cuda"), torch.empty_like(v)
+        for t in range(T):
+            S = decay[t][:, :, None] * S + k[t][:, :, None] * v[t][:, None]
+            want[t] = (q[t][:, None] @ S)[:, 0]
+        errors.append([float((o.view(T, H, D) - want).norm() / want.norm()), float((state.view(H, D, D) - S).norm() / S.norm())])
+    e_o, e_state = np.mean(errors, 0)
+    assert e_o < most_o and e_state < most_state, (e_o, e_state)
