@@ -343,7 +343,7 @@ def agreement(config, seed: int, prompts: Sequence[Sequence[int]]) -> dict:
 def product_times(engine, rows: int) -> dict:
     """Device time of the first layer's four matrix products at ``rows`` rows, each as this library's tcgen05 kernel
     with its fused epilogue and as the library product followed by this library's separate kernel: the measurement
-    by which ``ops.linear`` chooses (a captured graph of six calls, best of three replays), in microseconds."""
+    by which ``ops.linear`` chooses (a captured graph of six calls, best of four replays), in microseconds."""
     import sys
     from .ops import kernels
     L = sys.modules[__package__ + ".ops.linear"]

@@ -32,12 +32,15 @@ def timed(monkeypatch):
     monkeypatch.setattr(kernels, "rmsnorm", note("norm", lambda x, w, eps, dtype: x.to(dtype)))
     monkeypatch.setattr(kernels, "add_rmsnorm", note("sum and norm", lambda x, y, w, eps, dtype: x.add_(y.float()).to(dtype)))
 
-    def device_time(fn):
-        seen.clear()
-        fn()
-        return cost[tuple(seen)]
+    def device_times(*fns):
+        out = []
+        for fn in fns:
+            seen.clear()
+            fn()
+            out.append(cost[tuple(seen)])
+        return out
 
-    monkeypatch.setattr(L, "_device_time", device_time)
+    monkeypatch.setattr(L, "_device_times", device_times)
     return cost
 
 
@@ -54,7 +57,7 @@ def test_a_sum_that_may_wait_is_timed_with_the_norm_behind_it(timed):
     assert L.Choice.timings == {("accumulate_normed", 512, 16, 8): (11.4, 10.1), ("accumulate", 512, 16, 8): (7.7, 8.4)}
 
 
-@pytest.mark.parametrize("own,taken", [(100.0, "library"), (99.0, "library"), (97.0, "library"), (95.0, "tcgen05"), (104.0, "library")])
+@pytest.mark.parametrize("own,taken", [(100.0, "library"), (99.0, "library"), (98.0, "library"), (95.0, "tcgen05"), (104.0, "library")])
 def test_a_near_tie_is_the_librarys(timed, own, taken):
     timed.update({("own",): own, ("sum",): 100.0})
     L.linear(A, W, accumulate_into=torch.zeros(300, 16))
